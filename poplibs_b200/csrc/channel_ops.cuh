@@ -1,0 +1,513 @@
+// Per-channel sums over, and element-wise maps with per-channel operands of,
+// device-layout activations [rows][chans] (NHWC: the channels of a pixel are
+// contiguous): what batch normalisation and the bias of a convolution are made
+// of.
+//
+// Every operation here moves each element once or twice and does a handful of
+// flops on it, so it is bound by memory as long as enough 16-byte accesses are
+// in flight and nothing is recomputed per element.  Both forms therefore view
+// the tensor as SUPER-ROWS: the fewest rows whose elements are a whole number of
+// 16-byte vectors (1 row if the channel count is a multiple of the vector, up to
+// 8 if it is odd).  A vector's place inside its super-row fixes which channels it
+// holds, so a thread that keeps one place and walks the super-rows keeps its
+// per-channel operands (or sums) in registers, loads whole vectors at any channel
+// count, and never divides.  Only the last, partial super-row is done element by
+// element.  A tensor whose base is not 16-byte aligned takes vectors of one element.
+#pragma once
+
+#include <cuda_fp16.h>
+
+#include <algorithm>
+
+#include "runtime.h"
+#include "sm100_prims.cuh"
+
+namespace plb {
+
+template <typename T> __device__ __forceinline__ float toFloat(T v);
+template <> __device__ __forceinline__ float toFloat<__half>(__half v) { return __half2float(v); }
+template <> __device__ __forceinline__ float toFloat<float>(float v) { return v; }
+template <typename T> __device__ __forceinline__ T fromFloat(float v);
+template <> __device__ __forceinline__ __half fromFloat<__half>(float v) { return __float2half_rn(v); }
+template <> __device__ __forceinline__ float fromFloat<float>(float v) { return v; }
+
+// A vector of V elements as it is loaded and stored.
+template <typename T, int V> struct ChanVec {
+  using Raw = uint4;
+  static_assert(V * sizeof(T) == 16, "a vector is 16 bytes, or one element");
+  static __device__ __forceinline__ void unpack(const Raw &v, float (&f)[V]) {
+    if constexpr (sizeof(T) == 2) {
+      const __half2 *h = reinterpret_cast<const __half2 *>(&v);
+#pragma unroll
+      for (int j = 0; j < V / 2; ++j) {
+        const float2 t = __half22float2(h[j]);
+        f[2 * j] = t.x;
+        f[2 * j + 1] = t.y;
+      }
+    } else {
+      f[0] = __uint_as_float(v.x);
+      f[1] = __uint_as_float(v.y);
+      f[2] = __uint_as_float(v.z);
+      f[3] = __uint_as_float(v.w);
+    }
+  }
+  static __device__ __forceinline__ Raw pack(const float (&f)[V]) {
+    Raw v;
+    if constexpr (sizeof(T) == 2) {
+      __half2 *h = reinterpret_cast<__half2 *>(&v);
+#pragma unroll
+      for (int j = 0; j < V / 2; ++j) h[j] = __floats2half2_rn(f[2 * j], f[2 * j + 1]);
+    } else {
+      v = make_uint4(__float_as_uint(f[0]), __float_as_uint(f[1]), __float_as_uint(f[2]), __float_as_uint(f[3]));
+    }
+    return v;
+  }
+};
+template <typename T> struct ChanVec<T, 1> {
+  using Raw = T;
+  static __device__ __forceinline__ void unpack(const Raw &v, float (&f)[1]) { f[0] = toFloat(v); }
+  static __device__ __forceinline__ Raw pack(const float (&f)[1]) { return fromFloat<T>(f[0]); }
+};
+
+// How [rows][chans] is walked.  A block is vec_lanes x row_lanes threads: thread
+// (vx, ry) owns vector `blockIdx.x * vec_lanes + vx` of the super-rows ry,
+// ry + stride, ... of its slab blockIdx.y.
+struct ChanWalk {
+  uint32_t chans;
+  uint32_t fold;             // rows per super-row
+  uint32_t vecs;             // vectors per super-row
+  uint32_t vec_lanes_log2;   // <= 5
+  uint32_t slabs;            // gridDim.y
+  unsigned long long full;   // whole super-rows
+  unsigned long long total;  // elements of the tensor
+};
+
+// `per_sm`: blocks of `threads` threads wanted per SM once there is work for them.
+inline ChanWalk chanWalk(const plb_context *ctx, uint64_t rows, uint32_t chans, uint32_t V, uint32_t threads,
+                         uint32_t per_sm, dim3 *grid) {
+  ChanWalk w{};
+  w.chans = chans;
+  uint32_t g = chans, t = V;  // gcd
+  while (t) {
+    const uint32_t u = g % t;
+    g = t;
+    t = u;
+  }
+  w.fold = V / g;
+  w.vecs = chans / g;  // = fold * chans / V
+  w.full = rows / w.fold;
+  w.total = rows * chans;
+  // vectors side by side in a block: at least 64 bytes of a row, as many as leave
+  // the fewest threads without a vector
+  while (w.vec_lanes_log2 < 2 && (1u << w.vec_lanes_log2) < w.vecs) ++w.vec_lanes_log2;
+  for (uint32_t l = w.vec_lanes_log2 + 1; l <= 5; ++l)
+    if (((w.vecs + (1u << l) - 1) >> l << l) <= ((w.vecs + (1u << w.vec_lanes_log2) - 1) >> w.vec_lanes_log2 << w.vec_lanes_log2))
+      w.vec_lanes_log2 = l;
+  const uint32_t lanes = 1u << w.vec_lanes_log2, row_lanes = threads >> w.vec_lanes_log2;
+  const uint32_t cols = (w.vecs + lanes - 1) / lanes;
+  // one super-row per thread while that leaves SMs idle, then a grid that is
+  // resident at once and walks
+  const uint64_t want = std::max<uint64_t>(1, (w.full + row_lanes - 1) / row_lanes);
+  const uint64_t cap = std::max<uint64_t>(1, uint64_t(ctx->sm_count) * per_sm / cols);
+  w.slabs = uint32_t(std::min<uint64_t>(std::min(want, cap), 65535));
+  *grid = dim3(cols, w.slabs);
+  return w;
+}
+
+// ---- sums ------------------------------------------------------------------------
+
+// What is added up per channel (two sums at once).
+enum ChanSums : int {
+  kSumXAndXX = 0,     // sum x, sum x^2
+  kSumCentredXX = 1,  // -, sum (x - centre[c])^2     (centre in the activations' type)
+  kSumXYAndY = 2,     // sum x * y, sum y             (whitened activations x gradients)
+  kSumX = 3,          // sum x, -
+};
+
+// What becomes of the sums: a = scale * first sum, b = scale * second sum.  Any
+// pointer may be null; *_half says which of the two types it points to.
+struct ChanFinish {
+  float scale;
+  void *a, *b;
+  float *a_f32, *b_f32;  // the same in fp32
+  int a_half, b_half;
+  // 1 / sqrt((b - a^2 + eps) * scale_var), a rounded to its type first
+  void *inv_std;
+  float eps, scale_var;
+  // bias[c] += a
+  void *bias;
+  int bias_half;
+};
+
+constexpr int kChanSumThreads = 1024;
+
+__device__ __forceinline__ void storeChan(void *p, int is_half, uint32_t c, float v) {
+  if (is_half)
+    static_cast<__half *>(p)[c] = __float2half_rn(v);
+  else
+    static_cast<float *>(p)[c] = v;
+}
+
+// One launch: every block leaves the sums of its slab as one row of the partial
+// matrices [slabs * fold][chans], and the block that finishes last adds the rows.
+// Rows are added in a fixed order, whichever block that is, so the result does
+// not depend on timing.  One block of 1024 threads per SM: few rows for the last
+// block to add, and 4 vectors per thread in flight are 9.7 MB over the device,
+// above the 5 MB that 6.5 TB/s times the memory latency asks for.
+// The last block's share is latency: it takes four channels per thread so that
+// all 148 rows are requested at once (one channel per thread: 3 us more at 128).
+// Sums of 200704 x 128 halves (51 MB): 40.5 us as two kernels whose second read
+// its 1184 partial rows one after the other, now 14.7; of 200704 x 512 (205 MB):
+// 54.9 us, now 38.0 (5.4 TB/s; a read-only stream gets 5.6 here).
+template <typename T, int kMode, int V>
+__global__ void __launch_bounds__(kChanSumThreads, 1)
+chanSumsKernel(const T *__restrict__ x, const T *__restrict__ y, const T *__restrict__ centre, const ChanWalk w,
+               float *__restrict__ partial_a, float *__restrict__ partial_b, unsigned *__restrict__ ticket,
+               const ChanFinish fin) {
+  using Vec = ChanVec<T, V>;
+  using Raw = typename Vec::Raw;
+  constexpr bool kHasA = kMode != kSumCentredXX, kHasB = kMode != kSumX, kHasY = kMode == kSumXYAndY;
+  constexpr int kUnroll = kHasY ? 2 : 4;
+  __shared__ __align__(16) float red[32 * 32 * V];
+  __shared__ unsigned last;
+  pdl_launch_dependents();
+  const uint32_t lanes = 1u << w.vec_lanes_log2, row_lanes = kChanSumThreads >> w.vec_lanes_log2;
+  const uint32_t vx = threadIdx.x & (lanes - 1), ry = threadIdx.x >> w.vec_lanes_log2;
+  const uint32_t vec = blockIdx.x * lanes + vx;
+  const bool mine = vec < w.vecs;
+  const size_t pitch = size_t(w.vecs) * V;
+  float a[V], b[V];
+  [[maybe_unused]] float m[V];
+#pragma unroll
+  for (int j = 0; j < V; ++j) a[j] = b[j] = 0.f;
+  pdl_wait();  // inputs may come from the previous kernel in the stream
+  if constexpr (kMode == kSumCentredXX) {
+    if (mine)
+#pragma unroll
+      for (int j = 0; j < V; ++j) m[j] = toFloat(centre[(vec * V + j) % w.chans]);
+  }
+  auto add = [&](const float (&xv)[V], const float (&yv)[V], int j) {
+    if constexpr (kMode == kSumXAndXX) {
+      a[j] += xv[j];
+      b[j] += xv[j] * xv[j];
+    } else if constexpr (kMode == kSumCentredXX) {
+      // the deviation is formed in the activations' type, as the reference's
+      // "acts - cast(mean)" map does (lib/poplin/Norms.cpp:216-219)
+      const float d = toFloat(fromFloat<T>(xv[j] - m[j]));
+      b[j] += d * d;
+    } else if constexpr (kMode == kSumXYAndY) {
+      a[j] += xv[j] * yv[j];
+      b[j] += yv[j];
+    } else {
+      a[j] += xv[j];
+    }
+  };
+  if (mine) {
+    const size_t step = size_t(gridDim.y) * row_lanes;
+    const T *px = x + size_t(vec) * V;
+    const T *py = kHasY ? y + size_t(vec) * V : nullptr;
+    for (size_t r = size_t(blockIdx.y) * row_lanes + ry; r < w.full; r += kUnroll * step) {
+      Raw rx[kUnroll];
+      [[maybe_unused]] Raw rv[kUnroll];
+#pragma unroll
+      for (int u = 0; u < kUnroll; ++u) {
+        const size_t row = r + u * step;
+        if (row < w.full) {
+          rx[u] = *reinterpret_cast<const Raw *>(px + row * pitch);
+          if constexpr (kHasY) rv[u] = *reinterpret_cast<const Raw *>(py + row * pitch);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < kUnroll; ++u) {
+        if (r + u * step < w.full) {
+          float xv[V], yv[V];
+          Vec::unpack(rx[u], xv);
+          if constexpr (kHasY) Vec::unpack(rv[u], yv);
+#pragma unroll
+          for (int j = 0; j < V; ++j) add(xv, yv, j);
+        }
+      }
+    }
+    // the rows that do not fill a super-row
+    if (w.fold > 1 && blockIdx.y == 0 && ry == 0) {
+      const size_t base = w.full * pitch + size_t(vec) * V;
+      float xv[V], yv[V];
+#pragma unroll
+      for (int j = 0; j < V; ++j)
+        if (base + j < w.total) {
+          xv[j] = toFloat(x[base + j]);
+          if constexpr (kHasY) yv[j] = toFloat(y[base + j]);
+          add(xv, yv, j);
+        }
+    }
+  }
+  // Threads of a warp that share a vector first (a fixed tree of shuffles), then
+  // the warps in order.
+  const uint32_t warp = threadIdx.x >> 5, cols = lanes * V;
+  const uint32_t block_col0 = blockIdx.x * cols;
+  auto reduce_block = [&](float (&s)[V], float *partial) {
+#pragma unroll
+    for (int j = 0; j < V; ++j)
+      for (uint32_t d = 16; d >= lanes; d >>= 1) s[j] += __shfl_xor_sync(0xffffffffu, s[j], d);
+    __syncthreads();
+    if ((threadIdx.x & 31) < lanes)
+#pragma unroll
+      for (int j = 0; j < V; ++j) red[(warp * lanes + vx) * V + j] = s[j];
+    __syncthreads();
+    if (threadIdx.x < cols && block_col0 + threadIdx.x < pitch) {
+      float t = 0.f;
+#pragma unroll 8
+      for (int k = 0; k < kChanSumThreads / 32; ++k) t += red[k * cols + threadIdx.x];
+      partial[size_t(blockIdx.y) * pitch + block_col0 + threadIdx.x] = t;
+    }
+  };
+  if constexpr (kHasA) reduce_block(a, partial_a);
+  if constexpr (kHasB) reduce_block(b, partial_b);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    // one thread's release publishes the block's stores (the barrier above orders
+    // them before it), its acquire the other blocks' to this one
+    unsigned before;
+    asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(before) : "l"(ticket) : "memory");
+    last = before == gridDim.x * gridDim.y - 1;
+    if (last) *ticket = 0u;  // for the next launch in the stream
+  }
+  __syncthreads();
+  if (!last) return;
+  auto finish = [&](uint32_t c, float sa, float sb) {
+    const float va = __fmul_rn(sa, fin.scale), vb = __fmul_rn(sb, fin.scale);
+    if (fin.a) storeChan(fin.a, fin.a_half, c, va);
+    if (fin.b) storeChan(fin.b, fin.b_half, c, vb);
+    if (fin.a_f32) fin.a_f32[c] = va;
+    if (fin.b_f32) fin.b_f32[c] = vb;
+    if (fin.inv_std) {
+      // plb_norm_inv_std_dev's arithmetic on the values as stored: the mean
+      // rounded to its type, the power in fp32
+      const float mean = toFloat(fromFloat<T>(va));
+      float var = vb - mean * mean;
+      if (var < 0.f) var = 0.f;
+      var = (var + fin.eps) * fin.scale_var;
+      storeChan(fin.inv_std, fin.a_half, c, 1.0f / sqrtf(var));
+    }
+    if (fin.bias) {
+      const float old = fin.bias_half ? __half2float(static_cast<const __half *>(fin.bias)[c])
+                                      : static_cast<const float *>(fin.bias)[c];
+      storeChan(fin.bias, fin.bias_half, c, old + va);
+    }
+  };
+  // [slabs * fold][chans]: channels across threads, rows shared out between the
+  // threads of a channel, so that all rows are in flight at once.
+  const uint32_t parts = gridDim.y * w.fold;
+  if constexpr (V > 1) {
+    if (w.fold == 1 && w.chans % 4 == 0) {
+      // four channels per thread
+      uint32_t ql_log2 = 3;
+      while (ql_log2 < 8 && (4u << ql_log2) < w.chans) ++ql_log2;
+      const uint32_t ql = 1u << ql_log2, part_lanes = kChanSumThreads >> ql_log2;
+      const uint32_t cl = threadIdx.x & (ql - 1), pl = threadIdx.x >> ql_log2;
+      for (uint32_t q0 = 0; q0 < w.chans / 4; q0 += ql) {
+        float4 sa = make_float4(0.f, 0.f, 0.f, 0.f), sb = sa;
+        auto take = [](float4 &s, const float4 &v) {
+          s.x += v.x;
+          s.y += v.y;
+          s.z += v.z;
+          s.w += v.w;
+        };
+        if (q0 + cl < w.chans / 4) {
+          const size_t col = size_t(q0 + cl) * 4;
+#pragma unroll 4
+          for (uint32_t k = pl; k < parts; k += part_lanes) {
+            if constexpr (kHasA) take(sa, __ldcg(reinterpret_cast<const float4 *>(partial_a + size_t(k) * w.chans + col)));
+            if constexpr (kHasB) take(sb, __ldcg(reinterpret_cast<const float4 *>(partial_b + size_t(k) * w.chans + col)));
+          }
+        }
+        // part_lanes values per channel: 4 to a thread, then the rest
+        const uint32_t ch = threadIdx.x & (4 * ql - 1), group = threadIdx.x >> (ql_log2 + 2);
+        const uint32_t groups = kChanSumThreads >> (ql_log2 + 2);
+        auto over_lanes = [&](const float4 &s) {
+          __syncthreads();
+          reinterpret_cast<float4 *>(red)[pl * ql + cl] = s;
+          __syncthreads();
+          float t = 0.f;
+#pragma unroll
+          for (uint32_t k = 0; k < 4; ++k) t += red[(group + k * groups) * 4 * ql + ch];
+          __syncthreads();
+          red[threadIdx.x] = t;
+          __syncthreads();
+          t = 0.f;
+          if (group == 0)
+            for (uint32_t k = 0; k < groups; ++k) t += red[k * 4 * ql + ch];
+          return t;
+        };
+        float ta = 0.f, tb = 0.f;
+        if constexpr (kHasA) ta = over_lanes(sa);
+        if constexpr (kHasB) tb = over_lanes(sb);
+        if (group == 0 && q0 * 4 + ch < w.chans) finish(q0 * 4 + ch, ta, tb);
+      }
+      return;
+    }
+  }
+  uint32_t cl_log2 = 3;
+  while ((2u << cl_log2) <= kChanSumThreads && (1u << cl_log2) < w.chans) ++cl_log2;
+  const uint32_t chan_lanes = 1u << cl_log2, part_lanes = kChanSumThreads >> cl_log2;
+  const uint32_t cl = threadIdx.x & (chan_lanes - 1), pl = threadIdx.x >> cl_log2;
+  for (uint32_t c0 = 0; c0 < w.chans; c0 += chan_lanes) {
+    const uint32_t c = c0 + cl;
+    float sa = 0.f, sb = 0.f;
+    if (c < w.chans) {
+#pragma unroll 8
+      for (uint32_t k = pl; k < parts; k += part_lanes) {
+        if constexpr (kHasA) sa += __ldcg(partial_a + size_t(k) * w.chans + c);
+        if constexpr (kHasB) sb += __ldcg(partial_b + size_t(k) * w.chans + c);
+      }
+    }
+    auto over_lanes = [&](float s) {
+      __syncthreads();
+      red[threadIdx.x] = s;
+      __syncthreads();
+      float t = 0.f;
+      if (pl == 0)
+        for (uint32_t k = 0; k < part_lanes; ++k) t += red[k * chan_lanes + cl];
+      return t;
+    };
+    if constexpr (kHasA) sa = over_lanes(sa);
+    if constexpr (kHasB) sb = over_lanes(sb);
+    if (pl == 0 && c < w.chans) finish(c, sa, sb);
+  }
+}
+
+inline bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
+template <typename T, int kMode>
+int chanSums(plb_context *ctx, const T *x, const T *y, const T *centre, uint64_t rows, uint32_t chans,
+             const ChanFinish &fin) {
+  constexpr uint32_t kVec = 16 / sizeof(T);
+  const bool vec = aligned16(x) && (y == nullptr || aligned16(y));
+  dim3 grid;
+  const ChanWalk w = chanWalk(ctx, rows, chans, vec ? kVec : 1, kChanSumThreads, 1, &grid);
+  const size_t row = size_t(w.vecs) * (vec ? kVec : 1);
+  void *ws = nullptr;
+  if (int rc = scratch(ctx, kSlotChannelSums, size_t(2) * w.slabs * row * sizeof(float), &ws)) return rc;
+  float *pa = static_cast<float *>(ws), *pb = pa + size_t(w.slabs) * row;
+  if (vec)
+    return launchPdl(ctx, chanSumsKernel<T, kMode, int(kVec)>, grid, dim3(kChanSumThreads), 0, x, y, centre, w, pa,
+                     pb, ctx->d_ticket, fin);
+  return launchPdl(ctx, chanSumsKernel<T, kMode, 1>, grid, dim3(kChanSumThreads), 0, x, y, centre, w, pa, pb,
+                   ctx->d_ticket, fin);
+}
+
+// ---- maps ------------------------------------------------------------------------
+
+enum ChanMap : int {
+  kWhiten = 0,      // (x - p[c]) * q[c]
+  kScaleShift = 1,  // x * p[c] + q[c]
+  kScale = 2,       // x * p[c]
+  kStatsGrad = 3,   // (y + x * p[c] + q[c]) * r[c]     x = whitened, y = gradient
+  kNormalise = 4,   // w = (x - p[c]) * q[c] rounded to T (stored in out2 if given), w * r[c] + s[c]
+  kAddChan = 5,     // x + p[c]
+};
+
+template <typename T>
+struct ChanMapArgs {
+  const T *x, *y;
+  const T *p, *q, *r, *s;    // per channel
+  const float *pf, *qf;      // the same in fp32 (instead of p, q)
+  T *out, *out2;             // out may be x
+};
+
+constexpr int kChanMapThreads = 256;
+
+template <typename T, int kMode, int V>
+__global__ void __launch_bounds__(kChanMapThreads)
+chanMapKernel(const ChanMapArgs<T> g, const ChanWalk w) {
+  using Vec = ChanVec<T, V>;
+  using Raw = typename Vec::Raw;
+  constexpr bool kHasY = kMode == kStatsGrad;
+  constexpr int kUnroll = kHasY ? 2 : 4;
+  pdl_launch_dependents();
+  const uint32_t lanes = 1u << w.vec_lanes_log2, row_lanes = kChanMapThreads >> w.vec_lanes_log2;
+  const uint32_t vx = threadIdx.x & (lanes - 1), ry = threadIdx.x >> w.vec_lanes_log2;
+  const uint32_t vec = blockIdx.x * lanes + vx;
+  pdl_wait();  // inputs may come from the previous kernel in the stream
+  if (vec >= w.vecs) return;
+  float p[V], q[V], r[V], s[V];
+#pragma unroll
+  for (int j = 0; j < V; ++j) {
+    const uint32_t c = (vec * V + j) % w.chans;
+    p[j] = g.pf ? g.pf[c] : toFloat(g.p[c]);
+    if constexpr (kMode != kScale && kMode != kAddChan) q[j] = g.qf ? g.qf[c] : toFloat(g.q[c]);
+    if constexpr (kMode == kStatsGrad || kMode == kNormalise) r[j] = toFloat(g.r[c]);
+    if constexpr (kMode == kNormalise) s[j] = toFloat(g.s[c]);
+  }
+  auto map = [&](float x, float y, int j, float &white) -> float {
+    if constexpr (kMode == kWhiten) {
+      return (x - p[j]) * q[j];
+    } else if constexpr (kMode == kScaleShift) {
+      return x * p[j] + q[j];
+    } else if constexpr (kMode == kScale) {
+      return x * p[j];
+    } else if constexpr (kMode == kStatsGrad) {
+      return (y + x * p[j] + q[j]) * r[j];
+    } else if constexpr (kMode == kNormalise) {
+      // rounded before it is scaled: the bits of kWhiten followed by kScaleShift
+      white = toFloat(fromFloat<T>((x - p[j]) * q[j]));
+      return white * r[j] + s[j];
+    } else {
+      return x + p[j];
+    }
+  };
+  const size_t pitch = size_t(w.vecs) * V, step = size_t(gridDim.y) * row_lanes;
+  for (size_t row0 = size_t(blockIdx.y) * row_lanes + ry; row0 < w.full; row0 += kUnroll * step) {
+    Raw rx[kUnroll];
+    [[maybe_unused]] Raw rv[kUnroll];
+#pragma unroll
+    for (int u = 0; u < kUnroll; ++u) {
+      const size_t row = row0 + u * step;
+      if (row < w.full) {
+        rx[u] = *reinterpret_cast<const Raw *>(g.x + row * pitch + size_t(vec) * V);
+        if constexpr (kHasY) rv[u] = *reinterpret_cast<const Raw *>(g.y + row * pitch + size_t(vec) * V);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kUnroll; ++u) {
+      const size_t row = row0 + u * step;
+      if (row < w.full) {
+        float xv[V], yv[V], o[V], white[V];
+        Vec::unpack(rx[u], xv);
+        if constexpr (kHasY) Vec::unpack(rv[u], yv);
+#pragma unroll
+        for (int j = 0; j < V; ++j) o[j] = map(xv[j], kHasY ? yv[j] : 0.f, j, white[j]);
+        if constexpr (kMode == kNormalise)
+          if (g.out2) *reinterpret_cast<Raw *>(g.out2 + row * pitch + size_t(vec) * V) = Vec::pack(white);
+        *reinterpret_cast<Raw *>(g.out + row * pitch + size_t(vec) * V) = Vec::pack(o);
+      }
+    }
+  }
+  // the rows that do not fill a super-row
+  if (w.fold > 1 && blockIdx.y == 0 && ry == 0) {
+    const size_t base = w.full * pitch + size_t(vec) * V;
+#pragma unroll
+    for (int j = 0; j < V; ++j)
+      if (base + j < w.total) {
+        float white = 0.f;
+        const float o = map(toFloat(g.x[base + j]), kHasY ? toFloat(g.y[base + j]) : 0.f, j, white);
+        if constexpr (kMode == kNormalise)
+          if (g.out2) g.out2[base + j] = fromFloat<T>(white);
+        g.out[base + j] = fromFloat<T>(o);
+      }
+  }
+}
+
+template <typename T, int kMode>
+int chanMap(plb_context *ctx, const ChanMapArgs<T> &g, uint64_t rows, uint32_t chans) {
+  if (rows == 0 || chans == 0) return PLB_OK;
+  constexpr uint32_t kVec = 16 / sizeof(T);
+  const bool vec = aligned16(g.x) && aligned16(g.out) && (g.y == nullptr || aligned16(g.y)) &&
+                   (g.out2 == nullptr || aligned16(g.out2));
+  dim3 grid;
+  const ChanWalk w = chanWalk(ctx, rows, chans, vec ? kVec : 1, kChanMapThreads, 4, &grid);
+  if (vec) return launchPdl(ctx, chanMapKernel<T, kMode, int(kVec)>, grid, dim3(kChanMapThreads), 0, g, w);
+  return launchPdl(ctx, chanMapKernel<T, kMode, 1>, grid, dim3(kChanMapThreads), 0, g, w);
+}
+
+}  // namespace plb

@@ -1,5 +1,6 @@
 // Context, memory and error plumbing of the C ABI, TMA tensor-map encoding and
 // the small data-movement kernels (layout changes, casts, scaled add).
+#include "channel_ops.cuh"
 #include "conv_geometry.h"
 #include "runtime.h"
 
@@ -175,39 +176,70 @@ __global__ void transposeFlipKernel(const T *__restrict__ src, T *__restrict__ d
   }
 }
 
-template <typename T>
-__global__ void castFromF32Kernel(T *__restrict__ dst, const float *__restrict__ src, size_t n);
-template <>
-__global__ void castFromF32Kernel<__half>(__half *__restrict__ dst, const float *__restrict__ src,
-                                          size_t n) {
-  for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n;
-       i += size_t(gridDim.x) * blockDim.x)
-    dst[i] = __float2half_rn(src[i]);
-}
-template <>
-__global__ void castFromF32Kernel<float>(float *__restrict__ dst, const float *__restrict__ src,
-                                         size_t n) {
-  for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n;
-       i += size_t(gridDim.x) * blockDim.x)
-    dst[i] = src[i];
+// w[i] = d[i] (kAdd = false) or w[i] + scale * d[i]: fp32 to the type of w, one
+// rounding.  V elements of w are 16 bytes (or V = 1 where the addresses do not
+// allow it); 8 bytes per half element have to move, so all that matters is wide
+// accesses and two of them in flight per thread.  16.8 M halves: 38 us with one
+// element per thread and iteration, now 22 (6.1 TB/s).
+template <typename T, int V, bool kAdd>
+__global__ void __launch_bounds__(256)
+fromF32Kernel(T *w, const float *__restrict__ d, float scale, size_t n) {
+  using Vec = ChanVec<T, V>;
+  using Raw = typename Vec::Raw;
+  pdl_launch_dependents();
+  pdl_wait();  // the sums come from the previous kernel in the stream
+  auto one = [&](float old, float x) { return kAdd ? old + scale * x : x; };
+  const size_t vecs = n / V, threads = size_t(gridDim.x) * blockDim.x;
+  const size_t t0 = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
+  for (size_t v0 = t0; v0 < vecs; v0 += 2 * threads) {
+    Raw old[2];
+    float x[2][V];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const size_t v = v0 + u * threads;
+      if (v < vecs) {
+        if constexpr (kAdd) old[u] = *reinterpret_cast<const Raw *>(w + v * V);
+        if constexpr (V == 1) {
+          x[u][0] = d[v];
+        } else {
+#pragma unroll
+          for (int j = 0; j < V; j += 4) {
+            const float4 f = *reinterpret_cast<const float4 *>(d + v * V + j);
+            x[u][j] = f.x;
+            x[u][j + 1] = f.y;
+            x[u][j + 2] = f.z;
+            x[u][j + 3] = f.w;
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const size_t v = v0 + u * threads;
+      if (v < vecs) {
+        float o[V];
+        if constexpr (kAdd) Vec::unpack(old[u], o);
+#pragma unroll
+        for (int j = 0; j < V; ++j) o[j] = one(kAdd ? o[j] : 0.f, x[u][j]);
+        *reinterpret_cast<Raw *>(w + v * V) = Vec::pack(o);
+      }
+    }
+  }
+  if (t0 < n - vecs * V) {
+    const size_t i = vecs * V + t0;
+    w[i] = fromFloat<T>(one(kAdd ? toFloat(w[i]) : 0.f, d[i]));
+  }
 }
 
-template <typename T>
-__global__ void scaledAddKernel(T *__restrict__ w, const float *__restrict__ d, float scale,
-                                size_t n);
-template <>
-__global__ void scaledAddKernel<__half>(__half *__restrict__ w, const float *__restrict__ d,
-                                        float scale, size_t n) {
-  for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n;
-       i += size_t(gridDim.x) * blockDim.x)
-    w[i] = __float2half_rn(__half2float(w[i]) + scale * d[i]);
-}
-template <>
-__global__ void scaledAddKernel<float>(float *__restrict__ w, const float *__restrict__ d,
-                                       float scale, size_t n) {
-  for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n;
-       i += size_t(gridDim.x) * blockDim.x)
-    w[i] = w[i] + scale * d[i];
+template <typename T, bool kAdd>
+static int fromF32(plb_context *ctx, void *w, const float *d, float scale, size_t n) {
+  constexpr int kVec = 16 / int(sizeof(T));
+  const bool vec = aligned16(w) && aligned16(d);
+  const size_t threads = vec ? (n + kVec - 1) / kVec : n;
+  const dim3 grid(unsigned(std::min<size_t>((threads + 255) / 256, size_t(ctx->sm_count) * 8)));
+  if (vec)
+    return launchPdl(ctx, fromF32Kernel<T, kVec, kAdd>, grid, dim3(256), 0, static_cast<T *>(w), d, scale, n);
+  return launchPdl(ctx, fromF32Kernel<T, 1, kAdd>, grid, dim3(256), 0, static_cast<T *>(w), d, scale, n);
 }
 
 // out = beta * c (matrix product with an empty reduction dimension)
@@ -252,97 +284,10 @@ __global__ void stridedCopyKernel(const T *__restrict__ src, T *__restrict__ dst
 }
 
 template <typename T>
-__global__ void addBiasKernel(T *acts, const T *__restrict__ biases, size_t total, uint32_t chans);
-template <>
-__global__ void addBiasKernel<__half>(__half *acts, const __half *__restrict__ biases, size_t total,
-                                      uint32_t chans) {
-  for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < total;
-       i += size_t(gridDim.x) * blockDim.x)
-    acts[i] = __float2half_rn(__half2float(acts[i]) + __half2float(biases[i % chans]));
-}
-template <>
-__global__ void addBiasKernel<float>(float *acts, const float *__restrict__ biases, size_t total,
-                                     uint32_t chans) {
-  for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < total;
-       i += size_t(gridDim.x) * blockDim.x)
-    acts[i] += biases[i % chans];
-}
-
-template <typename T>
 __global__ void fillKernel(T *dst, T value, size_t n) {
   for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n;
        i += size_t(gridDim.x) * blockDim.x)
     dst[i] = value;
-}
-
-// Column sums of a [rows][chans] matrix (device-layout activations: one row per
-// pixel), first stage: block (x, y) adds the rows y, y + gridDim.y, ... of the
-// 8-channel vectors it owns into fp32 and leaves one partial row per slab.
-// Threads are arranged as (vector of 8 channels, row lane).
-template <typename T>
-__global__ void __launch_bounds__(256)
-columnSumPartialKernel(const T *__restrict__ in, float *__restrict__ partial, uint64_t rows,
-                       uint32_t chans, uint32_t vec_lanes) {
-  constexpr int kVec = 16 / int(sizeof(T));  // elements per 16-byte load
-  __shared__ float red[256 * 8];
-  const uint32_t vx = threadIdx.x % vec_lanes, ry = threadIdx.x / vec_lanes;
-  const uint32_t row_lanes = blockDim.x / vec_lanes;
-  const uint32_t vec = blockIdx.x * vec_lanes + vx;
-  const uint32_t vecs = chans / kVec;
-  float acc[8];
-#pragma unroll
-  for (int j = 0; j < 8; ++j) acc[j] = 0.f;
-  if (vec < vecs) {
-    for (uint64_t r = uint64_t(blockIdx.y) * row_lanes + ry; r < rows;
-         r += uint64_t(gridDim.y) * row_lanes) {
-      const uint4 v = *reinterpret_cast<const uint4 *>(in + r * chans + size_t(vec) * kVec);
-      if constexpr (sizeof(T) == 2) {
-        const __half2 *h = reinterpret_cast<const __half2 *>(&v);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float2 f = __half22float2(h[j]);
-          acc[2 * j] += f.x;
-          acc[2 * j + 1] += f.y;
-        }
-      } else {
-        const float *f = reinterpret_cast<const float *>(&v);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[j] += f[j];
-      }
-    }
-  }
-#pragma unroll
-  for (int j = 0; j < kVec; ++j) red[threadIdx.x * 8 + j] = acc[j];
-  __syncthreads();
-  // row lane 0 adds the lanes in order
-  if (ry == 0 && vec < vecs) {
-    for (uint32_t y = 1; y < row_lanes; ++y)
-#pragma unroll
-      for (int j = 0; j < kVec; ++j) acc[j] += red[(y * vec_lanes + vx) * 8 + j];
-#pragma unroll
-    for (int j = 0; j < kVec; ++j)
-      partial[size_t(blockIdx.y) * chans + size_t(vec) * kVec + j] = acc[j];
-  }
-}
-// Generic first stage (any channel count / alignment): one thread per channel.
-template <typename T>
-__global__ void columnSumPartialScalarKernel(const T *__restrict__ in, float *__restrict__ partial,
-                                             uint64_t rows, uint32_t chans) {
-  const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= chans) return;
-  float acc = 0.f;
-  for (uint64_t r = blockIdx.y; r < rows; r += gridDim.y) acc += float(in[r * chans + c]);
-  partial[size_t(blockIdx.y) * chans + c] = acc;
-}
-// Second stage: biases[c] += scale * (sum of the slabs' partial rows, in order).
-template <typename T>
-__global__ void biasUpdateKernel(const float *__restrict__ partial, uint32_t slabs, uint32_t chans,
-                                 T *__restrict__ biases, float scale) {
-  const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= chans) return;
-  float s = 0.f;
-  for (uint32_t k = 0; k < slabs; ++k) s += partial[size_t(k) * chans + c];
-  biases[c] = T(float(biases[c]) + scale * s);
 }
 
 // Copies rows of `c_src` elements into rows of `c_dst` elements (same row
@@ -649,6 +594,8 @@ int plb_context_create_on_stream(int device, void *cuda_stream, plb_context **ou
     e = cudaHostGetDevicePointer(&dev_word, host_word, 0);
     ctx->d_status = static_cast<int *>(dev_word);
   }
+  if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void **>(&ctx->d_ticket), 256);
+  if (e == cudaSuccess) e = cudaMemset(ctx->d_ticket, 0, 256);
   if (e != cudaSuccess) {
     plb_context_destroy(ctx);
     return cudaFail(e, "status word allocation");
@@ -675,6 +622,7 @@ void plb_context_destroy(plb_context *ctx) {
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
   for (int i = 0; i < plb_context::kScratchSlots; ++i)
     if (ctx->scratch[i]) cudaFree(ctx->scratch[i]);
+  if (ctx->d_ticket) cudaFree(ctx->d_ticket);
   if (ctx->h_status) cudaFreeHost(const_cast<int *>(ctx->h_status));
   if (ctx->timer_start) cudaEventDestroy(ctx->timer_start);
   if (ctx->timer_stop) cudaEventDestroy(ctx->timer_stop);
@@ -867,82 +815,6 @@ int plb_fill(plb_context *ctx, int32_t dtype, void *d_dst, float value, size_t c
   return PLB_OK;
 }
 
-int plb_add_bias(plb_context *ctx, int32_t dtype, void *d_acts, const void *d_biases,
-                 uint64_t pixels, uint32_t chans) {
-  if (int rc = activate(ctx)) return rc;
-  const size_t total = size_t(pixels) * chans;
-  if (total == 0) return PLB_OK;
-  const int grid = int(std::min<size_t>((total + 255) / 256, size_t(148) * 16));
-  if (dtype == PLB_HALF)
-    addBiasKernel<__half><<<grid, 256, 0, ctx->stream>>>(
-        static_cast<__half *>(d_acts), static_cast<const __half *>(d_biases), total, chans);
-  else if (dtype == PLB_FLOAT)
-    addBiasKernel<float><<<grid, 256, 0, ctx->stream>>>(
-        static_cast<float *>(d_acts), static_cast<const float *>(d_biases), total, chans);
-  else
-    return fail(PLB_ERR_INVALID_PARAMS, "bias add needs half or float activations");
-  PLB_CUDA(cudaGetLastError());
-  ctx->launches++;
-  return PLB_OK;
-}
-
-int plb_conv_bias_update(plb_context *ctx, int32_t acts_dtype, const void *d_out_grads,
-                         uint64_t pixels, uint32_t chans, int32_t bias_dtype, void *d_biases,
-                         float scale) {
-  if (int rc = activate(ctx)) return rc;
-  if ((acts_dtype != PLB_HALF && acts_dtype != PLB_FLOAT) ||
-      (bias_dtype != PLB_HALF && bias_dtype != PLB_FLOAT))
-    return fail(PLB_ERR_INVALID_PARAMS, "bias update needs half or float gradients and biases");
-  if (chans == 0) return PLB_OK;
-  // slabs of rows, enough blocks to fill the device; partial sums in fp32
-  const size_t es = dtypeBytes(acts_dtype);
-  const uint32_t vec = uint32_t(16 / es);
-  const bool vector_ok = chans % vec == 0 && (reinterpret_cast<uintptr_t>(d_out_grads) & 15) == 0;
-  uint32_t vec_lanes = 1, col_blocks = 1, slabs = 1;
-  if (vector_ok) {
-    const uint32_t vecs = chans / vec;
-    vec_lanes = 1;
-    while (vec_lanes < 32 && vec_lanes < vecs) vec_lanes <<= 1;
-    col_blocks = (vecs + vec_lanes - 1) / vec_lanes;
-    const uint32_t row_lanes = 256 / vec_lanes;
-    const uint64_t want = std::max<uint64_t>(1, uint64_t(ctx->sm_count) * 8 / col_blocks);
-    slabs = uint32_t(std::max<uint64_t>(1, std::min<uint64_t>(want, (pixels + row_lanes - 1) / row_lanes)));
-  } else {
-    col_blocks = (chans + 127) / 128;
-    slabs = uint32_t(std::max<uint64_t>(1, std::min<uint64_t>(pixels, uint64_t(ctx->sm_count) * 16 / col_blocks)));
-  }
-  void *ws = nullptr;
-  if (int rc = scratch(ctx, kSlotBiasUpdate, size_t(slabs) * chans * sizeof(float), &ws)) return rc;
-  float *partial = static_cast<float *>(ws);
-  if (vector_ok) {
-    if (acts_dtype == PLB_HALF)
-      columnSumPartialKernel<__half><<<dim3(col_blocks, slabs), 256, 0, ctx->stream>>>(
-          static_cast<const __half *>(d_out_grads), partial, pixels, chans, vec_lanes);
-    else
-      columnSumPartialKernel<float><<<dim3(col_blocks, slabs), 256, 0, ctx->stream>>>(
-          static_cast<const float *>(d_out_grads), partial, pixels, chans, vec_lanes);
-  } else {
-    if (acts_dtype == PLB_HALF)
-      columnSumPartialScalarKernel<__half><<<dim3(col_blocks, slabs), 128, 0, ctx->stream>>>(
-          static_cast<const __half *>(d_out_grads), partial, pixels, chans);
-    else
-      columnSumPartialScalarKernel<float><<<dim3(col_blocks, slabs), 128, 0, ctx->stream>>>(
-          static_cast<const float *>(d_out_grads), partial, pixels, chans);
-  }
-  PLB_CUDA(cudaGetLastError());
-  ctx->launches++;
-  const uint32_t ugrid = (chans + 127) / 128;
-  if (bias_dtype == PLB_HALF)
-    biasUpdateKernel<__half><<<ugrid, 128, 0, ctx->stream>>>(partial, slabs, chans,
-                                                            static_cast<__half *>(d_biases), scale);
-  else
-    biasUpdateKernel<float><<<ugrid, 128, 0, ctx->stream>>>(partial, slabs, chans,
-                                                           static_cast<float *>(d_biases), scale);
-  PLB_CUDA(cudaGetLastError());
-  ctx->launches++;
-  return PLB_OK;
-}
-
 int plb_timer_start(plb_context *ctx) {
   if (int rc = activate(ctx)) return rc;
   if (!ctx->timer_start) {
@@ -986,36 +858,18 @@ int plb_cast_from_f32(plb_context *ctx, int32_t dtype, void *d_dst, const float 
                       size_t count) {
   if (int rc = activate(ctx)) return rc;
   if (count == 0) return PLB_OK;
-  const int grid = int(std::min<size_t>((count + 255) / 256, 148 * 16));
-  if (dtype == PLB_HALF)
-    castFromF32Kernel<__half><<<grid, 256, 0, ctx->stream>>>(static_cast<__half *>(d_dst), d_src,
-                                                             count);
-  else if (dtype == PLB_FLOAT)
-    castFromF32Kernel<float><<<grid, 256, 0, ctx->stream>>>(static_cast<float *>(d_dst), d_src,
-                                                            count);
-  else
-    return fail(PLB_ERR_INVALID_PARAMS, "cast target must be half or float");
-  PLB_CUDA(cudaGetLastError());
-  ctx->launches++;
-  return PLB_OK;
+  if (dtype == PLB_HALF) return fromF32<__half, false>(ctx, d_dst, d_src, 0.f, count);
+  if (dtype == PLB_FLOAT) return fromF32<float, false>(ctx, d_dst, d_src, 0.f, count);
+  return fail(PLB_ERR_INVALID_PARAMS, "cast target must be half or float");
 }
 
 int plb_scaled_add_to(plb_context *ctx, int32_t dtype, void *d_weights, const float *d_deltas_f32,
                       float scale, size_t count) {
   if (int rc = activate(ctx)) return rc;
   if (count == 0) return PLB_OK;
-  const int grid = int(std::min<size_t>((count + 255) / 256, 148 * 16));
-  if (dtype == PLB_HALF)
-    scaledAddKernel<__half><<<grid, 256, 0, ctx->stream>>>(static_cast<__half *>(d_weights),
-                                                           d_deltas_f32, scale, count);
-  else if (dtype == PLB_FLOAT)
-    scaledAddKernel<float><<<grid, 256, 0, ctx->stream>>>(static_cast<float *>(d_weights),
-                                                          d_deltas_f32, scale, count);
-  else
-    return fail(PLB_ERR_INVALID_PARAMS, "weights must be half or float");
-  PLB_CUDA(cudaGetLastError());
-  ctx->launches++;
-  return PLB_OK;
+  if (dtype == PLB_HALF) return fromF32<__half, true>(ctx, d_weights, d_deltas_f32, scale, count);
+  if (dtype == PLB_FLOAT) return fromF32<float, true>(ctx, d_weights, d_deltas_f32, scale, count);
+  return fail(PLB_ERR_INVALID_PARAMS, "weights must be half or float");
 }
 
 }  // extern "C"

@@ -21,7 +21,7 @@ enum plb_scratch_slot {
   kSlotHostWeights,
   kSlotHostOut,
   kSlotHostBias,
-  kSlotBiasUpdate,      // column sums of the bias update
+  kSlotChannelSums,     // partial per-channel sums (normalisation, bias update)
   kSlotUsedTaps,        // taps of a truncated / flipped kernel
   kSlotPaddedChans,     // zero-padded channel counts
   kSlotFlipped,         // reversed input (input flip)
@@ -44,6 +44,9 @@ struct plb_context {
   // without a copy (a copy would queue behind other streams' transfers).
   int *d_status = nullptr;        // device address
   volatile int *h_status = nullptr;  // host address of the same word
+  // Arrival counter of kernels whose last block finishes the work of all; zero
+  // between launches (the last block clears it).
+  unsigned *d_ticket = nullptr;
   uint64_t launches = 0;          // kernels launched through this context
   int plan_flags = 0;             // PLB_PLAN_* bits added to every plan made through this context
   long long *trace = nullptr;     // device timeline buffer for builds with -DPLB_TRACE
@@ -90,6 +93,28 @@ int scratch(plb_context *ctx, int slot, size_t bytes, void **ptr);
 int encodeTensorMap(CUtensorMap *tm, CUtensorMapDataType type, int rank, const void *base,
                     const uint64_t *dims, const uint64_t *strides_bytes, const uint32_t *box,
                     const uint32_t *elem_strides, int swizzle_bytes = 128);
+
+// Launch with programmatic stream serialization: the kernel may become resident
+// while its predecessor in the stream drains.  It must execute
+// griddepcontrol.wait (in every block that touches global memory, and in at
+// least one block whatever its arguments) before it reads or writes.
+template <typename... KArgs, typename... Args>
+int launchPdl(plb_context *ctx, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, Args... args) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = ctx->stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = (ctx->plan_flags & PLB_PLAN_NO_PDL) ? 0 : 1;
+  PLB_CUDA(cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...));
+  PLB_CUDA(cudaGetLastError());
+  ctx->launches++;
+  return PLB_OK;
+}
 
 inline size_t dtypeBytes(int dtype) {
   return dtype == PLB_FLOAT ? 4 : (dtype == PLB_HALF || dtype == PLB_BFLOAT16) ? 2 : 1;
