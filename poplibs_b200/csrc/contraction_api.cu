@@ -9,6 +9,7 @@
 
 #include "conv_geometry.h"
 #include "runtime.h"
+#include "sm100_prims.cuh"
 
 namespace plb {
 
@@ -17,6 +18,26 @@ int launchScaleRows(plb_context *ctx, void *out, const void *c, float beta, bool
 int convFwdSmallChannels(plb_context *ctx, const plb_conv_params &p, const plb_conv_options *opt,
                          const void *d_in, const void *d_weights, const float *d_bias,
                          void *d_out, plb_plan *plan_only);
+
+plb_conv_params floatRouteConvParams(const plb_conv_params &p, int pass) {
+  plb_conv_params q = p;
+  q.input_type = PLB_BFLOAT16;
+  if (pass == PLB_PASS_TRAINING_BWD)
+    q.out_chans_per_group *= 3;
+  else if (pass == PLB_PASS_TRAINING_WU)
+    q.batch *= 3;
+  else
+    q.in_chans_per_group *= 3;
+  return q;
+}
+
+plb_matmul_desc floatRouteMatmulDesc(const plb_matmul_desc &d) {
+  plb_matmul_desc q = d;
+  q.input_type = PLB_BFLOAT16;
+  q.k *= 3;
+  q.lda = q.ldb = 0;
+  return q;
+}
 
 // TMA needs 16-byte pixel strides: 8 half / 16 quarter channels.
 static bool channelsFitTma(const plb_conv_params &p, uint32_t chans) {
@@ -54,9 +75,9 @@ Ld leadingDims(const plb_matmul_desc &d) {
   return l;
 }
 
-// Builds the igemm problem of one group of a matrix product.  `a` is [m][k]
-// (row stride lda), `b` either [n][k] (b_is_nk) or [k][n].
-IgemmProblem gemmProblem(const plb_matmul_desc &d, const void *a, long long lda, const void *b,
+// The igemm problem of a matrix product (all groups).  `a` is [m][k] (row stride
+// lda) or, with a_is_km, [k][m]; `b` either [n][k] (b_is_nk) or [k][n].
+IgemmProblem gemmProblem(const plb_matmul_desc &d, const void *a, long long lda, bool a_is_km, const void *b,
                          long long ldb, bool b_is_nk, const void *c, void *out, long long ldc) {
   IgemmProblem p;
   const size_t es = dtypeBytes(d.input_type);
@@ -64,32 +85,31 @@ IgemmProblem gemmProblem(const plb_matmul_desc &d, const void *a, long long lda,
   p.bf16 = d.input_type == PLB_BFLOAT16;
   p.fmt_a = d.format_a;
   p.fmt_b = d.format_b;
+  p.a_mn = a_is_km;
   p.b_mn = !b_is_nk;
+  p.groups = int(d.groups);
   p.act = a;
   p.act_dims[0] = d.k;
   p.act_dims[1] = d.m;
   p.act_strides[0] = uint64_t(lda) * es;
-  p.act_strides[1] = uint64_t(lda) * es * std::max<uint32_t>(d.m, 1);
+  p.act_strides[1] = uint64_t(lda) * es * std::max<uint32_t>(a_is_km ? d.k : d.m, 1);
   p.act_strides[2] = p.act_strides[1];
+  p.act_group_stride = p.act_strides[1];
   p.wgt = b;
-  if (b_is_nk) {
-    p.wgt_dims[0] = d.k;
-    p.wgt_dims[1] = d.n;
-    p.wgt_strides[0] = uint64_t(ldb) * es;
-    p.wgt_strides[1] = uint64_t(ldb) * es * std::max<uint32_t>(d.n, 1);
-  } else {
-    p.wgt_dims[0] = d.n;
-    p.wgt_dims[1] = d.k;
-    p.wgt_strides[0] = uint64_t(ldb) * es;
-    p.wgt_strides[1] = uint64_t(ldb) * es * std::max<uint32_t>(d.k, 1);
-  }
+  p.wgt_dims[0] = b_is_nk ? d.k : d.n;
+  p.wgt_dims[1] = b_is_nk ? d.n : d.k;
+  p.wgt_dims[2] = d.groups;
+  p.wgt_strides[0] = uint64_t(ldb) * es;
+  p.wgt_strides[1] = uint64_t(ldb) * es * std::max<uint64_t>(p.wgt_dims[1], 1);
   p.out_w = int(d.m);
   p.n_total = int(d.n);
   p.k_per_tap = int(d.k);
   p.out = out;
   p.ldc = ldc;
+  p.out_group_stride = (long long)d.m * ldc;
   p.addend = c;
   p.ld_addend = ldc;
+  p.addend_group_stride = p.out_group_stride;
   p.alpha = d.alpha;
   if (p.fp8) p.alpha *= std::ldexp(1.0f, d.scale_a + d.scale_b);
   p.beta = d.beta;
@@ -129,7 +149,7 @@ int igemmConvShape(const plb_conv_params &p, ConvShape *s) {
   if (!err.empty()) return fail(PLB_ERR_INVALID_PARAMS, err);
   if (p.num_field_dims > 2)
     return fail(PLB_ERR_UNSUPPORTED, "3-D convolutions are not implemented on this path yet");
-  if (!is16BitFloat(p.input_type) && p.input_type != PLB_QUARTER)
+  if (!is16BitFloat(p.input_type) && p.input_type != PLB_QUARTER && p.input_type != PLB_FLOAT)
     return fail(PLB_ERR_UNSUPPORTED, "convolution input type must be half, float or quarter");
   if (p.output_type != PLB_HALF && p.output_type != PLB_FLOAT)
     return fail(PLB_ERR_INVALID_PARAMS, "convolution output type must be half or float");
@@ -138,8 +158,8 @@ int igemmConvShape(const plb_conv_params &p, ConvShape *s) {
   // Input truncation, output truncation and output padding are views and
   // offsets (below).  Input dilation only arrives through the backward pass of
   // a strided layer, which plb_conv_bwd takes in forward terms.
-  // Kernel truncation selects a sub-rectangle of the taps (gathered by the
-  // entry points), kernel padding only shifts where the taps land.
+  // Kernel truncation selects a sub-rectangle of the taps (a sub-lattice of the
+  // stored filter, setTaps), kernel padding only shifts where the taps land.
   for (unsigned d = 0; d != p.num_field_dims; ++d) {
     if (p.in_dilation[d] != 1 || p.in_flip[d])
       return fail(PLB_ERR_UNSUPPORTED,
@@ -196,173 +216,165 @@ uint64_t convBytes(const plb_conv_params &p, const ConvShape &s, int pass) {
   }
 }
 
-// Forward problem of group g.
+// The operands of a pass as the kernel reads them: the activations (or output
+// gradients) with `act_pitch` channels per group and pixel, the weights as rows of
+// `w_pitch` elements, and `k` channels to reduce over per tap (three times the
+// layer's for float operands, whose type is then bfloat16).
+struct PassOperands {
+  int type;
+  const void *act, *wgt;
+  uint32_t k, act_pitch, w_pitch;
+};
+
+// The filter taps of a problem: tap (r, s) is stored tile
+// (first_h + r*step_h) * KWs + first_w + s*step_w of a filter of KHs x KWs.
+void setTaps(IgemmProblem *r, const ConvShape &s, int first_h, int step_h, int first_w, int step_w) {
+  r->tap_first_h = first_h;
+  r->tap_step_h = step_h;
+  r->tap_pitch_h = s.KWs;
+  r->tap_first_w = first_w;
+  r->tap_step_w = step_w;
+  r->taps_stored = s.KHs * s.KWs;
+}
+
+// What the passes have in common: operand types, weights, options.  `w_rows` is
+// the number of rows of a stored weight tile (its second dimension).
+IgemmProblem passProblem(const plb_conv_params &p, const plb_conv_options *opt, const ConvShape &s,
+                         const PassOperands &o, bool b_mn, uint64_t w_cols, uint64_t w_rows) {
+  const size_t es = dtypeBytes(o.type);
+  IgemmProblem r;
+  r.fp8 = o.type == PLB_QUARTER;
+  r.bf16 = o.type == PLB_BFLOAT16;
+  r.fmt_a = opt ? opt->format_in : 0;
+  r.fmt_b = opt ? opt->format_weights : 0;
+  r.groups = int(p.groups);
+  r.act_group_stride = uint64_t(o.act_pitch) * es;
+  r.wgt = o.wgt;
+  r.b_mn = b_mn;
+  r.wgt_dims[0] = w_cols;
+  r.wgt_dims[1] = w_rows;
+  r.wgt_dims[2] = uint64_t(p.groups) * s.KHs * s.KWs;
+  r.wgt_strides[0] = uint64_t(o.w_pitch) * es;
+  r.wgt_strides[1] = w_rows * o.w_pitch * es;
+  r.k_per_tap = int(o.k);
+  r.out_n = int(p.batch);
+  r.out_f32 = p.output_type == PLB_FLOAT;
+  r.force_tile_n = opt ? opt->tile_n : 0;
+  r.force_split_k = opt ? opt->split_k : 0;
+  r.plan_flags = opt ? opt->plan_flags : 0;
+  if (r.fp8 && opt) r.alpha = std::ldexp(1.0f, opt->scale_in + opt->scale_weights);
+  return r;
+}
+
+// Activations [N][H][W][G * act_pitch]: the view that starts at (h0, w0).
+void setActs(IgemmProblem *r, const plb_conv_params &p, const PassOperands &o, int H, int W, int h0, int w0) {
+  const size_t es = dtypeBytes(o.type);
+  const uint64_t ctot = uint64_t(p.groups) * o.act_pitch;
+  r->act = static_cast<const uint8_t *>(o.act) + (size_t(h0) * W + w0) * ctot * es;
+  r->act_dims[0] = o.k;
+  r->act_strides[0] = ctot * es;
+  r->act_strides[1] = uint64_t(W) * ctot * es;
+  r->act_strides[2] = uint64_t(H) * W * ctot * es;
+}
+
+// Forward problem (all groups).
 // With `swapped_weights` the weights are stored [G][tap][Ci][Co] (the forward
 // layout of the layer this convolution is the backward pass of) and are used
 // with their spatial axes flipped: they are read as a K-by-N (MN-major) operand.
-int convFwdProblem(const plb_conv_params &p, const plb_conv_options *opt, const ConvShape &s,
-                   unsigned g, const void *in, const void *w, const float *bias, void *out,
-                   IgemmProblem *q, bool swapped_weights = false) {
-  const size_t es = dtypeBytes(p.input_type), os = dtypeBytes(p.output_type);
-  const uint64_t ctot = uint64_t(p.groups) * p.in_chans_per_group;
-  const uint64_t cotot = uint64_t(p.groups) * p.out_chans_per_group;
-  const uint64_t ci = p.in_chans_per_group, co = p.out_chans_per_group;
-  IgemmProblem r;
-  r.fp8 = p.input_type == PLB_QUARTER;
-  r.bf16 = p.input_type == PLB_BFLOAT16;
-  r.fmt_a = opt ? opt->format_in : 0;
-  r.fmt_b = opt ? opt->format_weights : 0;
+// With `flipped_taps` they are stored [G][flipped tap][Co][Ci].
+IgemmProblem convFwdProblem(const plb_conv_params &p, const plb_conv_options *opt, const ConvShape &s,
+                            const PassOperands &o, const float *bias, void *out, bool swapped_weights = false,
+                            bool flipped_taps = false) {
+  const size_t os = dtypeBytes(p.output_type);
+  const uint64_t co = p.out_chans_per_group, cotot = uint64_t(p.groups) * co;
+  IgemmProblem r = swapped_weights ? passProblem(p, opt, s, o, true, co, o.k) : passProblem(p, opt, s, o, false, o.k, co);
   // the truncated input is a view: same strides, shifted base, smaller extents
-  r.act = static_cast<const uint8_t *>(in) +
-          ((size_t(s.tH) * s.W + s.tW) * ctot + size_t(g) * ci) * es;
+  setActs(&r, p, o, s.H, s.W, s.tH, s.tW);
   const bool pointwise = s.KH == 1 && s.KW == 1 && s.padH == 0 && s.padW == 0;
   if (pointwise) {
     // a strided 1x1 convolution reads a sub-lattice: describe only that (its
     // extent is what the input holds; outputs beyond it read zero padding)
-    r.act_dims[0] = ci;
     r.act_dims[1] = uint64_t(std::min(s.OWc, (s.We + s.strW - 1) / s.strW));
     r.act_dims[2] = uint64_t(std::min(s.OHc, (s.He + s.strH - 1) / s.strH));
-    r.act_dims[3] = p.batch;
-    r.act_strides[0] = uint64_t(s.strW) * ctot * es;
-    r.act_strides[1] = uint64_t(s.strH) * s.W * ctot * es;
-    r.act_strides[2] = uint64_t(s.H) * s.W * ctot * es;
+    r.act_strides[0] *= uint64_t(s.strW);
+    r.act_strides[1] *= uint64_t(s.strH);
   } else {
-    r.act_dims[0] = ci;
     r.act_dims[1] = uint64_t(s.We);
     r.act_dims[2] = uint64_t(s.He);
-    r.act_dims[3] = p.batch;
-    r.act_strides[0] = ctot * es;
-    r.act_strides[1] = uint64_t(s.W) * ctot * es;
-    r.act_strides[2] = uint64_t(s.H) * s.W * ctot * es;
     r.stride_h = s.strH;
     r.stride_w = s.strW;
     r.act_elem_strides[1] = uint32_t(s.strW);
     r.act_elem_strides[2] = uint32_t(s.strH);
   }
-  r.wgt = static_cast<const uint8_t *>(w) + size_t(g) * s.KH * s.KW * co * ci * es;
-  r.b_mn = swapped_weights;
-  r.wgt_dims[0] = swapped_weights ? co : ci;
-  r.wgt_dims[1] = swapped_weights ? ci : co;
-  r.wgt_dims[2] = uint64_t(s.KH) * s.KW;
-  r.wgt_strides[0] = (swapped_weights ? co : ci) * es;
-  r.wgt_strides[1] = co * ci * es;
+  r.act_dims[3] = p.batch;
   // the computed part of the output is a view of the stored (padded) one
   r.out_w = s.OWc;
   r.out_h = s.OHc;
-  r.out_n = int(p.batch);
   r.n_total = int(co);
-  r.k_per_tap = int(ci);
   r.taps_h = s.KH;
   r.taps_w = s.KW;
+  if (flipped_taps)
+    setTaps(&r, s, s.KHs - s.ktH - s.KH, 1, s.KWs - s.ktW - s.KW, 1);
+  else
+    setTaps(&r, s, s.ktH, 1, s.ktW, 1);
   r.pad_h = s.padH;
   r.pad_w = s.padW;
   r.dil_h = s.dilH;
   r.dil_w = s.dilW;
   r.flip_h = swapped_weights ? !s.flipH : s.flipH;
   r.flip_w = swapped_weights ? !s.flipW : s.flipW;
-  r.out = static_cast<uint8_t *>(out) +
-          ((size_t(s.opH) * s.OW + s.opW) * cotot + size_t(g) * co) * os;
+  r.out = static_cast<uint8_t *>(out) + (size_t(s.opH) * s.OW + s.opW) * cotot * os;
   r.ldc = (long long)cotot;
   r.out_stride_h = (long long)(cotot * s.OW);
   r.out_stride_n = (long long)(cotot * s.OW * s.OH);
-  r.bias = bias ? bias + size_t(g) * co : nullptr;
-  r.out_f32 = p.output_type == PLB_FLOAT;
-  r.force_tile_n = opt ? opt->tile_n : 0;
-  r.force_split_k = opt ? opt->split_k : 0;
-  r.plan_flags = opt ? opt->plan_flags : 0;
-  if (r.fp8 && opt) r.alpha = std::ldexp(1.0f, opt->scale_in + opt->scale_weights);
-  *q = r;
-  return PLB_OK;
+  r.out_group_stride = (long long)co;
+  r.bias = bias;
+  return r;
 }
 
-// Backward-data problem of group g (stride 1): the output gradients take the
+// Backward-data problem (stride 1, all groups): the output gradients take the
 // activations' role, the taps are traversed in the opposite order, the padding
 // becomes (k-1)*dilation - padding, and the stored [tap][Co][Ci] weights are
 // read as a K-by-N (MN-major) operand with K = Co, N = Ci.
-int convBwdProblem(const plb_conv_params &p, const plb_conv_options *opt, const ConvShape &s,
-                   unsigned g, const void *dy, const void *w, void *dx, bool weights_transposed,
-                   IgemmProblem *q) {
-  const size_t es = dtypeBytes(p.input_type), os = dtypeBytes(p.output_type);
-  const uint64_t ctot = uint64_t(p.groups) * p.in_chans_per_group;
-  const uint64_t cotot = uint64_t(p.groups) * p.out_chans_per_group;
-  const uint64_t ci = p.in_chans_per_group, co = p.out_chans_per_group;
-  IgemmProblem r;
-  r.fp8 = p.input_type == PLB_QUARTER;
-  r.bf16 = p.input_type == PLB_BFLOAT16;
-  r.fmt_a = opt ? opt->format_in : 0;
-  r.fmt_b = opt ? opt->format_weights : 0;
+IgemmProblem convBwdProblem(const plb_conv_params &p, const plb_conv_options *opt, const ConvShape &s,
+                            const PassOperands &o, void *dx, bool weights_transposed) {
+  const size_t os = dtypeBytes(p.output_type);
+  const uint64_t ci = p.in_chans_per_group, ctot = uint64_t(p.groups) * ci;
+  // transposed: [tap flipped][Ci][Co], a K-major operand with the taps already reversed
+  IgemmProblem r = weights_transposed ? passProblem(p, opt, s, o, false, o.k, ci) : passProblem(p, opt, s, o, true, ci, o.k);
   // computed part of the output gradients / used part of the input gradients
-  r.act = static_cast<const uint8_t *>(dy) +
-          ((size_t(s.opH) * s.OW + s.opW) * cotot + size_t(g) * co) * es;
-  r.act_dims[0] = co;
+  setActs(&r, p, o, s.OH, s.OW, s.opH, s.opW);
   r.act_dims[1] = uint64_t(s.OWc);
   r.act_dims[2] = uint64_t(s.OHc);
   r.act_dims[3] = p.batch;
-  r.act_strides[0] = cotot * es;
-  r.act_strides[1] = uint64_t(s.OW) * cotot * es;
-  r.act_strides[2] = uint64_t(s.OH) * s.OW * cotot * es;
-  r.wgt = static_cast<const uint8_t *>(w) + size_t(g) * s.KH * s.KW * co * ci * es;
-  if (weights_transposed) {
-    // [tap flipped][Ci][Co]: a K-major operand, taps already reversed
-    r.wgt_dims[0] = co;
-    r.wgt_dims[1] = ci;
-    r.wgt_strides[0] = co * es;
-    r.flip_h = s.flipH;
-    r.flip_w = s.flipW;
-  } else {
-    r.b_mn = true;
-    r.wgt_dims[0] = ci;
-    r.wgt_dims[1] = co;
-    r.wgt_strides[0] = ci * es;
-    r.flip_h = !s.flipH;
-    r.flip_w = !s.flipW;
-  }
-  r.wgt_dims[2] = uint64_t(s.KH) * s.KW;
-  r.wgt_strides[1] = co * ci * es;
+  r.flip_h = weights_transposed ? s.flipH : !s.flipH;
+  r.flip_w = weights_transposed ? s.flipW : !s.flipW;
   r.out_w = s.We;
   r.out_h = s.He;
-  r.out_n = int(p.batch);
   r.n_total = int(ci);
-  r.k_per_tap = int(co);
   r.taps_h = s.KH;
   r.taps_w = s.KW;
+  if (weights_transposed)
+    setTaps(&r, s, s.KHs - s.ktH - s.KH, 1, s.KWs - s.ktW - s.KW, 1);
+  else
+    setTaps(&r, s, s.ktH, 1, s.ktW, 1);
   r.pad_h = (s.KH - 1) * s.dilH - s.padH;
   r.pad_w = (s.KW - 1) * s.dilW - s.padW;
   r.dil_h = s.dilH;
   r.dil_w = s.dilW;
-  r.out = static_cast<uint8_t *>(dx) + ((size_t(s.tH) * s.W + s.tW) * ctot + size_t(g) * ci) * os;
+  r.out = static_cast<uint8_t *>(dx) + (size_t(s.tH) * s.W + s.tW) * ctot * os;
   r.ldc = (long long)ctot;
   r.out_stride_h = (long long)(ctot * s.W);
   r.out_stride_n = (long long)(ctot * s.W * s.H);
-  r.out_f32 = p.output_type == PLB_FLOAT;
-  r.force_tile_n = opt ? opt->tile_n : 0;
-  r.force_split_k = opt ? opt->split_k : 0;
-  r.plan_flags = opt ? opt->plan_flags : 0;
-  if (r.fp8 && opt) r.alpha = std::ldexp(1.0f, opt->scale_in + opt->scale_weights);
-  *q = r;
-  return PLB_OK;
+  r.out_group_stride = (long long)ci;
+  return r;
 }
 
-// Filter taps (r0h + jh*sh, r0w + jw*sw), jh < JH, jw < JW, of [G][KH*KW][inner]
-// weights gathered into [G][JH*JW][inner]; 16-byte vectors.  With flip_h /
-// flip_w the tap indices count from the far end of the stored filter (the
-// filter is used spatially flipped).
-__global__ void gatherTapsKernel(const uint4 *__restrict__ src, uint4 *__restrict__ dst, int groups,
-                                 int KH, int KW, int JH, int JW, int r0h, int r0w, int sh, int sw,
-                                 size_t inner_vecs, int flip_h = 0, int flip_w = 0) {
-  const size_t total = size_t(groups) * JH * JW * inner_vecs;
-  for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < total;
-       i += size_t(gridDim.x) * blockDim.x) {
-    const size_t v = i % inner_vecs;
-    size_t t = i / inner_vecs;
-    const int jw = int(t % JW);
-    t /= JW;
-    const int jh = int(t % JH);
-    const int g = int(t / JH);
-    const int th = r0h + jh * sh, tw = r0w + jw * sw;
-    const size_t tap = size_t(flip_h ? KH - 1 - th : th) * KW + size_t(flip_w ? KW - 1 - tw : tw);
-    dst[i] = src[(size_t(g) * KH * KW + tap) * inner_vecs + v];
-  }
+int runProblem(plb_context *ctx, IgemmProblem &r) {
+  r.plan_flags |= ctx->plan_flags;
+  plb_plan plan{};
+  if (int rc = planIgemm(r, ctx->sm_count, &plan)) return rc;
+  return launchIgemm(ctx, r, plan);
 }
 
 // out[pixel][c] = bias[c]: what a convolution with a fused bias leaves where
@@ -411,56 +423,112 @@ void bwdPhase(int phase, int in_size, int kernel, int pad, int dil, int stride, 
   }
 }
 
-// ---- channel counts TMA cannot address -------------------------------------------
-// A pixel must be a multiple of 16 bytes for the tensor maps (8 half / 16 quarter
-// channels per group).  Other counts run on zero-padded copies: activations
-// [pixels][G][C -> Cp], weights [G][taps][Co -> Cop][Ci -> Cip]; padded input
-// channels meet zero weights, padded output channels are dropped.  One arena
-// (scratch slot 7) holds the copies.
-struct PaddedChans {
-  uint32_t ci, co, cip, cop;
-  bool needed;
-};
-PaddedChans paddedChans(const plb_conv_params &p) {
-  const uint32_t q = uint32_t(16 / dtypeBytes(p.input_type));
-  PaddedChans c{p.in_chans_per_group, p.out_chans_per_group, 0, 0, false};
-  c.cip = (c.ci + q - 1) / q * q;
-  c.cop = (c.co + q - 1) / q * q;
-  c.needed = c.cip != c.ci || c.cop != c.co;
-  return c;
-}
-// [G][taps][rows][cols] -> [G][taps][rows_p][cols_p]
-int padWeights(plb_context *ctx, const void *src, void *tmp, void *dst, size_t g_taps, uint32_t rows,
-               uint32_t cols, uint32_t rows_p, uint32_t cols_p, size_t es) {
-  if (int rc = resizeRows(ctx, src, tmp, g_taps * rows, cols * es, cols_p * es)) return rc;
-  return resizeRows(ctx, tmp, dst, g_taps, size_t(rows) * cols_p * es, size_t(rows_p) * cols_p * es);
-}
-size_t align256(size_t n) { return (n + 255) & ~size_t(255); }
-
-// Weights of a truncated kernel: the used sub-rectangle of taps gathered into
-// scratch as a dense [G][KH*KW][Co*Ci] filter.  Returns `w` itself when the
-// kernel is not truncated.
-int usedTaps(plb_context *ctx, const plb_conv_params &p, const ConvShape &s, const void *w,
-             const void **out) {
-  *out = w;
-  if (s.KH == s.KHs && s.KW == s.KWs) return PLB_OK;
-  const size_t es = dtypeBytes(p.input_type);
-  const size_t inner = size_t(p.out_chans_per_group) * p.in_chans_per_group * es;
-  if (inner % 16 != 0 || (reinterpret_cast<uintptr_t>(w) & 15) != 0)
-    return fail(PLB_ERR_UNSUPPORTED, "weights must be 16-byte aligned per tap");
-  if (s.KH <= 0 || s.KW <= 0) return PLB_OK;  // nothing is used; callers zero the result
+// ---- operands TMA cannot address, float operands -----------------------------------
+// A pixel's channels of one group, and a row of a weight tile, must be a multiple
+// of 16 bytes for the tensor maps (8 half / 16 quarter channels).  Other counts
+// run on copies with the rows rounded up; the output is written as it is.  Float
+// operands are split into their bfloat16 pieces by the same pass.
+//
+// `rows` of `cols` elements each become the activations; the weights are `w_rows`
+// rows of `w_cols` elements, the reduction along their rows (w_k_rows = false) or
+// along `w_k_rows` rows of each tile.
+int prepareOperands(plb_context *ctx, int type, const void *act, uint64_t rows, uint32_t cols, const void *wgt,
+                    uint64_t w_rows, uint32_t w_cols, uint64_t w_k_rows, PassOperands *o) {
+  const size_t es = dtypeBytes(type);
+  const bool is_float = type == PLB_FLOAT;
+  o->type = is_float ? PLB_BFLOAT16 : type;
+  o->act = act;
+  o->wgt = wgt;
+  o->k = is_float ? 3 * cols : cols;
+  o->act_pitch = cols;
+  o->w_pitch = w_cols;
+  auto unfit = [&](const void *base, uint32_t c) {
+    return is_float || (c * es) % 16 != 0 || (reinterpret_cast<uintptr_t>(base) & 15) != 0;
+  };
+  Repack jobs[2];
+  const void **operand[2];
+  size_t offset[2] = {0, 0}, total = 0;
+  int n = 0;
+  if (unfit(act, cols)) {
+    o->act_pitch = is_float ? roundToVec(3 * uint64_t(cols), 2) : roundToVec(cols, es);
+    jobs[n] = Repack{act, nullptr, rows, cols, cols, o->act_pitch, uint32_t(es),
+                     is_float ? kRepackSplitCols : kRepackCopy, false, 0};
+    operand[n++] = &o->act;
+  }
+  if (unfit(wgt, w_cols)) {
+    const bool along_rows = is_float && w_k_rows == 0;
+    o->w_pitch = along_rows ? roundToVec(3 * uint64_t(w_cols), 2) : roundToVec(w_cols, is_float ? 2 : es);
+    jobs[n] = Repack{wgt, nullptr, w_rows, w_cols, w_cols, o->w_pitch, uint32_t(es),
+                     !is_float ? kRepackCopy : along_rows ? kRepackSplitCols : kRepackSplitPlanes, true, w_k_rows};
+    operand[n++] = &o->wgt;
+  }
+  if (n == 0) return PLB_OK;
+  for (int i = 0; i < n; ++i) {
+    offset[i] = total;
+    total += (repackBytes(jobs[i]) + 255) & ~size_t(255);
+  }
   void *ws = nullptr;
-  const size_t bytes = size_t(p.groups) * s.KH * s.KW * inner;
-  if (int rc = scratch(ctx, kSlotUsedTaps, bytes + 256, &ws)) return rc;
-  const size_t vecs = bytes / 16;
-  const int grid = int(std::min<size_t>((vecs + 255) / 256, size_t(ctx->sm_count) * 8));
-  gatherTapsKernel<<<grid, 256, 0, ctx->stream>>>(static_cast<const uint4 *>(w),
-                                                  static_cast<uint4 *>(ws), int(p.groups), s.KHs,
-                                                  s.KWs, s.KH, s.KW, s.ktH, s.ktW, 1, 1, inner / 16);
-  PLB_CUDA(cudaGetLastError());
-  ctx->launches++;
+  if (int rc = scratch(ctx, kSlotRepacked, total + 256, &ws)) return rc;
+  for (int i = 0; i < n; ++i) {
+    jobs[i].dst = static_cast<uint8_t *>(ws) + offset[i];
+    *operand[i] = jobs[i].dst;
+  }
+  return repack(ctx, jobs, n);
+}
+
+// Quarter weights of a pass that reduces over their rows: 8-bit operands have no
+// MN-major form, so [G][tap][rows][cols] is transposed into
+// [G][flipped tap][cols][rows -> pitch].
+int transposedWeights(plb_context *ctx, const void *w, uint32_t groups, uint64_t taps, uint32_t rows, uint32_t cols,
+                      const void **out, uint32_t *pitch) {
+  *pitch = roundToVec(rows, 1);
+  void *ws = nullptr;
+  if (int rc = scratch(ctx, kSlotOperands, size_t(groups) * taps * cols * *pitch + 256, &ws)) return rc;
   *out = ws;
-  return PLB_OK;
+  return transposeFlipWeights(ctx, 1, groups, rows, cols, taps, *pitch, w, ws);
+}
+
+// Zeroes the pixels of [images][H][W] whose row phase (h mod str_h) or column phase
+// (w mod str_w) is not in the masks, inside the window that starts at (h0, w0):
+// the input positions of a strided layer that no output reads.  Only those are
+// written (clearing the whole gradient first cost the layer 1x1, stride 2, 256
+// images of 56x56x256 a third more bytes: 67 us of memset, now 50).
+template <typename V>
+__global__ void __launch_bounds__(256)
+zeroPhasesKernel(V *__restrict__ dst, uint32_t H, uint32_t W, uint32_t h0, uint32_t w0, uint32_t He, uint32_t We,
+                 uint32_t str_h, uint32_t str_w, uint64_t rows_used, uint64_t cols_used, uint32_t vecs) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const uint32_t h = blockIdx.x % He, n = blockIdx.x / He;
+  V *row = dst + ((size_t(n) * H + h0 + h) * W + w0) * vecs;
+  const bool all = !(rows_used >> (h % str_h) & 1);
+  const V zero{};
+  if (all) {
+    for (uint32_t i = threadIdx.x; i < We * vecs; i += blockDim.x) row[i] = zero;
+    return;
+  }
+  // a warp per pixel
+  for (uint32_t w = threadIdx.x / 32; w < We; w += blockDim.x / 32)
+    if (!(cols_used >> (w % str_w) & 1))
+      for (uint32_t i = threadIdx.x & 31; i < vecs; i += 32) row[size_t(w) * vecs + i] = zero;
+}
+
+int zeroPhases(plb_context *ctx, void *dx, const plb_conv_params &p, const ConvShape &s, uint64_t rows_used,
+               uint64_t cols_used) {
+  const size_t pixel = size_t(p.groups) * p.in_chans_per_group * dtypeBytes(p.output_type);
+  const uint64_t rows = uint64_t(p.batch) * s.He;
+  if (rows > 0x7fffffffull || uint64_t(s.We) * pixel > 0x7fffffffull)
+    return fail(PLB_ERR_UNSUPPORTED, "input gradient too large");
+  auto launch = [&](auto v) {
+    using V = decltype(v);
+    return launchPdl(ctx, zeroPhasesKernel<V>, dim3(unsigned(rows)), dim3(256), 0, static_cast<V *>(dx), uint32_t(s.H),
+                     uint32_t(s.W), uint32_t(s.tH), uint32_t(s.tW), uint32_t(s.He), uint32_t(s.We), uint32_t(s.strH),
+                     uint32_t(s.strW), rows_used, cols_used, uint32_t(pixel / sizeof(V)));
+  };
+  const size_t at = pixel | (reinterpret_cast<uintptr_t>(dx) & 15);
+  if (at % 16 == 0) return launch(uint4());
+  if (at % 4 == 0) return launch(uint32_t());
+  return launch(uint16_t());
 }
 
 // Backward pass of a strided convolution (the reference's getGradientParams
@@ -468,120 +536,67 @@ int usedTaps(plb_context *ctx, const plb_conv_params &p, const ConvShape &s, con
 // lib/poplin/ConvUtil.cpp:728-795).  Multiplying the inserted zeros would
 // waste stride^2 of the work: instead the input gradient is computed per
 // phase (ih mod stride_h, iw mod stride_w).  The positions of one phase see a
-// fixed, evenly spaced subset of the filter taps, so each phase is a stride-1
-// convolution of the output gradients with the gathered sub-filter, written
-// to the strided sub-lattice of the input gradient.
+// fixed, evenly spaced subset of the filter taps (a sub-lattice of the stored
+// filter), so each phase is a stride-1 convolution of the output gradients with
+// that sub-filter, written to the strided sub-lattice of the input gradient.
 int convBwdStrided(plb_context *ctx, const plb_conv_params &p, const plb_conv_options *opt,
-                   const ConvShape &s, const void *dy, const void *w, void *dx) {
-  // 8-bit operands have no MN-major form: their gathered sub-filters are
-  // transposed per tap ([Co][Ci] -> [Ci][Co]) into a second buffer
-  const bool fp8 = p.input_type == PLB_QUARTER;
-  const size_t es = dtypeBytes(p.input_type), os = dtypeBytes(p.output_type);
-  const uint64_t ci = p.in_chans_per_group, co = p.out_chans_per_group;
-  const uint64_t ctot = uint64_t(p.groups) * ci, cotot = uint64_t(p.groups) * co;
-  const size_t inner = size_t(co) * ci;  // elements per tap and group
-  if ((inner * es) % 16 != 0 || (reinterpret_cast<uintptr_t>(w) & 15) != 0)
-    return fail(PLB_ERR_UNSUPPORTED, "weights must be 16-byte aligned per tap");
+                   const ConvShape &s, const PassOperands &o, void *dx, bool weights_transposed) {
+  const size_t os = dtypeBytes(p.output_type);
+  const uint64_t ci = p.in_chans_per_group, ctot = uint64_t(p.groups) * ci;
   // phases and their taps
   std::vector<BwdPhase> ph(size_t(s.strH)), pw(size_t(s.strW));
   for (int a = 0; a < s.strH; ++a) bwdPhase(a, s.He, s.KH, s.padH, s.dilH, s.strH, &ph[size_t(a)]);
   for (int b = 0; b < s.strW; ++b) bwdPhase(b, s.We, s.KW, s.padW, s.dilW, s.strW, &pw[size_t(b)]);
   // positions no tap reaches get zero
   bool any_empty = false;
-  size_t scratch_elems = 0;
-  for (const auto &a : ph)
-    for (const auto &b : pw) {
-      if (a.extent == 0 || b.extent == 0) continue;
-      if (a.taps == 0 || b.taps == 0) any_empty = true;
-      scratch_elems = std::max(scratch_elems, size_t(p.groups) * a.taps * b.taps * inner);
+  uint64_t rows_used = 0, cols_used = 0;
+  for (int a = 0; a < s.strH; ++a) {
+    if (ph[size_t(a)].extent && ph[size_t(a)].taps == 0) any_empty = true;
+    if (ph[size_t(a)].taps && a < 64) rows_used |= uint64_t(1) << a;
+  }
+  for (int b = 0; b < s.strW; ++b) {
+    if (pw[size_t(b)].extent && pw[size_t(b)].taps == 0) any_empty = true;
+    if (pw[size_t(b)].taps && b < 64) cols_used |= uint64_t(1) << b;
+  }
+  if (any_empty && !s.zero_fill_in) {  // (otherwise the caller has cleared it)
+    if (s.strH <= 64 && s.strW <= 64) {
+      if (int rc = zeroPhases(ctx, dx, p, s, rows_used, cols_used)) return rc;
+    } else {
+      PLB_CUDA(cudaMemsetAsync(dx, 0, size_t(p.batch) * s.H * s.W * ctot * os, ctx->stream));
     }
-  if (any_empty && !s.zero_fill_in)  // (otherwise the caller has cleared it)
-    PLB_CUDA(cudaMemsetAsync(dx, 0, size_t(p.batch) * s.H * s.W * ctot * os, ctx->stream));
-  void *ws = nullptr;
-  // one buffer per phase: the launches of different phases are in flight together
-  const size_t slot = (scratch_elems * es + 255) & ~size_t(255);
-  const size_t phases = size_t(s.strH) * s.strW;
-  if (int rc = scratch(ctx, kSlotOperands, slot * phases * (fp8 ? 2 : 1) + 256, &ws)) return rc;
+  }
   for (int a = 0; a < s.strH; ++a)
     for (int b = 0; b < s.strW; ++b) {
       const BwdPhase &A = ph[size_t(a)], &B = pw[size_t(b)];
       if (A.extent == 0 || B.extent == 0 || A.taps == 0 || B.taps == 0) continue;
-      uint8_t *wsub = static_cast<uint8_t *>(ws) + slot * (size_t(a) * s.strW + b);
-      const size_t vecs = size_t(p.groups) * A.taps * B.taps * (inner * es / 16);
-      const int grid = int(std::min<size_t>((vecs + 255) / 256, size_t(ctx->sm_count) * 8));
-      gatherTapsKernel<<<grid, 256, 0, ctx->stream>>>(
-          static_cast<const uint4 *>(w), reinterpret_cast<uint4 *>(wsub), int(p.groups), s.KH, s.KW,
-          A.taps, B.taps, A.first_tap, B.first_tap, A.step, B.step, inner * es / 16, s.flipH,
-          s.flipW);
-      PLB_CUDA(cudaGetLastError());
-      ctx->launches++;
-      if (fp8) {
-        uint8_t *wt = static_cast<uint8_t *>(ws) + slot * (phases + size_t(a) * s.strW + b);
-        if (int rc = plb_transpose_matrix(ctx, 1, uint32_t(p.groups * A.taps * B.taps), uint32_t(co),
-                                          uint32_t(ci), wsub, wt))
-          return rc;
-        wsub = wt;
-      }
-      for (unsigned g = 0; g < p.groups; ++g) {
-        IgemmProblem r;
-        r.fp8 = fp8;
-        r.bf16 = p.input_type == PLB_BFLOAT16;
-        r.fmt_a = opt ? opt->format_in : 0;
-        r.fmt_b = opt ? opt->format_weights : 0;
-        r.act = static_cast<const uint8_t *>(dy) +
-                ((size_t(s.opH) * s.OW + s.opW) * cotot + size_t(g) * co) * es;
-        r.act_dims[0] = co;
-        r.act_dims[1] = uint64_t(s.OWc);
-        r.act_dims[2] = uint64_t(s.OHc);
-        r.act_dims[3] = p.batch;
-        r.act_strides[0] = cotot * es;
-        r.act_strides[1] = uint64_t(s.OW) * cotot * es;
-        r.act_strides[2] = uint64_t(s.OH) * s.OW * cotot * es;
-        r.wgt = wsub + size_t(g) * A.taps * B.taps * inner * es;
-        if (fp8) {
-          // transposed [tap][Ci][Co]: a K-major right operand
-          r.wgt_dims[0] = co;
-          r.wgt_dims[1] = ci;
-          r.wgt_strides[0] = co * es;
-          if (opt) r.alpha = std::ldexp(1.0f, opt->scale_in + opt->scale_weights);
-        } else {
-          // gathered [tap][Co][Ci]: K = co rows of N = ci, an MN-major right operand
-          r.b_mn = true;
-          r.wgt_dims[0] = ci;
-          r.wgt_dims[1] = co;
-          r.wgt_strides[0] = ci * es;
-        }
-        r.wgt_dims[2] = uint64_t(A.taps) * B.taps;
-        r.wgt_strides[1] = inner * es;
-        r.out_w = B.extent;
-        r.out_h = A.extent;
-        r.out_n = int(p.batch);
-        r.n_total = int(ci);
-        r.k_per_tap = int(co);
-        r.taps_h = A.taps;
-        r.taps_w = B.taps;
-        // position i of the phase reads output index i + offset - j*dil for the
-        // j-th gathered tap: a correlation with the taps reversed
-        r.dil_h = A.dil;
-        r.dil_w = B.dil;
-        r.pad_h = (A.taps - 1) * A.dil - A.offset;
-        r.pad_w = (B.taps - 1) * B.dil - B.offset;
-        // (a flipped forward kernel was un-flipped by the gather)
-        r.flip_h = 1;
-        r.flip_w = 1;
-        r.out = static_cast<uint8_t *>(dx) +
-                ((size_t(s.tH + a) * s.W + (s.tW + b)) * ctot + size_t(g) * ci) * os;
-        r.ldc = (long long)(ctot * s.strW);
-        r.out_stride_h = (long long)(ctot * s.W * s.strH);
-        r.out_stride_n = (long long)(ctot * s.W * s.H);
-        r.out_f32 = p.output_type == PLB_FLOAT;
-        r.force_tile_n = opt ? opt->tile_n : 0;
-        r.force_split_k = opt ? opt->split_k : 0;
-        r.plan_flags = (opt ? opt->plan_flags : 0) | ctx->plan_flags;
-        plb_plan plan{};
-        if (int rc = planIgemm(r, ctx->sm_count, &plan)) return rc;
-        if (int rc = launchIgemm(ctx, r, plan)) return rc;
-      }
+      IgemmProblem r = convBwdProblem(p, opt, s, o, dx, weights_transposed);
+      r.out_w = B.extent;
+      r.out_h = A.extent;
+      r.taps_h = A.taps;
+      r.taps_w = B.taps;
+      // tap j of the phase is used tap first + j*step of the (possibly flipped)
+      // filter, stored where the flip, the truncation and (weights_transposed)
+      // the reversal of all stored taps put it
+      auto stored = [&](int used, int K, int Ks, int kt, int flip) {
+        const int at = kt + (flip ? K - 1 - used : used);
+        return weights_transposed ? Ks - 1 - at : at;
+      };
+      const int h0 = stored(A.first_tap, s.KH, s.KHs, s.ktH, s.flipH);
+      const int w0 = stored(B.first_tap, s.KW, s.KWs, s.ktW, s.flipW);
+      setTaps(&r, s, h0, (s.flipH != 0) != weights_transposed ? -A.step : A.step, w0,
+              (s.flipW != 0) != weights_transposed ? -B.step : B.step);
+      // position i of the phase reads output index i + offset - j*dil for its
+      // j-th tap: a correlation with the taps reversed
+      r.dil_h = A.dil;
+      r.dil_w = B.dil;
+      r.pad_h = (A.taps - 1) * A.dil - A.offset;
+      r.pad_w = (B.taps - 1) * B.dil - B.offset;
+      r.flip_h = 1;
+      r.flip_w = 1;
+      r.out = static_cast<uint8_t *>(dx) + (size_t(s.tH + a) * s.W + (s.tW + b)) * ctot * os;
+      r.ldc = (long long)(ctot * s.strW);
+      r.out_stride_h = (long long)(ctot * s.W * s.strH);
+      if (int rc = runProblem(ctx, r)) return rc;
     }
   return PLB_OK;
 }
@@ -597,7 +612,7 @@ int plb_matmul_plan(const plb_matmul_desc *desc, plb_plan *plan) {
   if (!desc || !plan) return fail(PLB_ERR_INVALID_PARAMS, "null argument");
   if (int rc = checkMatmulDesc(*desc)) return rc;
   if (desc->input_type == PLB_FLOAT) {
-    // what runs: bfloat16 operands, three terms per product (float_route.cu)
+    // what runs: bfloat16 operands, three terms per product (repack.cu)
     const plb_matmul_desc q = floatRouteMatmulDesc(*desc);
     if (int rc = plb_matmul_plan(&q, plan)) return rc;
     plan->flops = 2ull * desc->groups * desc->m * desc->k * desc->n;
@@ -611,10 +626,11 @@ int plb_matmul_plan(const plb_matmul_desc *desc, plb_plan *plan) {
   if (desc->groups == 0 || desc->m == 0 || desc->n == 0 || desc->k == 0) return PLB_OK;
   const Ld ld = leadingDims(*desc);
   const bool b_is_nk = desc->transpose_b || desc->input_type == PLB_QUARTER;
-  IgemmProblem p = gemmProblem(*desc, nullptr, ld.a, nullptr, ld.b, b_is_nk, nullptr, nullptr, ld.c);
+  const bool a_is_km = desc->transpose_a && desc->input_type != PLB_QUARTER;
+  IgemmProblem p = gemmProblem(*desc, nullptr, ld.a, a_is_km, nullptr, ld.b, b_is_nk, nullptr, nullptr, ld.c);
   if (int rc = planIgemm(p, 148, plan)) return rc;
   const size_t es = dtypeBytes(desc->input_type);
-  if (desc->transpose_a) plan->workspace_bytes += size_t(desc->groups) * desc->m * desc->k * es;
+  if (desc->transpose_a && !a_is_km) plan->workspace_bytes += size_t(desc->groups) * desc->m * desc->k * es;
   if (!desc->transpose_b && desc->input_type == PLB_QUARTER)
     plan->workspace_bytes += size_t(desc->groups) * desc->n * desc->k * es;
   return PLB_OK;
@@ -645,90 +661,79 @@ int plb_matmul(plb_context *ctx, const plb_matmul_desc *desc, const void *d_a, c
     }
     return PLB_OK;
   }
-  if (d.input_type == PLB_FLOAT) return floatMatmul(ctx, d, d_a, d_b, d_c, d_d);
-  // operand layouts the kernel takes directly: A as [m][k]; B as [n][k], or
-  // (half only) [k][n].  Anything else goes through a transpose into scratch.
-  const uint8_t *a = static_cast<const uint8_t *>(d_a);
-  const uint8_t *b = static_cast<const uint8_t *>(d_b);
+  // Operand layouts the kernel takes directly: A as [m][k], B as [n][k], or (not
+  // 8-bit) A as [k][m] and B as [k][n].  8-bit operands stored the other way go
+  // through a transpose into scratch.
+  plb_matmul_desc q = d;
+  const void *a = d_a, *b = d_b;
   long long lda = ld.a, ldb = ld.b;
-  bool b_is_nk = d.transpose_b != 0;
-  size_t scratch_bytes = 0;
-  const size_t a_bytes = size_t(d.groups) * d.m * d.k * es, b_bytes = size_t(d.groups) * d.n * d.k * es;
-  const bool transpose_b_now = !d.transpose_b && d.input_type == PLB_QUARTER;
-  if (d.transpose_a) scratch_bytes += (a_bytes + 255) & ~size_t(255);
-  if (transpose_b_now) scratch_bytes += b_bytes;
-  if (scratch_bytes) {
+  bool a_is_km = d.transpose_a != 0, b_is_nk = d.transpose_b != 0;
+  if (d.input_type == PLB_QUARTER && (a_is_km || !b_is_nk)) {
+    const size_t a_bytes = a_is_km ? (size_t(d.groups) * d.m * d.k + 255) & ~size_t(255) : 0;
+    const size_t b_bytes = b_is_nk ? 0 : size_t(d.groups) * d.n * d.k;
     void *ws = nullptr;
-    if (int rc = scratch(ctx, kSlotOperands, scratch_bytes, &ws)) return rc;
-    uint8_t *cursor = static_cast<uint8_t *>(ws);
-    if (d.transpose_a) {
+    if (int rc = scratch(ctx, kSlotOperands, a_bytes + b_bytes, &ws)) return rc;
+    if (a_is_km) {
       if (ld.a != (long long)d.m)
-        return fail(PLB_ERR_UNSUPPORTED, "transposed A must be densely packed");
-      if (int rc = plb_transpose_matrix(ctx, uint32_t(es), d.groups, d.k, d.m, d_a, cursor)) return rc;
-      a = cursor;
+        return fail(PLB_ERR_UNSUPPORTED, "transposed quarter A must be densely packed");
+      if (int rc = plb_transpose_matrix(ctx, 1, d.groups, d.k, d.m, d_a, ws)) return rc;
+      a = ws;
       lda = d.k;
-      cursor += (a_bytes + 255) & ~size_t(255);
+      a_is_km = false;
     }
-    if (transpose_b_now) {
+    if (!b_is_nk) {
       if (ld.b != (long long)d.n)
         return fail(PLB_ERR_UNSUPPORTED, "quarter B in [k][n] layout must be densely packed");
-      if (int rc = plb_transpose_matrix(ctx, uint32_t(es), d.groups, d.k, d.n, d_b, cursor)) return rc;
-      b = cursor;
+      uint8_t *bt = static_cast<uint8_t *>(ws) + a_bytes;
+      if (int rc = plb_transpose_matrix(ctx, 1, d.groups, d.k, d.n, d_b, bt)) return rc;
+      b = bt;
       ldb = d.k;
       b_is_nk = true;
     }
   }
   // Operands whose rows TMA cannot address (base or row pitch not a multiple of
-  // 16 bytes: a [k][n] right matrix with n % 8 != 0, odd leading dimensions)
-  // are copied once into scratch with the pitch rounded up and the padding
-  // zeroed, the way the convolution path pads channel counts.  The output needs
-  // no such copy: the epilogue falls back to plain stores.
+  // 16 bytes: n % 8 != 0, odd leading dimensions) are copied once into scratch
+  // with the pitch rounded up, float operands are split into their bfloat16
+  // pieces, both operands in one launch.  The output needs no such copy.
   {
-    const size_t a_rows = size_t(d.groups) * d.m, b_rows = size_t(d.groups) * (b_is_nk ? d.n : d.k);
-    const size_t a_cols = d.k, b_cols = b_is_nk ? d.k : d.n;
-    auto unaligned = [&](const uint8_t *base, long long pitch) {
-      return (reinterpret_cast<uintptr_t>(base) & 15) != 0 || (size_t(pitch) * es) % 16 != 0;
+    const bool is_float = d.input_type == PLB_FLOAT;
+    const uint64_t a_rows = uint64_t(d.groups) * (a_is_km ? d.k : d.m), b_rows = uint64_t(d.groups) * (b_is_nk ? d.n : d.k);
+    const uint32_t a_cols = a_is_km ? d.m : d.k, b_cols = b_is_nk ? d.k : d.n;
+    if (is_float && (lda < (long long)a_cols || ldb < (long long)b_cols))
+      return fail(PLB_ERR_INVALID_PARAMS, "leading dimension shorter than a row");
+    auto unfit = [&](const void *base, long long pitch) {
+      return is_float || (reinterpret_cast<uintptr_t>(base) & 15) != 0 || (size_t(pitch) * es) % 16 != 0;
     };
-    const bool pad_a = unaligned(a, lda), pad_b = unaligned(b, ldb);
-    if (pad_a || pad_b) {
-      const size_t per16 = 16 / es;
-      const size_t a_pitch = (a_cols + per16 - 1) / per16 * per16, b_pitch = (b_cols + per16 - 1) / per16 * per16;
-      const size_t a_pad_bytes = pad_a ? ((a_rows * a_pitch * es + 255) & ~size_t(255)) : 0;
-      const size_t b_pad_bytes = pad_b ? b_rows * b_pitch * es : 0;
+    Repack jobs[2];
+    const void **operand[2];
+    int n = 0;
+    // (all groups' rows are uniformly `pitch` elements apart)
+    auto add = [&](const void **base, long long *pitch, uint64_t rows, uint32_t cols, bool k_along_rows, bool weights) {
+      if (!unfit(*base, *pitch)) return;
+      const int mode = !is_float ? kRepackCopy : k_along_rows ? kRepackSplitPlanes : kRepackSplitCols;
+      const uint32_t pitch_out = mode == kRepackCopy ? roundToVec(cols, es)
+                                                     : roundToVec(mode == kRepackSplitCols ? 3 * uint64_t(cols) : cols, 2);
+      jobs[n] = Repack{*base, nullptr, rows, cols, uint64_t(*pitch), pitch_out, uint32_t(es), mode, weights, d.k};
+      *pitch = pitch_out;
+      operand[n++] = base;
+    };
+    add(&a, &lda, a_rows, a_cols, a_is_km, false);
+    add(&b, &ldb, b_rows, b_cols, !b_is_nk, true);
+    if (n) {
+      size_t bytes[2] = {0, 0};
+      for (int i = 0; i < n; ++i) bytes[i] = (repackBytes(jobs[i]) + 255) & ~size_t(255);
       void *ws = nullptr;
-      if (int rc = scratch(ctx, kSlotPaddedChans, a_pad_bytes + b_pad_bytes + 256, &ws)) return rc;
-      uint8_t *cursor = static_cast<uint8_t *>(ws);
-      // (all groups' rows are uniformly `pitch` elements apart)
-      auto repitch = [&](const uint8_t *src, long long src_pitch, size_t rows, size_t cols,
-                         size_t dst_pitch, uint8_t *dst) -> int {
-        return copyRowsPitched(ctx, src, size_t(src_pitch) * es, dst, dst_pitch * es, rows, cols * es);
-      };
-      if (pad_a) {
-        if (int rc = repitch(a, lda, a_rows, a_cols, a_pitch, cursor)) return rc;
-        a = cursor;
-        lda = (long long)a_pitch;
-        cursor += a_pad_bytes;
-      }
-      if (pad_b) {
-        if (int rc = repitch(b, ldb, b_rows, b_cols, b_pitch, cursor)) return rc;
-        b = cursor;
-        ldb = (long long)b_pitch;
-      }
+      if (int rc = scratch(ctx, kSlotRepacked, bytes[0] + bytes[1] + 256, &ws)) return rc;
+      for (int i = 0; i < n; ++i) *operand[i] = jobs[i].dst = static_cast<uint8_t *>(ws) + (i ? bytes[0] : 0);
+      if (int rc = repack(ctx, jobs, n)) return rc;
+    }
+    if (is_float) {
+      q.input_type = PLB_BFLOAT16;
+      q.k = 3 * d.k;
     }
   }
-  for (uint32_t g = 0; g < d.groups; ++g) {
-    const uint8_t *ag = a + size_t(g) * d.m * lda * es;
-    const uint8_t *bg = b + size_t(g) * (b_is_nk ? d.n : d.k) * ldb * es;
-    const size_t coff = size_t(g) * d.m * ld.c * os;
-    IgemmProblem p = gemmProblem(d, ag, lda, bg, ldb, b_is_nk,
-                                 d_c ? static_cast<const uint8_t *>(d_c) + coff : nullptr,
-                                 static_cast<uint8_t *>(d_d) + coff, ld.c);
-    p.plan_flags |= ctx->plan_flags;
-    plb_plan plan{};
-    if (int rc = planIgemm(p, ctx->sm_count, &plan)) return rc;
-    if (int rc = launchIgemm(ctx, p, plan)) return rc;
-  }
-  return PLB_OK;
+  IgemmProblem p = gemmProblem(q, a, lda, a_is_km, b, ldb, b_is_nk, d_c, d_d, ld.c);
+  return runProblem(ctx, p);
 }
 
 int plb_matmul_host(plb_context *ctx, const plb_matmul_desc *desc, const void *h_a,
@@ -791,7 +796,7 @@ int plb_conv_plan(const plb_conv_params *p_in, const plb_conv_options *opt, int3
                   plb_plan *plan) {
   if (!p_in || !plan) return fail(PLB_ERR_INVALID_PARAMS, "null argument");
   if (p_in->input_type == PLB_FLOAT) {
-    // what runs: bfloat16 operands, three terms per product (float_route.cu)
+    // what runs: bfloat16 operands, three terms per product (repack.cu)
     const std::string err = validate(*p_in);
     if (!err.empty()) return fail(PLB_ERR_INVALID_PARAMS, err);
     const plb_conv_params q = floatRouteConvParams(*p_in, pass);
@@ -821,21 +826,13 @@ int plb_conv_plan(const plb_conv_params *p_in, const plb_conv_options *opt, int3
     }
     if (rc != PLB_ERR_UNSUPPORTED) return rc;
   }
-  // channel counts TMA cannot address run zero-padded: plan what will run
-  plb_conv_params padded = *p;
-  const PaddedChans pc = paddedChans(*p);
-  if (pc.needed && (pass == PLB_PASS_TRAINING_BWD || !channelsFitTma(*p, pc.ci))) {
-    padded.in_chans_per_group = pc.cip;
-    padded.out_chans_per_group = pc.cop;
-  }
   IgemmProblem q;
-  if (pass == PLB_PASS_TRAINING_BWD) {
-    if (int rc = convBwdProblem(padded, opt, s, 0, nullptr, nullptr, nullptr,
-                                p->input_type == PLB_QUARTER, &q))
-      return rc;
-  } else {
-    if (int rc = convFwdProblem(padded, opt, s, 0, nullptr, nullptr, nullptr, nullptr, &q)) return rc;
-  }
+  const bool bwd = pass == PLB_PASS_TRAINING_BWD;
+  PassOperands o{p->input_type, nullptr, nullptr, bwd ? p->out_chans_per_group : p->in_chans_per_group, 0, 0};
+  o.act_pitch = roundToVec(o.k, dtypeBytes(p->input_type));
+  o.w_pitch = roundToVec(p->in_chans_per_group, dtypeBytes(p->input_type));
+  q = bwd ? convBwdProblem(*p, opt, s, o, nullptr, p->input_type == PLB_QUARTER)
+          : convFwdProblem(*p, opt, s, o, nullptr, nullptr);
   if (q.n_total > 0 && q.out_w > 0 && q.out_h > 0 && q.out_n > 0 && q.k_per_tap > 0)
     if (int rc = planIgemm(q, 148, plan)) return rc;
   plan->flops = 2 * numberOfMacs(*p);
@@ -855,11 +852,6 @@ int plb_convolution(plb_context *ctx, const plb_conv_params *p, const plb_conv_o
     if (n_in == 0 || n_w == 0) n_in = n_w = 0;  // nothing is read: the output is zero (or the bias)
     if (int rc = checkConvRequest(*p, false, d_in, n_out ? n_in : 0, d_weights, n_out ? n_w : 0, d_out, n_out))
       return rc;
-  }
-  if (p->input_type == PLB_FLOAT) {
-    const std::string err = validate(*p);
-    if (!err.empty()) return fail(PLB_ERR_INVALID_PARAMS, err);
-    return floatConvFwd(ctx, *p, opt, d_in, d_weights, d_bias, d_out, transpose_and_flip_weights);
   }
   if (p->num_field_dims == 3)
     return conv3dFwd(ctx, *p, opt, d_in, d_weights, d_bias, d_out, transpose_and_flip_weights);
@@ -918,46 +910,16 @@ int plb_convolution(plb_context *ctx, const plb_conv_params *p, const plb_conv_o
     }
     if (s.OHc <= 0 || s.OWc <= 0 || s.He <= 0 || s.We <= 0) return PLB_OK;
   }
-  if (!channelsFitTma(*p, p->in_chans_per_group) && !transpose_and_flip_weights) {
+  if (p->input_type != PLB_FLOAT && !channelsFitTma(*p, p->in_chans_per_group) && !transpose_and_flip_weights) {
     // few input channels (a stem): space-to-depth path, where it applies
     const int rc = convFwdSmallChannels(ctx, *p, opt, d_in, d_weights, d_bias, d_out, nullptr);
     if (rc != PLB_ERR_UNSUPPORTED) return rc;
-  }
-  const PaddedChans pc = paddedChans(*p);
-  if (pc.needed && !channelsFitTma(*p, pc.ci)) {
-    // run on zero-padded channel counts
-    const size_t es = dtypeBytes(p->input_type), os = dtypeBytes(p->output_type);
-    const size_t G = p->groups, taps = size_t(s.KHs) * s.KWs;
-    const size_t in_px = size_t(p->batch) * s.H * s.W, out_px = size_t(p->batch) * s.OH * s.OW;
-    const size_t x_b = align256(in_px * G * pc.cip * es), w_b = align256(G * taps * pc.cop * pc.cip * es),
-                 o_b = align256(out_px * G * pc.cop * os), b_b = align256(G * pc.cop * sizeof(float));
-    void *arena = nullptr;
-    if (int rc = scratch(ctx, kSlotPaddedChans, x_b + 2 * w_b + o_b + b_b, &arena)) return rc;
-    uint8_t *xp = static_cast<uint8_t *>(arena), *wp = xp + x_b, *wtmp = wp + w_b, *op = wtmp + w_b,
-            *bp = op + o_b;
-    if (int rc = resizeRows(ctx, d_in, xp, in_px * G, pc.ci * es, pc.cip * es)) return rc;
-    // stored [G][taps][Co][Ci], or [G][taps][Ci][Co] for transposed weights
-    if (transpose_and_flip_weights) {
-      if (int rc = padWeights(ctx, d_weights, wtmp, wp, G * taps, pc.ci, pc.co, pc.cip, pc.cop, es)) return rc;
-    } else {
-      if (int rc = padWeights(ctx, d_weights, wtmp, wp, G * taps, pc.co, pc.ci, pc.cop, pc.cip, es)) return rc;
-    }
-    if (d_bias)
-      if (int rc = resizeRows(ctx, d_bias, bp, G, pc.co * sizeof(float), pc.cop * sizeof(float))) return rc;
-    plb_conv_params q = *p;
-    q.in_chans_per_group = pc.cip;
-    q.out_chans_per_group = pc.cop;
-    if (int rc = plb_convolution(ctx, &q, opt, xp, wp, d_bias ? reinterpret_cast<const float *>(bp) : nullptr,
-                                 op, transpose_and_flip_weights))
-      return rc;
-    return resizeRows(ctx, op, d_out, out_px * G, pc.cop * os, pc.co * os);
   }
   if (s.strH > 1 || s.strW > 1) {
     const bool pointwise = s.KH == 1 && s.KW == 1 && s.padH == 0 && s.padW == 0;
     if (!pointwise && (s.strH > 8 || s.strW > 8))
       return fail(PLB_ERR_UNSUPPORTED, "strides above 8 are not implemented for k > 1");
   }
-  const size_t es = dtypeBytes(p->input_type);
   if (s.KH <= 0 || s.KW <= 0) {
     // every tap is truncated away: the result is zero
     PLB_CUDA(cudaMemsetAsync(d_out, 0,
@@ -966,34 +928,28 @@ int plb_convolution(plb_context *ctx, const plb_conv_params *p, const plb_conv_o
                              ctx->stream));
     return PLB_OK;
   }
-  const void *w = nullptr;
-  if (int rc = usedTaps(ctx, *p, s, d_weights, &w)) return rc;
-  const void *const w_used = w;
-  bool swapped = transpose_and_flip_weights != 0;
-  if (swapped && (p->input_type == PLB_QUARTER || !channelsFitTma(*p, p->out_chans_per_group))) {
-    // no MN-major path for 8-bit operands (or for rows TMA cannot address):
-    // transpose + flip the (small) weights into scratch, then run as usual
-    const size_t bytes = size_t(p->groups) * s.KH * s.KW * p->in_chans_per_group *
-                         p->out_chans_per_group * es;
-    void *ws = nullptr;
-    if (int rc = scratch(ctx, kSlotOperands, bytes, &ws)) return rc;
+  const uint64_t in_rows = uint64_t(p->batch) * s.H * s.W * p->groups, taps = uint64_t(s.KHs) * s.KWs;
+  const uint32_t ci = p->in_chans_per_group, co = p->out_chans_per_group;
+  PassOperands o;
+  bool swapped = transpose_and_flip_weights != 0, flipped_taps = false;
+  if (swapped && p->input_type == PLB_QUARTER) {
+    const void *wt = nullptr;
+    uint32_t pitch = 0;
     // stored [G][k][Ci][Co] -> [G][flipped k][Co][Ci]
-    if (int rc = plb_weights_transpose_chans_flip_xy(ctx, uint32_t(es), p->groups,
-                                                     p->in_chans_per_group, p->out_chans_per_group,
-                                                     uint64_t(s.KH) * s.KW, w_used, ws))
-      return rc;
-    w = ws;
+    if (int rc = transposedWeights(ctx, d_weights, p->groups, taps, ci, co, &wt, &pitch)) return rc;
+    if (int rc = prepareOperands(ctx, p->input_type, d_in, in_rows, ci, wt, p->groups * taps * co, pitch, 0, &o)) return rc;
     swapped = false;
+    flipped_taps = true;
+  } else if (swapped) {
+    // stored [G][k][Ci][Co], the reduction along the rows
+    if (int rc = prepareOperands(ctx, p->input_type, d_in, in_rows, ci, d_weights, p->groups * taps * ci, co, ci, &o))
+      return rc;
+  } else {
+    if (int rc = prepareOperands(ctx, p->input_type, d_in, in_rows, ci, d_weights, p->groups * taps * co, ci, 0, &o))
+      return rc;
   }
-  for (unsigned g = 0; g < p->groups; ++g) {
-    IgemmProblem q;
-    if (int rc = convFwdProblem(*p, opt, s, g, d_in, w, d_bias, d_out, &q, swapped)) return rc;
-    q.plan_flags |= ctx->plan_flags;
-    plb_plan plan{};
-    if (int rc = planIgemm(q, ctx->sm_count, &plan)) return rc;
-    if (int rc = launchIgemm(ctx, q, plan)) return rc;
-  }
-  return PLB_OK;
+  IgemmProblem q = convFwdProblem(*p, opt, s, o, d_bias, d_out, swapped, flipped_taps);
+  return runProblem(ctx, q);
 }
 
 int plb_conv_fwd(plb_context *ctx, const plb_conv_params *p, const plb_conv_options *opt,
@@ -1013,11 +969,6 @@ int plb_conv_bwd(plb_context *ctx, const plb_conv_params *p, const plb_conv_opti
     if (int rc = checkConvRequest(*p, false, d_out_grads, n_in ? n_out : 0, d_weights, n_in ? n_w : 0,
                                   d_in_grads, n_in))
       return rc;
-  }
-  if (p->input_type == PLB_FLOAT) {
-    const std::string err = validate(*p);
-    if (!err.empty()) return fail(PLB_ERR_INVALID_PARAMS, err);
-    return floatConvBwd(ctx, *p, opt, d_out_grads, d_weights, d_in_grads);
   }
   if (p->num_field_dims == 3) return conv3dBwd(ctx, *p, opt, d_out_grads, d_weights, d_in_grads);
   {
@@ -1055,7 +1006,6 @@ int plb_conv_bwd(plb_context *ctx, const plb_conv_params *p, const plb_conv_opti
   if (int rc = igemmConvShape(*p, &s)) return rc;
   if (p->batch == 0 || p->groups == 0 || p->in_chans_per_group == 0 || s.H == 0 || s.W == 0)
     return PLB_OK;
-  const size_t es = dtypeBytes(p->input_type);
   if (s.zero_fill_in)  // truncated input positions receive no gradient
     PLB_CUDA(cudaMemsetAsync(d_in_grads, 0,
                              size_t(p->batch) * s.H * s.W * p->groups * p->in_chans_per_group *
@@ -1069,25 +1019,6 @@ int plb_conv_bwd(plb_context *ctx, const plb_conv_params *p, const plb_conv_opti
                                ctx->stream));
     return PLB_OK;
   }
-  const PaddedChans pc = paddedChans(*p);
-  if (pc.needed) {
-    // run on zero-padded channel counts (see plb_convolution)
-    const size_t os = dtypeBytes(p->output_type);
-    const size_t G = p->groups, taps = size_t(s.KHs) * s.KWs;
-    const size_t in_px = size_t(p->batch) * s.H * s.W, out_px = size_t(p->batch) * s.OH * s.OW;
-    const size_t dy_b = align256(out_px * G * pc.cop * es), w_b = align256(G * taps * pc.cop * pc.cip * es),
-                 dx_b = align256(in_px * G * pc.cip * os);
-    void *arena = nullptr;
-    if (int rc = scratch(ctx, kSlotPaddedChans, dy_b + 2 * w_b + dx_b, &arena)) return rc;
-    uint8_t *dyp = static_cast<uint8_t *>(arena), *wp = dyp + dy_b, *wtmp = wp + w_b, *dxp = wtmp + w_b;
-    if (int rc = resizeRows(ctx, d_out_grads, dyp, out_px * G, pc.co * es, pc.cop * es)) return rc;
-    if (int rc = padWeights(ctx, d_weights, wtmp, wp, G * taps, pc.co, pc.ci, pc.cop, pc.cip, es)) return rc;
-    plb_conv_params q = *p;
-    q.in_chans_per_group = pc.cip;
-    q.out_chans_per_group = pc.cop;
-    if (int rc = plb_conv_bwd(ctx, &q, opt, dyp, wp, dxp)) return rc;
-    return resizeRows(ctx, dxp, d_in_grads, in_px * G, pc.cip * os, pc.ci * os);
-  }
   if (s.KH <= 0 || s.KW <= 0) {
     if (!s.zero_fill_in)
       PLB_CUDA(cudaMemsetAsync(d_in_grads, 0,
@@ -1096,33 +1027,25 @@ int plb_conv_bwd(plb_context *ctx, const plb_conv_params *p, const plb_conv_opti
                                ctx->stream));
     return PLB_OK;
   }
-  const void *w = nullptr;
-  if (int rc = usedTaps(ctx, *p, s, d_weights, &w)) return rc;
-  if (s.strH != 1 || s.strW != 1) return convBwdStrided(ctx, *p, opt, s, d_out_grads, w, d_in_grads);
-  const void *const w_used = w;
-  bool transposed = false;
-  if (p->input_type == PLB_QUARTER) {
-    // no MN-major path for 8-bit operands: transpose + flip the (small) weights
-    const size_t bytes = size_t(p->groups) * s.KH * s.KW * p->in_chans_per_group *
-                         p->out_chans_per_group * es;
-    void *ws = nullptr;
-    if (int rc = scratch(ctx, kSlotOperands, bytes, &ws)) return rc;
-    if (int rc = plb_weights_transpose_chans_flip_xy(ctx, uint32_t(es), p->groups,
-                                                     p->out_chans_per_group, p->in_chans_per_group,
-                                                     uint64_t(s.KH) * s.KW, w_used, ws))
+  const uint64_t out_rows = uint64_t(p->batch) * s.OH * s.OW * p->groups, taps = uint64_t(s.KHs) * s.KWs;
+  const uint32_t ci = p->in_chans_per_group, co = p->out_chans_per_group;
+  PassOperands o;
+  const bool transposed = p->input_type == PLB_QUARTER;
+  if (transposed) {
+    const void *wt = nullptr;
+    uint32_t pitch = 0;
+    // [G][k][Co][Ci] -> [G][flipped k][Ci][Co]
+    if (int rc = transposedWeights(ctx, d_weights, p->groups, taps, co, ci, &wt, &pitch)) return rc;
+    if (int rc = prepareOperands(ctx, p->input_type, d_out_grads, out_rows, co, wt, p->groups * taps * ci, pitch, 0, &o))
       return rc;
-    w = ws;
-    transposed = true;
+  } else {
+    // the reduction runs over the output channels, the rows of a weight tile
+    if (int rc = prepareOperands(ctx, p->input_type, d_out_grads, out_rows, co, d_weights, p->groups * taps * co, ci, co, &o))
+      return rc;
   }
-  for (unsigned g = 0; g < p->groups; ++g) {
-    IgemmProblem q;
-    if (int rc = convBwdProblem(*p, opt, s, g, d_out_grads, w, d_in_grads, transposed, &q)) return rc;
-    q.plan_flags |= ctx->plan_flags;
-    plb_plan plan{};
-    if (int rc = planIgemm(q, ctx->sm_count, &plan)) return rc;
-    if (int rc = launchIgemm(ctx, q, plan)) return rc;
-  }
-  return PLB_OK;
+  if (s.strH != 1 || s.strW != 1) return convBwdStrided(ctx, *p, opt, s, o, d_in_grads, transposed);
+  IgemmProblem q = convBwdProblem(*p, opt, s, o, d_in_grads, transposed);
+  return runProblem(ctx, q);
 }
 
 int plb_conv_fwd_host(plb_context *ctx, const plb_conv_params *p, const plb_conv_options *opt,

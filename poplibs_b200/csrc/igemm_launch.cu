@@ -4,6 +4,7 @@
 // (lib/poplin/ConvPlan.cpp:1100-1224, 1674-1768): the quantities chosen here
 // are the CTA tile (128 pixels x 64/128/256 channels), the pixel box that makes
 // up the 128 rows, the pipeline depth and the number of persistent CTAs.
+#include "igemm_dispatch.cuh"
 #include "igemm_sm100.cuh"
 #include "runtime.h"
 
@@ -14,73 +15,6 @@
 namespace plb {
 
 namespace {
-
-template <int BN, bool kFp8, bool kBMn, bool kResB, bool kHalo, bool k2Cta>
-int launchInstance(plb_context *ctx, const CUtensorMap &ta, const CUtensorMap &tb,
-                   const CUtensorMap &tout, const IgemmArgs &args, int grid, int resident_bytes,
-                   bool pdl) {
-  if constexpr (k2Cta && kBMn && BN < 128) {
-    return fail(PLB_ERR_INVALID_OPTION, "a CTA pair needs tile_n >= 128 for a row-major B");
-  } else {
-    using S = IgemmSmem<BN, kResB, k2Cta>;
-    static bool configured[64] = {};
-    static int max_clusters[64] = {};
-    auto kernel = igemm_kernel<BN, kFp8, kBMn, kResB, kHalo, k2Cta>;
-    const int dev = ctx->device & 63;
-    if (!configured[dev]) {
-      PLB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    kIgemmSmemLimit));
-      configured[dev] = true;
-    }
-    const int smem =
-        S::totalBytes(args.a_stage_bytes, args.b_tiles_per_stage, args.num_stages, resident_bytes);
-    // Launch attributes: programmatic stream serialization (the kernel's set-up
-    // may overlap the previous kernel's tail; it waits before touching global
-    // memory) and, for CTA pairs, clusters of two.
-    cudaLaunchConfig_t cfg{};
-    cfg.blockDim = dim3(kIgemmThreads);
-    cfg.dynamicSmemBytes = size_t(smem);
-    cfg.stream = ctx->stream;
-    cudaLaunchAttribute attr[2];
-    unsigned n_attr = 0;
-    if (pdl) {
-      attr[n_attr].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-      attr[n_attr].val.programmaticStreamSerializationAllowed = 1;
-      ++n_attr;
-    }
-    if constexpr (!k2Cta) {
-      cfg.gridDim = dim3(unsigned(grid));
-    } else {
-      // a persistent grid of as many clusters as can be resident at once
-      // (pairs of SMs in one GPC), each walking tile pairs
-      attr[n_attr].id = cudaLaunchAttributeClusterDimension;
-      attr[n_attr].val.clusterDim.x = 2;
-      attr[n_attr].val.clusterDim.y = 1;
-      attr[n_attr].val.clusterDim.z = 1;
-      ++n_attr;
-      if (max_clusters[dev] == 0) {
-        // queried with the largest shared-memory size, a lower bound for smaller ones
-        cudaLaunchConfig_t q = cfg;
-        q.gridDim = dim3(unsigned(2 * ctx->sm_count));
-        q.dynamicSmemBytes = size_t(kIgemmSmemLimit);
-        q.attrs = &attr[n_attr - 1];
-        q.numAttrs = 1;
-        int n = 0;
-        PLB_CUDA(cudaOccupancyMaxActiveClusters(&n, kernel, &q));
-        if (n <= 0) return fail(PLB_ERR_CUDA, "no cluster of two CTAs can be resident on this device");
-        max_clusters[dev] = n;
-      }
-      const int clusters = std::max(1, std::min(grid / 2, max_clusters[dev]));
-      cfg.gridDim = dim3(unsigned(2 * clusters));
-    }
-    cfg.attrs = attr;
-    cfg.numAttrs = n_attr;
-    PLB_CUDA(cudaLaunchKernelEx(&cfg, kernel, ta, tb, tout, args));
-    PLB_CUDA(cudaGetLastError());
-    ctx->launches++;
-    return PLB_OK;
-  }
-}
 
 int stagesFor(int bn, int a_stage_bytes, int b_tiles, bool resident, int resident_bytes,
               bool pair) {
@@ -111,6 +45,9 @@ int planIgemm(const IgemmProblem &p, int sm_count, plb_plan *plan) {
     return fail(PLB_ERR_INVALID_PARAMS, "empty contraction reached the kernel planner");
   if (p.fp8 && p.b_mn)
     return fail(PLB_ERR_UNSUPPORTED, "MN-major right operand is only implemented for half");
+  if (p.a_mn && (p.fp8 || p.taps_h * p.taps_w != 1 || p.out_h != 1 || p.out_n != 1))
+    return fail(PLB_ERR_UNSUPPORTED, "a transposed left operand is only implemented for half matrix products");
+  const long groups = std::max(1, p.groups);
   // ---- N tile ---------------------------------------------------------------
   // Cost model: waves of tiles over the SMs times the measured duration of a
   // 128 x BN x 16 tensor-core instruction (operand fetch bound: 75 / 95 / 155
@@ -128,7 +65,7 @@ int planIgemm(const IgemmProblem &p, int sm_count, plb_plan *plan) {
     long best = -1;
     for (int cand : {256, 128, 64}) {
       const long n_tiles_c = (p.n_total + cand - 1) / cand;
-      const long waves = (pixel_tiles * n_tiles_c + sms - 1) / sms;
+      const long waves = (pixel_tiles * n_tiles_c * groups + sms - 1) / sms;
       const long cost = waves * (cand == 256 ? 155 : cand == 128 ? 95 : 75);
       if (best < 0 || cost < best) {
         best = cost;
@@ -153,7 +90,7 @@ int planIgemm(const IgemmProblem &p, int sm_count, plb_plan *plan) {
       }
     }
   const int n_tiles = (p.n_total + bn - 1) / bn;
-  if (best_tiles * n_tiles > 0x7fffffffL)
+  if (best_tiles * n_tiles * groups > 0x7fffffffL)
     return fail(PLB_ERR_UNSUPPORTED, "too many output tiles for one launch");
   plan->kernel = 0;
   plan->tile_m = kTileM;
@@ -163,7 +100,7 @@ int planIgemm(const IgemmProblem &p, int sm_count, plb_plan *plan) {
   plan->box_h = bh;
   plan->box_n = bb;
   plan->split_k = 1;
-  plan->tiles = int(best_tiles * n_tiles);
+  plan->tiles = int(best_tiles * n_tiles * groups);
   // CTA pairs: two M tiles share one 256-row MMA, each CTA holding half of the
   // weight tile.  Needs two M tiles and, for a row-major B, a whole 64-column
   // block per CTA.
@@ -180,12 +117,12 @@ int planIgemm(const IgemmProblem &p, int sm_count, plb_plan *plan) {
                     ((p.plan_flags & PLB_PLAN_FORCE_CTA_PAIR) != 0
                          ? best_tiles >= 2
                          : (k_steps_per_tile >= (bn >= 256 ? 4 : 8) &&
-                            best_tiles * n_tiles >= 2L * sms_for_pair));
+                            best_tiles * n_tiles * groups >= 2L * sms_for_pair));
   plan->cta_pair = pair ? 1 : 0;
   auto grid_for = [&](long m_tiles) {
     const int sms = sm_count > 0 ? sm_count : 148;
-    if (!pair) return int(std::min<long>(m_tiles * n_tiles, sms));
-    return int(2 * std::min<long>(((m_tiles + 1) / 2) * n_tiles, sms / 2));
+    if (!pair) return int(std::min<long>(m_tiles * n_tiles * groups, sms));
+    return int(2 * std::min<long>(((m_tiles + 1) / 2) * n_tiles * groups, sms / 2));
   };
   plan->grid = grid_for(best_tiles);
   const int k_elems = kStageKBytes / elem;
@@ -195,7 +132,7 @@ int planIgemm(const IgemmProblem &p, int sm_count, plb_plan *plan) {
   const bool want_resident = (p.plan_flags & PLB_PLAN_FORCE_RESIDENT_WEIGHTS) != 0 ||
                              plan->tiles >= 2 * plan->grid;
   plan->resident_weights =
-      ((p.plan_flags & PLB_PLAN_NO_RESIDENT_WEIGHTS) == 0 && n_tiles == 1 &&
+      ((p.plan_flags & PLB_PLAN_NO_RESIDENT_WEIGHTS) == 0 && n_tiles == 1 && groups == 1 && !p.a_mn &&
        resident_bytes <= kMaxResidentBytes && want_resident)
           ? 1
           : 0;
@@ -246,7 +183,7 @@ int planIgemm(const IgemmProblem &p, int sm_count, plb_plan *plan) {
         plan->box_h = hh;
         plan->box_n = hn;
         plan->stages = st;
-        plan->tiles = int(best_t * n_tiles);
+        plan->tiles = int(best_t * n_tiles * groups);
         plan->grid = grid_for(best_t);
       }
     }
@@ -270,7 +207,7 @@ int planIgemm(const IgemmProblem &p, int sm_count, plb_plan *plan) {
     if (p.force_split_k > 0) {
       split = int(std::min<long>(p.force_split_k, steps));
     } else if (units * 2 <= sms && steps >= 16) {
-      const double out_mb = double(p.out_w) * p.out_h * p.out_n * p.n_total * 4 / 1e6;
+      const double out_mb = double(groups) * p.out_w * p.out_h * p.out_n * p.n_total * 4 / 1e6;
       double best = 0.17 * double(steps);
       for (long sp = 2; sp <= std::min<long>(steps / 4, sms / units); ++sp) {
         const double t = 0.17 * double((steps + sp - 1) / sp) + 5.0 + out_mb * double(sp + 1) / 4000.0;
@@ -286,7 +223,7 @@ int planIgemm(const IgemmProblem &p, int sm_count, plb_plan *plan) {
       const long units_total = units * split;
       plan->grid = pair ? int(2 * std::min<long>(units_total, sms / 2)) : int(std::min<long>(units_total, sms));
       const size_t ld_p = (size_t(p.n_total) + 31) / 32 * 32;
-      plan->workspace_bytes = uint64_t(split) * p.out_w * p.out_h * p.out_n * ld_p * sizeof(float);
+      plan->workspace_bytes = uint64_t(split) * groups * p.out_w * p.out_h * p.out_n * ld_p * sizeof(float);
     }
   }
   return PLB_OK;
@@ -304,11 +241,11 @@ struct SplitKReduceArgs {
   int split_k;
   long long split_stride;  // elements between splits
   int ld_p;                // elements between pixels in the partial sums
-  int n_total, out_w, out_h, out_n;
+  int groups, n_total, out_w, out_h, out_n;
   void *out;
-  long long ldc, out_stride_h, out_stride_n;
+  long long ldc, out_stride_h, out_stride_n, out_group_stride;
   const void *addend;
-  long long ld_addend;
+  long long ld_addend, addend_group_stride;
   const float *bias;
   float alpha, beta;
   int out_is_f32;
@@ -319,11 +256,11 @@ __global__ void __launch_bounds__(256) igemm_splitk_reduce_kernel(const SplitKRe
   pdl_wait();  // the partial sums come from the previous kernel in the stream
   const int quads = (a.n_total + 3) / 4;
   const long long pixels = (long long)a.out_w * a.out_h * a.out_n;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < pixels * quads;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < a.groups * pixels * quads;
        i += (long long)gridDim.x * blockDim.x) {
-    const long long pixel = i / quads;
-    const int c = int(i - pixel * quads) * 4;
-    const float *src = a.partial + pixel * a.ld_p + c;
+    const long long row = i / quads, g = row / pixels, pixel = row - g * pixels;
+    const int c = int(i - row * quads) * 4;
+    const float *src = a.partial + row * a.ld_p + c;
     float4 s = *reinterpret_cast<const float4 *>(src);
     for (int k = 1; k < a.split_k; ++k) {
       const float4 v = *reinterpret_cast<const float4 *>(src + k * a.split_stride);
@@ -337,19 +274,19 @@ __global__ void __launch_bounds__(256) igemm_splitk_reduce_kernel(const SplitKRe
     if (a.alpha != 1.f)
       for (int j = 0; j < 4; ++j) f[j] *= a.alpha;
     if (a.bias != nullptr)
-      for (int j = 0; j < valid; ++j) f[j] += a.bias[c + j];
+      for (int j = 0; j < valid; ++j) f[j] += a.bias[g * a.n_total + c + j];
     if (a.addend != nullptr) {
       if (a.out_is_f32) {
-        const float *ad = static_cast<const float *>(a.addend) + pixel * a.ld_addend + c;
+        const float *ad = static_cast<const float *>(a.addend) + g * a.addend_group_stride + pixel * a.ld_addend + c;
         for (int j = 0; j < valid; ++j) f[j] += a.beta * ad[j];
       } else {
-        const __half *ad = static_cast<const __half *>(a.addend) + pixel * a.ld_addend + c;
+        const __half *ad = static_cast<const __half *>(a.addend) + g * a.addend_group_stride + pixel * a.ld_addend + c;
         for (int j = 0; j < valid; ++j) f[j] += a.beta * __half2float(ad[j]);
       }
     }
     const long long ow = pixel % a.out_w, rest = pixel / a.out_w;
     const long long oh = rest % a.out_h, on = rest / a.out_h;
-    const long long off = on * a.out_stride_n + oh * a.out_stride_h + ow * a.ldc + c;
+    const long long off = g * a.out_group_stride + on * a.out_stride_n + oh * a.out_stride_h + ow * a.ldc + c;
     if (a.out_is_f32) {
       float *dst = static_cast<float *>(a.out) + off;
       if (valid == 4 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0)
@@ -384,23 +321,45 @@ int launchIgemm(plb_context *ctx, const IgemmProblem &p, const plb_plan &plan) {
     out3[1] = halo ? n : h;
     out3[2] = halo ? h : n;
   };
+  const int groups = std::max(1, p.groups);
   CUtensorMap ta, tb;
-  {
-    uint64_t dims[4] = {p.act_dims[0], 0, 0, 0}, strides[3];
-    order(p.act_dims[1], p.act_dims[2], p.act_dims[3], dims + 1);
-    strides[0] = p.act_strides[0];
-    strides[1] = halo ? p.act_strides[2] : p.act_strides[1];
-    strides[2] = halo ? p.act_strides[1] : p.act_strides[2];
-    uint64_t b3[3];
+  if (p.a_mn) {
+    // [group][k][m], rows of m: boxes of 64 K rows x 64 output rows
+    const uint64_t dims[3] = {p.act_dims[1], p.act_dims[0], uint64_t(groups)};
+    const uint64_t strides[2] = {p.act_strides[0], groups > 1 ? uint64_t(p.act_group_stride) : p.act_strides[1]};
+    const uint32_t box[3] = {64, 64, 1}, es[3] = {1, 1, 1};
+    if (int rc = encodeTensorMap(&ta, dt, 3, p.act, dims, strides, box, es)) return rc;
+  } else {
+    // (k, w, h, n), with groups (k, group, w, h, n)
+    uint64_t dims[5] = {p.act_dims[0]}, strides[4], b3[3], e3[3];
+    uint32_t box[5] = {uint32_t(k_elems_per_stage)}, es[5] = {1};
+    int rank = 1;
+    if (groups > 1) {
+      dims[1] = uint64_t(groups);
+      strides[0] = uint64_t(p.act_group_stride);
+      box[1] = es[1] = 1;
+      rank = 2;
+    }
+    order(p.act_dims[1], p.act_dims[2], p.act_dims[3], dims + rank);
+    strides[rank - 1] = p.act_strides[0];
+    strides[rank] = halo ? p.act_strides[2] : p.act_strides[1];
+    strides[rank + 1] = halo ? p.act_strides[1] : p.act_strides[2];
     order(uint64_t((plan.box_w - 1) * p.stride_w + 1),
           uint64_t((plan.box_h + plan.halo_rows - 1) * p.stride_h + 1), uint64_t(plan.box_n), b3);
-    const uint32_t box[4] = {uint32_t(k_elems_per_stage), uint32_t(b3[0]), uint32_t(b3[1]),
-                             uint32_t(b3[2])};
-    uint64_t e3[3];
     order(uint64_t(p.stride_w), uint64_t(p.stride_h), 1, e3);
-    const uint32_t es[4] = {1, uint32_t(e3[0]), uint32_t(e3[1]), uint32_t(e3[2])};
-    if (int rc = encodeTensorMap(&ta, dt, 4, p.act, dims, strides, box, es)) return rc;
+    for (int i = 0; i < 3; ++i) {
+      box[rank + i] = uint32_t(b3[i]);
+      es[rank + i] = uint32_t(e3[i]);
+    }
+    if (int rc = encodeTensorMap(&ta, dt, rank + 3, p.act, dims, strides, box, es)) return rc;
   }
+  // One narrow tile covering all output channels: the instruction computes, and
+  // a K-major weight box loads, only the columns that exist (16 at least, 32 for
+  // a pair, whose CTAs hold half of them each).
+  const int n_quantum = plan.cta_pair ? 32 : 16;
+  const int n_mma = plan.cta_pair && p.b_mn ? plan.tile_n
+                                            : std::min(plan.tile_n, (p.n_total + n_quantum - 1) / n_quantum * n_quantum);
+  const int b_rows = p.b_mn ? plan.tile_n / (plan.cta_pair ? 2 : 1) : n_mma / (plan.cta_pair ? 2 : 1);
   {
     uint32_t box[3];
     if (p.b_mn) {
@@ -409,7 +368,7 @@ int launchIgemm(plb_context *ctx, const IgemmProblem &p, const plb_plan &plan) {
       box[2] = 1;
     } else {
       box[0] = uint32_t(k_elems_per_stage);
-      box[1] = uint32_t(plan.tile_n / (plan.cta_pair ? 2 : 1));
+      box[1] = uint32_t(b_rows);
       box[2] = 1;
     }
     const uint32_t es[3] = {1, 1, 1};
@@ -424,7 +383,7 @@ int launchIgemm(plb_context *ctx, const IgemmProblem &p, const plb_plan &plan) {
   float *partial = nullptr;
   if (split) {
     void *ws = nullptr;
-    a.split_stride = (long long)p.out_w * p.out_h * p.out_n * (long long)ld_p;
+    a.split_stride = (long long)groups * p.out_w * p.out_h * p.out_n * (long long)ld_p;
     if (int rc = scratch(ctx, kSlotSplitK, size_t(a.split_k) * size_t(a.split_stride) * sizeof(float), &ws))
       return rc;
     partial = static_cast<float *>(ws);
@@ -448,23 +407,39 @@ int launchIgemm(plb_context *ctx, const IgemmProblem &p, const plb_plan &plan) {
   if (!split && (p.plan_flags & PLB_PLAN_NO_TMA_STORE) == 0 &&
       (reinterpret_cast<uintptr_t>(p.out) & 15) == 0 &&
       (size_t(p.ldc) * out_es) % 16 == 0 && (size_t(out_stride_h) * out_es) % 16 == 0 &&
-      (size_t(out_stride_n) * out_es) % 16 == 0) {
-    uint64_t dims[4] = {uint64_t(p.n_total), 0, 0, 0}, strides[3];
-    order(uint64_t(p.out_w), uint64_t(p.out_h), uint64_t(p.out_n), dims + 1);
+      (size_t(out_stride_n) * out_es) % 16 == 0 && (groups == 1 || (size_t(p.out_group_stride) * out_es) % 16 == 0)) {
+    uint64_t dims[5] = {uint64_t(p.n_total)}, strides[4];
+    uint32_t box[5] = {32u};
+    int rank = 1;
+    if (groups > 1) {
+      dims[1] = uint64_t(groups);
+      strides[0] = uint64_t(p.out_group_stride) * out_es;
+      box[1] = 1;
+      rank = 2;
+    }
+    order(uint64_t(p.out_w), uint64_t(p.out_h), uint64_t(p.out_n), dims + rank);
     const uint64_t sw = uint64_t(p.ldc) * out_es, sh = uint64_t(out_stride_h) * out_es,
                    sn = uint64_t(out_stride_n) * out_es;
-    strides[0] = sw;
-    strides[1] = halo ? sn : sh;
-    strides[2] = halo ? sh : sn;
-    const uint32_t box[4] = {32u, uint32_t(a.sub_w), uint32_t(a.sub_h), uint32_t(sub_3)};
-    const uint32_t es[4] = {1, 1, 1, 1};
+    strides[rank - 1] = sw;
+    strides[rank] = halo ? sn : sh;
+    strides[rank + 1] = halo ? sh : sn;
+    box[rank] = uint32_t(a.sub_w);
+    box[rank + 1] = uint32_t(a.sub_h);
+    box[rank + 2] = uint32_t(sub_3);
+    const uint32_t es[5] = {1, 1, 1, 1, 1};
     if (int rc = encodeTensorMap(&tout,
                                  p.out_f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
                                            : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,
-                                 4, p.out, dims, strides, box, es, p.out_f32 ? 128 : 64))
+                                 rank + 3, p.out, dims, strides, box, es, p.out_f32 ? 128 : 64))
       return rc;
     a.use_tma_store = 1;
   }
+  a.scatter_rows = !split && !a.use_tma_store &&
+                           ((reinterpret_cast<uintptr_t>(p.out) & 15) != 0 || (size_t(p.ldc) * out_es) % 16 != 0 ||
+                            (size_t(out_stride_h) * out_es) % 16 != 0 || (size_t(out_stride_n) * out_es) % 16 != 0 ||
+                            (groups > 1 && (size_t(p.out_group_stride) * out_es) % 16 != 0))
+                       ? 1
+                       : 0;
   a.box_w = plan.box_w;
   a.box_h = plan.box_h;
   a.box_n = plan.box_n;
@@ -479,6 +454,20 @@ int launchIgemm(plb_context *ctx, const IgemmProblem &p, const plb_plan &plan) {
   a.taps_h = p.taps_h;
   a.taps_w = p.taps_w;
   a.k_chunks = (p.k_per_tap + k_elems_per_stage - 1) / k_elems_per_stage;
+  const int k_elems_mma = 32 / elem;
+  a.k_last = (p.k_per_tap - (a.k_chunks - 1) * k_elems_per_stage + k_elems_mma - 1) / k_elems_mma;
+  a.groups = groups;
+  a.fd_groups = make_fastdiv(uint32_t(groups));
+  a.out_group_stride = groups > 1 ? p.out_group_stride : 0;
+  a.addend_group_stride = groups > 1 ? p.addend_group_stride : 0;
+  a.n_mma = n_mma;
+  a.b_box_bytes = b_rows * kStageKBytes;
+  a.tap_first_h = p.tap_first_h;
+  a.tap_step_h = p.tap_step_h;
+  a.tap_pitch_h = p.tap_pitch_h ? p.tap_pitch_h : p.taps_w;
+  a.tap_first_w = p.tap_first_w;
+  a.tap_step_w = p.tap_step_w;
+  a.taps_stored = p.taps_stored ? p.taps_stored : p.taps_h * p.taps_w;
   a.pad_h = p.pad_h;
   a.pad_w = p.pad_w;
   a.dil_h = p.dil_h;
@@ -526,6 +515,7 @@ int launchIgemm(plb_context *ctx, const IgemmProblem &p, const plb_plan &plan) {
     a.ldc = (long long)ld_p;
     a.out_stride_h = (long long)p.out_w * a.ldc;
     a.out_stride_n = (long long)p.out_h * a.out_stride_h;
+    a.out_group_stride = (long long)p.out_n * a.out_stride_n;
     a.addend = nullptr;
     a.bias = nullptr;
   }
@@ -538,51 +528,26 @@ int launchIgemm(plb_context *ctx, const IgemmProblem &p, const plb_plan &plan) {
   a.status = ctx->d_status;
   a.trace = ctx->trace;
 
-  const int grid = plan.grid;
   const bool pdl = (p.plan_flags & PLB_PLAN_NO_PDL) == 0;
-  auto dispatch = [&]() -> int {
-#define PLB_DISPATCH3(BN, RES, HALO, PAIR)                                                            \
-  if (p.fp8)                                                                                          \
-    return launchInstance<BN, true, false, RES, HALO, PAIR>(ctx, ta, tb, tout, a, grid,               \
-                                                            resident_bytes, pdl);                          \
-  if (p.b_mn)                                                                                         \
-    return launchInstance<BN, false, true, RES, HALO, PAIR>(ctx, ta, tb, tout, a, grid,               \
-                                                            resident_bytes, pdl);                          \
-  return launchInstance<BN, false, false, RES, HALO, PAIR>(ctx, ta, tb, tout, a, grid, resident_bytes, pdl);
-#define PLB_DISPATCH2(BN, RES, HALO)     \
-  if (plan.cta_pair) {                   \
-    PLB_DISPATCH3(BN, RES, HALO, true)   \
-  } else {                               \
-    PLB_DISPATCH3(BN, RES, HALO, false)  \
-  }
-#define PLB_DISPATCH(BN)                       \
-  if (halo && plan.resident_weights) {         \
-    PLB_DISPATCH2(BN, true, true)              \
-  } else if (halo) {                           \
-    PLB_DISPATCH2(BN, false, true)             \
-  } else if (plan.resident_weights) {          \
-    PLB_DISPATCH2(BN, true, false)             \
-  } else {                                     \
-    PLB_DISPATCH2(BN, false, false)            \
-  }
+  const IgemmVariant variant{p.fp8, p.a_mn, p.b_mn, plan.resident_weights != 0, halo, plan.cta_pair != 0, plan.grid,
+                             resident_bytes, pdl};
+  int rc = PLB_OK;
   switch (plan.tile_n) {
-    case 64: PLB_DISPATCH(64)
-    case 128: PLB_DISPATCH(128)
-    case 256: PLB_DISPATCH(256)
-    default: break;
+    case 64: rc = launchIgemm64(ctx, ta, tb, tout, a, variant); break;
+    case 128: rc = launchIgemm128(ctx, ta, tb, tout, a, variant); break;
+    case 256: rc = launchIgemm256(ctx, ta, tb, tout, a, variant); break;
+    default: return fail(PLB_ERR_INVALID_OPTION, "unsupported tile_n in plan");
   }
-#undef PLB_DISPATCH
-#undef PLB_DISPATCH2
-#undef PLB_DISPATCH3
-    return fail(PLB_ERR_INVALID_OPTION, "unsupported tile_n in plan");
-  };
-  if (int rc = dispatch()) return rc;
+  if (rc) return rc;
   if (!split) return PLB_OK;
   SplitKReduceArgs r{};
   r.partial = partial;
   r.split_k = a.split_k;
   r.split_stride = a.split_stride;
   r.ld_p = int(ld_p);
+  r.groups = groups;
+  r.out_group_stride = p.out_group_stride;
+  r.addend_group_stride = p.addend_group_stride;
   r.n_total = p.n_total;
   r.out_w = p.out_w;
   r.out_h = p.out_h;
@@ -597,7 +562,7 @@ int launchIgemm(plb_context *ctx, const IgemmProblem &p, const plb_plan &plan) {
   r.alpha = p.alpha;
   r.beta = p.beta;
   r.out_is_f32 = p.out_f32 ? 1 : 0;
-  const long long work = (long long)p.out_w * p.out_h * p.out_n * ((p.n_total + 3) / 4);
+  const long long work = (long long)groups * p.out_w * p.out_h * p.out_n * ((p.n_total + 3) / 4);
   cudaLaunchAttribute pdl_attr[1];
   pdl_attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   pdl_attr[0].val.programmaticStreamSerializationAllowed = 1;

@@ -69,16 +69,32 @@ struct IgemmArgs {
   int halo_step_bytes;
   int a_stage_bytes;        // bytes of activations per stage
   int b_tiles_per_stage;    // streamed weight tiles per stage (taps_h with a halo strip, else 1)
+  // ---- groups ---------------------------------------------------------------
+  // Independent contractions of one shape in one launch (channel groups of a
+  // convolution, a batch of matrix products).  With more than one, the tensor
+  // maps of the activations and the output carry the group as their second
+  // dimension (so that a group's channels end where the next group's begin), and
+  // group g uses the weight tiles [g * taps, (g + 1) * taps).
+  int groups;
+  FastDiv fd_groups;
+  long long out_group_stride, addend_group_stride;  // elements
   // ---- N side ---------------------------------------------------------------
   int n_tiles;  // tiles of BN output channels
-  int n_total;  // valid output channels
+  int n_total;  // valid output channels (of one group)
+  int n_mma;    // columns of one instruction: BN, or fewer when one narrow tile covers all
+  int b_box_bytes;  // bytes one CTA loads of a streamed or resident weight tile
   // ---- K side ---------------------------------------------------------------
   int taps_h, taps_w;  // filter extent (1 x 1 for a matrix product)
   int k_chunks;        // stages per tap = ceil(bytes of K per tap / 128)
+  int k_last;          // instructions (32 bytes of K each) of a tap's last chunk: 1..4
   int pad_h, pad_w;    // tap (r, s) reads input pixel (oh*stride_h + r*dil_h - pad_h, ...)
   int dil_h, dil_w;
   int stride_h, stride_w;  // output pixel oh starts at input row oh*stride_h (TMA traversal stride)
   int flip_h, flip_w;  // tap (r, s) uses the weights stored at (R-1-r, ...) / (..., S-1-s)
+  // Tap (r, s) of the (flipped) filter is tile (first_h + r * step_h) * pitch_h +
+  // first_w + s * step_w of the taps_stored tiles of a group: a sub-lattice of a
+  // stored filter needs no gathering.
+  int tap_first_h, tap_step_h, tap_pitch_h, tap_first_w, tap_step_w, taps_stored;
   int group_m;    // tile rasterisation: M tiles per band
   // division by group_m * n_tiles, group_m, tiles_w and (h_outer ? tiles_n : tiles_h)
   FastDiv fd_band, fd_gm, fd_tw, fd_inner;
@@ -103,6 +119,7 @@ struct IgemmArgs {
   const float *bias;
   float alpha, beta;
   int out_is_f32;
+  int scatter_rows;         // output rows allow no vector stores: turn blocks in shared memory
   int use_tma_store;        // tm_out is valid: stage through shared memory + TMA store
   int sub_w, sub_h;         // pixel box of one epilogue warp's 32 rows: (sub_w, sub_h, 32/(sub_w*sub_h))
   int *status;
@@ -156,6 +173,8 @@ struct IgemmSmem {
 // kBMn: the B operand is stored K-by-N with N contiguous (a row-major right-hand
 //       matrix); it is loaded as 64-column blocks and fed to the tensor core as
 //       an MN-major operand.  fp16 only.
+// kAMn: the same for the left operand of a matrix product, stored K-by-M (a
+//       transposed A): two blocks of 64 rows per stage.  fp16, no halo.
 // kResB: weight-stationary.  All K steps' weight tiles are loaded once per CTA
 //       and stay in shared memory; the pipeline then streams activations only.
 //       Used when there is a single N tile and the weights fit (small filters
@@ -177,7 +196,7 @@ struct IgemmSmem {
 //       CTA halves their shared-memory fill and operand fetch per FLOP, and
 //       the instruction is twice as large, which matters because a
 //       128-row instruction is bound by operand fetch, not by arithmetic.
-template <int BN, bool kFp8, bool kBMn, bool kResB, bool kHalo, bool k2Cta>
+template <int BN, bool kFp8, bool kAMn, bool kBMn, bool kResB, bool kHalo, bool k2Cta>
 __global__ void __launch_bounds__(kIgemmThreads, 1)
 igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
              const __grid_constant__ CUtensorMap tm_out, const IgemmArgs args) {
@@ -190,7 +209,8 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
   constexpr int P = kIgemmProducers;
   constexpr uint32_t kTmemCols = 2 * BN;  // two accumulators
   static_assert(kTmemCols >= 32 && kTmemCols <= 512 && (kTmemCols & (kTmemCols - 1)) == 0, "");
-  static_assert(!(kFp8 && kBMn), "MN-major B is implemented for fp16 only");
+  static_assert(!(kFp8 && (kAMn || kBMn)), "MN-major operands are implemented for fp16 only");
+  static_assert(!kAMn || (!kHalo && !kResB), "a transposed A is a plain matrix product");
 
   extern __shared__ uint8_t smem_raw[];
   if (threadIdx.x == 0) PLB_TRACE_STAMP(2, 4000);
@@ -269,7 +289,7 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
   // last one is padded: its copies read zeros and its stores are clipped).
   const int m_tiles = args.tiles_w * args.tiles_h * args.tiles_n;
   const int m_units = k2Cta ? (m_tiles + 1) / 2 : m_tiles;
-  const int total_tiles = m_units * args.n_tiles;
+  const int total_tiles = m_units * args.n_tiles * args.groups;
   // a unit of work is an output tile, or with split-K one of its K ranges
   // (the splits of a tile are consecutive units, i.e. run on different CTAs)
   const int total_units = total_tiles * args.split_k;
@@ -287,8 +307,10 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
   // put four 64-bit divisions into every thread's prologue)
   const FastDiv fd_band = args.fd_band, fd_gm = args.fd_gm, fd_tw = args.fd_tw, fd_inner = args.fd_inner;
 
-  // unit -> (tile, range [it_begin, it_end) of the tile's pipeline steps)
-  auto unit_coords = [&](int unit, int &tile, int &split, int &it_begin, int &it_end) {
+  // unit -> (tile, group, range [it_begin, it_end) of the tile's pipeline steps).
+  // The groups of a tile are consecutive units: CTAs working side by side then
+  // read neighbouring channels of the same pixels.
+  auto unit_coords = [&](int unit, int &tile, int &group, int &split, int &it_begin, int &it_end) {
     if (args.split_k == 1) {
       tile = unit;
       split = 0;
@@ -299,6 +321,12 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
       split = unit - tile * args.split_k;
       it_begin = int(fast_div(uint32_t(p_iters * split), args.fd_split));
       it_end = int(fast_div(uint32_t(p_iters * (split + 1)), args.fd_split));
+    }
+    group = 0;
+    if (args.groups > 1) {
+      const int t = int(fast_div(uint32_t(tile), args.fd_groups));
+      group = tile - t * args.groups;
+      tile = t;
     }
   };
   // tile index -> (m tile, n tile): bands of group_m M tiles, M fastest inside a band
@@ -347,12 +375,13 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
 
   // B tile of K step (r, s, kc) -> shared memory at `dst`; with kPrefetch the
   // same box is only pulled towards L2
-  auto load_b = [&](uint32_t dst, uint32_t bar, int r, int s, int kc, int n_col, bool prefetch) {
-    const int b_tap = (args.flip_h ? args.taps_h - 1 - r : r) * args.taps_w +
-                      (args.flip_w ? args.taps_w - 1 - s : s);
+  auto load_b = [&](uint32_t dst, uint32_t bar, int group, int r, int s, int kc, int n_col, bool prefetch) {
+    const int b_tap = ((args.flip_h ? args.taps_h - 1 - r : r) * args.tap_step_h + args.tap_first_h) * args.tap_pitch_h +
+                      (args.flip_w ? args.taps_w - 1 - s : s) * args.tap_step_w + args.tap_first_w +
+                      group * args.taps_stored;
     // a CTA of a pair loads its half of the tile's N rows / columns
     constexpr int kMyN = k2Cta ? BN / 2 : BN;
-    const int my_col = n_col + int(cta_rank) * kMyN;
+    const int my_col = n_col + (kBMn ? int(cta_rank) * kMyN : k2Cta ? int(cta_rank) * (args.n_mma / 2) : 0);
     if constexpr (kBMn) {
       // K rows x 64 columns per block; blocks of 64 columns are 64 rows apart
 #pragma unroll
@@ -398,29 +427,51 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
       // resident, the weight tile(s) of step (r, s, kc) -> stage memory at a_dst
       // (or, before the predecessor kernel is known to have finished, only
       // towards L2).
-      auto issue_step = [&](bool prefetch, uint32_t a_dst, uint32_t full, int r, int s, int kc,
+      auto issue_step = [&](bool prefetch, uint32_t a_dst, uint32_t full, int group, int r, int s, int kc,
                             int w_base, int h_base, int n0, int n_col) {
-        const int cw = w_base + s * args.dil_w, ch = h_base + r * args.dil_h;
-        const int c2 = args.h_outer ? n0 : ch, c3 = args.h_outer ? ch : n0;
-        if (prefetch)
-          tma_prefetch_l2_4d(&tm_a, kc * kElemsPerStage, cw, c2, c3);
-        else if constexpr (k2Cta)
-          tma_load_4d_pair(a_dst, &tm_a, full, kc * kElemsPerStage, cw, c2, c3);
-        else
-          tma_load_4d(a_dst, &tm_a, full, kc * kElemsPerStage, cw, c2, c3);
+        if constexpr (kAMn) {
+          // [k][m] rows of one group: two boxes of 64 K rows x 64 output rows
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            if (prefetch)
+              tma_prefetch_l2_3d(&tm_a, w_base + j * 64, kc * 64, group);
+            else if constexpr (k2Cta)
+              tma_load_3d_pair(a_dst + j * (64 * kStageKBytes), &tm_a, full, w_base + j * 64, kc * 64, group);
+            else
+              tma_load_3d(a_dst + j * (64 * kStageKBytes), &tm_a, full, w_base + j * 64, kc * 64, group);
+          }
+        } else {
+          const int cw = w_base + s * args.dil_w, ch = h_base + r * args.dil_h;
+          const int c2 = args.h_outer ? n0 : ch, c3 = args.h_outer ? ch : n0;
+          const int ck = kc * kElemsPerStage;
+          if (args.groups > 1) {
+            if (prefetch)
+              tma_prefetch_l2_5d(&tm_a, ck, group, cw, c2, c3);
+            else if constexpr (k2Cta)
+              tma_load_5d_pair(a_dst, &tm_a, full, ck, group, cw, c2, c3);
+            else
+              tma_load_5d(a_dst, &tm_a, full, ck, group, cw, c2, c3);
+          } else if (prefetch) {
+            tma_prefetch_l2_4d(&tm_a, ck, cw, c2, c3);
+          } else if constexpr (k2Cta) {
+            tma_load_4d_pair(a_dst, &tm_a, full, ck, cw, c2, c3);
+          } else {
+            tma_load_4d(a_dst, &tm_a, full, ck, cw, c2, c3);
+          }
+        }
         if constexpr (!kResB) {
           // with a halo strip the stage carries the weight tiles of every filter row
           const int row_taps = kHalo ? args.taps_h : 1;
           for (int rr = 0; rr < row_taps; ++rr)
-            load_b(a_dst + args.a_stage_bytes + rr * S::kBBytes, full, kHalo ? rr : r, s, kc, n_col,
+            load_b(a_dst + args.a_stage_bytes + rr * S::kBBytes, full, group, kHalo ? rr : r, s, kc, n_col,
                    prefetch);
         }
       };
       // While the predecessor kernel may still be running: pull the boxes of
       // this producer's first steps towards L2.
       if (first_unit < total_units) {
-        int tile, split, it_begin, it_end;
-        unit_coords(first_unit, tile, split, it_begin, it_end);
+        int tile, group, split, it_begin, it_end;
+        unit_coords(first_unit, tile, group, split, it_begin, it_end);
         int m_idx, n_idx;
         tile_coords(tile, m_idx, n_idx);
         int w0, h0, n0;
@@ -429,7 +480,7 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
         for (int it = it_begin + me; it < steps; it += P) {
           int r, s, kc;
           step_coords(it, r, s, kc);
-          issue_step(true, 0u, 0u, r, s, kc, w0 * args.stride_w - args.pad_w,
+          issue_step(true, 0u, 0u, group, r, s, kc, w0 * args.stride_w - args.pad_w,
                      h0 * args.stride_h - args.pad_h, n0, n_idx * BN);
         }
       }
@@ -437,8 +488,8 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
       if (me == 0) PLB_TRACE_STAMP(2, 4002);
       for (int unit = first_unit; unit < total_units && ok; unit += unit_stride) {
         if (me == 0) { PLB_TRACE_STAMP(0, trace_slot); ++trace_slot; }
-        int tile, split, it_begin, it_end;
-        unit_coords(unit, tile, split, it_begin, it_end);
+        int tile, group, split, it_begin, it_end;
+        unit_coords(unit, tile, group, split, it_begin, it_end);
         int m_idx, n_idx;
         tile_coords(tile, m_idx, n_idx);
         int w0, h0, n0;
@@ -459,9 +510,12 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
             }
             if (me == 0) { PLB_TRACE_STAMP(0, trace_slot); ++trace_slot; }
             const uint32_t a_dst = smem_base + stage * stage_bytes;
-            if (leader) mbar_expect_tx(full_bar(stage), kPairFactor * uint32_t(stage_bytes));
+            if (leader)
+              mbar_expect_tx(full_bar(stage),
+                             kPairFactor * uint32_t(args.a_stage_bytes +
+                                                    (kResB ? 0 : args.b_tiles_per_stage * args.b_box_bytes)));
             const uint32_t full = lead_bar(full_bar(stage));
-            issue_step(false, a_dst, full, r, s, kc, w_base, h_base, n0, n_col);
+            issue_step(false, a_dst, full, group, r, s, kc, w_base, h_base, n0, n_col);
             if (me == 0) { PLB_TRACE_STAMP(0, trace_slot); ++trace_slot; }
             stage += P;
             if (stage >= kStages) {
@@ -489,7 +543,7 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
     const int n_issuers = args.dual_issue ? 2 : 1;
     if (mi < n_issuers && leader && elect_one()) {
       const uint32_t idesc =
-          make_idesc(k2Cta ? 2 * kTileM : kTileM, BN, 0, 0, false, kBMn) | args.idesc_formats;
+          make_idesc(k2Cta ? 2 * kTileM : kTileM, uint32_t(args.n_mma), 0, 0, kAMn, kBMn) | args.idesc_formats;
       // completion of the MMAs issued so far -> barrier (in both CTAs of a pair)
       auto commit = [&](uint32_t bar) {
         if constexpr (k2Cta)
@@ -497,7 +551,7 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
         else
           umma_commit(bar);
       };
-      const uint64_t a_desc0 = make_smem_desc(smem_base, 16, 1024);
+      const uint64_t a_desc0 = make_smem_desc(smem_base, kAMn ? 64 * kStageKBytes : 16, 1024);
       // B tiles: resident ones start at resb_base, streamed ones follow the
       // activations inside their stage
       const uint64_t b_desc0 =
@@ -523,8 +577,8 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
         }
       }
       for (int unit = first_unit; unit < total_units && ok; unit += unit_stride, ++local_tile) {
-        int tile, split, it_begin, it_end;
-        unit_coords(unit, tile, split, it_begin, it_end);
+        int tile, group, split, it_begin, it_end;
+        unit_coords(unit, tile, group, split, it_begin, it_end);
         if (n_issuers == 2 && (local_tile & 1) != mi) {
           // the other issuer's tile: step over its pipeline stages
           stage += it_end - it_begin;
@@ -547,7 +601,7 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
         if (mi == 0) { PLB_TRACE_STAMP(1, trace_slot); ++trace_slot; }
         const uint32_t d_tmem = tmem_base + acc * BN;
         int s_tap = 0, kc = 0;  // halo mode: pipeline step = (s_tap, kc), kc fastest
-        if (kHalo && it_begin != 0) {
+        if (it_begin != 0) {
           kc = it_begin % args.k_chunks;
           s_tap = it_begin / args.k_chunks;
         }
@@ -573,12 +627,15 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
           else
             b_desc = b_desc0 + stage_off16;
           const int row_taps = kHalo ? args.taps_h : 1;
+          // (the K range past the last channel holds zeros: no instruction for it)
+          const int k_steps = kc == args.k_chunks - 1 ? args.k_last : 4;
           for (int r = 0; r < row_taps; ++r) {
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
+              if (k >= k_steps) break;
               // one instruction consumes 32 bytes of K: advance the start address
               // inside the swizzle span (K-major) or by 16 rows (MN-major B)
-              const uint64_t a_k = a_desc + uint64_t(k * 2);
+              const uint64_t a_k = a_desc + uint64_t(kAMn ? k * ((16 * kStageKBytes) >> 4) : k * 2);
               const uint64_t b_k =
                   b_desc + uint64_t(kBMn ? k * ((16 * kStageKBytes) >> 4) : k * 2);
               if constexpr (k2Cta)
@@ -668,16 +725,16 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
         for (int it = warp - 4; it < k_iters; it += 16) {
           int r, s, kc;
           step_coords(it, r, s, kc);
-          load_b(0u, 0u, r, s, kc, 0, true);
+          load_b(0u, 0u, 0, r, s, kc, 0, true);
         }
         pdl_wait();
         if (warp == 4 && leader)
-          mbar_expect_tx(resb_bar, kPairFactor * uint32_t(k_iters) * S::kBBytes);
+          mbar_expect_tx(resb_bar, kPairFactor * uint32_t(k_iters * args.b_box_bytes));
         const uint32_t resb_bar_lead = lead_bar(resb_bar);
         for (int it = warp - 4; it < k_iters; it += 16) {
           int r, s, kc;
           step_coords(it, r, s, kc);
-          load_b(resb_base + it * S::kBBytes, resb_bar_lead, r, s, kc, 0, false);
+          load_b(resb_base + it * S::kBBytes, resb_bar_lead, 0, r, s, kc, 0, false);
         }
         if (warp == 4) PLB_TRACE_STAMP(2, 4012);
       }
@@ -686,8 +743,8 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
     pdl_wait();
     for (int unit = first_unit + group * unit_stride; unit < total_units;
          unit += 2 * unit_stride, local_tile += 2) {
-      int tile, split, it_begin, it_end;
-      unit_coords(unit, tile, split, it_begin, it_end);
+      int tile, cgroup, split, it_begin, it_end;
+      unit_coords(unit, tile, cgroup, split, it_begin, it_end);
       int m_idx, n_idx;
       tile_coords(tile, m_idx, n_idx);
       int w0, h0, n0;
@@ -698,7 +755,7 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
       const long long pixel = (static_cast<long long>(on) * args.out_h + oh) * args.out_w + ow;
       const long long out_off = static_cast<long long>(on) * args.out_stride_n +
                                 static_cast<long long>(oh) * args.out_stride_h +
-                                static_cast<long long>(ow) * args.ldc;
+                                static_cast<long long>(ow) * args.ldc + cgroup * args.out_group_stride;
       if (stamp) PLB_TRACE_STAMP(2, local_tile * 4 + 0);
       if (!mbar_wait(tmem_full_bar(acc), acc_phase, abort_flag)) {
         atomicCAS(args.status, kStatusOk, kStatusEpilogueTimeout);
@@ -709,6 +766,8 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
       if (stamp) PLB_TRACE_STAMP(2, local_tile * 4 + 1);
       const uint32_t t_addr = tmem_base + acc * BN + (static_cast<uint32_t>(quarter * 32) << 16);
       const int col_base = n_idx * BN;
+      // columns of the tile that exist, in blocks of 32
+      const int cols_end = min(BN, (args.n_total - col_base + 31) & ~31);
       const bool box_ok = w0 + qw < args.out_w && h0 + qh < args.out_h && n0 + qn < args.out_n;
       auto release_accumulator = [&]() {
         tc_fence_before_sync();
@@ -736,16 +795,18 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
         if (args.bias != nullptr) {
 #pragma unroll
           for (int j = 0; j < 32; ++j)
-            if (j < valid) f[j] += args.bias[col0 + j];
+            if (j < valid) f[j] += args.bias[cgroup * args.n_total + col0 + j];
         }
         if (args.addend != nullptr && row_ok) {
           if (out_f32) {
-            const float *src = static_cast<const float *>(args.addend) + pixel * args.ld_addend + col0;
+            const float *src = static_cast<const float *>(args.addend) + pixel * args.ld_addend +
+                               cgroup * args.addend_group_stride + col0;
 #pragma unroll
             for (int j = 0; j < 32; ++j)
               if (j < valid) f[j] += args.beta * src[j];
           } else {
-            const __half *src = static_cast<const __half *>(args.addend) + pixel * args.ld_addend + col0;
+            const __half *src = static_cast<const __half *>(args.addend) + pixel * args.ld_addend +
+                                cgroup * args.addend_group_stride + col0;
 #pragma unroll
             for (int j = 0; j < 32; ++j)
               if (j < valid) f[j] += args.beta * __half2float(src[j]);
@@ -802,15 +863,85 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
           }
         }
       };
+      // The same for rows whose addresses allow no vector (a row pitch that is not
+      // a multiple of 16 bytes): lane after lane writing its own row would touch a
+      // sector per element, so the block is turned in shared memory (16-byte
+      // pieces XOR-swizzled with the row) and leaves row by row, consecutive lanes
+      // at consecutive columns, two rows per instruction.
+      auto store_rows = [&](const float (&f)[32], const int c) {
+        const uint32_t wbuf = staging_base + uint32_t(warp - 4) * 2048u;
+        const uint32_t wrow = wbuf + uint32_t(lane) * 64u, sw = (uint32_t(lane) >> 1) & 3u;
+        const int col0 = col_base + c, valid = min(32, args.n_total - col0);
+        const long long my_off = row_ok ? split * args.split_stride + out_off + col0 : -1ll;
+        const uint32_t lo = uint32_t(my_off), hi = uint32_t(my_off >> 32);
+        if (out_f32) {
+          // 16 columns (64 bytes of fp32) at a time
+#pragma unroll
+          for (int b = 0; b < 2; ++b) {
+            __syncwarp();
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              st_shared_v4(wrow + ((uint32_t(j) ^ sw) << 4), __float_as_uint(f[16 * b + 4 * j]),
+                           __float_as_uint(f[16 * b + 4 * j + 1]), __float_as_uint(f[16 * b + 4 * j + 2]),
+                           __float_as_uint(f[16 * b + 4 * j + 3]));
+            __syncwarp();
+            const int cc = lane & 15;
+#pragma unroll 4
+            for (int r0 = 0; r0 < 32; r0 += 2) {
+              const int r = r0 + (lane >> 4);
+              const uint32_t v0 = ld_shared_b32(wbuf + uint32_t(r) * 64u +
+                                                (((uint32_t(cc) >> 2) ^ ((uint32_t(r) >> 1) & 3u)) << 4) +
+                                                (uint32_t(cc) & 3u) * 4u);
+              const long long off = (long long)(uint64_t(__shfl_sync(0xffffffffu, hi, r)) << 32 |
+                                                __shfl_sync(0xffffffffu, lo, r));
+              if (off >= 0 && 16 * b + cc < valid) static_cast<float *>(args.out)[off + 16 * b + cc] = __uint_as_float(v0);
+            }
+          }
+        } else {
+          __syncwarp();
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            __half2 h0 = __floats2half2_rn(f[8 * j], f[8 * j + 1]);
+            __half2 h1 = __floats2half2_rn(f[8 * j + 2], f[8 * j + 3]);
+            __half2 h2 = __floats2half2_rn(f[8 * j + 4], f[8 * j + 5]);
+            __half2 h3 = __floats2half2_rn(f[8 * j + 6], f[8 * j + 7]);
+            st_shared_v4(wrow + ((uint32_t(j) ^ sw) << 4), *reinterpret_cast<uint32_t *>(&h0),
+                         *reinterpret_cast<uint32_t *>(&h1), *reinterpret_cast<uint32_t *>(&h2),
+                         *reinterpret_cast<uint32_t *>(&h3));
+          }
+          __syncwarp();
+          // lanes 0..15 and 16..31: a row each, two columns per lane
+          const int cc = (lane & 15) * 2;
+#pragma unroll 4
+          for (int r0 = 0; r0 < 32; r0 += 2) {
+            const int r = r0 + (lane >> 4);
+            const uint32_t v0 = ld_shared_b32(wbuf + uint32_t(r) * 64u +
+                                              (((uint32_t(cc) >> 3) ^ ((uint32_t(r) >> 1) & 3u)) << 4) +
+                                              (uint32_t(cc) & 7u) * 2u);
+            const long long off = (long long)(uint64_t(__shfl_sync(0xffffffffu, hi, r)) << 32 |
+                                              __shfl_sync(0xffffffffu, lo, r));
+            if (off >= 0) {
+              uint16_t *dst = static_cast<uint16_t *>(args.out) + off + cc;
+              if (cc + 1 < valid && (reinterpret_cast<uintptr_t>(dst) & 3) == 0) {
+                *reinterpret_cast<uint32_t *>(dst) = v0;
+              } else {
+                if (cc < valid) dst[0] = uint16_t(v0);
+                if (cc + 1 < valid) dst[1] = uint16_t(v0 >> 16);
+              }
+            }
+          }
+        }
+      };
       // issue (lane 0) the tensor store of the staged buffer: columns [store_col, +128 bytes)
       auto store_staged = [&](const uint32_t buf, const int store_col) {
         if (lane == 0) {
           // a box that starts outside the tensor has nothing to write
           if (store_col < args.n_total && box_ok) {
-            if (args.h_outer)
-              tma_store_4d(&tm_out, buf, store_col, w0 + qw, n0 + qn, h0 + qh);
+            const int c2 = args.h_outer ? n0 + qn : h0 + qh, c3 = args.h_outer ? h0 + qh : n0 + qn;
+            if (args.groups > 1)
+              tma_store_5d(&tm_out, buf, store_col, cgroup, w0 + qw, c2, c3);
             else
-              tma_store_4d(&tm_out, buf, store_col, w0 + qw, h0 + qh, n0 + qn);
+              tma_store_4d(&tm_out, buf, store_col, w0 + qw, c2, c3);
           }
           tma_store_commit();
         }
@@ -821,22 +952,26 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
       if (!tma_store) {
         // each warp stores its own 32 columns of every 64-column block
 #pragma unroll 1
-        for (int c = half * 32; c < BN; c += 64) {
+        for (int c = half * 32; c < cols_end; c += 64) {
           __syncwarp();
           tmem_ld_32x32(t_addr + c, v);
           tmem_ld_wait_for(v);
-          if (c + 64 >= BN) release_accumulator();
+          if (c + 64 >= cols_end) release_accumulator();
           finish(v, f, c);
-          store_direct(f, c);
+          if (args.scatter_rows)
+            store_rows(f, c);
+          else
+            store_direct(f, c);
         }
+        if (half * 32 >= cols_end) release_accumulator();
       } else if (out_f32) {
         // (half == 0 warps only) one 32-column chunk per staged buffer and store
 #pragma unroll 1
-        for (int c = 0; c < BN; c += 32) {
+        for (int c = 0; c < cols_end; c += 32) {
           __syncwarp();
           tmem_ld_32x32(t_addr + c, v);
           tmem_ld_wait_for(v);
-          if (c + 32 >= BN) release_accumulator();
+          if (c + 32 >= cols_end) release_accumulator();
           finish(v, f, c);
           if (lane == 0) tma_store_wait_read<0>();  // the previous store has read the buffer
           __syncwarp();
@@ -859,11 +994,11 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
         const uint32_t wrow = wbuf + uint32_t(lane) * 64u;
         const uint32_t sw = (uint32_t(lane) >> 1) & 3u;
 #pragma unroll 1
-        for (int c = half * 32; c < BN; c += 64) {
+        for (int c = half * 32; c < cols_end; c += 64) {
           __syncwarp();
           tmem_ld_32x32(t_addr + c, v);
           tmem_ld_wait_for(v);
-          if (c + 64 >= BN) release_accumulator();
+          if (c + 64 >= cols_end) release_accumulator();
           finish(v, f, c);
           if (lane == 0) tma_store_wait_read<0>();  // this warp's previous store has read the buffer
           __syncwarp();
@@ -881,6 +1016,7 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
           __syncwarp();
           store_staged(wbuf, col_base + c);
         }
+        if (half * 32 >= cols_end) release_accumulator();
       }
       if (stamp) PLB_TRACE_STAMP(2, local_tile * 4 + 2);
       if (stamp) PLB_TRACE_STAMP(2, local_tile * 4 + 3);
@@ -906,8 +1042,8 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
     int my_tiles = 0;
     long long total_steps = 0;
     for (int unit = first_unit; unit < total_units; unit += unit_stride, ++my_tiles) {
-      int tile, split, it_begin, it_end;
-      unit_coords(unit, tile, split, it_begin, it_end);
+      int tile, group, split, it_begin, it_end;
+      unit_coords(unit, tile, group, split, it_begin, it_end);
       total_steps += it_end - it_begin;
     }
     const long long start = clock64();

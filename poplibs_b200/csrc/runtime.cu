@@ -159,20 +159,22 @@ static int launchTranspose(plb_context *ctx, uint32_t elem_bytes, uint64_t batch
   return PLB_OK;
 }
 
-// [G][K][Co][Ci] -> [G][K flipped][Ci][Co]; weights are small, one element per thread.
+// [G][K][Co][Ci] -> [G][K flipped][Ci][Co -> co_pitch]; weights are small, one element per thread.
 template <typename T>
-__global__ void transposeFlipKernel(const T *__restrict__ src, T *__restrict__ dst,
-                                    uint32_t groups, uint32_t kelems, uint32_t co, uint32_t ci) {
-  const size_t total = size_t(groups) * kelems * co * ci;
+__global__ void transposeFlipKernel(const T *__restrict__ src, T *__restrict__ dst, uint32_t groups,
+                                    uint32_t kelems, uint32_t co, uint32_t ci, uint32_t co_pitch) {
+  pdl_launch_dependents();
+  pdl_wait();  // the weights may come from the previous kernel in the stream
+  const size_t total = size_t(groups) * kelems * co_pitch * ci;
   for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < total;
        i += size_t(gridDim.x) * blockDim.x) {
-    const uint32_t o = uint32_t(i % co);
-    size_t r = i / co;
+    const uint32_t o = uint32_t(i % co_pitch);
+    size_t r = i / co_pitch;
     const uint32_t c = uint32_t(r % ci);
     r /= ci;
     const uint32_t k = uint32_t(r % kelems);
     const uint32_t g = uint32_t(r / kelems);
-    dst[i] = src[((size_t(g) * kelems + (kelems - 1 - k)) * co + o) * ci + c];
+    dst[i] = o < co ? src[((size_t(g) * kelems + (kelems - 1 - k)) * co + o) * ci + c] : T(0);
   }
 }
 
@@ -288,61 +290,6 @@ __global__ void fillKernel(T *dst, T value, size_t n) {
   for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n;
        i += size_t(gridDim.x) * blockDim.x)
     dst[i] = value;
-}
-
-// Copies rows of `c_src` elements into rows of `c_dst` elements (same row
-// count), zero-filling the tail when the destination rows are longer and
-// dropping it when they are shorter: channel padding / un-padding.
-__global__ void resizeRowsKernel(const uint8_t *__restrict__ src, uint8_t *__restrict__ dst,
-                                 size_t rows, uint32_t src_bytes, uint32_t dst_bytes) {
-  // 2-byte granularity covers half and quarter-pairs; odd byte counts use bytes
-  const size_t total = rows * dst_bytes;
-  for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < total;
-       i += size_t(gridDim.x) * blockDim.x) {
-    const size_t r = i / dst_bytes;
-    const uint32_t b = uint32_t(i - r * dst_bytes);
-    dst[i] = b < src_bytes ? src[r * src_bytes + b] : uint8_t(0);
-  }
-}
-
-int resizeRows(plb_context *ctx, const void *src, void *dst, size_t rows, size_t src_bytes,
-               size_t dst_bytes) {
-  if (rows == 0 || dst_bytes == 0) return PLB_OK;
-  const size_t total = rows * dst_bytes;
-  const int grid = int(std::min<size_t>((total + 255) / 256, size_t(ctx->sm_count) * 16));
-  resizeRowsKernel<<<grid, 256, 0, ctx->stream>>>(static_cast<const uint8_t *>(src),
-                                                  static_cast<uint8_t *>(dst), rows,
-                                                  uint32_t(src_bytes), uint32_t(dst_bytes));
-  PLB_CUDA(cudaGetLastError());
-  ctx->launches++;
-  return PLB_OK;
-}
-
-// The same for source rows `src_pitch` bytes apart: dst row r = the first
-// `row_bytes` bytes of source row r, zero-filled up to `dst_pitch`.
-__global__ void copyRowsPitchedKernel(const uint8_t *__restrict__ src, size_t src_pitch,
-                                      uint8_t *__restrict__ dst, uint32_t dst_pitch, size_t rows,
-                                      uint32_t row_bytes) {
-  const size_t total = rows * dst_pitch;
-  for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < total;
-       i += size_t(gridDim.x) * blockDim.x) {
-    const size_t r = i / dst_pitch;
-    const uint32_t b = uint32_t(i - r * dst_pitch);
-    dst[i] = b < row_bytes ? src[r * src_pitch + b] : uint8_t(0);
-  }
-}
-
-int copyRowsPitched(plb_context *ctx, const void *src, size_t src_pitch, void *dst, size_t dst_pitch,
-                    size_t rows, size_t row_bytes) {
-  if (rows == 0 || dst_pitch == 0) return PLB_OK;
-  const size_t total = rows * dst_pitch;
-  const int grid = int(std::min<size_t>((total + 255) / 256, size_t(ctx->sm_count) * 16));
-  copyRowsPitchedKernel<<<grid, 256, 0, ctx->stream>>>(static_cast<const uint8_t *>(src), src_pitch,
-                                                       static_cast<uint8_t *>(dst), uint32_t(dst_pitch),
-                                                       rows, uint32_t(row_bytes));
-  PLB_CUDA(cudaGetLastError());
-  ctx->launches++;
-  return PLB_OK;
 }
 
 // dst[n][h][w][:] = src[n][flip_h ? H-1-h : h][flip_w ? W-1-w : w][:], pixels of
@@ -512,6 +459,24 @@ int dilateField(plb_context *ctx, const void *src, void *dst, size_t n_images, c
   PLB_CUDA(cudaGetLastError());
   ctx->launches++;
   return PLB_OK;
+}
+
+int transposeFlipWeights(plb_context *ctx, uint32_t elem_bytes, uint32_t groups, uint32_t out_chans,
+                         uint32_t in_chans, uint64_t kernel_elems, uint32_t dst_pitch, const void *src, void *dst) {
+  const size_t total = size_t(groups) * kernel_elems * dst_pitch * in_chans;
+  if (total == 0) return PLB_OK;
+  const dim3 grid(unsigned(std::min<size_t>((total + 255) / 256, size_t(ctx->sm_count) * 16)));
+  auto launch = [&](auto t) {
+    using T = decltype(t);
+    return launchPdl(ctx, transposeFlipKernel<T>, grid, dim3(256), 0, static_cast<const T *>(src),
+                     static_cast<T *>(dst), groups, uint32_t(kernel_elems), out_chans, in_chans, dst_pitch);
+  };
+  switch (elem_bytes) {
+    case 1: return launch(uint8_t());
+    case 2: return launch(uint16_t());
+    case 4: return launch(uint32_t());
+    default: return fail(PLB_ERR_INVALID_PARAMS, "element size must be 1, 2 or 4 bytes");
+  }
 }
 
 int launchScaleRows(plb_context *ctx, void *out, const void *c, float beta, bool out_f32,
@@ -728,31 +693,7 @@ int plb_weights_transpose_chans_flip_xy(plb_context *ctx, uint32_t elem_bytes, u
                                         uint32_t out_chans, uint32_t in_chans,
                                         uint64_t kernel_elems, const void *d_src, void *d_dst) {
   if (int rc = activate(ctx)) return rc;
-  const size_t total = size_t(groups) * kernel_elems * out_chans * in_chans;
-  if (total == 0) return PLB_OK;
-  const int grid = int(std::min<size_t>((total + 255) / 256, 148 * 16));
-  switch (elem_bytes) {
-    case 1:
-      transposeFlipKernel<uint8_t><<<grid, 256, 0, ctx->stream>>>(
-          static_cast<const uint8_t *>(d_src), static_cast<uint8_t *>(d_dst), groups,
-          uint32_t(kernel_elems), out_chans, in_chans);
-      break;
-    case 2:
-      transposeFlipKernel<uint16_t><<<grid, 256, 0, ctx->stream>>>(
-          static_cast<const uint16_t *>(d_src), static_cast<uint16_t *>(d_dst), groups,
-          uint32_t(kernel_elems), out_chans, in_chans);
-      break;
-    case 4:
-      transposeFlipKernel<uint32_t><<<grid, 256, 0, ctx->stream>>>(
-          static_cast<const uint32_t *>(d_src), static_cast<uint32_t *>(d_dst), groups,
-          uint32_t(kernel_elems), out_chans, in_chans);
-      break;
-    default:
-      return fail(PLB_ERR_INVALID_PARAMS, "element size must be 1, 2 or 4 bytes");
-  }
-  PLB_CUDA(cudaGetLastError());
-  ctx->launches++;
-  return PLB_OK;
+  return transposeFlipWeights(ctx, elem_bytes, groups, out_chans, in_chans, kernel_elems, out_chans, d_src, d_dst);
 }
 
 int plb_transpose_matrix(plb_context *ctx, uint32_t elem_bytes, uint32_t groups, uint32_t rows,

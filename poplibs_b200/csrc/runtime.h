@@ -16,21 +16,21 @@
 // another (3-D -> 2-D -> flipped -> dilated -> padded channels ...), so every
 // pre-pass has a slot of its own.
 enum plb_scratch_slot {
-  kSlotOperands = 0,    // rearranged operands, split-K partial sums, gathered sub-filters
+  kSlotOperands = 0,    // rearranged operands (transposed, space-to-depth)
+  kSlotWuPartials,      // fp32 partial sums of a weight update
   kSlotHostIn,          // staging of the host-buffer entry points
   kSlotHostWeights,
   kSlotHostOut,
   kSlotHostBias,
   kSlotChannelSums,     // partial per-channel sums (normalisation, bias update)
-  kSlotUsedTaps,        // taps of a truncated / flipped kernel
-  kSlotPaddedChans,     // zero-padded channel counts
+  kSlotUsedTaps,        // gradient of a truncated / flipped kernel's taps
+  kSlotRepacked,        // operands with rows rounded up to 16 bytes / split into bfloat16 pieces
   kSlotFlipped,         // reversed input (input flip)
   kSlotDepthFold,       // depth taps of a 3-D field gathered into the channels
   kSlotFoldedWeights,
   kSlotFoldedGrads,
   kSlotDilated,         // zero-stuffed input (input dilation)
   kSlotSplitK,          // fp32 partial sums of a split-K forward / backward / matrix product
-  kSlotFloatSplit,      // bfloat16 pieces of float operands
   kSlotCount
 };
 
@@ -122,11 +122,33 @@ inline size_t dtypeBytes(int dtype) {
 // 16-bit floating-point operands (the kind::f16 instruction takes either)
 inline bool is16BitFloat(int dtype) { return dtype == PLB_HALF || dtype == PLB_BFLOAT16; }
 
-// Row resize (runtime.cu): rows of src_bytes -> rows of dst_bytes, zero fill / drop of the tail.
-int resizeRows(plb_context *ctx, const void *src, void *dst, size_t rows, size_t src_bytes,
-               size_t dst_bytes);
-int copyRowsPitched(plb_context *ctx, const void *src, size_t src_pitch, void *dst, size_t dst_pitch,
-                    size_t rows, size_t row_bytes);
+// ---- operands brought into a form TMA can address (repack.cu) -------------------
+enum RepackMode : int {
+  kRepackCopy = 0,        // row -> row, zero-filled up to dst_pitch
+  kRepackSplitCols = 1,   // float row of c -> one row of 3c bfloat16 (the pieces side by side), zero-filled
+  kRepackSplitPlanes = 2, // float [outer][mid] rows -> [outer][3][mid] rows of bfloat16, each zero-filled
+};
+struct Repack {
+  const void *src;
+  void *dst;              // 16-byte aligned
+  uint64_t rows;
+  uint32_t cols;          // elements of a source row
+  uint64_t src_pitch;     // elements
+  uint32_t dst_pitch;     // elements, a multiple of 16 bytes
+  uint32_t elem_bytes;    // of the source
+  int mode;
+  bool weights;           // pieces (hi, hi, lo), else (hi, lo, hi)
+  uint64_t mid;           // kRepackSplitPlanes: rows per plane (0 = all)
+};
+// Bytes of the destination.
+size_t repackBytes(const Repack &r);
+// One launch for up to two operands.
+int repack(plb_context *ctx, const Repack *jobs, int n);
+// Rows of `elems` elements rounded up to whole 16-byte vectors.
+inline uint32_t roundToVec(uint64_t elems, size_t elem_bytes) {
+  const uint64_t q = 16 / elem_bytes;
+  return uint32_t((elems + q - 1) / q * q);
+}
 
 // Input flip of the reference's input transform: the convolution of a flipped
 // input equals the convolution of the reversed tensor with the input padding and
@@ -186,6 +208,12 @@ struct IgemmProblem {
   bool bf16 = false;     // 16-bit operands are bfloat16 (else half)
   int fmt_a = 0, fmt_b = 0;  // plb_quarter_format of the activations / weights when fp8
   bool b_mn = false;     // right operand stored [tap][K][N], N contiguous
+  bool a_mn = false;     // matrix product whose left operand is stored [K][M] (act_dims = (K, M), stride of a K row)
+  // Groups: independent contractions of one shape.  The weights of group g are
+  // the tiles [g * taps_stored, (g + 1) * taps_stored) of wgt_dims[2].
+  int groups = 1;
+  uint64_t act_group_stride = 0;                               // bytes
+  long long out_group_stride = 0, addend_group_stride = 0;     // elements
   // activations: 4-D tensor (C, W, H, N) with byte strides of W, H, N
   const void *act = nullptr;
   uint64_t act_dims[4] = {1, 1, 1, 1};
@@ -201,6 +229,9 @@ struct IgemmProblem {
   int k_per_tap = 0;                    // reduction length per tap (elements)
   int taps_h = 1, taps_w = 1, pad_h = 0, pad_w = 0, dil_h = 1, dil_w = 1;
   int flip_h = 0, flip_w = 0;
+  // Sub-lattice of a stored filter (0 = dense): tap (r, s) after the flip is tile
+  // (tap_first_h + r * tap_step_h) * tap_pitch_h + tap_first_w + s * tap_step_w.
+  int tap_first_h = 0, tap_step_h = 1, tap_pitch_h = 0, tap_first_w = 0, tap_step_w = 1, taps_stored = 0;
   int stride_h = 1, stride_w = 1;
   void *out = nullptr;
   long long ldc = 0;  // elements between output pixels along w
@@ -220,21 +251,13 @@ struct IgemmProblem {
 // problem cannot be run by the igemm kernel (message recorded).
 int planIgemm(const IgemmProblem &p, int sm_count, plb_plan *plan);
 
-// ---- float operands (float_route.cu) ------------------------------------------
-// The layer / product that runs for float operands: bfloat16, the reduction
-// dimension of the pass three times as long.
+// What runs for float operands: bfloat16, the reduction dimension of the pass
+// three times as long (repack.cu).  For the plans.
 plb_conv_params floatRouteConvParams(const plb_conv_params &p, int pass);
 plb_matmul_desc floatRouteMatmulDesc(const plb_matmul_desc &d);
-int floatConvFwd(plb_context *ctx, const plb_conv_params &p, const plb_conv_options *opt,
-                 const void *d_in, const void *d_weights, const float *d_bias, void *d_out,
-                 int transpose_and_flip_weights);
-int floatConvBwd(plb_context *ctx, const plb_conv_params &p, const plb_conv_options *opt,
-                 const void *d_out_grads, const void *d_weights, void *d_in_grads);
-int floatConvWu(plb_context *ctx, const plb_conv_params &p, const plb_conv_options *opt,
-                const void *d_acts, const void *d_out_grads, void *d_weight_grads,
-                float *d_weight_grads_f32);
-int floatMatmul(plb_context *ctx, const plb_matmul_desc &d, const void *d_a, const void *d_b,
-                const void *d_c, void *d_d);
+// weights_transpose_chans_flip_xy with a row pitch (elements) of the result.
+int transposeFlipWeights(plb_context *ctx, uint32_t elem_bytes, uint32_t groups, uint32_t out_chans,
+                         uint32_t in_chans, uint64_t kernel_elems, uint32_t dst_pitch, const void *src, void *dst);
 
 int launchIgemm(plb_context *ctx, const IgemmProblem &p, const plb_plan &plan);
 

@@ -24,18 +24,10 @@
 
 #include "conv_geometry.h"
 #include "runtime.h"
+#include "small_channel.h"
+#include "sm100_prims.cuh"
 
 namespace plb {
-
-struct S2dShape {
-  int N, H, W, C;       // input
-  int s, padH, padW;    // stride (both dims), padding
-  int KH, KW;
-  int OH, OW;
-  int Cp, C2;           // padded channels per original pixel, channels of X2
-  int K2h, K2w;         // taps after folding the stride
-  int H2, W2;           // extent of X2
-};
 
 // X2[n][h2][w2][(ph*s + pw)*Cp + c] = X[n][h2*s + ph - padH][w2*s + pw - padW][c]
 __global__ void s2dInputKernel(const __half *__restrict__ x, __half *__restrict__ x2, S2dShape g) {
@@ -163,7 +155,8 @@ s2dStem3Kernel(const uint32_t *__restrict__ x32, uint4 *__restrict__ x2, S2dShap
                const __half *__restrict__ w, __half *__restrict__ w2, int co_total) {
   // the convolution that follows may set itself up meanwhile; it waits for this
   // grid to finish before it reads
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  pdl_launch_dependents();
+  pdl_wait();  // (the input, or X2 of an earlier call, may belong to the previous kernel)
   const unsigned rows = unsigned(g.N) * unsigned(g.H2);
   if (blockIdx.x >= rows) {
     const unsigned total = unsigned(g.K2h) * unsigned(co_total) * 64u;
@@ -221,10 +214,9 @@ s2dStem3Kernel(const uint32_t *__restrict__ x32, uint4 *__restrict__ x2, S2dShap
 }
 
 
-// Returns PLB_ERR_UNSUPPORTED (with a message) when the layer does not fit this path.
-int convFwdSmallChannels(plb_context *ctx, const plb_conv_params &p, const plb_conv_options *opt,
-                         const void *d_in, const void *d_weights, const float *d_bias,
-                         void *d_out, plb_plan *plan_only) {
+// The shape of the rearranged layer; PLB_ERR_UNSUPPORTED (with a message) when it
+// does not fit this path.
+int smallChannelShape(const plb_conv_params &p, S2dShape *out) {
   if (p.num_field_dims != 2 || p.groups != 1 || !is16BitFloat(p.input_type))
     return fail(PLB_ERR_UNSUPPORTED,
                 "input channel count must be a multiple of 8 (half) / 16 (quarter) unless the "
@@ -262,13 +254,61 @@ int convFwdSmallChannels(plb_context *ctx, const plb_conv_params &p, const plb_c
                     std::to_string(g.K2w * g.C2) + " elements exceeds one 128-byte K step");
   g.H2 = g.OH + g.K2h - 1;
   g.W2 = g.OW + g.K2w - 1;
+  *out = g;
+  return PLB_OK;
+}
+
+// Elements of X2, the window of the last pixel included: it may run past the
+// K2w*C2 elements that carry weights (64 elements, cleared).
+size_t smallChannelElems(const S2dShape &g) { return size_t(g.N) * g.H2 * g.W2 * g.C2 + 64; }
+
+// Writes X2, and with `w2` the folded weights ([K2h][co][64]).
+int smallChannelPrepare(plb_context *ctx, const S2dShape &g, const void *d_in, __half *x2, const void *d_weights,
+                        __half *w2, int co) {
+  const size_t w2_elems = w2 ? size_t(g.K2h) * co * 64 : 0;
+  const int row_elems = g.W * g.C;
+  const size_t smem = size_t(g.s) * ((row_elems + 7) & ~7) * 2 + size_t(g.C2) * sizeof(int);
+  if (g.C == 3 && g.s == 2 && g.Cp == 4 && row_elems % 2 == 0 &&
+      (reinterpret_cast<uintptr_t>(d_in) & 3) == 0 && size_t(g.N) * g.H2 < (size_t(1) << 31)) {
+    // (at least one block past the rows: it clears the tail of X2)
+    const unsigned wblocks = unsigned(std::max<size_t>(1, (w2_elems + 127) / 128));
+    return launchPdl(ctx, s2dStem3Kernel, dim3(unsigned(g.N) * unsigned(g.H2) + wblocks), dim3(128), 0,
+                     static_cast<const uint32_t *>(d_in), reinterpret_cast<uint4 *>(x2), g,
+                     static_cast<const __half *>(d_weights), w2, w2 ? co : 0);
+  }
+  if (smem <= 48 * 1024 && g.C < 256 && g.s < 256) {
+    const int rows_aligned = (row_elems % 8 == 0 && (reinterpret_cast<uintptr_t>(d_in) & 15) == 0) ? 1 : 0;
+    const int grid = int(std::min<size_t>(size_t(g.N) * g.H2, size_t(ctx->sm_count) * 16));
+    s2dInputRowsKernel<<<grid, 128, smem, ctx->stream>>>(static_cast<const __half *>(d_in), x2, g, rows_aligned);
+  } else {
+    const size_t vecs = size_t(g.N) * g.H2 * g.W2 * (g.C2 / 8);
+    const int grid = int(std::min<size_t>((vecs + 255) / 256, size_t(ctx->sm_count) * 16));
+    s2dInputKernel<<<grid, 256, 0, ctx->stream>>>(static_cast<const __half *>(d_in), x2, g);
+  }
+  PLB_CUDA(cudaGetLastError());
+  ctx->launches++;
+  // the 64 trailing elements only ever meet zero weights, but must be finite
+  PLB_CUDA(cudaMemsetAsync(x2 + size_t(g.N) * g.H2 * g.W2 * g.C2, 0, 128, ctx->stream));
+  if (w2) {
+    const int wgrid = int((w2_elems + 255) / 256);
+    s2dWeightsKernel<<<wgrid, 256, 0, ctx->stream>>>(static_cast<const __half *>(d_weights), w2, g, co);
+    PLB_CUDA(cudaGetLastError());
+    ctx->launches++;
+  }
+  return PLB_OK;
+}
+
+int convFwdSmallChannels(plb_context *ctx, const plb_conv_params &p, const plb_conv_options *opt,
+                         const void *d_in, const void *d_weights, const float *d_bias,
+                         void *d_out, plb_plan *plan_only) {
+  S2dShape g{};
+  if (int rc = smallChannelShape(p, &g)) return rc;
   const int co = int(p.out_chans_per_group);
-  // tail of the last row: the 64-element window of the last pixel may run past
-  // the K2w*C2 elements that carry weights; pad the allocation so it stays inside
-  const size_t x2_elems = size_t(g.N) * g.H2 * g.W2 * g.C2 + 64;
+  const size_t x2_elems = smallChannelElems(g);
   const size_t w2_elems = size_t(g.K2h) * co * 64;
 
   IgemmProblem q;
+  q.bf16 = p.input_type == PLB_BFLOAT16;
   q.act_dims[0] = 64;
   q.act_dims[1] = uint64_t(g.OW);
   q.act_dims[2] = uint64_t(g.H2);
@@ -285,7 +325,7 @@ int convFwdSmallChannels(plb_context *ctx, const plb_conv_params &p, const plb_c
   q.out_h = g.OH;
   q.out_n = g.N;
   q.n_total = co;
-  q.k_per_tap = 64;
+  q.k_per_tap = g.K2w * g.C2;  // (the rest of a window meets zero weights)
   q.taps_h = g.K2h;
   q.taps_w = 1;
   q.ldc = co;
@@ -313,40 +353,7 @@ int convFwdSmallChannels(plb_context *ctx, const plb_conv_params &p, const plb_c
   if (int rc = scratch(ctx, kSlotOperands, plan.workspace_bytes + 256, &ws)) return rc;
   __half *x2 = static_cast<__half *>(ws);
   __half *w2 = x2 + ((x2_elems + 127) & ~size_t(127));
-  {
-    bool fused_prep = false;
-    const int row_elems = g.W * g.C;
-    const size_t smem = size_t(g.s) * ((row_elems + 7) & ~7) * 2 + size_t(g.C2) * sizeof(int);
-    if (g.C == 3 && g.s == 2 && g.Cp == 4 && row_elems % 2 == 0 &&
-        (reinterpret_cast<uintptr_t>(d_in) & 3) == 0 && size_t(g.N) * g.H2 < (size_t(1) << 31)) {
-      const unsigned wblocks = unsigned((w2_elems + 127) / 128);
-      s2dStem3Kernel<<<unsigned(g.N) * unsigned(g.H2) + wblocks, 128, 0, ctx->stream>>>(
-          static_cast<const uint32_t *>(d_in), reinterpret_cast<uint4 *>(x2), g,
-          static_cast<const __half *>(d_weights), w2, co);
-      fused_prep = true;
-    } else if (smem <= 48 * 1024 && g.C < 256 && g.s < 256) {
-      const int rows_aligned =
-          (row_elems % 8 == 0 && (reinterpret_cast<uintptr_t>(d_in) & 15) == 0) ? 1 : 0;
-      const int grid = int(std::min<size_t>(size_t(g.N) * g.H2, size_t(ctx->sm_count) * 16));
-      s2dInputRowsKernel<<<grid, 128, smem, ctx->stream>>>(static_cast<const __half *>(d_in), x2, g,
-                                                           rows_aligned);
-    } else {
-      const size_t vecs = size_t(g.N) * g.H2 * g.W2 * (g.C2 / 8);
-      const int grid = int(std::min<size_t>((vecs + 255) / 256, size_t(ctx->sm_count) * 16));
-      s2dInputKernel<<<grid, 256, 0, ctx->stream>>>(static_cast<const __half *>(d_in), x2, g);
-    }
-    PLB_CUDA(cudaGetLastError());
-    ctx->launches++;
-    if (!fused_prep) {
-      // the 64 trailing elements only ever meet zero weights, but must be finite
-      PLB_CUDA(cudaMemsetAsync(x2 + size_t(g.N) * g.H2 * g.W2 * g.C2, 0, 128, ctx->stream));
-      const int wgrid = int((w2_elems + 255) / 256);
-      s2dWeightsKernel<<<wgrid, 256, 0, ctx->stream>>>(static_cast<const __half *>(d_weights), w2, g,
-                                                       co);
-      PLB_CUDA(cudaGetLastError());
-      ctx->launches++;
-    }
-  }
+  if (int rc = smallChannelPrepare(ctx, g, d_in, x2, d_weights, w2, co)) return rc;
   q.act = x2;
   q.wgt = w2;
   q.out = d_out;

@@ -6,6 +6,7 @@
 
 #include "conv_geometry.h"
 #include "runtime.h"
+#include "small_channel.h"
 #include "wu_sm100.cuh"
 
 namespace plb {
@@ -23,7 +24,7 @@ int wuShape(const plb_conv_params &p, WuShape *s) {
   if (!err.empty()) return fail(PLB_ERR_INVALID_PARAMS, err);
   if (p.num_field_dims > 2)
     return fail(PLB_ERR_UNSUPPORTED, "3-D convolutions are not implemented on this path yet");
-  if (!is16BitFloat(p.input_type))
+  if (!is16BitFloat(p.input_type) && p.input_type != PLB_FLOAT)
     // the reference never runs the weight update in quarter either
     // (tools/single_conv_layer.cpp:725-733)
     return fail(PLB_ERR_UNSUPPORTED, "weight update is implemented for half and float input only");
@@ -63,10 +64,50 @@ int wuShape(const plb_conv_params &p, WuShape *s) {
   return PLB_OK;
 }
 
-// Tiling of one group's weight update.
-void planWu(const plb_conv_params &p, const WuShape &s, int sm_count, int force_split,
-            unsigned plan_flags, WuArgs *a, plb_plan *plan) {
-  const int co = int(p.out_chans_per_group), ci = int(p.in_chans_per_group);
+// One contraction of the weight-gradient kernel: the operands as it reads them.
+struct WuProblem {
+  bool bf16 = false;
+  int batch = 0;
+  int ci = 0, co = 0;               // channels of a super-group (as stored)
+  int sgroups = 1, sub = 1;         // super-groups, groups in each
+  int sub_ci = 0, sub_co = 0;       // stored channels per group
+  WuShape s;                        // field, taps, padding, stride
+  // base address, channels of a pixel, byte strides of w, h, n
+  const void *x = nullptr, *dy = nullptr;
+  uint64_t x_chans = 0, dy_chans = 0, x_strides[3] = {}, dy_strides[3] = {};
+};
+
+// The layer's tensors [N][H][W][groups * pitch] with `sub` groups contracted
+// together (every sub'th group starts a super-group).
+WuProblem wuProblem(const plb_conv_params &p, const WuShape &s, uint32_t ci_pitch, uint32_t co_pitch, uint32_t groups,
+                    uint32_t sub) {
+  const size_t es = 2;
+  WuProblem q;
+  q.bf16 = p.input_type == PLB_BFLOAT16;
+  q.batch = int(p.batch);
+  q.sub = int(sub);
+  q.sgroups = int((groups + sub - 1) / sub);
+  q.sub_ci = int(ci_pitch);
+  q.sub_co = int(co_pitch);
+  q.ci = int(sub * ci_pitch);
+  q.co = int(sub * co_pitch);
+  q.s = s;
+  q.x_chans = uint64_t(groups) * ci_pitch;
+  q.dy_chans = uint64_t(groups) * co_pitch;
+  const uint64_t xp = uint64_t(p.groups) * ci_pitch * es, yp = uint64_t(p.groups) * co_pitch * es;
+  q.x_strides[0] = xp;
+  q.x_strides[1] = uint64_t(s.W) * xp;
+  q.x_strides[2] = uint64_t(s.H) * s.W * xp;
+  q.dy_strides[0] = yp;
+  q.dy_strides[1] = uint64_t(s.OW) * yp;
+  q.dy_strides[2] = uint64_t(s.OH) * s.OW * yp;
+  return q;
+}
+
+// Tiling of a weight update.
+void planWu(const WuProblem &p, int sm_count, int force_split, unsigned plan_flags, WuArgs *a, plb_plan *plan) {
+  const WuShape &s = p.s;
+  const int co = p.co, ci = p.ci;
   const int taps = s.KH * s.KW;
   a->taps_h = s.KH;
   a->taps_w = s.KW;
@@ -76,6 +117,12 @@ void planWu(const plb_conv_params &p, const WuShape &s, int sm_count, int force_
   a->dil_w = s.dilW;
   a->stride_h = s.strH;
   a->stride_w = s.strW;
+  a->sgroups = p.sgroups;
+  a->x_step = ci;
+  a->dy_step = co;
+  a->sub = p.sub;
+  a->sub_ci = p.sub_ci;
+  a->sub_co = p.sub_co;
   a->co_total = co;
   a->ci_total = ci;
   a->co_blocks = (co + 127) / 128;
@@ -116,7 +163,7 @@ void planWu(const plb_conv_params &p, const WuShape &s, int sm_count, int force_
   a->strip_mode = 0;
   // PLB_PLAN_NO_A_COLLECTOR: fetch the outGrad tile for every instruction (A/B timing)
   a->reuse_a = (plan_flags & PLB_PLAN_NO_A_COLLECTOR) ? 0 : 1;
-  a->idesc_formats = p.input_type == PLB_BFLOAT16 ? (make_idesc(0, 0, 1, 1, false, false) & ~(1u << 4)) : 0u;
+  a->idesc_formats = p.bf16 ? (make_idesc(0, 0, 1, 1, false, false) & ~(1u << 4)) : 0u;
   const int halo = (s.KH - 1) * s.dilH;
   if (s.KH > 1 && s.strH == 1 && s.KH * a->ci_blk <= 512 && (plan_flags & PLB_PLAN_NO_HALO) == 0) {
     long sbest = -1;
@@ -156,7 +203,7 @@ void planWu(const plb_conv_params &p, const WuShape &s, int sm_count, int force_
   a->tiles_n = (int(p.batch) + a->box_n - 1) / a->box_n;
   a->stage_bytes = stage_bytes;
   a->stages = std::max(2, std::min(kWuMaxStages, (200 * 1024) / stage_bytes));
-  const int units = a->co_blocks * a->ci_blocks * a->tap_groups;
+  const int units = a->sgroups * a->co_blocks * a->ci_blocks * a->tap_groups;
   int ksplit = force_split > 0 ? force_split : std::max(1, (sm_count > 0 ? sm_count : 148) / units);
   ksplit = int(std::min<long>(ksplit, std::max<long>(best, 1)));
   a->ksplit = ksplit;
@@ -174,7 +221,7 @@ void planWu(const plb_conv_params &p, const WuShape &s, int sm_count, int force_
     plan->grid = units * ksplit;
     plan->b_mn_major = 1;
     plan->halo_rows = a->strip_mode ? halo : 0;
-    plan->workspace_bytes = size_t(ksplit) * taps * co * ci * sizeof(float);
+    plan->workspace_bytes = size_t(ksplit) * p.sgroups * taps * co * ci * sizeof(float);
   }
 }
 
@@ -215,131 +262,166 @@ int configureWuKernel(int device) {
   return PLB_OK;
 }
 
-// Reduction over the K splits of group g (and, with `peer`, over the ranks).
-int launchWuReduce(cudaStream_t stream, const WuArgs &a, size_t w_elems, unsigned g,
-                   void *d_weight_grads, float *d_weight_grads_f32, const WuPeerArgs *peer) {
-  const size_t es = 2;
+cudaLaunchConfig_t wuReduceConfig(cudaStream_t stream, size_t blocks, cudaLaunchAttribute *pdl) {
+  pdl->id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  pdl->val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(unsigned(blocks));
+  cfg.blockDim = dim3(32, kWuReduceLanes);
+  cfg.stream = stream;
+  cfg.attrs = pdl;
+  cfg.numAttrs = 1;
+  return cfg;
+}
+
+// Reduction over the K splits (and, with `peer`, over the ranks) into one
+// gradient of w_elems.  The partial sums are in the gradient's order unless
+// `gather` says otherwise.
+int launchWuReduce(cudaStream_t stream, const WuArgs &a, size_t w_elems, void *d_weight_grads,
+                   float *d_weight_grads_f32, const WuGather *gather, const WuPeerArgs *peer = nullptr,
+                   unsigned group = 0) {
   cudaLaunchAttribute pdl[1];
-  pdl[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  pdl[0].val.programmaticStreamSerializationAllowed = 1;
-  float *out32 = d_weight_grads_f32 ? d_weight_grads_f32 + size_t(g) * w_elems : nullptr;
-  uint8_t *out16 =
-      d_weight_grads ? static_cast<uint8_t *>(d_weight_grads) + size_t(g) * w_elems * es : nullptr;
+  __half *out16 = static_cast<__half *>(d_weight_grads);
+  const bool vec = w_elems % 4 == 0 && (reinterpret_cast<uintptr_t>(d_weight_grads_f32) & 15) == 0 &&
+                   (reinterpret_cast<uintptr_t>(out16) & 7) == 0;
+  const size_t count4 = w_elems / 4;
   if (peer != nullptr) {
-    const size_t count4 = w_elems / 4;
     const unsigned rgrid = unsigned((count4 + kWuFusedChunk - 1) / kWuFusedChunk);
     WuPeerArgs pa = *peer;
     for (int r = 0; r < pa.world; ++r) {
-      pa.grads[r] += size_t(g) * count4;
-      if (pa.results[r] != nullptr) pa.results[r] += size_t(g) * count4;
+      pa.grads[r] += size_t(group) * count4;
+      if (pa.results[r] != nullptr) pa.results[r] += size_t(group) * count4;
     }
-    pa.chunk_base = g * rgrid;
-    cudaLaunchConfig_t rcfg{};
-    rcfg.gridDim = dim3(rgrid);
-    rcfg.blockDim = dim3(32, kWuReduceLanes);
-    rcfg.stream = stream;
-    rcfg.attrs = pdl;
-    rcfg.numAttrs = 1;
-    PLB_CUDA(cudaLaunchKernelEx(&rcfg, wu_reduce_allreduce_kernel,
-                                reinterpret_cast<const float4 *>(a.partial), a.ksplit, count4, pa,
-                                reinterpret_cast<float4 *>(out32), reinterpret_cast<uint2 *>(out16)));
-  } else if (w_elems % 4 == 0 && (reinterpret_cast<uintptr_t>(out32) & 15) == 0 &&
-             (reinterpret_cast<uintptr_t>(out16) & 7) == 0) {
-    const size_t count4 = w_elems / 4;
-    const unsigned rgrid = unsigned((count4 + 31) / 32);
-    cudaLaunchConfig_t rcfg{};
-    rcfg.gridDim = dim3(rgrid);
-    rcfg.blockDim = dim3(32, kWuReduceLanes);
-    rcfg.stream = stream;
-    rcfg.attrs = pdl;
-    rcfg.numAttrs = 1;
-    PLB_CUDA(cudaLaunchKernelEx(&rcfg, wu_reduce4_kernel,
-                                reinterpret_cast<const float4 *>(a.partial), a.ksplit, count4,
-                                reinterpret_cast<float4 *>(out32), reinterpret_cast<uint2 *>(out16)));
+    pa.chunk_base = group * rgrid;
+    const cudaLaunchConfig_t cfg = wuReduceConfig(stream, rgrid, pdl);
+    PLB_CUDA(cudaLaunchKernelEx(&cfg, wu_reduce_allreduce_kernel, reinterpret_cast<const float4 *>(a.partial),
+                                a.ksplit, count4, pa, reinterpret_cast<float4 *>(d_weight_grads_f32),
+                                reinterpret_cast<uint2 *>(out16)));
+  } else if (gather == nullptr && vec) {
+    const cudaLaunchConfig_t cfg = wuReduceConfig(stream, (count4 + 31) / 32, pdl);
+    PLB_CUDA(cudaLaunchKernelEx(&cfg, wu_reduce4_kernel, reinterpret_cast<const float4 *>(a.partial), a.ksplit,
+                                count4, reinterpret_cast<float4 *>(d_weight_grads_f32),
+                                reinterpret_cast<uint2 *>(out16)));
   } else {
-    const int rgrid = int(std::min<size_t>((w_elems + 255) / 256, size_t(148) * 8));
-    wu_reduce_kernel<<<rgrid, 256, 0, stream>>>(a.partial, a.ksplit, w_elems, out32, out16, 0);
+    WuGather g{};
+    if (gather) {
+      g = *gather;
+    } else {
+      g.taps = g.p_taps = uint32_t(a.taps_h * a.taps_w);
+      g.co = g.co_pitch = g.p_co = uint32_t(a.co_total);
+      g.ci = g.ci_pitch = g.p_ci = uint32_t(a.ci_total);
+      g.sub = 1;
+    }
+    g.split_stride = (unsigned long long)a.sgroups * a.taps_h * a.taps_w * a.co_total * a.ci_total;
+    g.total = w_elems;
+    // four channels at once where they are neighbours on both sides
+    if (vec && g.mode == kWuGroups && g.ci % 4 == 0 && g.ci_pitch % 4 == 0) {
+      const cudaLaunchConfig_t cfg = wuReduceConfig(stream, (count4 + 31) / 32, pdl);
+      PLB_CUDA(cudaLaunchKernelEx(&cfg, wu_gather_kernel<4>, (const float *)a.partial, a.ksplit, g,
+                                  d_weight_grads_f32, out16));
+    } else {
+      const cudaLaunchConfig_t cfg = wuReduceConfig(stream, (w_elems + 31) / 32, pdl);
+      PLB_CUDA(cudaLaunchKernelEx(&cfg, wu_gather_kernel<1>, (const float *)a.partial, a.ksplit, g,
+                                  d_weight_grads_f32, out16));
+    }
   }
   PLB_CUDA(cudaGetLastError());
   return PLB_OK;
 }
 
-// Launches the weight-gradient kernel and the reduction over K splits for every
-// group.  `a.partial` and `a.status` are set by the caller.
-// With `peer` the reduction also adds the gradients of the other ranks
-// (wu_reduce_allreduce_kernel); the caller has checked that the shapes allow it.
-int launchWu(cudaStream_t stream, const plb_conv_params &p, const WuShape &s, const WuArgs &a,
-             const void *d_acts, const void *d_out_grads, void *d_weight_grads,
-             float *d_weight_grads_f32, uint64_t *launches, const WuPeerArgs *peer = nullptr) {
-  const int co = int(p.out_chans_per_group), ci = int(p.in_chans_per_group);
+// Launches the weight-gradient kernel.  `a.partial` and `a.status` are set by the caller.
+int launchWuKernel(cudaStream_t stream, const WuProblem &p, const WuArgs &a) {
+  const WuShape &s = p.s;
   const int taps = s.KH * s.KW;
-  const size_t w_elems = size_t(taps) * co * ci;
-  const size_t es = 2;
-  const uint64_t ctot = uint64_t(p.groups) * ci, cotot = uint64_t(p.groups) * co;
   const int smem = a.stages * a.stage_bytes + 256 + 1024;
   const uint32_t ones[4] = {1, 1, 1, 1};
-  CUtensorMap tout;
+  CUtensorMap tout, tdy, tx;
   {
-    // partial sums [ksplit][taps][co][ci] fp32, stored in blocks of 32 x 32
-    const uint64_t dims[4] = {uint64_t(ci), uint64_t(co), uint64_t(taps), uint64_t(a.ksplit)};
-    const uint64_t strides[3] = {uint64_t(ci) * 4, uint64_t(co) * ci * 4, uint64_t(w_elems) * 4};
+    // partial sums [ksplit][sgroups * taps][co][ci] fp32, stored in blocks of 32 x 32
+    const uint64_t w_elems = uint64_t(p.sgroups) * taps * p.co * p.ci;
+    const uint64_t dims[4] = {uint64_t(p.ci), uint64_t(p.co), uint64_t(p.sgroups) * taps, uint64_t(a.ksplit)};
+    const uint64_t strides[3] = {uint64_t(p.ci) * 4, uint64_t(p.co) * p.ci * 4, w_elems * 4};
     const uint32_t box[4] = {32, 32, 1, 1};
-    if (int rc = encodeTensorMap(&tout, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, a.partial, dims,
-                                 strides, box, ones))
+    if (int rc = encodeTensorMap(&tout, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, a.partial, dims, strides, box, ones))
       return rc;
   }
+  // pixel dimensions (w, h, n); strip mode orders them (w, n, h)
+  const bool strip = a.strip_mode != 0;
+  const int halo = strip ? (s.KH - 1) * s.dilH : 0;
+  const uint64_t batch = uint64_t(p.batch);
+  {
+    const uint64_t dims[4] = {p.dy_chans, uint64_t(s.OWc), strip ? batch : uint64_t(s.OHc),
+                              strip ? uint64_t(s.OHc) : batch};
+    const uint64_t strides[3] = {p.dy_strides[0], p.dy_strides[strip ? 2 : 1], p.dy_strides[strip ? 1 : 2]};
+    const uint32_t box[4] = {64, uint32_t(a.box_w), uint32_t(strip ? a.box_n : a.box_h),
+                             uint32_t(strip ? a.box_h : a.box_n)};
+    if (int rc = encodeTensorMap(&tdy, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4,
+                                 static_cast<const uint8_t *>(p.dy) + uint64_t(s.opH) * p.dy_strides[1] +
+                                     uint64_t(s.opW) * p.dy_strides[0],
+                                 dims, strides, box, ones))
+      return rc;
+  }
+  {
+    const uint64_t dims[4] = {p.x_chans, uint64_t(s.We), strip ? batch : uint64_t(s.He),
+                              strip ? uint64_t(s.He) : batch};
+    const uint64_t strides[3] = {p.x_strides[0], p.x_strides[strip ? 2 : 1], p.x_strides[strip ? 1 : 2]};
+    const uint32_t bw = uint32_t((a.box_w - 1) * s.strW + 1);
+    const uint32_t bh = strip ? uint32_t(a.box_h + halo) : uint32_t((a.box_h - 1) * s.strH + 1);
+    const uint32_t box[4] = {64, bw, strip ? uint32_t(a.box_n) : bh, strip ? bh : uint32_t(a.box_n)};
+    const uint32_t estr[4] = {1, uint32_t(s.strW), strip ? 1u : uint32_t(s.strH), 1};
+    if (int rc = encodeTensorMap(&tx, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4,
+                                 static_cast<const uint8_t *>(p.x) + uint64_t(s.tH) * p.x_strides[1] +
+                                     uint64_t(s.tW) * p.x_strides[0],
+                                 dims, strides, box, estr))
+      return rc;
+  }
+  const int grid = a.sgroups * a.co_blocks * a.ci_blocks * a.tap_groups * a.ksplit;
+  // programmatic stream serialization: the kernel's set-up overlaps the tail of
+  // whatever runs before it; it waits before touching global memory
+  cudaLaunchAttribute pdl[1];
+  pdl[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  pdl[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(unsigned(grid));
+  cfg.blockDim = dim3(kWuThreads);
+  cfg.dynamicSmemBytes = size_t(smem);
+  cfg.stream = stream;
+  cfg.attrs = pdl;
+  cfg.numAttrs = 1;
+  PLB_CUDA(cudaLaunchKernelEx(&cfg, wu_kernel, tdy, tx, tout, a));
+  PLB_CUDA(cudaGetLastError());
+  return PLB_OK;
+}
+
+// The groups of a layer one after the other, through one group's worth of scratch
+// (the entry points that cannot hold more).  With `peer` the reduction also adds
+// the gradients of the other ranks; the caller has checked that the shapes allow it.
+int launchWuPerGroup(cudaStream_t stream, const plb_conv_params &p, const WuShape &s, const WuArgs &a,
+                     const void *d_acts, const void *d_out_grads, void *d_weight_grads,
+                     float *d_weight_grads_f32, uint64_t *launches, const WuPeerArgs *peer = nullptr) {
+  const uint32_t co = p.out_chans_per_group, ci = p.in_chans_per_group;
+  const size_t w_elems = size_t(s.KH) * s.KW * co * ci, es = 2;
   for (unsigned g = 0; g < p.groups; ++g) {
-    CUtensorMap tdy, tx;
-    // pixel dimensions (w, h, n); strip mode orders them (w, n, h)
-    const bool strip = a.strip_mode != 0;
-    const int halo = strip ? (s.KH - 1) * s.dilH : 0;
-    {
-      const uint64_t sh = uint64_t(s.OW) * cotot * es, sn = uint64_t(s.OH) * s.OW * cotot * es;
-      const uint64_t dims[4] = {uint64_t(co), uint64_t(s.OWc), strip ? p.batch : uint64_t(s.OHc),
-                                strip ? uint64_t(s.OHc) : p.batch};
-      const uint64_t strides[3] = {cotot * es, strip ? sn : sh, strip ? sh : sn};
-      const uint32_t box[4] = {64, uint32_t(a.box_w), uint32_t(strip ? a.box_n : a.box_h),
-                               uint32_t(strip ? a.box_h : a.box_n)};
-      if (int rc = encodeTensorMap(&tdy, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4,
-                                   static_cast<const uint8_t *>(d_out_grads) +
-                                       ((size_t(s.opH) * s.OW + s.opW) * cotot + size_t(g) * co) * es,
-                                   dims, strides, box, ones))
-        return rc;
-    }
-    {
-      const uint64_t sh = uint64_t(s.W) * ctot * es, sn = uint64_t(s.H) * s.W * ctot * es;
-      const uint64_t dims[4] = {uint64_t(ci), uint64_t(s.We), strip ? p.batch : uint64_t(s.He),
-                                strip ? uint64_t(s.He) : p.batch};
-      const uint64_t strides[3] = {ctot * es, strip ? sn : sh, strip ? sh : sn};
-      const uint32_t bw = uint32_t((a.box_w - 1) * s.strW + 1);
-      const uint32_t bh = strip ? uint32_t(a.box_h + halo) : uint32_t((a.box_h - 1) * s.strH + 1);
-      const uint32_t box[4] = {64, bw, strip ? uint32_t(a.box_n) : bh, strip ? bh : uint32_t(a.box_n)};
-      const uint32_t estr[4] = {1, uint32_t(s.strW), strip ? 1u : uint32_t(s.strH), 1};
-      if (int rc = encodeTensorMap(&tx, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4,
-                                   static_cast<const uint8_t *>(d_acts) +
-                                       ((size_t(s.tH) * s.W + s.tW) * ctot + size_t(g) * ci) * es,
-                                   dims, strides, box, estr))
-        return rc;
-    }
-    const int grid = a.co_blocks * a.ci_blocks * a.tap_groups * a.ksplit;
-    // programmatic stream serialization: the kernels' set-up overlaps the tail
-    // of whatever runs before them; they wait before touching global memory
-    cudaLaunchAttribute pdl[1];
-    pdl[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    pdl[0].val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(unsigned(grid));
-    cfg.blockDim = dim3(kWuThreads);
-    cfg.dynamicSmemBytes = size_t(smem);
-    cfg.stream = stream;
-    cfg.attrs = pdl;
-    cfg.numAttrs = 1;
-    PLB_CUDA(cudaLaunchKernelEx(&cfg, wu_kernel, tdy, tx, tout, a));
-    if (int rc = launchWuReduce(stream, a, w_elems, g, d_weight_grads, d_weight_grads_f32, peer))
+    WuProblem q = wuProblem(p, s, ci, co, 1, 1);
+    q.x = static_cast<const uint8_t *>(d_acts) + size_t(g) * ci * es;
+    q.dy = static_cast<const uint8_t *>(d_out_grads) + size_t(g) * co * es;
+    if (int rc = launchWuKernel(stream, q, a)) return rc;
+    if (int rc = launchWuReduce(
+            stream, a, w_elems, d_weight_grads ? static_cast<uint8_t *>(d_weight_grads) + g * w_elems * es : nullptr,
+            d_weight_grads_f32 ? d_weight_grads_f32 + g * w_elems : nullptr, nullptr, peer, g))
       return rc;
     if (launches) *launches += 2;
   }
   return PLB_OK;
+}
+
+// Channel groups contracted together: as many as fill the 128 output-channel rows
+// of the tensor-core tile without exceeding 128 input channels.  32 groups of 8
+// channels run as two dense blocks of 128 x 128 instead of 32 launches whose
+// tiles are 15/16 padding.
+uint32_t wuGroupsTogether(uint32_t groups, uint32_t ci_pitch, uint32_t co_pitch) {
+  return std::max<uint32_t>(1, std::min(groups, std::min(128 / std::max<uint32_t>(co_pitch, 1),
+                                                         128 / std::max<uint32_t>(ci_pitch, 1))));
 }
 
 }  // namespace
@@ -384,7 +466,9 @@ int plb_conv_wu_plan(const plb_conv_params *p_in, const plb_conv_options *opt, p
   if (int rc = wuShape(*p, &s)) return rc;
   *plan = plb_plan{};
   WuArgs a{};
-  planWu(*p, s, 148, opt ? opt->split_k : 0, opt ? opt->plan_flags : 0, &a, plan);
+  const uint32_t cip = roundToVec(p->in_chans_per_group, 2), cop = roundToVec(p->out_chans_per_group, 2);
+  planWu(wuProblem(*p, s, cip, cop, p->groups, wuGroupsTogether(p->groups, cip, cop)), 148, opt ? opt->split_k : 0,
+         opt ? opt->plan_flags : 0, &a, plan);
   plan->flops = 2 * numberOfMacs(*p);
   const uint64_t es = dtypeBytes(p->input_type);
   plan->bytes = es * (uint64_t(p->batch) * s.H * s.W * p->groups * p->in_chans_per_group +
@@ -408,10 +492,15 @@ int plb_conv_wu(plb_context *ctx, const plb_conv_params *p, const plb_conv_optio
     if (int rc = checkConvRequest(*p, true, d_acts, n_w ? n_in : 0, d_out_grads, n_w ? n_out : 0, result, n_w))
       return rc;
   }
-  if (p->input_type == PLB_FLOAT) {
-    const std::string err = validate(*p);
-    if (!err.empty()) return fail(PLB_ERR_INVALID_PARAMS, err);
-    return floatConvWu(ctx, *p, opt, d_acts, d_out_grads, d_weight_grads, d_weight_grads_f32);
+  if (p->input_type == PLB_FLOAT && d_weight_grads) {
+    // a float layer's weight gradient is float either way
+    float *result = d_weight_grads_f32 ? d_weight_grads_f32 : static_cast<float *>(d_weight_grads);
+    if (int rc = plb_conv_wu(ctx, p, opt, d_acts, d_out_grads, nullptr, result)) return rc;
+    size_t n_in, n_w, n_out;
+    convElementCounts(*p, &n_in, &n_w, &n_out);
+    if (n_w && d_weight_grads != static_cast<void *>(result))
+      PLB_CUDA(cudaMemcpyAsync(d_weight_grads, result, n_w * sizeof(float), cudaMemcpyDeviceToDevice, ctx->stream));
+    return PLB_OK;
   }
   if (p->input_type == PLB_BFLOAT16 && d_weight_grads)
     return fail(PLB_ERR_UNSUPPORTED, "a bfloat16 layer's weight gradient is returned as fp32 only");
@@ -519,57 +608,104 @@ int plb_conv_wu(plb_context *ctx, const plb_conv_params *p, const plb_conv_optio
     if (d_weight_grads_f32) PLB_CUDA(cudaMemsetAsync(d_weight_grads_f32, 0, n * sizeof(float), ctx->stream));
     return PLB_OK;
   }
-  if (ci % 8 != 0 || co % 8 != 0) {
-    // Channel counts TMA cannot address (a pixel must be a multiple of 16
-    // bytes): run on zero-padded copies and drop the padded rows / columns of
-    // the gradient.  Arena in scratch slot 7.
-    const size_t es2 = 2, G = p->groups;
-    const uint32_t cip = uint32_t((ci + 7) / 8 * 8), cop = uint32_t((co + 7) / 8 * 8);
-    const size_t in_px = size_t(p->batch) * s.H * s.W, out_px = size_t(p->batch) * s.OH * s.OW;
-    auto al = [](size_t n) { return (n + 255) & ~size_t(255); };
-    const size_t x_b = al(in_px * G * cip * es2), dy_b = al(out_px * G * cop * es2);
-    const size_t wp_elems = G * size_t(taps) * cop * cip;
-    const size_t w16_b = al(wp_elems * es2), w32_b = al(wp_elems * 4);
-    void *arena = nullptr;
-    if (int rc = scratch(ctx, kSlotPaddedChans, x_b + dy_b + 2 * w16_b + 2 * w32_b, &arena)) return rc;
-    uint8_t *xp = static_cast<uint8_t *>(arena), *dyp = xp + x_b, *w16 = dyp + dy_b, *t16 = w16 + w16_b,
-            *w32 = t16 + w16_b, *t32 = w32 + w32_b;
-    if (int rc = resizeRows(ctx, d_acts, xp, in_px * G, size_t(ci) * es2, cip * es2)) return rc;
-    if (int rc = resizeRows(ctx, d_out_grads, dyp, out_px * G, size_t(co) * es2, cop * es2)) return rc;
-    plb_conv_params q = *p;
-    q.in_chans_per_group = cip;
-    q.out_chans_per_group = cop;
-    if (int rc = plb_conv_wu(ctx, &q, opt, xp, dyp, d_weight_grads ? w16 : nullptr,
-                             d_weight_grads_f32 ? reinterpret_cast<float *>(w32) : nullptr))
-      return rc;
-    // [G][taps][cop][cip] -> drop rows, then columns
-    const size_t gt = G * size_t(taps);
-    if (d_weight_grads) {
-      if (int rc = resizeRows(ctx, w16, t16, gt, size_t(cop) * cip * es2, size_t(co) * cip * es2)) return rc;
-      if (int rc = resizeRows(ctx, t16, d_weight_grads, gt * co, cip * es2, size_t(ci) * es2)) return rc;
-    }
-    if (d_weight_grads_f32) {
-      if (int rc = resizeRows(ctx, w32, t32, gt, size_t(cop) * cip * 4, size_t(co) * cip * 4)) return rc;
-      if (int rc = resizeRows(ctx, t32, d_weight_grads_f32, gt * co, cip * 4, size_t(ci) * 4)) return rc;
-    }
-    return PLB_OK;
-  }
-  WuArgs a{};
-  planWu(*p, s, ctx->sm_count, opt ? opt->split_k : 0, (opt ? opt->plan_flags : 0) | ctx->plan_flags, &a,
-         nullptr);
-  a.status = ctx->d_status;
-  a.trace = ctx->trace;
-  void *ws = nullptr;
-  if (int rc = scratch(ctx, kSlotOperands, size_t(a.ksplit) * w_elems * sizeof(float), &ws)) return rc;
-  a.partial = static_cast<float *>(ws);
-
   if (int rc = configureWuKernel(ctx->device)) return rc;
-  uint64_t launches = 0;
-  if (int rc = launchWu(ctx->stream, *p, s, a, d_acts, d_out_grads, d_weight_grads,
-                        d_weight_grads_f32, &launches))
-    return rc;
-  ctx->launches += launches;
-  return PLB_OK;
+  const int force_split = opt ? opt->split_k : 0;
+  const unsigned plan_flags = unsigned((opt ? opt->plan_flags : 0) | ctx->plan_flags);
+  WuGather gather{};
+  gather.mode = kWuGroups;
+  gather.taps = gather.p_taps = uint32_t(taps);
+  gather.co = uint32_t(co);
+  gather.ci = uint32_t(ci);
+  auto run = [&](const WuProblem &q, const WuGather *g) -> int {
+    WuArgs a{};
+    planWu(q, ctx->sm_count, force_split, plan_flags, &a, nullptr);
+    a.status = ctx->d_status;
+    a.trace = ctx->trace;
+    void *ws = nullptr;
+    const size_t partial = size_t(a.ksplit) * q.sgroups * q.s.KH * q.s.KW * q.co * q.ci * sizeof(float);
+    if (int rc = scratch(ctx, kSlotWuPartials, partial, &ws)) return rc;
+    a.partial = static_cast<float *>(ws);
+    if (int rc = launchWuKernel(ctx->stream, q, a)) return rc;
+    ctx->launches += 2;
+    return launchWuReduce(ctx->stream, a, p->groups * w_elems, d_weight_grads, d_weight_grads_f32, g);
+  };
+  // Few input channels (an image network's first layer): the rearranged input of
+  // the forward pass, whose pixels hold a window of the filter's columns, so that
+  // the KW taps of a filter row are 64 channels of one tap.  (On channels padded to
+  // 8 the layer 7x7, stride 2, 3 -> 64 channels, 256 images of 224x224, took
+  // 49 taps of 5/8 padding and 5.5 ms.)
+  S2dShape g2{};
+  if (ci % 8 != 0 && co % 8 == 0 && p->input_type != PLB_FLOAT && smallChannelShape(*p, &g2) == PLB_OK) {
+    void *ws = nullptr;
+    if (int rc = scratch(ctx, kSlotOperands, smallChannelElems(g2) * 2 + 256, &ws)) return rc;
+    if (int rc = smallChannelPrepare(ctx, g2, d_acts, static_cast<__half *>(ws), nullptr, nullptr, co)) return rc;
+    WuShape s2 = s;
+    s2.H = s2.He = g2.H2;
+    s2.W = g2.W2;
+    s2.We = g2.OW;  // windows per row
+    s2.KH = g2.K2h;
+    s2.KW = 1;
+    s2.padH = s2.padW = 0;
+    s2.strH = s2.strW = 1;
+    WuProblem q = wuProblem(*p, s2, 64, uint32_t(co), 1, 1);
+    q.x = ws;
+    q.x_strides[0] = uint64_t(g2.C2) * 2;
+    q.x_strides[1] = uint64_t(g2.W2) * g2.C2 * 2;
+    q.x_strides[2] = uint64_t(g2.H2) * g2.W2 * g2.C2 * 2;
+    q.dy = d_out_grads;
+    gather.mode = kWuFolded;
+    gather.kw = uint32_t(s.KW);
+    gather.stride = uint32_t(g2.s);
+    gather.chan_pitch = uint32_t(g2.Cp);
+    gather.p_taps = uint32_t(g2.K2h);
+    gather.p_co = uint32_t(co);
+    gather.p_ci = 64;
+    return run(q, &gather);
+  }
+  // Channel counts TMA cannot address (a pixel must be a multiple of 16 bytes) run
+  // on copies with the channels rounded up; float operands as three batches of
+  // bfloat16 pieces side by side.  The padded rows and columns of the partial sums
+  // are not read.
+  const bool is_float = p->input_type == PLB_FLOAT;
+  const uint32_t G = p->groups, cip = roundToVec(uint64_t(ci), 2), cop = roundToVec(uint64_t(co), 2);
+  const uint64_t x_rows = uint64_t(p->batch) * s.H * s.W * G, dy_rows = uint64_t(p->batch) * s.OH * s.OW * G;
+  const void *x = d_acts, *dy = d_out_grads;
+  {
+    Repack jobs[2];
+    const void **operand[2];
+    int n = 0;
+    auto add = [&](const void **base, uint64_t rows, uint32_t cols, uint32_t pitch, bool second) {
+      if (!is_float && cols == pitch && (reinterpret_cast<uintptr_t>(*base) & 15) == 0) return;
+      jobs[n] = Repack{*base, nullptr, rows, cols, cols, pitch, is_float ? 4u : 2u,
+                       is_float ? kRepackSplitPlanes : kRepackCopy, second, 0};
+      operand[n++] = base;
+    };
+    add(&x, x_rows, uint32_t(ci), cip, false);
+    add(&dy, dy_rows, uint32_t(co), cop, true);
+    size_t bytes[2] = {0, 0};
+    for (int i = 0; i < n; ++i) bytes[i] = (repackBytes(jobs[i]) + 255) & ~size_t(255);
+    if (n) {
+      void *ws = nullptr;
+      if (int rc = scratch(ctx, kSlotRepacked, bytes[0] + bytes[1] + 256, &ws)) return rc;
+      for (int i = 0; i < n; ++i) *operand[i] = jobs[i].dst = static_cast<uint8_t *>(ws) + (i ? bytes[0] : 0);
+      if (int rc = repack(ctx, jobs, n)) return rc;
+    }
+  }
+  plb_conv_params q16 = *p;
+  if (is_float) {
+    q16.input_type = PLB_BFLOAT16;
+    q16.batch *= 3;
+  }
+  WuProblem q = wuProblem(q16, s, cip, cop, G, wuGroupsTogether(G, cip, cop));
+  q.x = x;
+  q.dy = dy;
+  gather.sub = uint32_t(q.sub);
+  gather.co_pitch = cop;
+  gather.ci_pitch = cip;
+  gather.p_co = uint32_t(q.co);
+  gather.p_ci = uint32_t(q.ci);
+  const bool same_order = q.sub == 1 && cip == uint32_t(ci) && cop == uint32_t(co);
+  return run(q, same_order ? nullptr : &gather);
 }
 
 // Chunks (= blocks of the fused reduction, = flags per sender) of one call.
@@ -645,25 +781,29 @@ static int wuAllreduce(plb_context *ctx, const plb_conv_params *p, const plb_con
   if (p->batch == 0 || s.OHc <= 0 || s.OWc <= 0 || s.He <= 0 || s.We <= 0) {
     // this rank has no share of the batch: it contributes zeros, through one
     // split of zero partial sums, so that the peers still get its flags
-    planWu(*p, s, ctx->sm_count, 1, opt ? opt->plan_flags : 0, &a, nullptr);
+    planWu(wuProblem(*p, s, uint32_t(ci), uint32_t(co), 1, 1), ctx->sm_count, 1, opt ? opt->plan_flags : 0, &a, nullptr);
     a.ksplit = 1;
     void *ws = nullptr;
-    if (int rc = scratch(ctx, kSlotOperands, w_elems * sizeof(float), &ws)) return rc;
+    if (int rc = scratch(ctx, kSlotWuPartials, w_elems * sizeof(float), &ws)) return rc;
     PLB_CUDA(cudaMemsetAsync(ws, 0, w_elems * sizeof(float), ctx->stream));
     a.partial = static_cast<float *>(ws);
     for (unsigned g = 0; g < p->groups; ++g) {
-      if (int rc = launchWuReduce(ctx->stream, a, w_elems, g, d_weight_grads, d_weight_grads_f32, &pa))
+      if (int rc = launchWuReduce(
+              ctx->stream, a, w_elems,
+              d_weight_grads ? static_cast<uint8_t *>(d_weight_grads) + g * w_elems * 2 : nullptr,
+              d_weight_grads_f32 ? d_weight_grads_f32 + g * w_elems : nullptr, nullptr, &pa, g))
         return rc;
       ++launches;
     }
     ctx->launches += launches;
     return PLB_OK;
   }
-  planWu(*p, s, ctx->sm_count, opt ? opt->split_k : 0, opt ? opt->plan_flags : 0, &a, nullptr);
+  planWu(wuProblem(*p, s, uint32_t(ci), uint32_t(co), 1, 1), ctx->sm_count, opt ? opt->split_k : 0,
+         opt ? opt->plan_flags : 0, &a, nullptr);
   void *ws = nullptr;
-  if (int rc = scratch(ctx, kSlotOperands, size_t(a.ksplit) * w_elems * sizeof(float), &ws)) return rc;
+  if (int rc = scratch(ctx, kSlotWuPartials, size_t(a.ksplit) * w_elems * sizeof(float), &ws)) return rc;
   a.partial = static_cast<float *>(ws);
-  if (int rc = launchWu(ctx->stream, *p, s, a, d_acts, d_out_grads, d_weight_grads, d_weight_grads_f32,
+  if (int rc = launchWuPerGroup(ctx->stream, *p, s, a, d_acts, d_out_grads, d_weight_grads, d_weight_grads_f32,
                         &launches, &pa))
     return rc;
   ctx->launches += launches;
@@ -789,7 +929,8 @@ extern "C" int plb_conv_wu_static_scratch(int device, void *cuda_stream, const p
     return PLB_OK;
   }
   WuArgs a{};
-  planWu(*p, s, scratch.sm_count, opt ? opt->split_k : 0, opt ? opt->plan_flags : 0, &a, nullptr);
+  planWu(wuProblem(*p, s, uint32_t(ci), uint32_t(co), 1, 1), scratch.sm_count, opt ? opt->split_k : 0,
+         opt ? opt->plan_flags : 0, &a, nullptr);
   // as many K splits as the fixed scratch can hold
   const int max_split = int(kStaticScratchBytes / (w_elems * sizeof(float)));
   a.ksplit = std::max(1, std::min(a.ksplit, max_split));
@@ -799,7 +940,7 @@ extern "C" int plb_conv_wu_static_scratch(int device, void *cuda_stream, const p
   // at zero; the partial sums need no clearing, every CTA overwrites its slice
   PLB_CUDA(cudaMemsetAsync(scratch.status, 0, sizeof(int), stream));
 
-  if (int rc = launchWu(stream, *p, s, a, d_acts, d_out_grads, d_weight_grads, d_weight_grads_f32,
+  if (int rc = launchWuPerGroup(stream, *p, s, a, d_acts, d_out_grads, d_weight_grads, d_weight_grads_f32,
                         nullptr))
     return rc;
   // report a kernel that gave up on a bounded wait; this also makes the call
