@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "conv_geometry.h"
+#include "grouped.h"
 #include "runtime.h"
 #include "sm100_prims.cuh"
 
@@ -539,8 +540,11 @@ int zeroPhases(plb_context *ctx, void *dx, const plb_conv_params &p, const ConvS
 // fixed, evenly spaced subset of the filter taps (a sub-lattice of the stored
 // filter), so each phase is a stride-1 convolution of the output gradients with
 // that sub-filter, written to the strided sub-lattice of the input gradient.
-int convBwdStrided(plb_context *ctx, const plb_conv_params &p, const plb_conv_options *opt,
-                   const ConvShape &s, const PassOperands &o, void *dx, bool weights_transposed) {
+// `separate`: `p` contracts groups together; each phase's outputs are repaired from
+// these operands of the separate groups (`separate_p`).
+int convBwdStrided(plb_context *ctx, const plb_conv_params &p, const plb_conv_options *opt, const ConvShape &s,
+                   const PassOperands &o, void *dx, bool weights_transposed, const plb_conv_params *separate_p,
+                   const PassOperands *separate) {
   const size_t os = dtypeBytes(p.output_type);
   const uint64_t ci = p.in_chans_per_group, ctot = uint64_t(p.groups) * ci;
   // phases and their taps
@@ -569,36 +573,61 @@ int convBwdStrided(plb_context *ctx, const plb_conv_params &p, const plb_conv_op
     for (int b = 0; b < s.strW; ++b) {
       const BwdPhase &A = ph[size_t(a)], &B = pw[size_t(b)];
       if (A.extent == 0 || B.extent == 0 || A.taps == 0 || B.taps == 0) continue;
-      IgemmProblem r = convBwdProblem(p, opt, s, o, dx, weights_transposed);
-      r.out_w = B.extent;
-      r.out_h = A.extent;
-      r.taps_h = A.taps;
-      r.taps_w = B.taps;
-      // tap j of the phase is used tap first + j*step of the (possibly flipped)
-      // filter, stored where the flip, the truncation and (weights_transposed)
-      // the reversal of all stored taps put it
-      auto stored = [&](int used, int K, int Ks, int kt, int flip) {
-        const int at = kt + (flip ? K - 1 - used : used);
-        return weights_transposed ? Ks - 1 - at : at;
+      auto phase = [&](const plb_conv_params &pp, const PassOperands &oo, bool weights_transposed) {
+        IgemmProblem r = convBwdProblem(pp, opt, s, oo, dx, weights_transposed);
+        r.out_w = B.extent;
+        r.out_h = A.extent;
+        r.taps_h = A.taps;
+        r.taps_w = B.taps;
+        // tap j of the phase is used tap first + j*step of the (possibly flipped)
+        // filter, stored where the flip, the truncation and (weights_transposed)
+        // the reversal of all stored taps put it
+        auto stored = [&](int used, int K, int Ks, int kt, int flip) {
+          const int at = kt + (flip ? K - 1 - used : used);
+          return weights_transposed ? Ks - 1 - at : at;
+        };
+        const int h0 = stored(A.first_tap, s.KH, s.KHs, s.ktH, s.flipH);
+        const int w0 = stored(B.first_tap, s.KW, s.KWs, s.ktW, s.flipW);
+        setTaps(&r, s, h0, (s.flipH != 0) != weights_transposed ? -A.step : A.step, w0,
+                (s.flipW != 0) != weights_transposed ? -B.step : B.step);
+        // position i of the phase reads output index i + offset - j*dil for its
+        // j-th tap: a correlation with the taps reversed
+        r.dil_h = A.dil;
+        r.dil_w = B.dil;
+        r.pad_h = (A.taps - 1) * A.dil - A.offset;
+        r.pad_w = (B.taps - 1) * B.dil - B.offset;
+        r.flip_h = 1;
+        r.flip_w = 1;
+        r.out = static_cast<uint8_t *>(dx) + (size_t(s.tH + a) * s.W + (s.tW + b)) * ctot * os;
+        r.ldc = (long long)(ctot * s.strW);
+        r.out_stride_h = (long long)(ctot * s.W * s.strH);
+        return r;
       };
-      const int h0 = stored(A.first_tap, s.KH, s.KHs, s.ktH, s.flipH);
-      const int w0 = stored(B.first_tap, s.KW, s.KWs, s.ktW, s.flipW);
-      setTaps(&r, s, h0, (s.flipH != 0) != weights_transposed ? -A.step : A.step, w0,
-              (s.flipW != 0) != weights_transposed ? -B.step : B.step);
-      // position i of the phase reads output index i + offset - j*dil for its
-      // j-th tap: a correlation with the taps reversed
-      r.dil_h = A.dil;
-      r.dil_w = B.dil;
-      r.pad_h = (A.taps - 1) * A.dil - A.offset;
-      r.pad_w = (B.taps - 1) * B.dil - B.offset;
-      r.flip_h = 1;
-      r.flip_w = 1;
-      r.out = static_cast<uint8_t *>(dx) + (size_t(s.tH + a) * s.W + (s.tW + b)) * ctot * os;
-      r.ldc = (long long)(ctot * s.strW);
-      r.out_stride_h = (long long)(ctot * s.W * s.strH);
+      IgemmProblem r = phase(p, o, weights_transposed);
+      if (separate) r.nonfinite = nonfiniteFlag(ctx);
       if (int rc = runProblem(ctx, r)) return rc;
+      if (separate)
+        if (int rc = repairNonFinite(ctx, phase(*separate_p, *separate, false), separate->type)) return rc;
     }
   return PLB_OK;
+}
+
+// Narrow channel groups are contracted together (grouped.cu): `q` = the layer of
+// wider groups and its weights, [G][taps][rows][cols] made block-diagonal.
+// Returns whether it applies through `together`.
+int gatherGroups(plb_context *ctx, const plb_conv_params &p, const ConvShape &s, const void *weights, bool rows_are_co,
+                 plb_conv_params *q, const void **out, bool *together) {
+  *q = p;
+  *out = weights;
+  const uint32_t ci = p.in_chans_per_group, co = p.out_chans_per_group;
+  const uint32_t S = groupsTogether(p.groups, ci, co, p.input_type);
+  *together = S > 1;
+  if (S == 1) return PLB_OK;
+  q->groups = p.groups / S;
+  q->in_chans_per_group = S * ci;
+  q->out_chans_per_group = S * co;
+  return blockDiagonalWeights(ctx, p.input_type, weights, p.groups, S, uint32_t(s.KHs * s.KWs), rows_are_co ? co : ci,
+                              rows_are_co ? ci : co, out);
 }
 
 }  // namespace
@@ -826,13 +855,18 @@ int plb_conv_plan(const plb_conv_params *p_in, const plb_conv_options *opt, int3
     }
     if (rc != PLB_ERR_UNSUPPORTED) return rc;
   }
-  IgemmProblem q;
+  // narrow groups run together, channel counts TMA cannot address rounded up
+  plb_conv_params run = *p;
+  const uint32_t together = groupsTogether(p->groups, p->in_chans_per_group, p->out_chans_per_group, p->input_type);
+  run.groups /= together;
+  run.in_chans_per_group *= together;
+  run.out_chans_per_group *= together;
   const bool bwd = pass == PLB_PASS_TRAINING_BWD;
-  PassOperands o{p->input_type, nullptr, nullptr, bwd ? p->out_chans_per_group : p->in_chans_per_group, 0, 0};
-  o.act_pitch = roundToVec(o.k, dtypeBytes(p->input_type));
-  o.w_pitch = roundToVec(p->in_chans_per_group, dtypeBytes(p->input_type));
-  q = bwd ? convBwdProblem(*p, opt, s, o, nullptr, p->input_type == PLB_QUARTER)
-          : convFwdProblem(*p, opt, s, o, nullptr, nullptr);
+  PassOperands o{run.input_type, nullptr, nullptr, bwd ? run.out_chans_per_group : run.in_chans_per_group, 0, 0};
+  o.act_pitch = roundToVec(o.k, dtypeBytes(run.input_type));
+  o.w_pitch = roundToVec(run.in_chans_per_group, dtypeBytes(run.input_type));
+  const IgemmProblem q = bwd ? convBwdProblem(run, opt, s, o, nullptr, run.input_type == PLB_QUARTER)
+                             : convFwdProblem(run, opt, s, o, nullptr, nullptr);
   if (q.n_total > 0 && q.out_w > 0 && q.out_h > 0 && q.out_n > 0 && q.k_per_tap > 0)
     if (int rc = planIgemm(q, 148, plan)) return rc;
   plan->flops = 2 * numberOfMacs(*p);
@@ -928,28 +962,33 @@ int plb_convolution(plb_context *ctx, const plb_conv_params *p, const plb_conv_o
                              ctx->stream));
     return PLB_OK;
   }
-  const uint64_t in_rows = uint64_t(p->batch) * s.H * s.W * p->groups, taps = uint64_t(s.KHs) * s.KWs;
-  const uint32_t ci = p->in_chans_per_group, co = p->out_chans_per_group;
+  const bool swapped = transpose_and_flip_weights != 0;
+  plb_conv_params q;
+  const void *w = nullptr;
+  bool together = false;
+  // stored [G][k][Ci][Co] when swapped, else [G][k][Co][Ci]
+  if (int rc = gatherGroups(ctx, *p, s, d_weights, !swapped, &q, &w, &together)) return rc;
+  const uint64_t in_rows = uint64_t(q.batch) * s.H * s.W * q.groups, tiles = uint64_t(q.groups) * s.KHs * s.KWs;
+  const uint32_t ci = q.in_chans_per_group, co = q.out_chans_per_group;
+  const bool transposed = swapped && q.input_type == PLB_QUARTER;  // -> [G][flipped k][Co][Ci]
   PassOperands o;
-  bool swapped = transpose_and_flip_weights != 0, flipped_taps = false;
-  if (swapped && p->input_type == PLB_QUARTER) {
-    const void *wt = nullptr;
+  if (transposed) {
     uint32_t pitch = 0;
-    // stored [G][k][Ci][Co] -> [G][flipped k][Co][Ci]
-    if (int rc = transposedWeights(ctx, d_weights, p->groups, taps, ci, co, &wt, &pitch)) return rc;
-    if (int rc = prepareOperands(ctx, p->input_type, d_in, in_rows, ci, wt, p->groups * taps * co, pitch, 0, &o)) return rc;
-    swapped = false;
-    flipped_taps = true;
+    if (int rc = transposedWeights(ctx, w, q.groups, uint64_t(s.KHs) * s.KWs, ci, co, &w, &pitch)) return rc;
+    if (int rc = prepareOperands(ctx, q.input_type, d_in, in_rows, ci, w, tiles * co, pitch, 0, &o)) return rc;
   } else if (swapped) {
-    // stored [G][k][Ci][Co], the reduction along the rows
-    if (int rc = prepareOperands(ctx, p->input_type, d_in, in_rows, ci, d_weights, p->groups * taps * ci, co, ci, &o))
-      return rc;
+    // the reduction along the rows
+    if (int rc = prepareOperands(ctx, q.input_type, d_in, in_rows, ci, w, tiles * ci, co, ci, &o)) return rc;
   } else {
-    if (int rc = prepareOperands(ctx, p->input_type, d_in, in_rows, ci, d_weights, p->groups * taps * co, ci, 0, &o))
-      return rc;
+    if (int rc = prepareOperands(ctx, q.input_type, d_in, in_rows, ci, w, tiles * co, ci, 0, &o)) return rc;
   }
-  IgemmProblem q = convFwdProblem(*p, opt, s, o, d_bias, d_out, swapped, flipped_taps);
-  return runProblem(ctx, q);
+  IgemmProblem r = convFwdProblem(q, opt, s, o, d_bias, d_out, swapped && !transposed, transposed);
+  if (together) r.nonfinite = nonfiniteFlag(ctx);
+  if (int rc = runProblem(ctx, r)) return rc;
+  if (!together) return PLB_OK;
+  const PassOperands separate{p->input_type, d_in, d_weights, p->in_chans_per_group, p->in_chans_per_group,
+                              swapped ? p->out_chans_per_group : p->in_chans_per_group};
+  return repairNonFinite(ctx, convFwdProblem(*p, opt, s, separate, d_bias, d_out, swapped), p->input_type);
 }
 
 int plb_conv_fwd(plb_context *ctx, const plb_conv_params *p, const plb_conv_options *opt,
@@ -1027,25 +1066,32 @@ int plb_conv_bwd(plb_context *ctx, const plb_conv_params *p, const plb_conv_opti
                                ctx->stream));
     return PLB_OK;
   }
-  const uint64_t out_rows = uint64_t(p->batch) * s.OH * s.OW * p->groups, taps = uint64_t(s.KHs) * s.KWs;
-  const uint32_t ci = p->in_chans_per_group, co = p->out_chans_per_group;
+  plb_conv_params q;
+  const void *w = nullptr;
+  bool together = false;
+  if (int rc = gatherGroups(ctx, *p, s, d_weights, true, &q, &w, &together)) return rc;
+  const uint64_t out_rows = uint64_t(q.batch) * s.OH * s.OW * q.groups, tiles = uint64_t(q.groups) * s.KHs * s.KWs;
+  const uint32_t ci = q.in_chans_per_group, co = q.out_chans_per_group;
   PassOperands o;
-  const bool transposed = p->input_type == PLB_QUARTER;
+  const bool transposed = q.input_type == PLB_QUARTER;
   if (transposed) {
-    const void *wt = nullptr;
     uint32_t pitch = 0;
     // [G][k][Co][Ci] -> [G][flipped k][Ci][Co]
-    if (int rc = transposedWeights(ctx, d_weights, p->groups, taps, co, ci, &wt, &pitch)) return rc;
-    if (int rc = prepareOperands(ctx, p->input_type, d_out_grads, out_rows, co, wt, p->groups * taps * ci, pitch, 0, &o))
-      return rc;
+    if (int rc = transposedWeights(ctx, w, q.groups, uint64_t(s.KHs) * s.KWs, co, ci, &w, &pitch)) return rc;
+    if (int rc = prepareOperands(ctx, q.input_type, d_out_grads, out_rows, co, w, tiles * ci, pitch, 0, &o)) return rc;
   } else {
     // the reduction runs over the output channels, the rows of a weight tile
-    if (int rc = prepareOperands(ctx, p->input_type, d_out_grads, out_rows, co, d_weights, p->groups * taps * co, ci, co, &o))
-      return rc;
+    if (int rc = prepareOperands(ctx, q.input_type, d_out_grads, out_rows, co, w, tiles * co, ci, co, &o)) return rc;
   }
-  if (s.strH != 1 || s.strW != 1) return convBwdStrided(ctx, *p, opt, s, o, d_in_grads, transposed);
-  IgemmProblem q = convBwdProblem(*p, opt, s, o, d_in_grads, transposed);
-  return runProblem(ctx, q);
+  const PassOperands separate{p->input_type, d_out_grads, d_weights, p->out_chans_per_group, p->out_chans_per_group,
+                              p->in_chans_per_group};
+  if (s.strH != 1 || s.strW != 1)
+    return convBwdStrided(ctx, q, opt, s, o, d_in_grads, transposed, p, together ? &separate : nullptr);
+  IgemmProblem r = convBwdProblem(q, opt, s, o, d_in_grads, transposed);
+  if (together) r.nonfinite = nonfiniteFlag(ctx);
+  if (int rc = runProblem(ctx, r)) return rc;
+  if (!together) return PLB_OK;
+  return repairNonFinite(ctx, convBwdProblem(*p, opt, s, separate, d_in_grads, false), p->input_type);
 }
 
 int plb_conv_fwd_host(plb_context *ctx, const plb_conv_params *p, const plb_conv_options *opt,

@@ -434,12 +434,6 @@ int launchIgemm(plb_context *ctx, const IgemmProblem &p, const plb_plan &plan) {
       return rc;
     a.use_tma_store = 1;
   }
-  a.scatter_rows = !split && !a.use_tma_store &&
-                           ((reinterpret_cast<uintptr_t>(p.out) & 15) != 0 || (size_t(p.ldc) * out_es) % 16 != 0 ||
-                            (size_t(out_stride_h) * out_es) % 16 != 0 || (size_t(out_stride_n) * out_es) % 16 != 0 ||
-                            (groups > 1 && (size_t(p.out_group_stride) * out_es) % 16 != 0))
-                       ? 1
-                       : 0;
   a.box_w = plan.box_w;
   a.box_h = plan.box_h;
   a.box_n = plan.box_n;
@@ -525,6 +519,7 @@ int launchIgemm(plb_context *ctx, const IgemmProblem &p, const plb_plan &plan) {
   a.alpha = split ? 1.f : p.alpha;
   a.beta = split ? 0.f : p.beta;
   a.out_is_f32 = split || p.out_f32 ? 1 : 0;
+  a.nonfinite = p.nonfinite;
   a.status = ctx->d_status;
   a.trace = ctx->trace;
 

@@ -22,12 +22,15 @@
 //                 tensor copy costs a thread a few hundred cycles, so a single
 //                 producer cannot keep the tensor core fed on narrow tiles.
 //   warp 3        issues tcgen05.mma with fp32 accumulators in tensor memory.
-//   warp 20       a second issuer for short tiles: issuing an MMA costs its
-//                 thread about 28 cycles and every tile a few hundred more in
-//                 barrier waits and commits, which on a tile of 16 instructions
-//                 exceeds the 46 cycles the tensor core needs per instruction.
-//                 The two issuers take alternate tiles (and so always the
-//                 same accumulator each).
+//   warp 2        for short tiles not a producer but a second issuer: issuing an
+//                 MMA costs its thread about 28 cycles and every tile a few hundred
+//                 more in barrier waits and commits, which on a tile of 16
+//                 instructions exceeds the 46 cycles the tensor core needs per
+//                 instruction.  The two issuers take alternate tiles (and so
+//                 always the same accumulator each).  (Not a warp of its own: with
+//                 21 warps one of the SM's four register files serves six of them,
+//                 which leaves 80 registers per thread; 20 warps leave 96, and the
+//                 epilogue needs more than 80.)
 //   warps 4..19   epilogue, two groups of eight warps: drain a finished
 //                 accumulator (tcgen05.ld), scale / add / cast, stage 32 rows
 //                 x 128 bytes per pair of warps in shared memory and hand them
@@ -51,12 +54,12 @@ namespace plb {
 
 constexpr int kTileM = 128;        // pixels (rows) per tile = TMEM lanes
 constexpr int kStageKBytes = 128;  // bytes of K per pipeline stage row (one swizzle span)
-constexpr int kIgemmThreads = 672;
+constexpr int kIgemmThreads = 640;
 constexpr int kIgemmProducers = PLB_IGEMM_PRODUCERS;
 constexpr int kIgemmMmaWarp = 3;
-constexpr int kIgemmMmaWarp2 = 20;  // second MMA issuer (short tiles), after the 16 epilogue warps
+constexpr int kIgemmMmaWarp2 = 2;  // second MMA issuer (short tiles), else the third producer
 constexpr int kEpiStagingBytes = 8 * 4096;  // 8 pairs of epilogue warps x (32 rows x 128 B)
-static_assert(kIgemmProducers >= 1 && kIgemmProducers <= 3, "producer warps are warps 0..2");
+static_assert(kIgemmProducers > kIgemmMmaWarp2 && kIgemmProducers <= 3, "producer warps are warps 0..2");
 
 struct IgemmArgs {
   // ---- M side: output pixels, tiled by a (w, h, n) box of 128 pixels ------
@@ -119,9 +122,9 @@ struct IgemmArgs {
   const float *bias;
   float alpha, beta;
   int out_is_f32;
-  int scatter_rows;         // output rows allow no vector stores: turn blocks in shared memory
   int use_tma_store;        // tm_out is valid: stage through shared memory + TMA store
   int sub_w, sub_h;         // pixel box of one epilogue warp's 32 rows: (sub_w, sub_h, 32/(sub_w*sub_h))
+  int *nonfinite;  // set to 1 if a sum is not finite (null: not asked for)
   int *status;
   // Optional timeline (only written by builds with -DPLB_TRACE): CTA 0 stores
   // clock64() stamps, 4096 slots per role (producer 0, MMA issuer, epilogue).
@@ -206,7 +209,7 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
   const bool leader = cta_rank == 0;
   constexpr int kMaxStages = kIgemmMaxStages;
   const int kStages = args.num_stages;
-  constexpr int P = kIgemmProducers;
+  const int P = args.dual_issue ? kIgemmMmaWarp2 : kIgemmProducers;
   constexpr uint32_t kTmemCols = 2 * BN;  // two accumulators
   static_assert(kTmemCols >= 32 && kTmemCols <= 512 && (kTmemCols & (kTmemCols - 1)) == 0, "");
   static_assert(!(kFp8 && (kAMn || kBMn)), "MN-major operands are implemented for fp16 only");
@@ -536,7 +539,7 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
       }
       if (me == 0) PLB_TRACE_STAMP(2, 4014);
     }
-  } else if (warp == kIgemmMmaWarp || warp == kIgemmMmaWarp2) {
+  } else if (warp <= kIgemmMmaWarp) {
     // ===================== MMA issuer(s) =====================
     // (with a CTA pair only the CTA of rank 0 issues)
     const int mi = warp == kIgemmMmaWarp ? 0 : 1;
@@ -678,7 +681,7 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
       }
       if (mi == 0) PLB_TRACE_STAMP(2, 4015);
     }
-  } else if (warp >= 4 && warp < 20) {
+  } else {
     // ===================== epilogue (warps 4..19) =====================
     // Accumulator g is drained by the eight warps of group g.  A warp can read
     // the 32 TMEM lanes (tile rows) [32*(warp%4), +32); the two warps that share
@@ -709,7 +712,7 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
     const bool out_f32 = args.out_is_f32 != 0;
     // fp32 rows fill the 128-byte staged row with 32 columns: the `half == 1`
     // warps then leave the work to their partners
-    const bool idle = tma_store && out_f32 && half == 1;
+    const bool idle = out_f32 && args.split_k == 1 && half == 1;
     const bool stamp = threadIdx.x == 128;
     const int acc = group;
     int local_tile = group;
@@ -781,10 +784,38 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
         continue;
       }
 
-      // 32 accumulator columns [c, c + 32) of this thread's row: scale / add / cast
-      auto finish = [&](const uint32_t (&v)[32], float (&f)[32], const int c) {
+      // The accumulator in blocks of 32 columns: scale / add, then
+      //  - the fp32 sums of a K split: vector stores of each lane's own row (the
+      //    scratch rows are padded to whole blocks),
+      //  - else the block is staged in swizzled shared memory (half: each warp its
+      //    own 32 rows x 64 bytes, so that no barrier between warps lies on the
+      //    chain load -> convert -> stage -> store; fp32: 32 rows x 128 bytes) and
+      //    leaves with a tensor store, or, where the output cannot be described to
+      //    TMA, row by row: lane after lane writing its own row would touch a
+      //    sector per element, consecutive lanes take consecutive columns instead.
+      // One loop for all of them: a short kernel's instructions come from L2.
+      const uint32_t wbuf = staging_base + uint32_t(warp - 4) * 2048u;
+      const uint32_t wrow = wbuf + uint32_t(lane) * 64u, sw = (uint32_t(lane) >> 1) & 3u;
+      const bool whole_rows = out_f32 && args.split_k == 1;  // 128-byte rows, the half == 0 warps only
+      const int c_first = whole_rows ? 0 : half * 32, c_step = whole_rows ? 32 : 64;
+      if (c_first >= cols_end) release_accumulator();
+#pragma unroll 1
+      for (int c = c_first; c < cols_end; c += c_step) {
+        uint32_t v[32];
+        float f[32];
+        __syncwarp();
+        tmem_ld_32x32(t_addr + c, v);
+        tmem_ld_wait_for(v);
+        if (c + c_step >= cols_end) release_accumulator();
         const int col0 = col_base + c;
-        const int valid = min(32, args.n_total - col0);  // may be <= 0 on a padded N tile
+        const int valid = min(32, args.n_total - col0);
+        if (args.nonfinite != nullptr) {
+          uint32_t largest = 0u;
+#pragma unroll
+          for (int j = 0; j < 32; ++j)
+            if (j < valid) largest = max(largest, v[j] & 0x7fffffffu);
+          if (largest >= 0x7f800000u) *args.nonfinite = 1;
+        }
         if (args.alpha != 1.f) {
 #pragma unroll
           for (int j = 0; j < 32; ++j) f[j] = __uint_as_float(v[j]) * args.alpha;
@@ -793,230 +824,111 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
           for (int j = 0; j < 32; ++j) f[j] = __uint_as_float(v[j]);
         }
         if (args.bias != nullptr) {
+          // (the same addresses in every lane: one 16-byte broadcast per four columns;
+          // as 32 predicated words the bias cost the 7x7 layer 60 of 180 us)
+          const float *bias = args.bias + cgroup * args.n_total + col0;
+          if (valid == 32 && (reinterpret_cast<uintptr_t>(bias) & 15) == 0) {
 #pragma unroll
-          for (int j = 0; j < 32; ++j)
-            if (j < valid) f[j] += args.bias[cgroup * args.n_total + col0 + j];
+            for (int j = 0; j < 32; j += 4) {
+              const float4 b4 = *reinterpret_cast<const float4 *>(bias + j);
+              f[j] += b4.x;
+              f[j + 1] += b4.y;
+              f[j + 2] += b4.z;
+              f[j + 3] += b4.w;
+            }
+          } else {
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+              if (j < valid) f[j] += bias[j];
+          }
         }
         if (args.addend != nullptr && row_ok) {
+          const long long at = pixel * args.ld_addend + cgroup * args.addend_group_stride + col0;
           if (out_f32) {
-            const float *src = static_cast<const float *>(args.addend) + pixel * args.ld_addend +
-                               cgroup * args.addend_group_stride + col0;
+            const float *src = static_cast<const float *>(args.addend) + at;
 #pragma unroll
             for (int j = 0; j < 32; ++j)
               if (j < valid) f[j] += args.beta * src[j];
           } else {
-            const __half *src = static_cast<const __half *>(args.addend) + pixel * args.ld_addend +
-                                cgroup * args.addend_group_stride + col0;
+            const __half *src = static_cast<const __half *>(args.addend) + at;
 #pragma unroll
             for (int j = 0; j < 32; ++j)
               if (j < valid) f[j] += args.beta * __half2float(src[j]);
           }
         }
-      };
-      // plain vector stores of 32 finished columns (output not describable to TMA)
-      auto store_direct = [&](const float (&f)[32], const int c) {
-        const int col0 = col_base + c;
-        const int valid = min(32, args.n_total - col0);
-        if (!row_ok || valid <= 0) return;
-        if (out_f32) {
-          // (with split-K: this split's slice of the partial sums)
-          float *dst = static_cast<float *>(args.out) + split * args.split_stride + out_off + col0;
-          if (valid == 32 && (reinterpret_cast<uintptr_t>(dst) & 31) == 0) {
-            // whole 32-byte sectors per lane
+        if (args.split_k > 1) {
+          // (this split's slice of the partial sums, whole 32-byte sectors per lane)
+          if (row_ok) {
+            float *dst = static_cast<float *>(args.out) + split * args.split_stride + out_off + col0;
 #pragma unroll
             for (int j = 0; j < 32; j += 8)
-              st_global_v8(dst + j, __float_as_uint(f[j]), __float_as_uint(f[j + 1]),
-                           __float_as_uint(f[j + 2]), __float_as_uint(f[j + 3]),
-                           __float_as_uint(f[j + 4]), __float_as_uint(f[j + 5]),
+              st_global_v8(dst + j, __float_as_uint(f[j]), __float_as_uint(f[j + 1]), __float_as_uint(f[j + 2]),
+                           __float_as_uint(f[j + 3]), __float_as_uint(f[j + 4]), __float_as_uint(f[j + 5]),
                            __float_as_uint(f[j + 6]), __float_as_uint(f[j + 7]));
-          } else if (valid == 32 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
-#pragma unroll
-            for (int j = 0; j < 32; j += 4)
-              *reinterpret_cast<float4 *>(dst + j) = make_float4(f[j], f[j + 1], f[j + 2], f[j + 3]);
-          } else {
-#pragma unroll
-            for (int j = 0; j < 32; ++j)
-              if (j < valid) dst[j] = f[j];
           }
-        } else {
-          __half *dst = static_cast<__half *>(args.out) + out_off + col0;
-          if (valid == 32 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
-            uint32_t pk[16];
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              __half2 h = __floats2half2_rn(f[2 * j], f[2 * j + 1]);
-              pk[j] = *reinterpret_cast<uint32_t *>(&h);
-            }
-            if ((reinterpret_cast<uintptr_t>(dst) & 31) == 0) {
-              st_global_v8(dst, pk[0], pk[1], pk[2], pk[3], pk[4], pk[5], pk[6], pk[7]);
-              st_global_v8(dst + 16, pk[8], pk[9], pk[10], pk[11], pk[12], pk[13], pk[14], pk[15]);
-            } else {
-#pragma unroll
-              for (int j = 0; j < 4; ++j)
-                *reinterpret_cast<uint4 *>(dst + 8 * j) =
-                    make_uint4(pk[4 * j], pk[4 * j + 1], pk[4 * j + 2], pk[4 * j + 3]);
-            }
-          } else {
-#pragma unroll
-            for (int j = 0; j < 32; ++j)
-              if (j < valid) dst[j] = __float2half_rn(f[j]);
-          }
+          continue;
         }
-      };
-      // The same for rows whose addresses allow no vector (a row pitch that is not
-      // a multiple of 16 bytes): lane after lane writing its own row would touch a
-      // sector per element, so the block is turned in shared memory (16-byte
-      // pieces XOR-swizzled with the row) and leaves row by row, consecutive lanes
-      // at consecutive columns, two rows per instruction.
-      auto store_rows = [&](const float (&f)[32], const int c) {
-        const uint32_t wbuf = staging_base + uint32_t(warp - 4) * 2048u;
-        const uint32_t wrow = wbuf + uint32_t(lane) * 64u, sw = (uint32_t(lane) >> 1) & 3u;
-        const int col0 = col_base + c, valid = min(32, args.n_total - col0);
-        const long long my_off = row_ok ? split * args.split_stride + out_off + col0 : -1ll;
-        const uint32_t lo = uint32_t(my_off), hi = uint32_t(my_off >> 32);
-        if (out_f32) {
-          // 16 columns (64 bytes of fp32) at a time
-#pragma unroll
-          for (int b = 0; b < 2; ++b) {
-            __syncwarp();
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-              st_shared_v4(wrow + ((uint32_t(j) ^ sw) << 4), __float_as_uint(f[16 * b + 4 * j]),
-                           __float_as_uint(f[16 * b + 4 * j + 1]), __float_as_uint(f[16 * b + 4 * j + 2]),
-                           __float_as_uint(f[16 * b + 4 * j + 3]));
-            __syncwarp();
-            const int cc = lane & 15;
-#pragma unroll 4
-            for (int r0 = 0; r0 < 32; r0 += 2) {
-              const int r = r0 + (lane >> 4);
-              const uint32_t v0 = ld_shared_b32(wbuf + uint32_t(r) * 64u +
-                                                (((uint32_t(cc) >> 2) ^ ((uint32_t(r) >> 1) & 3u)) << 4) +
-                                                (uint32_t(cc) & 3u) * 4u);
-              const long long off = (long long)(uint64_t(__shfl_sync(0xffffffffu, hi, r)) << 32 |
-                                                __shfl_sync(0xffffffffu, lo, r));
-              if (off >= 0 && 16 * b + cc < valid) static_cast<float *>(args.out)[off + 16 * b + cc] = __uint_as_float(v0);
-            }
-          }
-        } else {
-          __syncwarp();
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            __half2 h0 = __floats2half2_rn(f[8 * j], f[8 * j + 1]);
-            __half2 h1 = __floats2half2_rn(f[8 * j + 2], f[8 * j + 3]);
-            __half2 h2 = __floats2half2_rn(f[8 * j + 4], f[8 * j + 5]);
-            __half2 h3 = __floats2half2_rn(f[8 * j + 6], f[8 * j + 7]);
-            st_shared_v4(wrow + ((uint32_t(j) ^ sw) << 4), *reinterpret_cast<uint32_t *>(&h0),
-                         *reinterpret_cast<uint32_t *>(&h1), *reinterpret_cast<uint32_t *>(&h2),
-                         *reinterpret_cast<uint32_t *>(&h3));
-          }
-          __syncwarp();
-          // lanes 0..15 and 16..31: a row each, two columns per lane
-          const int cc = (lane & 15) * 2;
-#pragma unroll 4
-          for (int r0 = 0; r0 < 32; r0 += 2) {
-            const int r = r0 + (lane >> 4);
-            const uint32_t v0 = ld_shared_b32(wbuf + uint32_t(r) * 64u +
-                                              (((uint32_t(cc) >> 3) ^ ((uint32_t(r) >> 1) & 3u)) << 4) +
-                                              (uint32_t(cc) & 7u) * 2u);
-            const long long off = (long long)(uint64_t(__shfl_sync(0xffffffffu, hi, r)) << 32 |
-                                              __shfl_sync(0xffffffffu, lo, r));
-            if (off >= 0) {
-              uint16_t *dst = static_cast<uint16_t *>(args.out) + off + cc;
-              if (cc + 1 < valid && (reinterpret_cast<uintptr_t>(dst) & 3) == 0) {
-                *reinterpret_cast<uint32_t *>(dst) = v0;
-              } else {
-                if (cc < valid) dst[0] = uint16_t(v0);
-                if (cc + 1 < valid) dst[1] = uint16_t(v0 >> 16);
-              }
-            }
-          }
-        }
-      };
-      // issue (lane 0) the tensor store of the staged buffer: columns [store_col, +128 bytes)
-      auto store_staged = [&](const uint32_t buf, const int store_col) {
-        if (lane == 0) {
-          // a box that starts outside the tensor has nothing to write
-          if (store_col < args.n_total && box_ok) {
-            const int c2 = args.h_outer ? n0 + qn : h0 + qh, c3 = args.h_outer ? h0 + qh : n0 + qn;
-            if (args.groups > 1)
-              tma_store_5d(&tm_out, buf, store_col, cgroup, w0 + qw, c2, c3);
-            else
-              tma_store_4d(&tm_out, buf, store_col, w0 + qw, c2, c3);
-          }
-          tma_store_commit();
-        }
-      };
-
-      uint32_t v[32];
-      float f[32];
-      if (!tma_store) {
-        // each warp stores its own 32 columns of every 64-column block
-#pragma unroll 1
-        for (int c = half * 32; c < cols_end; c += 64) {
-          __syncwarp();
-          tmem_ld_32x32(t_addr + c, v);
-          tmem_ld_wait_for(v);
-          if (c + 64 >= cols_end) release_accumulator();
-          finish(v, f, c);
-          if (args.scatter_rows)
-            store_rows(f, c);
-          else
-            store_direct(f, c);
-        }
-        if (half * 32 >= cols_end) release_accumulator();
-      } else if (out_f32) {
-        // (half == 0 warps only) one 32-column chunk per staged buffer and store
-#pragma unroll 1
-        for (int c = 0; c < cols_end; c += 32) {
-          __syncwarp();
-          tmem_ld_32x32(t_addr + c, v);
-          tmem_ld_wait_for(v);
-          if (c + 32 >= cols_end) release_accumulator();
-          finish(v, f, c);
-          if (lane == 0) tma_store_wait_read<0>();  // the previous store has read the buffer
-          __syncwarp();
+        if (tma_store && lane == 0) tma_store_wait_read<0>();  // the previous store has read the buffer
+        __syncwarp();
+        if (whole_rows) {
 #pragma unroll
           for (int j = 0; j < 8; ++j)
             st_shared_v4(row_addr + (uint32_t(j ^ (lane & 7)) << 4), __float_as_uint(f[4 * j]),
                          __float_as_uint(f[4 * j + 1]), __float_as_uint(f[4 * j + 2]),
                          __float_as_uint(f[4 * j + 3]));
-          fence_proxy_async_smem();
-          __syncwarp();
-          store_staged(buf, col_base + c);
-        }
-      } else {
-        // half output: each warp stages its own 32 rows x 32 columns (64-byte
-        // rows; 16-byte pieces XOR-swizzled with bits 1-2 of the row index, the
-        // tensor map's 64-byte swizzle, which also keeps the stores free of bank
-        // conflicts) and hands them to a tensor store of its own, so no barrier
-        // between warps lies on the chain load -> convert -> stage -> store.
-        const uint32_t wbuf = staging_base + uint32_t(warp - 4) * 2048u;
-        const uint32_t wrow = wbuf + uint32_t(lane) * 64u;
-        const uint32_t sw = (uint32_t(lane) >> 1) & 3u;
-#pragma unroll 1
-        for (int c = half * 32; c < cols_end; c += 64) {
-          __syncwarp();
-          tmem_ld_32x32(t_addr + c, v);
-          tmem_ld_wait_for(v);
-          if (c + 64 >= cols_end) release_accumulator();
-          finish(v, f, c);
-          if (lane == 0) tma_store_wait_read<0>();  // this warp's previous store has read the buffer
-          __syncwarp();
+        } else {
+          // 16-byte pieces XOR-swizzled with bits 1-2 of the row index: the tensor
+          // map's 64-byte swizzle, free of bank conflicts
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
-            __half2 h0 = __floats2half2_rn(f[8 * j], f[8 * j + 1]);
-            __half2 h1 = __floats2half2_rn(f[8 * j + 2], f[8 * j + 3]);
-            __half2 h2 = __floats2half2_rn(f[8 * j + 4], f[8 * j + 5]);
-            __half2 h3 = __floats2half2_rn(f[8 * j + 6], f[8 * j + 7]);
-            st_shared_v4(wrow + ((uint32_t(j) ^ sw) << 4), *reinterpret_cast<uint32_t *>(&h0),
-                         *reinterpret_cast<uint32_t *>(&h1), *reinterpret_cast<uint32_t *>(&h2),
-                         *reinterpret_cast<uint32_t *>(&h3));
+            uint32_t pk[4];
+            pack_half8(f + 8 * j, pk);
+            st_shared_v4(wrow + ((uint32_t(j) ^ sw) << 4), pk[0], pk[1], pk[2], pk[3]);
           }
+        }
+        if (tma_store) {
           fence_proxy_async_smem();
           __syncwarp();
-          store_staged(wbuf, col_base + c);
+          if (lane == 0) {
+            // a box that starts outside the tensor has nothing to write
+            if (box_ok) {
+              const uint32_t src = whole_rows ? buf : wbuf;
+              const int c2 = args.h_outer ? n0 + qn : h0 + qh, c3 = args.h_outer ? h0 + qh : n0 + qn;
+              if (args.groups > 1)
+                tma_store_5d(&tm_out, src, col0, cgroup, w0 + qw, c2, c3);
+              else
+                tma_store_4d(&tm_out, src, col0, w0 + qw, c2, c3);
+            }
+            tma_store_commit();
+          }
+          continue;
         }
-        if (half * 32 >= cols_end) release_accumulator();
+        __syncwarp();
+        const uint32_t lo = uint32_t(out_off), hi = row_ok ? uint32_t(out_off >> 32) : 0x80000000u;
+#pragma unroll 2
+        for (int i = 0; i < (whole_rows ? 32 : 16); ++i) {
+          // fp32: a row of 32 columns; half: two rows of 16 words
+          const int r = whole_rows ? i : 2 * i + (lane >> 4), cc = whole_rows ? lane : 2 * (lane & 15);
+          const uint32_t piece = uint32_t(whole_rows ? lane : lane & 15) >> 2, word = (uint32_t(lane) & 3u) << 2;
+          const uint32_t bits = ld_shared_b32(
+              whole_rows ? buf + uint32_t(r) * 128u + ((piece ^ (uint32_t(r) & 7u)) << 4) + word
+                         : wbuf + uint32_t(r) * 64u + ((piece ^ ((uint32_t(r) >> 1) & 3u)) << 4) + word);
+          const uint32_t off_hi = __shfl_sync(0xffffffffu, hi, r), off_lo = __shfl_sync(0xffffffffu, lo, r);
+          if (int32_t(off_hi) >= 0 && cc < valid) {
+            const long long off = (long long)(uint64_t(off_hi) << 32 | off_lo) + col0 + cc;
+            if (out_f32) {
+              static_cast<uint32_t *>(args.out)[off] = bits;
+            } else {
+              uint16_t *dst = static_cast<uint16_t *>(args.out) + off;
+              if (cc + 1 < valid && (reinterpret_cast<uintptr_t>(dst) & 3) == 0) {
+                *reinterpret_cast<uint32_t *>(dst) = bits;
+              } else {
+                dst[0] = uint16_t(bits);
+                if (cc + 1 < valid) dst[1] = uint16_t(bits >> 16);
+              }
+            }
+          }
+        }
       }
       if (stamp) PLB_TRACE_STAMP(2, local_tile * 4 + 2);
       if (stamp) PLB_TRACE_STAMP(2, local_tile * 4 + 3);

@@ -23,6 +23,7 @@ enum plb_scratch_slot {
   kSlotHostOut,
   kSlotHostBias,
   kSlotChannelSums,     // partial per-channel sums (normalisation, bias update)
+  kSlotBlockDiagonal,   // block-diagonal weights of channel groups contracted together
   kSlotUsedTaps,        // gradient of a truncated / flipped kernel's taps
   kSlotRepacked,        // operands with rows rounded up to 16 bytes / split into bfloat16 pieces
   kSlotFlipped,         // reversed input (input flip)
@@ -241,6 +242,7 @@ struct IgemmProblem {
   long long ld_addend = 0;
   const float *bias = nullptr;
   float alpha = 1.f, beta = 0.f;
+  int *nonfinite = nullptr;  // device word set to 1 if a sum is not finite
   bool out_f32 = false;
   int force_tile_n = 0;  // 0 = planner's choice
   int force_split_k = 0; // 0 = planner's choice; n = n CTAs per output tile (clamped to the K steps)

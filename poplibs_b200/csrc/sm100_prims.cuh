@@ -227,6 +227,14 @@ __device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t a, uint32_t
                : "memory");
 }
 
+// Eight fp32 values rounded to half, packed in order.
+__device__ __forceinline__ void pack_half8(const float *f, uint32_t (&pk)[4]) {
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const __half2 h = __floats2half2_rn(f[2 * j], f[2 * j + 1]);
+    pk[j] = *reinterpret_cast<const uint32_t *>(&h);
+  }
+}
 __device__ __forceinline__ uint32_t ld_shared_b32(uint32_t addr) {
   uint32_t v;
   asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");

@@ -77,10 +77,43 @@ struct WuProblem {
   uint64_t x_chans = 0, dy_chans = 0, x_strides[3] = {}, dy_strides[3] = {};
 };
 
-// The layer's tensors [N][H][W][groups * pitch] with `sub` groups contracted
-// together (every sub'th group starts a super-group).
-WuProblem wuProblem(const plb_conv_params &p, const WuShape &s, uint32_t ci_pitch, uint32_t co_pitch, uint32_t groups,
-                    uint32_t sub) {
+// How the channels of a pixel lie in the operands the kernel reads, and how many
+// groups are contracted together (every sub'th group starts a super-group).
+struct WuLayout {
+  uint32_t sub, ci_pitch, co_pitch;  // channels from one group to the next
+  uint64_t x_pixel, dy_pixel;        // from one pixel to the next
+};
+
+// Groups together: as many as fill the 128 output-channel rows of the tensor-core
+// tile without exceeding 128 input channels.  32 groups of 8 channels run as two
+// dense blocks of 128 x 128 instead of 32 launches whose tiles are 15/16 padding.
+// A super-group has to start on a 16-byte boundary; only where no number of groups
+// does are the channels of each group rounded up.
+WuLayout wuLayout(uint32_t groups, uint32_t ci, uint32_t co) {
+  WuLayout l{};
+  const uint32_t most = std::max<uint32_t>(1, std::min(groups, std::min(128 / std::max(co, 1u), 128 / std::max(ci, 1u))));
+  auto quantum = [](uint32_t c) {
+    uint32_t q = 1;
+    while ((q * c) % 8 != 0) q *= 2;
+    return q;
+  };
+  const uint32_t q = std::max(quantum(ci), quantum(co));
+  l.sub = most == groups ? groups : most / q * q;
+  l.ci_pitch = ci;
+  l.co_pitch = co;
+  if (l.sub == 0) {
+    l.ci_pitch = roundToVec(ci, 2);
+    l.co_pitch = roundToVec(co, 2);
+    l.sub = std::max<uint32_t>(1, std::min(groups, std::min(128 / l.co_pitch, 128 / l.ci_pitch)));
+  }
+  l.x_pixel = roundToVec(uint64_t(groups) * l.ci_pitch, 2);
+  l.dy_pixel = roundToVec(uint64_t(groups) * l.co_pitch, 2);
+  return l;
+}
+
+// The layer's tensors [N][H][W][x_pixel] with the channels laid out as `l` says.
+WuProblem wuProblem(const plb_conv_params &p, const WuShape &s, const WuLayout &l, uint32_t groups) {
+  const uint32_t ci_pitch = l.ci_pitch, co_pitch = l.co_pitch, sub = l.sub;
   const size_t es = 2;
   WuProblem q;
   q.bf16 = p.input_type == PLB_BFLOAT16;
@@ -89,12 +122,13 @@ WuProblem wuProblem(const plb_conv_params &p, const WuShape &s, uint32_t ci_pitc
   q.sgroups = int((groups + sub - 1) / sub);
   q.sub_ci = int(ci_pitch);
   q.sub_co = int(co_pitch);
-  q.ci = int(sub * ci_pitch);
-  q.co = int(sub * co_pitch);
+  // (a single super-group may include the channels the pixel was rounded up by)
+  q.ci = int(q.sgroups == 1 ? roundToVec(sub * ci_pitch, 2) : sub * ci_pitch);
+  q.co = int(q.sgroups == 1 ? roundToVec(sub * co_pitch, 2) : sub * co_pitch);
   q.s = s;
-  q.x_chans = uint64_t(groups) * ci_pitch;
-  q.dy_chans = uint64_t(groups) * co_pitch;
-  const uint64_t xp = uint64_t(p.groups) * ci_pitch * es, yp = uint64_t(p.groups) * co_pitch * es;
+  q.x_chans = std::min<uint64_t>(l.x_pixel, uint64_t(q.sgroups) * q.ci);
+  q.dy_chans = std::min<uint64_t>(l.dy_pixel, uint64_t(q.sgroups) * q.co);
+  const uint64_t xp = l.x_pixel * es, yp = l.dy_pixel * es;
   q.x_strides[0] = xp;
   q.x_strides[1] = uint64_t(s.W) * xp;
   q.x_strides[2] = uint64_t(s.H) * s.W * xp;
@@ -393,6 +427,12 @@ int launchWuKernel(cudaStream_t stream, const WuProblem &p, const WuArgs &a) {
   return PLB_OK;
 }
 
+// One group of a layer whose groups are contracted one after the other.
+WuLayout oneGroup(const plb_conv_params &p) {
+  const uint32_t ci = p.in_chans_per_group, co = p.out_chans_per_group;
+  return WuLayout{1, ci, co, uint64_t(p.groups) * ci, uint64_t(p.groups) * co};
+}
+
 // The groups of a layer one after the other, through one group's worth of scratch
 // (the entry points that cannot hold more).  With `peer` the reduction also adds
 // the gradients of the other ranks; the caller has checked that the shapes allow it.
@@ -402,7 +442,7 @@ int launchWuPerGroup(cudaStream_t stream, const plb_conv_params &p, const WuShap
   const uint32_t co = p.out_chans_per_group, ci = p.in_chans_per_group;
   const size_t w_elems = size_t(s.KH) * s.KW * co * ci, es = 2;
   for (unsigned g = 0; g < p.groups; ++g) {
-    WuProblem q = wuProblem(p, s, ci, co, 1, 1);
+    WuProblem q = wuProblem(p, s, oneGroup(p), 1);
     q.x = static_cast<const uint8_t *>(d_acts) + size_t(g) * ci * es;
     q.dy = static_cast<const uint8_t *>(d_out_grads) + size_t(g) * co * es;
     if (int rc = launchWuKernel(stream, q, a)) return rc;
@@ -413,15 +453,6 @@ int launchWuPerGroup(cudaStream_t stream, const plb_conv_params &p, const WuShap
     if (launches) *launches += 2;
   }
   return PLB_OK;
-}
-
-// Channel groups contracted together: as many as fill the 128 output-channel rows
-// of the tensor-core tile without exceeding 128 input channels.  32 groups of 8
-// channels run as two dense blocks of 128 x 128 instead of 32 launches whose
-// tiles are 15/16 padding.
-uint32_t wuGroupsTogether(uint32_t groups, uint32_t ci_pitch, uint32_t co_pitch) {
-  return std::max<uint32_t>(1, std::min(groups, std::min(128 / std::max<uint32_t>(co_pitch, 1),
-                                                         128 / std::max<uint32_t>(ci_pitch, 1))));
 }
 
 }  // namespace
@@ -466,9 +497,8 @@ int plb_conv_wu_plan(const plb_conv_params *p_in, const plb_conv_options *opt, p
   if (int rc = wuShape(*p, &s)) return rc;
   *plan = plb_plan{};
   WuArgs a{};
-  const uint32_t cip = roundToVec(p->in_chans_per_group, 2), cop = roundToVec(p->out_chans_per_group, 2);
-  planWu(wuProblem(*p, s, cip, cop, p->groups, wuGroupsTogether(p->groups, cip, cop)), 148, opt ? opt->split_k : 0,
-         opt ? opt->plan_flags : 0, &a, plan);
+  planWu(wuProblem(*p, s, wuLayout(p->groups, p->in_chans_per_group, p->out_chans_per_group), p->groups), 148,
+         opt ? opt->split_k : 0, opt ? opt->plan_flags : 0, &a, plan);
   plan->flops = 2 * numberOfMacs(*p);
   const uint64_t es = dtypeBytes(p->input_type);
   plan->bytes = es * (uint64_t(p->batch) * s.H * s.W * p->groups * p->in_chans_per_group +
@@ -647,7 +677,7 @@ int plb_conv_wu(plb_context *ctx, const plb_conv_params *p, const plb_conv_optio
     s2.KW = 1;
     s2.padH = s2.padW = 0;
     s2.strH = s2.strW = 1;
-    WuProblem q = wuProblem(*p, s2, 64, uint32_t(co), 1, 1);
+    WuProblem q = wuProblem(*p, s2, WuLayout{1, 64, uint32_t(co), 64, uint64_t(co)}, 1);
     q.x = ws;
     q.x_strides[0] = uint64_t(g2.C2) * 2;
     q.x_strides[1] = uint64_t(g2.W2) * g2.C2 * 2;
@@ -667,21 +697,26 @@ int plb_conv_wu(plb_context *ctx, const plb_conv_params *p, const plb_conv_optio
   // bfloat16 pieces side by side.  The padded rows and columns of the partial sums
   // are not read.
   const bool is_float = p->input_type == PLB_FLOAT;
-  const uint32_t G = p->groups, cip = roundToVec(uint64_t(ci), 2), cop = roundToVec(uint64_t(co), 2);
-  const uint64_t x_rows = uint64_t(p->batch) * s.H * s.W * G, dy_rows = uint64_t(p->batch) * s.OH * s.OW * G;
+  const WuLayout l = wuLayout(p->groups, uint32_t(ci), uint32_t(co));
+  const uint64_t x_pixels = uint64_t(p->batch) * s.H * s.W, dy_pixels = uint64_t(p->batch) * s.OH * s.OW;
   const void *x = d_acts, *dy = d_out_grads;
   {
     Repack jobs[2];
     const void **operand[2];
     int n = 0;
-    auto add = [&](const void **base, uint64_t rows, uint32_t cols, uint32_t pitch, bool second) {
-      if (!is_float && cols == pitch && (reinterpret_cast<uintptr_t>(*base) & 15) == 0) return;
-      jobs[n] = Repack{*base, nullptr, rows, cols, cols, pitch, is_float ? 4u : 2u,
-                       is_float ? kRepackSplitPlanes : kRepackCopy, second, 0};
+    // whole pixels, or where the groups' channels are rounded up, each group's
+    auto add = [&](const void **base, uint64_t pixels, uint32_t chans, uint32_t chans_pitch, uint64_t pixel, bool second) {
+      if (!is_float && chans == chans_pitch && pixel == uint64_t(p->groups) * chans &&
+          (reinterpret_cast<uintptr_t>(*base) & 15) == 0)
+        return;
+      const bool whole = chans == chans_pitch;
+      const uint32_t cols = whole ? p->groups * chans : chans;
+      jobs[n] = Repack{*base, nullptr, whole ? pixels : pixels * p->groups, cols, cols, whole ? uint32_t(pixel) : chans_pitch,
+                       is_float ? 4u : 2u, is_float ? kRepackSplitPlanes : kRepackCopy, second, 0};
       operand[n++] = base;
     };
-    add(&x, x_rows, uint32_t(ci), cip, false);
-    add(&dy, dy_rows, uint32_t(co), cop, true);
+    add(&x, x_pixels, uint32_t(ci), l.ci_pitch, l.x_pixel, false);
+    add(&dy, dy_pixels, uint32_t(co), l.co_pitch, l.dy_pixel, true);
     size_t bytes[2] = {0, 0};
     for (int i = 0; i < n; ++i) bytes[i] = (repackBytes(jobs[i]) + 255) & ~size_t(255);
     if (n) {
@@ -696,15 +731,15 @@ int plb_conv_wu(plb_context *ctx, const plb_conv_params *p, const plb_conv_optio
     q16.input_type = PLB_BFLOAT16;
     q16.batch *= 3;
   }
-  WuProblem q = wuProblem(q16, s, cip, cop, G, wuGroupsTogether(G, cip, cop));
+  WuProblem q = wuProblem(q16, s, l, p->groups);
   q.x = x;
   q.dy = dy;
   gather.sub = uint32_t(q.sub);
-  gather.co_pitch = cop;
-  gather.ci_pitch = cip;
+  gather.co_pitch = l.co_pitch;
+  gather.ci_pitch = l.ci_pitch;
   gather.p_co = uint32_t(q.co);
   gather.p_ci = uint32_t(q.ci);
-  const bool same_order = q.sub == 1 && cip == uint32_t(ci) && cop == uint32_t(co);
+  const bool same_order = q.sub == 1 && q.ci == ci && q.co == co;
   return run(q, same_order ? nullptr : &gather);
 }
 
@@ -781,7 +816,7 @@ static int wuAllreduce(plb_context *ctx, const plb_conv_params *p, const plb_con
   if (p->batch == 0 || s.OHc <= 0 || s.OWc <= 0 || s.He <= 0 || s.We <= 0) {
     // this rank has no share of the batch: it contributes zeros, through one
     // split of zero partial sums, so that the peers still get its flags
-    planWu(wuProblem(*p, s, uint32_t(ci), uint32_t(co), 1, 1), ctx->sm_count, 1, opt ? opt->plan_flags : 0, &a, nullptr);
+    planWu(wuProblem(*p, s, oneGroup(*p), 1), ctx->sm_count, 1, opt ? opt->plan_flags : 0, &a, nullptr);
     a.ksplit = 1;
     void *ws = nullptr;
     if (int rc = scratch(ctx, kSlotWuPartials, w_elems * sizeof(float), &ws)) return rc;
@@ -798,7 +833,7 @@ static int wuAllreduce(plb_context *ctx, const plb_conv_params *p, const plb_con
     ctx->launches += launches;
     return PLB_OK;
   }
-  planWu(wuProblem(*p, s, uint32_t(ci), uint32_t(co), 1, 1), ctx->sm_count, opt ? opt->split_k : 0,
+  planWu(wuProblem(*p, s, oneGroup(*p), 1), ctx->sm_count, opt ? opt->split_k : 0,
          opt ? opt->plan_flags : 0, &a, nullptr);
   void *ws = nullptr;
   if (int rc = scratch(ctx, kSlotWuPartials, size_t(a.ksplit) * w_elems * sizeof(float), &ws)) return rc;
@@ -929,7 +964,7 @@ extern "C" int plb_conv_wu_static_scratch(int device, void *cuda_stream, const p
     return PLB_OK;
   }
   WuArgs a{};
-  planWu(wuProblem(*p, s, uint32_t(ci), uint32_t(co), 1, 1), scratch.sm_count, opt ? opt->split_k : 0,
+  planWu(wuProblem(*p, s, oneGroup(*p), 1), scratch.sm_count, opt ? opt->split_k : 0,
          opt ? opt->plan_flags : 0, &a, nullptr);
   // as many K splits as the fixed scratch can hold
   const int max_split = int(kStaticScratchBytes / (w_elems * sizeof(float)));

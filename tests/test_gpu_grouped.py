@@ -1,0 +1,118 @@
+"""Grouped contractions, operands with ragged rows and few-channel layers, at the
+sizes where the route changes: groups that fill a fraction of, exactly or more
+than one 128-byte operand row; group counts whose dense blocks divide them or
+not; channel counts that start a block on a 16-byte boundary only every second,
+fourth or eighth group, or never; first layers of 1 to 7 channels.  Small
+integer data: sums are exact in fp32 and, below 2^11, in half, so the CPU oracle's
+results must come back bit for bit."""
+import numpy as np
+import pytest
+
+import common as T
+import oracle
+from poplibs_b200 import capi
+
+pytestmark = pytest.mark.gpu
+
+
+def exact(got, want, what):
+    got = np.asarray(got, dtype=np.float64)
+    want = np.asarray(want, dtype=np.float64).reshape(got.shape)
+    assert np.array_equal(got, want), f"{what}: {int((got != want).sum())} of {got.size} differ"
+
+
+def ints(r, shape, dtype):
+    return r.integers(-1, 2, shape).astype(dtype)
+
+
+# groups, channels in and out per group
+GROUPS = [(32, 8, 8), (32, 4, 4), (16, 5, 5), (6, 10, 6), (7, 9, 3), (2, 32, 32), (4, 16, 24), (3, 64, 64), (5, 48, 16),
+          (64, 1, 1), (9, 1, 2), (8, 12, 20), (2, 136, 40), (3, 33, 17)]
+
+
+@pytest.mark.parametrize("stride", [1, 2])
+@pytest.mark.parametrize("groups,ci,co", GROUPS)
+def test_grouped_convolution(gpu_ctx, groups, ci, co, stride):
+    kw = dict(batch=3, field=[9, 7], kernel=[3, 3], in_chans=ci, out_chans=co, groups=groups, padding=1, stride=stride)
+    r = T.rng(groups * 100 + ci + co)
+    for dtype, plb in ((np.float16, capi.HALF), (np.float32, capi.FLOAT)):
+        p = capi.ConvParams.make(input_type=plb, output_type=plb, **kw)
+        spec = T.spec_from_params(p)
+        x = ints(r, (3, groups * ci, 9, 7), dtype)
+        w = ints(r, (groups, co, ci, 3, 3), dtype)
+        dy = ints(r, (3, groups * co, *p.output_field()), dtype)
+        bias = r.integers(-3, 4, groups * co).astype(np.float32)
+        exact(T.gpu_conv_fwd(p, x, w, bias=bias), oracle.conv_fwd(spec, x, w, bias), f"fwd {dtype}")
+        exact(T.gpu_conv_bwd(p, dy, w), oracle.conv_bwd(spec, dy, w), f"bwd {dtype}")
+        exact(T.gpu_conv_wu(p, x, dy)[1], oracle.conv_wu(spec, x, dy)[0], f"wu {dtype}")
+
+
+@pytest.mark.parametrize("stride", [1, 2])
+@pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan])
+@pytest.mark.parametrize("groups,ci,co", [(32, 8, 8), (6, 10, 6)])
+def test_infinities_stay_in_their_group(gpu_ctx, groups, ci, co, value, stride):
+    """A non-finite element changes the outputs of its own group alone, although
+    neighbouring groups are contracted together."""
+    p = capi.ConvParams.make(batch=2, field=[8, 6], kernel=[3, 3], in_chans=ci, out_chans=co, groups=groups, padding=1,
+                             stride=stride)
+    r = T.rng(5)
+    x = ints(r, (2, groups * ci, 8, 6), np.float16)
+    w = ints(r, (groups, co, ci, 3, 3), np.float16)
+    w[w == 0] = 1  # every product with the element is non-finite
+    dy = ints(r, (2, groups * co, *p.output_field()), np.float16)
+    y, dx = T.gpu_conv_fwd(p, x, w), T.gpu_conv_bwd(p, dy, w)
+    g = groups // 2
+    x2, dy2 = x.copy(), dy.copy()
+    x2[1, g * ci + 1, 4, 2] = value
+    dy2[1, g * co + 1, 2, 2] = value
+    for got, was, c in ((T.gpu_conv_fwd(p, x2, w), y, co), (T.gpu_conv_bwd(p, dy2, w), dx, ci)):
+        mine = slice(g * c, (g + 1) * c)
+        assert not np.isfinite(got[1, mine]).all()
+        same = np.isfinite(got[1, mine])
+        exact(got[1, mine][same], was[1, mine][same], "own group, elements the value does not reach")
+        got = got.copy()
+        got[1, mine] = was[1, mine]
+        exact(got, was, "other groups")
+    # and the next call is unaffected
+    exact(T.gpu_conv_fwd(p, x, w), y, "after")
+
+
+@pytest.mark.parametrize("groups,m,k,n", [(1, 197, 70, 103), (5, 197, 70, 103), (3, 8, 8, 8), (64, 33, 64, 130),
+                                          (2, 1, 513, 1), (7, 129, 65, 257), (4, 300, 1100, 40)])
+@pytest.mark.parametrize("dtype", ["half", "float", "quarter"])
+def test_ragged_and_grouped_products(gpu_ctx, groups, m, k, n, dtype):
+    """All operand layouts: rows of any length on both sides, one launch for all groups."""
+    r = T.rng(m + k + n)
+    av = r.integers(-1, 2, (groups, m, k)).astype(np.float64)
+    bv = r.integers(-1, 2, (groups, k, n)).astype(np.float64)
+    want = np.stack([av[g] @ bv[g] for g in range(groups)])
+    cast = {"half": lambda v: v.astype(np.float16), "float": lambda v: v.astype(np.float32),
+            "quarter": oracle.e4m3_encode}[dtype]
+    out = np.float32 if dtype == "float" else np.float16
+    for ta in (False, True):
+        for tb in (False, True):
+            a = cast(np.ascontiguousarray(av.transpose(0, 2, 1)) if ta else av)
+            b = cast(np.ascontiguousarray(bv.transpose(0, 2, 1)) if tb else bv)
+            exact(T.gpu_matmul(a, b, transpose_a=ta, transpose_b=tb, out_dtype=out), want, f"ta={ta} tb={tb}")
+    if dtype == "half":
+        c = ints(r, (groups, m, n), np.float32)
+        exact(T.gpu_matmul(cast(av), cast(bv), c, alpha=2.0, beta=-1.0, out_dtype=np.float32), 2 * want - c, "alpha, beta")
+
+
+@pytest.mark.parametrize("kernel,stride", [(7, 2), (3, 1), (3, 2), (1, 1), (5, 2)])
+@pytest.mark.parametrize("chans", [1, 2, 3, 4, 5, 7])
+def test_first_layer_weight_gradient(gpu_ctx, chans, kernel, stride):
+    """Few input channels: the gradient from the rearranged input (where a folded
+    filter row fits 64 elements) and from rounded-up channels (where it does not)."""
+    for width, co in ((13, 64), (22, 24), (16, 136)):
+        p = capi.ConvParams.make(batch=3, field=[11, width], kernel=[kernel, kernel], in_chans=chans, out_chans=co,
+                                 padding=kernel // 2, stride=stride)
+        spec = T.spec_from_params(p)
+        r = T.rng(chans * 10 + kernel)
+        x = ints(r, (3, chans, 11, width), np.float16)
+        w = ints(r, (1, co, chans, kernel, kernel), np.float16)
+        dy = ints(r, (3, co, *p.output_field()), np.float16)
+        dw16, dw32 = T.gpu_conv_wu(p, x, dy)
+        exact(dw32, oracle.conv_wu(spec, x, dy)[0], f"wu width {width} co {co}")
+        exact(dw16, dw32.astype(np.float16), "half gradient")
+        exact(T.gpu_conv_fwd(p, x, w), oracle.conv_fwd(spec, x, w), f"fwd width {width} co {co}")
