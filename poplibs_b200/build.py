@@ -8,6 +8,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
@@ -66,7 +67,25 @@ def build(force: bool = False, verbose: bool = False) -> str:
     if force or procs or not _newer(OUT, objs):
         cmd = [nvcc, "-shared", "-gencode", "arch=compute_100a,code=sm_100a", "-o", OUT] + objs
         subprocess.run(cmd, check=True)
+    build_binding(force)
     return OUT
+
+
+BINDING_SRC = os.path.join(CSRC, "python", "binding.c")
+BINDING_OUT = os.path.join(HERE, "_binding.so")
+
+
+def build_binding(force: bool = False):
+    """The CPython binding of the per-layer calls -> _binding.so, where the
+    interpreter's headers are installed (capi.py goes through ctypes without it)."""
+    include = sysconfig.get_paths()["include"]
+    if not os.path.exists(os.path.join(include, "Python.h")):
+        return None
+    if force or not _newer(BINDING_OUT, [BINDING_SRC, OUT, os.path.join(ROOT, "include", "poplibs_b200.h")]):
+        subprocess.run([shutil.which("gcc") or "gcc", "-O2", "-shared", "-fPIC", "-Wall", "-I" + include,
+                        "-I" + os.path.join(ROOT, "include"), BINDING_SRC, "-o", BINDING_OUT, "-L" + HERE,
+                        "-lpoplibs_b200", "-Wl,-rpath,$ORIGIN"], check=True)
+    return BINDING_OUT
 
 
 if __name__ == "__main__":

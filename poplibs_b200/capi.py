@@ -1,4 +1,5 @@
-"""ctypes binding of include/poplibs_b200.h (one-to-one, no logic of its own)."""
+"""Python binding of include/poplibs_b200.h (one-to-one, no logic of its own):
+ctypes, and for the calls made once per layer a CPython extension."""
 from __future__ import annotations
 
 import ctypes as C
@@ -131,6 +132,9 @@ class Plan(C.Structure):
 
 
 _LIB = None
+# The CPython binding of the per-layer calls (csrc/python/binding.c), None where it
+# was not built: the same entry points are then called through ctypes.
+_BINDING = None
 
 # every symbol include/poplibs_b200.h declares
 SYMBOLS = (
@@ -236,8 +240,16 @@ def lib():
     L.plb_matmul_plan.argtypes = [MP, PP]
     L.plb_conv_plan.argtypes = [CP, OP, i32, PP]
     L.plb_conv_wu_plan.argtypes = [CP, OP, PP]
+    _load_binding()
     _LIB = L
     return L
+
+
+def _load_binding():
+    global _BINDING
+    if os.path.exists(os.path.join(_HERE, "_binding.so")):
+        from . import _binding
+        _BINDING = _binding
 
 
 def _check(rc: int):
@@ -307,11 +319,13 @@ class Context:
             _check(lib().plb_context_create(device, C.byref(self._h)))
         else:
             _check(lib().plb_context_create_on_stream(device, C.c_void_p(stream), C.byref(self._h)))
+        self._ctx = self._h.value  # what the binding takes
 
     def close(self):
         if self._h:
             lib().plb_context_destroy(self._h)
             self._h = C.c_void_p()
+            self._ctx = 0
 
     def __del__(self):
         try:
@@ -343,6 +357,8 @@ class Context:
 
     # ---- hot path ---------------------------------------------------------
     def matmul(self, desc: MatmulDesc, a, b, c, d):
+        if _BINDING is not None:
+            return _check(_BINDING.matmul(self._ctx, desc, a, b, c, d))
         _check(lib().plb_matmul(self._h, C.byref(desc), _ptr(a), _ptr(b), _ptr(c), _ptr(d)))
 
     def matmul_host(self, desc: MatmulDesc, a, b, c, d, sync: bool = True):
@@ -352,6 +368,8 @@ class Context:
         _check(fn(self._h, C.byref(desc), _ptr(a), _ptr(b), _ptr(c), _ptr(d)))
 
     def conv_fwd(self, p: ConvParams, x, w, out, bias=None, opt: Optional[ConvOptions] = None):
+        if _BINDING is not None:
+            return _check(_BINDING.convolution(self._ctx, p, opt, x, w, bias, out, 0))
         _check(lib().plb_conv_fwd(self._h, C.byref(p), C.byref(opt) if opt else None,
                                   _ptr(x), _ptr(w), _ptr(bias), _ptr(out)))
 
@@ -365,21 +383,31 @@ class Context:
 
     def convolution(self, p: ConvParams, x, w, out, bias=None, opt: Optional[ConvOptions] = None,
                     transpose_and_flip_weights=False):
+        if _BINDING is not None:
+            return _check(_BINDING.convolution(self._ctx, p, opt, x, w, bias, out, int(transpose_and_flip_weights)))
         _check(lib().plb_convolution(self._h, C.byref(p), C.byref(opt) if opt else None, _ptr(x),
                                      _ptr(w), _ptr(bias), _ptr(out), int(transpose_and_flip_weights)))
 
     def conv_bwd(self, p: ConvParams, dy, w, dx, opt: Optional[ConvOptions] = None):
+        if _BINDING is not None:
+            return _check(_BINDING.conv_bwd(self._ctx, p, opt, dy, w, dx))
         _check(lib().plb_conv_bwd(self._h, C.byref(p), C.byref(opt) if opt else None,
                                   _ptr(dy), _ptr(w), _ptr(dx)))
 
     def conv_wu(self, p: ConvParams, x, dy, dw, dw_f32=None, opt: Optional[ConvOptions] = None):
+        if _BINDING is not None:
+            return _check(_BINDING.conv_wu(self._ctx, p, opt, x, dy, dw, dw_f32))
         _check(lib().plb_conv_wu(self._h, C.byref(p), C.byref(opt) if opt else None,
                                  _ptr(x), _ptr(dy), _ptr(dw), _ptr(dw_f32)))
 
     def scaled_add_to(self, dtype, weights, deltas_f32, scale, count):
+        if _BINDING is not None:
+            return _check(_BINDING.scaled_add_to(self._ctx, dtype, weights, deltas_f32, scale, count))
         _check(lib().plb_scaled_add_to(self._h, dtype, _ptr(weights), _ptr(deltas_f32), scale, count))
 
     def conv_bias_update(self, acts_dtype, out_grads, pixels, chans, bias_dtype, biases, scale):
+        if _BINDING is not None:
+            return _check(_BINDING.conv_bias_update(self._ctx, acts_dtype, out_grads, pixels, chans, bias_dtype, biases, scale))
         _check(lib().plb_conv_bias_update(self._h, acts_dtype, _ptr(out_grads), pixels, chans,
                                           bias_dtype, _ptr(biases), scale))
 
@@ -419,6 +447,8 @@ class Context:
 
     # ---- batch normalisation (device layout [pixels][chans]) -------------------
     def norm_moments(self, dtype, acts, pixels, chans, scale, centre, mean, power):
+        if _BINDING is not None:
+            return _check(_BINDING.norm_moments(self._ctx, dtype, acts, pixels, chans, scale, centre, mean, power))
         _check(lib().plb_norm_moments(self._h, dtype, _ptr(acts), pixels, chans, scale, _ptr(centre),
                                       _ptr(mean), _ptr(power)))
 
@@ -432,35 +462,51 @@ class Context:
 
     def norm_statistics(self, dtype, acts, pixels, chans, eps, scale_var, mean, inv_std, power=None):
         """Mean and 1/sigma per channel in one call (the default estimator)."""
+        if _BINDING is not None:
+            return _check(_BINDING.norm_statistics(self._ctx, dtype, acts, pixels, chans, eps, scale_var, mean, inv_std, power))
         _check(lib().plb_norm_statistics(self._h, dtype, _ptr(acts), pixels, chans, eps, scale_var, _ptr(mean),
                                          _ptr(inv_std), _ptr(power)))
 
     def norm_normalise(self, dtype, acts, mean, inv_std, gamma, beta, pixels, chans, whitened, out):
         """Whiten, then scale and shift, in one pass; `whitened` may be None."""
+        if _BINDING is not None:
+            return _check(_BINDING.norm_normalise(self._ctx, dtype, acts, mean, inv_std, gamma, beta, pixels, chans, whitened, out))
         _check(lib().plb_norm_normalise(self._h, dtype, _ptr(acts), _ptr(mean), _ptr(inv_std), _ptr(gamma),
                                         _ptr(beta), pixels, chans, _ptr(whitened), _ptr(out)))
 
     def norm_whiten(self, dtype, acts, mean, inv_std, pixels, chans, out):
+        if _BINDING is not None:
+            return _check(_BINDING.norm_whiten(self._ctx, dtype, acts, mean, inv_std, pixels, chans, out))
         _check(lib().plb_norm_whiten(self._h, dtype, _ptr(acts), _ptr(mean), _ptr(inv_std), pixels, chans,
                                      _ptr(out)))
 
     def norm_scale_shift(self, dtype, acts, scale, shift, pixels, chans, out):
+        if _BINDING is not None:
+            return _check(_BINDING.norm_scale_shift(self._ctx, dtype, acts, scale, shift, pixels, chans, out))
         _check(lib().plb_norm_scale_shift(self._h, dtype, _ptr(acts), _ptr(scale), _ptr(shift), pixels,
                                           chans, _ptr(out)))
 
     def norm_param_gradients(self, dtype, whitened, grads, pixels, chans, scale, gamma_delta, beta_delta,
                              gamma_delta_f32=None, beta_delta_f32=None):
+        if _BINDING is not None:
+            return _check(_BINDING.norm_param_gradients(self._ctx, dtype, whitened, grads, pixels, chans, scale, gamma_delta,
+                                                         beta_delta, gamma_delta_f32, beta_delta_f32))
         _check(lib().plb_norm_param_gradients(self._h, dtype, _ptr(whitened), _ptr(grads), pixels, chans,
                                               scale, _ptr(gamma_delta), _ptr(beta_delta),
                                               _ptr(gamma_delta_f32), _ptr(beta_delta_f32)))
 
     def norm_statistics_gradients(self, dtype, whitened, grads, inv_std, pixels, chans, out,
                                   var_delta=None, mean_delta=None):
+        if _BINDING is not None:
+            return _check(_BINDING.norm_statistics_gradients(self._ctx, dtype, whitened, grads, inv_std, var_delta, mean_delta,
+                                                              pixels, chans, out))
         _check(lib().plb_norm_statistics_gradients(self._h, dtype, _ptr(whitened), _ptr(grads),
                                                    _ptr(inv_std), _ptr(var_delta), _ptr(mean_delta),
                                                    pixels, chans, _ptr(out)))
 
     def cast_from_f32(self, dtype, dst, src, count):
+        if _BINDING is not None:
+            return _check(_BINDING.cast_from_f32(self._ctx, dtype, dst, src, count))
         _check(lib().plb_cast_from_f32(self._h, dtype, _ptr(dst), _ptr(src), count))
 
     # ---- layouts ----------------------------------------------------------
