@@ -11,7 +11,7 @@ namespace plb {
 
 // Which instance, and how it is launched.
 struct IgemmVariant {
-  bool fp8, a_mn, b_mn, resident, halo, pair;
+  bool fp8, a_mn, b_mn, resident, halo, pair, groups;
   int grid, resident_bytes;
   bool pdl;
 };
@@ -23,7 +23,7 @@ int launchIgemm128(plb_context *ctx, const CUtensorMap &ta, const CUtensorMap &t
 int launchIgemm256(plb_context *ctx, const CUtensorMap &ta, const CUtensorMap &tb, const CUtensorMap &tout,
                    const IgemmArgs &args, const IgemmVariant &v);
 
-template <int BN, bool kFp8, bool kAMn, bool kBMn, bool kResB, bool kHalo, bool k2Cta>
+template <int BN, bool kFp8, bool kAMn, bool kBMn, bool kResB, bool kHalo, bool k2Cta, bool kGroups>
 int launchInstance(plb_context *ctx, const CUtensorMap &ta, const CUtensorMap &tb,
                    const CUtensorMap &tout, const IgemmArgs &args, const IgemmVariant &v) {
   if constexpr (k2Cta && kBMn && BN < 128) {
@@ -32,7 +32,7 @@ int launchInstance(plb_context *ctx, const CUtensorMap &ta, const CUtensorMap &t
     using S = IgemmSmem<BN, kResB, k2Cta>;
     static bool configured[64] = {};
     static int max_clusters[64] = {};
-    auto kernel = igemm_kernel<BN, kFp8, kAMn, kBMn, kResB, kHalo, k2Cta>;
+    auto kernel = igemm_kernel<BN, kFp8, kAMn, kBMn, kResB, kHalo, k2Cta, kGroups>;
     const int dev = ctx->device & 63;
     if (!configured[dev]) {
       PLB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -92,27 +92,38 @@ int launchInstance(plb_context *ctx, const CUtensorMap &ta, const CUtensorMap &t
 template <int BN>
 int launchForTile(plb_context *ctx, const CUtensorMap &ta, const CUtensorMap &tb, const CUtensorMap &tout,
                   const IgemmArgs &args, const IgemmVariant &v) {
-#define PLB_LAUNCH(FP8, AMN, BMN, RES, HALO)                                                          \
-  return v.pair ? launchInstance<BN, FP8, AMN, BMN, RES, HALO, true>(ctx, ta, tb, tout, args, v)      \
-                : launchInstance<BN, FP8, AMN, BMN, RES, HALO, false>(ctx, ta, tb, tout, args, v)
-#define PLB_LAUNCH_OPERANDS(RES, HALO)                       \
-  if (v.fp8) PLB_LAUNCH(true, false, false, RES, HALO);      \
-  if (v.b_mn) PLB_LAUNCH(false, false, true, RES, HALO);     \
-  PLB_LAUNCH(false, false, false, RES, HALO)
+#define PLB_LAUNCH(FP8, AMN, BMN, RES, HALO, GROUPS)                                                          \
+  return v.pair ? launchInstance<BN, FP8, AMN, BMN, RES, HALO, true, GROUPS>(ctx, ta, tb, tout, args, v)      \
+                : launchInstance<BN, FP8, AMN, BMN, RES, HALO, false, GROUPS>(ctx, ta, tb, tout, args, v)
+#define PLB_LAUNCH_OPERANDS(RES, HALO, GROUPS)                       \
+  if (v.fp8) PLB_LAUNCH(true, false, false, RES, HALO, GROUPS);      \
+  if (v.b_mn) PLB_LAUNCH(false, false, true, RES, HALO, GROUPS);     \
+  PLB_LAUNCH(false, false, false, RES, HALO, GROUPS)
+  if (v.a_mn && v.groups) {
+    if (v.b_mn) PLB_LAUNCH(false, true, true, false, false, true);
+    PLB_LAUNCH(false, true, false, false, false, true);
+  }
   if (v.a_mn) {
-    if (v.b_mn) PLB_LAUNCH(false, true, true, false, false);
-    PLB_LAUNCH(false, true, false, false, false);
+    if (v.b_mn) PLB_LAUNCH(false, true, true, false, false, false);
+    PLB_LAUNCH(false, true, false, false, false, false);
+  }
+  // (several groups never have resident weights)
+  if (v.groups && v.halo) {
+    PLB_LAUNCH_OPERANDS(false, true, true);
+  }
+  if (v.groups) {
+    PLB_LAUNCH_OPERANDS(false, false, true);
   }
   if (v.halo && v.resident) {
-    PLB_LAUNCH_OPERANDS(true, true);
+    PLB_LAUNCH_OPERANDS(true, true, false);
   }
   if (v.halo) {
-    PLB_LAUNCH_OPERANDS(false, true);
+    PLB_LAUNCH_OPERANDS(false, true, false);
   }
   if (v.resident) {
-    PLB_LAUNCH_OPERANDS(true, false);
+    PLB_LAUNCH_OPERANDS(true, false, false);
   }
-  PLB_LAUNCH_OPERANDS(false, false);
+  PLB_LAUNCH_OPERANDS(false, false, false);
 #undef PLB_LAUNCH_OPERANDS
 #undef PLB_LAUNCH
 }

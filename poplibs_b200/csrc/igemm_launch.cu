@@ -322,6 +322,26 @@ int launchIgemm(plb_context *ctx, const IgemmProblem &p, const plb_plan &plan) {
     out3[2] = halo ? h : n;
   };
   const int groups = std::max(1, p.groups);
+  // The kernel instance for groups, also taken where a short K (one chunk, not
+  // full) saves instructions on every tile.  Its copies and stores carry the group
+  // coordinate whatever the number of groups, so the tensor maps of activations
+  // and output must have the dimension.
+  const int k_chunks = (p.k_per_tap + k_elems_per_stage - 1) / k_elems_per_stage;
+  const int k_elems_mma = 32 / elem;
+  const int k_last = (p.k_per_tap - (k_chunks - 1) * k_elems_per_stage + k_elems_mma - 1) / k_elems_mma;
+  const bool with_groups =
+      groups > 1 || (!plan.resident_weights && k_chunks == 1 && k_last < 4 && p.taps_h * p.taps_w > 1);
+  // Rows of an activation box.  A single tile along the slowest dimension of the
+  // box loads only what the output needs of it: a product of 16 rows would
+  // otherwise spend most of its copy time filling 112 rows with zeros.  (What the
+  // unused rows of shared memory hold reaches unused accumulator rows alone.)
+  int load_w = plan.box_w, load_h = plan.box_h, load_n = plan.box_n;
+  if (!plan.cta_pair) {
+    int *slowest = halo ? (load_h > 1 ? &load_h : load_n > 1 ? &load_n : &load_w)
+                        : (load_n > 1 ? &load_n : load_h > 1 ? &load_h : &load_w);
+    *slowest = std::min(*slowest, slowest == &load_w ? p.out_w : slowest == &load_h ? p.out_h : p.out_n);
+  }
+  const int a_blocks = p.a_mn ? (load_w + 63) / 64 : 0;
   CUtensorMap ta, tb;
   if (p.a_mn) {
     // [group][k][m], rows of m: boxes of 64 K rows x 64 output rows
@@ -334,9 +354,9 @@ int launchIgemm(plb_context *ctx, const IgemmProblem &p, const plb_plan &plan) {
     uint64_t dims[5] = {p.act_dims[0]}, strides[4], b3[3], e3[3];
     uint32_t box[5] = {uint32_t(k_elems_per_stage)}, es[5] = {1};
     int rank = 1;
-    if (groups > 1) {
+    if (with_groups) {
       dims[1] = uint64_t(groups);
-      strides[0] = uint64_t(p.act_group_stride);
+      strides[0] = groups > 1 ? p.act_group_stride : p.act_strides[0];
       box[1] = es[1] = 1;
       rank = 2;
     }
@@ -344,8 +364,8 @@ int launchIgemm(plb_context *ctx, const IgemmProblem &p, const plb_plan &plan) {
     strides[rank - 1] = p.act_strides[0];
     strides[rank] = halo ? p.act_strides[2] : p.act_strides[1];
     strides[rank + 1] = halo ? p.act_strides[1] : p.act_strides[2];
-    order(uint64_t((plan.box_w - 1) * p.stride_w + 1),
-          uint64_t((plan.box_h + plan.halo_rows - 1) * p.stride_h + 1), uint64_t(plan.box_n), b3);
+    order(uint64_t((load_w - 1) * p.stride_w + 1), uint64_t((load_h + plan.halo_rows - 1) * p.stride_h + 1),
+          uint64_t(load_n), b3);
     order(uint64_t(p.stride_w), uint64_t(p.stride_h), 1, e3);
     for (int i = 0; i < 3; ++i) {
       box[rank + i] = uint32_t(b3[i]);
@@ -411,9 +431,9 @@ int launchIgemm(plb_context *ctx, const IgemmProblem &p, const plb_plan &plan) {
     uint64_t dims[5] = {uint64_t(p.n_total)}, strides[4];
     uint32_t box[5] = {32u};
     int rank = 1;
-    if (groups > 1) {
+    if (with_groups) {
       dims[1] = uint64_t(groups);
-      strides[0] = uint64_t(p.out_group_stride) * out_es;
+      strides[0] = uint64_t(groups > 1 ? p.out_group_stride : p.ldc) * out_es;
       box[1] = 1;
       rank = 2;
     }
@@ -447,9 +467,8 @@ int launchIgemm(plb_context *ctx, const IgemmProblem &p, const plb_plan &plan) {
   a.n_total = p.n_total;
   a.taps_h = p.taps_h;
   a.taps_w = p.taps_w;
-  a.k_chunks = (p.k_per_tap + k_elems_per_stage - 1) / k_elems_per_stage;
-  const int k_elems_mma = 32 / elem;
-  a.k_last = (p.k_per_tap - (a.k_chunks - 1) * k_elems_per_stage + k_elems_mma - 1) / k_elems_mma;
+  a.k_chunks = k_chunks;
+  a.k_last = k_last;
   a.groups = groups;
   a.fd_groups = make_fastdiv(uint32_t(groups));
   a.out_group_stride = groups > 1 ? p.out_group_stride : 0;
@@ -478,6 +497,9 @@ int launchIgemm(plb_context *ctx, const IgemmProblem &p, const plb_plan &plan) {
   a.fd_inner = make_fastdiv(uint32_t(std::max(1, a.h_outer ? a.tiles_n : a.tiles_h)));
   a.a_stage_bytes = plan.box_w * plan.box_n * (plan.box_h + plan.halo_rows) * kStageKBytes;
   a.b_tiles_per_stage = (halo && !plan.resident_weights) ? p.taps_h : 1;
+  a.a_blocks = a_blocks;
+  a.stage_tx_bytes = (p.a_mn ? a_blocks * 64 * 64 * 2 : load_w * load_n * (load_h + plan.halo_rows) * kStageKBytes) +
+                     (plan.resident_weights ? 0 : a.b_tiles_per_stage * a.b_box_bytes);
   a.halo_step_bytes = p.dil_h * plan.box_w * plan.box_n * kStageKBytes;
   a.num_stages = plan.stages;
   // Short tiles (few tensor-core instructions each) are bound by what one
@@ -524,7 +546,7 @@ int launchIgemm(plb_context *ctx, const IgemmProblem &p, const plb_plan &plan) {
   a.trace = ctx->trace;
 
   const bool pdl = (p.plan_flags & PLB_PLAN_NO_PDL) == 0;
-  const IgemmVariant variant{p.fp8, p.a_mn, p.b_mn, plan.resident_weights != 0, halo, plan.cta_pair != 0, plan.grid,
+  const IgemmVariant variant{p.fp8, p.a_mn, p.b_mn, plan.resident_weights != 0, halo, plan.cta_pair != 0, with_groups, plan.grid,
                              resident_bytes, pdl};
   int rc = PLB_OK;
   switch (plan.tile_n) {

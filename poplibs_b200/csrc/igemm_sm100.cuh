@@ -71,6 +71,8 @@ struct IgemmArgs {
   // serves all taps_h vertical taps (row r starts halo_step_bytes * r further on).
   int halo_step_bytes;
   int a_stage_bytes;        // bytes of activations per stage
+  int stage_tx_bytes;       // bytes one CTA's copies bring into a stage
+  int a_blocks;             // transposed A: blocks of 64 output rows that exist (1 or 2)
   int b_tiles_per_stage;    // streamed weight tiles per stage (taps_h with a halo strip, else 1)
   // ---- groups ---------------------------------------------------------------
   // Independent contractions of one shape in one launch (channel groups of a
@@ -188,6 +190,9 @@ struct IgemmSmem {
 //       by whole 8-row groups, which the descriptor's start address can express.
 //       Cuts the activation traffic of a KxK filter K-fold.  Streamed weights
 //       (no kResB) then travel as taps_h tiles per stage.
+// kGroups: several groups (args.groups), and a last K chunk of fewer than four
+//       instructions.  Without it neither is looked at: the tests for them cost a
+//       product of eight K steps 0.9 of 4.5 us.
 // k2Cta: the kernel is launched in clusters of two CTAs that share one
 //       tcgen05.mma of 256 rows (cta_group::2): the CTA of rank r works on M
 //       tile 2 * pair + r, loads its own activations and rows
@@ -199,7 +204,7 @@ struct IgemmSmem {
 //       CTA halves their shared-memory fill and operand fetch per FLOP, and
 //       the instruction is twice as large, which matters because a
 //       128-row instruction is bound by operand fetch, not by arithmetic.
-template <int BN, bool kFp8, bool kAMn, bool kBMn, bool kResB, bool kHalo, bool k2Cta>
+template <int BN, bool kFp8, bool kAMn, bool kBMn, bool kResB, bool kHalo, bool k2Cta, bool kGroups>
 __global__ void __launch_bounds__(kIgemmThreads, 1)
 igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
              const __grid_constant__ CUtensorMap tm_out, const IgemmArgs args) {
@@ -292,7 +297,7 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
   // last one is padded: its copies read zeros and its stores are clipped).
   const int m_tiles = args.tiles_w * args.tiles_h * args.tiles_n;
   const int m_units = k2Cta ? (m_tiles + 1) / 2 : m_tiles;
-  const int total_tiles = m_units * args.n_tiles * args.groups;
+  const int total_tiles = m_units * args.n_tiles * (kGroups ? args.groups : 1);
   // a unit of work is an output tile, or with split-K one of its K ranges
   // (the splits of a tile are consecutive units, i.e. run on different CTAs)
   const int total_units = total_tiles * args.split_k;
@@ -326,7 +331,7 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
       it_end = int(fast_div(uint32_t(p_iters * (split + 1)), args.fd_split));
     }
     group = 0;
-    if (args.groups > 1) {
+    if (kGroups) {
       const int t = int(fast_div(uint32_t(tile), args.fd_groups));
       group = tile - t * args.groups;
       tile = t;
@@ -381,7 +386,7 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
   auto load_b = [&](uint32_t dst, uint32_t bar, int group, int r, int s, int kc, int n_col, bool prefetch) {
     const int b_tap = ((args.flip_h ? args.taps_h - 1 - r : r) * args.tap_step_h + args.tap_first_h) * args.tap_pitch_h +
                       (args.flip_w ? args.taps_w - 1 - s : s) * args.tap_step_w + args.tap_first_w +
-                      group * args.taps_stored;
+                      (kGroups ? group * args.taps_stored : 0);
     // a CTA of a pair loads its half of the tile's N rows / columns
     constexpr int kMyN = k2Cta ? BN / 2 : BN;
     const int my_col = n_col + (kBMn ? int(cta_rank) * kMyN : k2Cta ? int(cta_rank) * (args.n_mma / 2) : 0);
@@ -417,6 +422,77 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
   // which alone announces the byte count (both CTAs' shares)
   constexpr uint32_t kPairFactor = k2Cta ? 2u : 1u;
 
+  // One pipeline step: the activation box and, unless the weights are
+  // resident, the weight tile(s) of step (r, s, kc) -> stage memory at a_dst
+  // (or, before the predecessor kernel is known to have finished, only
+  // towards L2).
+  auto issue_step = [&](bool prefetch, uint32_t a_dst, uint32_t full, int group, int r, int s, int kc,
+                        int w_base, int h_base, int n0, int n_col) {
+    if constexpr (kAMn) {
+      // [k][m] rows of one group: two boxes of 64 K rows x 64 output rows
+        for (int j = 0; j < args.a_blocks; ++j) {
+        if (prefetch)
+          tma_prefetch_l2_3d(&tm_a, w_base + j * 64, kc * 64, group);
+        else if constexpr (k2Cta)
+          tma_load_3d_pair(a_dst + j * (64 * kStageKBytes), &tm_a, full, w_base + j * 64, kc * 64, group);
+        else
+          tma_load_3d(a_dst + j * (64 * kStageKBytes), &tm_a, full, w_base + j * 64, kc * 64, group);
+      }
+    } else {
+      const int cw = w_base + s * args.dil_w, ch = h_base + r * args.dil_h;
+      const int c2 = args.h_outer ? n0 : ch, c3 = args.h_outer ? ch : n0;
+      const int ck = kc * kElemsPerStage;
+      if (kGroups) {
+        if (prefetch)
+          tma_prefetch_l2_5d(&tm_a, ck, group, cw, c2, c3);
+        else if constexpr (k2Cta)
+          tma_load_5d_pair(a_dst, &tm_a, full, ck, group, cw, c2, c3);
+        else
+          tma_load_5d(a_dst, &tm_a, full, ck, group, cw, c2, c3);
+      } else if (prefetch) {
+        tma_prefetch_l2_4d(&tm_a, ck, cw, c2, c3);
+      } else if constexpr (k2Cta) {
+        tma_load_4d_pair(a_dst, &tm_a, full, ck, cw, c2, c3);
+      } else {
+        tma_load_4d(a_dst, &tm_a, full, ck, cw, c2, c3);
+      }
+    }
+    if constexpr (!kResB) {
+      // with a halo strip the stage carries the weight tiles of every filter row
+      const int row_taps = kHalo ? args.taps_h : 1;
+      for (int rr = 0; rr < row_taps; ++rr)
+        load_b(a_dst + args.a_stage_bytes + rr * S::kBBytes, full, group, kHalo ? rr : r, s, kc, n_col,
+               prefetch);
+    }
+  };
+  // The pipeline is empty when the kernel starts, and a copy costs its issuing
+  // thread a few hundred cycles: the first unit's first steps, one per stage, are
+  // issued by as many warps at once, the epilogue warps, which have nothing to do
+  // yet.  (With resident weights those load the weights, and the producers start
+  // on the activations themselves.)
+  int first_steps = 0;
+  int f_tile = 0, f_group = 0, f_split = 0, f_begin = 0, f_end = 0;
+  if (first_unit < total_units) {
+    unit_coords(first_unit, f_tile, f_group, f_split, f_begin, f_end);
+    first_steps = min(f_end - f_begin, kStages);
+  }
+  // Step f_begin + i of the first unit towards L2 while the predecessor kernel may
+  // still be running, and with `load`, once it has finished, into stage i.
+  auto first_step = [&](int i, bool load) {
+    int m_idx, n_idx, w0, h0, n0, r, s, kc;
+    tile_coords(f_tile, m_idx, n_idx);
+    tile_origin(m_idx, w0, h0, n0);
+    step_coords(f_begin + i, r, s, kc);
+    const uint32_t dst = smem_base + i * stage_bytes, full = lead_bar(full_bar(i));
+    const int w_base = w0 * args.stride_w - args.pad_w, h_base = h0 * args.stride_h - args.pad_h;
+    issue_step(true, dst, full, f_group, r, s, kc, w_base, h_base, n0, n_idx * BN);
+    if (!load) return;
+    pdl_wait();
+    if (leader)
+      mbar_expect_tx(full_bar(i), kPairFactor * uint32_t(args.stage_tx_bytes));
+    issue_step(false, dst, full, f_group, r, s, kc, w_base, h_base, n0, n_idx * BN);
+  };
+
   if (warp < P) {
     // ===================== TMA producers =====================
     if (elect_one()) {
@@ -426,67 +502,8 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
       int turn = 0;            // (global K step) mod P
       bool ok = true;
       [[maybe_unused]] int trace_slot = 0;
-      // One pipeline step: the activation box and, unless the weights are
-      // resident, the weight tile(s) of step (r, s, kc) -> stage memory at a_dst
-      // (or, before the predecessor kernel is known to have finished, only
-      // towards L2).
-      auto issue_step = [&](bool prefetch, uint32_t a_dst, uint32_t full, int group, int r, int s, int kc,
-                            int w_base, int h_base, int n0, int n_col) {
-        if constexpr (kAMn) {
-          // [k][m] rows of one group: two boxes of 64 K rows x 64 output rows
-#pragma unroll
-          for (int j = 0; j < 2; ++j) {
-            if (prefetch)
-              tma_prefetch_l2_3d(&tm_a, w_base + j * 64, kc * 64, group);
-            else if constexpr (k2Cta)
-              tma_load_3d_pair(a_dst + j * (64 * kStageKBytes), &tm_a, full, w_base + j * 64, kc * 64, group);
-            else
-              tma_load_3d(a_dst + j * (64 * kStageKBytes), &tm_a, full, w_base + j * 64, kc * 64, group);
-          }
-        } else {
-          const int cw = w_base + s * args.dil_w, ch = h_base + r * args.dil_h;
-          const int c2 = args.h_outer ? n0 : ch, c3 = args.h_outer ? ch : n0;
-          const int ck = kc * kElemsPerStage;
-          if (args.groups > 1) {
-            if (prefetch)
-              tma_prefetch_l2_5d(&tm_a, ck, group, cw, c2, c3);
-            else if constexpr (k2Cta)
-              tma_load_5d_pair(a_dst, &tm_a, full, ck, group, cw, c2, c3);
-            else
-              tma_load_5d(a_dst, &tm_a, full, ck, group, cw, c2, c3);
-          } else if (prefetch) {
-            tma_prefetch_l2_4d(&tm_a, ck, cw, c2, c3);
-          } else if constexpr (k2Cta) {
-            tma_load_4d_pair(a_dst, &tm_a, full, ck, cw, c2, c3);
-          } else {
-            tma_load_4d(a_dst, &tm_a, full, ck, cw, c2, c3);
-          }
-        }
-        if constexpr (!kResB) {
-          // with a halo strip the stage carries the weight tiles of every filter row
-          const int row_taps = kHalo ? args.taps_h : 1;
-          for (int rr = 0; rr < row_taps; ++rr)
-            load_b(a_dst + args.a_stage_bytes + rr * S::kBBytes, full, group, kHalo ? rr : r, s, kc, n_col,
-                   prefetch);
-        }
-      };
-      // While the predecessor kernel may still be running: pull the boxes of
-      // this producer's first steps towards L2.
-      if (first_unit < total_units) {
-        int tile, group, split, it_begin, it_end;
-        unit_coords(first_unit, tile, group, split, it_begin, it_end);
-        int m_idx, n_idx;
-        tile_coords(tile, m_idx, n_idx);
-        int w0, h0, n0;
-        tile_origin(m_idx, w0, h0, n0);
-        const int steps = min(it_end, it_begin + kStages);
-        for (int it = it_begin + me; it < steps; it += P) {
-          int r, s, kc;
-          step_coords(it, r, s, kc);
-          issue_step(true, 0u, 0u, group, r, s, kc, w0 * args.stride_w - args.pad_w,
-                     h0 * args.stride_h - args.pad_h, n0, n_idx * BN);
-        }
-      }
+      if constexpr (kResB)
+        for (int i = me; i < first_steps; i += P) first_step(i, false);
       pdl_wait();
       if (me == 0) PLB_TRACE_STAMP(2, 4002);
       for (int unit = first_unit; unit < total_units && ok; unit += unit_stride) {
@@ -504,7 +521,15 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
         int r = 0, s = 0, kc = 0;
         if (it_begin != 0) step_coords(it_begin, r, s, kc);
         for (int it = it_begin; it < it_end; ++it) {
-          if (turn == me) {
+          // (the first unit's first steps are on their way already)
+          const bool issued = !kResB && unit == first_unit && it - it_begin < first_steps;
+          if (turn == me && issued) {
+            stage += P;
+            if (stage >= kStages) {
+              stage -= kStages;
+              phase ^= 1u;
+            }
+          } else if (turn == me) {
             if (me == 0) { PLB_TRACE_STAMP(0, trace_slot); ++trace_slot; }
             if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag)) {
               atomicCAS(args.status, kStatusOk, kStatusProducerTimeout);
@@ -513,10 +538,7 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
             }
             if (me == 0) { PLB_TRACE_STAMP(0, trace_slot); ++trace_slot; }
             const uint32_t a_dst = smem_base + stage * stage_bytes;
-            if (leader)
-              mbar_expect_tx(full_bar(stage),
-                             kPairFactor * uint32_t(args.a_stage_bytes +
-                                                    (kResB ? 0 : args.b_tiles_per_stage * args.b_box_bytes)));
+            if (leader) mbar_expect_tx(full_bar(stage), kPairFactor * uint32_t(args.stage_tx_bytes));
             const uint32_t full = lead_bar(full_bar(stage));
             issue_step(false, a_dst, full, group, r, s, kc, w_base, h_base, n0, n_col);
             if (me == 0) { PLB_TRACE_STAMP(0, trace_slot); ++trace_slot; }
@@ -630,21 +652,24 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
           else
             b_desc = b_desc0 + stage_off16;
           const int row_taps = kHalo ? args.taps_h : 1;
+          // one instruction consumes 32 bytes of K: the start address advances inside
+          // the swizzle span (K-major) or by 16 rows (MN-major)
+          auto mma = [&](int r, int k) {
+            const uint64_t a_k = a_desc + uint64_t(kAMn ? k * ((16 * kStageKBytes) >> 4) : k * 2);
+            const uint64_t b_k = b_desc + uint64_t(kBMn ? k * ((16 * kStageKBytes) >> 4) : k * 2);
+            if constexpr (k2Cta)
+              umma_ss_pair<kFp8>(d_tmem, a_k, b_k, idesc, ((it - it_begin) | r | k) != 0 ? 1u : 0u);
+            else
+              umma_ss<kFp8>(d_tmem, a_k, b_k, idesc, ((it - it_begin) | r | k) != 0 ? 1u : 0u);
+          };
           // (the K range past the last channel holds zeros: no instruction for it)
-          const int k_steps = kc == args.k_chunks - 1 ? args.k_last : 4;
+          const int k_steps = kGroups && kc == args.k_chunks - 1 ? args.k_last : 4;
           for (int r = 0; r < row_taps; ++r) {
+            if (k_steps == 4) {
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              if (k >= k_steps) break;
-              // one instruction consumes 32 bytes of K: advance the start address
-              // inside the swizzle span (K-major) or by 16 rows (MN-major B)
-              const uint64_t a_k = a_desc + uint64_t(kAMn ? k * ((16 * kStageKBytes) >> 4) : k * 2);
-              const uint64_t b_k =
-                  b_desc + uint64_t(kBMn ? k * ((16 * kStageKBytes) >> 4) : k * 2);
-              if constexpr (k2Cta)
-                umma_ss_pair<kFp8>(d_tmem, a_k, b_k, idesc, ((it - it_begin) | r | k) != 0 ? 1u : 0u);
-              else
-                umma_ss<kFp8>(d_tmem, a_k, b_k, idesc, ((it - it_begin) | r | k) != 0 ? 1u : 0u);
+              for (int k = 0; k < 4; ++k) mma(r, k);
+            } else {
+              for (int k = 0; k < k_steps; ++k) mma(r, k);
             }
             if constexpr (kHalo) {
               // next filter row: the strip shifted by whole 8-row groups; its
@@ -742,6 +767,11 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
         if (warp == 4) PLB_TRACE_STAMP(2, 4012);
       }
       __syncwarp();
+    } else {
+      if (lane == 0 && warp - 4 < first_steps) {
+        first_step(warp - 4, true);
+      }
+      __syncwarp();
     }
     pdl_wait();
     for (int unit = first_unit + group * unit_stride; unit < total_units;
@@ -758,7 +788,7 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
       const long long pixel = (static_cast<long long>(on) * args.out_h + oh) * args.out_w + ow;
       const long long out_off = static_cast<long long>(on) * args.out_stride_n +
                                 static_cast<long long>(oh) * args.out_stride_h +
-                                static_cast<long long>(ow) * args.ldc + cgroup * args.out_group_stride;
+                                static_cast<long long>(ow) * args.ldc + (kGroups ? cgroup * args.out_group_stride : 0);
       if (stamp) PLB_TRACE_STAMP(2, local_tile * 4 + 0);
       if (!mbar_wait(tmem_full_bar(acc), acc_phase, abort_flag)) {
         atomicCAS(args.status, kStatusOk, kStatusEpilogueTimeout);
@@ -894,7 +924,7 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
             if (box_ok) {
               const uint32_t src = whole_rows ? buf : wbuf;
               const int c2 = args.h_outer ? n0 + qn : h0 + qh, c3 = args.h_outer ? h0 + qh : n0 + qn;
-              if (args.groups > 1)
+              if (kGroups)
                 tma_store_5d(&tm_out, src, col0, cgroup, w0 + qw, c2, c3);
               else
                 tma_store_4d(&tm_out, src, col0, w0 + qw, c2, c3);
