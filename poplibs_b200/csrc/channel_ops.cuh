@@ -83,8 +83,9 @@ struct ChanWalk {
 };
 
 // `per_sm`: blocks of `threads` threads wanted per SM once there is work for them.
+// `most_slabs`: a cap on the slabs besides that (0: none).
 inline ChanWalk chanWalk(const plb_context *ctx, uint64_t rows, uint32_t chans, uint32_t V, uint32_t threads,
-                         uint32_t per_sm, dim3 *grid) {
+                         uint32_t per_sm, uint64_t most_slabs, dim3 *grid) {
   ChanWalk w{};
   w.chans = chans;
   uint32_t g = chans, t = V;  // gcd
@@ -108,7 +109,8 @@ inline ChanWalk chanWalk(const plb_context *ctx, uint64_t rows, uint32_t chans, 
   // one super-row per thread while that leaves SMs idle, then a grid that is
   // resident at once and walks
   const uint64_t want = std::max<uint64_t>(1, (w.full + row_lanes - 1) / row_lanes);
-  const uint64_t cap = std::max<uint64_t>(1, uint64_t(ctx->sm_count) * per_sm / cols);
+  uint64_t cap = std::max<uint64_t>(1, uint64_t(ctx->sm_count) * per_sm / cols);
+  if (most_slabs) cap = std::min(cap, most_slabs);
   w.slabs = uint32_t(std::min<uint64_t>(std::min(want, cap), 65535));
   *grid = dim3(cols, w.slabs);
   return w;
@@ -137,9 +139,11 @@ struct ChanFinish {
   // bias[c] += a
   void *bias;
   int bias_half;
+  int totals_fit;  // (set by chanSums) the last block can hold all column totals in shared memory
 };
 
 constexpr int kChanSumThreads = 1024;
+constexpr int kChanSumQuads = kChanSumThreads + kChanSumThreads / 2;  // float4s of the last block's table
 
 __device__ __forceinline__ void storeChan(void *p, int is_half, uint32_t c, float v) {
   if (is_half)
@@ -154,8 +158,8 @@ __device__ __forceinline__ void storeChan(void *p, int is_half, uint32_t c, floa
 // not depend on timing.  One block of 1024 threads per SM: few rows for the last
 // block to add, and 4 vectors per thread in flight are 9.7 MB over the device,
 // above the 5 MB that 6.5 TB/s times the memory latency asks for.
-// The last block's share is latency: it takes four channels per thread so that
-// all 148 rows are requested at once (one channel per thread: 3 us more at 128).
+// The last block's share is latency: it takes four columns per thread so that
+// all rows are requested at once (one channel per thread: 3 us more at 128).
 // Sums of 200704 x 128 halves (51 MB): 40.5 us as two kernels whose second read
 // its 1184 partial rows one after the other, now 14.7; of 200704 x 512 (205 MB):
 // 54.9 us, now 38.0 (5.4 TB/s; a read-only stream gets 5.6 here).
@@ -168,7 +172,8 @@ chanSumsKernel(const T *__restrict__ x, const T *__restrict__ y, const T *__rest
   using Raw = typename Vec::Raw;
   constexpr bool kHasA = kMode != kSumCentredXX, kHasB = kMode != kSumX, kHasY = kMode == kSumXYAndY;
   constexpr int kUnroll = kHasY ? 2 : 4;
-  __shared__ __align__(16) float red[32 * 32 * V];
+  extern __shared__ float4 chan_smem[];
+  float *red = reinterpret_cast<float *>(chan_smem);
   __shared__ unsigned last;
   pdl_launch_dependents();
   const uint32_t lanes = 1u << w.vec_lanes_log2, row_lanes = kChanSumThreads >> w.vec_lanes_log2;
@@ -241,28 +246,42 @@ chanSumsKernel(const T *__restrict__ x, const T *__restrict__ y, const T *__rest
         }
     }
   }
-  // Threads of a warp that share a vector first (a fixed tree of shuffles), then
-  // the warps in order.
+  // Threads of a warp that share a vector first, then the warps: `per` neighbouring
+  // threads share the 32 warps' values of a column (both sums' columns at once; a
+  // row pitch of cols + 1 words keeps them in different banks).  Every tree is
+  // fixed, so the result does not depend on timing.
   const uint32_t warp = threadIdx.x >> 5, cols = lanes * V;
   const uint32_t block_col0 = blockIdx.x * cols;
-  auto reduce_block = [&](float (&s)[V], float *partial) {
+  {
+    constexpr uint32_t kSums = (kHasA ? 1 : 0) + (kHasB ? 1 : 0);
+    float *rb = red + (kHasA ? 32 * (cols + 1) : 0);
 #pragma unroll
     for (int j = 0; j < V; ++j)
-      for (uint32_t d = 16; d >= lanes; d >>= 1) s[j] += __shfl_xor_sync(0xffffffffu, s[j], d);
-    __syncthreads();
+      for (uint32_t d = 16; d >= lanes; d >>= 1) {
+        if constexpr (kHasA) a[j] += __shfl_xor_sync(0xffffffffu, a[j], d);
+        if constexpr (kHasB) b[j] += __shfl_xor_sync(0xffffffffu, b[j], d);
+      }
     if ((threadIdx.x & 31) < lanes)
 #pragma unroll
-      for (int j = 0; j < V; ++j) red[(warp * lanes + vx) * V + j] = s[j];
+      for (int j = 0; j < V; ++j) {
+        if constexpr (kHasA) red[warp * (cols + 1) + vx * V + j] = a[j];
+        if constexpr (kHasB) rb[warp * (cols + 1) + vx * V + j] = b[j];
+      }
     __syncthreads();
-    if (threadIdx.x < cols && block_col0 + threadIdx.x < pitch) {
-      float t = 0.f;
-#pragma unroll 8
-      for (int k = 0; k < kChanSumThreads / 32; ++k) t += red[k * cols + threadIdx.x];
-      partial[size_t(blockIdx.y) * pitch + block_col0 + threadIdx.x] = t;
+    const uint32_t items = kSums * cols, per = min(32u, kChanSumThreads / items);  // powers of two
+    const uint32_t item = threadIdx.x / per, part = threadIdx.x & (per - 1), rows = 32 / per;
+    float t = 0.f;
+    const bool second = kHasA && item >= cols;
+    const uint32_t col = second ? item - cols : item;
+    if (item < items) {
+      const float *r = (second ? rb : red) + part * rows * (cols + 1) + col;
+#pragma unroll 4
+      for (uint32_t k = 0; k < rows; ++k) t += r[k * (cols + 1)];
     }
-  };
-  if constexpr (kHasA) reduce_block(a, partial_a);
-  if constexpr (kHasB) reduce_block(b, partial_b);
+    for (uint32_t d = per >> 1; d >= 1; d >>= 1) t += __shfl_xor_sync(0xffffffffu, t, d);
+    if (part == 0 && item < items && block_col0 + col < pitch)
+      (second || !kHasA ? partial_b : partial_a)[size_t(blockIdx.y) * pitch + block_col0 + col] = t;
+  }
   __syncthreads();
   if (threadIdx.x == 0) {
     // one thread's release publishes the block's stores (the barrier above orders
@@ -295,88 +314,98 @@ chanSumsKernel(const T *__restrict__ x, const T *__restrict__ y, const T *__rest
       storeChan(fin.bias, fin.bias_half, c, old + va);
     }
   };
-  // [slabs * fold][chans]: channels across threads, rows shared out between the
-  // threads of a channel, so that all rows are in flight at once.
-  const uint32_t parts = gridDim.y * w.fold;
   if constexpr (V > 1) {
-    if (w.fold == 1 && w.chans % 4 == 0) {
-      // four channels per thread
-      uint32_t ql_log2 = 3;
-      while (ql_log2 < 8 && (4u << ql_log2) < w.chans) ++ql_log2;
+    if (fin.totals_fit) {
+      // The slabs' rows of `pitch` columns: four columns per thread, the rows shared
+      // out between the threads of a column so that all are in flight at once, their
+      // sums added through shared memory, then the rows of a super-row.
+      const uint32_t quads = uint32_t(pitch / 4);
+      uint32_t ql_log2 = 1;
+      while (ql_log2 < 8 && (1u << ql_log2) < quads) ++ql_log2;
       const uint32_t ql = 1u << ql_log2, part_lanes = kChanSumThreads >> ql_log2;
       const uint32_t cl = threadIdx.x & (ql - 1), pl = threadIdx.x >> ql_log2;
-      for (uint32_t q0 = 0; q0 < w.chans / 4; q0 += ql) {
+      // (rows of ql + 1: neighbouring threads' reads below fall into different banks)
+      float4 *sums_a = chan_smem, *sums_b = sums_a + kChanSumQuads;
+      float *total_a = red + 8 * kChanSumQuads, *total_b = total_a + pitch;
+      auto take = [](float4 &s, const float4 &v) {
+        s.x += v.x;
+        s.y += v.y;
+        s.z += v.z;
+        s.w += v.w;
+      };
+      for (uint32_t q0 = 0; q0 < quads; q0 += ql) {
         float4 sa = make_float4(0.f, 0.f, 0.f, 0.f), sb = sa;
-        auto take = [](float4 &s, const float4 &v) {
-          s.x += v.x;
-          s.y += v.y;
-          s.z += v.z;
-          s.w += v.w;
-        };
-        if (q0 + cl < w.chans / 4) {
-          const size_t col = size_t(q0 + cl) * 4;
+        if (q0 + cl < quads) {
+          const size_t at = size_t(q0 + cl) * 4;
 #pragma unroll 4
-          for (uint32_t k = pl; k < parts; k += part_lanes) {
-            if constexpr (kHasA) take(sa, __ldcg(reinterpret_cast<const float4 *>(partial_a + size_t(k) * w.chans + col)));
-            if constexpr (kHasB) take(sb, __ldcg(reinterpret_cast<const float4 *>(partial_b + size_t(k) * w.chans + col)));
+          for (uint32_t k = pl; k < gridDim.y; k += part_lanes) {
+            if constexpr (kHasA) take(sa, __ldcg(reinterpret_cast<const float4 *>(partial_a + k * pitch + at)));
+            if constexpr (kHasB) take(sb, __ldcg(reinterpret_cast<const float4 *>(partial_b + k * pitch + at)));
           }
         }
-        // part_lanes values per channel: 4 to a thread, then the rest
-        const uint32_t ch = threadIdx.x & (4 * ql - 1), group = threadIdx.x >> (ql_log2 + 2);
-        const uint32_t groups = kChanSumThreads >> (ql_log2 + 2);
-        auto over_lanes = [&](const float4 &s) {
-          __syncthreads();
-          reinterpret_cast<float4 *>(red)[pl * ql + cl] = s;
-          __syncthreads();
+        if (kHasA) sums_a[pl * (ql + 1) + cl] = sa;
+        if (kHasB) sums_b[pl * (ql + 1) + cl] = sb;
+        __syncthreads();
+        // columns of both sums over the threads, `per` neighbouring threads to a column
+        const uint32_t cols4 = 4 * ql, items = cols4 * ((kHasA ? 1 : 0) + (kHasB ? 1 : 0));
+        const uint32_t per = items >= kChanSumThreads ? 1u : min(32u, min(part_lanes, kChanSumThreads / items));
+        for (uint32_t i0 = 0; i0 < items; i0 += kChanSumThreads / per) {
+          const uint32_t item = i0 + threadIdx.x / per, part = threadIdx.x & (per - 1);
+          const bool second = kHasA && item >= cols4;
+          const uint32_t col = second ? item - cols4 : item;
           float t = 0.f;
-#pragma unroll
-          for (uint32_t k = 0; k < 4; ++k) t += red[(group + k * groups) * 4 * ql + ch];
-          __syncthreads();
-          red[threadIdx.x] = t;
-          __syncthreads();
-          t = 0.f;
-          if (group == 0)
-            for (uint32_t k = 0; k < groups; ++k) t += red[k * 4 * ql + ch];
-          return t;
-        };
+          if (item < items) {
+            const float *src = reinterpret_cast<const float *>(second || !kHasA ? sums_b : sums_a);
+            for (uint32_t k = part; k < part_lanes; k += per) t += src[k * (cols4 + 4) + col];
+          }
+          for (uint32_t d = per >> 1; d >= 1; d >>= 1) t += __shfl_xor_sync(0xffffffffu, t, d);
+          if (part == 0 && item < items && q0 * 4 + col < pitch) (second || !kHasA ? total_b : total_a)[q0 * 4 + col] = t;
+        }
+        __syncthreads();
+      }
+      for (uint32_t c = threadIdx.x; c < w.chans; c += kChanSumThreads) {
         float ta = 0.f, tb = 0.f;
-        if constexpr (kHasA) ta = over_lanes(sa);
-        if constexpr (kHasB) tb = over_lanes(sb);
-        if (group == 0 && q0 * 4 + ch < w.chans) finish(q0 * 4 + ch, ta, tb);
+        for (uint32_t r = 0; r < w.fold; ++r) {
+          if constexpr (kHasA) ta += total_a[r * w.chans + c];
+          if constexpr (kHasB) tb += total_b[r * w.chans + c];
+        }
+        finish(c, ta, tb);
       }
       return;
     }
   }
-  uint32_t cl_log2 = 3;
-  while ((2u << cl_log2) <= kChanSumThreads && (1u << cl_log2) < w.chans) ++cl_log2;
-  const uint32_t chan_lanes = 1u << cl_log2, part_lanes = kChanSumThreads >> cl_log2;
-  const uint32_t cl = threadIdx.x & (chan_lanes - 1), pl = threadIdx.x >> cl_log2;
-  for (uint32_t c0 = 0; c0 < w.chans; c0 += chan_lanes) {
-    const uint32_t c = c0 + cl;
+  // any channel count: [slabs * fold][chans], a channel per thread
+  const uint32_t parts = gridDim.y * w.fold;
+  for (uint32_t c = threadIdx.x; c < w.chans; c += kChanSumThreads) {
     float sa = 0.f, sb = 0.f;
-    if (c < w.chans) {
 #pragma unroll 8
-      for (uint32_t k = pl; k < parts; k += part_lanes) {
-        if constexpr (kHasA) sa += __ldcg(partial_a + size_t(k) * w.chans + c);
-        if constexpr (kHasB) sb += __ldcg(partial_b + size_t(k) * w.chans + c);
-      }
+    for (uint32_t k = 0; k < parts; ++k) {
+      if constexpr (kHasA) sa += __ldcg(partial_a + size_t(k) * w.chans + c);
+      if constexpr (kHasB) sb += __ldcg(partial_b + size_t(k) * w.chans + c);
     }
-    auto over_lanes = [&](float s) {
-      __syncthreads();
-      red[threadIdx.x] = s;
-      __syncthreads();
-      float t = 0.f;
-      if (pl == 0)
-        for (uint32_t k = 0; k < part_lanes; ++k) t += red[k * chan_lanes + cl];
-      return t;
-    };
-    if constexpr (kHasA) sa = over_lanes(sa);
-    if constexpr (kHasB) sb = over_lanes(sb);
-    if (pl == 0 && c < w.chans) finish(c, sa, sb);
+    finish(c, sa, sb);
   }
 }
 
 inline bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
+template <typename T, int kMode, int V>
+int launchChanSums(plb_context *ctx, dim3 grid, const T *x, const T *y, const T *centre, const ChanWalk &w, float *pa,
+                   float *pb, ChanFinish fin) {
+  constexpr size_t kMost = 160 * 1024;
+  const size_t pitch = size_t(w.vecs) * V, cols = size_t(V) << w.vec_lanes_log2;
+  const size_t finish = 8 * kChanSumQuads * sizeof(float) + 2 * pitch * sizeof(float);
+  fin.totals_fit = V > 1 && finish <= kMost ? 1 : 0;
+  const size_t smem = std::max(2 * 32 * (cols + 1) * sizeof(float), fin.totals_fit ? finish : size_t(0));
+  static bool configured[64] = {};
+  bool &done = configured[ctx->device & 63];
+  if (!done) {
+    PLB_CUDA(cudaFuncSetAttribute(chanSumsKernel<T, kMode, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kMost)));
+    done = true;
+  }
+  return launchPdl(ctx, chanSumsKernel<T, kMode, V>, grid, dim3(kChanSumThreads), smem, x, y, centre, w, pa, pb,
+                   ctx->d_ticket, fin);
+}
 
 template <typename T, int kMode>
 int chanSums(plb_context *ctx, const T *x, const T *y, const T *centre, uint64_t rows, uint32_t chans,
@@ -384,16 +413,18 @@ int chanSums(plb_context *ctx, const T *x, const T *y, const T *centre, uint64_t
   constexpr uint32_t kVec = 16 / sizeof(T);
   const bool vec = aligned16(x) && (y == nullptr || aligned16(y));
   dim3 grid;
-  const ChanWalk w = chanWalk(ctx, rows, chans, vec ? kVec : 1, kChanSumThreads, 1, &grid);
+  // Slabs: one per SM, but each slab's row of sums is work for the last block.  Up
+  // to 128 columns that is nothing; wider rows take fewer slabs unless a slab has
+  // 256 KB to read and more (25088 x 256 halves: 9.4 us with 148 slabs, 8.9 with 74).
+  const uint64_t most_slabs = std::max<uint64_t>({37, uint64_t(ctx->sm_count) * 128 / std::max(chans, 1u),
+                                                  rows * chans * sizeof(T) / (256 * 1024)});
+  const ChanWalk w = chanWalk(ctx, rows, chans, vec ? kVec : 1, kChanSumThreads, 1, most_slabs, &grid);
   const size_t row = size_t(w.vecs) * (vec ? kVec : 1);
   void *ws = nullptr;
-  if (int rc = scratch(ctx, kSlotChannelSums, size_t(2) * w.slabs * row * sizeof(float), &ws)) return rc;
-  float *pa = static_cast<float *>(ws), *pb = pa + size_t(w.slabs) * row;
-  if (vec)
-    return launchPdl(ctx, chanSumsKernel<T, kMode, int(kVec)>, grid, dim3(kChanSumThreads), 0, x, y, centre, w, pa,
-                     pb, ctx->d_ticket, fin);
-  return launchPdl(ctx, chanSumsKernel<T, kMode, 1>, grid, dim3(kChanSumThreads), 0, x, y, centre, w, pa, pb,
-                   ctx->d_ticket, fin);
+  if (int rc = scratch(ctx, kSlotChannelSums, size_t(2) * w.slabs * row * sizeof(float) + 16, &ws)) return rc;
+  float *pa = static_cast<float *>(ws), *pb = pa + (size_t(w.slabs) * row + 3) / 4 * 4;
+  if (vec) return launchChanSums<T, kMode, int(kVec)>(ctx, grid, x, y, centre, w, pa, pb, fin);
+  return launchChanSums<T, kMode, 1>(ctx, grid, x, y, centre, w, pa, pb, fin);
 }
 
 // ---- maps ------------------------------------------------------------------------
@@ -505,7 +536,7 @@ int chanMap(plb_context *ctx, const ChanMapArgs<T> &g, uint64_t rows, uint32_t c
   const bool vec = aligned16(g.x) && aligned16(g.out) && (g.y == nullptr || aligned16(g.y)) &&
                    (g.out2 == nullptr || aligned16(g.out2));
   dim3 grid;
-  const ChanWalk w = chanWalk(ctx, rows, chans, vec ? kVec : 1, kChanMapThreads, 4, &grid);
+  const ChanWalk w = chanWalk(ctx, rows, chans, vec ? kVec : 1, kChanMapThreads, 4, 0, &grid);
   if (vec) return launchPdl(ctx, chanMapKernel<T, kMode, int(kVec)>, grid, dim3(kChanMapThreads), 0, g, w);
   return launchPdl(ctx, chanMapKernel<T, kMode, 1>, grid, dim3(kChanMapThreads), 0, g, w);
 }

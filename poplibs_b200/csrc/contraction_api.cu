@@ -225,6 +225,7 @@ struct PassOperands {
   int type;
   const void *act, *wgt;
   uint32_t k, act_pitch, w_pitch;
+  bool lattice = false;  // the activations hold only the pixels a strided pointwise layer reads
 };
 
 // The filter taps of a problem: tap (r, s) is stored tile
@@ -278,6 +279,10 @@ void setActs(IgemmProblem *r, const plb_conv_params &p, const PassOperands &o, i
   r->act_strides[2] = uint64_t(H) * W * ctot * es;
 }
 
+// A 1x1 convolution without padding reads every stride'th pixel alone.
+bool pointwise(const ConvShape &s) { return s.KH == 1 && s.KW == 1 && s.padH == 0 && s.padW == 0; }
+int latticeExtent(int in, int out, int stride) { return std::min(out, (in + stride - 1) / stride); }
+
 // Forward problem (all groups).
 // With `swapped_weights` the weights are stored [G][tap][Ci][Co] (the forward
 // layout of the layer this convolution is the backward pass of) and are used
@@ -291,12 +296,15 @@ IgemmProblem convFwdProblem(const plb_conv_params &p, const plb_conv_options *op
   IgemmProblem r = swapped_weights ? passProblem(p, opt, s, o, true, co, o.k) : passProblem(p, opt, s, o, false, o.k, co);
   // the truncated input is a view: same strides, shifted base, smaller extents
   setActs(&r, p, o, s.H, s.W, s.tH, s.tW);
-  const bool pointwise = s.KH == 1 && s.KW == 1 && s.padH == 0 && s.padW == 0;
-  if (pointwise) {
+  if (o.lattice) {
+    r.act_dims[1] = uint64_t(latticeExtent(s.We, s.OWc, s.strW));
+    r.act_dims[2] = uint64_t(latticeExtent(s.He, s.OHc, s.strH));
+    setActs(&r, p, o, int(r.act_dims[2]), int(r.act_dims[1]), 0, 0);
+  } else if (pointwise(s)) {
     // a strided 1x1 convolution reads a sub-lattice: describe only that (its
     // extent is what the input holds; outputs beyond it read zero padding)
-    r.act_dims[1] = uint64_t(std::min(s.OWc, (s.We + s.strW - 1) / s.strW));
-    r.act_dims[2] = uint64_t(std::min(s.OHc, (s.He + s.strH - 1) / s.strH));
+    r.act_dims[1] = uint64_t(latticeExtent(s.We, s.OWc, s.strW));
+    r.act_dims[2] = uint64_t(latticeExtent(s.He, s.OHc, s.strH));
     r.act_strides[0] *= uint64_t(s.strW);
     r.act_strides[1] *= uint64_t(s.strH);
   } else {
@@ -433,8 +441,10 @@ void bwdPhase(int phase, int in_size, int kernel, int pad, int dil, int stride, 
 // `rows` of `cols` elements each become the activations; the weights are `w_rows`
 // rows of `w_cols` elements, the reduction along their rows (w_k_rows = false) or
 // along `w_k_rows` rows of each tile.
+// With a lattice only its pixels are copied, if a copy is made at all (`o->lattice`).
 int prepareOperands(plb_context *ctx, int type, const void *act, uint64_t rows, uint32_t cols, const void *wgt,
-                    uint64_t w_rows, uint32_t w_cols, uint64_t w_k_rows, PassOperands *o) {
+                    uint64_t w_rows, uint32_t w_cols, uint64_t w_k_rows, PassOperands *o,
+                    const Repack::Lattice *lattice = nullptr) {
   const size_t es = dtypeBytes(type);
   const bool is_float = type == PLB_FLOAT;
   o->type = is_float ? PLB_BFLOAT16 : type;
@@ -453,14 +463,19 @@ int prepareOperands(plb_context *ctx, int type, const void *act, uint64_t rows, 
   if (unfit(act, cols)) {
     o->act_pitch = is_float ? roundToVec(3 * uint64_t(cols), 2) : roundToVec(cols, es);
     jobs[n] = Repack{act, nullptr, rows, cols, cols, o->act_pitch, uint32_t(es),
-                     is_float ? kRepackSplitCols : kRepackCopy, false, 0};
+                     is_float ? kRepackSplitCols : kRepackCopy, false, 0, {}};
+    if (lattice) {
+      jobs[n].lattice = *lattice;
+      jobs[n].rows = rows / (uint64_t(lattice->full_h) * lattice->full_w) * lattice->sub_h * lattice->sub_w;
+      o->lattice = true;
+    }
     operand[n++] = &o->act;
   }
   if (unfit(wgt, w_cols)) {
     const bool along_rows = is_float && w_k_rows == 0;
     o->w_pitch = along_rows ? roundToVec(3 * uint64_t(w_cols), 2) : roundToVec(w_cols, is_float ? 2 : es);
     jobs[n] = Repack{wgt, nullptr, w_rows, w_cols, w_cols, o->w_pitch, uint32_t(es),
-                     !is_float ? kRepackCopy : along_rows ? kRepackSplitCols : kRepackSplitPlanes, true, w_k_rows};
+                     !is_float ? kRepackCopy : along_rows ? kRepackSplitCols : kRepackSplitPlanes, true, w_k_rows, {}};
     operand[n++] = &o->wgt;
   }
   if (n == 0) return PLB_OK;
@@ -742,7 +757,7 @@ int plb_matmul(plb_context *ctx, const plb_matmul_desc *desc, const void *d_a, c
       const int mode = !is_float ? kRepackCopy : k_along_rows ? kRepackSplitPlanes : kRepackSplitCols;
       const uint32_t pitch_out = mode == kRepackCopy ? roundToVec(cols, es)
                                                      : roundToVec(mode == kRepackSplitCols ? 3 * uint64_t(cols) : cols, 2);
-      jobs[n] = Repack{*base, nullptr, rows, cols, uint64_t(*pitch), pitch_out, uint32_t(es), mode, weights, d.k};
+      jobs[n] = Repack{*base, nullptr, rows, cols, uint64_t(*pitch), pitch_out, uint32_t(es), mode, weights, d.k, {}};
       *pitch = pitch_out;
       operand[n++] = base;
     };
@@ -950,8 +965,7 @@ int plb_convolution(plb_context *ctx, const plb_conv_params *p, const plb_conv_o
     if (rc != PLB_ERR_UNSUPPORTED) return rc;
   }
   if (s.strH > 1 || s.strW > 1) {
-    const bool pointwise = s.KH == 1 && s.KW == 1 && s.padH == 0 && s.padW == 0;
-    if (!pointwise && (s.strH > 8 || s.strW > 8))
+    if (!pointwise(s) && (s.strH > 8 || s.strW > 8))
       return fail(PLB_ERR_UNSUPPORTED, "strides above 8 are not implemented for k > 1");
   }
   if (s.KH <= 0 || s.KW <= 0) {
@@ -971,16 +985,24 @@ int plb_convolution(plb_context *ctx, const plb_conv_params *p, const plb_conv_o
   const uint64_t in_rows = uint64_t(q.batch) * s.H * s.W * q.groups, tiles = uint64_t(q.groups) * s.KHs * s.KWs;
   const uint32_t ci = q.in_chans_per_group, co = q.out_chans_per_group;
   const bool transposed = swapped && q.input_type == PLB_QUARTER;  // -> [G][flipped k][Co][Ci]
+  // a strided pointwise layer whose input has to be copied: only the pixels it reads
+  Repack::Lattice sub{}, *lattice = nullptr;
+  if (pointwise(s) && (s.strH > 1 || s.strW > 1) && s.tH == 0 && s.tW == 0) {
+    sub = Repack::Lattice{q.groups, uint32_t(latticeExtent(s.We, s.OWc, s.strW)),
+                          uint32_t(latticeExtent(s.He, s.OHc, s.strH)), uint32_t(s.W), uint32_t(s.H),
+                          uint32_t(s.strW), uint32_t(s.strH)};
+    if (uint64_t(q.batch) * sub.sub_h * sub.sub_w <= 0xffffffffull) lattice = &sub;
+  }
   PassOperands o;
   if (transposed) {
     uint32_t pitch = 0;
     if (int rc = transposedWeights(ctx, w, q.groups, uint64_t(s.KHs) * s.KWs, ci, co, &w, &pitch)) return rc;
-    if (int rc = prepareOperands(ctx, q.input_type, d_in, in_rows, ci, w, tiles * co, pitch, 0, &o)) return rc;
+    if (int rc = prepareOperands(ctx, q.input_type, d_in, in_rows, ci, w, tiles * co, pitch, 0, &o, lattice)) return rc;
   } else if (swapped) {
     // the reduction along the rows
-    if (int rc = prepareOperands(ctx, q.input_type, d_in, in_rows, ci, w, tiles * ci, co, ci, &o)) return rc;
+    if (int rc = prepareOperands(ctx, q.input_type, d_in, in_rows, ci, w, tiles * ci, co, ci, &o, lattice)) return rc;
   } else {
-    if (int rc = prepareOperands(ctx, q.input_type, d_in, in_rows, ci, w, tiles * co, ci, 0, &o)) return rc;
+    if (int rc = prepareOperands(ctx, q.input_type, d_in, in_rows, ci, w, tiles * co, ci, 0, &o, lattice)) return rc;
   }
   IgemmProblem r = convFwdProblem(q, opt, s, o, d_bias, d_out, swapped && !transposed, transposed);
   if (together) r.nonfinite = nonfiniteFlag(ctx);

@@ -12,7 +12,7 @@ namespace plb {
 // Which instance, and how it is launched.
 struct IgemmVariant {
   bool fp8, a_mn, b_mn, resident, halo, pair, groups;
-  int grid, resident_bytes;
+  int grid, grid_multiple, resident_bytes;  // grid_multiple: of the CTAs (pairs of them)
   bool pdl;
 };
 
@@ -77,7 +77,9 @@ int launchInstance(plb_context *ctx, const CUtensorMap &ta, const CUtensorMap &t
         if (n <= 0) return fail(PLB_ERR_CUDA, "no cluster of two CTAs can be resident on this device");
         max_clusters[dev] = n;
       }
-      const int clusters = std::max(1, std::min(v.grid / 2, max_clusters[dev]));
+      int clusters = std::max(1, std::min(v.grid / 2, max_clusters[dev]));
+      clusters = clusters / v.grid_multiple * v.grid_multiple;
+      if (clusters == 0) return fail(PLB_ERR_CUDA, "too few clusters can be resident for this number of groups");
       cfg.gridDim = dim3(unsigned(2 * clusters));
     }
     cfg.attrs = attr;
@@ -107,7 +109,12 @@ int launchForTile(plb_context *ctx, const CUtensorMap &ta, const CUtensorMap &tb
     if (v.b_mn) PLB_LAUNCH(false, true, true, false, false, false);
     PLB_LAUNCH(false, true, false, false, false, false);
   }
-  // (several groups never have resident weights)
+  if (v.groups && v.halo && v.resident) {
+    PLB_LAUNCH_OPERANDS(true, true, true);
+  }
+  if (v.groups && v.resident) {
+    PLB_LAUNCH_OPERANDS(true, false, true);
+  }
   if (v.groups && v.halo) {
     PLB_LAUNCH_OPERANDS(false, true, true);
   }

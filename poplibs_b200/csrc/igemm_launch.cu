@@ -36,6 +36,8 @@ int stagesFor(int bn, int a_stage_bytes, int b_tiles, bool resident, int residen
 // every CTA gets several pixel tiles to amortise the load over, and the
 // weights leave room for a pipeline of at least six activation stages.
 constexpr int kMaxResidentBytes = 96 * 1024;
+// Groups beside which a grid that is a multiple of their number still fills the device.
+constexpr int kMaxResidentGroups = 16;
 
 }  // namespace
 
@@ -121,9 +123,12 @@ int planIgemm(const IgemmProblem &p, int sm_count, plb_plan *plan) {
   plan->cta_pair = pair ? 1 : 0;
   auto grid_for = [&](long m_tiles) {
     const int sms = sm_count > 0 ? sm_count : 148;
-    if (!pair) return int(std::min<long>(m_tiles * n_tiles * groups, sms));
-    return int(2 * std::min<long>(((m_tiles + 1) / 2) * n_tiles * groups, sms / 2));
+    // (with resident weights a CTA, or pair, keeps to one group)
+    const long units = pair ? std::min<long>(((m_tiles + 1) / 2) * n_tiles * groups, sms / 2)
+                            : std::min<long>(m_tiles * n_tiles * groups, sms);
+    return int((pair ? 2 : 1) * (plan->resident_weights ? units / groups * groups : units));
   };
+  plan->resident_weights = 0;
   plan->grid = grid_for(best_tiles);
   const int k_elems = kStageKBytes / elem;
   const long k_iters = long(p.taps_h) * p.taps_w * ((p.k_per_tap + k_elems - 1) / k_elems);
@@ -132,10 +137,11 @@ int planIgemm(const IgemmProblem &p, int sm_count, plb_plan *plan) {
   const bool want_resident = (p.plan_flags & PLB_PLAN_FORCE_RESIDENT_WEIGHTS) != 0 ||
                              plan->tiles >= 2 * plan->grid;
   plan->resident_weights =
-      ((p.plan_flags & PLB_PLAN_NO_RESIDENT_WEIGHTS) == 0 && n_tiles == 1 && groups == 1 && !p.a_mn &&
+      ((p.plan_flags & PLB_PLAN_NO_RESIDENT_WEIGHTS) == 0 && n_tiles == 1 && groups <= kMaxResidentGroups && !p.a_mn && p.force_split_k <= 1 &&
        resident_bytes <= kMaxResidentBytes && want_resident)
           ? 1
           : 0;
+  plan->grid = grid_for(best_tiles);
   plan->halo_rows = 0;
   plan->stages = stagesFor(bn, kTileM * kStageKBytes, 1, plan->resident_weights != 0,
                            plan->resident_weights ? int(resident_bytes) : 0, pair);
@@ -161,6 +167,8 @@ int planIgemm(const IgemmProblem &p, int sm_count, plb_plan *plan) {
         if ((w * n) % 8 != 0 || h + halo > 256 || (w - 1) * p.stride_w + 1 > 256) continue;
         const long tiles = long((p.out_w + w - 1) / w) * ((p.out_h + h - 1) / h) *
                            ((p.out_n + n - 1) / n);
+        // without much more tensor-core work (padded tiles)
+        if (tiles * 8 > best_tiles * 9) continue;
         const long cost =
             tiles * p.taps_w * (long(w) * n * (h + halo) * kStageKBytes + p.taps_h * b_tile);
         if (best_cost < 0 || cost < best_cost || (cost == best_cost && tiles < best_t)) {
@@ -175,9 +183,8 @@ int planIgemm(const IgemmProblem &p, int sm_count, plb_plan *plan) {
       const int a_stage = hw * hn * (hh + halo) * kStageKBytes;
       const int st = stagesFor(bn, a_stage, res ? 1 : p.taps_h, res, res ? int(resident_bytes) : 0,
                                pair);
-      // worthwhile only if it really fills less, without much more tensor-core
-      // work (padded tiles), and still leaves a pipeline
-      if (st >= 3 && best_cost < base_cost && best_t * 8 <= best_tiles * 9) {
+      // worthwhile only if it really fills less and still leaves a pipeline
+      if (st >= 3 && best_cost < base_cost) {
         plan->halo_rows = halo;
         plan->box_w = hw;
         plan->box_h = hh;
@@ -547,6 +554,7 @@ int launchIgemm(plb_context *ctx, const IgemmProblem &p, const plb_plan &plan) {
 
   const bool pdl = (p.plan_flags & PLB_PLAN_NO_PDL) == 0;
   const IgemmVariant variant{p.fp8, p.a_mn, p.b_mn, plan.resident_weights != 0, halo, plan.cta_pair != 0, with_groups, plan.grid,
+                             plan.resident_weights ? groups : 1,
                              resident_bytes, pdl};
   int rc = PLB_OK;
   switch (plan.tile_n) {

@@ -185,6 +185,8 @@ struct IgemmSmem {
 //       Used when there is a single N tile and the weights fit (small filters
 //       with few channels), where re-fetching them per pixel tile would cost
 //       as much shared-memory fill bandwidth as the activations themselves.
+//       With several groups the grid is a multiple of their number, so that all
+//       units of a CTA belong to one group.
 // kHalo: one activation strip per (horizontal tap, channel chunk) feeds all
 //       vertical taps: the strip of tap row r is the same shared memory shifted
 //       by whole 8-row groups, which the descriptor's start address can express.
@@ -753,7 +755,7 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
         for (int it = warp - 4; it < k_iters; it += 16) {
           int r, s, kc;
           step_coords(it, r, s, kc);
-          load_b(0u, 0u, 0, r, s, kc, 0, true);
+          load_b(0u, 0u, f_group, r, s, kc, 0, true);
         }
         pdl_wait();
         if (warp == 4 && leader)
@@ -762,7 +764,7 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
         for (int it = warp - 4; it < k_iters; it += 16) {
           int r, s, kc;
           step_coords(it, r, s, kc);
-          load_b(resb_base + it * S::kBBytes, resb_bar_lead, 0, r, s, kc, 0, false);
+          load_b(resb_base + it * S::kBBytes, resb_bar_lead, f_group, r, s, kc, 0, false);
         }
         if (warp == 4) PLB_TRACE_STAMP(2, 4012);
       }
@@ -934,31 +936,43 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
           continue;
         }
         __syncwarp();
+        // fp32: a row of 32 columns per instruction; half: two rows of 16 words.
+        // Four instructions' words and row offsets first, then their stores: one at
+        // a time is a chain of latencies (3.7 of 14.8 us on a 77x293 fp32 output).
         const uint32_t lo = uint32_t(out_off), hi = row_ok ? uint32_t(out_off >> 32) : 0x80000000u;
-#pragma unroll 2
-        for (int i = 0; i < (whole_rows ? 32 : 16); ++i) {
-          // fp32: a row of 32 columns; half: two rows of 16 words
-          const int r = whole_rows ? i : 2 * i + (lane >> 4), cc = whole_rows ? lane : 2 * (lane & 15);
-          const uint32_t piece = uint32_t(whole_rows ? lane : lane & 15) >> 2, word = (uint32_t(lane) & 3u) << 2;
-          const uint32_t bits = ld_shared_b32(
-              whole_rows ? buf + uint32_t(r) * 128u + ((piece ^ (uint32_t(r) & 7u)) << 4) + word
-                         : wbuf + uint32_t(r) * 64u + ((piece ^ ((uint32_t(r) >> 1) & 3u)) << 4) + word);
-          const uint32_t off_hi = __shfl_sync(0xffffffffu, hi, r), off_lo = __shfl_sync(0xffffffffu, lo, r);
-          if (int32_t(off_hi) >= 0 && cc < valid) {
-            const long long off = (long long)(uint64_t(off_hi) << 32 | off_lo) + col0 + cc;
+        const uint8_t *staged = smem_raw + ((whole_rows ? buf : wbuf) - smem_u32(smem_raw));
+        const int cc = whole_rows ? lane : 2 * (lane & 15);
+        const uint32_t piece = uint32_t(whole_rows ? lane : lane & 15) >> 2, word = (uint32_t(lane) & 3u) << 2;
+#pragma unroll 1
+        for (int i0 = 0; i0 < (whole_rows ? 32 : 16); i0 += 4) {
+          uint32_t bits[4], off_hi[4], off_lo[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const int r = whole_rows ? i0 + u : 2 * (i0 + u) + (lane >> 4);
+            bits[u] = *reinterpret_cast<const uint32_t *>(
+                staged + (whole_rows ? uint32_t(r) * 128u + ((piece ^ (uint32_t(r) & 7u)) << 4)
+                                     : uint32_t(r) * 64u + ((piece ^ ((uint32_t(r) >> 1) & 3u)) << 4)) + word);
+            off_hi[u] = __shfl_sync(0xffffffffu, hi, r);
+            off_lo[u] = __shfl_sync(0xffffffffu, lo, r);
+          }
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            if (int32_t(off_hi[u]) < 0 || cc >= valid) continue;
+            const long long off = (long long)(uint64_t(off_hi[u]) << 32 | off_lo[u]) + col0 + cc;
             if (out_f32) {
-              static_cast<uint32_t *>(args.out)[off] = bits;
+              static_cast<uint32_t *>(args.out)[off] = bits[u];
             } else {
               uint16_t *dst = static_cast<uint16_t *>(args.out) + off;
               if (cc + 1 < valid && (reinterpret_cast<uintptr_t>(dst) & 3) == 0) {
-                *reinterpret_cast<uint32_t *>(dst) = bits;
+                *reinterpret_cast<uint32_t *>(dst) = bits[u];
               } else {
-                dst[0] = uint16_t(bits);
-                if (cc + 1 < valid) dst[1] = uint16_t(bits >> 16);
+                dst[0] = uint16_t(bits[u]);
+                if (cc + 1 < valid) dst[1] = uint16_t(bits[u] >> 16);
               }
             }
           }
         }
+        __syncwarp();
       }
       if (stamp) PLB_TRACE_STAMP(2, local_tile * 4 + 2);
       if (stamp) PLB_TRACE_STAMP(2, local_tile * 4 + 3);

@@ -32,6 +32,7 @@ struct RepackArgs {
   int mode;                            // RepackMode
   int weights;                         // pieces (hi, hi, lo) instead of (hi, lo, hi)
   unsigned long long mid;              // rows per plane (kSplitPlanes)
+  uint32_t parts, sub_w, sub_h, full_w, full_h, step_w, step_h;  // Repack::lattice (sub_w 0: all rows)
 };
 
 constexpr int kRepackThreads = 256;
@@ -82,7 +83,14 @@ repackKernel(const RepackArgs first, const RepackArgs second, unsigned first_blo
     const uint32_t v = i - down * a.vecs;
     const unsigned long long row = row0 + down;
     if (row >= a.rows) return;
-    const uint8_t *src = a.src + row * a.src_pitch;
+    unsigned long long src_row = row;
+    if (a.sub_w != 0) {
+      // row = (image, h, w, part) of the sub-lattice
+      const uint32_t per_w = uint32_t(row / a.parts), part = uint32_t(row - (unsigned long long)per_w * a.parts);
+      const uint32_t rows = per_w / a.sub_w, w = per_w - rows * a.sub_w, n = rows / a.sub_h, h = rows - n * a.sub_h;
+      src_row = (((unsigned long long)n * a.full_h + h * a.step_h) * a.full_w + w * a.step_w) * a.parts + part;
+    }
+    const uint8_t *src = a.src + src_row * a.src_pitch;
     if (a.mode == kRepackCopy) {
       const int valid = int(a.cols * a.elem_bytes) - int(v) * 16;
       uint4 o = make_uint4(0u, 0u, 0u, 0u);
@@ -103,7 +111,15 @@ repackKernel(const RepackArgs first, const RepackArgs second, unsigned first_blo
     }
     const float *x = reinterpret_cast<const float *>(src);
     __align__(16) uint16_t o[3][8];
-    if (a.mode == kRepackSplitCols) {
+    if (a.mode == kRepackSplitCols && a.cols % 8 == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
+      // the eight elements are neighbours and of one piece
+      const uint32_t piece = v * 8 / a.cols, col = v * 8 - piece * a.cols;
+      const float4 f0 = *reinterpret_cast<const float4 *>(x + col), f1 = *reinterpret_cast<const float4 *>(x + col + 4);
+      const float f[8] = {f0.x, f0.y, f0.z, f0.w, f1.x, f1.y, f1.z, f1.w};
+#pragma unroll
+      for (int j = 0; j < 8; ++j) o[0][j] = floatPiece(f[j], int(piece), a.weights);
+      *reinterpret_cast<uint4 *>(a.dst + (row * a.vecs + v) * 16) = *reinterpret_cast<const uint4 *>(o[0]);
+    } else if (a.mode == kRepackSplitCols) {
       // (piece, column) of the eight elements
       uint32_t piece = v * 8 / a.cols, col = v * 8 - piece * a.cols;
 #pragma unroll
@@ -116,12 +132,25 @@ repackKernel(const RepackArgs first, const RepackArgs second, unsigned first_blo
       }
       *reinterpret_cast<uint4 *>(a.dst + (row * a.vecs + v) * 16) = *reinterpret_cast<const uint4 *>(o[0]);
     } else {
+      float f[8];
+      if (v * 8 + 8 <= a.cols && (reinterpret_cast<uintptr_t>(x) & 15) == 0) {
+        const float4 f0 = *reinterpret_cast<const float4 *>(x + v * 8), f1 = *reinterpret_cast<const float4 *>(x + v * 8 + 4);
+        f[0] = f0.x;
+        f[1] = f0.y;
+        f[2] = f0.z;
+        f[3] = f0.w;
+        f[4] = f1.x;
+        f[5] = f1.y;
+        f[6] = f1.z;
+        f[7] = f1.w;
+      } else {
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float f = v * 8 + j < a.cols ? x[v * 8 + j] : 0.f;
-#pragma unroll
-        for (int k = 0; k < 3; ++k) o[k][j] = floatPiece(f, k, a.weights);
+        for (int j = 0; j < 8; ++j) f[j] = v * 8 + j < a.cols ? x[v * 8 + j] : 0.f;
       }
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) o[k][j] = floatPiece(f[j], k, a.weights);
       const unsigned long long outer = a.mid < a.rows ? row / a.mid : 0, plane0 = outer * 2 * a.mid + row;
 #pragma unroll
       for (int k = 0; k < 3; ++k)
@@ -157,6 +186,13 @@ int repack(plb_context *ctx, const Repack *jobs, int n) {
     a.mode = r.mode;
     a.weights = r.weights ? 1 : 0;
     a.mid = r.mid ? r.mid : r.rows;
+    a.parts = r.lattice.parts;
+    a.sub_w = r.lattice.sub_w;
+    a.sub_h = r.lattice.sub_h;
+    a.full_w = r.lattice.full_w;
+    a.full_h = r.lattice.full_h;
+    a.step_w = r.lattice.step_w;
+    a.step_h = r.lattice.step_h;
     const uint64_t per_block = kRepackThreads * kRepackPerThread;
     const uint64_t b = (r.rows * a.vecs + per_block - 1) / per_block;
     if (b + blocks[0] > 0x7fffffffull || uint64_t(a.vecs) + per_block > 0x7fffffffull)

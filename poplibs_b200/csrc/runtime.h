@@ -140,6 +140,11 @@ struct Repack {
   int mode;
   bool weights;           // pieces (hi, hi, lo), else (hi, lo, hi)
   uint64_t mid;           // kRepackSplitPlanes: rows per plane (0 = all)
+  // Rows taken from every step_h'th / step_w'th pixel of [image][full_h][full_w][parts]
+  // (`rows` counts the taken ones, [image][sub_h][sub_w][parts]; sub_w 0: all rows).
+  struct Lattice {
+    uint32_t parts, sub_w, sub_h, full_w, full_h, step_w, step_h;
+  } lattice;
 };
 // Bytes of the destination.
 size_t repackBytes(const Repack &r);

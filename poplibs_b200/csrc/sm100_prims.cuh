@@ -235,11 +235,6 @@ __device__ __forceinline__ void pack_half8(const float *f, uint32_t (&pk)[4]) {
     pk[j] = *reinterpret_cast<const uint32_t *>(&h);
   }
 }
-__device__ __forceinline__ uint32_t ld_shared_b32(uint32_t addr) {
-  uint32_t v;
-  asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
-  return v;
-}
 
 // ---- tcgen05: tensor memory ---------------------------------------------------
 // Warp-collective.  `ncols` is a power of two in [32, 512]; the base address

@@ -29,13 +29,49 @@
 
 namespace plb {
 
+// W2[a][co][(b*s*s + ph*s + pw)*Cp + c] = W[a*s + ph][b*s + pw][co][c], rows padded to 64:
+// element i of the folded weights.
+__device__ __forceinline__ __half foldedWeight(const __half *__restrict__ w, const S2dShape &g,
+                                               unsigned co_total, unsigned i) {
+  const unsigned k = i & 63u;
+  const unsigned r = i >> 6;
+  const unsigned a = r / co_total, co = r - a * co_total;
+  const unsigned b = k / unsigned(g.C2);
+  if (b >= unsigned(g.K2w)) return __float2half(0.f);
+  const unsigned c2 = k - b * g.C2;
+  const unsigned sub = c2 / unsigned(g.Cp), c = c2 - sub * g.Cp;
+  const unsigned ph = sub / unsigned(g.s), pw = sub - ph * g.s;
+  const unsigned kh = a * g.s + ph, kw = b * g.s + pw;
+  if (c < unsigned(g.C) && kh < unsigned(g.KH) && kw < unsigned(g.KW))
+    return w[((size_t(kh) * g.KW + kw) * co_total + co) * g.C + c];
+  return __float2half(0.f);
+}
+
+// Block `block` (128 threads) of the blocks that fold the weights; the first of them
+// clears the 128 bytes after X2, which only ever meet zero weights but must be finite.
+__device__ __forceinline__ void foldWeightsAndTail(const S2dShape &g, unsigned block, __half *x2,
+                                                   const __half *__restrict__ w, __half *__restrict__ w2, int co_total) {
+  const unsigned total = unsigned(g.K2h) * unsigned(co_total) * 64u, i = block * 128u + threadIdx.x;
+  if (i < total) w2[i] = foldedWeight(w, g, unsigned(co_total), i);
+  if (block == 0 && threadIdx.x < 8)
+    reinterpret_cast<uint4 *>(x2 + size_t(g.N) * g.H2 * g.W2 * g.C2)[threadIdx.x] = make_uint4(0u, 0u, 0u, 0u);
+}
+
 // X2[n][h2][w2][(ph*s + pw)*Cp + c] = X[n][h2*s + ph - padH][w2*s + pw - padW][c]
-__global__ void s2dInputKernel(const __half *__restrict__ x, __half *__restrict__ x2, S2dShape g) {
+__global__ void __launch_bounds__(128)
+s2dInputKernel(const __half *__restrict__ x, __half *__restrict__ x2, S2dShape g, unsigned row_blocks,
+               const __half *__restrict__ w, __half *__restrict__ w2, int co_total) {
+  pdl_launch_dependents();
+  pdl_wait();
+  if (blockIdx.x >= row_blocks) {
+    foldWeightsAndTail(g, blockIdx.x - row_blocks, x2, w, w2, co_total);
+    return;
+  }
   // one thread per 8 output halves (16 bytes)
   const size_t vecs_per_pixel = size_t(g.C2) / 8;
   const size_t total = size_t(g.N) * g.H2 * g.W2 * vecs_per_pixel;
   for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < total;
-       i += size_t(gridDim.x) * blockDim.x) {
+       i += size_t(row_blocks) * blockDim.x) {
     const int v = int(i % vecs_per_pixel);
     size_t r = i / vecs_per_pixel;
     const int w2 = int(r % g.W2);
@@ -63,9 +99,17 @@ __global__ void s2dInputKernel(const __half *__restrict__ x, __half *__restrict_
 // (16-byte vectors when the rows are 16-byte aligned), then every thread
 // assembles 16-byte output vectors from them.  `lut` maps a channel of X2 to
 // (ph, pw, c) once per block instead of dividing per element.
+// Blocks past the first `row_blocks` fold the weights and clear the tail of X2.
 __global__ void __launch_bounds__(128)
 s2dInputRowsKernel(const __half *__restrict__ x, __half *__restrict__ x2, S2dShape g,
-                   int rows_aligned) {
+                   int rows_aligned, unsigned row_blocks, const __half *__restrict__ w, __half *__restrict__ w2,
+                   int co_total) {
+  pdl_launch_dependents();
+  pdl_wait();
+  if (blockIdx.x >= row_blocks) {
+    foldWeightsAndTail(g, blockIdx.x - row_blocks, x2, w, w2, co_total);
+    return;
+  }
   extern __shared__ __align__(16) unsigned char s2d_smem[];
   const int row_elems = g.W * g.C;
   const int row_stride = (row_elems + 7) & ~7;  // halves; keeps every staged row 16-byte aligned
@@ -78,7 +122,7 @@ s2dInputRowsKernel(const __half *__restrict__ x, __half *__restrict__ x2, S2dSha
   }
   const int vecs_per_pixel = g.C2 / 8;
   const int out_vecs = g.W2 * vecs_per_pixel;
-  for (int blk = blockIdx.x; blk < g.N * g.H2; blk += gridDim.x) {
+  for (int blk = blockIdx.x; blk < g.N * g.H2; blk += int(row_blocks)) {
     const int n = blk / g.H2, h2 = blk - n * g.H2;
     __syncthreads();  // previous iteration's readers are done (and the table is written)
     for (int ph = 0; ph < g.s; ++ph) {
@@ -114,31 +158,6 @@ s2dInputRowsKernel(const __half *__restrict__ x, __half *__restrict__ x2, S2dSha
   }
 }
 
-// W2[a][co][(b*s*s + ph*s + pw)*Cp + c] = W[a*s + ph][b*s + pw][co][c], rows padded to 64:
-// element i of the folded weights.
-__device__ __forceinline__ __half foldedWeight(const __half *__restrict__ w, const S2dShape &g,
-                                               unsigned co_total, unsigned i) {
-  const unsigned k = i & 63u;
-  const unsigned r = i >> 6;
-  const unsigned a = r / co_total, co = r - a * co_total;
-  const unsigned b = k / unsigned(g.C2);
-  if (b >= unsigned(g.K2w)) return __float2half(0.f);
-  const unsigned c2 = k - b * g.C2;
-  const unsigned sub = c2 / unsigned(g.Cp), c = c2 - sub * g.Cp;
-  const unsigned ph = sub / unsigned(g.s), pw = sub - ph * g.s;
-  const unsigned kh = a * g.s + ph, kw = b * g.s + pw;
-  if (c < unsigned(g.C) && kh < unsigned(g.KH) && kw < unsigned(g.KW))
-    return w[((size_t(kh) * g.KW + kw) * co_total + co) * g.C + c];
-  return __float2half(0.f);
-}
-
-__global__ void s2dWeightsKernel(const __half *__restrict__ w, __half *__restrict__ w2, S2dShape g,
-                                 int co_total) {
-  const unsigned total = unsigned(g.K2h) * unsigned(co_total) * 64u;
-  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x)
-    w2[i] = foldedWeight(w, g, unsigned(co_total), i);
-}
-
 // The same rearrangement for the common stem shape (3 channels, stride 2, so
 // Cp = 4 and one X2 pixel is two 16-byte vectors, one per vertical phase):
 // a vector is [X(ih, iw) c0..2, 0, X(ih, iw+1) c0..2, 0], i.e. six consecutive
@@ -159,11 +178,7 @@ s2dStem3Kernel(const uint32_t *__restrict__ x32, uint4 *__restrict__ x2, S2dShap
   pdl_wait();  // (the input, or X2 of an earlier call, may belong to the previous kernel)
   const unsigned rows = unsigned(g.N) * unsigned(g.H2);
   if (blockIdx.x >= rows) {
-    const unsigned total = unsigned(g.K2h) * unsigned(co_total) * 64u;
-    const unsigned i = (blockIdx.x - rows) * blockDim.x + threadIdx.x;
-    if (i < total) w2[i] = foldedWeight(w, g, unsigned(co_total), i);
-    if (blockIdx.x == rows && threadIdx.x < 8)
-      x2[(size_t(rows) * g.W2 << 1) + threadIdx.x] = make_uint4(0u, 0u, 0u, 0u);
+    foldWeightsAndTail(g, blockIdx.x - rows, reinterpret_cast<__half *>(x2), w, w2, co_total);
     return;
   }
   const int row_words = g.W * 3 / 2;  // W * 3 is even: rows start on a 32-bit word
@@ -268,34 +283,24 @@ int smallChannelPrepare(plb_context *ctx, const S2dShape &g, const void *d_in, _
   const size_t w2_elems = w2 ? size_t(g.K2h) * co * 64 : 0;
   const int row_elems = g.W * g.C;
   const size_t smem = size_t(g.s) * ((row_elems + 7) & ~7) * 2 + size_t(g.C2) * sizeof(int);
+  // (at least one block past the rows: it clears the tail of X2)
+  const unsigned wblocks = unsigned(std::max<size_t>(1, (w2_elems + 127) / 128));
+  const __half *w = static_cast<const __half *>(d_weights);
+  const int w_co = w2 ? co : 0;
   if (g.C == 3 && g.s == 2 && g.Cp == 4 && row_elems % 2 == 0 &&
-      (reinterpret_cast<uintptr_t>(d_in) & 3) == 0 && size_t(g.N) * g.H2 < (size_t(1) << 31)) {
-    // (at least one block past the rows: it clears the tail of X2)
-    const unsigned wblocks = unsigned(std::max<size_t>(1, (w2_elems + 127) / 128));
+      (reinterpret_cast<uintptr_t>(d_in) & 3) == 0 && size_t(g.N) * g.H2 < (size_t(1) << 31))
     return launchPdl(ctx, s2dStem3Kernel, dim3(unsigned(g.N) * unsigned(g.H2) + wblocks), dim3(128), 0,
-                     static_cast<const uint32_t *>(d_in), reinterpret_cast<uint4 *>(x2), g,
-                     static_cast<const __half *>(d_weights), w2, w2 ? co : 0);
-  }
+                     static_cast<const uint32_t *>(d_in), reinterpret_cast<uint4 *>(x2), g, w, w2, w_co);
+  const __half *x = static_cast<const __half *>(d_in);
   if (smem <= 48 * 1024 && g.C < 256 && g.s < 256) {
     const int rows_aligned = (row_elems % 8 == 0 && (reinterpret_cast<uintptr_t>(d_in) & 15) == 0) ? 1 : 0;
-    const int grid = int(std::min<size_t>(size_t(g.N) * g.H2, size_t(ctx->sm_count) * 16));
-    s2dInputRowsKernel<<<grid, 128, smem, ctx->stream>>>(static_cast<const __half *>(d_in), x2, g, rows_aligned);
-  } else {
-    const size_t vecs = size_t(g.N) * g.H2 * g.W2 * (g.C2 / 8);
-    const int grid = int(std::min<size_t>((vecs + 255) / 256, size_t(ctx->sm_count) * 16));
-    s2dInputKernel<<<grid, 256, 0, ctx->stream>>>(static_cast<const __half *>(d_in), x2, g);
+    const unsigned blocks = unsigned(std::min<size_t>(size_t(g.N) * g.H2, size_t(ctx->sm_count) * 16));
+    return launchPdl(ctx, s2dInputRowsKernel, dim3(blocks + wblocks), dim3(128), smem, x, x2, g, rows_aligned, blocks, w,
+                     w2, w_co);
   }
-  PLB_CUDA(cudaGetLastError());
-  ctx->launches++;
-  // the 64 trailing elements only ever meet zero weights, but must be finite
-  PLB_CUDA(cudaMemsetAsync(x2 + size_t(g.N) * g.H2 * g.W2 * g.C2, 0, 128, ctx->stream));
-  if (w2) {
-    const int wgrid = int((w2_elems + 255) / 256);
-    s2dWeightsKernel<<<wgrid, 256, 0, ctx->stream>>>(static_cast<const __half *>(d_weights), w2, g, co);
-    PLB_CUDA(cudaGetLastError());
-    ctx->launches++;
-  }
-  return PLB_OK;
+  const size_t vecs = size_t(g.N) * g.H2 * g.W2 * (g.C2 / 8);
+  const unsigned blocks = unsigned(std::min<size_t>((vecs + 127) / 128, size_t(ctx->sm_count) * 32));
+  return launchPdl(ctx, s2dInputKernel, dim3(blocks + wblocks), dim3(128), 0, x, x2, g, blocks, w, w2, w_co);
 }
 
 int convFwdSmallChannels(plb_context *ctx, const plb_conv_params &p, const plb_conv_options *opt,

@@ -349,7 +349,7 @@ int launchWuReduce(cudaStream_t stream, const WuArgs &a, size_t w_elems, void *d
     g.split_stride = (unsigned long long)a.sgroups * a.taps_h * a.taps_w * a.co_total * a.ci_total;
     g.total = w_elems;
     // four channels at once where they are neighbours on both sides
-    if (vec && g.mode == kWuGroups && g.ci % 4 == 0 && g.ci_pitch % 4 == 0) {
+    if (vec && g.ci % 4 == 0 && g.ci_pitch % 4 == 0) {
       const cudaLaunchConfig_t cfg = wuReduceConfig(stream, (count4 + 31) / 32, pdl);
       PLB_CUDA(cudaLaunchKernelEx(&cfg, wu_gather_kernel<4>, (const float *)a.partial, a.ksplit, g,
                                   d_weight_grads_f32, out16));
@@ -642,11 +642,10 @@ int plb_conv_wu(plb_context *ctx, const plb_conv_params *p, const plb_conv_optio
   const int force_split = opt ? opt->split_k : 0;
   const unsigned plan_flags = unsigned((opt ? opt->plan_flags : 0) | ctx->plan_flags);
   WuGather gather{};
-  gather.mode = kWuGroups;
   gather.taps = gather.p_taps = uint32_t(taps);
   gather.co = uint32_t(co);
   gather.ci = uint32_t(ci);
-  auto run = [&](const WuProblem &q, const WuGather *g) -> int {
+  auto run = [&](const WuProblem &q, const WuGather *g, const WuFold *fold = nullptr) -> int {
     WuArgs a{};
     planWu(q, ctx->sm_count, force_split, plan_flags, &a, nullptr);
     a.status = ctx->d_status;
@@ -657,6 +656,16 @@ int plb_conv_wu(plb_context *ctx, const plb_conv_params *p, const plb_conv_optio
     a.partial = static_cast<float *>(ws);
     if (int rc = launchWuKernel(ctx->stream, q, a)) return rc;
     ctx->launches += 2;
+    if (fold) {
+      WuFold f = *fold;
+      f.split_stride = (unsigned long long)q.s.KH * q.co * q.ci;
+      cudaLaunchAttribute pdl[1];
+      const cudaLaunchConfig_t cfg = wuReduceConfig(ctx->stream, (size_t(f.p_taps) * f.co * 16 + 31) / 32, pdl);
+      PLB_CUDA(cudaLaunchKernelEx(&cfg, wu_fold_kernel, (const float *)a.partial, a.ksplit, f, d_weight_grads_f32,
+                                  static_cast<__half *>(d_weight_grads)));
+      PLB_CUDA(cudaGetLastError());
+      return PLB_OK;
+    }
     return launchWuReduce(ctx->stream, a, p->groups * w_elems, d_weight_grads, d_weight_grads_f32, g);
   };
   // Few input channels (an image network's first layer): the rearranged input of
@@ -683,14 +692,9 @@ int plb_conv_wu(plb_context *ctx, const plb_conv_params *p, const plb_conv_optio
     q.x_strides[1] = uint64_t(g2.W2) * g2.C2 * 2;
     q.x_strides[2] = uint64_t(g2.H2) * g2.W2 * g2.C2 * 2;
     q.dy = d_out_grads;
-    gather.mode = kWuFolded;
-    gather.kw = uint32_t(s.KW);
-    gather.stride = uint32_t(g2.s);
-    gather.chan_pitch = uint32_t(g2.Cp);
-    gather.p_taps = uint32_t(g2.K2h);
-    gather.p_co = uint32_t(co);
-    gather.p_ci = 64;
-    return run(q, &gather);
+    const WuFold fold{uint32_t(s.KH), uint32_t(s.KW), uint32_t(co), uint32_t(ci), uint32_t(g2.s), uint32_t(g2.Cp),
+                      uint32_t(g2.K2h), 0};
+    return run(q, nullptr, &fold);
   }
   // Channel counts TMA cannot address (a pixel must be a multiple of 16 bytes) run
   // on copies with the channels rounded up; float operands as three batches of
@@ -712,7 +716,7 @@ int plb_conv_wu(plb_context *ctx, const plb_conv_params *p, const plb_conv_optio
       const bool whole = chans == chans_pitch;
       const uint32_t cols = whole ? p->groups * chans : chans;
       jobs[n] = Repack{*base, nullptr, whole ? pixels : pixels * p->groups, cols, cols, whole ? uint32_t(pixel) : chans_pitch,
-                       is_float ? 4u : 2u, is_float ? kRepackSplitPlanes : kRepackCopy, second, 0};
+                       is_float ? 4u : 2u, is_float ? kRepackSplitPlanes : kRepackCopy, second, 0, {}};
       operand[n++] = base;
     };
     add(&x, x_pixels, uint32_t(ci), l.ci_pitch, l.x_pixel, false);
