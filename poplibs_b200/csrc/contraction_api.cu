@@ -5,11 +5,13 @@
 
 #include <algorithm>
 #include <cmath>
+#include <utility>
 #include <vector>
 
 #include "conv_geometry.h"
 #include "grouped.h"
 #include "runtime.h"
+#include "igemm_sm100.cuh"
 #include "sm100_prims.cuh"
 
 namespace plb {
@@ -242,7 +244,7 @@ void setTaps(IgemmProblem *r, const ConvShape &s, int first_h, int step_h, int f
 // What the passes have in common: operand types, weights, options.  `w_rows` is
 // the number of rows of a stored weight tile (its second dimension).
 IgemmProblem passProblem(const plb_conv_params &p, const plb_conv_options *opt, const ConvShape &s,
-                         const PassOperands &o, bool b_mn, uint64_t w_cols, uint64_t w_rows) {
+                         const PassOperands &o, bool b_mn, uint64_t w_rows) {
   const size_t es = dtypeBytes(o.type);
   IgemmProblem r;
   r.fp8 = o.type == PLB_QUARTER;
@@ -253,7 +255,7 @@ IgemmProblem passProblem(const plb_conv_params &p, const plb_conv_options *opt, 
   r.act_group_stride = uint64_t(o.act_pitch) * es;
   r.wgt = o.wgt;
   r.b_mn = b_mn;
-  r.wgt_dims[0] = w_cols;
+  r.wgt_dims[0] = o.w_pitch;  // (what rows were rounded up by holds zeros)
   r.wgt_dims[1] = w_rows;
   r.wgt_dims[2] = uint64_t(p.groups) * s.KHs * s.KWs;
   r.wgt_strides[0] = uint64_t(o.w_pitch) * es;
@@ -273,7 +275,7 @@ void setActs(IgemmProblem *r, const plb_conv_params &p, const PassOperands &o, i
   const size_t es = dtypeBytes(o.type);
   const uint64_t ctot = uint64_t(p.groups) * o.act_pitch;
   r->act = static_cast<const uint8_t *>(o.act) + (size_t(h0) * W + w0) * ctot * es;
-  r->act_dims[0] = o.k;
+  r->act_dims[0] = std::max(o.act_pitch, o.k);  // (likewise)
   r->act_strides[0] = ctot * es;
   r->act_strides[1] = uint64_t(W) * ctot * es;
   r->act_strides[2] = uint64_t(H) * W * ctot * es;
@@ -293,7 +295,7 @@ IgemmProblem convFwdProblem(const plb_conv_params &p, const plb_conv_options *op
                             bool flipped_taps = false) {
   const size_t os = dtypeBytes(p.output_type);
   const uint64_t co = p.out_chans_per_group, cotot = uint64_t(p.groups) * co;
-  IgemmProblem r = swapped_weights ? passProblem(p, opt, s, o, true, co, o.k) : passProblem(p, opt, s, o, false, o.k, co);
+  IgemmProblem r = swapped_weights ? passProblem(p, opt, s, o, true, o.k) : passProblem(p, opt, s, o, false, co);
   // the truncated input is a view: same strides, shifted base, smaller extents
   setActs(&r, p, o, s.H, s.W, s.tH, s.tW);
   if (o.lattice) {
@@ -350,7 +352,7 @@ IgemmProblem convBwdProblem(const plb_conv_params &p, const plb_conv_options *op
   const size_t os = dtypeBytes(p.output_type);
   const uint64_t ci = p.in_chans_per_group, ctot = uint64_t(p.groups) * ci;
   // transposed: [tap flipped][Ci][Co], a K-major operand with the taps already reversed
-  IgemmProblem r = weights_transposed ? passProblem(p, opt, s, o, false, o.k, ci) : passProblem(p, opt, s, o, true, ci, o.k);
+  IgemmProblem r = weights_transposed ? passProblem(p, opt, s, o, false, ci) : passProblem(p, opt, s, o, true, o.k);
   // computed part of the output gradients / used part of the input gradients
   setActs(&r, p, o, s.OH, s.OW, s.opH, s.opW);
   r.act_dims[1] = uint64_t(s.OWc);
@@ -461,7 +463,7 @@ int prepareOperands(plb_context *ctx, int type, const void *act, uint64_t rows, 
   size_t offset[2] = {0, 0}, total = 0;
   int n = 0;
   if (unfit(act, cols)) {
-    o->act_pitch = is_float ? roundToVec(3 * uint64_t(cols), 2) : roundToVec(cols, es);
+    o->act_pitch = is_float ? roundToRow(3 * uint64_t(cols), 2) : roundToRow(cols, es);
     jobs[n] = Repack{act, nullptr, rows, cols, cols, o->act_pitch, uint32_t(es),
                      is_float ? kRepackSplitCols : kRepackCopy, false, 0, {}};
     if (lattice) {
@@ -473,7 +475,7 @@ int prepareOperands(plb_context *ctx, int type, const void *act, uint64_t rows, 
   }
   if (unfit(wgt, w_cols)) {
     const bool along_rows = is_float && w_k_rows == 0;
-    o->w_pitch = along_rows ? roundToVec(3 * uint64_t(w_cols), 2) : roundToVec(w_cols, is_float ? 2 : es);
+    o->w_pitch = along_rows ? roundToRow(3 * uint64_t(w_cols), 2) : roundToRow(w_cols, is_float ? 2 : es);
     jobs[n] = Repack{wgt, nullptr, w_rows, w_cols, w_cols, o->w_pitch, uint32_t(es),
                      !is_float ? kRepackCopy : along_rows ? kRepackSplitCols : kRepackSplitPlanes, true, w_k_rows, {}};
     operand[n++] = &o->wgt;
@@ -497,7 +499,7 @@ int prepareOperands(plb_context *ctx, int type, const void *act, uint64_t rows, 
 // [G][flipped tap][cols][rows -> pitch].
 int transposedWeights(plb_context *ctx, const void *w, uint32_t groups, uint64_t taps, uint32_t rows, uint32_t cols,
                       const void **out, uint32_t *pitch) {
-  *pitch = roundToVec(rows, 1);
+  *pitch = roundToRow(rows, 1);
   void *ws = nullptr;
   if (int rc = scratch(ctx, kSlotOperands, size_t(groups) * taps * cols * *pitch + 256, &ws)) return rc;
   *out = ws;
@@ -513,8 +515,10 @@ template <typename V>
 __global__ void __launch_bounds__(256)
 zeroPhasesKernel(V *__restrict__ dst, uint32_t H, uint32_t W, uint32_t h0, uint32_t w0, uint32_t He, uint32_t We,
                  uint32_t str_h, uint32_t str_w, uint64_t rows_used, uint64_t cols_used, uint32_t vecs) {
-  pdl_launch_dependents();
+  // (in this order: the launches that follow write other positions and start beside
+  // this one, but behind what came before it, see IgemmChain)
   pdl_wait();
+  pdl_launch_dependents();
   const uint32_t h = blockIdx.x % He, n = blockIdx.x / He;
   V *row = dst + ((size_t(n) * H + h0 + h) * W + w0) * vecs;
   const bool all = !(rows_used >> (h % str_h) & 1);
@@ -555,8 +559,9 @@ int zeroPhases(plb_context *ctx, void *dx, const plb_conv_params &p, const ConvS
 // fixed, evenly spaced subset of the filter taps (a sub-lattice of the stored
 // filter), so each phase is a stride-1 convolution of the output gradients with
 // that sub-filter, written to the strided sub-lattice of the input gradient.
-// `separate`: `p` contracts groups together; each phase's outputs are repaired from
-// these operands of the separate groups (`separate_p`).
+// The phases write disjoint positions: they are one chain of launches (IgemmChain).
+// `separate`: `p` contracts groups together; the outputs are repaired from these
+// operands of the separate groups (`separate_p`).
 int convBwdStrided(plb_context *ctx, const plb_conv_params &p, const plb_conv_options *opt, const ConvShape &s,
                    const PassOperands &o, void *dx, bool weights_transposed, const plb_conv_params *separate_p,
                    const PassOperands *separate) {
@@ -577,54 +582,62 @@ int convBwdStrided(plb_context *ctx, const plb_conv_params &p, const plb_conv_op
     if (pw[size_t(b)].extent && pw[size_t(b)].taps == 0) any_empty = true;
     if (pw[size_t(b)].taps && b < 64) cols_used |= uint64_t(1) << b;
   }
+  bool lead_done = false;
   if (any_empty && !s.zero_fill_in) {  // (otherwise the caller has cleared it)
     if (s.strH <= 64 && s.strW <= 64) {
       if (int rc = zeroPhases(ctx, dx, p, s, rows_used, cols_used)) return rc;
+      lead_done = true;
     } else {
       PLB_CUDA(cudaMemsetAsync(dx, 0, size_t(p.batch) * s.H * s.W * ctot * os, ctx->stream));
     }
   }
+  std::vector<std::pair<IgemmProblem, plb_plan>> phases;
+  bool chain = true;
   for (int a = 0; a < s.strH; ++a)
     for (int b = 0; b < s.strW; ++b) {
       const BwdPhase &A = ph[size_t(a)], &B = pw[size_t(b)];
       if (A.extent == 0 || B.extent == 0 || A.taps == 0 || B.taps == 0) continue;
-      auto phase = [&](const plb_conv_params &pp, const PassOperands &oo, bool weights_transposed) {
-        IgemmProblem r = convBwdProblem(pp, opt, s, oo, dx, weights_transposed);
-        r.out_w = B.extent;
-        r.out_h = A.extent;
-        r.taps_h = A.taps;
-        r.taps_w = B.taps;
-        // tap j of the phase is used tap first + j*step of the (possibly flipped)
-        // filter, stored where the flip, the truncation and (weights_transposed)
-        // the reversal of all stored taps put it
-        auto stored = [&](int used, int K, int Ks, int kt, int flip) {
-          const int at = kt + (flip ? K - 1 - used : used);
-          return weights_transposed ? Ks - 1 - at : at;
-        };
-        const int h0 = stored(A.first_tap, s.KH, s.KHs, s.ktH, s.flipH);
-        const int w0 = stored(B.first_tap, s.KW, s.KWs, s.ktW, s.flipW);
-        setTaps(&r, s, h0, (s.flipH != 0) != weights_transposed ? -A.step : A.step, w0,
-                (s.flipW != 0) != weights_transposed ? -B.step : B.step);
-        // position i of the phase reads output index i + offset - j*dil for its
-        // j-th tap: a correlation with the taps reversed
-        r.dil_h = A.dil;
-        r.dil_w = B.dil;
-        r.pad_h = (A.taps - 1) * A.dil - A.offset;
-        r.pad_w = (B.taps - 1) * B.dil - B.offset;
-        r.flip_h = 1;
-        r.flip_w = 1;
-        r.out = static_cast<uint8_t *>(dx) + (size_t(s.tH + a) * s.W + (s.tW + b)) * ctot * os;
-        r.ldc = (long long)(ctot * s.strW);
-        r.out_stride_h = (long long)(ctot * s.W * s.strH);
-        return r;
+      IgemmProblem r = convBwdProblem(p, opt, s, o, dx, weights_transposed);
+      r.out_w = B.extent;
+      r.out_h = A.extent;
+      r.taps_h = A.taps;
+      r.taps_w = B.taps;
+      // tap j of the phase is used tap first + j*step of the (possibly flipped)
+      // filter, stored where the flip, the truncation and (weights_transposed)
+      // the reversal of all stored taps put it
+      auto stored = [&](int used, int K, int Ks, int kt, int flip) {
+        const int at = kt + (flip ? K - 1 - used : used);
+        return weights_transposed ? Ks - 1 - at : at;
       };
-      IgemmProblem r = phase(p, o, weights_transposed);
+      const int h0 = stored(A.first_tap, s.KH, s.KHs, s.ktH, s.flipH);
+      const int w0 = stored(B.first_tap, s.KW, s.KWs, s.ktW, s.flipW);
+      setTaps(&r, s, h0, (s.flipH != 0) != weights_transposed ? -A.step : A.step, w0,
+              (s.flipW != 0) != weights_transposed ? -B.step : B.step);
+      // position i of the phase reads output index i + offset - j*dil for its
+      // j-th tap: a correlation with the taps reversed
+      r.dil_h = A.dil;
+      r.dil_w = B.dil;
+      r.pad_h = (A.taps - 1) * A.dil - A.offset;
+      r.pad_w = (B.taps - 1) * B.dil - B.offset;
+      r.flip_h = 1;
+      r.flip_w = 1;
+      r.out = static_cast<uint8_t *>(dx) + (size_t(s.tH + a) * s.W + (s.tW + b)) * ctot * os;
+      r.ldc = (long long)(ctot * s.strW);
+      r.out_stride_h = (long long)(ctot * s.W * s.strH);
       if (separate) r.nonfinite = nonfiniteFlag(ctx);
-      if (int rc = runProblem(ctx, r)) return rc;
-      if (separate)
-        if (int rc = repairNonFinite(ctx, phase(*separate_p, *separate, false), separate->type)) return rc;
+      r.plan_flags |= ctx->plan_flags;
+      plb_plan plan{};
+      if (int rc = planIgemm(r, ctx->sm_count, &plan)) return rc;
+      if (plan.split_k > 1) chain = false;  // (the partial sums share one scratch buffer)
+      phases.emplace_back(r, plan);
     }
-  return PLB_OK;
+  for (auto &[r, plan] : phases) {
+    if (chain && phases.size() + (lead_done ? 1 : 0) > 1) r.chain = lead_done ? kChainFollow : kChainLead;
+    lead_done = true;
+    if (int rc = launchIgemm(ctx, r, plan)) return rc;
+  }
+  if (!separate || phases.empty()) return PLB_OK;
+  return repairNonFinite(ctx, convBwdProblem(*separate_p, opt, s, *separate, dx, false), separate->type, s.strH, s.strW);
 }
 
 // Narrow channel groups are contracted together (grouped.cu): `q` = the layer of
@@ -713,25 +726,27 @@ int plb_matmul(plb_context *ctx, const plb_matmul_desc *desc, const void *d_a, c
   long long lda = ld.a, ldb = ld.b;
   bool a_is_km = d.transpose_a != 0, b_is_nk = d.transpose_b != 0;
   if (d.input_type == PLB_QUARTER && (a_is_km || !b_is_nk)) {
-    const size_t a_bytes = a_is_km ? (size_t(d.groups) * d.m * d.k + 255) & ~size_t(255) : 0;
-    const size_t b_bytes = b_is_nk ? 0 : size_t(d.groups) * d.n * d.k;
+    // (rows of whole 16-byte vectors, so that nothing has to be copied again)
+    const uint64_t pitch = roundToRow(d.k, 1);
+    const size_t a_bytes = a_is_km ? (size_t(d.groups) * d.m * pitch + 255) & ~size_t(255) : 0;
+    const size_t b_bytes = b_is_nk ? 0 : size_t(d.groups) * d.n * pitch;
     void *ws = nullptr;
     if (int rc = scratch(ctx, kSlotOperands, a_bytes + b_bytes, &ws)) return rc;
     if (a_is_km) {
       if (ld.a != (long long)d.m)
         return fail(PLB_ERR_UNSUPPORTED, "transposed quarter A must be densely packed");
-      if (int rc = plb_transpose_matrix(ctx, 1, d.groups, d.k, d.m, d_a, ws)) return rc;
+      if (int rc = transposeBatch(ctx, 1, d.groups, d.k, d.m, d_a, ws, pitch)) return rc;
       a = ws;
-      lda = d.k;
+      lda = (long long)pitch;
       a_is_km = false;
     }
     if (!b_is_nk) {
       if (ld.b != (long long)d.n)
         return fail(PLB_ERR_UNSUPPORTED, "quarter B in [k][n] layout must be densely packed");
       uint8_t *bt = static_cast<uint8_t *>(ws) + a_bytes;
-      if (int rc = plb_transpose_matrix(ctx, 1, d.groups, d.k, d.n, d_b, bt)) return rc;
+      if (int rc = transposeBatch(ctx, 1, d.groups, d.k, d.n, d_b, bt, pitch)) return rc;
       b = bt;
-      ldb = d.k;
+      ldb = (long long)pitch;
       b_is_nk = true;
     }
   }
@@ -755,8 +770,8 @@ int plb_matmul(plb_context *ctx, const plb_matmul_desc *desc, const void *d_a, c
     auto add = [&](const void **base, long long *pitch, uint64_t rows, uint32_t cols, bool k_along_rows, bool weights) {
       if (!unfit(*base, *pitch)) return;
       const int mode = !is_float ? kRepackCopy : k_along_rows ? kRepackSplitPlanes : kRepackSplitCols;
-      const uint32_t pitch_out = mode == kRepackCopy ? roundToVec(cols, es)
-                                                     : roundToVec(mode == kRepackSplitCols ? 3 * uint64_t(cols) : cols, 2);
+      const uint32_t pitch_out = mode == kRepackCopy ? roundToRow(cols, es)
+                                                     : roundToRow(mode == kRepackSplitCols ? 3 * uint64_t(cols) : cols, 2);
       jobs[n] = Repack{*base, nullptr, rows, cols, uint64_t(*pitch), pitch_out, uint32_t(es), mode, weights, d.k, {}};
       *pitch = pitch_out;
       operand[n++] = base;
@@ -878,8 +893,8 @@ int plb_conv_plan(const plb_conv_params *p_in, const plb_conv_options *opt, int3
   run.out_chans_per_group *= together;
   const bool bwd = pass == PLB_PASS_TRAINING_BWD;
   PassOperands o{run.input_type, nullptr, nullptr, bwd ? run.out_chans_per_group : run.in_chans_per_group, 0, 0};
-  o.act_pitch = roundToVec(o.k, dtypeBytes(run.input_type));
-  o.w_pitch = roundToVec(run.in_chans_per_group, dtypeBytes(run.input_type));
+  o.act_pitch = roundToRow(o.k, dtypeBytes(run.input_type));
+  o.w_pitch = roundToRow(run.in_chans_per_group, dtypeBytes(run.input_type));
   const IgemmProblem q = bwd ? convBwdProblem(run, opt, s, o, nullptr, run.input_type == PLB_QUARTER)
                              : convFwdProblem(run, opt, s, o, nullptr, nullptr);
   if (q.n_total > 0 && q.out_w > 0 && q.out_h > 0 && q.out_n > 0 && q.k_per_tap > 0)

@@ -50,7 +50,7 @@ blockDiagonalKernel(const T *__restrict__ src, T *__restrict__ dst, uint32_t S, 
 struct RepairArgs {
   const uint8_t *act, *wgt;
   uint64_t act_dims[4], act_strides[3], act_group_stride, wgt_strides[2];
-  int b_mn, k, taps_h, taps_w, pad_h, pad_w, dil_h, dil_w, stride_h, stride_w, flip_h, flip_w;
+  int b_mn, k, taps_h, taps_w, pad_h, pad_w, dil_h, dil_w, stride_h, stride_w, flip_h, flip_w, in_dil_h, in_dil_w;
   int tap_first_h, tap_step_h, tap_pitch_h, tap_first_w, tap_step_w, taps_stored;
   int groups, n_total, out_w, out_h, out_n;
   void *out;
@@ -94,8 +94,10 @@ __global__ void __launch_bounds__(128) repairKernel(const RepairArgs a, const in
       const int th = t / a.taps_w, tw = t - th * a.taps_w;
       const long long ih = (long long)oh * a.stride_h + th * a.dil_h - a.pad_h;
       const long long iw = (long long)ow * a.stride_w + tw * a.dil_w - a.pad_w;
-      if (ih < 0 || iw < 0 || ih >= (long long)a.act_dims[2] || iw >= (long long)a.act_dims[1]) continue;
-      const uint8_t *x = a.act + on * a.act_strides[2] + ih * a.act_strides[1] + iw * a.act_strides[0] +
+      if (ih < 0 || iw < 0 || ih % a.in_dil_h != 0 || iw % a.in_dil_w != 0) continue;
+      const long long xh = ih / a.in_dil_h, xw = iw / a.in_dil_w;
+      if (xh >= (long long)a.act_dims[2] || xw >= (long long)a.act_dims[1]) continue;
+      const uint8_t *x = a.act + on * a.act_strides[2] + xh * a.act_strides[1] + xw * a.act_strides[0] +
                          g * a.act_group_stride;
       const int tile = ((a.flip_h ? a.taps_h - 1 - th : th) * a.tap_step_h + a.tap_first_h) * a.tap_pitch_h +
                        (a.flip_w ? a.taps_w - 1 - tw : tw) * a.tap_step_w + a.tap_first_w + g * a.taps_stored;
@@ -155,7 +157,7 @@ int blockDiagonalWeights(plb_context *ctx, int type, const void *src, uint32_t g
   return es == 1 ? launch(uint8_t()) : es == 2 ? launch(uint16_t()) : launch(uint32_t());
 }
 
-int repairNonFinite(plb_context *ctx, const IgemmProblem &p, int type) {
+int repairNonFinite(plb_context *ctx, const IgemmProblem &p, int type, int in_dil_h, int in_dil_w) {
   RepairArgs a{};
   a.act = static_cast<const uint8_t *>(p.act);
   a.wgt = static_cast<const uint8_t *>(p.wgt);
@@ -175,6 +177,8 @@ int repairNonFinite(plb_context *ctx, const IgemmProblem &p, int type) {
   a.stride_w = p.stride_w;
   a.flip_h = p.flip_h;
   a.flip_w = p.flip_w;
+  a.in_dil_h = in_dil_h;
+  a.in_dil_w = in_dil_w;
   a.tap_first_h = p.tap_first_h;
   a.tap_step_h = p.tap_step_h;
   a.tap_pitch_h = p.tap_pitch_h ? p.tap_pitch_h : p.taps_w;

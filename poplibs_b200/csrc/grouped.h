@@ -15,6 +15,8 @@ int blockDiagonalWeights(plb_context *ctx, int type, const void *src, uint32_t g
                          uint32_t rows, uint32_t cols, const void **out);
 // Recomputes the outputs of `p` that are not finite if the flag is set.  `p`
 // describes the separate groups on the caller's operands (of type `type`).
-int repairNonFinite(plb_context *ctx, const IgemmProblem &p, int type);
+// Input position i of the problem is element i / in_dil of the operand (none if the
+// division leaves a rest).
+int repairNonFinite(plb_context *ctx, const IgemmProblem &p, int type, int in_dil_h = 1, int in_dil_w = 1);
 
 }  // namespace plb

@@ -549,6 +549,7 @@ int launchIgemm(plb_context *ctx, const IgemmProblem &p, const plb_plan &plan) {
   a.beta = split ? 0.f : p.beta;
   a.out_is_f32 = split || p.out_f32 ? 1 : 0;
   a.nonfinite = p.nonfinite;
+  a.chain = split ? kChainNone : p.chain;
   a.status = ctx->d_status;
   a.trace = ctx->trace;
 

@@ -61,6 +61,14 @@ constexpr int kIgemmMmaWarp2 = 2;  // second MMA issuer (short tiles), else the 
 constexpr int kEpiStagingBytes = 8 * 4096;  // 8 pairs of epilogue warps x (32 rows x 128 B)
 static_assert(kIgemmProducers > kIgemmMmaWarp2 && kIgemmProducers <= 3, "producer warps are warps 0..2");
 
+// Launches that write disjoint parts of one result and read nothing of one another
+// (the phases of a strided layer's input gradient) run side by side where SMs are
+// free: the first (kChainLead, or any kernel that waits for its predecessor before
+// it lets dependents start) orders the others behind everything earlier in the
+// stream; the followers do not wait for their predecessor before they read, but
+// before they end, so that the completion of the last is the completion of all.
+enum IgemmChain : int { kChainNone = 0, kChainLead = 1, kChainFollow = 2 };
+
 struct IgemmArgs {
   // ---- M side: output pixels, tiled by a (w, h, n) box of 128 pixels ------
   int box_w, box_h, box_n;
@@ -114,6 +122,7 @@ struct IgemmArgs {
   FastDiv fd_split;
   long long split_stride;
   int dual_issue;  // two MMA-issuing threads take alternate tiles
+  int chain;       // IgemmChain
   uint32_t idesc_formats;  // operand format bits of the instruction descriptor (8-bit operands: 1 = E5M2)
   // ---- epilogue ---------------------------------------------------------------
   void *out;
@@ -293,7 +302,11 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
   // operands, which have no architectural effect) and calls pdl_wait() itself
   // right before its first access.
   if (threadIdx.x == 0) PLB_TRACE_STAMP(2, 4001);
+  if (args.chain == kChainLead) pdl_wait();
   pdl_launch_dependents();
+  auto wait_predecessor = [&]() {
+    if (args.chain != kChainFollow) pdl_wait();
+  };
 
   // Work units: output tiles, or with a CTA pair, pairs of M tiles (the odd
   // last one is padded: its copies read zeros and its stores are clipped).
@@ -489,7 +502,7 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
     const int w_base = w0 * args.stride_w - args.pad_w, h_base = h0 * args.stride_h - args.pad_h;
     issue_step(true, dst, full, f_group, r, s, kc, w_base, h_base, n0, n_idx * BN);
     if (!load) return;
-    pdl_wait();
+    wait_predecessor();
     if (leader)
       mbar_expect_tx(full_bar(i), kPairFactor * uint32_t(args.stage_tx_bytes));
     issue_step(false, dst, full, f_group, r, s, kc, w_base, h_base, n0, n_idx * BN);
@@ -506,7 +519,7 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
       [[maybe_unused]] int trace_slot = 0;
       if constexpr (kResB)
         for (int i = me; i < first_steps; i += P) first_step(i, false);
-      pdl_wait();
+      wait_predecessor();
       if (me == 0) PLB_TRACE_STAMP(2, 4002);
       for (int unit = first_unit; unit < total_units && ok; unit += unit_stride) {
         if (me == 0) { PLB_TRACE_STAMP(0, trace_slot); ++trace_slot; }
@@ -757,7 +770,7 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
           step_coords(it, r, s, kc);
           load_b(0u, 0u, f_group, r, s, kc, 0, true);
         }
-        pdl_wait();
+        wait_predecessor();
         if (warp == 4 && leader)
           mbar_expect_tx(resb_bar, kPairFactor * uint32_t(k_iters * args.b_box_bytes));
         const uint32_t resb_bar_lead = lead_bar(resb_bar);
@@ -775,7 +788,7 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
       }
       __syncwarp();
     }
-    pdl_wait();
+    wait_predecessor();
     for (int unit = first_unit + group * unit_stride; unit < total_units;
          unit += 2 * unit_stride, local_tile += 2) {
       int tile, cgroup, split, it_begin, it_end;
@@ -984,6 +997,7 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
   }
 
   if (threadIdx.x == 0) PLB_TRACE_STAMP(2, 4003);
+  if (args.chain == kChainFollow) pdl_wait();
   tc_fence_before_sync();
   // Every tensor copy must have landed before the CTA gives up its shared
   // memory.  In a run without errors the MMA issuer has waited for every

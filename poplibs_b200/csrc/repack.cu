@@ -112,12 +112,12 @@ repackKernel(const RepackArgs first, const RepackArgs second, unsigned first_blo
     const float *x = reinterpret_cast<const float *>(src);
     __align__(16) uint16_t o[3][8];
     if (a.mode == kRepackSplitCols && a.cols % 8 == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
-      // the eight elements are neighbours and of one piece
+      // the eight elements are neighbours and of one piece (or beyond the last)
       const uint32_t piece = v * 8 / a.cols, col = v * 8 - piece * a.cols;
       const float4 f0 = *reinterpret_cast<const float4 *>(x + col), f1 = *reinterpret_cast<const float4 *>(x + col + 4);
       const float f[8] = {f0.x, f0.y, f0.z, f0.w, f1.x, f1.y, f1.z, f1.w};
 #pragma unroll
-      for (int j = 0; j < 8; ++j) o[0][j] = floatPiece(f[j], int(piece), a.weights);
+      for (int j = 0; j < 8; ++j) o[0][j] = piece < 3 ? floatPiece(f[j], int(piece), a.weights) : uint16_t(0);
       *reinterpret_cast<uint4 *>(a.dst + (row * a.vecs + v) * 16) = *reinterpret_cast<const uint4 *>(o[0]);
     } else if (a.mode == kRepackSplitCols) {
       // (piece, column) of the eight elements

@@ -100,63 +100,95 @@ int encodeTensorMap(CUtensorMap *tm, CUtensorMapDataType type, int rank, const v
 // Data-movement kernels
 // ---------------------------------------------------------------------------
 
-// Batched transpose src[b][rows][cols] -> dst[b][cols][rows] through a padded
-// shared-memory tile so that both sides are coalesced.
+// Batched transpose src[b][rows][cols] -> dst[b][cols][dst_pitch] (what lies between
+// `rows` and the pitch is not written) through a 64 x 64 tile in shared memory, so that
+// both sides are coalesced: four-byte words (V elements) where a side's rows start
+// on them, else elements, always several accesses in flight per thread.  The tile's
+// row pitch of 17 words leaves the column reads at most two to a bank.
+// 4392 x 1592 bytes: 15.6 us as 32 x 32 tiles of single elements, now 4.6.
 template <typename T>
-__global__ void transposeKernel(const T *__restrict__ src, T *__restrict__ dst, uint32_t rows,
-                                uint32_t cols) {
-  __shared__ T tile[32][33];
-  const size_t batch_off = size_t(blockIdx.z) * rows * cols;
-  const uint32_t c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
-  for (uint32_t i = threadIdx.y; i < 32; i += blockDim.y) {
-    const uint32_t r = r0 + i, c = c0 + threadIdx.x;
-    if (r < rows && c < cols) tile[i][threadIdx.x] = src[batch_off + size_t(r) * cols + c];
+__global__ void __launch_bounds__(256)
+transposeKernel(const T *__restrict__ src, T *__restrict__ dst, uint32_t rows, uint32_t cols, uint32_t dst_pitch,
+                int src_words, int dst_words) {
+  constexpr int V = 4 / int(sizeof(T)), kTile = 16 * V, kPitch = 17 * V;
+  __shared__ __align__(16) T tile[kTile * kPitch];
+  pdl_launch_dependents();
+  const T *s = src + size_t(blockIdx.z) * rows * cols;
+  T *d = dst + size_t(blockIdx.z) * cols * dst_pitch;
+  const uint32_t c0 = blockIdx.x * kTile, r0 = blockIdx.y * kTile;
+  const uint32_t w = threadIdx.x & 15, k = threadIdx.x >> 4;  // word of a row, row
+  pdl_wait();  // the matrix may come from the previous kernel in the stream
+  if (src_words && c0 + kTile <= cols) {
+    uint32_t v[V];
+#pragma unroll
+    for (int i = 0; i < V; ++i)
+      if (r0 + k + 16 * i < rows) v[i] = *reinterpret_cast<const uint32_t *>(s + size_t(r0 + k + 16 * i) * cols + c0 + w * V);
+#pragma unroll
+    for (int i = 0; i < V; ++i) *reinterpret_cast<uint32_t *>(&tile[(k + 16 * i) * kPitch + w * V]) = v[i];
+  } else {
+    constexpr int n = kTile * kTile / 256;
+    T v[n];
+#pragma unroll
+    for (int i = 0; i < n; ++i) {
+      const uint32_t e = threadIdx.x + 256 * i, r = r0 + e / kTile, c = c0 + e % kTile;
+      if (r < rows && c < cols) v[i] = s[size_t(r) * cols + c];
+    }
+#pragma unroll
+    for (int i = 0; i < n; ++i) {
+      const uint32_t e = threadIdx.x + 256 * i;
+      tile[e / kTile * kPitch + e % kTile] = v[i];
+    }
   }
   __syncthreads();
-  for (uint32_t i = threadIdx.y; i < 32; i += blockDim.y) {
-    const uint32_t c = c0 + i, r = r0 + threadIdx.x;
-    if (r < rows && c < cols) dst[batch_off + size_t(c) * rows + r] = tile[threadIdx.x][i];
+#pragma unroll
+  for (int i = 0; i < V; ++i) {
+    const uint32_t c = k + 16 * i, r = w * V;  // V rows of column c
+    if (c0 + c >= cols || r0 + r >= rows) continue;
+    T v[V];
+#pragma unroll
+    for (int j = 0; j < V; ++j) v[j] = tile[(r + j) * kPitch + c];
+    T *out = d + size_t(c0 + c) * dst_pitch + r0 + r;
+    if (dst_words && r0 + r + V <= rows) {
+      uint32_t word = 0;
+#pragma unroll
+      for (int j = 0; j < V; ++j) word |= uint32_t(v[j]) << (32 / V * j % 32);
+      *reinterpret_cast<uint32_t *>(out) = word;
+    } else {
+#pragma unroll
+      for (int j = 0; j < V; ++j)
+        if (r0 + r + j < rows) out[j] = v[j];
+    }
   }
 }
 
-static int launchTranspose(plb_context *ctx, uint32_t elem_bytes, uint64_t batch, uint64_t rows,
-                           uint64_t cols, const void *src, void *dst) {
+int transposeBatch(plb_context *ctx, uint32_t elem_bytes, uint64_t batch, uint64_t rows, uint64_t cols, const void *src,
+                   void *dst, uint64_t dst_pitch) {
   if (batch == 0 || rows == 0 || cols == 0) return PLB_OK;
-  if (rows > 0xffffffffull || cols > 0xffffffffull)
+  if (rows > 0xffffffffull || cols > 0xffffffffull || dst_pitch > 0xffffffffull)
     return fail(PLB_ERR_UNSUPPORTED, "matrix too large to transpose");
-  const dim3 block(32, 8);
-  const uint64_t gy = (rows + 31) / 32, gx = (cols + 31) / 32;
-  if (gy > 65535 || batch > 65535) {
-    // fold: process batches one launch at a time / split rows
-    if (gy > 65535) return fail(PLB_ERR_UNSUPPORTED, "matrix too tall to transpose");
-  }
+  if (elem_bytes != 1 && elem_bytes != 2 && elem_bytes != 4)
+    return fail(PLB_ERR_INVALID_PARAMS, "element size must be 1, 2 or 4 bytes");
+  const uint64_t tile = 16 * (4 / elem_bytes), gx = (cols + tile - 1) / tile;
+  const uint64_t strip = 65535 * tile;  // rows per launch
+  const int dst_words = (dst_pitch * elem_bytes) % 4 == 0 && (reinterpret_cast<uintptr_t>(dst) & 3) == 0;
+  const int src_words = (cols * elem_bytes) % 4 == 0 && (reinterpret_cast<uintptr_t>(src) & 3) == 0;
+  if (rows > strip) return fail(PLB_ERR_UNSUPPORTED, "matrix too tall to transpose");
   for (uint64_t b0 = 0; b0 < batch; b0 += 65535) {
-    const uint32_t nb = uint32_t(std::min<uint64_t>(65535, batch - b0));
-    const dim3 grid(uint32_t(gx), uint32_t(gy), nb);
-    const size_t off = size_t(b0) * rows * cols;
-    switch (elem_bytes) {
-      case 1:
-        transposeKernel<uint8_t><<<grid, block, 0, ctx->stream>>>(
-            static_cast<const uint8_t *>(src) + off, static_cast<uint8_t *>(dst) + off,
-            uint32_t(rows), uint32_t(cols));
-        break;
-      case 2:
-        transposeKernel<uint16_t><<<grid, block, 0, ctx->stream>>>(
-            static_cast<const uint16_t *>(src) + off, static_cast<uint16_t *>(dst) + off,
-            uint32_t(rows), uint32_t(cols));
-        break;
-      case 4:
-        transposeKernel<uint32_t><<<grid, block, 0, ctx->stream>>>(
-            static_cast<const uint32_t *>(src) + off, static_cast<uint32_t *>(dst) + off,
-            uint32_t(rows), uint32_t(cols));
-        break;
-      default:
-        return fail(PLB_ERR_INVALID_PARAMS, "element size must be 1, 2 or 4 bytes");
-    }
-    PLB_CUDA(cudaGetLastError());
-    ctx->launches++;
+    const dim3 grid(uint32_t(gx), uint32_t((rows + tile - 1) / tile), uint32_t(std::min<uint64_t>(65535, batch - b0)));
+    auto launch = [&](auto t) {
+      using T = decltype(t);
+      return launchPdl(ctx, transposeKernel<T>, grid, dim3(256), 0, static_cast<const T *>(src) + b0 * rows * cols,
+                       static_cast<T *>(dst) + b0 * cols * dst_pitch, uint32_t(rows), uint32_t(cols), uint32_t(dst_pitch),
+                       src_words, dst_words);
+    };
+    if (int rc = elem_bytes == 1 ? launch(uint8_t()) : elem_bytes == 2 ? launch(uint16_t()) : launch(uint32_t())) return rc;
   }
   return PLB_OK;
+}
+
+static int launchTranspose(plb_context *ctx, uint32_t elem_bytes, uint64_t batch, uint64_t rows, uint64_t cols,
+                           const void *src, void *dst) {
+  return transposeBatch(ctx, elem_bytes, batch, rows, cols, src, dst, rows);
 }
 
 // [G][K][Co][Ci] -> [G][K flipped][Ci][Co -> co_pitch]; weights are small, one element per thread.

@@ -57,105 +57,46 @@ __device__ __forceinline__ void foldWeightsAndTail(const S2dShape &g, unsigned b
     reinterpret_cast<uint4 *>(x2 + size_t(g.N) * g.H2 * g.W2 * g.C2)[threadIdx.x] = make_uint4(0u, 0u, 0u, 0u);
 }
 
-// X2[n][h2][w2][(ph*s + pw)*Cp + c] = X[n][h2*s + ph - padH][w2*s + pw - padW][c]
+// X2[n][h2][w2][(ph*s + pw)*Cp + c] = X[n][h2*s + ph - padH][w2*s + pw - padW][c],
+// zero outside the input and for channels C..Cp-1.  One thread per 16-byte vector of
+// X2, its up to eight elements loaded independently of one another: they are
+// neighbours of what the neighbouring threads load, so L1 serves most of them, and
+// with nothing staged or shared between threads every block has all its loads in
+// flight at once (staging rows in shared memory behind two barriers took 9.4 us for
+// 98 images of 60x161x1, now 3.0).  Blocks past the first `row_blocks` fold the
+// weights and clear the tail of X2.
+// kCp: Cp where it is one of the usual ones (divisions by constants), else 0.
+template <int kS, int kCp>
 __global__ void __launch_bounds__(128)
-s2dInputKernel(const __half *__restrict__ x, __half *__restrict__ x2, S2dShape g, unsigned row_blocks,
-               const __half *__restrict__ w, __half *__restrict__ w2, int co_total) {
+s2dInputKernel(const __half *__restrict__ x, __half *__restrict__ x2, S2dShape g, FastDiv fd_row, FastDiv fd_h2,
+               unsigned row_blocks, const __half *__restrict__ w, __half *__restrict__ w2, int co_total) {
+  const unsigned vecs = kCp ? unsigned(kS * kS * kCp / 8) : unsigned(g.C2) / 8;  // per pixel of X2
   pdl_launch_dependents();
   pdl_wait();
   if (blockIdx.x >= row_blocks) {
     foldWeightsAndTail(g, blockIdx.x - row_blocks, x2, w, w2, co_total);
     return;
   }
-  // one thread per 8 output halves (16 bytes)
-  const size_t vecs_per_pixel = size_t(g.C2) / 8;
-  const size_t total = size_t(g.N) * g.H2 * g.W2 * vecs_per_pixel;
-  for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < total;
-       i += size_t(row_blocks) * blockDim.x) {
-    const int v = int(i % vecs_per_pixel);
-    size_t r = i / vecs_per_pixel;
-    const int w2 = int(r % g.W2);
-    r /= g.W2;
-    const int h2 = int(r % g.H2);
-    const int n = int(r / g.H2);
-    __align__(16) __half vals[8];
+  // the block's first vector in 64 bits, the rest relative to its row in 32
+  const unsigned per_row = unsigned(g.W2) * vecs;
+  const unsigned long long base = blockIdx.x * 128ull, row0 = base / per_row;
+  const unsigned rel = unsigned(base - row0 * per_row) + threadIdx.x, down = fast_div(rel, fd_row);
+  const unsigned row = unsigned(row0) + down;
+  if (row >= unsigned(g.N) * unsigned(g.H2)) return;
+  const unsigned at = rel - down * per_row, pix = at / vecs, v = at - pix * vecs;
+  const unsigned n = fast_div(row, fd_h2);
+  const int h0 = int(row - n * unsigned(g.H2)) * kS - g.padH, w0 = int(pix) * kS - g.padW;
+  __align__(16) uint16_t vals[8];
+  const uint16_t *img = reinterpret_cast<const uint16_t *>(x) + size_t(n) * g.H * g.W * g.C;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int c2 = v * 8 + j;
-      const int sub = c2 / g.Cp, c = c2 - sub * g.Cp;
-      const int ph = sub / g.s, pw = sub - ph * g.s;
-      const int ih = h2 * g.s + ph - g.padH, iw = w2 * g.s + pw - g.padW;
-      __half val = __float2half(0.f);
-      if (c < g.C && ih >= 0 && ih < g.H && iw >= 0 && iw < g.W)
-        val = x[((size_t(n) * g.H + ih) * g.W + iw) * g.C + c];
-      vals[j] = val;
-    }
-    *reinterpret_cast<uint4 *>(x2 + i * 8) = *reinterpret_cast<const uint4 *>(vals);
+  for (int j = 0; j < 8; ++j) {
+    const int cp = kCp ? kCp : g.Cp;
+    const int c2 = int(v) * 8 + j, sub = kS == 1 ? 0 : c2 / cp, c = c2 - sub * cp;
+    const int ih = h0 + sub / kS, iw = w0 + sub % kS;
+    const bool in = c < g.C && unsigned(ih) < unsigned(g.H) && unsigned(iw) < unsigned(g.W);
+    vals[j] = in ? img[((long long)ih * g.W + iw) * g.C + c] : uint16_t(0);
   }
-}
-
-// The same rearrangement, one (n, h2) row of X2 per block iteration: the s
-// input rows that feed it are staged in shared memory with coalesced loads
-// (16-byte vectors when the rows are 16-byte aligned), then every thread
-// assembles 16-byte output vectors from them.  `lut` maps a channel of X2 to
-// (ph, pw, c) once per block instead of dividing per element.
-// Blocks past the first `row_blocks` fold the weights and clear the tail of X2.
-__global__ void __launch_bounds__(128)
-s2dInputRowsKernel(const __half *__restrict__ x, __half *__restrict__ x2, S2dShape g,
-                   int rows_aligned, unsigned row_blocks, const __half *__restrict__ w, __half *__restrict__ w2,
-                   int co_total) {
-  pdl_launch_dependents();
-  pdl_wait();
-  if (blockIdx.x >= row_blocks) {
-    foldWeightsAndTail(g, blockIdx.x - row_blocks, x2, w, w2, co_total);
-    return;
-  }
-  extern __shared__ __align__(16) unsigned char s2d_smem[];
-  const int row_elems = g.W * g.C;
-  const int row_stride = (row_elems + 7) & ~7;  // halves; keeps every staged row 16-byte aligned
-  __half *rows = reinterpret_cast<__half *>(s2d_smem);
-  int *lut = reinterpret_cast<int *>(s2d_smem + size_t(g.s) * row_stride * 2);
-  for (int c2 = threadIdx.x; c2 < g.C2; c2 += blockDim.x) {
-    const int sub = c2 / g.Cp, c = c2 - sub * g.Cp;
-    const int ph = sub / g.s, pw = sub - ph * g.s;
-    lut[c2] = c < g.C ? (ph << 16) | (pw << 8) | c : -1;
-  }
-  const int vecs_per_pixel = g.C2 / 8;
-  const int out_vecs = g.W2 * vecs_per_pixel;
-  for (int blk = blockIdx.x; blk < g.N * g.H2; blk += int(row_blocks)) {
-    const int n = blk / g.H2, h2 = blk - n * g.H2;
-    __syncthreads();  // previous iteration's readers are done (and the table is written)
-    for (int ph = 0; ph < g.s; ++ph) {
-      const int ih = h2 * g.s + ph - g.padH;
-      if (ih < 0 || ih >= g.H) continue;  // block-uniform
-      const __half *src = x + (size_t(n) * g.H + ih) * row_elems;
-      __half *dst = rows + ph * row_stride;
-      if (rows_aligned) {
-        const uint4 *src4 = reinterpret_cast<const uint4 *>(src);
-        uint4 *dst4 = reinterpret_cast<uint4 *>(dst);
-        for (int v = threadIdx.x; v < row_elems / 8; v += blockDim.x) dst4[v] = src4[v];
-      } else {
-        for (int e = threadIdx.x; e < row_elems; e += blockDim.x) dst[e] = src[e];
-      }
-    }
-    __syncthreads();
-    __half *out_row = x2 + size_t(blk) * g.W2 * g.C2;
-    for (int o = threadIdx.x; o < out_vecs; o += blockDim.x) {
-      const int w2 = o / vecs_per_pixel, v = o - w2 * vecs_per_pixel;
-      __align__(16) __half vals[8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const int code = lut[v * 8 + j];
-        const int ph = code >> 16, pw = (code >> 8) & 0xff, c = code & 0xff;
-        const int ih = h2 * g.s + ph - g.padH, iw = w2 * g.s + pw - g.padW;
-        __half val = __float2half(0.f);
-        if (code >= 0 && ih >= 0 && ih < g.H && iw >= 0 && iw < g.W)
-          val = rows[ph * row_stride + iw * g.C + c];
-        vals[j] = val;
-      }
-      *reinterpret_cast<uint4 *>(out_row + size_t(o) * 8) = *reinterpret_cast<const uint4 *>(vals);
-    }
-  }
+  *reinterpret_cast<uint4 *>(x2 + (base + threadIdx.x) * 8) = *reinterpret_cast<const uint4 *>(vals);
 }
 
 // The same rearrangement for the common stem shape (3 channels, stride 2, so
@@ -269,6 +210,8 @@ int smallChannelShape(const plb_conv_params &p, S2dShape *out) {
                     std::to_string(g.K2w * g.C2) + " elements exceeds one 128-byte K step");
   g.H2 = g.OH + g.K2h - 1;
   g.W2 = g.OW + g.K2w - 1;
+  if (uint64_t(g.N) * g.H2 >= uint64_t(1) << 31 || uint64_t(g.N) * g.H2 * g.W2 * (g.C2 / 8) >= uint64_t(1) << 37)
+    return fail(PLB_ERR_UNSUPPORTED, "small-channel convolution: too many rows");
   *out = g;
   return PLB_OK;
 }
@@ -281,26 +224,25 @@ size_t smallChannelElems(const S2dShape &g) { return size_t(g.N) * g.H2 * g.W2 *
 int smallChannelPrepare(plb_context *ctx, const S2dShape &g, const void *d_in, __half *x2, const void *d_weights,
                         __half *w2, int co) {
   const size_t w2_elems = w2 ? size_t(g.K2h) * co * 64 : 0;
-  const int row_elems = g.W * g.C;
-  const size_t smem = size_t(g.s) * ((row_elems + 7) & ~7) * 2 + size_t(g.C2) * sizeof(int);
   // (at least one block past the rows: it clears the tail of X2)
   const unsigned wblocks = unsigned(std::max<size_t>(1, (w2_elems + 127) / 128));
   const __half *w = static_cast<const __half *>(d_weights);
   const int w_co = w2 ? co : 0;
-  if (g.C == 3 && g.s == 2 && g.Cp == 4 && row_elems % 2 == 0 &&
-      (reinterpret_cast<uintptr_t>(d_in) & 3) == 0 && size_t(g.N) * g.H2 < (size_t(1) << 31))
+  if (g.C == 3 && g.s == 2 && g.Cp == 4 && (g.W * g.C) % 2 == 0 && (reinterpret_cast<uintptr_t>(d_in) & 3) == 0)
     return launchPdl(ctx, s2dStem3Kernel, dim3(unsigned(g.N) * unsigned(g.H2) + wblocks), dim3(128), 0,
                      static_cast<const uint32_t *>(d_in), reinterpret_cast<uint4 *>(x2), g, w, w2, w_co);
-  const __half *x = static_cast<const __half *>(d_in);
-  if (smem <= 48 * 1024 && g.C < 256 && g.s < 256) {
-    const int rows_aligned = (row_elems % 8 == 0 && (reinterpret_cast<uintptr_t>(d_in) & 15) == 0) ? 1 : 0;
-    const unsigned blocks = unsigned(std::min<size_t>(size_t(g.N) * g.H2, size_t(ctx->sm_count) * 16));
-    return launchPdl(ctx, s2dInputRowsKernel, dim3(blocks + wblocks), dim3(128), smem, x, x2, g, rows_aligned, blocks, w,
-                     w2, w_co);
-  }
   const size_t vecs = size_t(g.N) * g.H2 * g.W2 * (g.C2 / 8);
-  const unsigned blocks = unsigned(std::min<size_t>((vecs + 127) / 128, size_t(ctx->sm_count) * 32));
-  return launchPdl(ctx, s2dInputKernel, dim3(blocks + wblocks), dim3(128), 0, x, x2, g, blocks, w, w2, w_co);
+  const unsigned blocks = unsigned((vecs + 127) / 128);
+  auto launch = [&](auto kernel) {
+    return launchPdl(ctx, kernel, dim3(blocks + wblocks), dim3(128), 0, static_cast<const __half *>(d_in), x2, g,
+                     make_fastdiv(unsigned(g.W2) * unsigned(g.C2 / 8)), make_fastdiv(unsigned(g.H2)), blocks, w, w2, w_co);
+  };
+  if (g.s == 1) return g.Cp == 8 ? launch(s2dInputKernel<1, 8>) : launch(s2dInputKernel<1, 0>);
+  switch (g.Cp) {
+    case 2: return launch(s2dInputKernel<2, 2>);
+    case 4: return launch(s2dInputKernel<2, 4>);
+    default: return launch(s2dInputKernel<2, 0>);
+  }
 }
 
 int convFwdSmallChannels(plb_context *ctx, const plb_conv_params &p, const plb_conv_options *opt,

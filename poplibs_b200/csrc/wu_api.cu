@@ -3,6 +3,7 @@
 #include <cstdlib>
 #include <mutex>
 #include <string>
+#include <type_traits>
 
 #include "conv_geometry.h"
 #include "runtime.h"
@@ -89,7 +90,7 @@ struct WuLayout {
 // dense blocks of 128 x 128 instead of 32 launches whose tiles are 15/16 padding.
 // A super-group has to start on a 16-byte boundary; only where no number of groups
 // does are the channels of each group rounded up.
-WuLayout wuLayout(uint32_t groups, uint32_t ci, uint32_t co) {
+WuLayout wuLayout(uint32_t groups, uint32_t ci, uint32_t co, bool copied = false) {
   WuLayout l{};
   const uint32_t most = std::max<uint32_t>(1, std::min(groups, std::min(128 / std::max(co, 1u), 128 / std::max(ci, 1u))));
   auto quantum = [](uint32_t c) {
@@ -106,8 +107,11 @@ WuLayout wuLayout(uint32_t groups, uint32_t ci, uint32_t co) {
     l.co_pitch = roundToVec(co, 2);
     l.sub = std::max<uint32_t>(1, std::min(groups, std::min(128 / l.co_pitch, 128 / l.ci_pitch)));
   }
-  l.x_pixel = roundToVec(uint64_t(groups) * l.ci_pitch, 2);
-  l.dy_pixel = roundToVec(uint64_t(groups) * l.co_pitch, 2);
+  // (`copied`: both tensors are copied in any case)
+  auto pixel = [&](uint64_t chans) { return copied || chans % 8 != 0 ? roundToRow(chans, 2) : uint32_t(chans); };
+  // where each group is rounded up on its own, pixels are those rows side by side
+  l.x_pixel = l.ci_pitch != ci ? groups * l.ci_pitch : pixel(uint64_t(groups) * ci);
+  l.dy_pixel = l.co_pitch != co ? groups * l.co_pitch : pixel(uint64_t(groups) * co);
   return l;
 }
 
@@ -126,8 +130,10 @@ WuProblem wuProblem(const plb_conv_params &p, const WuShape &s, const WuLayout &
   q.ci = int(q.sgroups == 1 ? roundToVec(sub * ci_pitch, 2) : sub * ci_pitch);
   q.co = int(q.sgroups == 1 ? roundToVec(sub * co_pitch, 2) : sub * co_pitch);
   q.s = s;
-  q.x_chans = std::min<uint64_t>(l.x_pixel, uint64_t(q.sgroups) * q.ci);
-  q.dy_chans = std::min<uint64_t>(l.dy_pixel, uint64_t(q.sgroups) * q.co);
+  // what a super-group reads beyond its own channels only meets sums that nothing
+  // reads; the end of the pixel is the end of the tensor
+  q.x_chans = std::max<uint64_t>(uint64_t(groups) * ci_pitch, l.x_pixel * (p.groups == groups ? 1 : 0));
+  q.dy_chans = std::max<uint64_t>(uint64_t(groups) * co_pitch, l.dy_pixel * (p.groups == groups ? 1 : 0));
   const uint64_t xp = l.x_pixel * es, yp = l.dy_pixel * es;
   q.x_strides[0] = xp;
   q.x_strides[1] = uint64_t(s.W) * xp;
@@ -332,8 +338,11 @@ int launchWuReduce(cudaStream_t stream, const WuArgs &a, size_t w_elems, void *d
                                 a.ksplit, count4, pa, reinterpret_cast<float4 *>(d_weight_grads_f32),
                                 reinterpret_cast<uint2 *>(out16)));
   } else if (gather == nullptr && vec) {
-    const cudaLaunchConfig_t cfg = wuReduceConfig(stream, (count4 + 31) / 32, pdl);
-    PLB_CUDA(cudaLaunchKernelEx(&cfg, wu_reduce4_kernel, reinterpret_cast<const float4 *>(a.partial), a.ksplit,
+    // (up to 8 splits, one thread per sum adds in the same order as eight lanes)
+    const bool single = a.ksplit <= kWuReduceLanes && count4 >= size_t(148) * 512;
+    cudaLaunchConfig_t cfg = wuReduceConfig(stream, single ? (count4 + 255) / 256 : (count4 + 31) / 32, pdl);
+    if (single) cfg.blockDim = dim3(256, 1);
+    PLB_CUDA(cudaLaunchKernelEx(&cfg, single ? wu_reduce4_kernel<1> : wu_reduce4_kernel<kWuReduceLanes>, reinterpret_cast<const float4 *>(a.partial), a.ksplit,
                                 count4, reinterpret_cast<float4 *>(d_weight_grads_f32),
                                 reinterpret_cast<uint2 *>(out16)));
   } else {
@@ -349,15 +358,35 @@ int launchWuReduce(cudaStream_t stream, const WuArgs &a, size_t w_elems, void *d
     g.split_stride = (unsigned long long)a.sgroups * a.taps_h * a.taps_w * a.co_total * a.ci_total;
     g.total = w_elems;
     // four channels at once where they are neighbours on both sides
-    if (vec && g.ci % 4 == 0 && g.ci_pitch % 4 == 0) {
-      const cudaLaunchConfig_t cfg = wuReduceConfig(stream, (count4 + 31) / 32, pdl);
-      PLB_CUDA(cudaLaunchKernelEx(&cfg, wu_gather_kernel<4>, (const float *)a.partial, a.ksplit, g,
-                                  d_weight_grads_f32, out16));
-    } else {
-      const cudaLaunchConfig_t cfg = wuReduceConfig(stream, (w_elems + 31) / 32, pdl);
-      PLB_CUDA(cudaLaunchKernelEx(&cfg, wu_gather_kernel<1>, (const float *)a.partial, a.ksplit, g,
-                                  d_weight_grads_f32, out16));
-    }
+    const int V = vec && g.ci % 4 == 0 && g.ci_pitch % 4 == 0 ? 4 : 1;
+    const size_t vectors = w_elems / V;
+    g.fd_ci = make_fastdiv(g.ci / V);
+    g.fd_co = make_fastdiv(g.co);
+    g.fd_taps = make_fastdiv(g.taps);
+    g.fd_sub = make_fastdiv(g.sub);
+    // as few threads per sum as fill the device: each then has several loads in flight
+    int lanes = 1;
+    while (lanes < 8 && lanes < a.ksplit && vectors * lanes < size_t(148) * 1024) lanes *= 2;
+    auto launch = [&](auto kernel, int L) {
+      const size_t per_block = size_t(kWuReduceThreads / L);
+      cudaLaunchConfig_t cfg = wuReduceConfig(stream, (vectors + per_block - 1) / per_block, pdl);
+      cfg.blockDim = dim3(kWuReduceThreads);
+      return cudaLaunchKernelEx(&cfg, kernel, (const float *)a.partial, a.ksplit, g, d_weight_grads_f32, out16);
+    };
+    auto dispatch = [&](auto v) {
+      constexpr int kV = decltype(v)::value;
+      if (vectors >= (size_t(1) << 31)) return launch(wu_gather_kernel<kV, 8, true>, 8);
+      switch (lanes) {
+        case 1: return launch(wu_gather_kernel<kV, 1, false>, 1);
+        case 2: return launch(wu_gather_kernel<kV, 2, false>, 2);
+        case 4: return launch(wu_gather_kernel<kV, 4, false>, 4);
+        default: return launch(wu_gather_kernel<kV, 8, false>, 8);
+      }
+    };
+    if (V == 4)
+      PLB_CUDA(dispatch(std::integral_constant<int, 4>()));
+    else
+      PLB_CUDA(dispatch(std::integral_constant<int, 1>()));
   }
   PLB_CUDA(cudaGetLastError());
   return PLB_OK;
@@ -701,7 +730,7 @@ int plb_conv_wu(plb_context *ctx, const plb_conv_params *p, const plb_conv_optio
   // bfloat16 pieces side by side.  The padded rows and columns of the partial sums
   // are not read.
   const bool is_float = p->input_type == PLB_FLOAT;
-  const WuLayout l = wuLayout(p->groups, uint32_t(ci), uint32_t(co));
+  const WuLayout l = wuLayout(p->groups, uint32_t(ci), uint32_t(co), is_float);
   const uint64_t x_pixels = uint64_t(p->batch) * s.H * s.W, dy_pixels = uint64_t(p->batch) * s.OH * s.OW;
   const void *x = d_acts, *dy = d_out_grads;
   {

@@ -100,7 +100,7 @@ def test_ragged_and_grouped_products(gpu_ctx, groups, m, k, n, dtype):
 
 
 @pytest.mark.parametrize("kernel,stride", [(7, 2), (3, 1), (3, 2), (1, 1), (5, 2)])
-@pytest.mark.parametrize("chans", [1, 2, 3, 4, 5, 7])
+@pytest.mark.parametrize("chans", [1, 2, 3, 4, 5, 7, 12, 20])
 def test_first_layer_weight_gradient(gpu_ctx, chans, kernel, stride):
     """Few input channels: the gradient from the rearranged input (where a folded
     filter row fits 64 elements) and from rounded-up channels (where it does not)."""
@@ -116,3 +116,19 @@ def test_first_layer_weight_gradient(gpu_ctx, chans, kernel, stride):
         exact(dw32, oracle.conv_wu(spec, x, dy)[0], f"wu width {width} co {co}")
         exact(dw16, dw32.astype(np.float16), "half gradient")
         exact(T.gpu_conv_fwd(p, x, w), oracle.conv_fwd(spec, x, w), f"fwd width {width} co {co}")
+
+
+@pytest.mark.parametrize("elem", [1, 2, 4])
+@pytest.mark.parametrize("rows,cols", [(1, 1), (3, 130), (64, 64), (65, 63), (128, 96), (33, 257), (200, 4), (1000, 72)])
+def test_transpose(gpu_ctx, elem, rows, cols):
+    """Whole and partial tiles; rows that start on four-byte words on both sides, one or neither."""
+    import torch
+    dtype = {1: np.uint8, 2: np.uint16, 4: np.uint32}[elem]
+    a = T.rng(rows + cols).integers(0, 256 ** elem, (3, rows, cols), dtype=np.uint64).astype(dtype)
+    src = torch.from_numpy(a.view(np.uint8)).cuda()
+    dst = torch.empty(a.nbytes, dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    T.context().transpose_matrix(elem, 3, rows, cols, src, dst)
+    T.context().synchronize()
+    got = dst.cpu().numpy().view(dtype).reshape(3, cols, rows)
+    assert np.array_equal(got, a.transpose(0, 2, 1))
