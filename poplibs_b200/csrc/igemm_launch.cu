@@ -200,11 +200,16 @@ int planIgemm(const IgemmProblem &p, int sm_count, plb_plan *plan) {
   // ---- split-K ---------------------------------------------------------------
   // A product with few output tiles and a long reduction leaves most SMs idle:
   // let several CTAs share a tile, each taking a range of its pipeline steps,
-  // and add their fp32 partial sums in a second kernel.  Model (microseconds):
-  // a pipeline step of one CTA takes about 0.17 (the producers' issue rate
-  // bounds short tiles), the extra kernel about 5 plus its traffic at a few
-  // TB/s; the split must save more than it costs.  512 x 1024 x 1024 stays
-  // unsplit (16 steps: 2.7 against 1.4 + 5), 256 x 8192 x 256 splits.
+  // and add their fp32 partial sums in a second kernel.  Model (microseconds): a
+  // pipeline step of one CTA takes about 0.15 per weight tile that it streams, more
+  // where an operand's rows begin at odd multiples of 16 bytes (0.24 for a left operand
+  // of 1800 columns, 0.28 with a right one of 200 too: such rows are copied in more,
+  // partly filled sectors); the second kernel 3.4 plus the partial sums written and read at 4 TB/s (MB per
+  // microsecond below); the split must save more than it costs.  From sweeps of long
+  // products and of small images: 128 x 2048 x 64 splits (8.3 -> 7.0 us), so do 3x3
+  // layers of 256 and 512 channels on one 14 x 14 image (8.6 -> 7.5, 13.7 -> 9.3);
+  // 512 x 1024 x 1024 and 256 channels on four such images stay whole (6.1 against
+  // 7.8, 8.7 against 9.7).
   {
     const long units = plan->tiles / (pair ? 2 : 1) + (pair ? plan->tiles % 2 : 0);
     const long steps = plan->halo_rows > 0 ? long(p.taps_w) * ((p.k_per_tap + k_elems - 1) / k_elems)
@@ -213,11 +218,14 @@ int planIgemm(const IgemmProblem &p, int sm_count, plb_plan *plan) {
     int split = 1;
     if (p.force_split_k > 0) {
       split = int(std::min<long>(p.force_split_k, steps));
-    } else if (units * 2 <= sms && steps >= 16) {
+    } else if (const int b_tiles = plan->halo_rows > 0 && !plan->resident_weights ? p.taps_h : 1;
+               units * 2 <= sms && steps * b_tiles >= 20) {
       const double out_mb = double(groups) * p.out_w * p.out_h * p.out_n * p.n_total * 4 / 1e6;
-      double best = 0.17 * double(steps);
-      for (long sp = 2; sp <= std::min<long>(steps / 4, sms / units); ++sp) {
-        const double t = 0.17 * double((steps + sp - 1) / sp) + 5.0 + out_mb * double(sp + 1) / 4000.0;
+      const double odd_rows = (p.act_strides[0] % 32 != 0 ? 0.09 : 0.0) + (p.wgt_strides[0] % 32 != 0 ? 0.045 : 0.0);
+      const double step_us = 0.15 * b_tiles + odd_rows;
+      double best = step_us * double(steps);
+      for (long sp = 2; sp <= std::min<long>(steps * b_tiles / 4, std::min(steps, sms / units)); ++sp) {
+        const double t = step_us * double((steps + sp - 1) / sp) + 3.4 + out_mb * double(sp + 1) / 4.0;
         if (t < best) {
           best = t;
           split = int(sp);
