@@ -27,7 +27,10 @@ struct RepackArgs {
   unsigned long long rows, src_pitch;  // src_pitch in bytes
   uint32_t cols;                       // elements of a row
   uint32_t vecs;                       // 16-byte vectors of a destination row
-  FastDiv fd_vecs;
+  uint32_t units;                      // steps per row: vecs, or groups of elements (kSplitCols)
+  uint32_t group;                      // elements a thread splits at a time (kSplitCols), 8 or 2
+  int aligned;                         // kSplitCols: pairs start at multiples of 8 bytes
+  FastDiv fd_units;
   uint32_t elem_bytes;
   int mode;                            // RepackMode
   int weights;                         // pieces (hi, hi, lo) instead of (hi, lo, hi)
@@ -37,15 +40,23 @@ struct RepackArgs {
 
 constexpr int kRepackThreads = 256;
 constexpr int kRepackPerThread = 2;
+constexpr int kSplitPerThread = 4;  // kSplitCols in pairs
 
-// `bytes` (a multiple of G) bytes from an address aligned to G, zero beyond `valid`
-template <typename G>
+// The first `valid` bytes from any address, zero beyond, out of the up to five aligned
+// words that hold them.
 __device__ __forceinline__ uint4 gatherBytes(const uint8_t *src, int valid) {
-  constexpr int n = 16 / int(sizeof(G));
-  __align__(16) G g[n];
+  const uint32_t off = uint32_t(reinterpret_cast<uintptr_t>(src)) & 3, bytes = uint32_t(min(valid, 16));
+  const uint32_t *at = reinterpret_cast<const uint32_t *>(src - off);
+  uint32_t w[5], o[4];
 #pragma unroll
-  for (int j = 0; j < n; ++j) g[j] = int(j * sizeof(G)) < valid ? reinterpret_cast<const G *>(src)[j] : G(0);
-  return *reinterpret_cast<const uint4 *>(g);
+  for (int j = 0; j < 5; ++j) w[j] = 4 * j < off + bytes ? at[j] : 0u;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    o[j] = __funnelshift_r(w[j], w[j + 1], off * 8);
+    const int n = int(bytes) - 4 * j;
+    if (n < 4) o[j] = n <= 0 ? 0u : o[j] & ((1u << (8 * n)) - 1);
+  }
+  return make_uint4(o[0], o[1], o[2], o[3]);
 }
 
 // Piece 0..2 of a float.  An infinity or NaN stays in the first piece alone: in
@@ -59,12 +70,179 @@ __device__ __forceinline__ uint16_t floatPiece(float x, int piece, int weights) 
   return __bfloat16_as_ushort(low ? __float2bfloat16_rn(x - __bfloat162float(hi)) : hi);
 }
 
-// One 16-byte destination vector per step (three in kSplitPlanes).  Rows start
-// anywhere, so a vector is gathered with the widest loads its source address
-// allows; neighbouring threads read neighbouring bytes, and the overlap of their
-// narrow loads is caught by L1.  Bound by those loads (4.5 TB/s at 2 bytes per
-// lane), which beats what a byte per thread with two divisions reached 10 to 20
-// times over.  Both operands of a call go in one launch.
+// The pieces of two floats, packed.
+struct Pieces {
+  uint32_t piece[3];
+};
+__device__ __forceinline__ Pieces splitPair(float x, float y, int weights) {
+  const __nv_bfloat162 hi = __floats2bfloat162_rn(x, y);
+  const float2 back = __bfloat1622float2(hi);
+  const __nv_bfloat162 lo = __floats2bfloat162_rn(x - back.x, y - back.y);
+  const uint32_t finite = (isfinite(x) ? 0xffffu : 0u) | (isfinite(y) ? 0xffff0000u : 0u);
+  const uint32_t h = *reinterpret_cast<const uint32_t *>(&hi);
+  const uint32_t h2 = h & finite, l = *reinterpret_cast<const uint32_t *>(&lo) & finite;
+  return Pieces{{h, weights ? h2 : l, weights ? l : h2}};
+}
+
+// The source row of a destination row.
+__device__ __forceinline__ unsigned long long sourceRow(const RepackArgs &a, unsigned long long row) {
+  if (a.sub_w == 0) return row;
+  // row = (image, h, w, part) of the sub-lattice
+  const uint32_t per_w = uint32_t(row / a.parts), part = uint32_t(row - (unsigned long long)per_w * a.parts);
+  const uint32_t rows = per_w / a.sub_w, w = per_w - rows * a.sub_w, n = rows / a.sub_h, h = rows - n * a.sub_h;
+  return (((unsigned long long)n * a.full_h + h * a.step_h) * a.full_w + w * a.step_w) * a.parts + part;
+}
+
+// Both splits below: a thread loads neighbouring floats once and stores their three
+// pieces; steps beyond the columns zero the row's padding, and all of a thread's steps
+// load before any of them stores.  Destination vectors gathered one by one instead load
+// and convert each float three times, with the lanes' loads 32 bytes apart.
+
+// kSplitCols, eight floats at a time (16-byte aligned rows of a multiple of 8):
+// 6689 rows of 1104 floats 27 -> 11 us.
+__device__ __forceinline__ void splitEights(const RepackArgs &a, unsigned long long row0, uint32_t rest) {
+  const uint32_t in_row = a.cols / 8;
+  __align__(16) float f[kRepackPerThread][8];
+  uint4 *dst[kRepackPerThread];
+  bool pad[kRepackPerThread];
+#pragma unroll
+  for (int u = 0; u < kRepackPerThread; ++u) {
+    const uint32_t i = rest + uint32_t(u) * kRepackThreads + threadIdx.x;
+    const uint32_t down = fast_div(i, a.fd_units);
+    const uint32_t v = i - down * a.units;
+    const unsigned long long row = row0 + down;
+    dst[u] = nullptr;
+    if (row >= a.rows) continue;
+    pad[u] = v >= in_row;
+    dst[u] = reinterpret_cast<uint4 *>(a.dst) + row * a.vecs + (pad[u] ? 2 * in_row : 0) + v;
+    if (pad[u]) continue;
+    const float4 *x = reinterpret_cast<const float4 *>(a.src + sourceRow(a, row) * a.src_pitch) + 2 * v;
+    *reinterpret_cast<float4 *>(&f[u][0]) = x[0];
+    *reinterpret_cast<float4 *>(&f[u][4]) = x[1];
+  }
+#pragma unroll
+  for (int u = 0; u < kRepackPerThread; ++u) {
+    if (dst[u] == nullptr) continue;
+    if (pad[u]) {
+      *dst[u] = make_uint4(0u, 0u, 0u, 0u);
+      continue;
+    }
+    Pieces o[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) o[j] = splitPair(f[u][2 * j], f[u][2 * j + 1], a.weights);
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+      dst[u][k * in_row] = make_uint4(o[0].piece[k], o[1].piece[k], o[2].piece[k], o[3].piece[k]);
+  }
+}
+
+// kSplitCols, two floats at a time.  Every store is 4 bytes and aligned, which in a row
+// of odd length the second pieces are one element earlier.  kAligned: rows of even length
+// at multiples of 8 bytes.  6689 rows of 1102 and of 1103 floats 45 -> 17 and
+// 21 us.
+template <bool kAligned>
+__device__ __forceinline__ void splitPairs(const RepackArgs &a, unsigned long long row0, uint32_t rest) {
+  const uint32_t odd = kAligned ? 0 : a.cols & 1, pitch = a.vecs * 8;
+  float f[kSplitPerThread][3];
+  uint16_t *dst[kSplitPerThread];
+  uint32_t col[kSplitPerThread];
+#pragma unroll
+  for (int u = 0; u < kSplitPerThread; ++u) {
+    const uint32_t i = rest + uint32_t(u) * kRepackThreads + threadIdx.x;
+    const uint32_t down = fast_div(i, a.fd_units);
+    const uint32_t c = 2 * (i - down * a.units);
+    const unsigned long long row = row0 + down;
+    dst[u] = nullptr;
+    if (row >= a.rows) continue;
+    dst[u] = reinterpret_cast<uint16_t *>(a.dst) + row * pitch + c;
+    col[u] = c;
+    if (c >= a.cols) continue;
+    const float *x = reinterpret_cast<const float *>(a.src + sourceRow(a, row) * a.src_pitch) + c;
+    if constexpr (kAligned) {
+      const float2 t = *reinterpret_cast<const float2 *>(x);
+      f[u][0] = t.x;
+      f[u][1] = t.y;
+    } else {
+      f[u][0] = x[0];
+      f[u][1] = c + 1 < a.cols ? x[1] : 0.f;
+      f[u][2] = odd && c ? x[-1] : 0.f;
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < kSplitPerThread; ++u) {
+    if (dst[u] == nullptr) continue;
+    const uint32_t c = col[u];
+    uint32_t *const third = reinterpret_cast<uint32_t *>(dst[u] + 2 * a.cols);
+    if (c >= a.cols) {  // the padding, from its first even element on
+      *third = 0u;
+      continue;
+    }
+    const Pieces o = splitPair(f[u][0], f[u][1], a.weights);
+    *third = o.piece[2];  // (an odd row's last: its element and the first of the padding)
+    if (!odd) {
+      *reinterpret_cast<uint32_t *>(dst[u]) = o.piece[0];
+      *reinterpret_cast<uint32_t *>(dst[u] + a.cols) = o.piece[1];
+      continue;
+    }
+    const Pieces q = splitPair(f[u][2], f[u][0], a.weights);  // the pair one element earlier
+    if (c + 1 < a.cols)
+      *reinterpret_cast<uint32_t *>(dst[u]) = o.piece[0];
+    else
+      *dst[u] = uint16_t(o.piece[0]);
+    if (c)
+      *reinterpret_cast<uint32_t *>(dst[u] + a.cols - 1) = q.piece[1];
+    else
+      dst[u][a.cols] = uint16_t(o.piece[1]);
+  }
+}
+
+// A step of kRepackCopy (one 16-byte destination vector) or kSplitPlanes (three).
+// Rows start anywhere, so a vector is gathered from the aligned words that hold it;
+// neighbouring threads read neighbouring bytes, and the overlap of their loads is
+// caught by L1.  Bound by those loads: five words beat 8 halves or 16 bytes (quarter
+// operands of 331 x 145 x 2588 8.5 -> 8.2 us with the product, half of 20000 x 33 x 40
+// 9.7 -> 9.0); one 4-byte destination word per step, or two 16-byte loads shifted into
+// place, were no faster.
+__device__ __forceinline__ void vectorStep(const RepackArgs &a, unsigned long long row, uint32_t v) {
+  const uint8_t *src = a.src + sourceRow(a, row) * a.src_pitch;
+  if (a.mode == kRepackCopy) {
+    const int valid = int(a.cols * a.elem_bytes) - int(v) * 16;
+    uint4 o = make_uint4(0u, 0u, 0u, 0u);
+    if (valid > 0) {
+      src += size_t(v) * 16;
+      const uintptr_t at = reinterpret_cast<uintptr_t>(src);
+      if ((at & 15) == 0 && valid >= 16)
+        o = *reinterpret_cast<const uint4 *>(src);
+      else
+        o = gatherBytes(src, valid);
+    }
+    *reinterpret_cast<uint4 *>(a.dst + (row * a.vecs + v) * 16) = o;
+    return;
+  }
+  const float *x = reinterpret_cast<const float *>(src) + v * 8;
+  __align__(16) uint16_t o[3][8];
+  __align__(16) float f[8];
+  if (v * 8 + 8 <= a.cols && (reinterpret_cast<uintptr_t>(x) & 15) == 0) {
+    *reinterpret_cast<float4 *>(&f[0]) = *reinterpret_cast<const float4 *>(x);
+    *reinterpret_cast<float4 *>(&f[4]) = *reinterpret_cast<const float4 *>(x + 4);
+  } else {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) f[j] = v * 8 + j < a.cols ? x[j] : 0.f;
+  }
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+#pragma unroll
+    for (int k = 0; k < 3; ++k) o[k][j] = floatPiece(f[j], k, a.weights);
+  const unsigned long long outer = a.mid < a.rows ? row / a.mid : 0, plane0 = outer * 2 * a.mid + row;
+#pragma unroll
+  for (int k = 0; k < 3; ++k)
+    *reinterpret_cast<uint4 *>(a.dst + ((plane0 + k * a.mid) * a.vecs + v) * 16) =
+        *reinterpret_cast<const uint4 *>(o[k]);
+}
+
+// Both operands of a call go in one launch.  kCols: one of them is kSplitCols (an
+// instance of its own, since it takes more registers).
+template <bool kCols>
 __global__ void __launch_bounds__(kRepackThreads)
 repackKernel(const RepackArgs first, const RepackArgs second, unsigned first_blocks) {
   pdl_launch_dependents();
@@ -72,91 +250,29 @@ repackKernel(const RepackArgs first, const RepackArgs second, unsigned first_blo
   const bool is_first = blockIdx.x < first_blocks;
   const RepackArgs &a = is_first ? first : second;
   const unsigned block = is_first ? blockIdx.x : blockIdx.x - first_blocks;
-  // the block's first vector in 64 bits, the rest relative to its row in 32
-  const unsigned long long base = (unsigned long long)block * (kRepackThreads * kRepackPerThread);
-  const unsigned long long row0 = base / a.vecs;
-  const uint32_t rest = uint32_t(base - row0 * a.vecs);
+  const bool cols = kCols && a.mode == kRepackSplitCols;
+  // the block's first step in 64 bits, the rest relative to its row in 32
+  const uint32_t per_thread = cols && a.group < 8 ? kSplitPerThread : kRepackPerThread;
+  const unsigned long long base = (unsigned long long)block * (kRepackThreads * per_thread);
+  const unsigned long long row0 = base / a.units;
+  const uint32_t rest = uint32_t(base - row0 * a.units);
+  if (cols) {
+    if (a.group == 8)
+      splitEights(a, row0, rest);
+    else if (a.aligned)
+      splitPairs<true>(a, row0, rest);
+    else
+      splitPairs<false>(a, row0, rest);
+    return;
+  }
 #pragma unroll
   for (int u = 0; u < kRepackPerThread; ++u) {
     const uint32_t i = rest + uint32_t(u) * kRepackThreads + threadIdx.x;
-    const uint32_t down = fast_div(i, a.fd_vecs);
-    const uint32_t v = i - down * a.vecs;
+    const uint32_t down = fast_div(i, a.fd_units);
+    const uint32_t v = i - down * a.units;
     const unsigned long long row = row0 + down;
     if (row >= a.rows) return;
-    unsigned long long src_row = row;
-    if (a.sub_w != 0) {
-      // row = (image, h, w, part) of the sub-lattice
-      const uint32_t per_w = uint32_t(row / a.parts), part = uint32_t(row - (unsigned long long)per_w * a.parts);
-      const uint32_t rows = per_w / a.sub_w, w = per_w - rows * a.sub_w, n = rows / a.sub_h, h = rows - n * a.sub_h;
-      src_row = (((unsigned long long)n * a.full_h + h * a.step_h) * a.full_w + w * a.step_w) * a.parts + part;
-    }
-    const uint8_t *src = a.src + src_row * a.src_pitch;
-    if (a.mode == kRepackCopy) {
-      const int valid = int(a.cols * a.elem_bytes) - int(v) * 16;
-      uint4 o = make_uint4(0u, 0u, 0u, 0u);
-      if (valid > 0) {
-        src += size_t(v) * 16;
-        const uintptr_t at = reinterpret_cast<uintptr_t>(src);
-        if ((at & 15) == 0 && valid >= 16)
-          o = *reinterpret_cast<const uint4 *>(src);
-        else if ((at & 3) == 0 && (valid & 3) == 0)
-          o = gatherBytes<uint32_t>(src, valid);
-        else if ((at & 1) == 0 && (valid & 1) == 0)
-          o = gatherBytes<uint16_t>(src, valid);
-        else
-          o = gatherBytes<uint8_t>(src, valid);
-      }
-      *reinterpret_cast<uint4 *>(a.dst + (row * a.vecs + v) * 16) = o;
-      continue;
-    }
-    const float *x = reinterpret_cast<const float *>(src);
-    __align__(16) uint16_t o[3][8];
-    if (a.mode == kRepackSplitCols && a.cols % 8 == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
-      // the eight elements are neighbours and of one piece (or beyond the last)
-      const uint32_t piece = v * 8 / a.cols, col = v * 8 - piece * a.cols;
-      const float4 f0 = *reinterpret_cast<const float4 *>(x + col), f1 = *reinterpret_cast<const float4 *>(x + col + 4);
-      const float f[8] = {f0.x, f0.y, f0.z, f0.w, f1.x, f1.y, f1.z, f1.w};
-#pragma unroll
-      for (int j = 0; j < 8; ++j) o[0][j] = piece < 3 ? floatPiece(f[j], int(piece), a.weights) : uint16_t(0);
-      *reinterpret_cast<uint4 *>(a.dst + (row * a.vecs + v) * 16) = *reinterpret_cast<const uint4 *>(o[0]);
-    } else if (a.mode == kRepackSplitCols) {
-      // (piece, column) of the eight elements
-      uint32_t piece = v * 8 / a.cols, col = v * 8 - piece * a.cols;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        o[0][j] = piece < 3 ? floatPiece(x[col], int(piece), a.weights) : uint16_t(0);
-        if (++col == a.cols) {
-          col = 0;
-          ++piece;
-        }
-      }
-      *reinterpret_cast<uint4 *>(a.dst + (row * a.vecs + v) * 16) = *reinterpret_cast<const uint4 *>(o[0]);
-    } else {
-      float f[8];
-      if (v * 8 + 8 <= a.cols && (reinterpret_cast<uintptr_t>(x) & 15) == 0) {
-        const float4 f0 = *reinterpret_cast<const float4 *>(x + v * 8), f1 = *reinterpret_cast<const float4 *>(x + v * 8 + 4);
-        f[0] = f0.x;
-        f[1] = f0.y;
-        f[2] = f0.z;
-        f[3] = f0.w;
-        f[4] = f1.x;
-        f[5] = f1.y;
-        f[6] = f1.z;
-        f[7] = f1.w;
-      } else {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) f[j] = v * 8 + j < a.cols ? x[v * 8 + j] : 0.f;
-      }
-#pragma unroll
-      for (int j = 0; j < 8; ++j)
-#pragma unroll
-        for (int k = 0; k < 3; ++k) o[k][j] = floatPiece(f[j], k, a.weights);
-      const unsigned long long outer = a.mid < a.rows ? row / a.mid : 0, plane0 = outer * 2 * a.mid + row;
-#pragma unroll
-      for (int k = 0; k < 3; ++k)
-        *reinterpret_cast<uint4 *>(a.dst + ((plane0 + k * a.mid) * a.vecs + v) * 16) =
-            *reinterpret_cast<const uint4 *>(o[k]);
-    }
+    vectorStep(a, row, v);
   }
 }
 
@@ -181,11 +297,20 @@ int repack(plb_context *ctx, const Repack *jobs, int n) {
     a.src_pitch = r.src_pitch * r.elem_bytes;
     a.cols = r.cols;
     a.vecs = uint32_t(size_t(r.dst_pitch) * (r.mode == kRepackCopy ? r.elem_bytes : 2) / 16);
-    a.fd_vecs = make_fastdiv(a.vecs);
     a.elem_bytes = r.elem_bytes;
     a.mode = r.mode;
     a.weights = r.weights ? 1 : 0;
     a.mid = r.mid ? r.mid : r.rows;
+    a.units = a.vecs;
+    if (r.mode == kRepackSplitCols) {
+      const auto starts_at = [&](unsigned bytes) {
+        return reinterpret_cast<uintptr_t>(r.src) % bytes == 0 && a.src_pitch % bytes == 0;
+      };
+      a.group = r.cols % 8 == 0 && starts_at(16) ? 8 : 2;
+      a.aligned = r.cols % 2 == 0 && starts_at(8);
+      a.units = (r.dst_pitch - 2 * r.cols) / a.group;  // columns and padding
+    }
+    a.fd_units = make_fastdiv(a.units);
     a.parts = r.lattice.parts;
     a.sub_w = r.lattice.sub_w;
     a.sub_h = r.lattice.sub_h;
@@ -193,14 +318,16 @@ int repack(plb_context *ctx, const Repack *jobs, int n) {
     a.full_h = r.lattice.full_h;
     a.step_w = r.lattice.step_w;
     a.step_h = r.lattice.step_h;
-    const uint64_t per_block = kRepackThreads * kRepackPerThread;
-    const uint64_t b = (r.rows * a.vecs + per_block - 1) / per_block;
-    if (b + blocks[0] > 0x7fffffffull || uint64_t(a.vecs) + per_block > 0x7fffffffull)
+    const uint64_t per_block =
+        kRepackThreads * (r.mode == kRepackSplitCols && a.group < 8 ? kSplitPerThread : kRepackPerThread);
+    const uint64_t b = (r.rows * a.units + per_block - 1) / per_block;
+    if (b + blocks[0] > 0x7fffffffull || uint64_t(a.units) + per_block > 0x7fffffffull)
       return fail(PLB_ERR_UNSUPPORTED, "operand too large to be repacked");
     blocks[used++] = unsigned(b);
   }
   if (used == 0) return PLB_OK;
-  return launchPdl(ctx, repackKernel, dim3(blocks[0] + blocks[1]), dim3(kRepackThreads), 0, args[0], args[1],
+  const bool any_cols = args[0].mode == kRepackSplitCols || (used > 1 && args[1].mode == kRepackSplitCols);
+  return launchPdl(ctx, any_cols ? repackKernel<true> : repackKernel<false>, dim3(blocks[0] + blocks[1]), dim3(kRepackThreads), 0, args[0], args[1],
                    blocks[0]);
 }
 

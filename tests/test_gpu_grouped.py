@@ -132,3 +132,24 @@ def test_transpose(gpu_ctx, elem, rows, cols):
     T.context().synchronize()
     got = dst.cpu().numpy().view(dtype).reshape(3, cols, rows)
     assert np.array_equal(got, a.transpose(0, 2, 1))
+
+
+@pytest.mark.parametrize("offset", [0, 1, 2])
+@pytest.mark.parametrize("k", [1, 2, 5, 7, 8, 16, 21, 24, 42, 43, 130, 343])
+def test_float_operands_are_split_in_place_order(gpu_ctx, k, offset):
+    """Both pieces of a float at every alignment of the rows: elements +-1 + j / 1024
+    (|j| <= 3) round to +-1 and leave j / 1024, so against integers every sum is exact."""
+    import torch
+    m, n, r = 37, 19, T.rng(k)
+    fine = lambda *s: (r.choice([-1, 1], s) + r.integers(-3, 4, s) / 1024).astype(np.float32)
+    whole = lambda *s: ints(r, s, np.float32)
+    d = capi.MatmulDesc.make(m, k, n, transpose_b=True, input_type=capi.FLOAT, output_type=capi.FLOAT)
+    for a, b in ((fine(m, k), whole(n, k)), (whole(m, k), fine(n, k))):
+        on = [torch.zeros(x.size + offset, device="cuda") for x in (a, b)]
+        for t, x in zip(on, (a, b)):
+            t[offset:] = torch.from_numpy(x.ravel())
+        out = torch.empty(m, n, device="cuda")
+        torch.cuda.synchronize()
+        T.context().matmul(d, on[0][offset:], on[1][offset:], None, out)
+        T.context().synchronize()
+        exact(out.cpu().numpy(), a.astype(np.float64) @ b.T.astype(np.float64), "split")
