@@ -854,7 +854,8 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
         if (c + c_step >= cols_end) release_accumulator();
         const int col0 = col_base + c;
         const int valid = min(32, args.n_total - col0);
-        if (args.nonfinite != nullptr) {
+        // (rows beyond the output hold whatever the stage's shared memory held before)
+        if (args.nonfinite != nullptr && row_ok) {
           uint32_t largest = 0u;
 #pragma unroll
           for (int j = 0; j < 32; ++j)
