@@ -39,8 +39,13 @@ struct RepackArgs {
 };
 
 constexpr int kRepackThreads = 256;
-constexpr int kRepackPerThread = 2;
-constexpr int kSplitPerThread = 4;  // kSplitCols in pairs
+// Steps of a thread: one in operands that fill the device no more than twice, where the
+// length of a block counts (160 x 1472 and 1472 x 1120 floats with the product 16.5 ->
+// 15.9 us); else as many loads as help: four vectors of a copy (37845 rows of 396 halves
+// with the product 26.8 -> 25.6 us), two steps of a split (four: 68.6 -> 70.4 us with
+// the product at 4032 x 5312 floats), but twice as many pairs, which are short.
+constexpr int kFewSteps = 1, kSplitSteps = 2, kCopySteps = 4;
+__host__ __device__ constexpr int pairSteps(int steps) { return 2 * steps; }
 
 // The first `valid` bytes from any address, zero beyond, out of the up to five aligned
 // words that hold them.
@@ -100,13 +105,14 @@ __device__ __forceinline__ unsigned long long sourceRow(const RepackArgs &a, uns
 
 // kSplitCols, eight floats at a time (16-byte aligned rows of a multiple of 8):
 // 6689 rows of 1104 floats 27 -> 11 us.
+template <int kPer>
 __device__ __forceinline__ void splitEights(const RepackArgs &a, unsigned long long row0, uint32_t rest) {
   const uint32_t in_row = a.cols / 8;
-  __align__(16) float f[kRepackPerThread][8];
-  uint4 *dst[kRepackPerThread];
-  bool pad[kRepackPerThread];
+  __align__(16) float f[kPer][8];
+  uint4 *dst[kPer];
+  bool pad[kPer];
 #pragma unroll
-  for (int u = 0; u < kRepackPerThread; ++u) {
+  for (int u = 0; u < kPer; ++u) {
     const uint32_t i = rest + uint32_t(u) * kRepackThreads + threadIdx.x;
     const uint32_t down = fast_div(i, a.fd_units);
     const uint32_t v = i - down * a.units;
@@ -121,7 +127,7 @@ __device__ __forceinline__ void splitEights(const RepackArgs &a, unsigned long l
     *reinterpret_cast<float4 *>(&f[u][4]) = x[1];
   }
 #pragma unroll
-  for (int u = 0; u < kRepackPerThread; ++u) {
+  for (int u = 0; u < kPer; ++u) {
     if (dst[u] == nullptr) continue;
     if (pad[u]) {
       *dst[u] = make_uint4(0u, 0u, 0u, 0u);
@@ -140,14 +146,14 @@ __device__ __forceinline__ void splitEights(const RepackArgs &a, unsigned long l
 // of odd length the second pieces are one element earlier.  kAligned: rows of even length
 // at multiples of 8 bytes.  6689 rows of 1102 and of 1103 floats 45 -> 17 and
 // 21 us.
-template <bool kAligned>
+template <bool kAligned, int kPer>
 __device__ __forceinline__ void splitPairs(const RepackArgs &a, unsigned long long row0, uint32_t rest) {
   const uint32_t odd = kAligned ? 0 : a.cols & 1, pitch = a.vecs * 8;
-  float f[kSplitPerThread][3];
-  uint16_t *dst[kSplitPerThread];
-  uint32_t col[kSplitPerThread];
+  float f[kPer][3];
+  uint16_t *dst[kPer];
+  uint32_t col[kPer];
 #pragma unroll
-  for (int u = 0; u < kSplitPerThread; ++u) {
+  for (int u = 0; u < kPer; ++u) {
     const uint32_t i = rest + uint32_t(u) * kRepackThreads + threadIdx.x;
     const uint32_t down = fast_div(i, a.fd_units);
     const uint32_t c = 2 * (i - down * a.units);
@@ -169,7 +175,7 @@ __device__ __forceinline__ void splitPairs(const RepackArgs &a, unsigned long lo
     }
   }
 #pragma unroll
-  for (int u = 0; u < kSplitPerThread; ++u) {
+  for (int u = 0; u < kPer; ++u) {
     if (dst[u] == nullptr) continue;
     const uint32_t c = col[u];
     uint32_t *const third = reinterpret_cast<uint32_t *>(dst[u] + 2 * a.cols);
@@ -242,7 +248,7 @@ __device__ __forceinline__ void vectorStep(const RepackArgs &a, unsigned long lo
 
 // Both operands of a call go in one launch.  kCols: one of them is kSplitCols (an
 // instance of its own, since it takes more registers).
-template <bool kCols>
+template <bool kCols, int kPer>
 __global__ void __launch_bounds__(kRepackThreads)
 repackKernel(const RepackArgs first, const RepackArgs second, unsigned first_blocks) {
   pdl_launch_dependents();
@@ -252,21 +258,21 @@ repackKernel(const RepackArgs first, const RepackArgs second, unsigned first_blo
   const unsigned block = is_first ? blockIdx.x : blockIdx.x - first_blocks;
   const bool cols = kCols && a.mode == kRepackSplitCols;
   // the block's first step in 64 bits, the rest relative to its row in 32
-  const uint32_t per_thread = cols && a.group < 8 ? kSplitPerThread : kRepackPerThread;
+  const uint32_t per_thread = cols && a.group < 8 ? pairSteps(kPer) : kPer;
   const unsigned long long base = (unsigned long long)block * (kRepackThreads * per_thread);
   const unsigned long long row0 = base / a.units;
   const uint32_t rest = uint32_t(base - row0 * a.units);
   if (cols) {
     if (a.group == 8)
-      splitEights(a, row0, rest);
+      splitEights<kPer>(a, row0, rest);
     else if (a.aligned)
-      splitPairs<true>(a, row0, rest);
+      splitPairs<true, pairSteps(kPer)>(a, row0, rest);
     else
-      splitPairs<false>(a, row0, rest);
+      splitPairs<false, pairSteps(kPer)>(a, row0, rest);
     return;
   }
 #pragma unroll
-  for (int u = 0; u < kRepackPerThread; ++u) {
+  for (int u = 0; u < kPer; ++u) {
     const uint32_t i = rest + uint32_t(u) * kRepackThreads + threadIdx.x;
     const uint32_t down = fast_div(i, a.fd_units);
     const uint32_t v = i - down * a.units;
@@ -287,6 +293,7 @@ int repack(plb_context *ctx, const Repack *jobs, int n) {
   RepackArgs args[2] = {};
   unsigned blocks[2] = {0, 0};
   int used = 0;
+  uint64_t steps = 0;
   for (int i = 0; i < n; ++i) {
     const Repack &r = jobs[i];
     if (r.rows == 0 || r.cols == 0) continue;
@@ -318,17 +325,25 @@ int repack(plb_context *ctx, const Repack *jobs, int n) {
     a.full_h = r.lattice.full_h;
     a.step_w = r.lattice.step_w;
     a.step_h = r.lattice.step_h;
-    const uint64_t per_block =
-        kRepackThreads * (r.mode == kRepackSplitCols && a.group < 8 ? kSplitPerThread : kRepackPerThread);
-    const uint64_t b = (r.rows * a.units + per_block - 1) / per_block;
-    if (b + blocks[0] > 0x7fffffffull || uint64_t(a.units) + per_block > 0x7fffffffull)
-      return fail(PLB_ERR_UNSUPPORTED, "operand too large to be repacked");
-    blocks[used++] = unsigned(b);
+    steps += r.rows * a.units;
+    ++used;
   }
   if (used == 0) return PLB_OK;
-  const bool any_cols = args[0].mode == kRepackSplitCols || (used > 1 && args[1].mode == kRepackSplitCols);
-  return launchPdl(ctx, any_cols ? repackKernel<true> : repackKernel<false>, dim3(blocks[0] + blocks[1]), dim3(kRepackThreads), 0, args[0], args[1],
-                   blocks[0]);
+  const bool cols = args[0].mode == kRepackSplitCols || (used > 1 && args[1].mode == kRepackSplitCols);
+  const bool copy = args[0].mode == kRepackCopy;  // (the operands of a call have one type)
+  const int per = steps <= uint64_t(2 * 2048) * uint64_t(ctx->sm_count) ? kFewSteps : copy ? kCopySteps : kSplitSteps;
+  for (int i = 0; i < used; ++i) {
+    const RepackArgs &a = args[i];
+    const uint64_t block = kRepackThreads * (a.mode == kRepackSplitCols && a.group < 8 ? pairSteps(per) : per);
+    const uint64_t b = (a.rows * a.units + block - 1) / block;
+    if (b + blocks[0] > 0x7fffffffull || uint64_t(a.units) + block > 0x7fffffffull)
+      return fail(PLB_ERR_UNSUPPORTED, "operand too large to be repacked");
+    blocks[i] = unsigned(b);
+  }
+  auto kernel = per == kFewSteps     ? (cols ? repackKernel<true, kFewSteps> : repackKernel<false, kFewSteps>)
+                : per == kSplitSteps ? (cols ? repackKernel<true, kSplitSteps> : repackKernel<false, kSplitSteps>)
+                                     : repackKernel<false, kCopySteps>;
+  return launchPdl(ctx, kernel, dim3(blocks[0] + blocks[1]), dim3(kRepackThreads), 0, args[0], args[1], blocks[0]);
 }
 
 }  // namespace plb
