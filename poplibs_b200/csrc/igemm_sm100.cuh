@@ -726,12 +726,7 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
     // Accumulator g is drained by the eight warps of group g.  A warp can read
     // the 32 TMEM lanes (tile rows) [32*(warp%4), +32); the two warps that share
     // a lane quarter split every block of 64 columns between them (columns
-    // [0,32) and [32,64) of the block) and stage their halves of the same
-    // 32-row x 128-byte buffer, which one of them then hands to a tensor store.
-    // The two synchronise through two mbarriers (bounded waits, like every wait
-    // in this kernel): "buffer free" before writing, "buffer staged" before the
-    // store; the storing role alternates so that both wait for their own stores
-    // in turn.
+    // [0,32) and [32,64) of the block), each staging and storing its own half.
     const int group = (warp - 4) >> 3;       // drains accumulator `group`
     const int half = ((warp - 4) >> 2) & 1;  // which 32 columns of each 64-column block
     const int quarter = warp & 3;            // TMEM lanes [32*quarter, 32*quarter+32)

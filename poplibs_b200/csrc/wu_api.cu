@@ -494,7 +494,7 @@ extern "C" {
 int plb_conv_wu_plan(const plb_conv_params *p_in, const plb_conv_options *opt, plb_plan *plan) {
   if (!p_in || !plan) return fail(PLB_ERR_INVALID_PARAMS, "null argument");
   if (p_in->input_type == PLB_FLOAT) {
-    // what runs: bfloat16 operands, three batches side by side (float_route.cu)
+    // what runs: bfloat16 operands, three batches side by side (repack.cu)
     const std::string err = validate(*p_in);
     if (!err.empty()) return fail(PLB_ERR_INVALID_PARAMS, err);
     const plb_conv_params q = floatRouteConvParams(*p_in, PLB_PASS_TRAINING_WU);
