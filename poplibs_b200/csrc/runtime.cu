@@ -101,21 +101,23 @@ int encodeTensorMap(CUtensorMap *tm, CUtensorMapDataType type, int rank, const v
 // ---------------------------------------------------------------------------
 
 // Batched transpose src[b][rows][cols] -> dst[b][cols][dst_pitch] (what lies between
-// `rows` and the pitch is not written) through a 64 x 64 tile in shared memory, so that
+// `rows` and the pitch is not written) through a square tile of 16 words of rows in
+// shared memory (64 x 64 bytes, 32 x 32 halves, 16 x 16 words), so that
 // both sides are coalesced: four-byte words (V elements) where a side's rows start
 // on them, else elements, always several accesses in flight per thread.  The tile's
-// row pitch of 17 words leaves the column reads at most two to a bank.
+// row pitch of 17 words leaves the column reads at most two to a bank.  `row0` is the
+// first row of this launch's tiles.
 // 4392 x 1592 bytes: 15.6 us as 32 x 32 tiles of single elements, now 4.6.
 template <typename T>
 __global__ void __launch_bounds__(256)
 transposeKernel(const T *__restrict__ src, T *__restrict__ dst, uint32_t rows, uint32_t cols, uint32_t dst_pitch,
-                int src_words, int dst_words) {
+                uint32_t row0, int src_words, int dst_words) {
   constexpr int V = 4 / int(sizeof(T)), kTile = 16 * V, kPitch = 17 * V;
   __shared__ __align__(16) T tile[kTile * kPitch];
   pdl_launch_dependents();
   const T *s = src + size_t(blockIdx.z) * rows * cols;
   T *d = dst + size_t(blockIdx.z) * cols * dst_pitch;
-  const uint32_t c0 = blockIdx.x * kTile, r0 = blockIdx.y * kTile;
+  const uint32_t c0 = blockIdx.x * kTile, r0 = row0 + blockIdx.y * kTile;
   const uint32_t w = threadIdx.x & 15, k = threadIdx.x >> 4;  // word of a row, row
   pdl_wait();  // the matrix may come from the previous kernel in the stream
   if (src_words && c0 + kTile <= cols) {
@@ -172,17 +174,19 @@ int transposeBatch(plb_context *ctx, uint32_t elem_bytes, uint64_t batch, uint64
   const uint64_t strip = 65535 * tile;  // rows per launch
   const int dst_words = (dst_pitch * elem_bytes) % 4 == 0 && (reinterpret_cast<uintptr_t>(dst) & 3) == 0;
   const int src_words = (cols * elem_bytes) % 4 == 0 && (reinterpret_cast<uintptr_t>(src) & 3) == 0;
-  if (rows > strip) return fail(PLB_ERR_UNSUPPORTED, "matrix too tall to transpose");
-  for (uint64_t b0 = 0; b0 < batch; b0 += 65535) {
-    const dim3 grid(uint32_t(gx), uint32_t((rows + tile - 1) / tile), uint32_t(std::min<uint64_t>(65535, batch - b0)));
-    auto launch = [&](auto t) {
-      using T = decltype(t);
-      return launchPdl(ctx, transposeKernel<T>, grid, dim3(256), 0, static_cast<const T *>(src) + b0 * rows * cols,
-                       static_cast<T *>(dst) + b0 * cols * dst_pitch, uint32_t(rows), uint32_t(cols), uint32_t(dst_pitch),
-                       src_words, dst_words);
-    };
-    if (int rc = elem_bytes == 1 ? launch(uint8_t()) : elem_bytes == 2 ? launch(uint16_t()) : launch(uint32_t())) return rc;
-  }
+  for (uint64_t b0 = 0; b0 < batch; b0 += 65535)
+    for (uint64_t row0 = 0; row0 < rows; row0 += strip) {
+      const dim3 grid(uint32_t(gx), uint32_t((std::min(strip, rows - row0) + tile - 1) / tile),
+                      uint32_t(std::min<uint64_t>(65535, batch - b0)));
+      auto launch = [&](auto t) {
+        using T = decltype(t);
+        return launchPdl(ctx, transposeKernel<T>, grid, dim3(256), 0, static_cast<const T *>(src) + b0 * rows * cols,
+                         static_cast<T *>(dst) + b0 * cols * dst_pitch, uint32_t(rows), uint32_t(cols), uint32_t(dst_pitch),
+                         uint32_t(row0), src_words, dst_words);
+      };
+      if (int rc = elem_bytes == 1 ? launch(uint8_t()) : elem_bytes == 2 ? launch(uint16_t()) : launch(uint32_t()))
+        return rc;
+    }
   return PLB_OK;
 }
 

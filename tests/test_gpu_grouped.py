@@ -134,6 +134,20 @@ def test_transpose(gpu_ctx, elem, rows, cols):
     assert np.array_equal(got, a.transpose(0, 2, 1))
 
 
+@pytest.mark.parametrize("elem,rows", [(4, 65535 * 16), (4, 65535 * 16 + 1), (4, 65535 * 32), (2, 65535 * 32 + 5),
+                                       (1, 65535 * 64 + 7)])
+def test_transpose_of_tall_matrices(gpu_ctx, elem, rows):
+    """More row tiles than one launch's grid holds."""
+    import torch
+    dtype = {1: torch.uint8, 2: torch.int16, 4: torch.int32}[elem]
+    a = torch.randint(0, 100, (2, rows, 3), device="cuda").to(dtype)
+    got = torch.empty((2, 3, rows), dtype=dtype, device="cuda")
+    torch.cuda.synchronize()
+    T.context().transpose_matrix(elem, 2, rows, 3, a, got)
+    T.context().synchronize()
+    assert torch.equal(got, a.transpose(1, 2))
+
+
 @pytest.mark.parametrize("offset", [0, 1, 2])
 @pytest.mark.parametrize("k", [1, 2, 5, 7, 8, 16, 21, 24, 42, 43, 130, 343])
 def test_float_operands_are_split_in_place_order(gpu_ctx, k, offset):
