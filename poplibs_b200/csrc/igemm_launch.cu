@@ -134,11 +134,15 @@ int planIgemm(const IgemmProblem &p, int sm_count, plb_plan *plan) {
   const long k_iters = long(p.taps_h) * p.taps_w * ((p.k_per_tap + k_elems - 1) / k_elems);
   // per CTA
   const long resident_bytes = k_iters * (bn / (pair ? 2 : 1)) * kStageKBytes;
-  const bool want_resident = (p.plan_flags & PLB_PLAN_FORCE_RESIDENT_WEIGHTS) != 0 ||
-                             plan->tiles >= 2 * plan->grid;
+  const bool force_resident = (p.plan_flags & PLB_PLAN_FORCE_RESIDENT_WEIGHTS) != 0;
+  const bool want_resident = force_resident || plan->tiles >= 2 * plan->grid;
+  // With several groups a CTA (pair) works on one of them alone: as many as can run
+  // side by side if residency is asked for, and no K splits, which are neighbouring
+  // units (a tile's splits would be different groups' units to the CTAs).
+  const long most_groups = force_resident ? (pair ? sms_for_pair / 2 : sms_for_pair) : kMaxResidentGroups;
   plan->resident_weights =
-      ((p.plan_flags & PLB_PLAN_NO_RESIDENT_WEIGHTS) == 0 && n_tiles == 1 && groups <= kMaxResidentGroups && !p.a_mn && p.force_split_k <= 1 &&
-       resident_bytes <= kMaxResidentBytes && want_resident)
+      ((p.plan_flags & PLB_PLAN_NO_RESIDENT_WEIGHTS) == 0 && n_tiles == 1 && groups <= most_groups && !p.a_mn &&
+       (groups == 1 || p.force_split_k <= 1) && resident_bytes <= kMaxResidentBytes && want_resident)
           ? 1
           : 0;
   plan->grid = grid_for(best_tiles);
@@ -219,7 +223,7 @@ int planIgemm(const IgemmProblem &p, int sm_count, plb_plan *plan) {
     if (p.force_split_k > 0) {
       split = int(std::min<long>(p.force_split_k, steps));
     } else if (const int b_tiles = plan->halo_rows > 0 && !plan->resident_weights ? p.taps_h : 1;
-               units * 2 <= sms && steps * b_tiles >= 20) {
+               units * 2 <= sms && steps * b_tiles >= 20 && !(plan->resident_weights && groups > 1)) {
       const double out_mb = double(groups) * p.out_w * p.out_h * p.out_n * p.n_total * 4 / 1e6;
       const double odd_rows = (p.act_strides[0] % 32 != 0 ? 0.09 : 0.0) + (p.wgt_strides[0] % 32 != 0 ? 0.045 : 0.0);
       const double step_us = 0.15 * b_tiles + odd_rows;

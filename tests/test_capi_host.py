@@ -173,6 +173,23 @@ def test_planner_rules_for_pairs_halo_tiles_and_padding():
     assert wide.halo_rows == 0 and wide.tile_n <= 10 * 32 and wide.stages >= 2
 
 
+def test_forced_resident_weights_with_splits_and_groups():
+    """Residency that is asked for is kept with a forced K split, and with any number of
+    groups that run side by side; with groups only one of the two is possible."""
+    def plan(groups, flags, split=0, kernel=(3, 3), chans=64):
+        p = capi.ConvParams.make(2, [12, 12], list(kernel), chans, chans, groups=groups, padding=1)
+        f = capi.conv_plan(p, capi.PASS_TRAINING_FWD, capi.ConvOptions.make(plan_flags=flags, split_k=split))
+        return f.resident_weights, f.split_k
+    forced, pair = capi.PLAN_FORCE_RESIDENT_WEIGHTS, capi.PLAN_FORCE_CTA_PAIR
+    for flags in (forced, forced | pair, forced | capi.PLAN_NO_HALO):
+        assert plan(1, flags, split=3) == (1, 3)
+        assert plan(3, flags, split=3) == (0, 3)
+        assert plan(3, flags) == (1, 1) and plan(40, flags) == (1, 1)
+    # 74 pairs or 148 CTAs run side by side
+    assert plan(100, forced | pair) == (0, 1) and plan(100, forced | capi.PLAN_NO_CTA_PAIR) == (1, 1)
+    assert plan(3, 0) == (0, 1)
+
+
 def test_3d_layers_plan_as_2d_layers_with_depth_folded_into_channels():
     """A 3-D field runs as the 2-D problem over the inner dimensions with the
     kernel depth folded into the channels: batch * out-depth images and KD * Ci

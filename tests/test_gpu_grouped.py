@@ -47,6 +47,23 @@ def test_grouped_convolution(gpu_ctx, groups, ci, co, stride):
         exact(T.gpu_conv_wu(p, x, dy)[1], oracle.conv_wu(spec, x, dy)[0], f"wu {dtype}")
 
 
+@pytest.mark.parametrize("split", [0, 3])
+@pytest.mark.parametrize("variant", ["resident", "pair", "halo", "halo pair"])
+@pytest.mark.parametrize("kernel,chans", [((3, 3), 64), ((3, 8), 56)])
+def test_resident_weights_with_groups_and_splits(gpu_ctx, kernel, chans, variant, split):
+    """Residency that is asked for, with groups and with splits that are forced or (24 steps
+    over rows at odd multiples of 16 bytes) the planner's own."""
+    flags = (capi.PLAN_FORCE_RESIDENT_WEIGHTS | (capi.PLAN_FORCE_CTA_PAIR if "pair" in variant else 0) |
+             (0 if "halo" in variant else capi.PLAN_NO_HALO))
+    for groups in (1, 3):
+        kw = dict(batch=2, field=[12, 12], kernel=list(kernel), in_chans=chans, out_chans=chans, groups=groups, padding=1)
+        p, opt = capi.ConvParams.make(**kw), capi.ConvOptions.make(plan_flags=flags, split_k=split)
+        spec = T.spec_from_params(p)
+        r = T.rng(groups)
+        x, w = ints(r, (2, groups * chans, 12, 12), np.float16), ints(r, (groups, chans, chans, *kernel), np.float16)
+        exact(T.gpu_conv_fwd(p, x, w, opt=opt), oracle.conv_fwd(spec, x, w), f"fwd groups {groups}")
+
+
 @pytest.mark.parametrize("stride", [1, 2])
 @pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan])
 @pytest.mark.parametrize("groups,ci,co", [(32, 8, 8), (6, 10, 6)])
