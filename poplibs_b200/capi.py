@@ -249,6 +249,7 @@ def _load_binding():
     global _BINDING
     if os.path.exists(os.path.join(_HERE, "_binding.so")):
         from . import _binding
+        _binding.set_types(C.ArgumentError, MatmulDesc, ConvParams, ConvOptions)
         _BINDING = _binding
 
 

@@ -13,6 +13,17 @@
 #include "poplibs_b200.h"
 
 static PyObject *s_data_ptr, *s_ctypes, *s_data;
+/* ctypes.ArgumentError and the structures of the ctypes layer (set_types) */
+static PyObject *t_error, *t_matmul_desc, *t_conv_params, *t_conv_options;
+
+/* A value of the wrong type raises what ctypes raises for it. */
+static int argument_error(PyObject *o, const char *expected) {
+  if (PyErr_ExceptionMatches(PyExc_TypeError)) {
+    PyErr_Clear();
+    PyErr_Format(t_error ? t_error : PyExc_TypeError, "expected %s instead of %s", expected, Py_TYPE(o)->tp_name);
+  }
+  return -1;
+}
 
 /* Device or host address of None, an int, a torch tensor or a numpy array. */
 static int address(PyObject *o, void **out) {
@@ -22,7 +33,8 @@ static int address(PyObject *o, void **out) {
   }
   PyObject *v = NULL;
   if (PyLong_Check(o)) {
-    v = Py_NewRef(o);
+    Py_INCREF(o);
+    v = o;
   } else {
     PyObject *method = PyObject_GetAttr(o, s_data_ptr);
     if (method != NULL) {
@@ -46,38 +58,48 @@ static int address(PyObject *o, void **out) {
   return *out == NULL && PyErr_Occurred() ? -1 : 0;
 }
 
-/* Address of a ctypes structure of at least `size` bytes (None: NULL).  The
- * caller's reference keeps it alive for the call. */
-static int structure(PyObject *o, size_t size, const void **out) {
+/* Address of a ctypes structure of type `type` (None: NULL, where it may be left
+ * out).  The caller's reference keeps it alive for the call. */
+static int structure(PyObject *o, PyObject *type, int optional, const void **out) {
   Py_buffer b;
-  if (o == Py_None) {
+  if (optional && o == Py_None) {
     *out = NULL;
     return 0;
   }
+  if (type == NULL || !PyObject_TypeCheck(o, (PyTypeObject *)type)) {
+    PyErr_Format(t_error ? t_error : PyExc_TypeError, "expected %s instead of %s",
+                 type ? ((PyTypeObject *)type)->tp_name : "a structure", Py_TYPE(o)->tp_name);
+    return -1;
+  }
   if (PyObject_GetBuffer(o, &b, PyBUF_SIMPLE) != 0) return -1;
   *out = b.buf;
-  const int ok = (size_t)b.len >= size;
   PyBuffer_Release(&b);
-  if (!ok) PyErr_SetString(PyExc_TypeError, "descriptor structure is too small");
-  return ok ? 0 : -1;
+  return 0;
 }
 
 static int as_float(PyObject *o, float *out) {
   const double v = PyFloat_AsDouble(o);
   *out = (float)v;
-  return v == -1.0 && PyErr_Occurred() ? -1 : 0;
+  return v == -1.0 && PyErr_Occurred() ? argument_error(o, "a number") : 0;
 }
-static int as_u64(PyObject *o, uint64_t *out) {
+/* An integer of at most `most`: what does not fit is an error, not cut off. */
+static int as_unsigned(PyObject *o, uint64_t most, uint64_t *out) {
   PyObject *v = PyNumber_Index(o);
-  if (v == NULL) return -1;
+  if (v == NULL) return argument_error(o, "an integer");
   *out = PyLong_AsUnsignedLongLong(v);
   Py_DECREF(v);
-  return *out == (uint64_t)-1 && PyErr_Occurred() ? -1 : 0;
+  if (*out == (uint64_t)-1 && PyErr_Occurred()) return -1;
+  if (*out <= most) return 0;
+  PyErr_Format(PyExc_OverflowError, "%R does not fit the argument's type", o);
+  return -1;
 }
 static int as_int(PyObject *o, int *out) {
   const long v = PyLong_AsLong(o);
   *out = (int)v;
-  return v == -1 && PyErr_Occurred() ? -1 : 0;
+  if (v == -1 && PyErr_Occurred()) return argument_error(o, "an integer");
+  if (v == *out) return 0;
+  PyErr_Format(PyExc_OverflowError, "%R does not fit the argument's type", o);
+  return -1;
 }
 
 #define FUNCTION(name) static PyObject *name(PyObject *self, PyObject *const *a, Py_ssize_t n)
@@ -90,16 +112,20 @@ static int as_int(PyObject *o, int *out) {
 #define PTR(i, p)         \
   void *p;                \
   if (address(a[i], &p)) return NULL
-#define STRUCT(i, type, p) \
-  const void *p##_v;       \
-  if (structure(a[i], sizeof(type), &p##_v)) return NULL; \
+#define STRUCT(i, type, py_type, optional, p)                         \
+  const void *p##_v;                                                  \
+  if (structure(a[i], py_type, optional, &p##_v)) return NULL;        \
   const type *p = (const type *)p##_v
 #define INT(i, v) \
   int v;          \
   if (as_int(a[i], &v)) return NULL
 #define U64(i, v) \
   uint64_t v;     \
-  if (as_u64(a[i], &v)) return NULL
+  if (as_unsigned(a[i], UINT64_MAX, &v)) return NULL
+#define U32(i, v)    \
+  uint64_t v##_wide; \
+  if (as_unsigned(a[i], UINT32_MAX, &v##_wide)) return NULL; \
+  const uint32_t v = (uint32_t)v##_wide
 #define FLOAT(i, v) \
   float v;          \
   if (as_float(a[i], &v)) return NULL
@@ -113,7 +139,7 @@ static int as_int(PyObject *o, int *out) {
 FUNCTION(matmul) {
   ARGS(6);
   CONTEXT(0);
-  STRUCT(1, plb_matmul_desc, d);
+  STRUCT(1, plb_matmul_desc, t_matmul_desc, 0, d);
   PTR(2, pa);
   PTR(3, pb);
   PTR(4, pc);
@@ -123,8 +149,8 @@ FUNCTION(matmul) {
 FUNCTION(convolution) {
   ARGS(8);
   CONTEXT(0);
-  STRUCT(1, plb_conv_params, p);
-  STRUCT(2, plb_conv_options, o);
+  STRUCT(1, plb_conv_params, t_conv_params, 0, p);
+  STRUCT(2, plb_conv_options, t_conv_options, 1, o);
   PTR(3, x);
   PTR(4, w);
   PTR(5, bias);
@@ -135,8 +161,8 @@ FUNCTION(convolution) {
 FUNCTION(conv_bwd) {
   ARGS(6);
   CONTEXT(0);
-  STRUCT(1, plb_conv_params, p);
-  STRUCT(2, plb_conv_options, o);
+  STRUCT(1, plb_conv_params, t_conv_params, 0, p);
+  STRUCT(2, plb_conv_options, t_conv_options, 1, o);
   PTR(3, dy);
   PTR(4, w);
   PTR(5, dx);
@@ -145,8 +171,8 @@ FUNCTION(conv_bwd) {
 FUNCTION(conv_wu) {
   ARGS(7);
   CONTEXT(0);
-  STRUCT(1, plb_conv_params, p);
-  STRUCT(2, plb_conv_options, o);
+  STRUCT(1, plb_conv_params, t_conv_params, 0, p);
+  STRUCT(2, plb_conv_options, t_conv_options, 1, o);
   PTR(3, x);
   PTR(4, dy);
   PTR(5, dw);
@@ -178,11 +204,11 @@ FUNCTION(conv_bias_update) {
   INT(1, dtype);
   PTR(2, dy);
   U64(3, pixels);
-  U64(4, chans);
+  U32(4, chans);
   INT(5, bias_dtype);
   PTR(6, bias);
   FLOAT(7, scale);
-  CALL(plb_conv_bias_update(ctx, dtype, dy, pixels, (uint32_t)chans, bias_dtype, bias, scale));
+  CALL(plb_conv_bias_update(ctx, dtype, dy, pixels, chans, bias_dtype, bias, scale));
 }
 FUNCTION(norm_moments) {
   ARGS(9);
@@ -190,12 +216,12 @@ FUNCTION(norm_moments) {
   INT(1, dtype);
   PTR(2, x);
   U64(3, pixels);
-  U64(4, chans);
+  U32(4, chans);
   FLOAT(5, scale);
   PTR(6, centre);
   PTR(7, mean);
   PTR(8, power);
-  CALL(plb_norm_moments(ctx, dtype, x, pixels, (uint32_t)chans, scale, centre, mean, (float *)power));
+  CALL(plb_norm_moments(ctx, dtype, x, pixels, chans, scale, centre, mean, (float *)power));
 }
 FUNCTION(norm_statistics) {
   ARGS(10);
@@ -203,13 +229,13 @@ FUNCTION(norm_statistics) {
   INT(1, dtype);
   PTR(2, x);
   U64(3, pixels);
-  U64(4, chans);
+  U32(4, chans);
   FLOAT(5, eps);
   FLOAT(6, scale_var);
   PTR(7, mean);
   PTR(8, inv_std);
   PTR(9, power);
-  CALL(plb_norm_statistics(ctx, dtype, x, pixels, (uint32_t)chans, eps, scale_var, mean, inv_std, (float *)power));
+  CALL(plb_norm_statistics(ctx, dtype, x, pixels, chans, eps, scale_var, mean, inv_std, (float *)power));
 }
 FUNCTION(norm_normalise) {
   ARGS(11);
@@ -221,10 +247,10 @@ FUNCTION(norm_normalise) {
   PTR(5, gamma);
   PTR(6, beta);
   U64(7, pixels);
-  U64(8, chans);
+  U32(8, chans);
   PTR(9, whitened);
   PTR(10, out);
-  CALL(plb_norm_normalise(ctx, dtype, x, mean, inv_std, gamma, beta, pixels, (uint32_t)chans, whitened, out));
+  CALL(plb_norm_normalise(ctx, dtype, x, mean, inv_std, gamma, beta, pixels, chans, whitened, out));
 }
 FUNCTION(norm_whiten) {
   ARGS(8);
@@ -234,9 +260,9 @@ FUNCTION(norm_whiten) {
   PTR(3, mean);
   PTR(4, inv_std);
   U64(5, pixels);
-  U64(6, chans);
+  U32(6, chans);
   PTR(7, out);
-  CALL(plb_norm_whiten(ctx, dtype, x, mean, inv_std, pixels, (uint32_t)chans, out));
+  CALL(plb_norm_whiten(ctx, dtype, x, mean, inv_std, pixels, chans, out));
 }
 FUNCTION(norm_scale_shift) {
   ARGS(8);
@@ -246,9 +272,9 @@ FUNCTION(norm_scale_shift) {
   PTR(3, scale);
   PTR(4, shift);
   U64(5, pixels);
-  U64(6, chans);
+  U32(6, chans);
   PTR(7, out);
-  CALL(plb_norm_scale_shift(ctx, dtype, x, scale, shift, pixels, (uint32_t)chans, out));
+  CALL(plb_norm_scale_shift(ctx, dtype, x, scale, shift, pixels, chans, out));
 }
 FUNCTION(norm_param_gradients) {
   ARGS(11);
@@ -257,13 +283,13 @@ FUNCTION(norm_param_gradients) {
   PTR(2, whitened);
   PTR(3, grads);
   U64(4, pixels);
-  U64(5, chans);
+  U32(5, chans);
   FLOAT(6, scale);
   PTR(7, gamma);
   PTR(8, beta);
   PTR(9, gamma32);
   PTR(10, beta32);
-  CALL(plb_norm_param_gradients(ctx, dtype, whitened, grads, pixels, (uint32_t)chans, scale, gamma, beta,
+  CALL(plb_norm_param_gradients(ctx, dtype, whitened, grads, pixels, chans, scale, gamma, beta,
                                 (float *)gamma32, (float *)beta32));
 }
 FUNCTION(norm_statistics_gradients) {
@@ -276,10 +302,24 @@ FUNCTION(norm_statistics_gradients) {
   PTR(5, var_delta);
   PTR(6, mean_delta);
   U64(7, pixels);
-  U64(8, chans);
+  U32(8, chans);
   PTR(9, out);
   CALL(plb_norm_statistics_gradients(ctx, dtype, whitened, grads, inv_std, var_delta, mean_delta, pixels,
-                                     (uint32_t)chans, out));
+                                     chans, out));
+}
+
+/* ctypes.ArgumentError, MatmulDesc, ConvParams, ConvOptions: once, by capi.py. */
+FUNCTION(set_types) {
+  ARGS(4);
+  PyObject **const to[] = {&t_error, &t_matmul_desc, &t_conv_params, &t_conv_options};
+  for (int i = 0; i < 4; ++i) {
+    if (!PyType_Check(a[i])) return PyErr_Format(PyExc_TypeError, "types expected");
+    Py_INCREF(a[i]);
+    PyObject *old = *to[i];
+    *to[i] = a[i];
+    Py_XDECREF(old);
+  }
+  Py_RETURN_NONE;
 }
 
 #define METHOD(name) {#name, (PyCFunction)(void (*)(void))name, METH_FASTCALL, NULL}
@@ -288,7 +328,7 @@ static PyMethodDef methods[] = {
     METHOD(conv_wu),        METHOD(scaled_add_to),  METHOD(cast_from_f32),
     METHOD(conv_bias_update), METHOD(norm_moments), METHOD(norm_statistics),
     METHOD(norm_normalise), METHOD(norm_whiten),    METHOD(norm_scale_shift),
-    METHOD(norm_param_gradients), METHOD(norm_statistics_gradients),
+    METHOD(norm_param_gradients), METHOD(norm_statistics_gradients), METHOD(set_types),
     {NULL, NULL, 0, NULL}};
 static struct PyModuleDef module = {PyModuleDef_HEAD_INIT, "_binding", NULL, -1, methods, NULL, NULL, NULL, NULL};
 

@@ -231,6 +231,66 @@ def test_option_and_type_errors():
     assert e.value.code == 2
 
 
+def _closed_context():
+    """A context whose handle is null: every call gets as far as the library's own check."""
+    ctx = capi.Context.__new__(capi.Context)
+    ctx._h, ctx._ctx = C.c_void_p(), 0
+    return ctx
+
+
+def _per_layer_calls(ctx, desc, p, o):
+    x = np.zeros(64, np.float32)
+    return {
+        "matmul": lambda: ctx.matmul(desc, x, x, None, x),
+        "conv_fwd": lambda: ctx.conv_fwd(p, x, x, x, bias=None, opt=o),
+        "convolution": lambda: ctx.convolution(p, x, x, x, x, o, True),
+        "conv_bwd": lambda: ctx.conv_bwd(p, x, x, x, o),
+        "conv_wu": lambda: ctx.conv_wu(p, x, x, None, x, o),
+        "scaled_add_to": lambda: ctx.scaled_add_to(capi.HALF, x, x, 0.5, 8),
+        "conv_bias_update": lambda: ctx.conv_bias_update(capi.HALF, x, 2, 4, capi.FLOAT, x, 0.5),
+        "norm_moments": lambda: ctx.norm_moments(capi.HALF, x, 2, 4, 0.5, None, x, x),
+        "norm_statistics": lambda: ctx.norm_statistics(capi.HALF, x, 2, 4, 1e-3, 1.0, x, x),
+        "norm_normalise": lambda: ctx.norm_normalise(capi.HALF, x, x, x, x, x, 2, 4, None, x),
+        "norm_whiten": lambda: ctx.norm_whiten(capi.HALF, x, x, x, 2, 4, x),
+        "norm_scale_shift": lambda: ctx.norm_scale_shift(capi.HALF, x, x, None, 2, 4, x),
+        "norm_param_gradients": lambda: ctx.norm_param_gradients(capi.HALF, x, x, 2, 4, 1.0, x, x),
+        "norm_statistics_gradients": lambda: ctx.norm_statistics_gradients(capi.HALF, x, x, x, 2, 4, x),
+        "cast_from_f32": lambda: ctx.cast_from_f32(capi.HALF, x, x, 8),
+    }
+
+
+@pytest.mark.parametrize("route", ["binding", "ctypes"])
+def test_per_layer_calls_and_their_errors_by_either_route(monkeypatch, route):
+    """The CPython binding and ctypes reach the same entry points and refuse the same arguments."""
+    capi.lib()
+    if route == "ctypes":
+        monkeypatch.setattr(capi, "_BINDING", None)
+    elif capi._BINDING is None:
+        pytest.skip("the binding was not built")
+    ctx, desc, p = _closed_context(), capi.MatmulDesc.make(4, 4, 4), capi.ConvParams.make(1, [4, 4], [3, 3], 8, 8)
+    for o in (None, capi.ConvOptions.make()):
+        for name, call in _per_layer_calls(ctx, desc, p, o).items():
+            with pytest.raises(capi.PlbError) as e:
+                call()
+            assert "null context" in e.value.message, name
+    # another structure, or bytes, in a descriptor's place
+    for desc2, p2, o2 in ((p, desc, None), (bytes(4096), bytes(4096), None), (None, None, None), (p, p, p)):
+        calls = _per_layer_calls(ctx, desc2, p2, o2)
+        for name in ("conv_fwd", "convolution", "conv_bwd", "conv_wu") + (("matmul",) if o2 is None else ()):
+            with pytest.raises((C.ArgumentError, TypeError)):
+                calls[name]()
+    for bad in (lambda: ctx.scaled_add_to("half", p, p, 0.5, 8), lambda: ctx.scaled_add_to(capi.HALF, None, None, 0.5, 8.0),
+                lambda: ctx.scaled_add_to(capi.HALF, None, None, "half", 8)):
+        with pytest.raises((C.ArgumentError, TypeError)):
+            bad()
+    if route == "binding":  # (ctypes cuts integers off)
+        for bad in (lambda: ctx.norm_scale_shift(capi.HALF, None, None, None, 2, 2 ** 32 + 4, None),
+                    lambda: ctx.cast_from_f32(2 ** 32 + capi.HALF, None, None, 8),
+                    lambda: ctx.scaled_add_to(capi.HALF, None, None, 0.5, 2 ** 64)):
+            with pytest.raises(OverflowError):
+                bad()
+
+
 def test_no_silent_fallback_without_a_gpu():
     import torch
     if torch.cuda.is_available():
