@@ -72,19 +72,32 @@ def build(force: bool = False, verbose: bool = False) -> str:
 
 
 BINDING_SRC = os.path.join(CSRC, "python", "binding.c")
-BINDING_OUT = os.path.join(HERE, "_binding.so")
+# (named after the interpreter it is built for: another one does not see it)
+BINDING_OUT = os.path.join(HERE, "_binding" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
 
 
 def build_binding(force: bool = False):
-    """The CPython binding of the per-layer calls -> _binding.so, where the
-    interpreter's headers are installed (capi.py goes through ctypes without it)."""
+    """The CPython binding of the per-layer calls -> _binding.<abi>.so, where the
+    interpreter's headers are installed and it compiles.  Without it capi.py goes
+    through ctypes, so a stale one is removed rather than left."""
+    untagged = os.path.join(HERE, "_binding.so")
+    if untagged != BINDING_OUT and os.path.exists(untagged):
+        os.remove(untagged)
+    if not force and _newer(BINDING_OUT, [BINDING_SRC, OUT, os.path.join(ROOT, "include", "poplibs_b200.h")]):
+        return BINDING_OUT
+    if os.path.exists(BINDING_OUT):
+        os.remove(BINDING_OUT)
     include = sysconfig.get_paths()["include"]
     if not os.path.exists(os.path.join(include, "Python.h")):
         return None
-    if force or not _newer(BINDING_OUT, [BINDING_SRC, OUT, os.path.join(ROOT, "include", "poplibs_b200.h")]):
-        subprocess.run([shutil.which("gcc") or "gcc", "-O2", "-shared", "-fPIC", "-Wall", "-I" + include,
-                        "-I" + os.path.join(ROOT, "include"), BINDING_SRC, "-o", BINDING_OUT, "-L" + HERE,
-                        "-lpoplibs_b200", "-Wl,-rpath,$ORIGIN"], check=True)
+    cmd = [shutil.which("gcc") or "gcc", "-O2", "-shared", "-fPIC", "-Wall", "-I" + include,
+           "-I" + os.path.join(ROOT, "include"), BINDING_SRC, "-o", BINDING_OUT, "-L" + HERE,
+           "-lpoplibs_b200", "-Wl,-rpath,$ORIGIN"]
+    try:
+        subprocess.run(cmd, check=True)
+    except (OSError, subprocess.CalledProcessError) as e:
+        print(f"the CPython binding was not built, calls go through ctypes: {e}", file=sys.stderr)
+        return None
     return BINDING_OUT
 
 

@@ -247,10 +247,13 @@ def lib():
 
 def _load_binding():
     global _BINDING
-    if os.path.exists(os.path.join(_HERE, "_binding.so")):
+    _BINDING = None
+    try:
         from . import _binding
-        _binding.set_types(C.ArgumentError, MatmulDesc, ConvParams, ConvOptions)
-        _BINDING = _binding
+    except ImportError:  # not built, or not for this interpreter
+        return
+    _binding.set_types(C.ArgumentError, MatmulDesc, ConvParams, ConvOptions)
+    _BINDING = _binding
 
 
 def _check(rc: int):

@@ -291,6 +291,30 @@ def test_per_layer_calls_and_their_errors_by_either_route(monkeypatch, route):
                 bad()
 
 
+def test_a_binding_that_cannot_be_used_is_passed_over(monkeypatch, tmp_path):
+    """One that does not import is not used; one that cannot be built again does not stay."""
+    import sys
+    from poplibs_b200 import build
+    capi.lib()
+    monkeypatch.setattr(capi, "_BINDING", capi._BINDING)
+    monkeypatch.setitem(sys.modules, "poplibs_b200._binding", None)  # importing it raises ImportError
+    monkeypatch.delattr("poplibs_b200._binding", raising=False)
+    capi._load_binding()
+    assert capi._BINDING is None
+    stale = tmp_path / "_binding.abi.so"
+    untagged = tmp_path / "_binding.so"
+    monkeypatch.setattr(build, "HERE", str(tmp_path))
+    monkeypatch.setattr(build, "BINDING_OUT", str(stale))
+    for why in ("no headers", "compile error"):
+        stale.write_bytes(b""), untagged.write_bytes(b"")
+        if why == "no headers":
+            monkeypatch.setattr(build.sysconfig, "get_paths", lambda: {"include": str(tmp_path)})
+        else:
+            (tmp_path / "Python.h").write_text("#error not this one")
+        assert build.build_binding(force=True) is None
+        assert not stale.exists() and not untagged.exists()
+
+
 def test_no_silent_fallback_without_a_gpu():
     import torch
     if torch.cuda.is_available():
