@@ -462,6 +462,71 @@ WuLayout oneGroup(const plb_conv_params &p) {
   return WuLayout{1, ci, co, uint64_t(p.groups) * ci, uint64_t(p.groups) * co};
 }
 
+// Few input channels (an image network's first layer): the rearranged input of
+// the forward pass, whose pixels hold a window of the filter's columns, so that
+// the KW taps of a filter row are 64 channels of one tap.  (On channels padded to
+// 8 the layer 7x7, stride 2, 3 -> 64 channels, 256 images of 224x224, took
+// 49 taps of 5/8 padding and 5.5 ms.)  Returns whether it applies.
+bool rearrangedProblem(const plb_conv_params &p, const WuShape &s, S2dShape *g, WuProblem *q) {
+  const uint32_t ci = p.in_chans_per_group, co = p.out_chans_per_group;
+  if (ci % 8 == 0 || co % 8 != 0 || p.input_type == PLB_FLOAT || smallChannelShape(p, g) != PLB_OK) return false;
+  WuShape s2 = s;
+  s2.H = s2.He = g->H2;
+  s2.W = g->W2;
+  s2.We = g->OW;  // windows per row
+  s2.KH = g->K2h;
+  s2.KW = 1;
+  s2.padH = s2.padW = 0;
+  s2.strH = s2.strW = 1;
+  *q = wuProblem(p, s2, WuLayout{1, 64, co, 64, uint64_t(co)}, 1);
+  q->x_strides[0] = uint64_t(g->C2) * 2;
+  q->x_strides[1] = uint64_t(g->W2) * g->C2 * 2;
+  q->x_strides[2] = uint64_t(g->H2) * g->W2 * g->C2 * 2;
+  return true;
+}
+size_t rearrangedBytes(const S2dShape &g) { return smallChannelElems(g) * 2 + 256; }
+
+// The general form: channel counts TMA cannot address (a pixel must be a multiple of
+// 16 bytes) run on copies with the channels rounded up; float operands as three
+// batches of bfloat16 pieces side by side.  The padded rows and columns of the
+// partial sums are not read.  `x` and `dy` become the operands as the kernel reads
+// them; up to two copies are left to do in `jobs`, `bytes` of scratch in all.
+struct WuOperands {
+  WuLayout layout;
+  Repack jobs[2];
+  const void **operand[2];
+  size_t offset[2];
+  int copies = 0;
+  size_t bytes = 0;
+};
+WuProblem generalProblem(const plb_conv_params &p, const WuShape &s, const void **x, const void **dy, WuOperands *o) {
+  const uint32_t ci = p.in_chans_per_group, co = p.out_chans_per_group;
+  const bool is_float = p.input_type == PLB_FLOAT;
+  const WuLayout l = wuLayout(p.groups, ci, co, is_float);
+  // whole pixels, or where the groups' channels are rounded up, each group's
+  auto add = [&](const void **base, uint64_t pixels, uint32_t chans, uint32_t chans_pitch, uint64_t pixel, bool second) {
+    if (!is_float && chans == chans_pitch && pixel == uint64_t(p.groups) * chans &&
+        (reinterpret_cast<uintptr_t>(*base) & 15) == 0)
+      return;
+    const bool whole = chans == chans_pitch;
+    const uint32_t cols = whole ? p.groups * chans : chans;
+    o->jobs[o->copies] = Repack{*base, nullptr, whole ? pixels : pixels * p.groups, cols, cols, whole ? uint32_t(pixel) : chans_pitch,
+                                is_float ? 4u : 2u, is_float ? kRepackSplitPlanes : kRepackCopy, second, 0, {}};
+    o->offset[o->copies] = o->bytes;
+    o->bytes += (repackBytes(o->jobs[o->copies]) + 255) & ~size_t(255);
+    o->operand[o->copies++] = base;
+  };
+  add(x, uint64_t(p.batch) * s.H * s.W, ci, l.ci_pitch, l.x_pixel, false);
+  add(dy, uint64_t(p.batch) * s.OH * s.OW, co, l.co_pitch, l.dy_pixel, true);
+  o->layout = l;
+  plb_conv_params q16 = p;
+  if (is_float) {
+    q16.input_type = PLB_BFLOAT16;
+    q16.batch *= 3;
+  }
+  return wuProblem(q16, s, l, p.groups);
+}
+
 // The groups of a layer one after the other, through one group's worth of scratch
 // (the entry points that cannot hold more).  With `peer` the reduction also adds
 // the gradients of the other ranks; the caller has checked that the shapes allow it.
@@ -493,18 +558,6 @@ extern "C" {
 
 int plb_conv_wu_plan(const plb_conv_params *p_in, const plb_conv_options *opt, plb_plan *plan) {
   if (!p_in || !plan) return fail(PLB_ERR_INVALID_PARAMS, "null argument");
-  if (p_in->input_type == PLB_FLOAT) {
-    // what runs: bfloat16 operands, three batches side by side (repack.cu)
-    const std::string err = validate(*p_in);
-    if (!err.empty()) return fail(PLB_ERR_INVALID_PARAMS, err);
-    const plb_conv_params q = floatRouteConvParams(*p_in, PLB_PASS_TRAINING_WU);
-    if (int rc = plb_conv_wu_plan(&q, opt, plan)) return rc;
-    plan->flops = 2 * numberOfMacs(*p_in);
-    size_t n_in, n_w, n_out;
-    convElementCounts(*p_in, &n_in, &n_w, &n_out);
-    plan->workspace_bytes += (n_in + n_out) * 6 + 768;
-    return PLB_OK;
-  }
   if (p_in->num_field_dims == 3) return conv3dPlan(*p_in, opt, PLB_PASS_TRAINING_WU, plan);
   // plan what plb_conv_wu runs: flipped inputs are reversed first, truncated /
   // flipped kernels are computed as ordinary kernels of the truncated extent
@@ -526,8 +579,17 @@ int plb_conv_wu_plan(const plb_conv_params *p_in, const plb_conv_options *opt, p
   if (int rc = wuShape(*p, &s)) return rc;
   *plan = plb_plan{};
   WuArgs a{};
-  planWu(wuProblem(*p, s, wuLayout(p->groups, p->in_chans_per_group, p->out_chans_per_group), p->groups), 148,
-         opt ? opt->split_k : 0, opt ? opt->plan_flags : 0, &a, plan);
+  if (p->groups == 0 || p->in_chans_per_group == 0 || p->out_chans_per_group == 0 || p->batch == 0 || s.OHc <= 0 ||
+      s.OWc <= 0 || s.He <= 0 || s.We <= 0)
+    return PLB_OK;  // nothing is contracted
+  S2dShape g2{};
+  WuProblem w;
+  const void *x = nullptr, *dy = nullptr;  // (as aligned as they need to be)
+  WuOperands operands;
+  const bool rearranged = rearrangedProblem(*p, s, &g2, &w);
+  if (!rearranged) w = generalProblem(*p, s, &x, &dy, &operands);
+  planWu(w, 148, opt ? opt->split_k : 0, opt ? opt->plan_flags : 0, &a, plan);
+  plan->workspace_bytes += rearranged ? rearrangedBytes(g2) : operands.bytes;
   plan->flops = 2 * numberOfMacs(*p);
   const uint64_t es = dtypeBytes(p->input_type);
   plan->bytes = es * (uint64_t(p->batch) * s.H * s.W * p->groups * p->in_chans_per_group +
@@ -697,74 +759,29 @@ int plb_conv_wu(plb_context *ctx, const plb_conv_params *p, const plb_conv_optio
     }
     return launchWuReduce(ctx->stream, a, p->groups * w_elems, d_weight_grads, d_weight_grads_f32, g);
   };
-  // Few input channels (an image network's first layer): the rearranged input of
-  // the forward pass, whose pixels hold a window of the filter's columns, so that
-  // the KW taps of a filter row are 64 channels of one tap.  (On channels padded to
-  // 8 the layer 7x7, stride 2, 3 -> 64 channels, 256 images of 224x224, took
-  // 49 taps of 5/8 padding and 5.5 ms.)
   S2dShape g2{};
-  if (ci % 8 != 0 && co % 8 == 0 && p->input_type != PLB_FLOAT && smallChannelShape(*p, &g2) == PLB_OK) {
+  WuProblem q;
+  if (rearrangedProblem(*p, s, &g2, &q)) {
     void *ws = nullptr;
-    if (int rc = scratch(ctx, kSlotOperands, smallChannelElems(g2) * 2 + 256, &ws)) return rc;
+    if (int rc = scratch(ctx, kSlotOperands, rearrangedBytes(g2), &ws)) return rc;
     if (int rc = smallChannelPrepare(ctx, g2, d_acts, static_cast<__half *>(ws), nullptr, nullptr, co)) return rc;
-    WuShape s2 = s;
-    s2.H = s2.He = g2.H2;
-    s2.W = g2.W2;
-    s2.We = g2.OW;  // windows per row
-    s2.KH = g2.K2h;
-    s2.KW = 1;
-    s2.padH = s2.padW = 0;
-    s2.strH = s2.strW = 1;
-    WuProblem q = wuProblem(*p, s2, WuLayout{1, 64, uint32_t(co), 64, uint64_t(co)}, 1);
     q.x = ws;
-    q.x_strides[0] = uint64_t(g2.C2) * 2;
-    q.x_strides[1] = uint64_t(g2.W2) * g2.C2 * 2;
-    q.x_strides[2] = uint64_t(g2.H2) * g2.W2 * g2.C2 * 2;
     q.dy = d_out_grads;
     const WuFold fold{uint32_t(s.KH), uint32_t(s.KW), uint32_t(co), uint32_t(ci), uint32_t(g2.s), uint32_t(g2.Cp),
                       uint32_t(g2.K2h), 0};
     return run(q, nullptr, &fold);
   }
-  // Channel counts TMA cannot address (a pixel must be a multiple of 16 bytes) run
-  // on copies with the channels rounded up; float operands as three batches of
-  // bfloat16 pieces side by side.  The padded rows and columns of the partial sums
-  // are not read.
-  const bool is_float = p->input_type == PLB_FLOAT;
-  const WuLayout l = wuLayout(p->groups, uint32_t(ci), uint32_t(co), is_float);
-  const uint64_t x_pixels = uint64_t(p->batch) * s.H * s.W, dy_pixels = uint64_t(p->batch) * s.OH * s.OW;
   const void *x = d_acts, *dy = d_out_grads;
-  {
-    Repack jobs[2];
-    const void **operand[2];
-    int n = 0;
-    // whole pixels, or where the groups' channels are rounded up, each group's
-    auto add = [&](const void **base, uint64_t pixels, uint32_t chans, uint32_t chans_pitch, uint64_t pixel, bool second) {
-      if (!is_float && chans == chans_pitch && pixel == uint64_t(p->groups) * chans &&
-          (reinterpret_cast<uintptr_t>(*base) & 15) == 0)
-        return;
-      const bool whole = chans == chans_pitch;
-      const uint32_t cols = whole ? p->groups * chans : chans;
-      jobs[n] = Repack{*base, nullptr, whole ? pixels : pixels * p->groups, cols, cols, whole ? uint32_t(pixel) : chans_pitch,
-                       is_float ? 4u : 2u, is_float ? kRepackSplitPlanes : kRepackCopy, second, 0, {}};
-      operand[n++] = base;
-    };
-    add(&x, x_pixels, uint32_t(ci), l.ci_pitch, l.x_pixel, false);
-    add(&dy, dy_pixels, uint32_t(co), l.co_pitch, l.dy_pixel, true);
-    size_t bytes[2] = {0, 0};
-    for (int i = 0; i < n; ++i) bytes[i] = (repackBytes(jobs[i]) + 255) & ~size_t(255);
-    if (n) {
-      void *ws = nullptr;
-      if (int rc = scratch(ctx, kSlotRepacked, bytes[0] + bytes[1] + 256, &ws)) return rc;
-      for (int i = 0; i < n; ++i) *operand[i] = jobs[i].dst = static_cast<uint8_t *>(ws) + (i ? bytes[0] : 0);
-      if (int rc = repack(ctx, jobs, n)) return rc;
-    }
+  WuOperands operands;
+  q = generalProblem(*p, s, &x, &dy, &operands);
+  if (operands.copies) {
+    void *ws = nullptr;
+    if (int rc = scratch(ctx, kSlotRepacked, operands.bytes + 256, &ws)) return rc;
+    for (int i = 0; i < operands.copies; ++i)
+      *operands.operand[i] = operands.jobs[i].dst = static_cast<uint8_t *>(ws) + operands.offset[i];
+    if (int rc = repack(ctx, operands.jobs, operands.copies)) return rc;
   }
-  plb_conv_params q16 = *p;
-  if (is_float) {
-    q16.input_type = PLB_BFLOAT16;
-    q16.batch *= 3;
-  }
-  WuProblem q = wuProblem(q16, s, l, p->groups);
+  const WuLayout &l = operands.layout;
   q.x = x;
   q.dy = dy;
   gather.sub = uint32_t(q.sub);

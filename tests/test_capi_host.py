@@ -190,6 +190,27 @@ def test_forced_resident_weights_with_splits_and_groups():
     assert plan(3, 0) == (0, 1)
 
 
+def test_weight_update_plans_describe_what_runs():
+    mk = capi.ConvParams.make
+    # a first layer contracts windows of 64 over the rearranged input (4 x 16 channels of
+    # 115 x 115 pixels), its 4 folded filter rows in one unit split over the device
+    stem = capi.conv_wu_plan(mk(256, [224, 224], [7, 7], 3, 64, padding=3, stride=2))
+    rearranged = (256 * 115 * 115 * 16 + 64) * 2
+    assert (stem.split_k, stem.grid, stem.tile_n) == (148, 148, 4 * 64)
+    assert stem.workspace_bytes == 148 * 4 * 64 * 64 * 4 + rearranged + 256
+    # whole layers need the partial sums only, others copies of whole 128-byte rows too
+    whole = capi.conv_wu_plan(mk(4, [9, 9], [3, 3], 64, 64, padding=1))
+    assert whole.workspace_bytes == whole.split_k * 9 * 64 * 64 * 4
+    ragged = capi.conv_wu_plan(mk(4, [9, 9], [3, 3], 20, 36, padding=1))
+    pixels = 4 * 9 * 9
+    assert ragged.workspace_bytes >= ragged.split_k * 9 * 20 * 36 * 4 + pixels * (64 + 128)
+    # float: three planes of each operand
+    pieces = capi.conv_wu_plan(mk(4, [9, 9], [3, 3], 64, 64, padding=1, input_type=capi.FLOAT, output_type=capi.FLOAT))
+    assert pieces.workspace_bytes == pieces.split_k * 9 * 64 * 64 * 4 + 2 * 3 * ((pixels * 128 + 255) // 256 * 256)
+    assert pieces.flops == whole.flops
+    assert capi.conv_wu_plan(mk(4, [9, 9], [3, 3], 0, 64, padding=1)).tiles == 0
+
+
 def test_3d_layers_plan_as_2d_layers_with_depth_folded_into_channels():
     """A 3-D field runs as the 2-D problem over the inner dimensions with the
     kernel depth folded into the channels: batch * out-depth images and KD * Ci
