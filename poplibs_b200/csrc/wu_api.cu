@@ -761,7 +761,8 @@ int plb_conv_wu(plb_context *ctx, const plb_conv_params *p, const plb_conv_optio
   };
   S2dShape g2{};
   WuProblem q;
-  if (rearrangedProblem(*p, s, &g2, &q)) {
+  // (output gradients off the 16-byte alignment have to be copied: the general form does)
+  if ((reinterpret_cast<uintptr_t>(d_out_grads) & 15) == 0 && rearrangedProblem(*p, s, &g2, &q)) {
     void *ws = nullptr;
     if (int rc = scratch(ctx, kSlotOperands, rearrangedBytes(g2), &ws)) return rc;
     if (int rc = smallChannelPrepare(ctx, g2, d_acts, static_cast<__half *>(ws), nullptr, nullptr, co)) return rc;

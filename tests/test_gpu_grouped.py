@@ -135,6 +135,29 @@ def test_first_layer_weight_gradient(gpu_ctx, chans, kernel, stride):
         exact(T.gpu_conv_fwd(p, x, w), oracle.conv_fwd(spec, x, w), f"fwd width {width} co {co}")
 
 
+@pytest.mark.parametrize("chans,co", [(3, 64), (1, 8), (20, 24), (16, 64)])
+def test_weight_gradient_of_operands_at_any_address(gpu_ctx, chans, co):
+    """Tensors that start at odd elements of an allocation."""
+    import torch
+    p = capi.ConvParams.make(batch=2, field=[11, 13], kernel=[3, 3], in_chans=chans, out_chans=co, padding=1, stride=2)
+    r = T.rng(chans)
+    x = ints(r, (2, chans, 11, 13), np.float16)
+    dy = ints(r, (2, co, *p.output_field()), np.float16)
+    want = oracle.conv_wu(T.spec_from_params(p), x, dy)[0]
+    for off in ((1, 0), (0, 1), (3, 5)):
+        on = []
+        for t, o in zip((x, dy), off):
+            a = T.acts_to_device_layout(t).ravel()
+            buf = torch.zeros(a.size + o, dtype=torch.float16, device="cuda")
+            buf[o:] = torch.from_numpy(a)
+            on.append(buf[o:])
+        dw = torch.empty((3, 3, co, chans), device="cuda")
+        torch.cuda.synchronize()
+        T.context().conv_wu(p, on[0], on[1], None, dw)
+        T.context().synchronize()
+        exact(T.weights_from_device_layout(dw.cpu().numpy()[None]), want, f"offsets {off}")
+
+
 @pytest.mark.parametrize("elem", [1, 2, 4])
 @pytest.mark.parametrize("rows,cols", [(1, 1), (3, 130), (64, 64), (65, 63), (128, 96), (33, 257), (200, 4), (1000, 72)])
 def test_transpose(gpu_ctx, elem, rows, cols):
