@@ -510,11 +510,12 @@ int transposedWeights(plb_context *ctx, const void *w, uint32_t groups, uint64_t
 // (w mod str_w) is not in the masks, inside the window that starts at (h0, w0):
 // the input positions of a strided layer that no output reads.  Only those are
 // written (clearing the whole gradient first cost the layer 1x1, stride 2, 256
-// images of 56x56x256 a third more bytes: 67 us of memset, now 50).
+// images of 56x56x256 a third more bytes: 67 us of memset, now 50).  A block takes
+// `each` pixels of a row: the rows of a 1-D layer are few and long.
 template <typename V>
 __global__ void __launch_bounds__(256)
 zeroPhasesKernel(V *__restrict__ dst, uint32_t H, uint32_t W, uint32_t h0, uint32_t w0, uint32_t He, uint32_t We,
-                 uint32_t str_h, uint32_t str_w, uint64_t rows_used, uint64_t cols_used, uint32_t vecs) {
+                 uint32_t str_h, uint32_t str_w, uint64_t rows_used, uint64_t cols_used, uint32_t vecs, uint32_t each) {
   // (in this order: the launches that follow write other positions and start beside
   // this one, but behind what came before it, see IgemmChain)
   pdl_wait();
@@ -522,13 +523,14 @@ zeroPhasesKernel(V *__restrict__ dst, uint32_t H, uint32_t W, uint32_t h0, uint3
   const uint32_t h = blockIdx.x % He, n = blockIdx.x / He;
   V *row = dst + ((size_t(n) * H + h0 + h) * W + w0) * vecs;
   const bool all = !(rows_used >> (h % str_h) & 1);
+  const uint32_t first = blockIdx.y * each, end = first + min(each, We - first);
   const V zero{};
   if (all) {
-    for (uint32_t i = threadIdx.x; i < We * vecs; i += blockDim.x) row[i] = zero;
+    for (size_t i = size_t(first) * vecs + threadIdx.x; i < size_t(end) * vecs; i += blockDim.x) row[i] = zero;
     return;
   }
   // a warp per pixel
-  for (uint32_t w = threadIdx.x / 32; w < We; w += blockDim.x / 32)
+  for (uint32_t w = first + threadIdx.x / 32; w < end; w += blockDim.x / 32)
     if (!(cols_used >> (w % str_w) & 1))
       for (uint32_t i = threadIdx.x & 31; i < vecs; i += 32) row[size_t(w) * vecs + i] = zero;
 }
@@ -537,13 +539,14 @@ int zeroPhases(plb_context *ctx, void *dx, const plb_conv_params &p, const ConvS
                uint64_t cols_used) {
   const size_t pixel = size_t(p.groups) * p.in_chans_per_group * dtypeBytes(p.output_type);
   const uint64_t rows = uint64_t(p.batch) * s.He;
-  if (rows > 0x7fffffffull || uint64_t(s.We) * pixel > 0x7fffffffull)
-    return fail(PLB_ERR_UNSUPPORTED, "input gradient too large");
+  // 64 KB a block, whole rows up to there
+  const uint64_t each = std::max<uint64_t>({1, 65536 / pixel, (uint64_t(s.We) + 65534) / 65535});
   auto launch = [&](auto v) {
     using V = decltype(v);
-    return launchPdl(ctx, zeroPhasesKernel<V>, dim3(unsigned(rows)), dim3(256), 0, static_cast<V *>(dx), uint32_t(s.H),
+    return launchPdl(ctx, zeroPhasesKernel<V>, dim3(unsigned(rows), unsigned((uint64_t(s.We) + each - 1) / each)), dim3(256),
+                     0, static_cast<V *>(dx), uint32_t(s.H),
                      uint32_t(s.W), uint32_t(s.tH), uint32_t(s.tW), uint32_t(s.He), uint32_t(s.We), uint32_t(s.strH),
-                     uint32_t(s.strW), rows_used, cols_used, uint32_t(pixel / sizeof(V)));
+                     uint32_t(s.strW), rows_used, cols_used, uint32_t(pixel / sizeof(V)), uint32_t(each));
   };
   const size_t at = pixel | (reinterpret_cast<uintptr_t>(dx) & 15);
   if (at % 16 == 0) return launch(uint4());
@@ -584,7 +587,7 @@ int convBwdStrided(plb_context *ctx, const plb_conv_params &p, const plb_conv_op
   }
   bool lead_done = false;
   if (any_empty && !s.zero_fill_in) {  // (otherwise the caller has cleared it)
-    if (s.strH <= 64 && s.strW <= 64) {
+    if (s.strH <= 64 && s.strW <= 64 && uint64_t(p.batch) * s.He <= 0x7fffffffull) {
       if (int rc = zeroPhases(ctx, dx, p, s, rows_used, cols_used)) return rc;
       lead_done = true;
     } else {

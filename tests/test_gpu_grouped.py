@@ -135,6 +135,29 @@ def test_first_layer_weight_gradient(gpu_ctx, chans, kernel, stride):
         exact(T.gpu_conv_fwd(p, x, w), oracle.conv_fwd(spec, x, w), f"fwd width {width} co {co}")
 
 
+@pytest.mark.parametrize("chans", [8, 3, 40])
+@pytest.mark.parametrize("width,stride", [(4096, 2), (4097, 2), (8200, 3), (21846, 5)])
+def test_unread_positions_of_long_rows_get_zero(gpu_ctx, width, stride, chans):
+    """Rows that several blocks clear (4096 pixels of 8 channels each)."""
+    p = capi.ConvParams.make(batch=2, field=[width], kernel=[1], in_chans=chans, out_chans=8, stride=stride)
+    r = T.rng(width)
+    w, dy = ints(r, (1, 8, chans, 1), np.float16), ints(r, (2, 8, *p.output_field()), np.float16)
+    exact(T.gpu_conv_bwd(p, dy, w), oracle.conv_bwd(T.spec_from_params(p), dy, w), "bwd")
+
+
+def test_unread_positions_of_a_row_beyond_2_gb(gpu_ctx):
+    import torch
+    width, chans = 2 ** 20 + 2, 1024
+    p = capi.ConvParams.make(batch=1, field=[width], kernel=[1], in_chans=chans, out_chans=8, stride=2)
+    dy = torch.randint(-1, 2, (1, width // 2, 8), device="cuda").half()
+    w = torch.randint(-1, 2, (1, 1, 8, chans), device="cuda").half()
+    dx = torch.full((1, width, chans), 7.0, dtype=torch.float16, device="cuda")
+    torch.cuda.synchronize()
+    T.context().conv_bwd(p, dy, w, dx)
+    T.context().synchronize()
+    assert torch.equal(dx[0, ::2], dy[0] @ w[0, 0]) and not dx[0, 1::2].any()
+
+
 @pytest.mark.parametrize("chans,co", [(3, 64), (1, 8), (20, 24), (16, 64)])
 def test_weight_gradient_of_operands_at_any_address(gpu_ctx, chans, co):
     """Tensors that start at odd elements of an allocation."""
