@@ -2,9 +2,8 @@
 // column-tile width are compiled in a file of their own (igemm_bn*.cu).
 #pragma once
 
-#include <algorithm>
-
 #include "igemm_sm100.cuh"
+#include "launch_shape.h"
 #include "runtime.h"
 
 namespace plb {
@@ -77,10 +76,7 @@ int launchInstance(plb_context *ctx, const CUtensorMap &ta, const CUtensorMap &t
         if (n <= 0) return fail(PLB_ERR_CUDA, "no cluster of two CTAs can be resident on this device");
         max_clusters[dev] = n;
       }
-      int clusters = std::max(1, std::min(v.grid / 2, max_clusters[dev]));
-      clusters = clusters / v.grid_multiple * v.grid_multiple;
-      if (clusters == 0) return fail(PLB_ERR_CUDA, "too few clusters can be resident for this number of groups");
-      cfg.gridDim = dim3(unsigned(2 * clusters));
+      cfg.gridDim = dim3(unsigned(2 * clusterCount(v.grid / 2, max_clusters[dev], v.grid_multiple)));
     }
     cfg.attrs = attr;
     cfg.numAttrs = n_attr;

@@ -139,7 +139,8 @@ int planIgemm(const IgemmProblem &p, int sm_count, plb_plan *plan) {
   // With several groups a CTA (pair) works on one of them alone: as many as can run
   // side by side if residency is asked for, and no K splits, which are neighbouring
   // units (a tile's splits would be different groups' units to the CTAs).
-  const long most_groups = force_resident ? (pair ? sms_for_pair / 2 : sms_for_pair) : kMaxResidentGroups;
+  const long side_by_side = pair ? sms_for_pair / 2 : sms_for_pair;
+  const long most_groups = force_resident ? side_by_side : std::min<long>(kMaxResidentGroups, side_by_side);
   plan->resident_weights =
       ((p.plan_flags & PLB_PLAN_NO_RESIDENT_WEIGHTS) == 0 && n_tiles == 1 && groups <= most_groups && !p.a_mn &&
        (groups == 1 || p.force_split_k <= 1) && resident_bytes <= kMaxResidentBytes && want_resident)

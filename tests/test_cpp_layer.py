@@ -27,6 +27,18 @@ def test_poplin_host_layer(tmp_path):
     assert "all host checks passed" in out.stdout
 
 
+def test_cluster_count_of_a_device_with_few_clusters(tmp_path):
+    """Resident weights with groups need a multiple of the groups' clusters, on any device."""
+    src = tmp_path / "clusters.cpp"
+    src.write_text('#include <cstdio>\n#include "launch_shape.h"\nint main() {'
+                   'for (int w : {7, 14, 70}) for (int r : {0, 1, 6, 7, 13, 66, 74})'
+                   'std::printf("%d\\n", plb::clusterCount(w, r, 7)); }')
+    exe = tmp_path / "clusters"
+    subprocess.run(["g++", "-std=c++17", "-I" + os.path.join(ROOT, "poplibs_b200", "csrc"), str(src), "-o", str(exe)], check=True)
+    got = [int(v) for v in subprocess.run([str(exe)], capture_output=True, text=True, check=True).stdout.split()]
+    assert got == [7] * 7 + [7, 7, 7, 7, 7, 14, 14] + [7, 7, 7, 7, 7, 63, 70]
+
+
 def tool(name):
     from poplibs_b200 import build
     build.build_tools()
