@@ -596,7 +596,8 @@ int plb_context_create_on_stream(int device, void *cuda_stream, plb_context **ou
     ctx->d_status = static_cast<int *>(dev_word);
   }
   if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void **>(&ctx->d_ticket), 256);
-  if (e == cudaSuccess) e = cudaMemset(ctx->d_ticket, 0, 256);
+  // (on the context's stream: the legacy stream's work is not ordered with a non-blocking one's)
+  if (e == cudaSuccess) e = cudaMemsetAsync(ctx->d_ticket, 0, 256, ctx->stream);
   if (e != cudaSuccess) {
     plb_context_destroy(ctx);
     return cudaFail(e, "status word allocation");
