@@ -802,7 +802,7 @@ static size_t wuPeerChunks(const plb_conv_params &p, const WuShape &s) {
 
 uint64_t plb_conv_wu_allreduce_flag_bytes(const plb_conv_params *p) {
   WuShape s;
-  if (!p || wuShape(*p, &s)) return 0;
+  if (!p || p->input_type == PLB_FLOAT || wuShape(*p, &s)) return 0;  // (the fused pass takes half operands)
   // per chunk a word per sender, then a word per chunk for the owner's "sum complete"
   return uint64_t(wuPeerChunks(*p, s)) * (kWuPeerMaxWorld + 1) * sizeof(uint32_t);
 }

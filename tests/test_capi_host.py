@@ -211,6 +211,12 @@ def test_weight_update_plans_describe_what_runs():
     assert capi.conv_wu_plan(mk(4, [9, 9], [3, 3], 0, 64, padding=1)).tiles == 0
 
 
+def test_fused_all_reduce_needs_no_flags_for_layers_it_refuses():
+    flags = lambda t: capi.lib().plb_conv_wu_allreduce_flag_bytes(
+        C.byref(capi.ConvParams.make(4, [9, 9], [3, 3], 64, 64, padding=1, input_type=t, output_type=t)))
+    assert flags(capi.HALF) > 0 and flags(capi.FLOAT) == 0
+
+
 def test_3d_layers_plan_as_2d_layers_with_depth_folded_into_channels():
     """A 3-D field runs as the 2-D problem over the inner dimensions with the
     kernel depth folded into the channels: batch * out-depth images and KD * Ci
