@@ -22,26 +22,6 @@ int convFwdSmallChannels(plb_context *ctx, const plb_conv_params &p, const plb_c
                          const void *d_in, const void *d_weights, const float *d_bias,
                          void *d_out, plb_plan *plan_only);
 
-plb_conv_params floatRouteConvParams(const plb_conv_params &p, int pass) {
-  plb_conv_params q = p;
-  q.input_type = PLB_BFLOAT16;
-  if (pass == PLB_PASS_TRAINING_BWD)
-    q.out_chans_per_group *= 3;
-  else if (pass == PLB_PASS_TRAINING_WU)
-    q.batch *= 3;
-  else
-    q.in_chans_per_group *= 3;
-  return q;
-}
-
-plb_matmul_desc floatRouteMatmulDesc(const plb_matmul_desc &d) {
-  plb_matmul_desc q = d;
-  q.input_type = PLB_BFLOAT16;
-  q.k *= 3;
-  q.lda = q.ldb = 0;
-  return q;
-}
-
 // TMA needs 16-byte pixel strides: 8 half / 16 quarter channels.
 static bool channelsFitTma(const plb_conv_params &p, uint32_t chans) {
   return (size_t(chans) * dtypeBytes(p.input_type)) % 16 == 0;
@@ -444,9 +424,32 @@ void bwdPhase(int phase, int in_size, int kernel, int pad, int dil, int stride, 
 // rows of `w_cols` elements, the reduction along their rows (w_k_rows = false) or
 // along `w_k_rows` rows of each tile.
 // With a lattice only its pixels are copied, if a copy is made at all (`o->lattice`).
-int prepareOperands(plb_context *ctx, int type, const void *act, uint64_t rows, uint32_t cols, const void *wgt,
-                    uint64_t w_rows, uint32_t w_cols, uint64_t w_k_rows, PassOperands *o,
-                    const Repack::Lattice *lattice = nullptr) {
+// planOperands says what has to be copied (with null pointers: for operands as aligned
+// as they need to be), prepareOperands does it.
+struct Copies {
+  Repack jobs[2];
+  const void **operand[2];
+  size_t offset[2];
+  int n = 0;
+  size_t bytes = 0;
+  void add(const Repack &job, const void **base) {
+    jobs[n] = job;
+    operand[n] = base;
+    offset[n++] = bytes;
+    bytes += (repackBytes(job) + 255) & ~size_t(255);
+  }
+};
+
+int runCopies(plb_context *ctx, Copies &c) {
+  if (c.n == 0) return PLB_OK;
+  void *ws = nullptr;
+  if (int rc = scratch(ctx, kSlotRepacked, c.bytes + 256, &ws)) return rc;
+  for (int i = 0; i < c.n; ++i) *c.operand[i] = c.jobs[i].dst = static_cast<uint8_t *>(ws) + c.offset[i];
+  return repack(ctx, c.jobs, c.n);
+}
+
+Copies planOperands(int type, const void *act, uint64_t rows, uint32_t cols, const void *wgt, uint64_t w_rows,
+                    uint32_t w_cols, uint64_t w_k_rows, PassOperands *o, const Repack::Lattice *lattice = nullptr) {
   const size_t es = dtypeBytes(type);
   const bool is_float = type == PLB_FLOAT;
   o->type = is_float ? PLB_BFLOAT16 : type;
@@ -458,40 +461,72 @@ int prepareOperands(plb_context *ctx, int type, const void *act, uint64_t rows, 
   auto unfit = [&](const void *base, uint32_t c) {
     return is_float || (c * es) % 16 != 0 || (reinterpret_cast<uintptr_t>(base) & 15) != 0;
   };
-  Repack jobs[2];
-  const void **operand[2];
-  size_t offset[2] = {0, 0}, total = 0;
-  int n = 0;
+  Copies c;
   if (unfit(act, cols)) {
     o->act_pitch = is_float ? roundToRow(3 * uint64_t(cols), 2) : roundToRow(cols, es);
-    jobs[n] = Repack{act, nullptr, rows, cols, cols, o->act_pitch, uint32_t(es),
-                     is_float ? kRepackSplitCols : kRepackCopy, false, 0, {}};
+    Repack job{act, nullptr, rows, cols, cols, o->act_pitch, uint32_t(es), is_float ? kRepackSplitCols : kRepackCopy, false, 0, {}};
     if (lattice) {
-      jobs[n].lattice = *lattice;
-      jobs[n].rows = rows / (uint64_t(lattice->full_h) * lattice->full_w) * lattice->sub_h * lattice->sub_w;
+      job.lattice = *lattice;
+      job.rows = rows / (uint64_t(lattice->full_h) * lattice->full_w) * lattice->sub_h * lattice->sub_w;
       o->lattice = true;
     }
-    operand[n++] = &o->act;
+    c.add(job, &o->act);
   }
   if (unfit(wgt, w_cols)) {
     const bool along_rows = is_float && w_k_rows == 0;
     o->w_pitch = along_rows ? roundToRow(3 * uint64_t(w_cols), 2) : roundToRow(w_cols, is_float ? 2 : es);
-    jobs[n] = Repack{wgt, nullptr, w_rows, w_cols, w_cols, o->w_pitch, uint32_t(es),
-                     !is_float ? kRepackCopy : along_rows ? kRepackSplitCols : kRepackSplitPlanes, true, w_k_rows, {}};
-    operand[n++] = &o->wgt;
+    c.add(Repack{wgt, nullptr, w_rows, w_cols, w_cols, o->w_pitch, uint32_t(es),
+                 !is_float ? kRepackCopy : along_rows ? kRepackSplitCols : kRepackSplitPlanes, true, w_k_rows, {}},
+          &o->wgt);
   }
-  if (n == 0) return PLB_OK;
-  for (int i = 0; i < n; ++i) {
-    offset[i] = total;
-    total += (repackBytes(jobs[i]) + 255) & ~size_t(255);
+  return c;
+}
+
+int prepareOperands(plb_context *ctx, int type, const void *act, uint64_t rows, uint32_t cols, const void *wgt,
+                    uint64_t w_rows, uint32_t w_cols, uint64_t w_k_rows, PassOperands *o,
+                    const Repack::Lattice *lattice = nullptr) {
+  Copies c = planOperands(type, act, rows, cols, wgt, w_rows, w_cols, w_k_rows, o, lattice);
+  return runCopies(ctx, c);
+}
+
+// The same for a matrix product: rows of any pitch.  The pitches become those of what
+// the kernel reads.
+Copies planCopies(const plb_matmul_desc &d, const void **a, long long *lda, bool a_is_km, const void **b, long long *ldb,
+                  bool b_is_nk) {
+  const bool is_float = d.input_type == PLB_FLOAT;
+  const size_t es = dtypeBytes(d.input_type);
+  Copies c;
+  // (all groups' rows are uniformly `pitch` elements apart)
+  auto add = [&](const void **base, long long *pitch, uint64_t rows, uint32_t cols, bool k_along_rows, bool weights) {
+    if (!is_float && (reinterpret_cast<uintptr_t>(*base) & 15) == 0 && (size_t(*pitch) * es) % 16 == 0) return;
+    const int mode = !is_float ? kRepackCopy : k_along_rows ? kRepackSplitPlanes : kRepackSplitCols;
+    const uint32_t pitch_out = mode == kRepackCopy ? roundToRow(cols, es)
+                                                   : roundToRow(mode == kRepackSplitCols ? 3 * uint64_t(cols) : cols, 2);
+    c.add(Repack{*base, nullptr, rows, cols, uint64_t(*pitch), pitch_out, uint32_t(es), mode, weights, d.k, {}}, base);
+    *pitch = pitch_out;
+  };
+  add(a, lda, uint64_t(d.groups) * (a_is_km ? d.k : d.m), a_is_km ? d.m : d.k, a_is_km, false);
+  add(b, ldb, uint64_t(d.groups) * (b_is_nk ? d.n : d.k), b_is_nk ? d.k : d.n, !b_is_nk, true);
+  return c;
+}
+
+// The product that is contracted: float operands as three bfloat16 terms per product.
+plb_matmul_desc contractionDesc(const plb_matmul_desc &d) {
+  plb_matmul_desc q = d;
+  if (d.input_type == PLB_FLOAT) {
+    q.input_type = PLB_BFLOAT16;
+    q.k = 3 * d.k;
   }
-  void *ws = nullptr;
-  if (int rc = scratch(ctx, kSlotRepacked, total + 256, &ws)) return rc;
-  for (int i = 0; i < n; ++i) {
-    jobs[i].dst = static_cast<uint8_t *>(ws) + offset[i];
-    *operand[i] = jobs[i].dst;
-  }
-  return repack(ctx, jobs, n);
+  return q;
+}
+
+// The pixels that a strided pointwise layer reads, where its input has to be copied.
+bool readPixels(const plb_conv_params &p, const ConvShape &s, Repack::Lattice *sub) {
+  if (!pointwise(s) || (s.strH == 1 && s.strW == 1) || s.tH != 0 || s.tW != 0) return false;
+  *sub = Repack::Lattice{p.groups, uint32_t(latticeExtent(s.We, s.OWc, s.strW)),
+                         uint32_t(latticeExtent(s.He, s.OHc, s.strH)), uint32_t(s.W), uint32_t(s.H),
+                         uint32_t(s.strW), uint32_t(s.strH)};
+  return uint64_t(p.batch) * sub->sub_h * sub->sub_w <= 0xffffffffull;
 }
 
 // Quarter weights of a pass that reduces over their rows: 8-bit operands have no
@@ -671,15 +706,6 @@ extern "C" {
 int plb_matmul_plan(const plb_matmul_desc *desc, plb_plan *plan) {
   if (!desc || !plan) return fail(PLB_ERR_INVALID_PARAMS, "null argument");
   if (int rc = checkMatmulDesc(*desc)) return rc;
-  if (desc->input_type == PLB_FLOAT) {
-    // what runs: bfloat16 operands, three terms per product (repack.cu)
-    const plb_matmul_desc q = floatRouteMatmulDesc(*desc);
-    if (int rc = plb_matmul_plan(&q, plan)) return rc;
-    plan->flops = 2ull * desc->groups * desc->m * desc->k * desc->n;
-    plan->bytes = gemmBytes(*desc);
-    plan->workspace_bytes += size_t(desc->groups) * desc->k * (size_t(desc->m) + desc->n) * 6 + 768;
-    return PLB_OK;
-  }
   *plan = plb_plan{};
   plan->flops = 2ull * desc->groups * desc->m * desc->k * desc->n;
   plan->bytes = gemmBytes(*desc);
@@ -687,12 +713,24 @@ int plb_matmul_plan(const plb_matmul_desc *desc, plb_plan *plan) {
   const Ld ld = leadingDims(*desc);
   const bool b_is_nk = desc->transpose_b || desc->input_type == PLB_QUARTER;
   const bool a_is_km = desc->transpose_a && desc->input_type != PLB_QUARTER;
-  IgemmProblem p = gemmProblem(*desc, nullptr, ld.a, a_is_km, nullptr, ld.b, b_is_nk, nullptr, nullptr, ld.c);
+  // quarter operands stored the other way are transposed, rows that TMA cannot address copied
+  const void *a = nullptr, *b = nullptr;  // (as aligned as they need to be)
+  long long lda = ld.a, ldb = ld.b;
+  const uint64_t pitch = roundToRow(desc->k, 1);
+  size_t transposed = 0;
+  if (desc->transpose_a && !a_is_km) {
+    transposed += (size_t(desc->groups) * desc->m * pitch + 255) & ~size_t(255);
+    lda = (long long)pitch;
+  }
+  if (!desc->transpose_b && b_is_nk) {
+    transposed += size_t(desc->groups) * desc->n * pitch;
+    ldb = (long long)pitch;
+  }
+  const Copies copies = planCopies(*desc, &a, &lda, a_is_km, &b, &ldb, b_is_nk);
+  const IgemmProblem p =
+      gemmProblem(contractionDesc(*desc), nullptr, lda, a_is_km, nullptr, ldb, b_is_nk, nullptr, nullptr, ld.c);
   if (int rc = planIgemm(p, 148, plan)) return rc;
-  const size_t es = dtypeBytes(desc->input_type);
-  if (desc->transpose_a && !a_is_km) plan->workspace_bytes += size_t(desc->groups) * desc->m * desc->k * es;
-  if (!desc->transpose_b && desc->input_type == PLB_QUARTER)
-    plan->workspace_bytes += size_t(desc->groups) * desc->n * desc->k * es;
+  plan->workspace_bytes += transposed + copies.bytes;
   return PLB_OK;
 }
 
@@ -724,7 +762,6 @@ int plb_matmul(plb_context *ctx, const plb_matmul_desc *desc, const void *d_a, c
   // Operand layouts the kernel takes directly: A as [m][k], B as [n][k], or (not
   // 8-bit) A as [k][m] and B as [k][n].  8-bit operands stored the other way go
   // through a transpose into scratch.
-  plb_matmul_desc q = d;
   const void *a = d_a, *b = d_b;
   long long lda = ld.a, ldb = ld.b;
   bool a_is_km = d.transpose_a != 0, b_is_nk = d.transpose_b != 0;
@@ -757,43 +794,11 @@ int plb_matmul(plb_context *ctx, const plb_matmul_desc *desc, const void *d_a, c
   // 16 bytes: n % 8 != 0, odd leading dimensions) are copied once into scratch
   // with the pitch rounded up, float operands are split into their bfloat16
   // pieces, both operands in one launch.  The output needs no such copy.
-  {
-    const bool is_float = d.input_type == PLB_FLOAT;
-    const uint64_t a_rows = uint64_t(d.groups) * (a_is_km ? d.k : d.m), b_rows = uint64_t(d.groups) * (b_is_nk ? d.n : d.k);
-    const uint32_t a_cols = a_is_km ? d.m : d.k, b_cols = b_is_nk ? d.k : d.n;
-    if (is_float && (lda < (long long)a_cols || ldb < (long long)b_cols))
-      return fail(PLB_ERR_INVALID_PARAMS, "leading dimension shorter than a row");
-    auto unfit = [&](const void *base, long long pitch) {
-      return is_float || (reinterpret_cast<uintptr_t>(base) & 15) != 0 || (size_t(pitch) * es) % 16 != 0;
-    };
-    Repack jobs[2];
-    const void **operand[2];
-    int n = 0;
-    // (all groups' rows are uniformly `pitch` elements apart)
-    auto add = [&](const void **base, long long *pitch, uint64_t rows, uint32_t cols, bool k_along_rows, bool weights) {
-      if (!unfit(*base, *pitch)) return;
-      const int mode = !is_float ? kRepackCopy : k_along_rows ? kRepackSplitPlanes : kRepackSplitCols;
-      const uint32_t pitch_out = mode == kRepackCopy ? roundToRow(cols, es)
-                                                     : roundToRow(mode == kRepackSplitCols ? 3 * uint64_t(cols) : cols, 2);
-      jobs[n] = Repack{*base, nullptr, rows, cols, uint64_t(*pitch), pitch_out, uint32_t(es), mode, weights, d.k, {}};
-      *pitch = pitch_out;
-      operand[n++] = base;
-    };
-    add(&a, &lda, a_rows, a_cols, a_is_km, false);
-    add(&b, &ldb, b_rows, b_cols, !b_is_nk, true);
-    if (n) {
-      size_t bytes[2] = {0, 0};
-      for (int i = 0; i < n; ++i) bytes[i] = (repackBytes(jobs[i]) + 255) & ~size_t(255);
-      void *ws = nullptr;
-      if (int rc = scratch(ctx, kSlotRepacked, bytes[0] + bytes[1] + 256, &ws)) return rc;
-      for (int i = 0; i < n; ++i) *operand[i] = jobs[i].dst = static_cast<uint8_t *>(ws) + (i ? bytes[0] : 0);
-      if (int rc = repack(ctx, jobs, n)) return rc;
-    }
-    if (is_float) {
-      q.input_type = PLB_BFLOAT16;
-      q.k = 3 * d.k;
-    }
-  }
+  if (d.input_type == PLB_FLOAT && (lda < (long long)(a_is_km ? d.m : d.k) || ldb < (long long)(b_is_nk ? d.k : d.n)))
+    return fail(PLB_ERR_INVALID_PARAMS, "leading dimension shorter than a row");
+  Copies copies = planCopies(d, &a, &lda, a_is_km, &b, &ldb, b_is_nk);
+  if (int rc = runCopies(ctx, copies)) return rc;
+  const plb_matmul_desc q = contractionDesc(d);
   IgemmProblem p = gemmProblem(q, a, lda, a_is_km, b, ldb, b_is_nk, d_c, d_d, ld.c);
   return runProblem(ctx, p);
 }
@@ -857,18 +862,6 @@ uint64_t plb_conv_macs(const plb_conv_params *p) { return p ? numberOfMacs(*p) :
 int plb_conv_plan(const plb_conv_params *p_in, const plb_conv_options *opt, int32_t pass,
                   plb_plan *plan) {
   if (!p_in || !plan) return fail(PLB_ERR_INVALID_PARAMS, "null argument");
-  if (p_in->input_type == PLB_FLOAT) {
-    // what runs: bfloat16 operands, three terms per product (repack.cu)
-    const std::string err = validate(*p_in);
-    if (!err.empty()) return fail(PLB_ERR_INVALID_PARAMS, err);
-    const plb_conv_params q = floatRouteConvParams(*p_in, pass);
-    if (int rc = plb_conv_plan(&q, opt, pass, plan)) return rc;
-    plan->flops = 2 * numberOfMacs(*p_in);
-    size_t n_in, n_w, n_out;
-    convElementCounts(*p_in, &n_in, &n_w, &n_out);
-    plan->workspace_bytes += ((pass == PLB_PASS_TRAINING_BWD ? n_out : n_in) + n_w) * 6 + 768;
-    return PLB_OK;
-  }
   if (p_in->num_field_dims == 3) return conv3dPlan(*p_in, opt, pass, plan);
   // a flipped input runs as the ordinary convolution of the reversed tensor
   plb_conv_params unflipped, undilated;
@@ -879,7 +872,7 @@ int plb_conv_plan(const plb_conv_params *p_in, const plb_conv_options *opt, int3
   ConvShape s;
   if (int rc = igemmConvShape(*p, &s)) return rc;
   *plan = plb_plan{};
-  if (pass != PLB_PASS_TRAINING_BWD && !channelsFitTma(*p, p->in_chans_per_group)) {
+  if (pass != PLB_PASS_TRAINING_BWD && p->input_type != PLB_FLOAT && !channelsFitTma(*p, p->in_chans_per_group)) {
     const int rc = convFwdSmallChannels(nullptr, *p, opt, nullptr, nullptr, nullptr, nullptr, plan);
     if (rc == PLB_OK) {
       plan->flops = 2 * numberOfMacs(*p);
@@ -888,20 +881,33 @@ int plb_conv_plan(const plb_conv_params *p_in, const plb_conv_options *opt, int3
     }
     if (rc != PLB_ERR_UNSUPPORTED) return rc;
   }
-  // narrow groups run together, channel counts TMA cannot address rounded up
+  // narrow groups run together; channel counts TMA cannot address and float operands on copies
   plb_conv_params run = *p;
   const uint32_t together = groupsTogether(p->groups, p->in_chans_per_group, p->out_chans_per_group, p->input_type);
   run.groups /= together;
   run.in_chans_per_group *= together;
   run.out_chans_per_group *= together;
-  const bool bwd = pass == PLB_PASS_TRAINING_BWD;
-  PassOperands o{run.input_type, nullptr, nullptr, bwd ? run.out_chans_per_group : run.in_chans_per_group, 0, 0};
-  o.act_pitch = roundToRow(o.k, dtypeBytes(run.input_type));
-  o.w_pitch = roundToRow(run.in_chans_per_group, dtypeBytes(run.input_type));
-  const IgemmProblem q = bwd ? convBwdProblem(run, opt, s, o, nullptr, run.input_type == PLB_QUARTER)
-                             : convFwdProblem(run, opt, s, o, nullptr, nullptr);
-  if (q.n_total > 0 && q.out_w > 0 && q.out_h > 0 && q.out_n > 0 && q.k_per_tap > 0)
+  const bool bwd = pass == PLB_PASS_TRAINING_BWD, transposed = bwd && run.input_type == PLB_QUARTER;
+  const uint64_t tiles = uint64_t(run.groups) * s.KHs * s.KWs, pixels = uint64_t(run.batch) * run.groups;
+  const uint32_t ci = run.in_chans_per_group, co = run.out_chans_per_group;
+  if (run.batch != 0 && run.groups != 0 && ci != 0 && co != 0 && s.KH > 0 && s.KW > 0 && s.OHc > 0 && s.OWc > 0 &&
+      s.He > 0 && s.We > 0) {
+    PassOperands o;
+    Repack::Lattice sub{};
+    const uint32_t pitch = transposed ? roundToRow(co, 1) : ci;
+    const Copies copies =
+        bwd ? planOperands(run.input_type, nullptr, pixels * s.OH * s.OW, co, nullptr, transposed ? tiles * ci : tiles * co,
+                           pitch, transposed ? 0 : co, &o)
+            : planOperands(run.input_type, nullptr, pixels * s.H * s.W, ci, nullptr, tiles * co, ci, 0, &o,
+                           readPixels(run, s, &sub) ? &sub : nullptr);
+    const IgemmProblem q = bwd ? convBwdProblem(run, opt, s, o, nullptr, transposed)
+                               : convFwdProblem(run, opt, s, o, nullptr, nullptr);
     if (int rc = planIgemm(q, 148, plan)) return rc;
+    const size_t es = dtypeBytes(run.input_type);
+    plan->workspace_bytes += copies.bytes;
+    if (transposed) plan->workspace_bytes += tiles * ci * pitch;
+    if (together > 1) plan->workspace_bytes += size_t(tiles) * ci * co * es;  // block-diagonal weights
+  }
   plan->flops = 2 * numberOfMacs(*p);
   plan->bytes = convBytes(*p, s, pass);
   return PLB_OK;
@@ -1003,14 +1009,8 @@ int plb_convolution(plb_context *ctx, const plb_conv_params *p, const plb_conv_o
   const uint64_t in_rows = uint64_t(q.batch) * s.H * s.W * q.groups, tiles = uint64_t(q.groups) * s.KHs * s.KWs;
   const uint32_t ci = q.in_chans_per_group, co = q.out_chans_per_group;
   const bool transposed = swapped && q.input_type == PLB_QUARTER;  // -> [G][flipped k][Co][Ci]
-  // a strided pointwise layer whose input has to be copied: only the pixels it reads
-  Repack::Lattice sub{}, *lattice = nullptr;
-  if (pointwise(s) && (s.strH > 1 || s.strW > 1) && s.tH == 0 && s.tW == 0) {
-    sub = Repack::Lattice{q.groups, uint32_t(latticeExtent(s.We, s.OWc, s.strW)),
-                          uint32_t(latticeExtent(s.He, s.OHc, s.strH)), uint32_t(s.W), uint32_t(s.H),
-                          uint32_t(s.strW), uint32_t(s.strH)};
-    if (uint64_t(q.batch) * sub.sub_h * sub.sub_w <= 0xffffffffull) lattice = &sub;
-  }
+  Repack::Lattice sub{};
+  const Repack::Lattice *lattice = readPixels(q, s, &sub) ? &sub : nullptr;
   PassOperands o;
   if (transposed) {
     uint32_t pitch = 0;

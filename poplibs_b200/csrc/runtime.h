@@ -269,10 +269,6 @@ struct IgemmProblem {
 // problem cannot be run by the igemm kernel (message recorded).
 int planIgemm(const IgemmProblem &p, int sm_count, plb_plan *plan);
 
-// What runs for float operands: bfloat16, the reduction dimension of the pass
-// three times as long (repack.cu).  For the plans.
-plb_conv_params floatRouteConvParams(const plb_conv_params &p, int pass);
-plb_matmul_desc floatRouteMatmulDesc(const plb_matmul_desc &d);
 // Matrices [batch][rows][cols] -> [batch][cols][dst_pitch].
 int transposeBatch(plb_context *ctx, uint32_t elem_bytes, uint64_t batch, uint64_t rows, uint64_t cols, const void *src,
                    void *dst, uint64_t dst_pitch);

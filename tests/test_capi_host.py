@@ -211,6 +211,36 @@ def test_weight_update_plans_describe_what_runs():
     assert capi.conv_wu_plan(mk(4, [9, 9], [3, 3], 0, 64, padding=1)).tiles == 0
 
 
+def test_plans_describe_the_operands_that_are_read():
+    """Copies, pieces of floats and block-diagonal weights count as workspace; rows that are read
+    where they lie are planned with their own pitch."""
+    mk, r256 = capi.ConvParams.make, lambda n: (n + 255) // 256 * 256
+    float_t = dict(input_type=capi.FLOAT, output_type=capi.FLOAT)
+    # 56 channels are read in place: rows at odd multiples of 16 bytes, a long reduction is split
+    flags = capi.PLAN_FORCE_CTA_PAIR | capi.PLAN_NO_RESIDENT_WEIGHTS | capi.PLAN_NO_HALO
+    plan = capi.conv_plan(mk(2, [12, 12], [3, 8], 56, 56, padding=1), capi.PASS_TRAINING_FWD,
+                          capi.ConvOptions.make(plan_flags=flags))
+    assert plan.split_k > 1 and plan.workspace_bytes == plan.split_k * 2 * 12 * 7 * 64 * 4
+    # with resident weights groups are not split
+    plan = capi.conv_plan(mk(2, [12, 12], [3, 8], 56, 56, groups=3, padding=1), capi.PASS_TRAINING_FWD, capi.ConvOptions.make(
+        plan_flags=capi.PLAN_FORCE_RESIDENT_WEIGHTS | capi.PLAN_FORCE_CTA_PAIR | capi.PLAN_NO_HALO))
+    assert (plan.resident_weights, plan.split_k) == (1, 1)
+    # 32 groups of 8: blocks of neighbouring groups, the same ones in both directions
+    for kw, split in (({}, False), (float_t, True)):
+        p = mk(4, [9, 9], [3, 3], 8, 8, groups=32, padding=1, **kw)
+        fwd, bwd = capi.conv_plan(p, capi.PASS_TRAINING_FWD), capi.conv_plan(p, capi.PASS_TRAINING_BWD)
+        assert fwd.tiles == bwd.tiles and fwd.tiles < 32 * 3
+        assert fwd.workspace_bytes > 32 * 9 * 8 * 8 * (4 if split else 2) * 4
+    # ragged rows: 40 bytes as 64; 3 pieces of 11 floats as 128 bytes; 33 quarters as 64
+    ragged = capi.conv_plan(mk(4, [9, 9], [3, 3], 20, 36, padding=1))
+    assert ragged.split_k == 1 and ragged.workspace_bytes == r256(4 * 81 * 64) + r256(9 * 36 * 64)
+    floats = capi.matmul_plan(capi.MatmulDesc.make(100, 11, 50, transpose_b=True, **float_t))
+    assert floats.workspace_bytes == r256(100 * 128) + r256(50 * 128)
+    quarter = capi.matmul_plan(capi.MatmulDesc.make(100, 33, 50, input_type=capi.QUARTER, transpose_a=True))
+    assert quarter.workspace_bytes == r256(100 * 64) + 50 * 64
+    assert capi.matmul_plan(capi.MatmulDesc.make(512, 1024, 1024)).workspace_bytes == 0
+
+
 def test_fused_all_reduce_needs_no_flags_for_layers_it_refuses():
     flags = lambda t: capi.lib().plb_conv_wu_allreduce_flag_bytes(
         C.byref(capi.ConvParams.make(4, [9, 9], [3, 3], 64, 64, padding=1, input_type=t, output_type=t)))
