@@ -929,7 +929,7 @@ int plb_convolution(plb_context *ctx, const plb_conv_params *p, const plb_conv_o
   if (p->num_field_dims == 3)
     return conv3dFwd(ctx, *p, opt, d_in, d_weights, d_bias, d_out, transpose_and_flip_weights);
   {
-    // a flipped input: reverse it once (scratch slot 8), then an ordinary convolution
+    // a flipped input: reverse it once, then an ordinary convolution
     plb_conv_params q;
     if (unflippedInputParams(*p, &q) && p->num_field_dims <= 2) {
       const std::string err = validate(*p);
@@ -946,7 +946,7 @@ int plb_convolution(plb_context *ctx, const plb_conv_params *p, const plb_conv_o
     }
   }
   {
-    // a dilated input: write the zero-stuffed tensor once (scratch slot 12)
+    // a dilated input: write the zero-stuffed tensor once
     plb_conv_params q;
     DilatedField df;
     if (undilatedInputParams(*p, &q, &df)) {
@@ -1067,7 +1067,7 @@ int plb_conv_bwd(plb_context *ctx, const plb_conv_params *p, const plb_conv_opti
     }
   }
   {
-    // a dilated input: the gradient of the zero-stuffed tensor (scratch slot 12),
+    // a dilated input: the gradient of the zero-stuffed tensor,
     // of which the lattice elements are the gradient of the input
     plb_conv_params q;
     DilatedField df;

@@ -628,7 +628,7 @@ int plb_conv_wu(plb_context *ctx, const plb_conv_params *p, const plb_conv_optio
   if (p->num_field_dims == 3)
     return conv3dWu(ctx, *p, opt, d_acts, d_out_grads, d_weight_grads, d_weight_grads_f32);
   {
-    // a flipped input: reverse it once (scratch slot 8), then an ordinary weight update
+    // a flipped input: reverse it once, then an ordinary weight update
     plb_conv_params q;
     if (unflippedInputParams(*p, &q) && p->num_field_dims <= 2) {
       const std::string err = validate(*p);
@@ -645,7 +645,7 @@ int plb_conv_wu(plb_context *ctx, const plb_conv_params *p, const plb_conv_optio
     }
   }
   {
-    // a dilated input: write the zero-stuffed tensor once (scratch slot 12)
+    // a dilated input: write the zero-stuffed tensor once
     plb_conv_params q;
     DilatedField df;
     if (undilatedInputParams(*p, &q, &df)) {
