@@ -94,6 +94,108 @@ def test_infinities_stay_in_their_group(gpu_ctx, groups, ci, co, value, stride):
     exact(T.gpu_conv_fwd(p, x, w), y, "after")
 
 
+PLAN_VARIANTS = {
+    "streamed": capi.PLAN_NO_RESIDENT_WEIGHTS,
+    "streamed no halo": capi.PLAN_NO_RESIDENT_WEIGHTS | capi.PLAN_NO_HALO,
+    "streamed pair": capi.PLAN_NO_RESIDENT_WEIGHTS | capi.PLAN_FORCE_CTA_PAIR,
+    "streamed no halo pair": capi.PLAN_NO_RESIDENT_WEIGHTS | capi.PLAN_NO_HALO | capi.PLAN_FORCE_CTA_PAIR,
+    "resident": capi.PLAN_FORCE_RESIDENT_WEIGHTS | capi.PLAN_NO_HALO,
+    "resident halo": capi.PLAN_FORCE_RESIDENT_WEIGHTS,
+    "resident pair": capi.PLAN_FORCE_RESIDENT_WEIGHTS | capi.PLAN_NO_HALO | capi.PLAN_FORCE_CTA_PAIR,
+    "resident halo pair": capi.PLAN_FORCE_RESIDENT_WEIGHTS | capi.PLAN_FORCE_CTA_PAIR,
+}
+
+
+@pytest.mark.parametrize("variant", sorted(PLAN_VARIANTS))
+@pytest.mark.parametrize("dtype", ["half", "float", "quarter"])
+@pytest.mark.parametrize("groups,ci,co", [(2, 32, 32), (3, 64, 64), (16, 8, 8), (5, 72, 40)])
+def test_every_instance_with_groups(gpu_ctx, groups, ci, co, dtype, variant):
+    """Each way the planner may run a grouped layer, on all operand types; (16, 8, 8) is
+    contracted in blocks of neighbouring groups."""
+    plb, cast, kind = {"half": (capi.HALF, lambda a: a.astype(np.float16), np.float16),
+                       "float": (capi.FLOAT, lambda a: a.astype(np.float32), np.float32),
+                       "quarter": (capi.QUARTER, oracle.e4m3_encode, np.float16)}[dtype]
+    p = capi.ConvParams.make(batch=3, field=[13, 11], kernel=[3, 3], in_chans=ci, out_chans=co, groups=groups, padding=1,
+                             input_type=plb, output_type=capi.FLOAT if dtype == "float" else capi.HALF)
+    opt = capi.ConvOptions.make(plan_flags=PLAN_VARIANTS[variant])
+    plan = capi.conv_plan(p, capi.PASS_TRAINING_FWD, opt)
+    assert plan.cta_pair == (1 if "pair" in variant else 0)
+    if "resident" in variant and dtype != "float" and ci <= 64:
+        assert plan.resident_weights == 1
+    spec, r = T.spec_from_params(p), T.rng(groups + ci)
+    x = r.integers(-1, 2, (3, groups * ci, 13, 11)).astype(np.float64)
+    w = r.integers(-1, 2, (groups, co, ci, 3, 3)).astype(np.float64)
+    dy = r.integers(-1, 2, (3, groups * co, *p.output_field())).astype(np.float64)
+    exact(T.gpu_conv_fwd(p, cast(x), cast(w), opt=opt), oracle.conv_fwd(spec, x, w), "fwd")
+    exact(T.gpu_conv_bwd(p, cast(dy), cast(w), opt=opt), oracle.conv_bwd(spec, dy, w), "bwd")
+
+
+@pytest.mark.parametrize("groups,ci,co", [(3, 64, 64), (5, 64, 32), (7, 64, 64), (32, 8, 8)])
+def test_many_tiles_with_groups(gpu_ctx, groups, ci, co):
+    """Layers large enough that the planner keeps weights resident and pairs CTAs by itself,
+    with group counts that do not divide the number of SMs."""
+    import torch
+    p = capi.ConvParams.make(batch=128, field=[28, 28], kernel=[3, 3], in_chans=ci, out_chans=co, groups=groups, padding=1)
+    plan = capi.conv_plan(p)
+    assert plan.resident_weights == 1 and plan.cta_pair == 1 and plan.tiles >= 2 * plan.grid
+    ints = lambda *s: torch.randint(-1, 2, s, device="cuda").half()
+    x, w, dy = ints(128, 28, 28, groups * ci), ints(groups, 3, 3, co, ci), ints(128, 28, 28, groups * co)
+    y, dx = torch.empty_like(dy), torch.empty_like(x)
+    torch.cuda.synchronize()
+    T.context().conv_fwd(p, x, w, y)
+    T.context().conv_bwd(p, dy, w, dx)
+    T.context().synchronize()
+    nchw = lambda t: t.permute(0, 3, 1, 2).double()
+    w64 = w.permute(0, 3, 4, 1, 2).reshape(groups * co, ci, 3, 3).double()
+    want = torch.nn.functional.conv2d(nchw(x), w64, padding=1, groups=groups)
+    assert torch.equal(nchw(y), want)
+    want = torch.nn.functional.conv_transpose2d(nchw(dy), w64, padding=1, groups=groups)
+    assert torch.equal(nchw(dx), want)
+
+
+@pytest.mark.parametrize("form", ["half, bias", "float", "quarter", "pointwise, stride 2", "transposed weights",
+                                  "float, transposed weights", "quarter, transposed weights", "split"])
+def test_infinities_stay_in_their_group_in_every_form(gpu_ctx, form):
+    """Operand types, a bias, a sub-lattice, weights stored the other way, K splits: a NaN or an
+    infinity reaches the outputs of its own group alone."""
+    import torch
+    groups, ci, co = 16, 8, 8
+    plb = capi.FLOAT if "float" in form else capi.QUARTER if "quarter" in form else capi.HALF
+    dtype = np.float32 if plb == capi.FLOAT else np.float16
+    kernel, stride = (1, 2) if "pointwise" in form else (3, 1)
+    swapped = "transposed" in form
+    p = capi.ConvParams.make(batch=2, field=[8, 6], kernel=[kernel] * 2, in_chans=ci, out_chans=co, groups=groups,
+                             padding=kernel // 2, stride=stride, input_type=plb,
+                             output_type=capi.FLOAT if plb == capi.FLOAT else capi.HALF)
+    r = T.rng(11)
+    cast = oracle.e4m3_encode if plb == capi.QUARTER else lambda a: a.astype(dtype)
+    x = cast(r.integers(-1, 2, (2, 8, 6, groups * ci)).astype(np.float64))
+    w = cast(r.choice([-1.0, 1.0], (groups, kernel, kernel) + ((ci, co) if swapped else (co, ci))))
+    bias = r.integers(-3, 4, groups * co).astype(np.float32) if "bias" in form else None
+    opt = capi.ConvOptions.make(split_k=3) if form == "split" else None
+    g = groups // 2 + 1
+
+    def run(x):
+        on = [T.to_dev(t) if t is not None else None for t in (x, w, bias)]
+        y = T.empty_dev([2] + p.output_field() + [groups * co], dtype)
+        torch.cuda.synchronize()
+        T.context().convolution(p, on[0], on[1], y, on[2], opt, swapped)
+        T.context().synchronize()
+        return y.cpu().numpy().astype(np.float64)
+
+    was = run(x)
+    for value in (0x7F,) if plb == capi.QUARTER else (np.inf, np.nan):
+        x2 = x.copy()
+        x2[1, 4, 2, g * ci + 3] = value
+        got, mine = run(x2), slice(g * co, (g + 1) * co)
+        assert not np.isfinite(got[1, ..., mine]).all()
+        same = np.isfinite(got[1, ..., mine])
+        exact(got[1, ..., mine][same], was[1, ..., mine][same], "own group, elements the value does not reach")
+        got[1, ..., mine] = was[1, ..., mine]
+        exact(got, was, "other groups")
+    exact(run(x), was, "after")
+
+
 @pytest.mark.parametrize("groups,m,k,n", [(1, 197, 70, 103), (5, 197, 70, 103), (3, 8, 8, 8), (64, 33, 64, 130),
                                           (2, 1, 513, 1), (7, 129, 65, 257), (4, 300, 1100, 40)])
 @pytest.mark.parametrize("dtype", ["half", "float", "quarter"])

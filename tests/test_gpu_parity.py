@@ -348,6 +348,10 @@ PLAN_VARIANTS = {
 }
 
 
+# layers whose weights fit beside the pipeline with and without a CTA pair
+RESIDENT = {"3x3_pad1", "kernel_dilation", "flipped_kernel", "batch1_big_field", "3x3_s2x3"}
+
+
 @pytest.mark.parametrize("variant", sorted(PLAN_VARIANTS))
 @pytest.mark.parametrize("name", ["3x3_pad1", "ragged_chans", "kernel_dilation", "asym_padding",
                                   "flipped_kernel", "batch1_big_field", "3x3_s2x3", "one_dim"])
@@ -363,6 +367,8 @@ def test_conv_plan_variants_agree_with_oracle(gpu_ctx, name, variant):
         plan = capi.conv_plan(p, capi.PASS_TRAINING_FWD, opt)
         pixel_tiles = plan.tiles // -(-p.out_chans_per_group // plan.tile_n)
         assert plan.cta_pair == (1 if pixel_tiles >= 2 else 0)
+    if variant.startswith("resident") and name in RESIDENT:
+        assert capi.conv_plan(p, capi.PASS_TRAINING_FWD, opt).resident_weights == 1
     r = T.rng(zlib.crc32((name + variant).encode()) % 1000)
     x, w, dy = conv_data(p, kw, r, exact=True)
     assert_exact(T.gpu_conv_fwd(p, x, w, opt=opt), oracle.conv_fwd(spec, x, w), f"fwd {name} {variant}")
@@ -383,6 +389,8 @@ def test_conv_split_k_agrees_with_oracle(gpu_ctx, name, variant, split):
     opt = capi.ConvOptions.make(plan_flags=PLAN_VARIANTS[variant], split_k=split)
     plan = capi.conv_plan(p, capi.PASS_TRAINING_FWD, opt)
     assert 1 <= plan.split_k <= split and (plan.split_k > 1) == (plan.workspace_bytes > 0)
+    if variant.startswith("resident") and name in RESIDENT:
+        assert plan.resident_weights == 1
     r = T.rng(zlib.crc32((name + variant).encode()) % 1000 + split)
     x, w, dy = conv_data(p, kw, r, exact=True)
     assert_exact(T.gpu_conv_fwd(p, x, w, opt=opt), oracle.conv_fwd(spec, x, w), f"fwd {name} {variant} /{split}")
