@@ -69,6 +69,24 @@ template <typename T> struct ChanVec<T, 1> {
   static __device__ __forceinline__ Raw pack(const float (&f)[1]) { return fromFloat<T>(f[0]); }
 };
 
+// Two neighbouring elements in one load.
+template <typename T> struct ChanPair;
+template <> struct ChanPair<__half> {
+  using Type = __half2;
+  static __device__ __forceinline__ void unpack(Type v, float (&f)[2]) {
+    const float2 t = __half22float2(v);
+    f[0] = t.x;
+    f[1] = t.y;
+  }
+};
+template <> struct ChanPair<float> {
+  using Type = float2;
+  static __device__ __forceinline__ void unpack(Type v, float (&f)[2]) {
+    f[0] = v.x;
+    f[1] = v.y;
+  }
+};
+
 // How [rows][chans] is walked.  A block is vec_lanes x row_lanes threads: thread
 // (vx, ry) owns vector `blockIdx.x * vec_lanes + vx` of the super-rows ry,
 // ry + stride, ... of its slab blockIdx.y.
@@ -147,6 +165,48 @@ __device__ __forceinline__ void storeChan(void *p, int is_half, uint32_t c, floa
     static_cast<__half *>(p)[c] = __float2half_rn(v);
   else
     static_cast<float *>(p)[c] = v;
+}
+
+template <typename T>
+__device__ __forceinline__ void finishChan(const ChanFinish &fin, uint32_t c, float sa, float sb) {
+  const float va = __fmul_rn(sa, fin.scale), vb = __fmul_rn(sb, fin.scale);
+  if (fin.a) storeChan(fin.a, fin.a_half, c, va);
+  if (fin.b) storeChan(fin.b, fin.b_half, c, vb);
+  if (fin.a_f32) fin.a_f32[c] = va;
+  if (fin.b_f32) fin.b_f32[c] = vb;
+  if (fin.inv_std) {
+    // plb_norm_inv_std_dev's arithmetic on the values as stored: the mean
+    // rounded to its type, the power in fp32
+    const float mean = toFloat(fromFloat<T>(va));
+    float var = vb - mean * mean;
+    if (var < 0.f) var = 0.f;
+    var = (var + fin.eps) * fin.scale_var;
+    storeChan(fin.inv_std, fin.a_half, c, 1.0f / sqrtf(var));
+  }
+  if (fin.bias) {
+    const float old = fin.bias_half ? __half2float(static_cast<const __half *>(fin.bias)[c])
+                                    : static_cast<const float *>(fin.bias)[c];
+    storeChan(fin.bias, fin.bias_half, c, old + va);
+  }
+}
+
+// What one element adds to the two sums; m is the centre.
+template <typename T, int kMode>
+__device__ __forceinline__ void addElement(float &a, float &b, float x, float y, float m) {
+  if constexpr (kMode == kSumXAndXX) {
+    a += x;
+    b += x * x;
+  } else if constexpr (kMode == kSumCentredXX) {
+    // the deviation is formed in the activations' type, as the reference's
+    // "acts - cast(mean)" map does (lib/poplin/Norms.cpp:216-219)
+    const float d = toFloat(fromFloat<T>(x - m));
+    b += d * d;
+  } else if constexpr (kMode == kSumXYAndY) {
+    a += x * y;
+    b += y;
+  } else {
+    a += x;
+  }
 }
 
 // The sums of the threads of a warp that hold the same vector (thread numbers that
@@ -228,20 +288,7 @@ chanSumsKernel(const T *__restrict__ x, const T *__restrict__ y, const T *__rest
       for (int j = 0; j < V; ++j) m[j] = toFloat(centre[(vec * V + j) % w.chans]);
   }
   auto add = [&](const float (&xv)[V], const float (&yv)[V], int j) {
-    if constexpr (kMode == kSumXAndXX) {
-      a[j] += xv[j];
-      b[j] += xv[j] * xv[j];
-    } else if constexpr (kMode == kSumCentredXX) {
-      // the deviation is formed in the activations' type, as the reference's
-      // "acts - cast(mean)" map does (lib/poplin/Norms.cpp:216-219)
-      const float d = toFloat(fromFloat<T>(xv[j] - m[j]));
-      b[j] += d * d;
-    } else if constexpr (kMode == kSumXYAndY) {
-      a[j] += xv[j] * yv[j];
-      b[j] += yv[j];
-    } else {
-      a[j] += xv[j];
-    }
+    addElement<T, kMode>(a[j], b[j], xv[j], kHasY ? yv[j] : 0.f, kMode == kSumCentredXX ? m[j] : 0.f);
   };
   if (mine) {
     const size_t step = size_t(gridDim.y) * row_lanes;
@@ -327,27 +374,6 @@ chanSumsKernel(const T *__restrict__ x, const T *__restrict__ y, const T *__rest
   }
   __syncthreads();
   if (!last) return;
-  auto finish = [&](uint32_t c, float sa, float sb) {
-    const float va = __fmul_rn(sa, fin.scale), vb = __fmul_rn(sb, fin.scale);
-    if (fin.a) storeChan(fin.a, fin.a_half, c, va);
-    if (fin.b) storeChan(fin.b, fin.b_half, c, vb);
-    if (fin.a_f32) fin.a_f32[c] = va;
-    if (fin.b_f32) fin.b_f32[c] = vb;
-    if (fin.inv_std) {
-      // plb_norm_inv_std_dev's arithmetic on the values as stored: the mean
-      // rounded to its type, the power in fp32
-      const float mean = toFloat(fromFloat<T>(va));
-      float var = vb - mean * mean;
-      if (var < 0.f) var = 0.f;
-      var = (var + fin.eps) * fin.scale_var;
-      storeChan(fin.inv_std, fin.a_half, c, 1.0f / sqrtf(var));
-    }
-    if (fin.bias) {
-      const float old = fin.bias_half ? __half2float(static_cast<const __half *>(fin.bias)[c])
-                                      : static_cast<const float *>(fin.bias)[c];
-      storeChan(fin.bias, fin.bias_half, c, old + va);
-    }
-  };
   if constexpr (V > 1) {
     if (fin.totals_fit) {
       // The slabs' rows of `pitch` columns: four columns per thread, the rows shared
@@ -411,7 +437,7 @@ chanSumsKernel(const T *__restrict__ x, const T *__restrict__ y, const T *__rest
           if constexpr (kHasA) ta += total_a[r * w.chans + c];
           if constexpr (kHasB) tb += total_b[r * w.chans + c];
         }
-        finish(c, ta, tb);
+        finishChan<T>(fin, c, ta, tb);
       }
       return;
     }
@@ -425,8 +451,100 @@ chanSumsKernel(const T *__restrict__ x, const T *__restrict__ y, const T *__rest
       if constexpr (kHasA) sa += __ldcg(partial_a + size_t(k) * w.chans + c);
       if constexpr (kHasB) sb += __ldcg(partial_b + size_t(k) * w.chans + c);
     }
-    finish(c, sa, sb);
+    finishChan<T>(fin, c, sa, sb);
   }
+}
+
+// Few rows, in two launches: a block covers 64 channels and a slab of rows (a thread two
+// neighbouring channels of every eighth row), then a warp per channel adds the slabs,
+// lane l slabs l, l + 32, ... in order, the lanes by a fixed tree.  kPairs: the two
+// channels are one load (an even count, aligned to it).
+constexpr int kColChans = 64, kColRows = 8, kColSlabs = 128;
+template <typename T, int kMode, bool kPairs>
+__global__ void __launch_bounds__(32 * kColRows)
+chanColumnsKernel(const T *__restrict__ x, const T *__restrict__ y, const T *__restrict__ centre, size_t rows,
+                  uint32_t chans, float *__restrict__ partial_a, float *__restrict__ partial_b) {
+  using Pair = typename ChanPair<T>::Type;
+  constexpr bool kHasY = kMode == kSumXYAndY;
+  __shared__ float sums[2][kColRows][kColChans];
+  pdl_launch_dependents();
+  pdl_wait();  // inputs may come from the previous kernel in the stream
+  const uint32_t c0 = blockIdx.x * kColChans + 2 * threadIdx.x;
+  float a[2] = {0.f, 0.f}, b[2] = {0.f, 0.f}, m[2] = {0.f, 0.f};
+  if constexpr (kMode == kSumCentredXX)
+    for (int j = 0; j < 2; ++j)
+      if (c0 + j < chans) m[j] = toFloat(centre[c0 + j]);
+  auto load = [&](const T *t, size_t r, float (&f)[2]) {
+    if constexpr (kPairs) {
+      ChanPair<T>::unpack(*reinterpret_cast<const Pair *>(t + r * chans + c0), f);
+    } else {
+      f[0] = toFloat(t[r * chans + c0]);
+      f[1] = c0 + 1 < chans ? toFloat(t[r * chans + c0 + 1]) : 0.f;
+    }
+  };
+  if (c0 < chans) {
+#pragma unroll 8
+    for (size_t r = blockIdx.y * size_t(kColRows) + threadIdx.y; r < rows; r += size_t(gridDim.y) * kColRows) {
+      float xv[2], yv[2] = {0.f, 0.f};
+      load(x, r, xv);
+      if constexpr (kHasY) load(y, r, yv);
+#pragma unroll
+      for (int j = 0; j < 2; ++j) addElement<T, kMode>(a[j], b[j], xv[j], yv[j], m[j]);
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    sums[0][threadIdx.y][2 * threadIdx.x + j] = a[j];
+    sums[1][threadIdx.y][2 * threadIdx.x + j] = b[j];
+  }
+  __syncthreads();
+  const uint32_t t = threadIdx.y * 32 + threadIdx.x, which = t / kColChans, col = t % kColChans;
+  const uint32_t c = blockIdx.x * kColChans + col;
+  if (which < 2 && c < chans) {
+    float total = sums[which][0][col];
+#pragma unroll
+    for (int l = 1; l < kColRows; ++l) total += sums[which][l][col];
+    (which ? partial_b : partial_a)[size_t(blockIdx.y) * chans + c] = total;
+  }
+}
+template <typename T>
+__global__ void __launch_bounds__(256)
+chanFinishKernel(const float *__restrict__ partial_a, const float *__restrict__ partial_b, uint32_t slabs,
+                 uint32_t chans, const ChanFinish fin) {
+  pdl_launch_dependents();
+  pdl_wait();  // the slabs' sums come from the previous kernel in the stream
+  const uint32_t c = blockIdx.x * 8 + threadIdx.y;
+  if (c >= chans) return;  // (whole warps leave together)
+  float a = 0.f, b = 0.f;
+  for (uint32_t k = threadIdx.x; k < slabs; k += 32) {
+    a += partial_a[size_t(k) * chans + c];
+    b += partial_b[size_t(k) * chans + c];
+  }
+#pragma unroll
+  for (int d = 16; d >= 1; d >>= 1) {
+    a += __shfl_xor_sync(0xffffffffu, a, d);
+    b += __shfl_xor_sync(0xffffffffu, b, d);
+  }
+  if (threadIdx.x == 0) finishChan<T>(fin, c, a, b);
+}
+
+template <typename T, int kMode>
+int launchChanColumns(plb_context *ctx, uint64_t rows, uint32_t chans, const T *x, const T *y, const T *centre,
+                      const ChanFinish &fin) {
+  const uint32_t cols = (chans + kColChans - 1) / kColChans;
+  // four rows per thread and more, four slabs per lane of the second kernel at most
+  const uint64_t want = std::max<uint64_t>(1, (rows + 4 * kColRows - 1) / (4 * kColRows));
+  const uint32_t slabs = uint32_t(std::min<uint64_t>(want, kColSlabs));
+  void *ws = nullptr;
+  if (int rc = scratch(ctx, kSlotChannelSums, size_t(2) * slabs * chans * sizeof(float), &ws)) return rc;
+  float *pa = static_cast<float *>(ws), *pb = pa + size_t(slabs) * chans;
+  const uintptr_t at = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y);
+  const bool pairs = chans % 2 == 0 && at % (2 * sizeof(T)) == 0;
+  if (int rc = launchPdl(ctx, pairs ? chanColumnsKernel<T, kMode, true> : chanColumnsKernel<T, kMode, false>,
+                         dim3(cols, slabs), dim3(32, kColRows), 0, x, y, centre, size_t(rows), chans, pa, pb))
+    return rc;
+  return launchPdl(ctx, chanFinishKernel<T>, dim3((chans + 7) / 8), dim3(32, 8), 0, (const float *)pa, (const float *)pb,
+                   slabs, chans, fin);
 }
 
 inline bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
@@ -462,13 +580,22 @@ template <typename T, int kMode>
 int chanSums(plb_context *ctx, const T *x, const T *y, const T *centre, uint64_t rows, uint32_t chans,
              const ChanFinish &fin) {
   constexpr int kVec = 16 / sizeof(T);
-  const bool vec = aligned16(x) && (y == nullptr || aligned16(y));
+  // (a super-row's columns are counted in 32 bits)
+  const bool vec = aligned16(x) && (y == nullptr || aligned16(y)) && uint64_t(chans) * kVec <= 0xffffffffull;
   // Slabs: one per SM, but each slab's row of sums is work for the last block.  Up
-  // to 128 columns that is nothing; wider rows take fewer slabs unless a slab has
-  // 256 KB to read and more (25088 x 256 halves: 9.4 us with 148 slabs, 8.9 with 74).
+  // to 128 columns that is nothing; wider rows take fewer slabs, down to one per four
+  // SMs, unless a slab has 256 KB to read and more (25088 x 256 halves: 9.4 us with 148
+  // slabs, 8.9 with 74).
   const uint64_t bytes = rows * chans * sizeof(T);
   const uint64_t most_slabs =
-      std::max<uint64_t>({37, uint64_t(ctx->sm_count) * 128 / std::max(chans, 1u), bytes / (256 * 1024)});
+      std::max<uint64_t>({uint64_t(ctx->sm_count) / 4, uint64_t(ctx->sm_count) * 128 / std::max(chans, 1u), bytes / (256 * 1024)});
+  // Few rows: two short launches over narrow columns, where a block's wide row of sums
+  // would be most of the work and the last block's finish most of the time (324 x 253
+  // halves 7.8 -> 3.6 us, 1058 x 351 floats 7.7 -> 4.2, 8281 x 64 halves 5.7 -> 5.5; 16641
+  // x 64 5.7 against 6.9).  Rows that are no whole vectors have several times their
+  // width to finish and take them for longer (16641 x 255 halves 10.8 -> 7.5).
+  if (rows <= (vec && chans % kVec == 0 ? 8192u : 24576u) && bytes <= (uint64_t(16) << 20))
+    return launchChanColumns<T, kMode>(ctx, rows, chans, x, y, centre, fin);
   if (!vec) return launchChanSums<T, kMode, 1, 512>(ctx, rows, chans, most_slabs, x, y, centre, fin);
   // Twice the warps keep the loads of a long slab going while a part of them adds (64
   // images of 56x56, 256 channels, 103 MB: 20.4 us, with 512 threads 22.0); elsewhere they only
@@ -495,31 +622,66 @@ struct ChanMapArgs {
   const T *p, *q, *r, *s;    // per channel
   const float *pf, *qf;      // the same in fp32 (instead of p, q)
   T *out, *out2;             // out may be x
+  int whole;                 // (set by chanMap) a vector's operands are whole vectors of p, q, r, s too
 };
 
 constexpr int kChanMapThreads = 256;
 
-template <typename T, int kMode, int V>
+// kRows: super-rows a thread has in flight.
+template <typename T, int kMode, int V, int kRows>
 __global__ void __launch_bounds__(kChanMapThreads)
 chanMapKernel(const ChanMapArgs<T> g, const ChanWalk w) {
   using Vec = ChanVec<T, V>;
   using Raw = typename Vec::Raw;
   constexpr bool kHasY = kMode == kStatsGrad;
-  constexpr int kUnroll = kHasY ? 2 : 4;
+  constexpr int kUnroll = kRows;
   pdl_launch_dependents();
   const uint32_t lanes = 1u << w.vec_lanes_log2, row_lanes = kChanMapThreads >> w.vec_lanes_log2;
   const uint32_t vx = threadIdx.x & (lanes - 1), ry = threadIdx.x >> w.vec_lanes_log2;
   const uint32_t vec = blockIdx.x * lanes + vx;
   pdl_wait();  // inputs may come from the previous kernel in the stream
   if (vec >= w.vecs) return;
-  float p[V], q[V], r[V], s[V];
+  const size_t pitch = size_t(w.vecs) * V, step = size_t(gridDim.y) * row_lanes;
+  size_t row0 = size_t(blockIdx.y) * row_lanes + ry;
+  Raw rx[kUnroll];
+  [[maybe_unused]] Raw rv[kUnroll];
+  auto fetch = [&]() {
 #pragma unroll
-  for (int j = 0; j < V; ++j) {
-    const uint32_t c = (vec * V + j) % w.chans;
-    p[j] = g.pf ? g.pf[c] : toFloat(g.p[c]);
-    if constexpr (kMode != kScale && kMode != kAddChan) q[j] = g.qf ? g.qf[c] : toFloat(g.q[c]);
-    if constexpr (kMode == kStatsGrad || kMode == kNormalise) r[j] = toFloat(g.r[c]);
-    if constexpr (kMode == kNormalise) s[j] = toFloat(g.s[c]);
+    for (int u = 0; u < kUnroll; ++u) {
+      const size_t row = row0 + u * step;
+      if (row < w.full) {
+        rx[u] = *reinterpret_cast<const Raw *>(g.x + row * pitch + size_t(vec) * V);
+        if constexpr (kHasY) rv[u] = *reinterpret_cast<const Raw *>(g.y + row * pitch + size_t(vec) * V);
+      }
+    }
+  };
+  fetch();  // (ahead of the operands, so that both are in flight)
+  float p[V], q[V], r[V], s[V];
+  constexpr bool kHasQ = kMode != kScale && kMode != kAddChan, kHasR = kMode == kStatsGrad || kMode == kNormalise;
+  if (g.whole) {
+    auto load = [&](const T *src, float (&f)[V]) { Vec::unpack(*reinterpret_cast<const Raw *>(src + size_t(vec) * V), f); };
+    if (kMode == kStatsGrad && g.pf) {
+#pragma unroll
+      for (int j = 0; j < V; ++j) {
+        p[j] = g.pf[size_t(vec) * V + j];
+        q[j] = g.qf[size_t(vec) * V + j];
+      }
+    } else {
+      load(g.p, p);
+      if constexpr (kHasQ) load(g.q, q);
+    }
+    if constexpr (kHasR) load(g.r, r);
+    if constexpr (kMode == kNormalise) load(g.s, s);
+  } else {
+    uint32_t c = uint32_t(size_t(vec) * V % w.chans);
+#pragma unroll
+    for (int j = 0; j < V; ++j) {
+      p[j] = g.pf ? g.pf[c] : toFloat(g.p[c]);
+      if constexpr (kHasQ) q[j] = g.qf ? g.qf[c] : toFloat(g.q[c]);
+      if constexpr (kHasR) r[j] = toFloat(g.r[c]);
+      if constexpr (kMode == kNormalise) s[j] = toFloat(g.s[c]);
+      if (++c == w.chans) c = 0;
+    }
   }
   auto map = [&](float x, float y, int j, float &white) -> float {
     if constexpr (kMode == kWhiten) {
@@ -538,18 +700,7 @@ chanMapKernel(const ChanMapArgs<T> g, const ChanWalk w) {
       return x + p[j];
     }
   };
-  const size_t pitch = size_t(w.vecs) * V, step = size_t(gridDim.y) * row_lanes;
-  for (size_t row0 = size_t(blockIdx.y) * row_lanes + ry; row0 < w.full; row0 += kUnroll * step) {
-    Raw rx[kUnroll];
-    [[maybe_unused]] Raw rv[kUnroll];
-#pragma unroll
-    for (int u = 0; u < kUnroll; ++u) {
-      const size_t row = row0 + u * step;
-      if (row < w.full) {
-        rx[u] = *reinterpret_cast<const Raw *>(g.x + row * pitch + size_t(vec) * V);
-        if constexpr (kHasY) rv[u] = *reinterpret_cast<const Raw *>(g.y + row * pitch + size_t(vec) * V);
-      }
-    }
+  for (; row0 < w.full; row0 += kUnroll * step, fetch()) {
 #pragma unroll
     for (int u = 0; u < kUnroll; ++u) {
       const size_t row = row0 + u * step;
@@ -581,15 +732,25 @@ chanMapKernel(const ChanMapArgs<T> g, const ChanWalk w) {
 }
 
 template <typename T, int kMode>
-int chanMap(plb_context *ctx, const ChanMapArgs<T> &g, uint64_t rows, uint32_t chans) {
+int chanMap(plb_context *ctx, ChanMapArgs<T> g, uint64_t rows, uint32_t chans) {
   if (rows == 0 || chans == 0) return PLB_OK;
   constexpr uint32_t kVec = 16 / sizeof(T);
-  const bool vec = aligned16(g.x) && aligned16(g.out) && (g.y == nullptr || aligned16(g.y)) &&
+  const bool vec = uint64_t(chans) * kVec <= 0xffffffffull && aligned16(g.x) && aligned16(g.out) && (g.y == nullptr || aligned16(g.y)) &&
                    (g.out2 == nullptr || aligned16(g.out2));
+  // Blocks that all are resident and walk, but a large tensor takes as many as fit: what
+  // counts there is loads in flight (whitening and scaling 100352 x 1024 halves: 57.1 us
+  // with 4 blocks per SM, 52.2 with 16; 3136 x 1024: 5.3 with 4, 7.7 with 16).
+  const uint32_t per_sm = rows * chans * sizeof(T) >= (uint64_t(32) << 20) ? 16 : 4;
   dim3 grid;
-  const ChanWalk w = chanWalk(ctx, rows, chans, vec ? kVec : 1, kChanMapThreads, 4, 1, 0, &grid);
-  if (vec) return launchPdl(ctx, chanMapKernel<T, kMode, int(kVec)>, grid, dim3(kChanMapThreads), 0, g, w);
-  return launchPdl(ctx, chanMapKernel<T, kMode, 1>, grid, dim3(kChanMapThreads), 0, g, w);
+  const ChanWalk w = chanWalk(ctx, rows, chans, vec ? kVec : 1, kChanMapThreads, per_sm, 1, 0, &grid);
+  g.whole = vec && w.fold == 1 && aligned16(g.p) && aligned16(g.q) && aligned16(g.r) && aligned16(g.s);
+  // Where a thread has one super-row the code for several only has to be fetched
+  // (whitening and scaling 4225 x 256 halves: 3.8 us).
+  constexpr int kMany = kMode == kStatsGrad ? 2 : 4;
+  const bool one = w.full <= uint64_t(grid.y) * (kChanMapThreads >> w.vec_lanes_log2);
+  if (!vec) return launchPdl(ctx, chanMapKernel<T, kMode, 1, kMany>, grid, dim3(kChanMapThreads), 0, g, w);
+  return launchPdl(ctx, one ? chanMapKernel<T, kMode, int(kVec), 1> : chanMapKernel<T, kMode, int(kVec), kMany>, grid,
+                   dim3(kChanMapThreads), 0, g, w);
 }
 
 }  // namespace plb

@@ -48,6 +48,39 @@ def test_channel_sums_and_maps(gpu_ctx, chans, rows, dtype):
         np.testing.assert_array_equal(dy.cpu().numpy().reshape(rows, chans), y + b)
 
 
+@pytest.mark.parametrize("dtype", ["half", "float"])
+@pytest.mark.parametrize("rows", [8192, 8193, 24576, 24577])
+@pytest.mark.parametrize("chans", [1, 7, 8, 64, 100, 257])
+def test_sums_and_maps_where_their_route_changes(gpu_ctx, chans, rows, dtype):
+    """One or two launches for the sums (by rows, for whole vectors and others), one or several
+    rows per thread for the maps.  |sum| <= 24577 * 16 < 2^24."""
+    import torch
+    ctx = T.context()
+    t_t, plb_t = (torch.float16, capi.HALF) if dtype == "half" else (torch.float32, capi.FLOAT)
+    g = torch.Generator(device="cuda").manual_seed(chans + rows)
+    ints = lambda *s: torch.randint(-4, 5, s, device="cuda", generator=g).to(t_t)
+    x, y, a, b = ints(rows, chans), ints(rows, chans), ints(chans), ints(chans)
+    bias, power = torch.full((chans,), 3.0, device="cuda"), torch.empty(chans, device="cuda")
+    ga, be = torch.empty(chans, device="cuda"), torch.empty(chans, device="cuda")
+    out, white, norm, grad = (torch.empty_like(x) for _ in range(4))
+    one = torch.ones_like(a)
+    torch.cuda.synchronize()
+    ctx.conv_bias_update(plb_t, x, rows, chans, capi.FLOAT, bias, 0.5)
+    ctx.norm_moments(plb_t, x, rows, chans, 1.0, None, torch.empty_like(a), power)
+    ctx.norm_param_gradients(plb_t, x, y, rows, chans, 1.0, None, None, ga, be)
+    ctx.norm_scale_shift(plb_t, x, a, b, rows, chans, out)
+    ctx.norm_normalise(plb_t, x, a, one, b, one, rows, chans, white, norm)
+    ctx.norm_statistics_gradients(plb_t, x, y, one, rows, chans, grad, var_delta=a, mean_delta=b)
+    ctx.synchronize()
+    x64, y64, a64, b64 = x.double(), y.double(), a.double(), b.double()
+    assert torch.equal(bias.double(), 3.0 + 0.5 * x64.sum(0))
+    assert torch.equal(power.double(), (x64 * x64).sum(0))
+    assert torch.equal(ga.double(), (x64 * y64).sum(0)) and torch.equal(be.double(), y64.sum(0))
+    assert torch.equal(out.double(), x64 * a64 + b64)
+    assert torch.equal(white.double(), x64 - a64) and torch.equal(norm.double(), (x64 - a64) * b64 + 1)
+    assert torch.equal(grad.double(), y64 + x64 * a64 + b64)
+
+
 @pytest.mark.parametrize("count", [1, 7, 8, 9, 2047, 2048 * 8 * 148 + 13])
 @pytest.mark.parametrize("dtype", ["half", "float"])
 def test_scaled_add_and_cast_tails(gpu_ctx, dtype, count):
