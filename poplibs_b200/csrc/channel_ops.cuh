@@ -18,6 +18,7 @@
 #include <cuda_fp16.h>
 
 #include <algorithm>
+#include <atomic>
 
 #include "runtime.h"
 #include "sm100_prims.cuh"
@@ -565,8 +566,8 @@ int launchChanSums(plb_context *ctx, uint64_t rows, uint32_t chans, uint64_t mos
   const size_t finish = 8 * (kThreads + kThreads / 2) * sizeof(float) + 2 * pitch * sizeof(float);
   fin.totals_fit = V > 1 && finish <= kMost ? 1 : 0;
   const size_t smem = std::max(2 * (kThreads / 32) * (cols + 1) * sizeof(float), fin.totals_fit ? finish : size_t(0));
-  static bool configured[64] = {};
-  bool &done = configured[ctx->device & 63];
+  static std::atomic<bool> configured[64] = {};  // (contexts may live on several threads)
+  std::atomic<bool> &done = configured[ctx->device & 63];
   if (!done) {
     PLB_CUDA(cudaFuncSetAttribute(chanSumsKernel<T, kMode, V, kThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   int(kMost)));

@@ -2,6 +2,8 @@
 // column-tile width are compiled in a file of their own (igemm_bn*.cu).
 #pragma once
 
+#include <atomic>
+
 #include "igemm_sm100.cuh"
 #include "launch_shape.h"
 #include "runtime.h"
@@ -29,8 +31,9 @@ int launchInstance(plb_context *ctx, const CUtensorMap &ta, const CUtensorMap &t
     return fail(PLB_ERR_INVALID_OPTION, "a CTA pair needs tile_n >= 128 for a row-major B");
   } else {
     using S = IgemmSmem<BN, kResB, k2Cta>;
-    static bool configured[64] = {};
-    static int max_clusters[64] = {};
+    // (contexts may live on several threads; each would store the same values)
+    static std::atomic<bool> configured[64] = {};
+    static std::atomic<int> max_clusters[64] = {};
     auto kernel = igemm_kernel<BN, kFp8, kAMn, kBMn, kResB, kHalo, k2Cta, kGroups>;
     const int dev = ctx->device & 63;
     if (!configured[dev]) {
