@@ -606,7 +606,7 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
           uint64_t(uint32_t(kResB ? args.taps_w * args.k_chunks : 1) * (S::kBBytes >> 4));
       int stage = 0;
       uint32_t phase = 0;
-      uint32_t acc_phase[2] = {0, 0};
+      uint32_t acc_phases = 0;  // a bit per accumulator (an array would lie in local memory)
       int local_tile = 0;
       bool ok = true;
       [[maybe_unused]] int trace_slot = 0;
@@ -631,12 +631,12 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
         const int acc = local_tile & 1;
         if (mi == 0) { PLB_TRACE_STAMP(1, trace_slot); ++trace_slot; }
         // wait for the epilogue to have drained this accumulator
-        if (!mbar_wait(tmem_empty_bar(acc), acc_phase[acc] ^ 1u, abort_flag)) {
+        if (!mbar_wait(tmem_empty_bar(acc), ((acc_phases >> acc) & 1u) ^ 1u, abort_flag)) {
           atomicCAS(args.status, kStatusOk, kStatusMmaTimeout);
           ok = false;
           break;
         }
-        acc_phase[acc] ^= 1u;
+        acc_phases ^= 1u << acc;
         tc_fence_after_sync();
         if (mi == 0) { PLB_TRACE_STAMP(1, trace_slot); ++trace_slot; }
         const uint32_t d_tmem = tmem_base + acc * BN;
@@ -748,6 +748,7 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
     // fp32 rows fill the 128-byte staged row with 32 columns: the `half == 1`
     // warps then leave the work to their partners
     const bool idle = out_f32 && args.split_k == 1 && half == 1;
+    const bool lean = tma_store && !out_f32 && args.bias == nullptr && args.addend == nullptr && args.nonfinite == nullptr;
     const bool stamp = threadIdx.x == 128;
     const int acc = group;
     int local_tile = group;
@@ -824,21 +825,93 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
         continue;
       }
 
-      // The accumulator in blocks of 32 columns: scale / add, then
+      // this warp's staged rows of 32 columns from `col` on -> output
+      auto store_staged = [&](uint32_t src, int col) {
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+          // a box that starts outside the tensor has nothing to write
+          if (box_ok) {
+            const int c2 = args.h_outer ? n0 + qn : h0 + qh, c3 = args.h_outer ? h0 + qh : n0 + qn;
+            if (kGroups)
+              tma_store_5d(&tm_out, src, col, cgroup, w0 + qw, c2, c3);
+            else
+              tma_store_4d(&tm_out, src, col, w0 + qw, c2, c3);
+          }
+          tma_store_commit();
+        }
+      };
+      auto note_nonfinite = [&](const uint32_t (&v)[32], int valid) {
+        // (rows beyond the output hold whatever the stage's shared memory held before)
+        if (args.nonfinite == nullptr || !row_ok) return;
+        uint32_t largest = 0u;
+#pragma unroll
+        for (int j = 0; j < 32; ++j)
+          if (j < valid) largest = max(largest, v[j] & 0x7fffffffu);
+        if (largest >= 0x7f800000u) *args.nonfinite = 1;
+      };
+
+      // The accumulator in blocks of 32 columns, in one of three loops:
       //  - the fp32 sums of a K split: vector stores of each lane's own row (the
-      //    scratch rows are padded to whole blocks),
-      //  - else the block is staged in swizzled shared memory (half: each warp its
-      //    own 32 rows x 64 bytes, so that no barrier between warps lies on the
-      //    chain load -> convert -> stage -> store; fp32: 32 rows x 128 bytes) and
-      //    leaves with a tensor store, or, where the output cannot be described to
-      //    TMA, row by row: lane after lane writing its own row would touch a
-      //    sector per element, consecutive lanes take consecutive columns instead.
-      // One loop for all of them: a short kernel's instructions come from L2.
+      //    scratch rows are padded to whole blocks);
+      //  - a half result that only has to be scaled and stored (products without C,
+      //    input gradients);
+      //  - all else: scale / add, then the block is staged in swizzled shared memory
+      //    (half: each warp its own 32 rows x 64 bytes, so that no barrier between
+      //    warps lies on the chain load -> convert -> stage -> store; fp32: 32 rows x
+      //    128 bytes) and leaves with a tensor store, or, where the output cannot be
+      //    described to TMA, row by row: lane after lane writing its own row would
+      //    touch a sector per element, consecutive lanes take consecutive columns
+      //    instead.
+      // As one loop for all of them it needed more than 96 registers: what was spilled
+      // (420 sectors a CTA) and the branches around what a product does not have cost
+      // 512 x 512 x 512 0.3 of 4.6 us.
       const uint32_t wbuf = staging_base + uint32_t(warp - 4) * 2048u;
       const uint32_t wrow = wbuf + uint32_t(lane) * 64u, sw = (uint32_t(lane) >> 1) & 3u;
       const bool whole_rows = out_f32 && args.split_k == 1;  // 128-byte rows, the half == 0 warps only
       const int c_first = whole_rows ? 0 : half * 32, c_step = whole_rows ? 32 : 64;
       if (c_first >= cols_end) release_accumulator();
+      if (args.split_k > 1) {
+        // (this split's slice of the partial sums, whole 32-byte sectors per lane)
+        float *const dst = static_cast<float *>(args.out) + split * args.split_stride + out_off + col_base;
+#pragma unroll 1
+        for (int c = c_first; c < cols_end; c += 64) {
+          uint32_t v[32];
+          __syncwarp();
+          tmem_ld_32x32(t_addr + c, v);
+          tmem_ld_wait_for(v);
+          if (c + 64 >= cols_end) release_accumulator();
+          note_nonfinite(v, min(32, args.n_total - col_base - c));
+          if (row_ok)
+#pragma unroll
+            for (int j = 0; j < 32; j += 8)
+              st_global_v8(dst + c + j, v[j], v[j + 1], v[j + 2], v[j + 3], v[j + 4], v[j + 5], v[j + 6], v[j + 7]);
+        }
+        continue;
+      }
+      if (lean) {
+#pragma unroll 1
+        for (int c = c_first; c < cols_end; c += 64) {
+          uint32_t v[32];
+          __syncwarp();
+          tmem_ld_32x32(t_addr + c, v);
+          tmem_ld_wait_for(v);
+          if (c + 64 >= cols_end) release_accumulator();
+          if (lane == 0) tma_store_wait_read<0>();  // the previous store has read the buffer
+          __syncwarp();
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            float f[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) f[i] = __uint_as_float(v[8 * j + i]) * args.alpha;
+            uint32_t pk[4];
+            pack_half8(f, pk);
+            st_shared_v4(wrow + ((uint32_t(j) ^ sw) << 4), pk[0], pk[1], pk[2], pk[3]);
+          }
+          store_staged(wbuf, col_base + c);
+        }
+        continue;
+      }
 #pragma unroll 1
       for (int c = c_first; c < cols_end; c += c_step) {
         uint32_t v[32];
@@ -849,14 +922,7 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
         if (c + c_step >= cols_end) release_accumulator();
         const int col0 = col_base + c;
         const int valid = min(32, args.n_total - col0);
-        // (rows beyond the output hold whatever the stage's shared memory held before)
-        if (args.nonfinite != nullptr && row_ok) {
-          uint32_t largest = 0u;
-#pragma unroll
-          for (int j = 0; j < 32; ++j)
-            if (j < valid) largest = max(largest, v[j] & 0x7fffffffu);
-          if (largest >= 0x7f800000u) *args.nonfinite = 1;
-        }
+        note_nonfinite(v, valid);
         if (args.alpha != 1.f) {
 #pragma unroll
           for (int j = 0; j < 32; ++j) f[j] = __uint_as_float(v[j]) * args.alpha;
@@ -897,18 +963,6 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
               if (j < valid) f[j] += args.beta * __half2float(src[j]);
           }
         }
-        if (args.split_k > 1) {
-          // (this split's slice of the partial sums, whole 32-byte sectors per lane)
-          if (row_ok) {
-            float *dst = static_cast<float *>(args.out) + split * args.split_stride + out_off + col0;
-#pragma unroll
-            for (int j = 0; j < 32; j += 8)
-              st_global_v8(dst + j, __float_as_uint(f[j]), __float_as_uint(f[j + 1]), __float_as_uint(f[j + 2]),
-                           __float_as_uint(f[j + 3]), __float_as_uint(f[j + 4]), __float_as_uint(f[j + 5]),
-                           __float_as_uint(f[j + 6]), __float_as_uint(f[j + 7]));
-          }
-          continue;
-        }
         if (tma_store && lane == 0) tma_store_wait_read<0>();  // the previous store has read the buffer
         __syncwarp();
         if (whole_rows) {
@@ -928,20 +982,7 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
           }
         }
         if (tma_store) {
-          fence_proxy_async_smem();
-          __syncwarp();
-          if (lane == 0) {
-            // a box that starts outside the tensor has nothing to write
-            if (box_ok) {
-              const uint32_t src = whole_rows ? buf : wbuf;
-              const int c2 = args.h_outer ? n0 + qn : h0 + qh, c3 = args.h_outer ? h0 + qh : n0 + qn;
-              if (kGroups)
-                tma_store_5d(&tm_out, src, col0, cgroup, w0 + qw, c2, c3);
-              else
-                tma_store_4d(&tm_out, src, col0, w0 + qw, c2, c3);
-            }
-            tma_store_commit();
-          }
+          store_staged(whole_rows ? buf : wbuf, col0);
           continue;
         }
         __syncwarp();
