@@ -122,6 +122,9 @@ struct IgemmArgs {
   FastDiv fd_split;
   long long split_stride;
   int dual_issue;  // two MMA-issuing threads take alternate tiles
+  // Steps of a CTA's first unit that idle warps issue, and how many of its steps they
+  // pull towards L2 before (streamed weights; the rule is in launchIgemm).
+  int first_loads, first_prefetches;
   int chain;       // IgemmChain
   uint32_t idesc_formats;  // operand format bits of the instruction descriptor (8-bit operands: 1 = E5M2)
   // ---- epilogue ---------------------------------------------------------------
@@ -491,6 +494,7 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
     unit_coords(first_unit, f_tile, f_group, f_split, f_begin, f_end);
     first_steps = min(f_end - f_begin, kStages);
   }
+  const int first_loads = min(first_steps, args.first_loads), first_prefetches = min(first_steps, args.first_prefetches);
   // Step f_begin + i of the first unit towards L2 while the predecessor kernel may
   // still be running, and with `load`, once it has finished, into stage i.
   auto first_step = [&](int i, bool load) {
@@ -500,7 +504,7 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
     step_coords(f_begin + i, r, s, kc);
     const uint32_t dst = smem_base + i * stage_bytes, full = lead_bar(full_bar(i));
     const int w_base = w0 * args.stride_w - args.pad_w, h_base = h0 * args.stride_h - args.pad_h;
-    issue_step(true, dst, full, f_group, r, s, kc, w_base, h_base, n0, n_idx * BN);
+    if (kResB || i < first_prefetches) issue_step(true, dst, full, f_group, r, s, kc, w_base, h_base, n0, n_idx * BN);
     if (!load) return;
     wait_predecessor();
     if (leader)
@@ -537,7 +541,7 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
         if (it_begin != 0) step_coords(it_begin, r, s, kc);
         for (int it = it_begin; it < it_end; ++it) {
           // (the first unit's first steps are on their way already)
-          const bool issued = !kResB && unit == first_unit && it - it_begin < first_steps;
+          const bool issued = !kResB && unit == first_unit && it - it_begin < first_loads;
           if (turn == me && issued) {
             stage += P;
             if (stage >= kStages) {
@@ -779,9 +783,7 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
       }
       __syncwarp();
     } else {
-      if (lane == 0 && warp - 4 < first_steps) {
-        first_step(warp - 4, true);
-      }
+      if (lane == 0 && warp - 4 < max(first_loads, first_prefetches)) first_step(warp - 4, warp - 4 < first_loads);
       __syncwarp();
     }
     wait_predecessor();
@@ -852,66 +854,27 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
       };
 
       // The accumulator in blocks of 32 columns, in one of three loops:
-      //  - the fp32 sums of a K split: vector stores of each lane's own row (the
-      //    scratch rows are padded to whole blocks);
-      //  - a half result that only has to be scaled and stored (products without C,
-      //    input gradients);
-      //  - all else: scale / add, then the block is staged in swizzled shared memory
-      //    (half: each warp its own 32 rows x 64 bytes, so that no barrier between
+      //  - the general one: scale / add, then the block is staged in swizzled shared
+      //    memory (half: each warp its own 32 rows x 64 bytes, so that no barrier between
       //    warps lies on the chain load -> convert -> stage -> store; fp32: 32 rows x
       //    128 bytes) and leaves with a tensor store, or, where the output cannot be
       //    described to TMA, row by row: lane after lane writing its own row would
       //    touch a sector per element, consecutive lanes take consecutive columns
-      //    instead.
+      //    instead;
+      //  - the fp32 sums of a K split: vector stores of each lane's own row (the
+      //    scratch rows are padded to whole blocks);
+      //  - a half result that only has to be scaled and stored (products without C,
+      //    input gradients).
       // As one loop for all of them it needed more than 96 registers: what was spilled
       // (420 sectors a CTA) and the branches around what a product does not have cost
-      // 512 x 512 x 512 0.3 of 4.6 us.
+      // 512 x 512 x 512 0.3 of 4.6 us.  The general one comes first, with nothing of the
+      // others between its instructions (7x7 layer on 64 images 49.4 us behind them, 48.8).
       const uint32_t wbuf = staging_base + uint32_t(warp - 4) * 2048u;
       const uint32_t wrow = wbuf + uint32_t(lane) * 64u, sw = (uint32_t(lane) >> 1) & 3u;
       const bool whole_rows = out_f32 && args.split_k == 1;  // 128-byte rows, the half == 0 warps only
       const int c_first = whole_rows ? 0 : half * 32, c_step = whole_rows ? 32 : 64;
       if (c_first >= cols_end) release_accumulator();
-      if (args.split_k > 1) {
-        // (this split's slice of the partial sums, whole 32-byte sectors per lane)
-        float *const dst = static_cast<float *>(args.out) + split * args.split_stride + out_off + col_base;
-#pragma unroll 1
-        for (int c = c_first; c < cols_end; c += 64) {
-          uint32_t v[32];
-          __syncwarp();
-          tmem_ld_32x32(t_addr + c, v);
-          tmem_ld_wait_for(v);
-          if (c + 64 >= cols_end) release_accumulator();
-          note_nonfinite(v, min(32, args.n_total - col_base - c));
-          if (row_ok)
-#pragma unroll
-            for (int j = 0; j < 32; j += 8)
-              st_global_v8(dst + c + j, v[j], v[j + 1], v[j + 2], v[j + 3], v[j + 4], v[j + 5], v[j + 6], v[j + 7]);
-        }
-        continue;
-      }
-      if (lean) {
-#pragma unroll 1
-        for (int c = c_first; c < cols_end; c += 64) {
-          uint32_t v[32];
-          __syncwarp();
-          tmem_ld_32x32(t_addr + c, v);
-          tmem_ld_wait_for(v);
-          if (c + 64 >= cols_end) release_accumulator();
-          if (lane == 0) tma_store_wait_read<0>();  // the previous store has read the buffer
-          __syncwarp();
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            float f[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) f[i] = __uint_as_float(v[8 * j + i]) * args.alpha;
-            uint32_t pk[4];
-            pack_half8(f, pk);
-            st_shared_v4(wrow + ((uint32_t(j) ^ sw) << 4), pk[0], pk[1], pk[2], pk[3]);
-          }
-          store_staged(wbuf, col_base + c);
-        }
-        continue;
-      }
+      if (!lean && args.split_k == 1) {
 #pragma unroll 1
       for (int c = c_first; c < cols_end; c += c_step) {
         uint32_t v[32];
@@ -1023,6 +986,49 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
           }
         }
         __syncwarp();
+      }
+        continue;
+      }
+      if (args.split_k > 1) {
+        // (this split's slice of the partial sums, whole 32-byte sectors per lane)
+        float *const dst = static_cast<float *>(args.out) + split * args.split_stride + out_off + col_base;
+#pragma unroll 1
+        for (int c = c_first; c < cols_end; c += 64) {
+          uint32_t v[32];
+          __syncwarp();
+          tmem_ld_32x32(t_addr + c, v);
+          tmem_ld_wait_for(v);
+          if (c + 64 >= cols_end) release_accumulator();
+          note_nonfinite(v, min(32, args.n_total - col_base - c));
+          if (row_ok)
+#pragma unroll
+            for (int j = 0; j < 32; j += 8)
+              st_global_v8(dst + c + j, v[j], v[j + 1], v[j + 2], v[j + 3], v[j + 4], v[j + 5], v[j + 6], v[j + 7]);
+        }
+        continue;
+      }
+      {
+#pragma unroll 1
+        for (int c = c_first; c < cols_end; c += 64) {
+          uint32_t v[32];
+          __syncwarp();
+          tmem_ld_32x32(t_addr + c, v);
+          tmem_ld_wait_for(v);
+          if (c + 64 >= cols_end) release_accumulator();
+          if (lane == 0) tma_store_wait_read<0>();  // the previous store has read the buffer
+          __syncwarp();
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            float f[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) f[i] = __uint_as_float(v[8 * j + i]) * args.alpha;
+            uint32_t pk[4];
+            pack_half8(f, pk);
+            st_shared_v4(wrow + ((uint32_t(j) ^ sw) << 4), pk[0], pk[1], pk[2], pk[3]);
+          }
+          store_staged(wbuf, col_base + c);
+        }
+        continue;
       }
       if (stamp) PLB_TRACE_STAMP(2, local_tile * 4 + 2);
       if (stamp) PLB_TRACE_STAMP(2, local_tile * 4 + 3);
