@@ -9,6 +9,7 @@
 #include <vector>
 
 #include "conv_geometry.h"
+#include "direct.h"
 #include "grouped.h"
 #include "runtime.h"
 #include "igemm_sm100.cuh"
@@ -510,6 +511,17 @@ Copies planCopies(const plb_matmul_desc &d, const void **a, long long *lda, bool
   return c;
 }
 
+// Whether the implicit-GEMM kernel can only read a copy of an operand.
+bool matmulCopies(const plb_matmul_desc &d, const void *a, const void *b) {
+  const Ld ld = leadingDims(d);
+  const size_t es = dtypeBytes(d.input_type);
+  auto fits = [&](const void *base, long long pitch) {
+    return (reinterpret_cast<uintptr_t>(base) & 15) == 0 && (size_t(pitch) * es) % 16 == 0;
+  };
+  return d.input_type == PLB_FLOAT || (d.input_type == PLB_QUARTER && (d.transpose_a || !d.transpose_b)) ||
+         !fits(a, ld.a) || !fits(b, ld.b);
+}
+
 // The product that is contracted: float operands as three bfloat16 terms per product.
 plb_matmul_desc contractionDesc(const plb_matmul_desc &d) {
   plb_matmul_desc q = d;
@@ -731,6 +743,9 @@ int plb_matmul_plan(const plb_matmul_desc *desc, plb_plan *plan) {
       gemmProblem(contractionDesc(*desc), nullptr, lda, a_is_km, nullptr, ldb, b_is_nk, nullptr, nullptr, ld.c);
   if (int rc = planIgemm(p, 148, plan)) return rc;
   plan->workspace_bytes += transposed + copies.bytes;
+  const IgemmProblem direct = gemmProblem(*desc, nullptr, ld.a, desc->transpose_a != 0, nullptr, ld.b, desc->transpose_b != 0,
+                                          nullptr, nullptr, ld.c);
+  if (directSuits(148, direct, desc->input_type, matmulCopies(*desc, nullptr, nullptr))) plan->kernel = 3;
   return PLB_OK;
 }
 
@@ -759,6 +774,18 @@ int plb_matmul(plb_context *ctx, const plb_matmul_desc *desc, const void *d_a, c
     }
     return PLB_OK;
   }
+  if (d.input_type == PLB_FLOAT && (ld.a < (long long)(d.transpose_a ? d.m : d.k) || ld.b < (long long)(d.transpose_b ? d.k : d.n)))
+    return fail(PLB_ERR_INVALID_PARAMS, "leading dimension shorter than a row");
+  if (d.input_type == PLB_QUARTER && d.transpose_a && ld.a != (long long)d.m)
+    return fail(PLB_ERR_UNSUPPORTED, "transposed quarter A must be densely packed");
+  if (d.input_type == PLB_QUARTER && !d.transpose_b && ld.b != (long long)d.n)
+    return fail(PLB_ERR_UNSUPPORTED, "quarter B in [k][n] layout must be densely packed");
+  {
+    // small products, and moderate ones that would need a copy, from the operands as they are
+    IgemmProblem p = gemmProblem(d, d_a, ld.a, d.transpose_a != 0, d_b, ld.b, d.transpose_b != 0, d_c, d_d, ld.c);
+    p.plan_flags = ctx->plan_flags;
+    if (directSuits(ctx->sm_count, p, d.input_type, matmulCopies(d, d_a, d_b))) return launchDirect(ctx, p, d.input_type);
+  }
   // Operand layouts the kernel takes directly: A as [m][k], B as [n][k], or (not
   // 8-bit) A as [k][m] and B as [k][n].  8-bit operands stored the other way go
   // through a transpose into scratch.
@@ -773,16 +800,12 @@ int plb_matmul(plb_context *ctx, const plb_matmul_desc *desc, const void *d_a, c
     void *ws = nullptr;
     if (int rc = scratch(ctx, kSlotOperands, a_bytes + b_bytes, &ws)) return rc;
     if (a_is_km) {
-      if (ld.a != (long long)d.m)
-        return fail(PLB_ERR_UNSUPPORTED, "transposed quarter A must be densely packed");
       if (int rc = transposeBatch(ctx, 1, d.groups, d.k, d.m, d_a, ws, pitch)) return rc;
       a = ws;
       lda = (long long)pitch;
       a_is_km = false;
     }
     if (!b_is_nk) {
-      if (ld.b != (long long)d.n)
-        return fail(PLB_ERR_UNSUPPORTED, "quarter B in [k][n] layout must be densely packed");
       uint8_t *bt = static_cast<uint8_t *>(ws) + a_bytes;
       if (int rc = transposeBatch(ctx, 1, d.groups, d.k, d.n, d_b, bt, pitch)) return rc;
       b = bt;
@@ -794,8 +817,6 @@ int plb_matmul(plb_context *ctx, const plb_matmul_desc *desc, const void *d_a, c
   // 16 bytes: n % 8 != 0, odd leading dimensions) are copied once into scratch
   // with the pitch rounded up, float operands are split into their bfloat16
   // pieces, both operands in one launch.  The output needs no such copy.
-  if (d.input_type == PLB_FLOAT && (lda < (long long)(a_is_km ? d.m : d.k) || ldb < (long long)(b_is_nk ? d.k : d.n)))
-    return fail(PLB_ERR_INVALID_PARAMS, "leading dimension shorter than a row");
   Copies copies = planCopies(d, &a, &lda, a_is_km, &b, &ldb, b_is_nk);
   if (int rc = runCopies(ctx, copies)) return rc;
   const plb_matmul_desc q = contractionDesc(d);

@@ -1,0 +1,13 @@
+// Matrix products that read their operands where they lie (direct.cuh, direct.cu).
+#pragma once
+
+#include "runtime.h"
+
+namespace plb {
+
+// The product as gemmProblem describes it, on the caller's operands of element type
+// `type`.  `copied`: the implicit-GEMM kernel could only read a copy of an operand.
+bool directSuits(int sm_count, const IgemmProblem &p, int type, bool copied);
+int launchDirect(plb_context *ctx, const IgemmProblem &p, int type);
+
+}  // namespace plb
