@@ -108,20 +108,34 @@ int planIgemm(const IgemmProblem &p, int sm_count, plb_plan *plan) {
   // CTA pairs: two M tiles share one 256-row MMA, each CTA holding half of the
   // weight tile.  Needs two M tiles and, for a row-major B, a whole 64-column
   // block per CTA.
-  // Worth it when every CTA pair gets several tile pairs and a tile's K loop is
-  // long: the two SMs advance in lockstep per tile, which costs more than the
-  // halved weight traffic saves on short tiles and on grids of a few tiles.
-  // With 256-column tiles the weight tile is two thirds of a stage's bytes and
-  // half the K length already pays (1x1 stride-2 layer 256 -> 512: 71 -> 67 us).
+  // Worth it, with a K loop that is not short, when every CTA pair gets several tile
+  // pairs: the two SMs advance in lockstep per tile, which costs short tiles more than the
+  // halved weight traffic saves.  With 256-column tiles the weight tile is two thirds of a
+  // stage's bytes and half the K length already pays (1x1 stride-2 layer 256 -> 512: 71 ->
+  // 67 us).  With fewer tiles, as long as the pairs need no wave more:
+  //  - filters of several rows: half the weights also make room for a halo strip, which a
+  //    vertical stride has not (3x3/2, 392 channels, 2 images of 59x59: 22.7 -> 24.2)
+  //    (3x3, 208 channels, 2 images of 76x76, 95 tiles: 20.6 -> 16.7 us; 3x3, 96 -> 176,
+  //    4 images of 29x20, 60 tiles: 7.2 -> 6.3);
+  //  - products of more than a wave of tiles (2048 x 4096 x 4096, 256 tiles: 65 -> 60 us);
+  //  - products whose rows start at odd multiples of 16 bytes, which take the copy engine
+  //    longer (1500 x 3000 x 3000, 144 tiles: 39 -> 31 us; with whole lines, 2238 x 1216 x
+  //    1792, 126 tiles: 11.2 -> 11.9).
   const int k_elems_stage = kStageKBytes / elem;
-  const long k_steps_per_tile =
-      long(p.taps_h) * p.taps_w * ((p.k_per_tap + k_elems_stage - 1) / k_elems_stage);
-  const int sms_for_pair = sm_count > 0 ? sm_count : 148;
+  const int taps = p.taps_h * p.taps_w;
+  const long k_steps_per_tile = long(taps) * ((p.k_per_tap + k_elems_stage - 1) / k_elems_stage);
+  const long sms_for_pair = sm_count > 0 ? sm_count : 148;
+  const long units_single = best_tiles * n_tiles * groups, units_pair = (best_tiles + 1) / 2 * n_tiles * groups;
+  const bool no_more_waves = (units_pair + sms_for_pair / 2 - 1) / (sms_for_pair / 2) <= (units_single + sms_for_pair - 1) / sms_for_pair;
+  const bool odd_rows = p.act_strides[0] % 32 != 0 || p.wgt_strides[0] % 32 != 0;
+  const bool several_taps = p.taps_h > 1 && p.stride_h == 1 && groups == 1 && k_steps_per_tile >= 8 && units_single >= 48;
+  const bool one_tap = bn >= 128 && k_steps_per_tile >= 7 &&
+                       (units_single > sms_for_pair || (odd_rows && 2 * units_single >= sms_for_pair));
   const bool pair = (p.plan_flags & PLB_PLAN_NO_CTA_PAIR) == 0 && (!p.b_mn || bn >= 128) &&
                     ((p.plan_flags & PLB_PLAN_FORCE_CTA_PAIR) != 0
                          ? best_tiles >= 2
-                         : (k_steps_per_tile >= (bn >= 256 ? 4 : 8) &&
-                            best_tiles * n_tiles * groups >= 2L * sms_for_pair));
+                         : (k_steps_per_tile >= (bn >= 256 ? 4 : 8) && units_single >= 2 * sms_for_pair) ||
+                               (best_tiles >= 2 && no_more_waves && (several_taps || one_tap)));
   plan->cta_pair = pair ? 1 : 0;
   auto grid_for = [&](long m_tiles) {
     const int sms = sm_count > 0 ? sm_count : 148;
