@@ -545,10 +545,12 @@ int launchIgemm(plb_context *ctx, const IgemmProblem &p, const plb_plan &plan) {
     const int mmas_per_tile = a.taps_h * a.taps_w * a.k_chunks * 4;
     // (only with CTA pairs and 64-column tiles, the case it was built and
     // verified for: weights resident or streamed, halo strips)
+    const int stages = dualIssueStages(plan.stages, steps_per_tile);
     a.dual_issue = ((p.plan_flags & PLB_PLAN_NO_DUAL_ISSUE) == 0 && steps_per_tile <= 4 && mmas_per_tile <= 48 &&
-                    plan.tiles >= 2 * plan.grid && plan.cta_pair && plan.tile_n == 64)
+                    plan.tiles >= 2 * plan.grid && plan.cta_pair && plan.tile_n == 64 && !split && stages > 0)
                        ? 1
                        : 0;
+    if (a.dual_issue) a.num_stages = stages;
   }
   // The first steps of every CTA, issued at once by idle warps and pulled towards L2
   // before the predecessor has ended, save a short product most of its time (16 x 512 x

@@ -39,6 +39,23 @@ def test_cluster_count_of_a_device_with_few_clusters(tmp_path):
     assert got == [7] * 7 + [7, 7, 7, 7, 7, 14, 14] + [7, 7, 7, 7, 7, 63, 70]
 
 
+def test_stages_of_two_instruction_issuers(tmp_path):
+    """Tiles alternate between the issuers: each has pipeline stages of its own, whatever fits."""
+    src = tmp_path / "stages.cpp"
+    src.write_text('#include <cstdio>\n#include "launch_shape.h"\nint main() {'
+                   'for (int k = 1; k <= 8; ++k) for (int s = 1; s <= 4; ++s)'
+                   'std::printf("%d %d %d\\n", k, s, plb::dualIssueStages(k, s)); }')
+    exe = tmp_path / "stages"
+    subprocess.run(["g++", "-std=c++17", "-I" + os.path.join(ROOT, "poplibs_b200", "csrc"), str(src), "-o", str(exe)], check=True)
+    for line in subprocess.run([str(exe)], capture_output=True, text=True, check=True).stdout.splitlines():
+        fits, steps, stages = map(int, line.split())
+        assert stages <= fits and (stages > 0) == (fits >= 2 * steps)
+        owner = {}
+        for tile in range(2 * 8 if stages else 0):
+            for g in range(tile * steps, (tile + 1) * steps):
+                assert owner.setdefault(g % stages, tile % 2) == tile % 2
+
+
 def tool(name):
     from poplibs_b200 import build
     build.build_tools()

@@ -332,3 +332,36 @@ def test_float_operands_are_split_in_place_order(gpu_ctx, k, offset):
         T.context().matmul(d, on[0][offset:], on[1][offset:], None, out)
         T.context().synchronize()
         exact(out.cpu().numpy(), a.astype(np.float64) @ b.T.astype(np.float64), "split")
+
+
+@pytest.mark.parametrize("groups,ci,field", [(2, 4, [13, 48]), (1, 8, [13, 48]), (1, 64, [14, 14])])
+def test_short_tiles_launch_after_launch(gpu_ctx, groups, ci, field):
+    """Layers whose tiles two threads issue in turn, on pipelines of few and of many stages, on
+    operands that are not in L2 when the first copies are asked for."""
+    import torch
+    images = 171
+    p = capi.ConvParams.make(batch=images, field=field, kernel=[3, 3], in_chans=ci, out_chans=ci, groups=groups, padding=1)
+    r = T.rng(ci)
+    w = ints(r, (groups, ci, ci, 3, 3), np.float16)
+    dw = T.to_dev(T.weights_to_device_layout(w))
+    xs = [ints(r, (images, groups * ci, *field), np.float16) for _ in range(2)]
+    dx = [T.to_dev(T.acts_to_device_layout(x)) for x in xs]
+    ys = [T.empty_dev([images, *field, groups * ci], np.float16) for _ in xs]
+    flush = torch.empty(1 << 28, dtype=torch.uint8, device="cuda")
+    ctx = capi.Context(0)
+    for plan_flags in (0, capi.PLAN_NO_PDL):
+        ctx.set_plan_flags(plan_flags)
+        for _ in range(20):
+            flush.zero_()
+            torch.cuda.synchronize()
+            for _ in range(5):
+                for x, y in zip(dx, ys):
+                    ctx.conv_fwd(p, x, dw, y)
+            ctx.synchronize()
+    spec = T.spec_from_params(capi.ConvParams.make(batch=3, field=field, kernel=[3, 3], in_chans=ci, out_chans=ci,
+                                                   groups=groups, padding=1))
+    for x, y in zip(xs, ys):
+        got = T.acts_from_device_layout(y[:3].cpu().numpy())
+        exact(got, oracle.conv_fwd(spec, x[:3], w), "first images")
+        got = T.acts_from_device_layout(y[-3:].cpu().numpy())
+        exact(got, oracle.conv_fwd(spec, x[-3:], w), "last images")
