@@ -578,6 +578,20 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
           }
         }
       }
+      if constexpr (k2Cta) {
+        // The leader's commits arrive on this CTA's barriers too: it must not leave, and
+        // its shared memory not become another block's, before the last of them has.
+        // (the producer whose turn it would be: its stage and phase are the next step's)
+        if (!leader && ok && turn == me)
+          for (int i = 0; i < kStages && ok; ++i) {
+            ok = mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag);
+            if (!ok) atomicCAS(args.status, kStatusOk, kStatusDrainTimeout);
+            if (++stage == kStages) {
+              stage = 0;
+              phase ^= 1u;
+            }
+          }
+      }
       if (me == 0) PLB_TRACE_STAMP(2, 4014);
     }
   } else if (warp <= kIgemmMmaWarp) {
@@ -722,6 +736,17 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
           atomicCAS(args.status, kStatusOk, kStatusDrainTimeout);
           break;
         }
+      }
+      if constexpr (k2Cta) {
+        // Likewise the other CTA's epilogue threads arrive here when they have read a tile
+        // (the rendezvous below does not order that): each accumulator's last tile is
+        // waited for as the next one's first instruction would.
+        for (int acc = 0; acc < 2; ++acc)
+          if (ok && (n_issuers == 1 || acc == mi) &&
+              !mbar_wait(tmem_empty_bar(acc), ((acc_phases >> acc) & 1u) ^ 1u, abort_flag)) {
+            atomicCAS(args.status, kStatusOk, kStatusDrainTimeout);
+            ok = false;
+          }
       }
       if (mi == 0) PLB_TRACE_STAMP(2, 4015);
     }
@@ -1088,8 +1113,9 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
     }
   }
   // Neither CTA of a pair may go away while the other can still touch its
-  // barriers, shared memory or tensor memory: the rendezvous of all threads of
-  // the cluster (which is also this CTA's own barrier) orders that.
+  // barriers, shared memory or tensor memory.  Arrivals that one leaves on the
+  // other's barriers have been waited for above; the rendezvous of all threads of
+  // the cluster (which is also this CTA's own barrier) orders the rest.
   if constexpr (k2Cta)
     cluster_sync_relaxed();
   else
