@@ -522,8 +522,9 @@ PLB_API int plb_timer_stop(plb_context *ctx, float *milliseconds);
 /* ------------------------------------------------------------------------ */
 typedef struct plb_plan {
   int32_t kernel;      /* 0 = implicit GEMM (fwd/bwd/matmul), 1 = weight update, 2 = small-channel,
-                          3 = a small product that reads its operands where they lie: it takes no
-                          workspace, and the tiling below is what it runs with under plan flags */
+                          3 = a small product or layer that reads its operands where they lie: it
+                          takes no workspace, and the tiling below is what it runs with under plan
+                          flags and constraints */
   int32_t tile_m;      /* output pixels (rows) per CTA tile                  */
   int32_t tile_n;      /* output channels (columns) per CTA tile             */
   int32_t tile_k_bytes;/* bytes of K per pipeline stage                      */

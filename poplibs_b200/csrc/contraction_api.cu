@@ -11,6 +11,7 @@
 #include "conv_geometry.h"
 #include "direct.h"
 #include "grouped.h"
+#include "patch.h"
 #include "runtime.h"
 #include "igemm_sm100.cuh"
 #include "sm100_prims.cuh"
@@ -483,6 +484,14 @@ Copies planOperands(int type, const void *act, uint64_t rows, uint32_t cols, con
   return c;
 }
 
+// Whether the implicit-GEMM kernel can only read a copy of an operand (`k` channels of
+// a group's pixel).
+bool operandsCopied(const PassOperands &o, uint32_t k) {
+  const size_t es = dtypeBytes(o.type);
+  return o.type == PLB_FLOAT || (k * es) % 16 != 0 || (o.w_pitch * es) % 16 != 0 ||
+         ((reinterpret_cast<uintptr_t>(o.act) | reinterpret_cast<uintptr_t>(o.wgt)) & 15) != 0;
+}
+
 int prepareOperands(plb_context *ctx, int type, const void *act, uint64_t rows, uint32_t cols, const void *wgt,
                     uint64_t w_rows, uint32_t w_cols, uint64_t w_k_rows, PassOperands *o,
                     const Repack::Lattice *lattice = nullptr) {
@@ -601,6 +610,43 @@ int zeroPhases(plb_context *ctx, void *dx, const plb_conv_params &p, const ConvS
   return launch(uint16_t());
 }
 
+// The input gradient at the positions of phase (a, b): a stride-1 convolution of the
+// output gradients with the phase's sub-filter.
+IgemmProblem bwdPhaseProblem(const plb_conv_params &p, const plb_conv_options *opt, const ConvShape &s,
+                             const PassOperands &o, void *dx, bool weights_transposed, int a, int b, const BwdPhase &A,
+                             const BwdPhase &B) {
+  const size_t os = dtypeBytes(p.output_type);
+  const uint64_t ctot = uint64_t(p.groups) * p.in_chans_per_group;
+  IgemmProblem r = convBwdProblem(p, opt, s, o, dx, weights_transposed);
+  r.out_w = B.extent;
+  r.out_h = A.extent;
+  r.taps_h = A.taps;
+  r.taps_w = B.taps;
+  // tap j of the phase is used tap first + j*step of the (possibly flipped)
+  // filter, stored where the flip, the truncation and (weights_transposed)
+  // the reversal of all stored taps put it
+  auto stored = [&](int used, int K, int Ks, int kt, int flip) {
+    const int at = kt + (flip ? K - 1 - used : used);
+    return weights_transposed ? Ks - 1 - at : at;
+  };
+  const int h0 = stored(A.first_tap, s.KH, s.KHs, s.ktH, s.flipH);
+  const int w0 = stored(B.first_tap, s.KW, s.KWs, s.ktW, s.flipW);
+  setTaps(&r, s, h0, (s.flipH != 0) != weights_transposed ? -A.step : A.step, w0,
+          (s.flipW != 0) != weights_transposed ? -B.step : B.step);
+  // position i of the phase reads output index i + offset - j*dil for its
+  // j-th tap: a correlation with the taps reversed
+  r.dil_h = A.dil;
+  r.dil_w = B.dil;
+  r.pad_h = (A.taps - 1) * A.dil - A.offset;
+  r.pad_w = (B.taps - 1) * B.dil - B.offset;
+  r.flip_h = 1;
+  r.flip_w = 1;
+  r.out = static_cast<uint8_t *>(dx) + (size_t(s.tH + a) * s.W + (s.tW + b)) * ctot * os;
+  r.ldc = (long long)(ctot * s.strW);
+  r.out_stride_h = (long long)(ctot * s.W * s.strH);
+  return r;
+}
+
 // Backward pass of a strided convolution (the reference's getGradientParams
 // gives the output gradients an input dilation equal to the forward stride,
 // lib/poplin/ConvUtil.cpp:728-795).  Multiplying the inserted zeros would
@@ -647,33 +693,7 @@ int convBwdStrided(plb_context *ctx, const plb_conv_params &p, const plb_conv_op
     for (int b = 0; b < s.strW; ++b) {
       const BwdPhase &A = ph[size_t(a)], &B = pw[size_t(b)];
       if (A.extent == 0 || B.extent == 0 || A.taps == 0 || B.taps == 0) continue;
-      IgemmProblem r = convBwdProblem(p, opt, s, o, dx, weights_transposed);
-      r.out_w = B.extent;
-      r.out_h = A.extent;
-      r.taps_h = A.taps;
-      r.taps_w = B.taps;
-      // tap j of the phase is used tap first + j*step of the (possibly flipped)
-      // filter, stored where the flip, the truncation and (weights_transposed)
-      // the reversal of all stored taps put it
-      auto stored = [&](int used, int K, int Ks, int kt, int flip) {
-        const int at = kt + (flip ? K - 1 - used : used);
-        return weights_transposed ? Ks - 1 - at : at;
-      };
-      const int h0 = stored(A.first_tap, s.KH, s.KHs, s.ktH, s.flipH);
-      const int w0 = stored(B.first_tap, s.KW, s.KWs, s.ktW, s.flipW);
-      setTaps(&r, s, h0, (s.flipH != 0) != weights_transposed ? -A.step : A.step, w0,
-              (s.flipW != 0) != weights_transposed ? -B.step : B.step);
-      // position i of the phase reads output index i + offset - j*dil for its
-      // j-th tap: a correlation with the taps reversed
-      r.dil_h = A.dil;
-      r.dil_w = B.dil;
-      r.pad_h = (A.taps - 1) * A.dil - A.offset;
-      r.pad_w = (B.taps - 1) * B.dil - B.offset;
-      r.flip_h = 1;
-      r.flip_w = 1;
-      r.out = static_cast<uint8_t *>(dx) + (size_t(s.tH + a) * s.W + (s.tW + b)) * ctot * os;
-      r.ldc = (long long)(ctot * s.strW);
-      r.out_stride_h = (long long)(ctot * s.W * s.strH);
+      IgemmProblem r = bwdPhaseProblem(p, opt, s, o, dx, weights_transposed, a, b, A, B);
       if (separate) r.nonfinite = nonfiniteFlag(ctx);
       r.plan_flags |= ctx->plan_flags;
       plb_plan plan{};
@@ -688,6 +708,48 @@ int convBwdStrided(plb_context *ctx, const plb_conv_params &p, const plb_conv_op
   }
   if (!separate || phases.empty()) return PLB_OK;
   return repairNonFinite(ctx, convBwdProblem(*separate_p, opt, s, *separate, dx, false), separate->type, s.strH, s.strW);
+}
+
+// Whether a pass runs on the patch kernel (patch.cu), and its problem(s); `o` are the
+// caller's operands, `groups` those that the general route contracts together.
+bool fwdOnPatches(int sm_count, const plb_conv_params &p, const plb_conv_options *opt, int plan_flags, const ConvShape &s,
+                  const PassOperands &o, const float *bias, void *out, bool swapped, int groups, IgemmProblem *r) {
+  if ((!pointwise(s) && (s.strH > 8 || s.strW > 8)) || s.KH <= 0 || s.KW <= 0) return false;
+  *r = convFwdProblem(p, opt, s, o, bias, out, swapped);
+  r->plan_flags |= plan_flags;
+  const int launches = 1 + (groups > 1 ? 2 : 0) + (operandsCopied(o, p.in_chans_per_group) ? 1 : 0);
+  const bool packed = p.groups == 1 && p.input_type != PLB_FLOAT && !swapped && !channelsFitTma(p, p.in_chans_per_group);
+  return patchSuits(sm_count, r, 1, p.input_type, launches, groups, packed);
+}
+// (the number of problems, 0 if it does not)
+int bwdOnPatches(int sm_count, const plb_conv_params &p, const plb_conv_options *opt, int plan_flags, const ConvShape &s,
+                 const PassOperands &o, void *dx, int groups, IgemmProblem *r) {
+  int n = 0, launches = 0;
+  if (s.strH == 1 && s.strW == 1) {
+    r[n++] = convBwdProblem(p, opt, s, o, dx, false);
+    launches = 1;
+  } else if (s.strH * s.strW <= kPatchMaxPhases) {
+    // (a phase that no tap reaches is a sum of nothing: it is cleared by the same launch;
+    // the general route clears all such phases in one)
+    bool clears = false;
+    for (int a = 0; a < s.strH; ++a)
+      for (int b = 0; b < s.strW; ++b) {
+        BwdPhase A, B;
+        bwdPhase(a, s.He, s.KH, s.padH, s.dilH, s.strH, &A);
+        bwdPhase(b, s.We, s.KW, s.padW, s.dilW, s.strW, &B);
+        if (A.extent <= 0 || B.extent <= 0) continue;
+        r[n++] = bwdPhaseProblem(p, opt, s, o, dx, false, a, b, A, B);
+        if (A.taps == 0 || B.taps == 0)
+          clears = true;
+        else
+          ++launches;
+      }
+    launches += clears ? 1 : 0;
+  }
+  if (n == 0) return 0;
+  r[0].plan_flags |= plan_flags;
+  launches += (groups > 1 ? 2 : 0) + (operandsCopied(o, p.out_chans_per_group) ? 1 : 0);
+  return patchSuits(sm_count, r, n, p.input_type, launches, groups, false) ? n : 0;
 }
 
 // Narrow channel groups are contracted together (grouped.cu): `q` = the layer of
@@ -929,6 +991,14 @@ int plb_conv_plan(const plb_conv_params *p_in, const plb_conv_options *opt, int3
     if (transposed) plan->workspace_bytes += tiles * ci * pitch;
     if (together > 1) plan->workspace_bytes += size_t(tiles) * ci * co * es;  // block-diagonal weights
   }
+  if (plan->tiles > 0) {
+    IgemmProblem r[kPatchMaxPhases];
+    const PassOperands o{p->input_type, nullptr, nullptr, bwd ? p->out_chans_per_group : p->in_chans_per_group,
+                         bwd ? p->out_chans_per_group : p->in_chans_per_group, p->in_chans_per_group};
+    if (bwd ? bwdOnPatches(148, *p, opt, 0, s, o, nullptr, int(together), r) > 0
+            : fwdOnPatches(148, *p, opt, 0, s, o, nullptr, nullptr, false, int(together), r))
+      plan->kernel = 3;
+  }
   plan->flops = 2 * numberOfMacs(*p);
   plan->bytes = convBytes(*p, s, pass);
   return PLB_OK;
@@ -1004,6 +1074,16 @@ int plb_convolution(plb_context *ctx, const plb_conv_params *p, const plb_conv_o
     }
     if (s.OHc <= 0 || s.OWc <= 0 || s.He <= 0 || s.We <= 0) return PLB_OK;
   }
+  const bool swapped = transpose_and_flip_weights != 0;
+  // the caller's operands, the groups apart
+  const PassOperands separate{p->input_type, d_in, d_weights, p->in_chans_per_group, p->in_chans_per_group,
+                              swapped ? p->out_chans_per_group : p->in_chans_per_group};
+  {
+    IgemmProblem r;
+    const int groups = groupsTogether(p->groups, p->in_chans_per_group, p->out_chans_per_group, p->input_type);
+    if (fwdOnPatches(ctx->sm_count, *p, opt, ctx->plan_flags, s, separate, d_bias, d_out, swapped, groups, &r))
+      return launchPatch(ctx, &r, 1, p->input_type, groups > 1);
+  }
   if (p->input_type != PLB_FLOAT && !channelsFitTma(*p, p->in_chans_per_group) && !transpose_and_flip_weights) {
     // few input channels (a stem): space-to-depth path, where it applies
     const int rc = convFwdSmallChannels(ctx, *p, opt, d_in, d_weights, d_bias, d_out, nullptr);
@@ -1021,7 +1101,6 @@ int plb_convolution(plb_context *ctx, const plb_conv_params *p, const plb_conv_o
                              ctx->stream));
     return PLB_OK;
   }
-  const bool swapped = transpose_and_flip_weights != 0;
   plb_conv_params q;
   const void *w = nullptr;
   bool together = false;
@@ -1047,8 +1126,6 @@ int plb_convolution(plb_context *ctx, const plb_conv_params *p, const plb_conv_o
   if (together) r.nonfinite = nonfiniteFlag(ctx);
   if (int rc = runProblem(ctx, r)) return rc;
   if (!together) return PLB_OK;
-  const PassOperands separate{p->input_type, d_in, d_weights, p->in_chans_per_group, p->in_chans_per_group,
-                              swapped ? p->out_chans_per_group : p->in_chans_per_group};
   return repairNonFinite(ctx, convFwdProblem(*p, opt, s, separate, d_bias, d_out, swapped), p->input_type);
 }
 
@@ -1127,6 +1204,15 @@ int plb_conv_bwd(plb_context *ctx, const plb_conv_params *p, const plb_conv_opti
                                ctx->stream));
     return PLB_OK;
   }
+  // the caller's operands, the groups apart
+  const PassOperands separate{p->input_type, d_out_grads, d_weights, p->out_chans_per_group, p->out_chans_per_group,
+                              p->in_chans_per_group};
+  {
+    IgemmProblem r[kPatchMaxPhases];
+    const int groups = groupsTogether(p->groups, p->in_chans_per_group, p->out_chans_per_group, p->input_type);
+    if (const int n = bwdOnPatches(ctx->sm_count, *p, opt, ctx->plan_flags, s, separate, d_in_grads, groups, r))
+      return launchPatch(ctx, r, n, p->input_type, groups > 1);
+  }
   plb_conv_params q;
   const void *w = nullptr;
   bool together = false;
@@ -1144,8 +1230,6 @@ int plb_conv_bwd(plb_context *ctx, const plb_conv_params *p, const plb_conv_opti
     // the reduction runs over the output channels, the rows of a weight tile
     if (int rc = prepareOperands(ctx, q.input_type, d_out_grads, out_rows, co, w, tiles * co, ci, co, &o)) return rc;
   }
-  const PassOperands separate{p->input_type, d_out_grads, d_weights, p->out_chans_per_group, p->out_chans_per_group,
-                              p->in_chans_per_group};
   if (s.strH != 1 || s.strW != 1)
     return convBwdStrided(ctx, q, opt, s, o, d_in_grads, transposed, p, together ? &separate : nullptr);
   IgemmProblem r = convBwdProblem(q, opt, s, o, d_in_grads, transposed);

@@ -86,26 +86,38 @@ template <bool kVec> struct DirectUnit<PLB_HALF, kVec> {
     }
   }
   __device__ __forceinline__ void loadSome(const uint8_t *p, int n) {
-    const uint16_t *x = reinterpret_cast<const uint16_t *>(p);
-    off = 0u;
-#pragma unroll
-    for (int j = 0; j < kWords; ++j) {
-      w[j] = 0u;
-      if (j < 4 && 2 * j < n) w[j] = x[2 * j];
-      if (j < 4 && 2 * j + 1 < n) w[j] |= uint32_t(x[2 * j + 1]) << 16;
+    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+    if constexpr (kVec) {
+      put(0, n > 0 ? *reinterpret_cast<const uint4 *>(p) : zero);
+      keep(n);
+    } else {
+      off = uint32_t(reinterpret_cast<uintptr_t>(p)) & 15;
+      const uint4 *x = reinterpret_cast<const uint4 *>(p - off);
+      put(0, n > 0 ? x[0] : zero);
+      put(4, n > 0 && int(off) + 2 * min(n, 8) > 16 ? x[1] : zero);
+      place();
+      keep(n);
+      off = 0u;
     }
   }
+  // the first n elements, the rest zero
+  __device__ __forceinline__ void keep(int n) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) w[j] = n >= 2 * j + 2 ? w[j] : n == 2 * j + 1 ? w[j] & 0xffffu : 0u;
+  }
+  // the elements to the front
+  __device__ __forceinline__ void place() {
+    const bool two = (off & 8) != 0, one = (off & 4) != 0;
+#pragma unroll
+    for (int j = 0; j < 6; ++j) w[j] = two ? w[j + 2] : w[j];
+#pragma unroll
+    for (int j = 0; j < 5; ++j) w[j] = one ? w[j + 1] : w[j];
+    const uint32_t shift = (off & 2) * 8;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) w[j] = __funnelshift_r(w[j], w[j + 1], shift);
+  }
   __device__ __forceinline__ void store(uint32_t dst, uint32_t, int, int &) {
-    if constexpr (!kVec) {
-      const bool two = (off & 8) != 0, one = (off & 4) != 0;
-#pragma unroll
-      for (int j = 0; j < 6; ++j) w[j] = two ? w[j + 2] : w[j];
-#pragma unroll
-      for (int j = 0; j < 5; ++j) w[j] = one ? w[j + 1] : w[j];
-      const uint32_t shift = (off & 2) * 8;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) w[j] = __funnelshift_r(w[j], w[j + 1], shift);
-    }
+    if constexpr (!kVec) place();
     st_shared_v4(dst, w[0], w[1], w[2], w[3]);
   }
 };
@@ -131,10 +143,18 @@ template <bool kVec> struct DirectUnit<PLB_QUARTER, kVec> {
     }
   }
   __device__ __forceinline__ void loadSome(const uint8_t *p, int n) {
-    w[0] = w[1] = w[2] = shift = 0u;
+    const uint32_t off = uint32_t(reinterpret_cast<uintptr_t>(p)) & 3;
+    const uint32_t *x = reinterpret_cast<const uint32_t *>(p - off);
+    const int bytes = n > 0 ? int(off) + min(n, 8) : 0;
 #pragma unroll
-    for (int j = 0; j < 8; ++j)
-      if (j < n) w[j / 4] |= uint32_t(p[j]) << (j % 4 * 8);
+    for (int j = 0; j < 3; ++j) w[j] = 4 * j < bytes ? x[j] : 0u;
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const uint32_t v = __funnelshift_r(w[j], w[j + 1], off * 8);
+      const int rest = n - 4 * j;
+      w[j] = rest >= 4 ? v : rest <= 0 ? 0u : v & ((1u << (8 * rest)) - 1);
+    }
+    w[2] = shift = 0u;
   }
   __device__ __forceinline__ void store(uint32_t dst, uint32_t, int fmt, int &) {
     const __nv_fp8_interpretation_t f = fmt == PLB_F152 ? __NV_E5M2 : __NV_E4M3;
@@ -163,18 +183,27 @@ template <bool kVec> struct DirectUnit<PLB_FLOAT, kVec> {
     if constexpr (!kVec) *reinterpret_cast<float4 *>(&f[8]) = off ? v[2] : make_float4(0.f, 0.f, 0.f, 0.f);
   }
   __device__ __forceinline__ void loadSome(const uint8_t *p, int n) {
+    off = kVec ? 0u : uint32_t(reinterpret_cast<uintptr_t>(p)) & 15;
+    const float4 *v = reinterpret_cast<const float4 *>(p - off);
+    const int bytes = n > 0 ? int(off) + 4 * min(n, 8) : 0;
+#pragma unroll
+    for (int j = 0; j < kWords / 4; ++j)
+      *reinterpret_cast<float4 *>(&f[4 * j]) = 16 * j < bytes ? v[j] : make_float4(0.f, 0.f, 0.f, 0.f);
+    if constexpr (!kVec) place();
     off = 0u;
 #pragma unroll
-    for (int j = 0; j < kWords; ++j) f[j] = j < n && j < 8 ? reinterpret_cast<const float *>(p)[j] : 0.f;
+    for (int j = 0; j < 8; ++j) f[j] = j < n ? f[j] : 0.f;
+  }
+  // the elements to the front
+  __device__ __forceinline__ void place() {
+    const bool two = (off & 8) != 0, one = (off & 4) != 0;
+#pragma unroll
+    for (int j = 0; j < 10; ++j) f[j] = two ? f[j + 2] : f[j];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) f[j] = one ? f[j + 1] : f[j];
   }
   __device__ __forceinline__ void store(uint32_t dst, uint32_t plane, int, int &odd) {
-    if constexpr (!kVec) {
-      const bool two = (off & 8) != 0, one = (off & 4) != 0;
-#pragma unroll
-      for (int j = 0; j < 10; ++j) f[j] = two ? f[j + 2] : f[j];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) f[j] = one ? f[j + 1] : f[j];
-    }
+    if constexpr (!kVec) place();
     uint32_t hi[4], lo[4];
     __nv_bfloat162 most;
 #pragma unroll

@@ -1,0 +1,21 @@
+// Convolutions of narrow channel groups and small ragged layers from input patches in
+// shared memory (patch.cuh, patch.cu).
+#pragma once
+
+#include "runtime.h"
+
+namespace plb {
+
+// Problems of one launch: the phases of a strided layer's input gradient, else one.
+constexpr int kPatchMaxPhases = 4;
+
+// Whether these problems (same operands, groups and channel counts; `type` is the
+// operands' element type, all pointers are the caller's) run on the patch kernel.
+// `launches`: what the general route takes; `together`: the groups that it contracts as one;
+// `packed`: whether it gathers the channels of several taps into one operand row.
+bool patchSuits(int sm_count, const IgemmProblem *p, int n, int type, int launches, int together, bool packed);
+// `repair`: outputs whose sum is not finite are formed again without the products
+// with padding, as repairNonFinite does.
+int launchPatch(plb_context *ctx, const IgemmProblem *p, int n, int type, bool repair);
+
+}  // namespace plb

@@ -603,9 +603,10 @@ void addBias(Graph &graph, const Tensor &acts, const Tensor &biases, Sequence &p
 // ---- plan reporting ------------------------------------------------------------------------
 static void printPlan(std::ostream &out, const plb_plan &plan, const char *pass) {
   static const char *kernels[] = {"implicit GEMM (TMA + tcgen05)", "weight update (split-K)",
-                                  "small-channel (space-to-depth + implicit GEMM)"};
+                                  "small-channel (space-to-depth + implicit GEMM)",
+                                  "operands where they lie (mma.sync)"};
   out << "  Plan (" << pass << "):\n"
-      << "        kernel                     " << kernels[std::min(std::max(plan.kernel, 0), 2)] << "\n"
+      << "        kernel                     " << kernels[std::min(std::max(plan.kernel, 0), 3)] << "\n"
       << "        CTA tile (pixels x chans)  " << plan.tile_m << " x " << plan.tile_n << "\n"
       << "        pixel box (w, h, n)        {" << plan.box_w << "," << plan.box_h << ","
       << plan.box_n << "}\n"
