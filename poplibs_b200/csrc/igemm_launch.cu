@@ -116,7 +116,9 @@ int planIgemm(const IgemmProblem &p, int sm_count, plb_plan *plan) {
   //  - filters of several rows: half the weights also make room for a halo strip, which a
   //    vertical stride has not (3x3/2, 392 channels, 2 images of 59x59: 22.7 -> 24.2)
   //    (3x3, 208 channels, 2 images of 76x76, 95 tiles: 20.6 -> 16.7 us; 3x3, 96 -> 176,
-  //    4 images of 29x20, 60 tiles: 7.2 -> 6.3);
+  //    4 images of 29x20, 60 tiles: 7.2 -> 6.3); not short tiles of 64 columns in a second
+  //    wave that is mostly empty (3x3, 48 channels, 42 images of 8x84, 231 tiles: 8.7 -> 9.2;
+  //    11 sampled layers 5 % slower);
   //  - products of more than a wave of tiles (2048 x 4096 x 4096, 256 tiles: 65 -> 60 us);
   //  - products whose rows start at odd multiples of 16 bytes, which take the copy engine
   //    longer (1500 x 3000 x 3000, 144 tiles: 39 -> 31 us; with whole lines, 2238 x 1216 x
@@ -128,7 +130,8 @@ int planIgemm(const IgemmProblem &p, int sm_count, plb_plan *plan) {
   const long units_single = best_tiles * n_tiles * groups, units_pair = (best_tiles + 1) / 2 * n_tiles * groups;
   const bool no_more_waves = (units_pair + sms_for_pair / 2 - 1) / (sms_for_pair / 2) <= (units_single + sms_for_pair - 1) / sms_for_pair;
   const bool odd_rows = p.act_strides[0] % 32 != 0 || p.wgt_strides[0] % 32 != 0;
-  const bool several_taps = p.taps_h > 1 && p.stride_h == 1 && groups == 1 && k_steps_per_tile >= 8 && units_single >= 48;
+  const bool several_taps = p.taps_h > 1 && p.stride_h == 1 && groups == 1 && k_steps_per_tile >= 8 && units_single >= 48 &&
+                            !(bn <= 64 && k_steps_per_tile < 16 && units_single > sms_for_pair);
   const bool one_tap = bn >= 128 && k_steps_per_tile >= 7 &&
                        (units_single > sms_for_pair || (odd_rows && 2 * units_single >= sms_for_pair));
   const bool pair = (p.plan_flags & PLB_PLAN_NO_CTA_PAIR) == 0 && (!p.b_mn || bn >= 128) &&
