@@ -15,6 +15,8 @@
 #include "runtime.h"
 #include "igemm_sm100.cuh"
 #include "sm100_prims.cuh"
+#include "small_channel.h"
+#include "stem.h"
 
 namespace plb {
 
@@ -1078,6 +1080,11 @@ int plb_convolution(plb_context *ctx, const plb_conv_params *p, const plb_conv_o
   // the caller's operands, the groups apart
   const PassOperands separate{p->input_type, d_in, d_weights, p->in_chans_per_group, p->in_chans_per_group,
                               swapped ? p->out_chans_per_group : p->in_chans_per_group};
+  if (is16BitFloat(p->input_type) && p->groups == 1 && !channelsFitTma(*p, p->in_chans_per_group) && !swapped) {
+    S2dShape g;
+    if (stemLayer(ctx, *p, opt, d_out, &g))
+      return launchStem(ctx, g, int(p->out_chans_per_group), p->input_type == PLB_BFLOAT16, d_in, d_weights, d_bias, d_out);
+  }
   {
     IgemmProblem r;
     const int groups = groupsTogether(p->groups, p->in_chans_per_group, p->out_chans_per_group, p->input_type);

@@ -26,6 +26,7 @@
 #include "runtime.h"
 #include "small_channel.h"
 #include "sm100_prims.cuh"
+#include "stem.h"
 
 namespace plb {
 
@@ -243,6 +244,12 @@ int smallChannelPrepare(plb_context *ctx, const S2dShape &g, const void *d_in, _
     case 4: return launch(s2dInputKernel<2, 4>);
     default: return launch(s2dInputKernel<2, 0>);
   }
+}
+
+// Whether the stem kernel runs the forward pass.
+bool stemLayer(const plb_context *ctx, const plb_conv_params &p, const plb_conv_options *opt, const void *d_out, S2dShape *g) {
+  return smallChannelShape(p, g) == PLB_OK && ctx->plan_flags == 0 && (!opt || (opt->plan_flags == 0 && opt->tile_n == 0)) &&
+         stemSuits(ctx->sm_count, *g, int(p.out_chans_per_group), p.output_type == PLB_FLOAT, d_out);
 }
 
 int convFwdSmallChannels(plb_context *ctx, const plb_conv_params &p, const plb_conv_options *opt,

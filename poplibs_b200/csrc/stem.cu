@@ -1,0 +1,433 @@
+// Forward convolution of few input channels (a stem: 7x7, stride 2, 3 channels) from the
+// image as it is.
+//
+// Rearranged in global memory (small_channel.cu), such a layer writes and reads its input
+// once more, in a launch of its own, and every filter row fetches 128 bytes of overlapping
+// windows for each output pixel.  Here a block loads the rows of a strip of output pixels
+// once, as superpixels of 16 bytes: the stride's pixels of a row side by side (3 channels,
+// stride 2: 6 halves and two zeros).  Output pixel i and horizontal tap t of a filter row
+// then meet at superpixel i + t, so consecutive output pixels' operand rows lie 16 bytes
+// apart.  That is the unswizzled K-major layout of tcgen05 (core matrices of eight 16-byte
+// rows), whose core-matrix stride along K is 16 bytes here: they overlap, nothing is copied
+// per tap, and the instruction is as fast as from 128-byte rows (48 cycles of 128 x 64 x 16
+// either way).  Filter rows of one parity of the stride share a plane of superpixel rows, P
+// apart; a tile is 128 consecutive positions of the strip, the last T-1 of every row not
+// stored.
+//
+// Roles: 7 warps load strips (two in flight), one thread issues the instructions, two groups
+// of 4 warps store alternate tiles.  Loads, results and operands share the SM's path to
+// shared memory and L1; a tile of 14 instructions (7x7) takes 1400 cycles of the 670 that the
+// instructions alone would, one of 6 (3x3) is bound by its results.  Measured: 3x3, 1 -> 96 on
+// 147 images of 118 x 118 137.5 -> 94.0 us, 3x3/2, 4 -> 64 on 11 of 102 x 192 10.1 -> 5.5,
+// 7x7/2, 3 -> 64 on 256 of 224 x 224 162.4 -> 156.5.  (Whole lines of results, stored from 16
+// x 256-bit reads of tensor memory, two issuers or four accumulators: no gain.)
+#include <algorithm>
+#include <atomic>
+#include <cmath>
+
+#include "sm100_prims.cuh"
+#include "stem.h"
+
+namespace plb {
+namespace {
+
+constexpr int kStemThreads = 512, kStemMmaWarp = 8, kStemLoaders = 224;
+
+struct StemArgs {
+  const uint16_t *x, *w;
+  const float *bias;
+  __half *out;
+  int *status;
+  S2dShape g;
+  int co, co_pad;         // co_pad: columns of an accumulator
+  int taps;               // superpixels of a filter row, even
+  int pad_w, shift;       // padding rounded up to the stride; by how much
+  int tile_w, rows, pitch;  // a strip: output columns and rows, superpixels of a row
+  int parts, h_blocks, units;
+  uint32_t plane_bytes, strip_bytes, weight_bytes;
+  uint32_t idesc, tmem_cols;
+  FastDiv fd_pitch, fd_parts, fd_h_blocks, fd_co, fd_taps;
+};
+
+// A sum over the pixels that exist.
+template <bool kBf16>
+__device__ __noinline__ float stemSum(const StemArgs &a, int n, int oh, int ow, int co) {
+  const S2dShape &g = a.g;
+  auto value = [](uint16_t v) {
+    return kBf16 ? __uint_as_float(uint32_t(v) << 16) : __half2float(__ushort_as_half(v));
+  };
+  float sum = 0.f;
+#pragma unroll 1
+  for (int r = 0; r < g.KH; ++r)
+#pragma unroll 1
+    for (int s = 0; s < g.KW; ++s) {
+      const int ih = oh * g.s + r - g.padH, iw = ow * g.s + s - g.padW;
+      if (ih < 0 || iw < 0 || ih >= g.H || iw >= g.W) continue;
+#pragma unroll 1
+      for (int c = 0; c < g.C; ++c)
+        sum += value(a.x[(((long long)n * g.H + ih) * g.W + iw) * g.C + c]) * value(a.w[((r * g.KW + s) * a.co + co) * g.C + c]);
+    }
+  return sum;
+}
+
+// K-major operand without swizzle: core matrices of eight 16-byte rows, `lbo` apart along K
+// and `sbo` along M or N.
+__device__ __forceinline__ uint64_t plainDesc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
+  return uint64_t((addr & 0x3ffffu) >> 4) | uint64_t(lbo >> 4) << 16 | uint64_t(sbo >> 4) << 32 | uint64_t(1) << 46;
+}
+
+// kWords: 32-bit words of a superpixel, 0 where its elements are loaded one by one.
+template <int kWords, bool kBf16>
+__global__ void __launch_bounds__(kStemThreads, 1)
+stemKernel(const __grid_constant__ StemArgs a) {
+  extern __shared__ __align__(128) uint8_t stem_smem[];
+  __shared__ __align__(8) uint64_t bars[9];  // strip full, strip free, accumulator full, accumulator free, drain
+  __shared__ uint32_t tmem_slot;
+  __shared__ int abort_word;
+  __shared__ __align__(16) float bias[256];
+  const S2dShape &g = a.g;
+  const int tid = int(threadIdx.x), warp = tid >> 5, lane = tid & 31;
+  const uint32_t weights = smem_u32(stem_smem), strips = weights + a.weight_bytes;
+  volatile int *abort_flag = &abort_word;
+  auto stripFull = [&](int i) { return smem_u32(bars + i); };
+  auto stripFree = [&](int i) { return smem_u32(bars + 2 + i); };
+  auto accFull = [&](int i) { return smem_u32(bars + 4 + i); };
+  auto accFree = [&](int i) { return smem_u32(bars + 6 + i); };
+  if (tid == 0) {
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(stripFull(i), kStemLoaders);
+      mbar_init(stripFree(i), 1);
+      mbar_init(accFull(i), 1);
+      mbar_init(accFree(i), 128);
+    }
+    mbar_init(smem_u32(bars + 8), 1);
+    abort_word = 0;
+    mbar_fence_init();
+  }
+  if (warp == kStemMmaWarp) {
+    tmem_alloc(smem_u32(&tmem_slot), a.tmem_cols);
+    tmem_relinquish();
+  }
+  pdl_wait();  // (all threads: they read the operands, or write over what the last kernel read)
+  // weights: [filter row][superpixel][output channel] of 16 bytes
+  for (int i = tid; i < g.KH * a.taps * a.co; i += kStemThreads) {
+    const int rt = int(fast_div(uint32_t(i), a.fd_co)), co = i - rt * a.co, r = int(fast_div(uint32_t(rt), a.fd_taps)), t = rt - r * a.taps;
+    uint32_t v[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      uint32_t both = 0;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int e = 2 * j + h, px = e >= g.C ? 1 : 0, c = e - px * g.C, s = t * g.s + px - a.shift;
+        if (e < g.s * g.C && s >= 0 && s < g.KW) both |= uint32_t(a.w[((r * g.KW + s) * a.co + co) * g.C + c]) << (16 * h);
+      }
+      v[j] = both;
+    }
+    st_shared_v4(weights + uint32_t(i) * 16, v[0], v[1], v[2], v[3]);
+  }
+  if (tid < a.co_pad) bias[tid] = a.bias && tid < a.co ? a.bias[tid] : 0.f;
+  fence_proxy_async_smem();
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  pdl_launch_dependents();  // (tensor memory is allocated: the next kernel cannot take it first)
+  const uint32_t tmem = *static_cast<volatile uint32_t *>(&tmem_slot);
+  // strip u: image, first output row and column, and its tiles
+  auto stripOf = [&](int u, int &n, int &oh0, int &ow0, int &rows, int &cols) {
+    const int v = int(fast_div(uint32_t(u), a.fd_parts));
+    n = int(fast_div(uint32_t(v), a.fd_h_blocks));
+    oh0 = (v - n * a.h_blocks) * a.rows;
+    ow0 = (u - v * a.parts) * a.tile_w;
+    rows = min(a.rows, g.OH - oh0);
+    cols = min(a.tile_w, g.OW - ow0);
+    return ((rows - 1) * a.pitch + cols + 127) >> 7;
+  };
+  bool ok = true;
+  auto failed = [&](int code) {
+    atomicCAS(a.status, kStatusOk, code);
+    ok = false;
+  };
+
+  if (warp > kStemMmaWarp) {
+    // ---- loaders
+    const int me = tid - (kStemMmaWarp + 1) * 32;
+    for (int u = int(blockIdx.x), k = 0; u < a.units; u += int(gridDim.x), ++k) {
+      int n, oh0, ow0, rows, cols;
+      stripOf(u, n, oh0, ow0, rows, cols);
+      const int buf = k & 1;
+      if (!mbar_wait(stripFree(buf), uint32_t(k >> 1 & 1) ^ 1u, abort_flag)) {
+        failed(kStatusProducerTimeout);
+        break;
+      }
+      const uint32_t strip = strips + uint32_t(buf) * a.strip_bytes;
+      const int total = ((rows - 1) * g.s + g.KH) * a.pitch, ih0 = oh0 * g.s - g.padH, px0 = ow0 * g.s - a.pad_w;
+      const uint16_t *img = a.x + (long long)n * g.H * g.W * g.C;
+#pragma unroll 1
+      for (int i0 = me; i0 < total; i0 += 4 * kStemLoaders) {
+        uint32_t v[4][4], dst[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int i = i0 + j * kStemLoaders;
+          const int y = int(fast_div(uint32_t(i), a.fd_pitch)), at = i - y * a.pitch;
+          const int q = g.s == 2 ? y >> 1 : y, plane = y - q * g.s;
+          const int ih = ih0 + y, px = px0 + at * g.s;
+          // (px is a multiple of the stride: all of a superpixel lies left of the image, or none)
+          const int there = i < total && uint32_t(ih) < uint32_t(g.H) && px >= 0 ? min(g.W - px, g.s) * g.C : 0;
+          dst[j] = strip + uint32_t(plane) * a.plane_bytes + uint32_t(q * a.pitch + at) * 16;
+          const uint16_t *p = img + (ih * g.W + px) * g.C;
+          if constexpr (kWords > 0) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              v[j][e] = e < kWords && 2 * e < there ? reinterpret_cast<const uint32_t *>(p)[e] : 0u;
+          } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const uint32_t lo = 2 * e < there ? p[2 * e] : 0u, hi = 2 * e + 1 < there ? p[2 * e + 1] : 0u;
+              v[j][e] = lo | hi << 16;
+            }
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (i0 + j * kStemLoaders < total) st_shared_v4(dst[j], v[j][0], v[j][1], v[j][2], v[j][3]);
+      }
+      fence_proxy_async_smem();
+      mbar_arrive(stripFull(buf));
+    }
+  } else if (warp == kStemMmaWarp) {
+    // ---- instructions
+    if (elect_one()) {
+      int c = 0, k = 0;
+      for (int u = int(blockIdx.x); ok && u < a.units; u += int(gridDim.x), ++k) {
+        int n, oh0, ow0, rows, cols;
+        const int tiles = stripOf(u, n, oh0, ow0, rows, cols), buf = k & 1;
+        if (!mbar_wait(stripFull(buf), uint32_t(k >> 1 & 1), abort_flag)) {
+          failed(kStatusMmaTimeout);
+          break;
+        }
+        tc_fence_after_sync();
+        const uint32_t strip = strips + uint32_t(buf) * a.strip_bytes;
+        for (int t = 0; t < tiles; ++t, ++c) {
+          const int acc = c & 1;
+          if (!mbar_wait(accFree(acc), uint32_t(c >> 1 & 1) ^ 1u, abort_flag)) {
+            failed(kStatusMmaTimeout);
+            break;
+          }
+          tc_fence_after_sync();
+          uint64_t b = plainDesc(weights, uint32_t(a.co) * 16, 128);
+          const uint32_t d = tmem + uint32_t(acc * a.co_pad), b_step = uint32_t(a.co) * 2;
+          const uint64_t a0 = plainDesc(strip + uint32_t(t * 128) * 16, 16, 128);
+          // (unrolled: a loop over single instructions paces them, 7x7 190 us)
+          auto filterRow = [&](uint64_t ad, bool first) {
+            umma_ss<false>(d, ad, b, a.idesc, first ? 0u : 1u);
+            b += b_step;
+#pragma unroll 1
+            for (int s = 2; s < a.taps; s += 2) {
+              ad += 2;
+              umma_ss<false>(d, ad, b, a.idesc, 1u);
+              b += b_step;
+            }
+          };
+          const uint32_t down = uint32_t(a.pitch), plane1 = g.s == 2 ? a.plane_bytes >> 4 : down;
+          const uint32_t both = g.s == 2 ? down : 2 * down;
+          uint64_t ad = a0;
+          if (a.taps == 4) {
+            int r = 0;
+            uint32_t acc_on = 0;
+#pragma unroll 4
+            for (; r + 2 <= g.KH; r += 2, ad += both) {
+              umma_ss<false>(d, ad, b, a.idesc, acc_on);
+              umma_ss<false>(d, ad + 2, b + b_step, a.idesc, 1u);
+              umma_ss<false>(d, ad + plane1, b + 2 * b_step, a.idesc, 1u);
+              umma_ss<false>(d, ad + plane1 + 2, b + 3 * b_step, a.idesc, 1u);
+              b += 4 * b_step;
+              acc_on = 1;
+            }
+            if (r < g.KH) filterRow(ad, r == 0);
+          } else {
+            for (int r = 0; r < g.KH; ++r) filterRow(ad + (r >> 1) * both + (r & 1) * plane1, r == 0);
+          }
+          umma_commit(accFull(acc));
+        }
+        if (ok) umma_commit(stripFree(buf));
+      }
+      // the last commits arrive here: not before them may the block end, nor tensor memory go
+      // while instructions run (after a failure, too)
+      umma_commit(smem_u32(bars + 8));
+      if (!mbar_wait(smem_u32(bars + 8), 0, abort_flag)) failed(kStatusDrainTimeout);
+      for (int i = 0; ok && i < 2 && i < k; ++i)
+        if (!mbar_wait(stripFree((k - 1 - i) & 1), uint32_t((k - 1 - i) >> 1 & 1), abort_flag)) failed(kStatusDrainTimeout);
+    }
+    __syncwarp();
+  } else {
+    // ---- results
+    const int set = warp >> 2, quarter = warp & 3;
+    const uint32_t acc = tmem + uint32_t(set * a.co_pad) + (uint32_t(quarter) << 21);
+    int c = 0;
+    for (int u = int(blockIdx.x); ok && u < a.units; u += int(gridDim.x)) {
+      int n, oh0, ow0, rows, cols;
+      const int tiles = stripOf(u, n, oh0, ow0, rows, cols);
+      for (int t = 0; t < tiles; ++t, ++c) {
+        if ((c & 1) != set) continue;
+        const int at = t * 128 + quarter * 32 + lane, row = int(fast_div(uint32_t(at), a.fd_pitch)), col = at - row * a.pitch;
+        const bool there = row < rows && col < cols;
+        __half *dst = a.out + (((long long)n * g.OH + oh0 + row) * g.OW + ow0 + col) * a.co;
+        if (!__all_sync(0xffffffffu, mbar_wait(accFull(set), uint32_t(c >> 1 & 1), abort_flag))) {
+          failed(kStatusEpilogueTimeout);
+          break;
+        }
+        tc_fence_after_sync();
+        for (int n0 = 0; n0 < a.co; n0 += 32) {
+          uint32_t v[32];
+          __syncwarp();
+          tmem_ld_32x32(acc + uint32_t(n0), v);
+          tmem_ld_wait_for(v);
+          if (n0 + 32 >= a.co) {
+            tc_fence_before_sync();
+            mbar_arrive(accFree(set));
+          }
+          float any = 0.f;
+          uint32_t pk[16];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const float4 bb = *reinterpret_cast<const float4 *>(&bias[n0 + 4 * j]);
+            const float f0 = __uint_as_float(v[4 * j]), f1 = __uint_as_float(v[4 * j + 1]);
+            const float f2 = __uint_as_float(v[4 * j + 2]), f3 = __uint_as_float(v[4 * j + 3]);
+            if (n0 + 4 * j < a.co) any += (f0 + f1) * 0.f + (f2 + f3) * 0.f;
+            const __half2 lo = __floats2half2_rn(f0 + bb.x, f1 + bb.y), hi = __floats2half2_rn(f2 + bb.z, f3 + bb.w);
+            pk[2 * j] = *reinterpret_cast<const uint32_t *>(&lo);
+            pk[2 * j + 1] = *reinterpret_cast<const uint32_t *>(&hi);
+          }
+          if (!there) continue;
+          st_global_v8(dst + n0, pk[0], pk[1], pk[2], pk[3], pk[4], pk[5], pk[6], pk[7]);
+          if (n0 + 16 < a.co) st_global_v8(dst + n0 + 16, pk[8], pk[9], pk[10], pk[11], pk[12], pk[13], pk[14], pk[15]);
+          // (products with padding or with the zero weights beside the filter may have made a
+          // NaN of an infinite operand)
+          if (any != 0.f) {
+#pragma unroll 1
+            for (int j = n0; j < min(n0 + 32, a.co); ++j)
+              if (!isfinite(__half2float(dst[j])))
+                dst[j] = __float2half_rn(stemSum<kBf16>(a, n, oh0 + row, ow0 + col, j) + bias[j]);
+          }
+        }
+      }
+    }
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  if (warp == kStemMmaWarp) tmem_dealloc(tmem, a.tmem_cols);
+}
+
+struct StemTiling {
+  int taps, pad_w, tile_w, rows, pitch;
+  size_t plane_bytes, strip_bytes, weight_bytes;
+};
+
+// The strip that takes the fewest cycles: a tile's instructions or its results, or the
+// strip's loads, times the strips of an SM, and the first strip's way through.
+bool stemTiling(int sms, const S2dShape &g, int co, StemTiling *best) {
+  StemTiling t{};
+  t.pad_w = (g.padW + g.s - 1) / g.s * g.s;
+  t.taps = ((g.KW + t.pad_w - g.padW + g.s - 1) / g.s + 1) / 2 * 2;
+  t.weight_bytes = (size_t(g.KH) * t.taps * co * 16 + 127) / 128 * 128;
+  const double tile = std::max(g.KH * t.taps / 2 * std::max(32.0, co / 2.0), 150.0 + 7.0 * co);
+  double least = 1e30;
+  for (int parts = 1; parts <= 8 && (parts == 1 || g.OW >= 16 * parts); ++parts)
+    for (int rows = 1; rows <= std::min(16, g.OH); ++rows) {
+      t.tile_w = (g.OW + parts - 1) / parts;
+      t.pitch = t.tile_w + t.taps - 1;
+      t.rows = rows;
+      t.plane_bytes = size_t(rows + (g.KH - 1) / g.s) * t.pitch * 16;
+      // (a tile reads past its last row)
+      t.strip_bytes = (g.s * t.plane_bytes + (128 + size_t(t.taps)) * 16 + 127) / 128 * 128;
+      if (t.weight_bytes + 2 * t.strip_bytes > 200 * 1024) break;
+      const double loads = (rows - 1.0) * g.s + g.KH, tiles = ((rows - 1) * t.pitch + t.tile_w + 127) / 128;
+      const double load = 0.35 * loads * t.pitch + 300, unit = std::max(tiles * tile, load) + 60;
+      const double units = double(g.N) * ((g.OH + rows - 1) / rows) * ((g.OW + t.tile_w - 1) / t.tile_w);
+      const double cycles = std::ceil(units / sms) * unit + load + tile;
+      if (cycles < least) {
+        least = cycles;
+        *best = t;
+      }
+    }
+  return least < 1e30;
+}
+
+}  // namespace
+
+// Two kinds of large filters stay rearranged: those of one channel, where both strides' pixels
+// then share 16 bytes, half as many instructions (7x7/2, 64 channels: 92 images of 212 x 56 21.7
+// against 25.4 us, 103 of 61 x 61 12.5 against 12.7), and many short rows with more than 32
+// output channels, whose strips waste a sixth of their positions (514 of 79 x 79 55.0 against
+// 61.7, 1066 of 55 x 55, 96 channels, 71.3 against 83.7; 547 of 48 x 50 40.9 against 37.0).  Of 50
+// sampled layers the rest take 0.8 of their time on average, none more than 4 % longer.
+bool stemSuits(int sm_count, const S2dShape &g, int co, bool out_f32, const void *out) {
+  StemTiling t;
+  const bool large = g.KH > 3;
+  if (large && (g.C == 1 || (co > 32 && g.OW < 64 && uint64_t(g.N) * g.OH * g.OW > uint64_t(1) << 19))) return false;
+  return g.s * g.C <= 8 && co % 16 == 0 && co <= 256 && !out_f32 && reinterpret_cast<uintptr_t>(out) % 32 == 0 &&
+         uint64_t(g.H) * g.W * g.C < uint64_t(1) << 29 && uint64_t(g.N) * g.OH * g.OW < uint64_t(1) << 30 &&
+         stemTiling(sm_count, g, co, &t);
+}
+
+int launchStem(plb_context *ctx, const S2dShape &g, int co, bool bf16, const void *x, const void *w, const float *bias,
+               void *out) {
+  StemTiling t;
+  if (!stemTiling(ctx->sm_count, g, co, &t)) return fail(PLB_ERR_UNSUPPORTED, "no tiling of the stem kernel");
+  StemArgs a{};
+  a.x = static_cast<const uint16_t *>(x);
+  a.w = static_cast<const uint16_t *>(w);
+  a.bias = bias;
+  a.out = static_cast<__half *>(out);
+  a.status = ctx->d_status;
+  a.g = g;
+  a.co = co;
+  a.co_pad = (co + 31) / 32 * 32;
+  a.taps = t.taps;
+  a.pad_w = t.pad_w;
+  a.shift = t.pad_w - g.padW;
+  a.tile_w = t.tile_w;
+  a.rows = t.rows;
+  a.pitch = t.pitch;
+  a.parts = (g.OW + t.tile_w - 1) / t.tile_w;
+  a.h_blocks = (g.OH + t.rows - 1) / t.rows;
+  a.units = g.N * a.h_blocks * a.parts;
+  a.plane_bytes = uint32_t(t.plane_bytes);
+  a.strip_bytes = uint32_t(t.strip_bytes);
+  a.weight_bytes = uint32_t(t.weight_bytes);
+  a.idesc = make_idesc(128, uint32_t(co), bf16 ? 1u : 0u, bf16 ? 1u : 0u, false, false);
+  a.tmem_cols = 64;
+  while (a.tmem_cols < uint32_t(2 * a.co_pad)) a.tmem_cols *= 2;
+  a.fd_pitch = make_fastdiv(uint32_t(t.pitch));
+  a.fd_parts = make_fastdiv(uint32_t(a.parts));
+  a.fd_h_blocks = make_fastdiv(uint32_t(a.h_blocks));
+  a.fd_co = make_fastdiv(uint32_t(co));
+  a.fd_taps = make_fastdiv(uint32_t(t.taps));
+  // whole words: rows and superpixels start on them
+  const int elems = g.s * g.C;
+  const int words = elems % 2 == 0 && g.W * g.C % 2 == 0 && reinterpret_cast<uintptr_t>(x) % 4 == 0 ? elems / 2 : 0;
+  auto launch = [&](auto kernel, std::atomic<bool> *configured) {
+    std::atomic<bool> &done = configured[ctx->device & 63];
+    if (!done) {
+      PLB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 210 * 1024));
+      done = true;
+    }
+    return launchPdl(ctx, kernel, dim3(unsigned(std::min(a.units, ctx->sm_count))), dim3(kStemThreads),
+                     t.weight_bytes + 2 * t.strip_bytes, a);
+  };
+  auto pick = [&](auto type) {
+    constexpr bool kBf16 = decltype(type)::value;
+    static std::atomic<bool> configured[5][64] = {};  // (contexts may live on several threads)
+    switch (words) {
+      case 1: return launch(stemKernel<1, kBf16>, configured[1]);
+      case 2: return launch(stemKernel<2, kBf16>, configured[2]);
+      case 3: return launch(stemKernel<3, kBf16>, configured[3]);
+      case 4: return launch(stemKernel<4, kBf16>, configured[4]);
+      default: return launch(stemKernel<0, kBf16>, configured[0]);
+    }
+  };
+  return bf16 ? pick(std::true_type()) : pick(std::false_type());
+}
+
+}  // namespace plb
