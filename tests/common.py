@@ -75,6 +75,7 @@ def empty_dev(shape, dtype):
     t = torch.empty(shape, dtype=td, device="cuda")
     if t.numel():
         t.view(torch.uint8).fill_(0x7D)
+        torch.cuda.synchronize()  # torch's stream: a late fill would poison what the library has written
     return t
 
 
