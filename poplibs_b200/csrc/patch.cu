@@ -45,7 +45,9 @@ bool shapeOf(const IgemmProblem *p, int n, int type, Shape *s) {
     s->first_h = std::min(s->first_h, -p[i].pad_h);
     s->first_w = std::min(s->first_w, -p[i].pad_w);
   }
-  if (s->first_h == 1 << 30) s->first_h = s->first_w = 0;
+  // (no filter tap reaches any output, or there are no channels: nothing to multiply, and the
+  // general route clears the outputs or refuses the layer)
+  if (s->weight_chunks == 0) return false;
   for (int i = 0; i < n; ++i) {
     if (s->chunks[i] == 0) continue;
     s->reach_h = std::max(s->reach_h, -p[i].pad_h + (p[i].taps_h - 1) * p[i].dil_h - s->first_h);

@@ -241,6 +241,16 @@ def test_plans_describe_the_operands_that_are_read():
     assert capi.matmul_plan(capi.MatmulDesc.make(512, 1024, 1024)).workspace_bytes == 0
 
 
+@pytest.mark.parametrize("t", [capi.HALF, capi.FLOAT, capi.QUARTER])
+def test_gradients_that_no_tap_reaches_are_cleared(t):
+    """Input gradients of strided layers whose filter meets padding alone: there is no product
+    for a kernel to form."""
+    kw = dict(groups=4, input_type=t, output_type=capi.FLOAT if t == capi.FLOAT else capi.HALF, stride=2)
+    for p in (capi.ConvParams.make(2, [1, 1], [1, 1], 8, 8, padding=1, **kw),
+              capi.ConvParams.make(2, [1, 9], [1, 3], 8, 8, in_pad_lo=[1, 1], in_pad_hi=[1, 1], **kw)):
+        assert capi.conv_plan(p, capi.PASS_TRAINING_BWD).kernel == 0
+
+
 def test_fused_all_reduce_needs_no_flags_for_layers_it_refuses():
     flags = lambda t: capi.lib().plb_conv_wu_allreduce_flag_bytes(
         C.byref(capi.ConvParams.make(4, [9, 9], [3, 3], 64, 64, padding=1, input_type=t, output_type=t)))

@@ -71,6 +71,24 @@ def test_layers(gpu_ctx, general_ctx, name, dtype):
         assert (got.astype(np.float64) == want.reshape(got.shape)).all(), "input gradient"
 
 
+@pytest.mark.parametrize("dtype", sorted(TYPES))
+@pytest.mark.parametrize("groups", [1, 4, 32])
+def test_gradients_that_no_tap_reaches_are_zero(gpu_ctx, dtype, groups):
+    """Strided layers whose filter meets padding alone have nothing to multiply; layers without
+    output channels are refused."""
+    plb, np_type = TYPES[dtype]
+    kw = dict(groups=groups, input_type=plb, output_type=capi.FLOAT if dtype == "float" else capi.HALF)
+    for field, kernel in (((1, 1), (1, 1)), ((1, 9), (1, 3))):
+        p = capi.ConvParams.make(2, list(field), list(kernel), 8, 8, stride=2, padding=1, **kw)
+        dy, w = np.ones((2, groups * 8, *p.output_field()), np_type), np.ones((groups, 8, 8, *kernel), np_type)
+        assert (T.gpu_conv_bwd(p, dy, w) == 0).all()
+    import torch
+    none = capi.ConvParams.make(2, [6, 5], [3, 3], 8, 0, padding=1, **kw)
+    x = torch.zeros((2, 6, 5, groups * 8), dtype=torch.float32, device="cuda")
+    with pytest.raises(capi.PlbError):
+        gpu_ctx.conv_bwd(none, x, x, x)
+
+
 def test_narrow_groups_take_one_launch(gpu_ctx):
     r = T.rng(1)
     p = capi.ConvParams.make(2, [8, 13], [3, 3], 8, 8, groups=32, padding=1, stride=2)
