@@ -239,23 +239,38 @@ int planIgemm(const IgemmProblem &p, int sm_count, plb_plan *plan) {
     const long steps = plan->halo_rows > 0 ? long(p.taps_w) * ((p.k_per_tap + k_elems - 1) / k_elems)
                                            : k_iters;
     const long sms = sm_count > 0 ? sm_count : 148;
-    int split = 1;
-    if (p.force_split_k > 0) {
-      split = int(std::min<long>(p.force_split_k, steps));
-    } else if (const int b_tiles = plan->halo_rows > 0 && !plan->resident_weights ? p.taps_h : 1;
-               units * 2 <= sms && steps * b_tiles >= 20 && !(plan->resident_weights && groups > 1)) {
+    const int b_tiles = plan->halo_rows > 0 && !plan->resident_weights ? p.taps_h : 1;
+    // The cheapest split of `tiles` units of work, at most one per SM or (pairs) two per
+    // pair of SMs.
+    auto cheapest = [&](long tiles) {
+      if (tiles * 2 > sms || steps * b_tiles < 20 || (plan->resident_weights && groups > 1)) return 1;
+      int split = 1;
       const double out_mb = double(groups) * p.out_w * p.out_h * p.out_n * p.n_total * 4 / 1e6;
       const double odd_rows = (p.act_strides[0] % 32 != 0 ? 0.09 : 0.0) + (p.wgt_strides[0] % 32 != 0 ? 0.045 : 0.0);
       const double step_us = 0.15 * b_tiles + odd_rows;
       double best = step_us * double(steps);
-      for (long sp = 2; sp <= std::min<long>(steps * b_tiles / 4, std::min(steps, sms / units)); ++sp) {
+      for (long sp = 2; sp <= std::min<long>(steps * b_tiles / 4, std::min(steps, sms / tiles)); ++sp) {
         const double t = step_us * double((steps + sp - 1) / sp) + 3.4 + out_mb * double(sp + 1) / 4.0;
         if (t < best) {
           best = t;
           split = int(sp);
         }
       }
-    }
+      return split;
+    };
+    // Pairs are split where their tiles would be on single SMs.  There they run in up to
+    // two waves and are quicker for it (3x3, 512 channels, one 28 x 28 image, 28 pairs:
+    // 5 splits 12.7 us, 2 splits 14.0, unpaired 13.0).  Elsewhere the second wave, the
+    // partial sums and the second kernel cost more than the shorter ranges save (5x5, 304 -> 368
+    // channels, 11 images of 16 x 16, 66 pairs: 2 splits 23.4 us, whole 17.5, unpaired 20.7;
+    // 180 sampled passes 0.92 of their time with every pair split as the model has it, 0.85
+    // of it unpaired).  A few would still gain (5x5, 499 -> 308, 3 of 20 x 20, 38 pairs:
+    // 3 splits 26.5, whole 30.9, unpaired 36.5), but take no scratch this way.
+    int split = 1;
+    if (p.force_split_k > 0)
+      split = int(std::min<long>(p.force_split_k, steps));
+    else if (!pair || cheapest(plan->tiles) > 1)
+      split = cheapest(units);
     if (split > 1 && long(plan->tiles) * split > 0x3fffffffL) split = 1;
     plan->split_k = split;
     if (split > 1) {

@@ -173,6 +173,35 @@ def test_planner_rules_for_pairs_halo_tiles_and_padding():
     assert wide.halo_rows == 0 and wide.tile_n <= 10 * 32 and wide.stages >= 2
 
 
+def test_pairs_are_split_only_where_single_tiles_are():
+    """A layer or product that runs whole on single SMs needs no scratch for pairs either."""
+    mk = capi.ConvParams.make
+    plan = lambda p, flags=0: capi.conv_plan(p, capi.PASS_TRAINING_FWD, capi.ConvOptions.make(plan_flags=flags))
+    # more pairs than half the pair slots (74 on 148 SMs)
+    for p in (mk(11, [16, 16], [5, 5], 304, 368, padding=2), mk(14, [15, 15], [5, 5], 248, 248, padding=2),
+              mk(29, [19, 19], [3, 3], 504, 80, padding=1)):
+        got = plan(p)
+        assert (got.cta_pair, got.split_k, got.workspace_bytes) == (1, 1, 0)
+    # a long reduction on few tiles
+    few = plan(mk(1, [28, 28], [3, 3], 512, 512, padding=1))
+    assert (few.cta_pair, few.split_k) == (1, 5)
+    long = capi.matmul_plan(capi.MatmulDesc.make(488, 4312, 3992, transpose_b=True))
+    assert (long.cta_pair, long.split_k, long.workspace_bytes) == (1, 1, 0)
+    r = np.random.default_rng(7)
+    split = 0
+    for _ in range(400):
+        chans_in, chans_out = (8 * int(r.integers(4, 64)) for _ in range(2))
+        field = [int(r.integers(7, 60)) for _ in range(2)]
+        kernel = int(r.choice([3, 5]))
+        p = mk(int(r.integers(1, 16)), field, [kernel] * 2, chans_in, chans_out, padding=kernel // 2)
+        got, single = plan(p), plan(p, capi.PLAN_NO_CTA_PAIR)
+        if got.cta_pair:
+            assert got.split_k == 1 or single.split_k > 1
+            assert got.workspace_bytes == 0 or single.workspace_bytes > 0
+            split += got.split_k > 1
+    assert split > 0
+
+
 def test_forced_resident_weights_with_splits_and_groups():
     """Residency that is asked for is kept with a forced K split, and with any number of
     groups that run side by side; with groups only one of the two is possible."""

@@ -401,6 +401,21 @@ def test_conv_split_k_agrees_with_oracle(gpu_ctx, name, variant, split):
                  f"fwd fp32 + bias {name} {variant} /{split}")
 
 
+@pytest.mark.parametrize("images,field,chans", [(10, (13, 19), (72, 72)), (22, (10, 26), (72, 64))])
+def test_pairs_split_by_the_planner(gpu_ctx, images, field, chans):
+    """More pieces of a reduction than CTA pairs that run at once (each takes several), with and
+    without halo strips, with an odd number of pixel tiles."""
+    mk = lambda n: capi.ConvParams.make(n, list(field), [5, 5], *chans, padding=2)
+    plan = capi.conv_plan(mk(images), capi.PASS_TRAINING_FWD)
+    assert plan.cta_pair and (plan.tiles + 1) // 2 * plan.split_k > 74
+    r = T.rng(chans[1])
+    x, w = T.binary_half(r, (images, chans[0], *field)), T.binary_half(r, (1, chans[1], chans[0], 5, 5))
+    got = T.gpu_conv_fwd(mk(images), x, w)
+    single = T.gpu_conv_fwd(mk(images), x, w, opt=capi.ConvOptions.make(plan_flags=capi.PLAN_NO_CTA_PAIR))
+    assert_exact(got, single, "pairs and single CTAs")
+    assert_exact(got[-2:], oracle.conv_fwd(T.spec_from_params(mk(2)), x[-2:], w), "last images")
+
+
 def test_matmul_long_k_is_split_by_the_planner(gpu_ctx):
     """Few output tiles and a long reduction: the planner gives each tile to
     several CTAs by itself; results stay exact, also with alpha, beta and C."""
