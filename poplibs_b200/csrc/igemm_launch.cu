@@ -119,8 +119,12 @@ int planIgemm(const IgemmProblem &p, int sm_count, plb_plan *plan) {
   //    4 images of 29x20, 60 tiles: 7.2 -> 6.3); not short tiles of 64 columns in a second
   //    wave that is mostly empty (3x3, 48 channels, 42 images of 8x84, 231 tiles: 8.7 -> 9.2;
   //    11 sampled layers 5 % slower);
-  //  - products of more than a wave of tiles (2048 x 4096 x 4096, 256 tiles: 65 -> 60 us);
-  //  - products whose rows start at odd multiples of 16 bytes, which take the copy engine
+  //  - more than a wave of wide tiles, whatever the taps, stride and groups: products
+  //    (2048 x 4096 x 4096, 256 tiles: 65 -> 60 us), strided filters (3x3/2, 128 channels, 32
+  //    images of 56x56, 196 tiles: 13.0 -> 12.0; 256 channels, 12 of 56x56, 168 tiles: 17.4 ->
+  //    16.5), groups (3x3, 2 groups of 128, 12 of 28x28, 168 tiles: 11.4 -> 9.2); 63 sampled
+  //    strided and grouped layers 0.86 of their time, one 5 % longer;
+  //  - wide tiles whose rows start at odd multiples of 16 bytes, which take the copy engine
   //    longer (1500 x 3000 x 3000, 144 tiles: 39 -> 31 us; with whole lines, 2238 x 1216 x
   //    1792, 126 tiles: 11.2 -> 11.9).
   const int k_elems_stage = kStageKBytes / elem;
@@ -132,13 +136,13 @@ int planIgemm(const IgemmProblem &p, int sm_count, plb_plan *plan) {
   const bool odd_rows = p.act_strides[0] % 32 != 0 || p.wgt_strides[0] % 32 != 0;
   const bool several_taps = p.taps_h > 1 && p.stride_h == 1 && groups == 1 && k_steps_per_tile >= 8 && units_single >= 48 &&
                             !(bn <= 64 && k_steps_per_tile < 16 && units_single > sms_for_pair);
-  const bool one_tap = bn >= 128 && k_steps_per_tile >= 7 &&
-                       (units_single > sms_for_pair || (odd_rows && 2 * units_single >= sms_for_pair));
+  const bool wide_tiles = bn >= 128 && k_steps_per_tile >= 7 &&
+                          (units_single > sms_for_pair || (odd_rows && 2 * units_single >= sms_for_pair));
   const bool pair = (p.plan_flags & PLB_PLAN_NO_CTA_PAIR) == 0 && (!p.b_mn || bn >= 128) &&
                     ((p.plan_flags & PLB_PLAN_FORCE_CTA_PAIR) != 0
                          ? best_tiles >= 2
                          : (k_steps_per_tile >= (bn >= 256 ? 4 : 8) && units_single >= 2 * sms_for_pair) ||
-                               (best_tiles >= 2 && no_more_waves && (several_taps || one_tap)));
+                               (best_tiles >= 2 && no_more_waves && (several_taps || wide_tiles)));
   plan->cta_pair = pair ? 1 : 0;
   auto grid_for = [&](long m_tiles) {
     const int sms = sm_count > 0 ? sm_count : 148;

@@ -173,6 +173,15 @@ def test_planner_rules_for_pairs_halo_tiles_and_padding():
     assert wide.halo_rows == 0 and wide.tile_n <= 10 * 32 and wide.stages >= 2
 
 
+def test_pairs_of_wide_tiles_from_a_wave_on():
+    """More than a wave (148) of tiles of 128 columns is paired whatever the stride and the groups."""
+    for batch, side, chans, kw, paired in ((32, 56, 128, dict(stride=2), True), (12, 56, 256, dict(stride=2), True),
+                                           (12, 28, 128, dict(groups=2), True), (5, 59, 392, dict(stride=2), True),
+                                           (2, 59, 392, dict(stride=2), False), (32, 40, 128, dict(stride=2), False)):
+        plan = capi.conv_plan(capi.ConvParams.make(batch, [side, side], [3, 3], chans, chans, padding=1, **kw))
+        assert (plan.tiles > 148, plan.cta_pair, plan.split_k) == (paired, paired, 1)
+
+
 def test_pairs_are_split_only_where_single_tiles_are():
     """A layer or product that runs whole on single SMs needs no scratch for pairs either."""
     mk = capi.ConvParams.make
