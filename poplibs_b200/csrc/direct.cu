@@ -100,6 +100,9 @@ float igemmTime(int sm_count, const IgemmProblem &p, int type, bool copied) {
 // leaves, a few would gain up to 10 %.
 bool directSuits(int sm_count, const IgemmProblem &p, int type, bool copied) {
   if (p.plan_flags != 0 || (type != PLB_HALF && type != PLB_FLOAT && type != PLB_QUARTER)) return false;
+  // (pitches that no tensor map holds, negative ones among them, are the general route's to refuse)
+  const uint64_t pitch_limit = uint64_t(1) << 40;
+  if (std::max({p.act_strides[0], p.act_strides[1], p.wgt_strides[0], p.wgt_strides[1]}) >= pitch_limit) return false;
   if (2.0 * std::max(1, p.groups) * p.out_w * double(p.n_total) * p.k_per_tap > 1e9) return false;
   float us = 0.f;
   directShape(sm_count, p, type, &us);

@@ -289,6 +289,17 @@ def test_gradients_that_no_tap_reaches_are_cleared(t):
         assert capi.conv_plan(p, capi.PASS_TRAINING_BWD).kernel == 0
 
 
+def test_products_of_impossible_pitches_keep_the_general_route():
+    """Negative leading dimensions, and those beyond a tensor map's, are refused there."""
+    for t, transpose_b, fields in ((capi.HALF, True, ("lda", "ldb")), (capi.HALF, False, ("lda", "ldb")),
+                                   (capi.QUARTER, False, ("lda",))):
+        for field in fields:
+            for pitch, kernel in ((0, 3), (272, 3), (-256, 0), (2 ** 39, 0)):
+                d = capi.MatmulDesc.make(16, 256, 128, input_type=t, transpose_b=transpose_b)
+                setattr(d, field, pitch)
+                assert capi.matmul_plan(d).kernel == kernel
+
+
 def test_fused_all_reduce_needs_no_flags_for_layers_it_refuses():
     flags = lambda t: capi.lib().plb_conv_wu_allreduce_flag_bytes(
         C.byref(capi.ConvParams.make(4, [9, 9], [3, 3], 64, 64, padding=1, input_type=t, output_type=t)))

@@ -94,6 +94,16 @@ def test_scaled_and_added(gpu_ctx, n, out):
     assert (got == 2 * (av @ bv) - 3 * cv).all()
 
 
+def test_impossible_pitches_are_refused(gpu_ctx):
+    import torch
+    x = torch.zeros(16 * 512, dtype=torch.float16, device="cuda")
+    for field in ("lda", "ldb"):
+        d = capi.MatmulDesc.make(16, 512, 16, transpose_b=True)
+        setattr(d, field, -512)
+        with pytest.raises(capi.PlbError):
+            gpu_ctx.matmul(d, x, x, None, x)
+
+
 def test_ragged_products_take_one_launch(gpu_ctx):
     r = T.rng(3)
     for dtype, n in ((np.float16, 181), (np.float32, 64), (np.float32, 61)):
