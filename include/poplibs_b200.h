@@ -521,10 +521,8 @@ PLB_API int plb_timer_stop(plb_context *ctx, float *milliseconds);
 /* poplin::reportPlanInfo prints, include/poplin/Convolution.hpp:584-594).    */
 /* ------------------------------------------------------------------------ */
 typedef struct plb_plan {
-  int32_t kernel;      /* 0 = implicit GEMM (fwd/bwd/matmul), 1 = weight update, 2 = small-channel,
-                          3 = a small product or layer that reads its operands where they lie: it
-                          takes no workspace, and the tiling below is what it runs with under plan
-                          flags and constraints */
+  int32_t kernel;      /* 0 = implicit GEMM (fwd/bwd/matmul), 1 = weight update, 2 = few input
+                          channels, 3 = a small product or layer (see in_place) */
   int32_t tile_m;      /* output pixels (rows) per CTA tile                  */
   int32_t tile_n;      /* output channels (columns) per CTA tile             */
   int32_t tile_k_bytes;/* bytes of K per pipeline stage                      */
@@ -538,7 +536,10 @@ typedef struct plb_plan {
   int32_t halo_rows;   /* extra input rows per activation load that let one load
                           serve every vertical filter tap (0 = one load per tap) */
   int32_t cta_pair;    /* 1 = clusters of two CTAs share 256-row tensor-core instructions */
-  int32_t reserved;
+  int32_t in_place;    /* 1 = one launch that reads the operands where they lie and takes no
+                          workspace (kernel 3, and kernel 2 without the rearranged input); the
+                          tiling and workspace here are then what the call has under plan flags
+                          and constraints, or with a result that is not 32-byte aligned */
   uint64_t flops;      /* 2 * MACs (padding excluded)                        */
   uint64_t bytes;      /* operands read once + output written once           */
   uint64_t workspace_bytes;

@@ -125,7 +125,7 @@ class Plan(C.Structure):
                 ("box_n", C.c_int32), ("stages", C.c_int32), ("split_k", C.c_int32),
                 ("grid", C.c_int32), ("tiles", C.c_int32), ("b_mn_major", C.c_int32),
                 ("resident_weights", C.c_int32), ("halo_rows", C.c_int32), ("cta_pair", C.c_int32),
-                ("reserved", C.c_int32), ("flops", C.c_uint64), ("bytes", C.c_uint64), ("workspace_bytes", C.c_uint64)]
+                ("in_place", C.c_int32), ("flops", C.c_uint64), ("bytes", C.c_uint64), ("workspace_bytes", C.c_uint64)]
 
     def as_dict(self):
         return {n: int(getattr(self, n)) for n, _ in self._fields_}

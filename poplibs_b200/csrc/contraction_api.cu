@@ -723,6 +723,16 @@ bool fwdOnPatches(int sm_count, const plb_conv_params &p, const plb_conv_options
   const bool packed = p.groups == 1 && p.input_type != PLB_FLOAT && !swapped && !channelsFitTma(p, p.in_chans_per_group);
   return patchSuits(sm_count, r, 1, p.input_type, launches, groups, packed);
 }
+// The one-launch routes of a forward pass, tried before the others: straight from the image
+// (`shape`), or on the patch kernel (`r`).
+enum class FwdRoute { kOther, kStem, kPatch };
+FwdRoute fwdRoute(int sm_count, const plb_conv_params &p, const plb_conv_options *opt, int plan_flags, const ConvShape &s,
+                  const PassOperands &o, const float *bias, void *out, bool swapped, int groups, IgemmProblem *r, S2dShape *shape) {
+  if (is16BitFloat(p.input_type) && p.groups == 1 && !channelsFitTma(p, p.in_chans_per_group) && !swapped &&
+      stemLayer(sm_count, plan_flags, p, opt, out, shape))
+    return FwdRoute::kStem;
+  return fwdOnPatches(sm_count, p, opt, plan_flags, s, o, bias, out, swapped, groups, r) ? FwdRoute::kPatch : FwdRoute::kOther;
+}
 // (the number of problems, 0 if it does not)
 int bwdOnPatches(int sm_count, const plb_conv_params &p, const plb_conv_options *opt, int plan_flags, const ConvShape &s,
                  const PassOperands &o, void *dx, int groups, IgemmProblem *r) {
@@ -809,7 +819,10 @@ int plb_matmul_plan(const plb_matmul_desc *desc, plb_plan *plan) {
   plan->workspace_bytes += transposed + copies.bytes;
   const IgemmProblem direct = gemmProblem(*desc, nullptr, ld.a, desc->transpose_a != 0, nullptr, ld.b, desc->transpose_b != 0,
                                           nullptr, nullptr, ld.c);
-  if (directSuits(148, direct, desc->input_type, matmulCopies(*desc, nullptr, nullptr))) plan->kernel = 3;
+  if (directSuits(148, direct, desc->input_type, matmulCopies(*desc, nullptr, nullptr))) {
+    plan->kernel = 3;
+    plan->in_place = 1;
+  }
   return PLB_OK;
 }
 
@@ -957,14 +970,12 @@ int plb_conv_plan(const plb_conv_params *p_in, const plb_conv_options *opt, int3
   ConvShape s;
   if (int rc = igemmConvShape(*p, &s)) return rc;
   *plan = plb_plan{};
-  if (pass != PLB_PASS_TRAINING_BWD && p->input_type != PLB_FLOAT && !channelsFitTma(*p, p->in_chans_per_group)) {
+  const bool bwd = pass == PLB_PASS_TRAINING_BWD;
+  bool rearranged = false;
+  if (!bwd && p->input_type != PLB_FLOAT && !channelsFitTma(*p, p->in_chans_per_group)) {
     const int rc = convFwdSmallChannels(nullptr, *p, opt, nullptr, nullptr, nullptr, nullptr, plan);
-    if (rc == PLB_OK) {
-      plan->flops = 2 * numberOfMacs(*p);
-      plan->bytes = convBytes(*p, s, pass);
-      return PLB_OK;
-    }
-    if (rc != PLB_ERR_UNSUPPORTED) return rc;
+    rearranged = rc == PLB_OK;
+    if (!rearranged && rc != PLB_ERR_UNSUPPORTED) return rc;
   }
   // narrow groups run together; channel counts TMA cannot address and float operands on copies
   plb_conv_params run = *p;
@@ -972,10 +983,10 @@ int plb_conv_plan(const plb_conv_params *p_in, const plb_conv_options *opt, int3
   run.groups /= together;
   run.in_chans_per_group *= together;
   run.out_chans_per_group *= together;
-  const bool bwd = pass == PLB_PASS_TRAINING_BWD, transposed = bwd && run.input_type == PLB_QUARTER;
+  const bool transposed = bwd && run.input_type == PLB_QUARTER;
   const uint64_t tiles = uint64_t(run.groups) * s.KHs * s.KWs, pixels = uint64_t(run.batch) * run.groups;
   const uint32_t ci = run.in_chans_per_group, co = run.out_chans_per_group;
-  if (run.batch != 0 && run.groups != 0 && ci != 0 && co != 0 && s.KH > 0 && s.KW > 0 && s.OHc > 0 && s.OWc > 0 &&
+  if (!rearranged && run.batch != 0 && run.groups != 0 && ci != 0 && co != 0 && s.KH > 0 && s.KW > 0 && s.OHc > 0 && s.OWc > 0 &&
       s.He > 0 && s.We > 0) {
     PassOperands o;
     Repack::Lattice sub{};
@@ -997,9 +1008,14 @@ int plb_conv_plan(const plb_conv_params *p_in, const plb_conv_options *opt, int3
     IgemmProblem r[kPatchMaxPhases];
     const PassOperands o{p->input_type, nullptr, nullptr, bwd ? p->out_chans_per_group : p->in_chans_per_group,
                          bwd ? p->out_chans_per_group : p->in_chans_per_group, p->in_chans_per_group};
-    if (bwd ? bwdOnPatches(148, *p, opt, 0, s, o, nullptr, int(together), r) > 0
-            : fwdOnPatches(148, *p, opt, 0, s, o, nullptr, nullptr, false, int(together), r))
-      plan->kernel = 3;
+    S2dShape g;
+    FwdRoute route = FwdRoute::kOther;
+    if (!bwd)
+      route = fwdRoute(148, *p, opt, 0, s, o, nullptr, nullptr, false, int(together), r, &g);
+    else if (bwdOnPatches(148, *p, opt, 0, s, o, nullptr, int(together), r) > 0)
+      route = FwdRoute::kPatch;
+    if (route == FwdRoute::kPatch) plan->kernel = 3;
+    plan->in_place = route == FwdRoute::kOther ? 0 : 1;
   }
   plan->flops = 2 * numberOfMacs(*p);
   plan->bytes = convBytes(*p, s, pass);
@@ -1080,16 +1096,16 @@ int plb_convolution(plb_context *ctx, const plb_conv_params *p, const plb_conv_o
   // the caller's operands, the groups apart
   const PassOperands separate{p->input_type, d_in, d_weights, p->in_chans_per_group, p->in_chans_per_group,
                               swapped ? p->out_chans_per_group : p->in_chans_per_group};
-  if (is16BitFloat(p->input_type) && p->groups == 1 && !channelsFitTma(*p, p->in_chans_per_group) && !swapped) {
-    S2dShape g;
-    if (stemLayer(ctx, *p, opt, d_out, &g))
-      return launchStem(ctx, g, int(p->out_chans_per_group), p->input_type == PLB_BFLOAT16, d_in, d_weights, d_bias, d_out);
-  }
   {
     IgemmProblem r;
+    S2dShape g;
     const int groups = groupsTogether(p->groups, p->in_chans_per_group, p->out_chans_per_group, p->input_type);
-    if (fwdOnPatches(ctx->sm_count, *p, opt, ctx->plan_flags, s, separate, d_bias, d_out, swapped, groups, &r))
-      return launchPatch(ctx, &r, 1, p->input_type, groups > 1);
+    switch (fwdRoute(ctx->sm_count, *p, opt, ctx->plan_flags, s, separate, d_bias, d_out, swapped, groups, &r, &g)) {
+      case FwdRoute::kStem:
+        return launchStem(ctx, g, int(p->out_chans_per_group), p->input_type == PLB_BFLOAT16, d_in, d_weights, d_bias, d_out);
+      case FwdRoute::kPatch: return launchPatch(ctx, &r, 1, p->input_type, groups > 1);
+      default: break;
+    }
   }
   if (p->input_type != PLB_FLOAT && !channelsFitTma(*p, p->in_chans_per_group) && !transpose_and_flip_weights) {
     // few input channels (a stem): space-to-depth path, where it applies

@@ -601,12 +601,18 @@ void addBias(Graph &graph, const Tensor &acts, const Tensor &biases, Sequence &p
 }
 
 // ---- plan reporting ------------------------------------------------------------------------
+static std::size_t workspaceOf(const plb_plan &plan) {
+  return plan.in_place ? 0 : std::size_t(plan.workspace_bytes);
+}
+
 static void printPlan(std::ostream &out, const plb_plan &plan, const char *pass) {
   static const char *kernels[] = {"implicit GEMM (TMA + tcgen05)", "weight update (split-K)",
                                   "small-channel (space-to-depth + implicit GEMM)",
                                   "operands where they lie (mma.sync)"};
+  const char *kernel = plan.kernel == 2 && plan.in_place ? "small-channel (image as it is, tcgen05)"
+                                                         : kernels[std::min(std::max(plan.kernel, 0), 3)];
   out << "  Plan (" << pass << "):\n"
-      << "        kernel                     " << kernels[std::min(std::max(plan.kernel, 0), 3)] << "\n"
+      << "        kernel                     " << kernel << "\n"
       << "        CTA tile (pixels x chans)  " << plan.tile_m << " x " << plan.tile_n << "\n"
       << "        pixel box (w, h, n)        {" << plan.box_w << "," << plan.box_h << ","
       << plan.box_n << "}\n"
@@ -619,7 +625,7 @@ static void printPlan(std::ostream &out, const plb_plan &plan, const char *pass)
       << "        halo rows per load         " << plan.halo_rows << "\n"
       << "        CTA pair (256-row MMA)     " << plan.cta_pair << "\n"
       << "        right operand MN-major     " << (plan.b_mn_major ? "yes" : "no") << "\n"
-      << "        workspace bytes            " << plan.workspace_bytes << "\n"
+      << "        workspace bytes            " << workspaceOf(plan) << "\n"
       << "        FLOPs (padding excluded)   " << plan.flops << "\n"
       << "        bytes (operands + output)  " << plan.bytes << "\n";
 }
@@ -659,7 +665,7 @@ PlanCosts reportPlanEstimatedCosts(const Graph &, const ConvParams &params,
   const double computeCycles = double(plan.flops) / (8192.0 * 148.0);
   const double memoryCycles = double(plan.bytes) / (3.5 * 148.0);
   c.cycles = std::size_t(std::max(computeCycles, memoryCycles));
-  c.memory = std::size_t(plan.workspace_bytes);
+  c.memory = workspaceOf(plan);
   return c;
 }
 
@@ -695,12 +701,12 @@ DetailedPlanCosts reportDetailedPlanEstimatedCosts(const Graph &graph, const Con
   const double macCycles = getFwdPerfectCycleCount(graph, params);
   c.compute.cycles = std::size_t(std::max(macCycles, memoryCycles(double(plan.bytes))));
   // reduction: split-K partial sums written once and read once by the second kernel
-  if (plan.split_k > 1) {
+  if (plan.split_k > 1 && !plan.in_place) {
     c.reduction.cycles = std::size_t(memoryCycles(2.0 * double(plan.workspace_bytes)));
     c.reduction.memory = std::size_t(plan.workspace_bytes);
   }
   // rearrangement: the small-channel path rewrites the activations once (space to depth)
-  if (plan.kernel == 2) {
+  if (plan.kernel == 2 && !plan.in_place) {
     double in_bytes = double(params.getBatchSize()) * double(params.getNumInputChans()) *
                       double(graph.getTarget().getTypeSize(params.inputType));
     for (std::size_t extent : params.inputFieldShape) in_bytes *= double(extent);
@@ -708,7 +714,7 @@ DetailedPlanCosts reportDetailedPlanEstimatedCosts(const Graph &graph, const Con
     c.rearrangement.memory = plan.split_k > 1 ? 0 : std::size_t(plan.workspace_bytes);
   }
   c.total.cycles = c.compute.cycles + c.reduction.cycles + c.rearrangement.cycles;
-  c.total.memory = std::size_t(plan.workspace_bytes);
+  c.total.memory = workspaceOf(plan);
   return c;
 }
 

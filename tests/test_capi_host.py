@@ -289,6 +289,27 @@ def test_gradients_that_no_tap_reaches_are_cleared(t):
         assert capi.conv_plan(p, capi.PASS_TRAINING_BWD).kernel == 0
 
 
+def test_plans_say_which_calls_read_their_operands_in_place():
+    """One launch without workspace: few input channels, narrow groups, small products; not under
+    constraints, whose tiling the plan holds."""
+    mk, opt = capi.ConvParams.make, capi.ConvOptions.make
+    route = lambda p, pass_=capi.PASS_TRAINING_FWD, o=None: (lambda q: (q.kernel, q.in_place))(capi.conv_plan(p, pass_, o))
+    first = mk(256, [224, 224], [7, 7], 3, 64, padding=3, stride=2)
+    assert route(first) == (2, 1) and capi.conv_plan(first).tile_n == 64
+    for o in (opt(tile_n=64), opt(plan_flags=capi.PLAN_NO_HALO)):
+        assert route(first, o=o) == (2, 0)
+    assert route(mk(256, [224, 224], [7, 7], 3, 64, padding=3, stride=2, output_type=capi.FLOAT)) == (2, 0)
+    # few channels in, and not 16 out
+    assert route(mk(1, [9, 9], [1, 1], 1, 4)) == (3, 1) and route(mk(64, [30, 30], [3, 3], 2, 24, padding=1)) == (2, 0)
+    groups = mk(2, [8, 13], [3, 3], 8, 8, groups=32, padding=1, stride=2)
+    assert route(groups) == route(groups, capi.PASS_TRAINING_BWD) == (3, 1)
+    assert route(groups, o=opt(split_k=1)) == (0, 0)
+    wide = mk(256, [28, 28], [3, 3], 128, 128, padding=1)
+    assert route(wide) == route(wide, capi.PASS_TRAINING_BWD) == (0, 0)
+    products = [capi.matmul_plan(capi.MatmulDesc.make(*s)) for s in ((16, 512, 512), (8192, 8192, 8192))]
+    assert [(q.kernel, q.in_place) for q in products] == [(3, 1), (0, 0)]
+
+
 def test_products_of_impossible_pitches_keep_the_general_route():
     """Negative leading dimensions, and those beyond a tensor map's, are refused there."""
     for t, transpose_b, fields in ((capi.HALF, True, ("lda", "ldb")), (capi.HALF, False, ("lda", "ldb")),
