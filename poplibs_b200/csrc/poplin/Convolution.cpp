@@ -57,8 +57,13 @@ std::string planConstraintsOf(const plb_plan &plan) {
   const bool igemm = plan.kernel != 1;
   os << "{\n"
      << "  \"0\": {\"partition\": {\"inChanSplit\": {\"serial\": 1, \"parallel\": "
-     << std::max(1, int(plan.split_k)) << "}}},\n"
-     << "  \"cuda\": {\"splitK\": " << std::max(1, int(plan.split_k));
+     << std::max(1, plan.in_place ? 1 : int(plan.split_k)) << "}}}";
+  // (any of these knobs would send such a layer to another kernel)
+  if (plan.in_place) {
+    os << "\n}\n";
+    return os.str();
+  }
+  os << ",\n  \"cuda\": {\"splitK\": " << std::max(1, int(plan.split_k));
   if (igemm)
     os << ", \"tileN\": " << plan.tile_n << ", \"residentWeights\": "
        << (plan.resident_weights ? "true" : "false") << ", \"ctaPair\": "

@@ -343,12 +343,18 @@ static void testGraphConstructionWithoutDevice() {
       CHECK(first.str() == second.str());
       std::remove((base + "_FWD.json").c_str());
     }
-    // layers that read their operands in place need no workspace: an image's first layer, narrow groups
+    // layers that read their operands in place stay there: an image's first layer, narrow groups
     for (const ConvParams &q : {ConvParams(HALF, HALF, 8, {64, 64}, {3, 3}, 3, 64, 1),
                                 ConvParams(HALF, HALF, 2, {9, 13}, {3, 3}, 8, 8, 16)}) {
-      std::ostringstream first;
-      reportPlanInfo(first, graph, q, {{"pass", "TRAINING_FWD"}});
+      std::ostringstream first, second;
+      reportPlanInfo(first, graph, q, {{"pass", "TRAINING_FWD"}, {"planConstraintsOutputFilename", base}});
       CHECK(first.str().find("implicit GEMM") == std::string::npos);
+      std::ifstream in(base + "_FWD.json");
+      std::stringstream text;
+      text << in.rdbuf();
+      reportPlanInfo(second, graph, q, {{"pass", "TRAINING_FWD"}, {"planConstraints", text.str()}});
+      CHECK(first.str() == second.str());
+      std::remove((base + "_FWD.json").c_str());
       const auto costs = internal::reportDetailedPlanEstimatedCosts(graph, q, {{"pass", "TRAINING_FWD"}});
       CHECK(costs.rearrangement.cycles == 0 && costs.total.memory == 0);
     }
