@@ -15,11 +15,20 @@ pytestmark = pytest.mark.gpu
 
 TYPES = {"half": (capi.HALF, np.float16, capi.HALF, np.float16), "float": (capi.FLOAT, np.float32, capi.FLOAT, np.float32),
          "quarter": (capi.QUARTER, np.uint8, capi.HALF, np.float16)}
-# edges of the 16, 32 and 64 wide tiles, remainders of the 64, 128 and 256 long K steps for
-# one and two teams, one row, one column, one product
+# remainders of the 64, 128 and 256 long K steps, one row, one column, one product; some types
+# and layouts of the larger ones take the general route
 SIZES = [(1, 1, 1, 1), (1, 16, 256, 32), (1, 17, 257, 33), (1, 15, 511, 31), (1, 33, 128, 64), (1, 31, 129, 65),
          (1, 132, 98, 181), (1, 64, 385, 7), (1, 65, 63, 129), (1, 300, 40, 280), (3, 47, 155, 85), (5, 112, 32, 48),
          (20, 33, 65, 17), (40, 64, 40, 64), (1, 16, 1030, 512), (2, 128, 576, 64), (1, 5, 3, 700)]
+# products that are direct in every layout: together they take every block (16 x 32, 32 x 32,
+# 32 x 64 and 64 x 64, with one or two teams of warps) that the planner chooses for the type
+DIRECT = {
+    "half": [(1, 8, 8, 8), (3, 280, 13, 261), (1, 4, 314, 5), (6, 40, 8, 288), (6, 197, 9, 296), (6, 196, 10, 395),
+             (6, 275, 160, 72), (6, 80, 96, 272)],
+    "float": [(1, 8, 8, 8), (2, 4, 280, 4), (6, 200, 8, 152), (6, 280, 8, 200), (6, 288, 16, 352), (6, 133, 138, 179)],
+    "quarter": [(1, 4, 21, 8), (3, 5, 213, 5), (1, 7, 389, 11), (6, 175, 15, 299), (2, 228, 147, 293), (1, 8, 25, 8),
+                (2, 8, 329, 8), (3, 8, 181, 40)],
+}
 
 
 @pytest.fixture(scope="module")
@@ -64,7 +73,7 @@ def test_small_products(gpu_ctx, general_ctx, dtype, ta, tb, pad, offset):
     plb_in, np_in, plb_out, np_out = TYPES[dtype]
     if dtype == "quarter" and (ta or not tb) and pad:
         pytest.skip("refused: transposed quarter operands are densely packed")
-    for g, m, k, n in SIZES:
+    for g, m, k, n in SIZES + DIRECT[dtype]:
         r = T.rng(m + 7 * k + n)
         av, bv = (r.integers(-2, 3, s).astype(np.float64) for s in ((g, m, k), (g, k, n)))
         want = av @ bv
@@ -75,6 +84,7 @@ def test_small_products(gpu_ctx, general_ctx, dtype, ta, tb, pad, offset):
         desc = capi.MatmulDesc.make(m, k, n, groups=g, input_type=plb_in, output_type=plb_out, transpose_a=ta,
                                     transpose_b=tb)
         desc.lda, desc.ldb, desc.ldc = lda, ldb, ldc
+        assert capi.matmul_plan(desc).kernel == 3 or (g, m, k, n) in SIZES
         got = _run(gpu_ctx, desc, a, b, None, (g, m, n), np_out, ldc, offset)
         general = _run(general_ctx, desc, a, b, None, (g, m, n), np_out, ldc, offset)
         assert (got == general).all(), (g, m, k, n)

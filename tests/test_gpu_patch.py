@@ -16,7 +16,7 @@ pytestmark = pytest.mark.gpu
 TYPES = {"half": (capi.HALF, np.float16), "float": (capi.FLOAT, np.float32), "quarter": (capi.QUARTER, np.uint8)}
 # groups, channels in / out, images, field, kernel, other parameters: one and several groups to
 # a block, chunks that are full and not, odd and even numbers of them, rows that are tiles,
-# parts and several images of one, several blocks of output channels
+# parts and several images of one, and layers of one group that stay on the general route
 LAYERS = {
     "8 to 8": (4, 8, 8, 3, (9, 7), (3, 3), dict(padding=1)),
     "32 groups": (32, 8, 8, 2, (8, 21), (3, 3), dict(padding=1)),
@@ -35,6 +35,41 @@ LAYERS = {
     "truncated": (4, 8, 8, 2, (12, 9), (3, 4), dict(k_trunc_lo=[1, 0], k_trunc_hi=[0, 1], in_trunc_lo=[1, 0], in_trunc_hi=[0, 2])),
     "padded output": (2, 8, 8, 2, (9, 9), (3, 3), dict(out_pad_lo=[1, 0], out_pad_hi=[0, 2], padding=1)),
 }
+GENERAL = [("24 to 24", "half")] + [(name, t) for name in ("one group, ragged", "one group, wide") for t in TYPES]
+# groups, channels in / out, images, field, kernel, stride, and the types (half, float, quarter)
+# whose forward pass and whose input gradient run on patches: every number of pixels (32, 64)
+# and of columns (8 to 32) of an item that the planner chooses, in one and in several blocks of
+# output channels, in each type and with the weights in either order
+SHAPES = [
+    (1, 3, 1, 1, (2, 2), 1, 2, "hfq", "hfq"),
+    (8, 15, 19, 1, (2, 2), 1, 2, "hfq", "hfq"),
+    (1, 36, 92, 4, (4, 3), 1, 2, "hfq", "hfq"),
+    (4, 1, 1, 41, (35, 31), 3, 1, "hq", "hq"),
+    (1, 59, 2, 1, (3, 2), 1, 2, "", "hfq"),
+    (2, 70, 2, 1, (4, 2), 1, 2, "h", "hfq"),
+    (1, 172, 4, 1, (2, 2), 1, 2, "hfq", "hfq"),
+    (2, 72, 4, 1, (2, 6), 1, 1, "hfq", "hfq"),
+    (16, 2, 34, 37, (7, 6), 1, 1, "hfq", ""),
+    (16, 3, 25, 37, (7, 44), 1, 2, "hfq", "hfq"),
+    (16, 4, 28, 37, (18, 13), 1, 1, "hq", "hfq"),
+    (3, 65, 1, 25, (11, 42), 3, 2, "", "q"),
+    (2, 104, 8, 34, (10, 9), 1, 1, "fq", "q"),
+    (16, 12, 2, 38, (3, 58), 7, 2, "", "hq"),
+    (2, 68, 8, 13, (22, 22), 1, 1, "h", "h"),
+    (8, 8, 12, 19, (24, 37), 1, 1, "q", ""),
+    (3, 36, 32, 54, (22, 20), 1, 2, "", "q"),
+    (8, 57, 2, 37, (32, 7), 7, 2, "", "hq"),
+    (16, 2, 22, 37, (12, 41), 3, 1, "hq", "f"),
+    (8, 1, 77, 17, (22, 16), 7, 1, "hq", ""),
+    (2, 2, 123, 37, (6, 34), 7, 1, "hq", ""),
+    (2, 178, 8, 34, (12, 37), 3, 2, "", "q"),
+    (2, 72, 8, 54, (13, 29), 5, 2, "", "hq"),
+    (3, 40, 4, 62, (14, 30), 7, 2, "", "hq"),
+    (4, 8, 96, 37, (9, 30), 5, 2, "q", "hfq"),
+    (1, 100, 3, 2, (14, 14), 3, 2, "", "hfq"),
+    (1, 8, 79, 1, (30, 11), 3, 1, "fq", ""),
+    (1, 20, 36, 2, (5, 5), 3, 2, "", "hfq"),
+]
 
 
 @pytest.fixture(scope="module")
@@ -56,6 +91,8 @@ def test_layers(gpu_ctx, general_ctx, name, dtype):
     cast = oracle.e4m3_encode if dtype == "quarter" else lambda v: v.astype(np_type)
     p = capi.ConvParams.make(images, list(field), list(kernel), ci, co, groups=groups, input_type=plb,
                              output_type=capi.FLOAT if dtype == "float" else capi.HALF, **kw)
+    for pass_ in (capi.PASS_TRAINING_FWD, capi.PASS_TRAINING_BWD):
+        assert (capi.conv_plan(p, pass_).kernel == 3) == ((name, dtype) not in GENERAL)
     spec = T.spec_from_params(p)
     r = T.rng(ci * 31 + co)
     x, w = ints(r, (images, groups * ci, *field)), ints(r, (groups, co, ci, *kernel))
@@ -69,6 +106,32 @@ def test_layers(gpu_ctx, general_ctx, name, dtype):
     for ctx in (gpu_ctx, general_ctx):
         got = T.gpu_conv_bwd(p, cast(dy), cast(w), ctx=ctx)
         assert (got.astype(np.float64) == want.reshape(got.shape)).all(), "input gradient"
+
+
+@pytest.mark.parametrize("dtype", sorted(TYPES))
+@pytest.mark.parametrize("layer", SHAPES, ids=str)
+def test_shapes_of_items_and_blocks(gpu_ctx, layer, dtype):
+    groups, ci, co, images, field, k, stride, fwd, bwd = layer
+    plb, np_type = TYPES[dtype]
+    cast = oracle.e4m3_encode if dtype == "quarter" else lambda v: v.astype(np_type)
+    p = capi.ConvParams.make(images, list(field), [k, k], ci, co, groups=groups, stride=stride, padding=k // 2,
+                             input_type=plb, output_type=capi.FLOAT if dtype == "float" else capi.HALF)
+    spec = T.spec_from_params(p)
+    r = T.rng(ci * 31 + co)
+    w = ints(r, (groups, co, ci, k, k))
+    for runs, pass_, shape, reference, run in (
+            (fwd, capi.PASS_TRAINING_FWD, (images, groups * ci, *field), oracle.conv_fwd, T.gpu_conv_fwd),
+            (bwd, capi.PASS_TRAINING_BWD, (images, groups * co, *p.output_field()), oracle.conv_bwd, T.gpu_conv_bwd)):
+        if dtype[0] not in runs:
+            continue
+        assert capi.conv_plan(p, pass_).kernel == 3
+        a = ints(r, shape)
+        want = reference(spec, a, w)
+        assert np.abs(want).max() <= 2048  # exact in half
+        before = gpu_ctx.launch_count()
+        got = run(p, cast(a), cast(w), ctx=gpu_ctx)
+        assert gpu_ctx.launch_count() == before + 1
+        assert (got.astype(np.float64) == want.reshape(got.shape)).all()
 
 
 @pytest.mark.parametrize("dtype", sorted(TYPES))
@@ -131,9 +194,12 @@ def test_float_layers_keep_their_precision(gpu_ctx, general_ctx):
 
 
 def test_wide_and_packed_layers_keep_the_general_route():
-    """Layers that the tensor cores' operand rows fill: wide channels, and few channels whose taps share a row."""
-    for p in (capi.ConvParams.make(256, [224, 224], [7, 7], 3, 64, padding=3, stride=2),
-              capi.ConvParams.make(1, [56, 56], [3, 3], 64, 64, padding=1),
+    """Layers that the tensor cores' operand rows fill: wide channels, and few channels whose taps
+    share a row (the forward pass of a first layer has a kernel of its own)."""
+    first = capi.ConvParams.make(256, [224, 224], [7, 7], 3, 64, padding=3, stride=2)
+    assert capi.conv_plan(first, capi.PASS_TRAINING_FWD).kernel == 2
+    assert capi.conv_plan(first, capi.PASS_TRAINING_BWD).kernel == 0
+    for p in (capi.ConvParams.make(1, [56, 56], [3, 3], 64, 64, padding=1),
               capi.ConvParams.make(256, [28, 28], [3, 3], 128, 128, padding=1)):
-        assert capi.conv_plan(p, capi.PASS_TRAINING_FWD).kernel != 3
-        assert capi.conv_plan(p, capi.PASS_TRAINING_BWD).kernel != 3
+        assert capi.conv_plan(p, capi.PASS_TRAINING_FWD).kernel == 0
+        assert capi.conv_plan(p, capi.PASS_TRAINING_BWD).kernel == 0
