@@ -22,15 +22,20 @@ int launchPatchInstance(plb_context *ctx, const PatchVariant &v, const PatchArgs
 
 template <int kType, bool kBMn>
 int launchPatchShape(plb_context *ctx, const PatchVariant &v, const PatchArgs &g) {
+  // (floats, two pieces of each operand in registers, keep to 32 pixels an item)
+  if constexpr (kType != PLB_FLOAT)
+    switch (v.mt * 8 + v.nt) {
+      case 4 * 8 + 1: return launchPatchInstance<kType, kBMn, 4, 1>(ctx, v, g);
+      case 4 * 8 + 2: return launchPatchInstance<kType, kBMn, 4, 2>(ctx, v, g);
+      case 4 * 8 + 3: return launchPatchInstance<kType, kBMn, 4, 3>(ctx, v, g);
+      case 4 * 8 + 4: return launchPatchInstance<kType, kBMn, 4, 4>(ctx, v, g);
+      default: break;
+    }
   switch (v.mt * 8 + v.nt) {
     case 2 * 8 + 1: return launchPatchInstance<kType, kBMn, 2, 1>(ctx, v, g);
     case 2 * 8 + 2: return launchPatchInstance<kType, kBMn, 2, 2>(ctx, v, g);
     case 2 * 8 + 3: return launchPatchInstance<kType, kBMn, 2, 3>(ctx, v, g);
     case 2 * 8 + 4: return launchPatchInstance<kType, kBMn, 2, 4>(ctx, v, g);
-    case 4 * 8 + 1: return launchPatchInstance<kType, kBMn, 4, 1>(ctx, v, g);
-    case 4 * 8 + 2: return launchPatchInstance<kType, kBMn, 4, 2>(ctx, v, g);
-    case 4 * 8 + 3: return launchPatchInstance<kType, kBMn, 4, 3>(ctx, v, g);
-    case 4 * 8 + 4: return launchPatchInstance<kType, kBMn, 4, 4>(ctx, v, g);
     default: return fail(PLB_ERR_UNSUPPORTED, "no instance of the patch kernel of this shape");
   }
 }
