@@ -719,9 +719,8 @@ bool fwdOnPatches(int sm_count, const plb_conv_params &p, const plb_conv_options
   if ((!pointwise(s) && (s.strH > 8 || s.strW > 8)) || s.KH <= 0 || s.KW <= 0) return false;
   *r = convFwdProblem(p, opt, s, o, bias, out, swapped);
   r->plan_flags |= plan_flags;
-  const int launches = 1 + (groups > 1 ? 2 : 0) + (operandsCopied(o, p.in_chans_per_group) ? 1 : 0);
   const bool packed = p.groups == 1 && p.input_type != PLB_FLOAT && !swapped && !channelsFitTma(p, p.in_chans_per_group);
-  return patchSuits(sm_count, r, 1, p.input_type, launches, groups, packed);
+  return patchSuits(sm_count, r, 1, p.input_type, 1, groups, operandsCopied(o, p.in_chans_per_group), packed);
 }
 // The one-launch routes of a forward pass, tried before the others: straight from the image
 // (`shape`), or on the patch kernel (`r`).
@@ -736,10 +735,10 @@ FwdRoute fwdRoute(int sm_count, const plb_conv_params &p, const plb_conv_options
 // (the number of problems, 0 if it does not)
 int bwdOnPatches(int sm_count, const plb_conv_params &p, const plb_conv_options *opt, int plan_flags, const ConvShape &s,
                  const PassOperands &o, void *dx, int groups, IgemmProblem *r) {
-  int n = 0, launches = 0;
+  int n = 0, contractions = 0;
   if (s.strH == 1 && s.strW == 1) {
     r[n++] = convBwdProblem(p, opt, s, o, dx, false);
-    launches = 1;
+    contractions = 1;
   } else if (s.strH * s.strW <= kPatchMaxPhases) {
     // (a phase that no tap reaches is a sum of nothing: it is cleared by the same launch;
     // the general route clears all such phases in one)
@@ -754,14 +753,13 @@ int bwdOnPatches(int sm_count, const plb_conv_params &p, const plb_conv_options 
         if (A.taps == 0 || B.taps == 0)
           clears = true;
         else
-          ++launches;
+          ++contractions;
       }
-    launches += clears ? 1 : 0;
+    contractions += clears ? 1 : 0;
   }
   if (n == 0) return 0;
   r[0].plan_flags |= plan_flags;
-  launches += (groups > 1 ? 2 : 0) + (operandsCopied(o, p.out_chans_per_group) ? 1 : 0);
-  return patchSuits(sm_count, r, n, p.input_type, launches, groups, false) ? n : 0;
+  return patchSuits(sm_count, r, n, p.input_type, contractions, groups, operandsCopied(o, p.out_chans_per_group), false) ? n : 0;
 }
 
 // Narrow channel groups are contracted together (grouped.cu): `q` = the layer of

@@ -13,7 +13,7 @@ struct Tiling {
   long tiles;
   size_t table_bytes, pixel_bytes, patch_pixel_bytes, weight_bytes, patch_bytes, smem;
   int stage_pitch, resident;
-  float us;
+  float us, us_later;
 };
 
 int ceilDiv(long a, long b) { return int((a + b - 1) / b); }
@@ -128,6 +128,14 @@ bool tilingOf(int sms, const IgemmProblem *p, int n, int type, bool vec, Tiling 
   t->us = float(1.6 + 0.0025 * t->group_block * s.weight_chunks * n8 +
                 rounds * (2.35 + 0.72 * rate * resident + 0.33 * std::max(latency - rate, 0.0) +
                           1.5 * std::ceil(loads * 1000 / (4 * kPatchThreads)) + (0.45 * loads + 1.2 * stores) * resident));
+  // and fitted to ten times as many passes, larger ones among them: with what all blocks fetch
+  // of the same weights at once from L2, and as many blocks to an SM as there are
+  const bool f = type == PLB_FLOAT;
+  const double blocks = double(sets) * columns, weights = double(t->group_block) * s.weight_chunks * n8;
+  const double fetched = blocks * weights * 64 * s.es / 1e6, shared = std::min(resident, std::max(1.0, std::ceil(blocks / sms)));
+  t->us_later = float((f ? 3.08 + 0.0088 * weights : 1.71 + 0.0046 * weights) + fetched * (p->b_mn ? 0.034 : 0.136) + 0.28 * (shared - 1) +
+                      rounds * (1.84 + 0.33 * (n - 1) + (f ? 0.794 : 0.624) * rate * shared + (f ? 1.09 : 0.49) * std::max(latency - rate, 0.0) +
+                                1.84 * std::ceil(loads * 1000 / (4 * kPatchThreads)) + (0.22 * loads + 1.34 * stores) * shared));
   return true;
 }
 
@@ -167,20 +175,42 @@ bool patchable(const IgemmProblem *p, int n, int type) {
 // 3 images of 14 x 95 8.5 -> 4.4 us; 3x3/2, 32 groups of 8, 2 of 8 x 108, input gradient 20.6 ->
 // 9.3); 32 groups of 8 on 32 images of 28 x 28 stay (17.8 against 21.2), and so do ungrouped
 // layers that are one launch (56 x 56, 64 channels: 5.3 against 11.2).
-bool patchSuits(int sm_count, const IgemmProblem *p, int n, int type, int launches, int together, bool packed) {
+// Unless the general route packs its operand rows, both times are estimated once more, fitted to
+// 4200 passes (median errors 7 and 8 %, a tenth of them 20 and 23 %): of 1800 that the first
+// estimates took, 103 were more than 8 % slower than on the general route, up to 1.7 times; the second
+// leave 26 of those, and give up 22 that gain (3x3, 2 groups of 32, 42 images of 13 x 13, where 294 blocks
+// wait for the same weights, 13.0 -> 7.5 us; 1x1, 2 groups of 32, 8 of 35 x 35 8.8 -> 5.6).
+bool patchSuits(int sm_count, const IgemmProblem *p, int n, int type, int contractions, int together, bool copied, bool packed) {
   if (!patchable(p, n, type)) return false;
   const double operand = (type == PLB_FLOAT ? 6.0 : type == PLB_QUARTER ? 1.0 : 2.0) * together * p->k_per_tap;
   const double columns = double(together) * p->n_total, wide = columns <= 64 ? 1 : columns <= 128 ? 1.6 : 2.6;
   const double tile_n = columns <= 64 ? 64 : columns <= 128 ? 128 : 256;
-  double steps = 0;
-  for (int i = 0; i < n; ++i)
-    steps += std::ceil(double(p[i].out_w) * p[i].out_h * p[i].out_n / 128) * p[i].taps_h *
-             (packed ? std::ceil(operand * p[i].taps_w / 128) : p[i].taps_w * std::ceil(operand / 128));
-  steps *= std::ceil(columns / tile_n) * wide * std::max(1, p->groups) / together;
-  const float general = float(3.4 + 2.25 * (launches - 1) + 0.134 * steps / sm_count);
+  double steps = 0, tiles = 0;
+  bool several_taps = false;
+  for (int i = 0; i < n; ++i) {
+    const double pixels = std::ceil(double(p[i].out_w) * p[i].out_h * p[i].out_n / 128);
+    tiles += pixels;
+    steps += pixels * p[i].taps_h * (packed ? std::ceil(operand * p[i].taps_w / 128) : p[i].taps_w * std::ceil(operand / 128));
+    several_taps |= p[i].taps_h * p[i].taps_w > 1;
+  }
+  const double waves = std::ceil(columns / tile_n) * std::max(1, p->groups) / together / sm_count;
+  steps *= wide * waves;
+  const int launches = contractions + (together > 1 ? 2 : 0) + (copied ? 1 : 0);
+  const float general = float(3.4 + 2.25 * (launches - 1) + 0.134 * steps);
+  // a contraction and further ones, steps and tiles, of which a device's first few cost most;
+  // block-diagonal weights and repair; copies
+  tiles = std::max(0.0, tiles * waves - 0.5);
+  double later = 2.37 + 3.54 * (contractions - 1) + 0.166 * steps + 0.116 * std::min(steps, 20.0) + 0.17 * tiles + 0.8 * std::min(tiles, 4.0);
+  if (together > 1) {
+    const int stored = p->taps_stored ? p->taps_stored : p->taps_h * p->taps_w;
+    later += 3.11 + (several_taps ? 1.68 : 0) + 3.81e-6 * p->groups * stored * double(p->k_per_tap) * p->n_total * together * dtypeBytes(type);
+  }
+  if (copied)
+    later += type == PLB_FLOAT ? 3.44 + 0.16e-6 * double(p->act_strides[2]) * p->out_n : type == PLB_QUARTER ? 1.92 : 2.72;
   Tiling t;
   // (no tiling takes less than 4 us)
-  return general > 4.0f && tilingOf(sm_count, p, n, type, wholeLoads(*p, type), &t) && t.us < general;
+  return general > 4.0f && tilingOf(sm_count, p, n, type, wholeLoads(*p, type), &t) && t.us < general &&
+         (packed || t.us_later < 0.98 * later);
 }
 
 int launchPatch(plb_context *ctx, const IgemmProblem *p, int n, int type, bool repair) {

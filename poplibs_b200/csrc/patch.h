@@ -11,9 +11,9 @@ constexpr int kPatchMaxPhases = 4;
 
 // Whether these problems (same operands, groups and channel counts; `type` is the
 // operands' element type, all pointers are the caller's) run on the patch kernel.
-// `launches`: what the general route takes; `together`: the groups that it contracts as one;
-// `packed`: whether it gathers the channels of several taps into one operand row.
-bool patchSuits(int sm_count, const IgemmProblem *p, int n, int type, int launches, int together, bool packed);
+// The general route: `contractions` launches, of `together` groups as one, on copies of the
+// operands (`copied`); `packed`: it gathers the channels of several taps into one operand row.
+bool patchSuits(int sm_count, const IgemmProblem *p, int n, int type, int contractions, int together, bool copied, bool packed);
 // `repair`: outputs whose sum is not finite are formed again without the products
 // with padding, as repairNonFinite does.
 int launchPatch(plb_context *ctx, const IgemmProblem *p, int n, int type, bool repair);

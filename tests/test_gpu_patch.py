@@ -41,33 +41,31 @@ GENERAL = [("24 to 24", "half")] + [(name, t) for name in ("one group, ragged", 
 # and of columns (8 to 32) of an item that the planner chooses, in one and in several blocks of
 # output channels, in each type and with the weights in either order
 SHAPES = [
-    (1, 3, 1, 1, (2, 2), 1, 2, "hfq", "hfq"),
+    (2, 2, 2, 1, (2, 2), 1, 2, "hfq", "hfq"),
     (8, 15, 19, 1, (2, 2), 1, 2, "hfq", "hfq"),
     (1, 36, 92, 4, (4, 3), 1, 2, "hfq", "hfq"),
     (4, 1, 1, 41, (35, 31), 3, 1, "hq", "hq"),
     (1, 59, 2, 1, (3, 2), 1, 2, "", "hfq"),
     (2, 70, 2, 1, (4, 2), 1, 2, "h", "hfq"),
-    (1, 172, 4, 1, (2, 2), 1, 2, "hfq", "hfq"),
+    (1, 172, 4, 1, (2, 2), 1, 2, "hq", "hfq"),
     (2, 72, 4, 1, (2, 6), 1, 1, "hfq", "hfq"),
-    (16, 2, 34, 37, (7, 6), 1, 1, "hfq", ""),
-    (16, 3, 25, 37, (7, 44), 1, 2, "hfq", "hfq"),
-    (16, 4, 28, 37, (18, 13), 1, 1, "hq", "hfq"),
+    (8, 4, 20, 37, (8, 23), 1, 1, "hfq", "hfq"),
+    (16, 3, 25, 37, (7, 44), 1, 2, "hq", "hfq"),
     (3, 65, 1, 25, (11, 42), 3, 2, "", "q"),
     (2, 104, 8, 34, (10, 9), 1, 1, "fq", "q"),
     (16, 12, 2, 38, (3, 58), 7, 2, "", "hq"),
-    (2, 68, 8, 13, (22, 22), 1, 1, "h", "h"),
-    (8, 8, 12, 19, (24, 37), 1, 1, "q", ""),
-    (3, 36, 32, 54, (22, 20), 1, 2, "", "q"),
+    (2, 68, 8, 13, (22, 22), 1, 1, "", "h"),
     (8, 57, 2, 37, (32, 7), 7, 2, "", "hq"),
     (16, 2, 22, 37, (12, 41), 3, 1, "hq", "f"),
+    (3, 40, 4, 62, (14, 30), 7, 2, "", "hq"),
     (8, 1, 77, 17, (22, 16), 7, 1, "hq", ""),
     (2, 2, 123, 37, (6, 34), 7, 1, "hq", ""),
     (2, 178, 8, 34, (12, 37), 3, 2, "", "q"),
+    (3, 8, 12, 50, (37, 30), 3, 1, "q", ""),
     (2, 72, 8, 54, (13, 29), 5, 2, "", "hq"),
-    (3, 40, 4, 62, (14, 30), 7, 2, "", "hq"),
+    (16, 8, 56, 37, (8, 8), 3, 1, "hfq", "f"),
     (4, 8, 96, 37, (9, 30), 5, 2, "q", "hfq"),
     (1, 100, 3, 2, (14, 14), 3, 2, "", "hfq"),
-    (1, 8, 79, 1, (30, 11), 3, 1, "fq", ""),
     (1, 20, 36, 2, (5, 5), 3, 2, "", "hfq"),
 ]
 
