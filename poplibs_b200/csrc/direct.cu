@@ -48,9 +48,11 @@ constexpr DirectTime kDirectTimes[] = {
 
 // The shape of the least time, and that time.
 const DirectTime &directShape(int sm_count, const IgemmProblem &p, int type, float *best) {
-  const int cls = type == PLB_FLOAT ? 2 : type == PLB_QUARTER ? 3 : wholeLoads(p, type) ? 0 : 1;
+  const bool whole = wholeLoads(p, type);
+  const int cls = type == PLB_FLOAT ? 2 : type == PLB_QUARTER ? 3 : whole ? 0 : 1;
   const DirectTime *found = nullptr;
   for (const DirectTime &t : kDirectTimes) {
+    if (!directHas(t.kind, type, whole)) continue;
     const Extent e = blockOf(t.kind);
     const double blocks = double((p.out_w + e.m - 1) / e.m) * ((p.n_total + e.n - 1) / e.n) * std::max(1, p.groups);
     const int at_once = sm_count * (t.teams == 1 ? 2 : 1), steps = (p.k_per_tap + e.k - 1) / e.k;

@@ -21,11 +21,12 @@ int launchDirectInstance(plb_context *ctx, const DirectVariant &v, const DirectA
   return launchPdl(ctx, kernel, dim3(v.blocks), dim3(v.teams * kDirectTeam), size_t(v.teams) * kTeamBytes, g);
 }
 
-template <int kType, class S>
+template <int kType, DirectKind kKind, class S>
 int launchDirectShape(plb_context *ctx, const DirectVariant &v, const DirectArgs &g) {
+  if (!directHas(kKind, kType, v.vec)) return fail(PLB_ERR_UNSUPPORTED, "no instance of the direct kernel of this shape");
 #define PLB_DIRECT(A, B)                                                      \
   return v.vec ? launchDirectInstance<kType, S, A, B, true>(ctx, v, g)        \
-               : launchDirectInstance<kType, S, A, B, false>(ctx, v, g)
+               : launchDirectInstance<kType, S, A, B, !directHas(kKind, kType, false)>(ctx, v, g)
   if (v.a_mn) {
     if (v.b_mn) PLB_DIRECT(true, true);
     PLB_DIRECT(true, false);
@@ -38,10 +39,10 @@ int launchDirectShape(plb_context *ctx, const DirectVariant &v, const DirectArgs
 template <int kType>
 int launchDirectType(plb_context *ctx, const DirectVariant &v, const DirectArgs &g) {
   switch (v.kind) {
-    case kDirectFew: return launchDirectShape<kType, DirectFew>(ctx, v, g);
-    case kDirectSmall: return launchDirectShape<kType, DirectSmall>(ctx, v, g);
-    case kDirectMid: return launchDirectShape<kType, DirectMid>(ctx, v, g);
-    default: return launchDirectShape<kType, DirectWide>(ctx, v, g);
+    case kDirectFew: return launchDirectShape<kType, kDirectFew, DirectFew>(ctx, v, g);
+    case kDirectSmall: return launchDirectShape<kType, kDirectSmall, DirectSmall>(ctx, v, g);
+    case kDirectMid: return launchDirectShape<kType, kDirectMid, DirectMid>(ctx, v, g);
+    default: return launchDirectShape<kType, kDirectWide, DirectWide>(ctx, v, g);
   }
 }
 

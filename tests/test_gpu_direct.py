@@ -25,7 +25,7 @@ SIZES = [(1, 1, 1, 1), (1, 16, 256, 32), (1, 17, 257, 33), (1, 15, 511, 31), (1,
 DIRECT = {
     "half": [(1, 8, 8, 8), (3, 280, 13, 261), (1, 4, 314, 5), (6, 40, 8, 288), (6, 197, 9, 296), (6, 196, 10, 395),
              (6, 275, 160, 72), (6, 80, 96, 272)],
-    "float": [(1, 8, 8, 8), (2, 4, 280, 4), (6, 200, 8, 152), (6, 280, 8, 200), (6, 288, 16, 352), (6, 133, 138, 179)],
+    "float": [(1, 8, 8, 8), (2, 4, 280, 4), (6, 200, 8, 152), (6, 280, 8, 200), (6, 288, 16, 352)],
     "quarter": [(1, 4, 21, 8), (3, 5, 213, 5), (1, 7, 389, 11), (6, 175, 15, 299), (2, 228, 147, 293), (1, 8, 25, 8),
                 (2, 8, 329, 8), (3, 8, 181, 40)],
 }
@@ -73,7 +73,9 @@ def test_small_products(gpu_ctx, general_ctx, dtype, ta, tb, pad, offset):
     plb_in, np_in, plb_out, np_out = TYPES[dtype]
     if dtype == "quarter" and (ta or not tb) and pad:
         pytest.skip("refused: transposed quarter operands are densely packed")
-    for g, m, k, n in SIZES + DIRECT[dtype]:
+    # (floats from any address take three of the shapes)
+    whole = [(20, 8, 168, 232)] if dtype == "float" and pad != 3 else []
+    for g, m, k, n in SIZES + DIRECT[dtype] + whole:
         r = T.rng(m + 7 * k + n)
         av, bv = (r.integers(-2, 3, s).astype(np.float64) for s in ((g, m, k), (g, k, n)))
         want = av @ bv
