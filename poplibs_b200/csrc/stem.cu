@@ -110,20 +110,17 @@ stemKernel(const __grid_constant__ StemArgs a) {
   }
   pdl_wait();  // (all threads: they read the operands, or write over what the last kernel read)
   // weights: [filter row][superpixel][output channel] of 16 bytes
-  for (int i = tid; i < g.KH * a.taps * a.co; i += kStemThreads) {
-    const int rt = int(fast_div(uint32_t(i), a.fd_co)), co = i - rt * a.co, r = int(fast_div(uint32_t(rt), a.fd_taps)), t = rt - r * a.taps;
-    uint32_t v[4];
+  const int weight_units = g.KH * a.taps * a.co, next_column = (a.co - 1) * g.C;
+  for (int i = tid; i < weight_units; i += kStemThreads) {
+    const int rt = int(fast_div(uint32_t(i), a.fd_co)), co = i - rt * a.co, r = int(fast_div(uint32_t(rt), a.fd_taps));
+    const int s = (rt - r * a.taps) * g.s - a.shift;  // the first pixel's filter column; C elements on, the next one's
+    const uint16_t *const p = a.w + ((r * g.KW + s) * a.co + co) * g.C;
+    const int first = s >= 0 && s < g.KW ? g.C : 0, last = g.s == 2 && s + 1 >= 0 && s + 1 < g.KW ? 2 * g.C : g.C;
+    uint16_t e[8];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      uint32_t both = 0;
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int e = 2 * j + h, px = e >= g.C ? 1 : 0, c = e - px * g.C, s = t * g.s + px - a.shift;
-        if (e < g.s * g.C && s >= 0 && s < g.KW) both |= uint32_t(a.w[((r * g.KW + s) * a.co + co) * g.C + c]) << (16 * h);
-      }
-      v[j] = both;
-    }
-    st_shared_v4(weights + uint32_t(i) * 16, v[0], v[1], v[2], v[3]);
+    for (int k = 0; k < 8; ++k) e[k] = k < g.C ? (k < first ? p[k] : uint16_t(0)) : k < last ? p[k + next_column] : uint16_t(0);
+    st_shared_v4(weights + uint32_t(i) * 16, e[0] | uint32_t(e[1]) << 16, e[2] | uint32_t(e[3]) << 16, e[4] | uint32_t(e[5]) << 16,
+                 e[6] | uint32_t(e[7]) << 16);
   }
   if (tid < a.co_pad) bias[tid] = a.bias && tid < a.co ? a.bias[tid] : 0.f;
   fence_proxy_async_smem();
@@ -322,17 +319,27 @@ stemKernel(const __grid_constant__ StemArgs a) {
 struct StemTiling {
   int taps, pad_w, tile_w, rows, pitch;
   size_t plane_bytes, strip_bytes, weight_bytes;
+  float us;
 };
 
-// The strip that takes the fewest cycles: a tile's instructions or its results, or the
-// strip's loads, times the strips of an SM, and the first strip's way through.
+// Whether the image is loaded in whole words: rows and superpixels start on them.
+bool wholeWords(const S2dShape &g) { return g.s * g.C % 2 == 0 && g.W * g.C % 2 == 0; }
+
+// The strip of the least time, and that time.  Cycles of a strip: its tiles (instructions, or
+// results where those take longer) or its loads (a round trip to memory, then so much for each
+// superpixel and element), and the lesser of the two once more, as they share the path to shared
+// memory.  The weights come first, 512 threads with eight loads each at a time.  Fitted to 571
+// sampled layers, median error 4 %, a tenth of them 13 %.  (Without the round trip, strips of
+// one tile looked best: 7x7/2, 3 -> 128 channels, 41 images of 86 x 117 18.2 us.)
 bool stemTiling(int sms, const S2dShape &g, int co, StemTiling *best) {
   StemTiling t{};
   t.pad_w = (g.padW + g.s - 1) / g.s * g.s;
   t.taps = ((g.KW + t.pad_w - g.padW + g.s - 1) / g.s + 1) / 2 * 2;
   t.weight_bytes = (size_t(g.KH) * t.taps * co * 16 + 127) / 128 * 128;
-  const double tile = std::max(g.KH * t.taps / 2 * std::max(32.0, co / 2.0), 150.0 + 7.0 * co);
-  double least = 1e30;
+  const double tile = std::max(g.KH * t.taps / 2 * (58.5 + 0.214 * co), 383 + 12.7 * co);
+  const double superpixel = 0.574 + 0.165 * (wholeWords(g) ? g.s * g.C / 2 : g.s * g.C);
+  const double first = 1.93 + 0.5 * std::ceil(g.KH * t.taps * co / 512.0);
+  bool found = false;
   for (int parts = 1; parts <= 8 && (parts == 1 || g.OW >= 16 * parts); ++parts)
     for (int rows = 1; rows <= std::min(16, g.OH); ++rows) {
       t.tile_w = (g.OW + parts - 1) / parts;
@@ -342,33 +349,52 @@ bool stemTiling(int sms, const S2dShape &g, int co, StemTiling *best) {
       // (a tile reads past its last row)
       t.strip_bytes = (g.s * t.plane_bytes + (128 + size_t(t.taps)) * 16 + 127) / 128 * 128;
       if (t.weight_bytes + 2 * t.strip_bytes > 200 * 1024) break;
-      const double loads = (rows - 1.0) * g.s + g.KH, tiles = ((rows - 1) * t.pitch + t.tile_w + 127) / 128;
-      const double load = 0.35 * loads * t.pitch + 300, unit = std::max(tiles * tile, load) + 60;
+      const double superpixels = ((rows - 1.0) * g.s + g.KH) * t.pitch, loads = superpixels * superpixel;
+      const double load = 1226 + 21 * (std::ceil(superpixels / (4 * kStemLoaders)) - 1) + loads;
+      const double tiles = tile * (((rows - 1) * t.pitch + t.tile_w + 127) / 128);
+      const double unit = std::max(tiles, load) + std::min(tiles, loads);
       const double units = double(g.N) * ((g.OH + rows - 1) / rows) * ((g.OW + t.tile_w - 1) / t.tile_w);
-      const double cycles = std::ceil(units / sms) * unit + load + tile;
-      if (cycles < least) {
-        least = cycles;
-        *best = t;
-      }
+      t.us = float(first + (std::ceil(units / sms) * unit + 0.16 * (load + tile)) / 1900);
+      if (!found || t.us < best->us) *best = t;
+      found = true;
     }
-  return least < 1e30;
+  return found;
+}
+
+// What the rearranged form takes, fitted to 729 layers: two launches, a thread for each 16 bytes
+// rearranged (3 channels, stride 2: a block for each row), then the tiles of whole pixel boxes;
+// median error 10 %.
+float rearrangedTime(int sms, const S2dShape &g, int co) {
+  double tiles = 1e30;
+  for (int w = 128; w >= 1; w >>= 1)
+    for (int h = 128 / w; h >= 1; h >>= 1) {
+      const int n = 128 / (w * h);
+      tiles = std::min(tiles, double((g.OW + w - 1) / w) * ((g.OH + h - 1) / h) * ((g.N + n - 1) / n));
+    }
+  const bool by_rows = g.C == 3 && g.s == 2 && g.W % 2 == 0;
+  const double rearrange = by_rows ? 3.43 * g.N * g.H2 * ((g.W2 + 127) / 128) / (16.0 * sms)
+                                   : 4.56 * g.N * g.H2 * g.W2 * (g.C2 / 8) / (2048.0 * sms);
+  const int bn = co <= 64 ? 64 : 128;
+  const double waves = std::max(1.0, tiles * ((co + bn - 1) / bn) / sms) + 3.43;
+  return float(2.47 + rearrange + waves * (0.358 + 0.054 * g.K2h * bn / 64 + 0.062 * co / 64));
 }
 
 }  // namespace
 
-// Two kinds of large filters stay rearranged: those of one channel, where both strides' pixels
-// then share 16 bytes, half as many instructions (7x7/2, 64 channels: 92 images of 212 x 56 21.7
-// against 25.4 us, 103 of 61 x 61 12.5 against 12.7), and many short rows with more than 32
-// output channels, whose strips waste a sixth of their positions (514 of 79 x 79 55.0 against
-// 61.7, 1066 of 55 x 55, 96 channels, 71.3 against 83.7; 547 of 48 x 50 40.9 against 37.0).  Of 50
-// sampled layers the rest take 0.8 of their time on average, none more than 4 % longer.
+// Layers whose estimated time is at most a microsecond above the rearranged form's, whose second
+// launch costs a host that issues it 1.9.  Of 652 sampled layers, 571 take it and run in 0.79 of the
+// other's time, 32 of them more than 8 % longer on the device.
+// Two kinds of large filters stay rearranged besides: those of one channel, where both strides' pixels then share 16
+// bytes, half as many instructions (7x7/2, 64 channels: 92 images of 212 x 56 18.6 against 20.2 us),
+// and many short rows with more than 32 output channels, whose strips waste a sixth of their
+// positions (514 of 79 x 79 51.0 against 61.0, 1066 of 55 x 55, 96 channels, 62.8 against 70.7).
 bool stemSuits(int sm_count, const S2dShape &g, int co, bool out_f32, const void *out) {
   StemTiling t;
   const bool large = g.KH > 3;
   if (large && (g.C == 1 || (co > 32 && g.OW < 64 && uint64_t(g.N) * g.OH * g.OW > uint64_t(1) << 19))) return false;
   return g.s * g.C <= 8 && co % 16 == 0 && co <= 256 && !out_f32 && reinterpret_cast<uintptr_t>(out) % 32 == 0 &&
          uint64_t(g.H) * g.W * g.C < uint64_t(1) << 29 && uint64_t(g.N) * g.OH * g.OW < uint64_t(1) << 30 &&
-         stemTiling(sm_count, g, co, &t);
+         stemTiling(sm_count, g, co, &t) && t.us < rearrangedTime(sm_count, g, co) + 1.0f;
 }
 
 int launchStem(plb_context *ctx, const S2dShape &g, int co, bool bf16, const void *x, const void *w, const float *bias,
@@ -404,9 +430,7 @@ int launchStem(plb_context *ctx, const S2dShape &g, int co, bool bf16, const voi
   a.fd_h_blocks = make_fastdiv(uint32_t(a.h_blocks));
   a.fd_co = make_fastdiv(uint32_t(co));
   a.fd_taps = make_fastdiv(uint32_t(t.taps));
-  // whole words: rows and superpixels start on them
-  const int elems = g.s * g.C;
-  const int words = elems % 2 == 0 && g.W * g.C % 2 == 0 && reinterpret_cast<uintptr_t>(x) % 4 == 0 ? elems / 2 : 0;
+  const int words = wholeWords(g) && reinterpret_cast<uintptr_t>(x) % 4 == 0 ? g.s * g.C / 2 : 0;
   auto launch = [&](auto kernel, std::atomic<bool> *configured) {
     std::atomic<bool> &done = configured[ctx->device & 63];
     if (!done) {
