@@ -715,26 +715,28 @@ int convBwdStrided(plb_context *ctx, const plb_conv_params &p, const plb_conv_op
 // Whether a pass runs on the patch kernel (patch.cu), and its problem(s); `o` are the
 // caller's operands, `groups` those that the general route contracts together.
 bool fwdOnPatches(int sm_count, const plb_conv_params &p, const plb_conv_options *opt, int plan_flags, const ConvShape &s,
-                  const PassOperands &o, const float *bias, void *out, bool swapped, int groups, IgemmProblem *r) {
+                  const PassOperands &o, const float *bias, void *out, bool swapped, int groups, bool slower_too, IgemmProblem *r) {
   if ((!pointwise(s) && (s.strH > 8 || s.strW > 8)) || s.KH <= 0 || s.KW <= 0) return false;
   *r = convFwdProblem(p, opt, s, o, bias, out, swapped);
   r->plan_flags |= plan_flags;
   const bool packed = p.groups == 1 && p.input_type != PLB_FLOAT && !swapped && !channelsFitTma(p, p.in_chans_per_group);
-  return patchSuits(sm_count, r, 1, p.input_type, 1, groups, operandsCopied(o, p.in_chans_per_group), packed);
+  return patchSuits(sm_count, r, 1, p.input_type, 1, groups, operandsCopied(o, p.in_chans_per_group), packed, slower_too);
 }
 // The one-launch routes of a forward pass, tried before the others: straight from the image
-// (`shape`), or on the patch kernel (`r`).
+// (`shape`), or on the patch kernel (`r`).  `slower_too`: where the others would be quicker, but
+// cannot have the scratch memory that they need.
 enum class FwdRoute { kOther, kStem, kPatch };
 FwdRoute fwdRoute(int sm_count, const plb_conv_params &p, const plb_conv_options *opt, int plan_flags, const ConvShape &s,
-                  const PassOperands &o, const float *bias, void *out, bool swapped, int groups, IgemmProblem *r, S2dShape *shape) {
+                  const PassOperands &o, const float *bias, void *out, bool swapped, int groups, bool slower_too, IgemmProblem *r,
+                  S2dShape *shape) {
   if (is16BitFloat(p.input_type) && p.groups == 1 && !channelsFitTma(p, p.in_chans_per_group) && !swapped &&
-      stemLayer(sm_count, plan_flags, p, opt, out, shape))
+      stemLayer(sm_count, plan_flags, p, opt, out, slower_too, shape))
     return FwdRoute::kStem;
-  return fwdOnPatches(sm_count, p, opt, plan_flags, s, o, bias, out, swapped, groups, r) ? FwdRoute::kPatch : FwdRoute::kOther;
+  return fwdOnPatches(sm_count, p, opt, plan_flags, s, o, bias, out, swapped, groups, slower_too, r) ? FwdRoute::kPatch : FwdRoute::kOther;
 }
 // (the number of problems, 0 if it does not)
 int bwdOnPatches(int sm_count, const plb_conv_params &p, const plb_conv_options *opt, int plan_flags, const ConvShape &s,
-                 const PassOperands &o, void *dx, int groups, IgemmProblem *r) {
+                 const PassOperands &o, void *dx, int groups, bool slower_too, IgemmProblem *r) {
   int n = 0, contractions = 0;
   if (s.strH == 1 && s.strW == 1) {
     r[n++] = convBwdProblem(p, opt, s, o, dx, false);
@@ -759,7 +761,7 @@ int bwdOnPatches(int sm_count, const plb_conv_params &p, const plb_conv_options 
   }
   if (n == 0) return 0;
   r[0].plan_flags |= plan_flags;
-  return patchSuits(sm_count, r, n, p.input_type, contractions, groups, operandsCopied(o, p.out_chans_per_group), false) ? n : 0;
+  return patchSuits(sm_count, r, n, p.input_type, contractions, groups, operandsCopied(o, p.out_chans_per_group), false, slower_too) ? n : 0;
 }
 
 // Narrow channel groups are contracted together (grouped.cu): `q` = the layer of
@@ -778,6 +780,124 @@ int gatherGroups(plb_context *ctx, const plb_conv_params &p, const ConvShape &s,
   q->out_chans_per_group = S * co;
   return blockDiagonalWeights(ctx, p.input_type, weights, p.groups, S, uint32_t(s.KHs * s.KWs), rows_are_co ? co : ci,
                               rows_are_co ? ci : co, out);
+}
+
+// The product by way of the implicit-GEMM kernel: operands transposed and copied as it needs them.
+int matmulGeneral(plb_context *ctx, const plb_matmul_desc &d, const Ld &ld, const void *d_a, const void *d_b, const void *d_c,
+                  void *d_d) {
+  // Operand layouts the kernel takes directly: A as [m][k], B as [n][k], or (not
+  // 8-bit) A as [k][m] and B as [k][n].  8-bit operands stored the other way go
+  // through a transpose into scratch.
+  const void *a = d_a, *b = d_b;
+  long long lda = ld.a, ldb = ld.b;
+  bool a_is_km = d.transpose_a != 0, b_is_nk = d.transpose_b != 0;
+  if (d.input_type == PLB_QUARTER && (a_is_km || !b_is_nk)) {
+    // (rows of whole 16-byte vectors, so that nothing has to be copied again)
+    const uint64_t pitch = roundToRow(d.k, 1);
+    const size_t a_bytes = a_is_km ? (size_t(d.groups) * d.m * pitch + 255) & ~size_t(255) : 0;
+    const size_t b_bytes = b_is_nk ? 0 : size_t(d.groups) * d.n * pitch;
+    void *ws = nullptr;
+    if (int rc = scratch(ctx, kSlotOperands, a_bytes + b_bytes, &ws)) return rc;
+    if (a_is_km) {
+      if (int rc = transposeBatch(ctx, 1, d.groups, d.k, d.m, d_a, ws, pitch)) return rc;
+      a = ws;
+      lda = (long long)pitch;
+      a_is_km = false;
+    }
+    if (!b_is_nk) {
+      uint8_t *bt = static_cast<uint8_t *>(ws) + a_bytes;
+      if (int rc = transposeBatch(ctx, 1, d.groups, d.k, d.n, d_b, bt, pitch)) return rc;
+      b = bt;
+      ldb = (long long)pitch;
+      b_is_nk = true;
+    }
+  }
+  // Operands whose rows TMA cannot address (base or row pitch not a multiple of
+  // 16 bytes: n % 8 != 0, odd leading dimensions) are copied once into scratch
+  // with the pitch rounded up, float operands are split into their bfloat16
+  // pieces, both operands in one launch.  The output needs no such copy.
+  Copies copies = planCopies(d, &a, &lda, a_is_km, &b, &ldb, b_is_nk);
+  if (int rc = runCopies(ctx, copies)) return rc;
+  const plb_matmul_desc q = contractionDesc(d);
+  IgemmProblem p = gemmProblem(q, a, lda, a_is_km, b, ldb, b_is_nk, d_c, d_d, ld.c);
+  return runProblem(ctx, p);
+}
+
+// The passes by way of the implicit-GEMM kernel: operands gathered and copied as it needs them.
+int convFwdGeneral(plb_context *ctx, const plb_conv_params *p, const plb_conv_options *opt, const ConvShape &s,
+                   const PassOperands &separate, const void *d_in, const void *d_weights, const float *d_bias, void *d_out,
+                   bool swapped) {
+  if (p->input_type != PLB_FLOAT && !channelsFitTma(*p, p->in_chans_per_group) && !swapped) {
+    // few input channels (a stem): space-to-depth path, where it applies
+    const int rc = convFwdSmallChannels(ctx, *p, opt, d_in, d_weights, d_bias, d_out, nullptr);
+    if (rc != PLB_ERR_UNSUPPORTED) return rc;
+  }
+  if (s.strH > 1 || s.strW > 1) {
+    if (!pointwise(s) && (s.strH > 8 || s.strW > 8))
+      return fail(PLB_ERR_UNSUPPORTED, "strides above 8 are not implemented for k > 1");
+  }
+  if (s.KH <= 0 || s.KW <= 0) {
+    // every tap is truncated away: the result is zero
+    PLB_CUDA(cudaMemsetAsync(d_out, 0,
+                             size_t(p->batch) * s.OH * s.OW * p->groups * p->out_chans_per_group *
+                                 dtypeBytes(p->output_type),
+                             ctx->stream));
+    return PLB_OK;
+  }
+  plb_conv_params q;
+  const void *w = nullptr;
+  bool together = false;
+  // stored [G][k][Ci][Co] when swapped, else [G][k][Co][Ci]
+  if (int rc = gatherGroups(ctx, *p, s, d_weights, !swapped, &q, &w, &together)) return rc;
+  const uint64_t in_rows = uint64_t(q.batch) * s.H * s.W * q.groups, tiles = uint64_t(q.groups) * s.KHs * s.KWs;
+  const uint32_t ci = q.in_chans_per_group, co = q.out_chans_per_group;
+  const bool transposed = swapped && q.input_type == PLB_QUARTER;  // -> [G][flipped k][Co][Ci]
+  Repack::Lattice sub{};
+  const Repack::Lattice *lattice = readPixels(q, s, &sub) ? &sub : nullptr;
+  PassOperands o;
+  if (transposed) {
+    uint32_t pitch = 0;
+    if (int rc = transposedWeights(ctx, w, q.groups, uint64_t(s.KHs) * s.KWs, ci, co, &w, &pitch)) return rc;
+    if (int rc = prepareOperands(ctx, q.input_type, d_in, in_rows, ci, w, tiles * co, pitch, 0, &o, lattice)) return rc;
+  } else if (swapped) {
+    // the reduction along the rows
+    if (int rc = prepareOperands(ctx, q.input_type, d_in, in_rows, ci, w, tiles * ci, co, ci, &o, lattice)) return rc;
+  } else {
+    if (int rc = prepareOperands(ctx, q.input_type, d_in, in_rows, ci, w, tiles * co, ci, 0, &o, lattice)) return rc;
+  }
+  IgemmProblem r = convFwdProblem(q, opt, s, o, d_bias, d_out, swapped && !transposed, transposed);
+  if (together) r.nonfinite = nonfiniteFlag(ctx);
+  if (int rc = runProblem(ctx, r)) return rc;
+  if (!together) return PLB_OK;
+  return repairNonFinite(ctx, convFwdProblem(*p, opt, s, separate, d_bias, d_out, swapped), p->input_type);
+}
+
+int convBwdGeneral(plb_context *ctx, const plb_conv_params *p, const plb_conv_options *opt, const ConvShape &s,
+                   const PassOperands &separate, const void *d_out_grads, const void *d_weights, void *d_in_grads) {
+  plb_conv_params q;
+  const void *w = nullptr;
+  bool together = false;
+  if (int rc = gatherGroups(ctx, *p, s, d_weights, true, &q, &w, &together)) return rc;
+  const uint64_t out_rows = uint64_t(q.batch) * s.OH * s.OW * q.groups, tiles = uint64_t(q.groups) * s.KHs * s.KWs;
+  const uint32_t ci = q.in_chans_per_group, co = q.out_chans_per_group;
+  PassOperands o;
+  const bool transposed = q.input_type == PLB_QUARTER;
+  if (transposed) {
+    uint32_t pitch = 0;
+    // [G][k][Co][Ci] -> [G][flipped k][Ci][Co]
+    if (int rc = transposedWeights(ctx, w, q.groups, uint64_t(s.KHs) * s.KWs, co, ci, &w, &pitch)) return rc;
+    if (int rc = prepareOperands(ctx, q.input_type, d_out_grads, out_rows, co, w, tiles * ci, pitch, 0, &o)) return rc;
+  } else {
+    // the reduction runs over the output channels, the rows of a weight tile
+    if (int rc = prepareOperands(ctx, q.input_type, d_out_grads, out_rows, co, w, tiles * co, ci, co, &o)) return rc;
+  }
+  if (s.strH != 1 || s.strW != 1)
+    return convBwdStrided(ctx, q, opt, s, o, d_in_grads, transposed, p, together ? &separate : nullptr);
+  IgemmProblem r = convBwdProblem(q, opt, s, o, d_in_grads, transposed);
+  if (together) r.nonfinite = nonfiniteFlag(ctx);
+  if (int rc = runProblem(ctx, r)) return rc;
+  if (!together) return PLB_OK;
+  return repairNonFinite(ctx, convBwdProblem(*p, opt, s, separate, d_in_grads, false), p->input_type);
 }
 
 }  // namespace
@@ -817,7 +937,7 @@ int plb_matmul_plan(const plb_matmul_desc *desc, plb_plan *plan) {
   plan->workspace_bytes += transposed + copies.bytes;
   const IgemmProblem direct = gemmProblem(*desc, nullptr, ld.a, desc->transpose_a != 0, nullptr, ld.b, desc->transpose_b != 0,
                                           nullptr, nullptr, ld.c);
-  if (directSuits(148, direct, desc->input_type, matmulCopies(*desc, nullptr, nullptr))) {
+  if (directSuits(148, direct, desc->input_type, matmulCopies(*desc, nullptr, nullptr), false)) {
     plan->kernel = 3;
     plan->in_place = 1;
   }
@@ -837,7 +957,7 @@ int plb_matmul(plb_context *ctx, const plb_matmul_desc *desc, const void *d_a, c
   if (d_d == nullptr || (d.k != 0 && (d_a == nullptr || d_b == nullptr)))
     return fail(PLB_ERR_INVALID_PARAMS, "null device pointer for a matrix that has elements");
   const Ld ld = leadingDims(d);
-  const size_t es = dtypeBytes(d.input_type), os = dtypeBytes(d.output_type);
+  const size_t os = dtypeBytes(d.output_type);
   if (d.k == 0) {
     // empty reduction: D = beta * C
     for (uint32_t g = 0; g < d.groups; ++g) {
@@ -855,48 +975,15 @@ int plb_matmul(plb_context *ctx, const plb_matmul_desc *desc, const void *d_a, c
     return fail(PLB_ERR_UNSUPPORTED, "transposed quarter A must be densely packed");
   if (d.input_type == PLB_QUARTER && !d.transpose_b && ld.b != (long long)d.n)
     return fail(PLB_ERR_UNSUPPORTED, "quarter B in [k][n] layout must be densely packed");
-  {
-    // small products, and moderate ones that would need a copy, from the operands as they are
-    IgemmProblem p = gemmProblem(d, d_a, ld.a, d.transpose_a != 0, d_b, ld.b, d.transpose_b != 0, d_c, d_d, ld.c);
-    p.plan_flags = ctx->plan_flags;
-    if (directSuits(ctx->sm_count, p, d.input_type, matmulCopies(d, d_a, d_b))) return launchDirect(ctx, p, d.input_type);
-  }
-  // Operand layouts the kernel takes directly: A as [m][k], B as [n][k], or (not
-  // 8-bit) A as [k][m] and B as [k][n].  8-bit operands stored the other way go
-  // through a transpose into scratch.
-  const void *a = d_a, *b = d_b;
-  long long lda = ld.a, ldb = ld.b;
-  bool a_is_km = d.transpose_a != 0, b_is_nk = d.transpose_b != 0;
-  if (d.input_type == PLB_QUARTER && (a_is_km || !b_is_nk)) {
-    // (rows of whole 16-byte vectors, so that nothing has to be copied again)
-    const uint64_t pitch = roundToRow(d.k, 1);
-    const size_t a_bytes = a_is_km ? (size_t(d.groups) * d.m * pitch + 255) & ~size_t(255) : 0;
-    const size_t b_bytes = b_is_nk ? 0 : size_t(d.groups) * d.n * pitch;
-    void *ws = nullptr;
-    if (int rc = scratch(ctx, kSlotOperands, a_bytes + b_bytes, &ws)) return rc;
-    if (a_is_km) {
-      if (int rc = transposeBatch(ctx, 1, d.groups, d.k, d.m, d_a, ws, pitch)) return rc;
-      a = ws;
-      lda = (long long)pitch;
-      a_is_km = false;
-    }
-    if (!b_is_nk) {
-      uint8_t *bt = static_cast<uint8_t *>(ws) + a_bytes;
-      if (int rc = transposeBatch(ctx, 1, d.groups, d.k, d.n, d_b, bt, pitch)) return rc;
-      b = bt;
-      ldb = (long long)pitch;
-      b_is_nk = true;
-    }
-  }
-  // Operands whose rows TMA cannot address (base or row pitch not a multiple of
-  // 16 bytes: n % 8 != 0, odd leading dimensions) are copied once into scratch
-  // with the pitch rounded up, float operands are split into their bfloat16
-  // pieces, both operands in one launch.  The output needs no such copy.
-  Copies copies = planCopies(d, &a, &lda, a_is_km, &b, &ldb, b_is_nk);
-  if (int rc = runCopies(ctx, copies)) return rc;
-  const plb_matmul_desc q = contractionDesc(d);
-  IgemmProblem p = gemmProblem(q, a, lda, a_is_km, b, ldb, b_is_nk, d_c, d_d, ld.c);
-  return runProblem(ctx, p);
+  // small products, and moderate ones that would need a copy, from the operands as they are
+  IgemmProblem p = gemmProblem(d, d_a, ld.a, d.transpose_a != 0, d_b, ld.b, d.transpose_b != 0, d_c, d_d, ld.c);
+  p.plan_flags = ctx->plan_flags;
+  const bool copied = matmulCopies(d, d_a, d_b);
+  if (directSuits(ctx->sm_count, p, d.input_type, copied, false)) return launchDirect(ctx, p, d.input_type);
+  ctx->scratch_refused = false;
+  const int rc = matmulGeneral(ctx, d, ld, d_a, d_b, d_c, d_d);
+  if (rc && ctx->scratch_refused && directSuits(ctx->sm_count, p, d.input_type, copied, true)) return launchDirect(ctx, p, d.input_type);
+  return rc;
 }
 
 int plb_matmul_host(plb_context *ctx, const plb_matmul_desc *desc, const void *h_a,
@@ -1009,8 +1096,8 @@ int plb_conv_plan(const plb_conv_params *p_in, const plb_conv_options *opt, int3
     S2dShape g;
     FwdRoute route = FwdRoute::kOther;
     if (!bwd)
-      route = fwdRoute(148, *p, opt, 0, s, o, nullptr, nullptr, false, int(together), r, &g);
-    else if (bwdOnPatches(148, *p, opt, 0, s, o, nullptr, int(together), r) > 0)
+      route = fwdRoute(148, *p, opt, 0, s, o, nullptr, nullptr, false, int(together), false, r, &g);
+    else if (bwdOnPatches(148, *p, opt, 0, s, o, nullptr, int(together), false, r) > 0)
       route = FwdRoute::kPatch;
     if (route == FwdRoute::kPatch) plan->kernel = 3;
     plan->in_place = route == FwdRoute::kOther ? 0 : 1;
@@ -1094,60 +1181,25 @@ int plb_convolution(plb_context *ctx, const plb_conv_params *p, const plb_conv_o
   // the caller's operands, the groups apart
   const PassOperands separate{p->input_type, d_in, d_weights, p->in_chans_per_group, p->in_chans_per_group,
                               swapped ? p->out_chans_per_group : p->in_chans_per_group};
-  {
+  // in one launch, without scratch, where that is quicker, or where scratch cannot be had
+  auto inPlace = [&](bool slower_too, int *rc) {
     IgemmProblem r;
     S2dShape g;
     const int groups = groupsTogether(p->groups, p->in_chans_per_group, p->out_chans_per_group, p->input_type);
-    switch (fwdRoute(ctx->sm_count, *p, opt, ctx->plan_flags, s, separate, d_bias, d_out, swapped, groups, &r, &g)) {
-      case FwdRoute::kStem:
-        return launchStem(ctx, g, int(p->out_chans_per_group), p->input_type == PLB_BFLOAT16, d_in, d_weights, d_bias, d_out);
-      case FwdRoute::kPatch: return launchPatch(ctx, &r, 1, p->input_type, groups > 1);
-      default: break;
-    }
-  }
-  if (p->input_type != PLB_FLOAT && !channelsFitTma(*p, p->in_chans_per_group) && !transpose_and_flip_weights) {
-    // few input channels (a stem): space-to-depth path, where it applies
-    const int rc = convFwdSmallChannels(ctx, *p, opt, d_in, d_weights, d_bias, d_out, nullptr);
-    if (rc != PLB_ERR_UNSUPPORTED) return rc;
-  }
-  if (s.strH > 1 || s.strW > 1) {
-    if (!pointwise(s) && (s.strH > 8 || s.strW > 8))
-      return fail(PLB_ERR_UNSUPPORTED, "strides above 8 are not implemented for k > 1");
-  }
-  if (s.KH <= 0 || s.KW <= 0) {
-    // every tap is truncated away: the result is zero
-    PLB_CUDA(cudaMemsetAsync(d_out, 0,
-                             size_t(p->batch) * s.OH * s.OW * p->groups * p->out_chans_per_group *
-                                 dtypeBytes(p->output_type),
-                             ctx->stream));
-    return PLB_OK;
-  }
-  plb_conv_params q;
-  const void *w = nullptr;
-  bool together = false;
-  // stored [G][k][Ci][Co] when swapped, else [G][k][Co][Ci]
-  if (int rc = gatherGroups(ctx, *p, s, d_weights, !swapped, &q, &w, &together)) return rc;
-  const uint64_t in_rows = uint64_t(q.batch) * s.H * s.W * q.groups, tiles = uint64_t(q.groups) * s.KHs * s.KWs;
-  const uint32_t ci = q.in_chans_per_group, co = q.out_chans_per_group;
-  const bool transposed = swapped && q.input_type == PLB_QUARTER;  // -> [G][flipped k][Co][Ci]
-  Repack::Lattice sub{};
-  const Repack::Lattice *lattice = readPixels(q, s, &sub) ? &sub : nullptr;
-  PassOperands o;
-  if (transposed) {
-    uint32_t pitch = 0;
-    if (int rc = transposedWeights(ctx, w, q.groups, uint64_t(s.KHs) * s.KWs, ci, co, &w, &pitch)) return rc;
-    if (int rc = prepareOperands(ctx, q.input_type, d_in, in_rows, ci, w, tiles * co, pitch, 0, &o, lattice)) return rc;
-  } else if (swapped) {
-    // the reduction along the rows
-    if (int rc = prepareOperands(ctx, q.input_type, d_in, in_rows, ci, w, tiles * ci, co, ci, &o, lattice)) return rc;
-  } else {
-    if (int rc = prepareOperands(ctx, q.input_type, d_in, in_rows, ci, w, tiles * co, ci, 0, &o, lattice)) return rc;
-  }
-  IgemmProblem r = convFwdProblem(q, opt, s, o, d_bias, d_out, swapped && !transposed, transposed);
-  if (together) r.nonfinite = nonfiniteFlag(ctx);
-  if (int rc = runProblem(ctx, r)) return rc;
-  if (!together) return PLB_OK;
-  return repairNonFinite(ctx, convFwdProblem(*p, opt, s, separate, d_bias, d_out, swapped), p->input_type);
+    const FwdRoute route = fwdRoute(ctx->sm_count, *p, opt, ctx->plan_flags, s, separate, d_bias, d_out, swapped, groups, slower_too, &r, &g);
+    if (route == FwdRoute::kStem)
+      *rc = launchStem(ctx, g, int(p->out_chans_per_group), p->input_type == PLB_BFLOAT16, d_in, d_weights, d_bias, d_out);
+    else if (route == FwdRoute::kPatch)
+      *rc = launchPatch(ctx, &r, 1, p->input_type, groups > 1);
+    return route != FwdRoute::kOther;
+  };
+  int done = PLB_OK;
+  if (inPlace(false, &done)) return done;
+  ctx->scratch_refused = false;
+  const int rc = convFwdGeneral(ctx, p, opt, s, separate, d_in, d_weights, d_bias, d_out, swapped);
+  if (rc == PLB_OK || !ctx->scratch_refused) return rc;
+  const std::string why = plb_last_error();
+  return inPlace(true, &done) ? done : fail(rc, why);
 }
 
 int plb_conv_fwd(plb_context *ctx, const plb_conv_params *p, const plb_conv_options *opt,
@@ -1228,36 +1280,21 @@ int plb_conv_bwd(plb_context *ctx, const plb_conv_params *p, const plb_conv_opti
   // the caller's operands, the groups apart
   const PassOperands separate{p->input_type, d_out_grads, d_weights, p->out_chans_per_group, p->out_chans_per_group,
                               p->in_chans_per_group};
-  {
+  // in one launch, without scratch, where that is quicker, or where scratch cannot be had
+  auto inPlace = [&](bool slower_too, int *rc) {
     IgemmProblem r[kPatchMaxPhases];
     const int groups = groupsTogether(p->groups, p->in_chans_per_group, p->out_chans_per_group, p->input_type);
-    if (const int n = bwdOnPatches(ctx->sm_count, *p, opt, ctx->plan_flags, s, separate, d_in_grads, groups, r))
-      return launchPatch(ctx, r, n, p->input_type, groups > 1);
-  }
-  plb_conv_params q;
-  const void *w = nullptr;
-  bool together = false;
-  if (int rc = gatherGroups(ctx, *p, s, d_weights, true, &q, &w, &together)) return rc;
-  const uint64_t out_rows = uint64_t(q.batch) * s.OH * s.OW * q.groups, tiles = uint64_t(q.groups) * s.KHs * s.KWs;
-  const uint32_t ci = q.in_chans_per_group, co = q.out_chans_per_group;
-  PassOperands o;
-  const bool transposed = q.input_type == PLB_QUARTER;
-  if (transposed) {
-    uint32_t pitch = 0;
-    // [G][k][Co][Ci] -> [G][flipped k][Ci][Co]
-    if (int rc = transposedWeights(ctx, w, q.groups, uint64_t(s.KHs) * s.KWs, co, ci, &w, &pitch)) return rc;
-    if (int rc = prepareOperands(ctx, q.input_type, d_out_grads, out_rows, co, w, tiles * ci, pitch, 0, &o)) return rc;
-  } else {
-    // the reduction runs over the output channels, the rows of a weight tile
-    if (int rc = prepareOperands(ctx, q.input_type, d_out_grads, out_rows, co, w, tiles * co, ci, co, &o)) return rc;
-  }
-  if (s.strH != 1 || s.strW != 1)
-    return convBwdStrided(ctx, q, opt, s, o, d_in_grads, transposed, p, together ? &separate : nullptr);
-  IgemmProblem r = convBwdProblem(q, opt, s, o, d_in_grads, transposed);
-  if (together) r.nonfinite = nonfiniteFlag(ctx);
-  if (int rc = runProblem(ctx, r)) return rc;
-  if (!together) return PLB_OK;
-  return repairNonFinite(ctx, convBwdProblem(*p, opt, s, separate, d_in_grads, false), p->input_type);
+    const int n = bwdOnPatches(ctx->sm_count, *p, opt, ctx->plan_flags, s, separate, d_in_grads, groups, slower_too, r);
+    if (n > 0) *rc = launchPatch(ctx, r, n, p->input_type, groups > 1);
+    return n > 0;
+  };
+  int done = PLB_OK;
+  if (inPlace(false, &done)) return done;
+  ctx->scratch_refused = false;
+  const int rc = convBwdGeneral(ctx, p, opt, s, separate, d_out_grads, d_weights, d_in_grads);
+  if (rc == PLB_OK || !ctx->scratch_refused) return rc;
+  const std::string why = plb_last_error();
+  return inPlace(true, &done) ? done : fail(rc, why);
 }
 
 int plb_conv_fwd_host(plb_context *ctx, const plb_conv_params *p, const plb_conv_options *opt,

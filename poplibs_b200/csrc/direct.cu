@@ -100,12 +100,13 @@ float igemmTime(int sm_count, const IgemmProblem &p, int type, bool copied) {
 // products this took 230 to 0.64 of their time on average (16 x 512 x 512 4.4 -> 2.9 us,
 // 132 x 98 x 181 7.4 -> 3.7, as float 48 x 112 x 288 in 47 groups 11.1 -> 7.0); of those it
 // leaves, a few would gain up to 10 %.
-bool directSuits(int sm_count, const IgemmProblem &p, int type, bool copied) {
+bool directSuits(int sm_count, const IgemmProblem &p, int type, bool copied, bool slower_too) {
   if (p.plan_flags != 0 || (type != PLB_HALF && type != PLB_FLOAT && type != PLB_QUARTER)) return false;
   // (pitches that no tensor map holds, negative ones among them, are the general route's to refuse)
   const uint64_t pitch_limit = uint64_t(1) << 40;
   if (std::max({p.act_strides[0], p.act_strides[1], p.wgt_strides[0], p.wgt_strides[1]}) >= pitch_limit) return false;
   if (2.0 * std::max(1, p.groups) * p.out_w * double(p.n_total) * p.k_per_tap > 1e9) return false;
+  if (slower_too) return true;
   float us = 0.f;
   directShape(sm_count, p, type, &us);
   return us < 0.86f * igemmTime(sm_count, p, type, copied);

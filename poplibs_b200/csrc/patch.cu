@@ -180,7 +180,8 @@ bool patchable(const IgemmProblem *p, int n, int type) {
 // estimates took, 103 were more than 8 % slower than on the general route, up to 1.7 times; the second
 // leave 26 of those, and give up 22 that gain (3x3, 2 groups of 32, 42 images of 13 x 13, where 294 blocks
 // wait for the same weights, 13.0 -> 7.5 us; 1x1, 2 groups of 32, 8 of 35 x 35 8.8 -> 5.6).
-bool patchSuits(int sm_count, const IgemmProblem *p, int n, int type, int contractions, int together, bool copied, bool packed) {
+bool patchSuits(int sm_count, const IgemmProblem *p, int n, int type, int contractions, int together, bool copied, bool packed,
+                bool slower_too) {
   if (!patchable(p, n, type)) return false;
   const double operand = (type == PLB_FLOAT ? 6.0 : type == PLB_QUARTER ? 1.0 : 2.0) * together * p->k_per_tap;
   const double columns = double(together) * p->n_total, wide = columns <= 64 ? 1 : columns <= 128 ? 1.6 : 2.6;
@@ -210,7 +211,7 @@ bool patchSuits(int sm_count, const IgemmProblem *p, int n, int type, int contra
   Tiling t;
   // (no tiling takes less than 4 us)
   return general > 4.0f && tilingOf(sm_count, p, n, type, wholeLoads(*p, type), &t) && t.us < general &&
-         (packed || t.us_later < 0.98 * later);
+         (packed || slower_too || t.us_later < 0.98 * later);
 }
 
 int launchPatch(plb_context *ctx, const IgemmProblem *p, int n, int type, bool repair) {

@@ -13,7 +13,9 @@ constexpr int kPatchMaxPhases = 4;
 // operands' element type, all pointers are the caller's) run on the patch kernel.
 // The general route: `contractions` launches, of `together` groups as one, on copies of the
 // operands (`copied`); `packed`: it gathers the channels of several taps into one operand row.
-bool patchSuits(int sm_count, const IgemmProblem *p, int n, int type, int contractions, int together, bool copied, bool packed);
+// `slower_too`: by the first estimates alone.
+bool patchSuits(int sm_count, const IgemmProblem *p, int n, int type, int contractions, int together, bool copied, bool packed,
+                bool slower_too);
 // `repair`: outputs whose sum is not finite are formed again without the products
 // with padding, as repairNonFinite does.
 int launchPatch(plb_context *ctx, const IgemmProblem *p, int n, int type, bool repair);

@@ -35,6 +35,12 @@ int scratch(plb_context *ctx, int slot, size_t bytes, void **ptr) {
   if (slot < 0 || slot >= plb_context::kScratchSlots)
     return fail(PLB_ERR_INVALID_PARAMS, "bad scratch slot");
   if (ctx->scratch_bytes[slot] < bytes) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    PLB_CUDA(cudaStreamIsCapturing(ctx->stream, &capture));
+    if (capture != cudaStreamCaptureStatusNone) {
+      ctx->scratch_refused = true;
+      return fail(PLB_ERR_CUDA, "scratch memory cannot grow while the stream is captured: make the call once before");
+    }
     // work already enqueued may still read the old buffer
     PLB_CUDA(cudaStreamSynchronize(ctx->stream));
     if (ctx->scratch[slot]) PLB_CUDA(cudaFree(ctx->scratch[slot]));

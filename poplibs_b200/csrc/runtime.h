@@ -56,6 +56,7 @@ struct plb_context {
   static constexpr int kScratchSlots = kSlotCount;
   void *scratch[kScratchSlots] = {};
   size_t scratch_bytes[kScratchSlots] = {};
+  bool scratch_refused = false;   // a buffer could not grow, as the stream is being captured
 };
 
 #include <nvtx3/nvToolsExt.h>
@@ -85,7 +86,8 @@ int cudaFail(cudaError_t err, const char *what);
 
 // Makes the context's device current.
 int activate(plb_context *ctx);
-// Returns a scratch buffer of at least `bytes` (grows, synchronising first, if needed).
+// Returns a scratch buffer of at least `bytes` (grows, synchronising first, if needed; not while
+// the stream is being captured, which is an error that leaves the capture as it is).
 int scratch(plb_context *ctx, int slot, size_t bytes, void **ptr);
 
 // cuTensorMapEncodeTiled with 128-byte swizzle and zero fill outside the

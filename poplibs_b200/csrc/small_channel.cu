@@ -247,9 +247,9 @@ int smallChannelPrepare(plb_context *ctx, const S2dShape &g, const void *d_in, _
 }
 
 // Whether the stem kernel runs the forward pass.
-bool stemLayer(int sm_count, int plan_flags, const plb_conv_params &p, const plb_conv_options *opt, const void *d_out, S2dShape *g) {
+bool stemLayer(int sm_count, int plan_flags, const plb_conv_params &p, const plb_conv_options *opt, const void *d_out, bool slower_too, S2dShape *g) {
   return smallChannelShape(p, g) == PLB_OK && plan_flags == 0 && (!opt || (opt->plan_flags == 0 && opt->tile_n == 0)) &&
-         stemSuits(sm_count, *g, int(p.out_chans_per_group), p.output_type == PLB_FLOAT, d_out);
+         stemSuits(sm_count, *g, int(p.out_chans_per_group), p.output_type == PLB_FLOAT, d_out, slower_too);
 }
 
 int convFwdSmallChannels(plb_context *ctx, const plb_conv_params &p, const plb_conv_options *opt,

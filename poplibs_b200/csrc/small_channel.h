@@ -19,7 +19,7 @@ struct S2dShape {
 };
 
 int smallChannelShape(const plb_conv_params &p, S2dShape *g);
-bool stemLayer(int sm_count, int plan_flags, const plb_conv_params &p, const plb_conv_options *opt, const void *d_out, S2dShape *g);
+bool stemLayer(int sm_count, int plan_flags, const plb_conv_params &p, const plb_conv_options *opt, const void *d_out, bool slower_too, S2dShape *g);
 size_t smallChannelElems(const S2dShape &g);
 int smallChannelPrepare(plb_context *ctx, const S2dShape &g, const void *d_in, __half *x2, const void *d_weights,
                         __half *w2, int co);

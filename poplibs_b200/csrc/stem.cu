@@ -388,13 +388,13 @@ float rearrangedTime(int sms, const S2dShape &g, int co) {
 // bytes, half as many instructions (7x7/2, 64 channels: 92 images of 212 x 56 18.6 against 20.2 us),
 // and many short rows with more than 32 output channels, whose strips waste a sixth of their
 // positions (514 of 79 x 79 51.0 against 61.0, 1066 of 55 x 55, 96 channels, 62.8 against 70.7).
-bool stemSuits(int sm_count, const S2dShape &g, int co, bool out_f32, const void *out) {
+bool stemSuits(int sm_count, const S2dShape &g, int co, bool out_f32, const void *out, bool slower_too) {
   StemTiling t;
   const bool large = g.KH > 3;
   if (large && (g.C == 1 || (co > 32 && g.OW < 64 && uint64_t(g.N) * g.OH * g.OW > uint64_t(1) << 19))) return false;
   return g.s * g.C <= 8 && co % 16 == 0 && co <= 256 && !out_f32 && reinterpret_cast<uintptr_t>(out) % 32 == 0 &&
          uint64_t(g.H) * g.W * g.C < uint64_t(1) << 29 && uint64_t(g.N) * g.OH * g.OW < uint64_t(1) << 30 &&
-         stemTiling(sm_count, g, co, &t) && t.us < rearrangedTime(sm_count, g, co) + 1.0f;
+         stemTiling(sm_count, g, co, &t) && (slower_too || t.us < rearrangedTime(sm_count, g, co) + 1.0f);
 }
 
 int launchStem(plb_context *ctx, const S2dShape &g, int co, bool bf16, const void *x, const void *w, const float *bias,

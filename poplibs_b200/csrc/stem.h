@@ -8,7 +8,8 @@
 namespace plb {
 
 // Whether the layer (g: smallChannelShape of it) runs on the stem kernel.
-bool stemSuits(int sm_count, const S2dShape &g, int co, bool out_f32, const void *out);
+// (`slower_too`: whatever the rearranged form takes)
+bool stemSuits(int sm_count, const S2dShape &g, int co, bool out_f32, const void *out, bool slower_too);
 int launchStem(plb_context *ctx, const S2dShape &g, int co, bool bf16, const void *x, const void *w, const float *bias,
                void *out);
 
