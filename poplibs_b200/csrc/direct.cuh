@@ -574,11 +574,11 @@ using DirectWide = DirectShape<64, 64, 2, 2, 2, 64>;
 
 enum DirectKind : int { kDirectFew, kDirectSmall, kDirectMid, kDirectWide };
 
-// Floats from any address hold three vectors for each unit in registers: the shapes whose
-// threads load most units take up to 2.4 times as long with them as with floats in whole loads, longer than
-// the general route (225 x 1442 x 59 17.1 us, there 10.1; 112 x 685 x 2151 26.7, there 17.9).
+// Floats from any address hold three vectors for each unit in registers.  In blocks of 32 x 64
+// they take 2.4 times as long as floats in whole loads, longer than in the others (112 x 685 x 2151
+// 26.7 us, on the general route 17.9; 127 sampled products 0.72 of the time without that shape).
 constexpr bool directHas(DirectKind kind, int type, bool whole) {
-  return type != PLB_FLOAT || whole || (kind != kDirectFew && kind != kDirectMid);
+  return type != PLB_FLOAT || whole || kind != kDirectMid;
 }
 
 struct DirectVariant {
