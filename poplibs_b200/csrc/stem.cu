@@ -17,9 +17,9 @@
 // Roles: 7 warps load strips (two in flight), one thread issues the instructions, two groups
 // of 4 warps store alternate tiles.  Loads, results and operands share the SM's path to
 // shared memory and L1; a tile of 14 instructions (7x7) takes 1400 cycles of the 670 that the
-// instructions alone would, one of 6 (3x3) is bound by its results.  Measured: 3x3, 1 -> 96 on
-// 147 images of 118 x 118 137.5 -> 94.0 us, 3x3/2, 4 -> 64 on 11 of 102 x 192 10.1 -> 5.5,
-// 7x7/2, 3 -> 64 on 256 of 224 x 224 162.4 -> 156.5.  (Whole lines of results, stored from 16
+// instructions alone would, one of 6 (3x3) is bound by its results.  Measured against the rearranged
+// form: 3x3, 1 -> 96 on 147 images of 118 x 118 122 -> 96 us, 3x3/2, 4 -> 64 on 11 of 102 x 192 9.1 ->
+// 5.4, 7x7/2, 3 -> 64 on 256 of 224 x 224 162 -> 156 (medians of six).  (Whole lines of results, stored from 16
 // x 256-bit reads of tensor memory, two issuers or four accumulators: no gain.)
 #include <algorithm>
 #include <atomic>
