@@ -467,7 +467,8 @@ int launchIgemm(plb_context *ctx, const IgemmProblem &p, const plb_plan &plan) {
     partial = static_cast<float *>(ws);
   }
   // Output through TMA when the tensor can be described to it: 16-byte aligned
-  // base and pixel stride.  Each epilogue warp stores a (columns, w, h, n) box
+  // base and pixel stride, and rows that end on 16 bytes (a shorter last vector is written whole,
+  // over what lies between the rows of a result with a leading dimension).  Each epilogue warp stores a (columns, w, h, n) box
   // holding its 32 pixels and 32 columns: 128-byte rows of fp32, 64-byte rows
   // (64-byte swizzle) of half.
   CUtensorMap tout;
@@ -483,7 +484,7 @@ int launchIgemm(plb_context *ctx, const IgemmProblem &p, const plb_plan &plan) {
   const int sub_3 = 32 / (a.sub_w * a.sub_h);
   a.use_tma_store = 0;
   if (!split && (p.plan_flags & PLB_PLAN_NO_TMA_STORE) == 0 &&
-      (reinterpret_cast<uintptr_t>(p.out) & 15) == 0 &&
+      (reinterpret_cast<uintptr_t>(p.out) & 15) == 0 && (size_t(p.n_total) * out_es) % 16 == 0 &&
       (size_t(p.ldc) * out_es) % 16 == 0 && (size_t(out_stride_h) * out_es) % 16 == 0 &&
       (size_t(out_stride_n) * out_es) % 16 == 0 && (groups == 1 || (size_t(p.out_group_stride) * out_es) % 16 == 0)) {
     uint64_t dims[5] = {uint64_t(p.n_total)}, strides[4];

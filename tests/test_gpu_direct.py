@@ -94,6 +94,21 @@ def test_small_products(gpu_ctx, general_ctx, dtype, ta, tb, pad, offset):
 
 
 @pytest.mark.parametrize("out", [capi.HALF, capi.FLOAT])
+@pytest.mark.parametrize("n", [7, 45, 250])
+def test_nothing_is_written_between_rows_of_whole_vectors(gpu_ctx, general_ctx, n, out):
+    """Rows of results that start on 16 bytes and end between: a column slice of a wider matrix."""
+    m, k, ldc = 150, 64, (n + 7) // 8 * 8
+    r = T.rng(n)
+    av, bv = (r.integers(-2, 3, s).astype(np.float64) for s in ((2, m, k), (2, k, n)))
+    desc = capi.MatmulDesc.make(m, k, n, groups=2, output_type=out)
+    desc.ldc = ldc
+    a, b = _operand(av, np.float16, 0, k), _operand(bv, np.float16, 0, n)
+    for ctx in (gpu_ctx, general_ctx):
+        got = _run(ctx, desc, a, b, None, (2, m, n), np.float32 if out == capi.FLOAT else np.float16, ldc, 0)
+        assert (got == av @ bv).all()
+
+
+@pytest.mark.parametrize("out", [capi.HALF, capi.FLOAT])
 @pytest.mark.parametrize("n", [48, 45])
 def test_scaled_and_added(gpu_ctx, n, out):
     g, m, k = 3, 37, 70
