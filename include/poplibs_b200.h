@@ -536,10 +536,11 @@ typedef struct plb_plan {
   int32_t halo_rows;   /* extra input rows per activation load that let one load
                           serve every vertical filter tap (0 = one load per tap) */
   int32_t cta_pair;    /* 1 = clusters of two CTAs share 256-row tensor-core instructions */
-  int32_t in_place;    /* 1 = one launch that reads the operands where they lie and takes no
-                          workspace (kernel 3, and kernel 2 without the rearranged input); the
-                          tiling and workspace here are then what the call has under plan flags
-                          and constraints, or with a result that is not 32-byte aligned */
+  int32_t in_place;    /* 1 = the contraction is one launch that reads the operands where they
+                          lie and takes no workspace (kernel 3, and kernel 2 without the
+                          rearranged input); the tiling and workspace here are then what the call
+                          has under plan flags and constraints, or with a result that is not
+                          32-byte aligned (3-D, flipped and dilated inputs are rearranged first) */
   uint64_t flops;      /* 2 * MACs (padding excluded)                        */
   uint64_t bytes;      /* operands read once + output written once           */
   uint64_t workspace_bytes;
