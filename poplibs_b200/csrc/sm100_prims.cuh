@@ -267,6 +267,16 @@ __device__ __forceinline__ void umma_commit(uint32_t bar) {
       : "memory");
 }
 
+// Zeros to 32 columns of the warp's 32 lanes; tmem_st_wait() before they are read.
+__device__ __forceinline__ void tmem_zero_32x32(uint32_t taddr) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+      "{%1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, "
+      "%1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1};" ::"r"(taddr), "r"(0u)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
 // 32 lanes x 32 consecutive 32-bit columns: thread i of the warp receives
 // lane (base lane + i), registers j = columns (base column + j).
 __device__ __forceinline__ void tmem_ld_32x32(uint32_t taddr, uint32_t (&v)[32]) {
@@ -357,44 +367,42 @@ __device__ __forceinline__ void umma_ss(uint32_t tmem_d, uint64_t adesc, uint64_
 }
 
 // ---- programmatic dependent launch -------------------------------------------
-// The same fp16 instruction with a collector hint for the A operand.  Consecutive
-// instructions of one thread that read the same A tile (same descriptor, same
-// shape) can keep it in the tensor core's collector buffer instead of fetching
-// it from shared memory again: the first says fill, the following ones use,
-// the last one lastuse.  kHint: 1 = fill, 2 = use, 3 = lastuse.
+// The fp16 instruction where `on` holds, for a warp that issues together: with one thread in a
+// branch of its own, the compiler moves the operands to the uniform registers for each instruction.
+// kHint is for the A operand: consecutive instructions that read the same A tile (same
+// descriptor, same shape) can keep it in the tensor core's collector buffer instead of fetching
+// it from shared memory again: 1 = fill, 2 = use, 3 = last use, 0 = neither.
 template <int kHint>
-__device__ __forceinline__ void umma_ss_f16_collect_a(uint32_t tmem_d, uint64_t adesc,
-                                                      uint64_t bdesc, uint32_t idesc,
-                                                      uint32_t accumulate) {
-  static_assert(kHint >= 1 && kHint <= 3, "collector hint");
-  if constexpr (kHint == 1) {
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16.collector::a::fill [%0], %1, %2, %3, p;\n\t"
-        "}\n" ::"r"(tmem_d),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
-  } else if constexpr (kHint == 2) {
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16.collector::a::use [%0], %1, %2, %3, p;\n\t"
-        "}\n" ::"r"(tmem_d),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
-  } else {
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16.collector::a::lastuse [%0], %1, %2, %3, p;\n\t"
-        "}\n" ::"r"(tmem_d),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
-  }
+__device__ __forceinline__ void umma_ss_f16_if(uint32_t on, uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
+                                               uint32_t idesc, uint32_t accumulate) {
+#define PLB_UMMA_IF(collector)                                                                      \
+  asm volatile(                                                                                     \
+      "{\n\t"                                                                                       \
+      ".reg .pred p, q;\n\t"                                                                        \
+      "setp.ne.b32 p, %4, 0;\n\t"                                                                   \
+      "setp.ne.b32 q, %5, 0;\n\t"                                                                   \
+      "@q tcgen05.mma.cta_group::1.kind::f16" collector " [%0], %1, %2, %3, p;\n\t"                 \
+      "}\n" ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(on) : "memory")
+  if constexpr (kHint == 0)
+    PLB_UMMA_IF("");
+  else if constexpr (kHint == 1)
+    PLB_UMMA_IF(".collector::a::fill");
+  else if constexpr (kHint == 2)
+    PLB_UMMA_IF(".collector::a::use");
+  else
+    PLB_UMMA_IF(".collector::a::lastuse");
+#undef PLB_UMMA_IF
+}
+// The same on the accumulator lanes whose bits in `keep_lo` (lanes 0-63) and `keep_hi` are clear.
+__device__ __forceinline__ void umma_ss_f16_masked(uint32_t on, uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
+                                                   uint32_t idesc, uint32_t keep_lo, uint32_t keep_hi) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p, q;\n\t"
+      "setp.eq.b32 p, 0, 0;\n\t"
+      "setp.ne.b32 q, %6, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%4, %4, %5, %5}, p;\n\t"
+      "}\n" ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(keep_lo), "r"(keep_hi), "r"(on) : "memory");
 }
 
 // A kernel launched with the programmatic-stream-serialization attribute may

@@ -238,8 +238,52 @@ void planWu(const WuProblem &p, int sm_count, int force_split, unsigned plan_fla
       best = sbest;
     }
   }
+  // Both halves of the instruction's rows for up to 64 output channels: where a 16-pixel step
+  // lies in one row, and all tiles then take less.  A tile takes what its instructions do (one of
+  // n columns about 35 + 0.47 n cycles: measured 75, 95, 155 at 64, 128 and 256), or its way into
+  // and out of shared memory at 100 bytes a cycle (measured 91 to 110); and the tiles of a CTA
+  // have to win the 2000 cycles that clearing the accumulators and the edge rows cost (3x3 float,
+  // 20 -> 36, 4 images of 33 x 29, four tiles a CTA: 12.6 us unpaired, 13.3 paired).
+  a->pair_rows = a->pair_shift = 0;
+  if (a->strip_mode && co <= 64) {
+    const int rows = (s.KH + 1) / 2, shift = rows * s.dilH;
+    auto cost = [&](int filter_rows, int fill) {
+      const int each = a->ci_blk == 64 ? std::min(4, filter_rows) : 1, count = (filter_rows + each - 1) / each;
+      const double columns = filter_rows * a->ci_blk;
+      return std::max(4 * (35 * count + 0.47 * columns), (fill + 4 * (4096 * count + 32 * columns)) / 100);
+    };
+    const double before = best * cost(s.KH, stage_bytes - kWuBlockBytes);
+    const int columns = a->sgroups * a->ci_blocks * s.KW;
+    const double splits = force_split > 0 ? force_split : std::max(1, (sm_count > 0 ? sm_count : 148) / columns);
+    double least = std::min(0.97 * before, before - 2000 * splits);
+    for (int h = 4; h >= 1; h >>= 1)
+      for (int w = 64 / h; w >= 1; w >>= 1) {
+        const int n = 64 / (w * h), dy_rows = w * n * (h + shift), strip_rows = w * n * (h + (rows - 1) * s.dilH);
+        const int bytes = (dy_rows + a->ci_blk64 * strip_rows) * 128;
+        if (h + shift > 256 || (w - 1) * s.strW + 1 > 256 || 3 * bytes > 200 * 1024) continue;
+        const long tiles = long((s.OWc + w - 1) / w) * ((s.OHc + shift + h - 1) / h) * ((long(p.batch) + n - 1) / n);
+        if (tiles * cost(rows, bytes) >= least) continue;
+        least = tiles * cost(rows, bytes);
+        a->box_w = w;
+        a->box_h = h;
+        a->box_n = n;
+        a->pair_rows = rows;
+        a->pair_shift = shift;
+        a->dy_rows = dy_rows;
+        a->strip_rows = strip_rows;
+        stage_bytes = bytes;
+        best = tiles;
+      }
+    if (a->pair_rows) {
+      a->halo_step_bytes = s.dilH * a->box_w * a->box_n * 128;
+      a->taps_per_group = rows;
+      a->tmem_cols = 32;
+      while (a->tmem_cols < rows * a->ci_blk) a->tmem_cols <<= 1;
+      a->last_row = s.OHc;
+    }
+  }
   a->tiles_w = (s.OWc + a->box_w - 1) / a->box_w;
-  a->tiles_h = (s.OHc + a->box_h - 1) / a->box_h;
+  a->tiles_h = (s.OHc + a->pair_shift + a->box_h - 1) / a->box_h;
   a->tiles_n = (int(p.batch) + a->box_n - 1) / a->box_n;
   a->stage_bytes = stage_bytes;
   a->stages = std::max(2, std::min(kWuMaxStages, (200 * 1024) / stage_bytes));
@@ -260,7 +304,7 @@ void planWu(const WuProblem &p, int sm_count, int force_split, unsigned plan_fla
     plan->tiles = units;
     plan->grid = units * ksplit;
     plan->b_mn_major = 1;
-    plan->halo_rows = a->strip_mode ? halo : 0;
+    plan->halo_rows = a->pair_rows ? a->pair_shift : a->strip_mode ? halo : 0;
     plan->workspace_bytes = size_t(ksplit) * p.sgroups * taps * co * ci * sizeof(float);
   }
 }
@@ -296,7 +340,8 @@ int configureWuKernel(int device) {
   std::lock_guard<std::mutex> lock(mutex);
   if (!configured[device]) {
     // the caller has made `device` current
-    PLB_CUDA(cudaFuncSetAttribute(wu_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    for (auto *kernel : {wu_kernel<false>, wu_kernel<true>})
+      PLB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
     configured[device] = true;
   }
   return PLB_OK;
@@ -410,14 +455,14 @@ int launchWuKernel(cudaStream_t stream, const WuProblem &p, const WuArgs &a) {
   }
   // pixel dimensions (w, h, n); strip mode orders them (w, n, h)
   const bool strip = a.strip_mode != 0;
-  const int halo = strip ? (s.KH - 1) * s.dilH : 0;
+  const int halo = strip ? ((a.pair_rows ? a.pair_rows : s.KH) - 1) * s.dilH : 0;
   const uint64_t batch = uint64_t(p.batch);
   {
     const uint64_t dims[4] = {p.dy_chans, uint64_t(s.OWc), strip ? batch : uint64_t(s.OHc),
                               strip ? uint64_t(s.OHc) : batch};
     const uint64_t strides[3] = {p.dy_strides[0], p.dy_strides[strip ? 2 : 1], p.dy_strides[strip ? 1 : 2]};
     const uint32_t box[4] = {64, uint32_t(a.box_w), uint32_t(strip ? a.box_n : a.box_h),
-                             uint32_t(strip ? a.box_h : a.box_n)};
+                             uint32_t(strip ? a.box_h + a.pair_shift : a.box_n)};
     if (int rc = encodeTensorMap(&tdy, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4,
                                  static_cast<const uint8_t *>(p.dy) + uint64_t(s.opH) * p.dy_strides[1] +
                                      uint64_t(s.opW) * p.dy_strides[0],
@@ -451,7 +496,7 @@ int launchWuKernel(cudaStream_t stream, const WuProblem &p, const WuArgs &a) {
   cfg.stream = stream;
   cfg.attrs = pdl;
   cfg.numAttrs = 1;
-  PLB_CUDA(cudaLaunchKernelEx(&cfg, wu_kernel, tdy, tx, tout, a));
+  PLB_CUDA(cudaLaunchKernelEx(&cfg, a.pair_rows ? wu_kernel<true> : wu_kernel<false>, tdy, tx, tout, a));
   PLB_CUDA(cudaGetLastError());
   return PLB_OK;
 }

@@ -1,0 +1,81 @@
+"""Weight gradients of up to 64 output channels whose filter rows are shared out between the two
+halves of the tensor-core instruction's rows (poplibs_b200/csrc/wu_sm100.cuh), against the oracle.
+
+Small-integer data are exact in fp32 sums: bit for bit.
+"""
+import numpy as np
+import pytest
+
+import common as T
+import oracle
+from poplibs_b200 import capi
+
+pytestmark = pytest.mark.gpu
+
+# images, field, kernel, channels in / out, other parameters: even and odd numbers of filter rows
+# (the odd ones leave half a row of accumulators unused), steps of one and several instructions,
+# rows of 16 to 64 pixels and of several images, rows of tiles that end inside a box, above it and
+# below it, dilated rows, a horizontal stride, more than 64 input channels, and first layers
+LAYERS = {
+    "3x3": (5, (34, 48), (3, 3), 64, 64, dict(padding=1)),
+    "3x3, 24 out": (2, (17, 64), (3, 3), 64, 24, dict(padding=1)),
+    "2 rows": (24, (12, 48), (2, 1), 64, 64, {}),
+    "4 rows": (2, (19, 35), (4, 3), 40, 8, dict(padding=1)),
+    "5x5": (8, (12, 48), (5, 5), 64, 64, dict(padding=2)),
+    "7 rows": (4, (24, 48), (7, 2), 64, 56, dict(padding=3)),
+    "8 rows": (2, (24, 16), (8, 1), 32, 32, dict(in_pad_lo=[3, 0], in_pad_hi=[4, 0])),
+    "many small images": (70, (14, 14), (3, 3), 64, 64, dict(padding=1)),
+    "dilated": (24, (17, 32), (3, 3), 64, 64, dict(k_dilation=[3, 2], padding=[3, 2])),
+    "strided columns": (32, (13, 64), (3, 3), 64, 64, dict(stride=[1, 2], padding=1)),
+    "128 in": (2, (24, 32), (3, 3), 128, 64, dict(padding=1)),
+    "160 in, 2 rows": (1, (24, 32), (2, 3), 160, 40, dict(padding=1)),
+    "first, 7x7/2": (2, (64, 96), (7, 7), 3, 64, dict(stride=2, padding=3)),
+    "first, 3x3": (24, (30, 30), (3, 3), 3, 32, dict(padding=1)),
+    "no padding": (2, (33, 33), (3, 3), 64, 64, {}),
+    "output truncated": (2, (32, 32), (3, 3), 64, 64, dict(padding=1, out_trunc_lo=[2, 0], out_trunc_hi=[1, 0])),
+}
+
+
+def _params(name):
+    n, field, kernel, ci, co, kw = LAYERS[name]
+    return capi.ConvParams.make(n, list(field), list(kernel), ci, co, **kw)
+
+
+@pytest.mark.parametrize("name", LAYERS)
+def test_wu_pair_matches_oracle(gpu_ctx, name):
+    p = _params(name)
+    n, field, _, ci, co, _ = LAYERS[name]
+    r = T.rng(len(name))
+    x = T.small_int_half(r, (n, ci) + field)
+    dy = T.small_int_half(r, (n, co) + tuple(p.output_field()))
+    want, _ = oracle.conv_wu(T.spec_from_params(p), x, dy)
+    plan = capi.conv_wu_plan(p, capi.ConvOptions.make(split_k=1))
+    ci_blk = 64 if name.startswith("first") else min(256, (ci + 31) // 32 * 32)
+    kernel_h = 4 if name == "first, 7x7/2" else p.kernel[0]  # (rearranged)
+    assert plan.tile_n == (kernel_h + 1) // 2 * ci_blk and plan.halo_rows > 0
+    for split in (0, 1, 3):
+        _, got = T.gpu_conv_wu(p, x, dy, opt=capi.ConvOptions.make(split_k=split))  # (1: paired, 0: if it pays)
+        assert (got.astype(np.float64) == want.reshape(got.shape)).all(), split
+
+
+@pytest.mark.parametrize("value", [np.inf, np.nan])
+@pytest.mark.parametrize("row", [0, 1, -2, -1])
+@pytest.mark.parametrize("pad", [1, 0])
+def test_wu_pair_keeps_infinities_of_edge_rows_to_their_taps(gpu_ctx, pad, row, value):
+    """Rows of the walk that have output gradients for one half only give the other half nothing."""
+    n, ci, co, oh, ow = 12, 64, 64, 34, 48  # (whole boxes of columns)
+    height, width = oh + 2 * (1 - pad), ow + 2 * (1 - pad)
+    p = capi.ConvParams.make(n, [height, width], [3, 3], ci, co, padding=pad)
+    opt = capi.ConvOptions.make(split_k=2)
+    assert capi.conv_wu_plan(p, opt).tile_n == 128
+    r = T.rng(5)
+    x = T.small_int_half(r, (n, ci, height, width))
+    dy = T.small_int_half(r, (n, co, oh, ow), 1, 4)
+    row %= height
+    x[0, 3, row, 9] = value
+    _, got = T.gpu_conv_wu(p, x, dy, opt=opt)
+    finite = np.isfinite(got[0])
+    assert finite[:, [c for c in range(ci) if c != 3]].all()
+    for k in range(3):
+        # tap k meets the input row where output row `row` + pad - k exists
+        assert finite[:, 3, k].all() != (0 <= row + pad - k < oh), k
