@@ -224,6 +224,12 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
              const __grid_constant__ CUtensorMap tm_out, const IgemmArgs args) {
   using S = IgemmSmem<BN, kResB, k2Cta>;
   static_assert(!k2Cta || !kBMn || BN >= 128, "a CTA needs a whole 64-column block of MN-major B");
+  // Copies are issued by warps that walk together, one lane of which copies, so that their operands
+  // stay in uniform registers (one thread in a branch of its own moves them there one by one): what
+  // they are made from is the same in all lanes, as the compiler sees it.  64 products 256 x 64 x 256
+  // 5.5 -> 5.1 us, one 56 x 56 image 5.3 -> 5.0, ragged 197 x 770 x 1003 10.2 -> 9.8.  CTA pairs keep one thread a
+  // role: their register budget is used up (3x3 of 128 channels, 256 images of 28 x 28, 45 -> 51 us).
+  constexpr bool kWalk = !k2Cta;
   const uint32_t cta_rank = k2Cta ? cluster_cta_rank() : 0u;
   const bool leader = cta_rank == 0;
   constexpr int kMaxStages = kIgemmMaxStages;
@@ -258,7 +264,7 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
       reinterpret_cast<volatile uint32_t *>(bar_gen + 8 * (2 * kMaxStages + 6));
   volatile int *abort_flag = reinterpret_cast<volatile int *>(bar_gen + 8 * (2 * kMaxStages + 7));
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = kWalk ? __shfl_sync(0xffffffffu, int(threadIdx.x >> 5), 0) : int(threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
 
   // Set-up is spread over the warps: the lanes of warp 0 initialise the barrier
@@ -400,8 +406,8 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
   };
 
   // B tile of K step (r, s, kc) -> shared memory at `dst`; with kPrefetch the
-  // same box is only pulled towards L2
-  auto load_b = [&](uint32_t dst, uint32_t bar, int group, int r, int s, int kc, int n_col, bool prefetch) {
+  // same box is only pulled towards L2.  All lanes of a warp call, the one with `on` copies.
+  auto load_b = [&](uint32_t on, uint32_t dst, uint32_t bar, int group, int r, int s, int kc, int n_col, bool prefetch) {
     const int b_tap = ((args.flip_h ? args.taps_h - 1 - r : r) * args.tap_step_h + args.tap_first_h) * args.tap_pitch_h +
                       (args.flip_w ? args.taps_w - 1 - s : s) * args.tap_step_w + args.tap_first_w +
                       (kGroups ? group * args.taps_stored : 0);
@@ -412,7 +418,8 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
       // K rows x 64 columns per block; blocks of 64 columns are 64 rows apart
 #pragma unroll
       for (int j = 0; j < kMyN / 64; ++j) {
-        if (prefetch)
+        if (!on) {
+        } else if (prefetch)
           tma_prefetch_l2_3d(&tm_b, my_col + j * 64, kc * 64, b_tap);
         else if constexpr (k2Cta)
           tma_load_3d_pair(dst + j * (64 * kStageKBytes), &tm_b, bar, my_col + j * 64, kc * 64,
@@ -421,7 +428,8 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
           tma_load_3d(dst + j * (64 * kStageKBytes), &tm_b, bar, my_col + j * 64, kc * 64, b_tap);
       }
     } else {
-      if (prefetch)
+      if (!on) {
+      } else if (prefetch)
         tma_prefetch_l2_3d(&tm_b, kc * kElemsPerStage, my_col, b_tap);
       else if constexpr (k2Cta)
         tma_load_3d_pair(dst, &tm_b, bar, kc * kElemsPerStage, my_col, b_tap);
@@ -444,12 +452,13 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
   // resident, the weight tile(s) of step (r, s, kc) -> stage memory at a_dst
   // (or, before the predecessor kernel is known to have finished, only
   // towards L2).
-  auto issue_step = [&](bool prefetch, uint32_t a_dst, uint32_t full, int group, int r, int s, int kc,
+  auto issue_step = [&](uint32_t on, bool prefetch, uint32_t a_dst, uint32_t full, int group, int r, int s, int kc,
                         int w_base, int h_base, int n0, int n_col) {
     if constexpr (kAMn) {
       // [k][m] rows of one group: two boxes of 64 K rows x 64 output rows
         for (int j = 0; j < args.a_blocks; ++j) {
-        if (prefetch)
+        if (!on) {
+        } else if (prefetch)
           tma_prefetch_l2_3d(&tm_a, w_base + j * 64, kc * 64, group);
         else if constexpr (k2Cta)
           tma_load_3d_pair(a_dst + j * (64 * kStageKBytes), &tm_a, full, w_base + j * 64, kc * 64, group);
@@ -460,7 +469,8 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
       const int cw = w_base + s * args.dil_w, ch = h_base + r * args.dil_h;
       const int c2 = args.h_outer ? n0 : ch, c3 = args.h_outer ? ch : n0;
       const int ck = kc * kElemsPerStage;
-      if (kGroups) {
+      if (!on) {
+      } else if (kGroups) {
         if (prefetch)
           tma_prefetch_l2_5d(&tm_a, ck, group, cw, c2, c3);
         else if constexpr (k2Cta)
@@ -479,7 +489,7 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
       // with a halo strip the stage carries the weight tiles of every filter row
       const int row_taps = kHalo ? args.taps_h : 1;
       for (int rr = 0; rr < row_taps; ++rr)
-        load_b(a_dst + args.a_stage_bytes + rr * S::kBBytes, full, group, kHalo ? rr : r, s, kc, n_col,
+        load_b(on, a_dst + args.a_stage_bytes + rr * S::kBBytes, full, group, kHalo ? rr : r, s, kc, n_col,
                prefetch);
     }
   };
@@ -497,24 +507,29 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
   const int first_loads = min(first_steps, args.first_loads), first_prefetches = min(first_steps, args.first_prefetches);
   // Step f_begin + i of the first unit towards L2 while the predecessor kernel may
   // still be running, and with `load`, once it has finished, into stage i.
-  auto first_step = [&](int i, bool load) {
+  auto first_step = [&](uint32_t on, int i, bool load) {
     int m_idx, n_idx, w0, h0, n0, r, s, kc;
     tile_coords(f_tile, m_idx, n_idx);
     tile_origin(m_idx, w0, h0, n0);
     step_coords(f_begin + i, r, s, kc);
     const uint32_t dst = smem_base + i * stage_bytes, full = lead_bar(full_bar(i));
     const int w_base = w0 * args.stride_w - args.pad_w, h_base = h0 * args.stride_h - args.pad_h;
-    if (kResB || i < first_prefetches) issue_step(true, dst, full, f_group, r, s, kc, w_base, h_base, n0, n_idx * BN);
+    if (kResB || i < first_prefetches) issue_step(on, true, dst, full, f_group, r, s, kc, w_base, h_base, n0, n_idx * BN);
     if (!load) return;
     wait_predecessor();
-    if (leader)
+    if (leader && on)
       mbar_expect_tx(full_bar(i), kPairFactor * uint32_t(args.stage_tx_bytes));
-    issue_step(false, dst, full, f_group, r, s, kc, w_base, h_base, n0, n_idx * BN);
+    issue_step(on, false, dst, full, f_group, r, s, kc, w_base, h_base, n0, n_idx * BN);
   };
 
   if (warp < P) {
     // ===================== TMA producers =====================
-    if (elect_one()) {
+    const uint32_t on = elect_one() ? 1u : 0u;
+    auto wait = [&](uint32_t bar, uint32_t parity) {
+      const bool done = mbar_wait(bar, parity, abort_flag);
+      return kWalk ? __all_sync(0xffffffffu, done) != 0 : done;
+    };
+    if (kWalk || on) {
       const int me = warp;
       int stage = me;          // stage of this producer's next K step
       uint32_t phase = 0;
@@ -522,7 +537,7 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
       bool ok = true;
       [[maybe_unused]] int trace_slot = 0;
       if constexpr (kResB)
-        for (int i = me; i < first_steps; i += P) first_step(i, false);
+        for (int i = me; i < first_steps; i += P) first_step(on, i, false);
       wait_predecessor();
       if (me == 0) PLB_TRACE_STAMP(2, 4002);
       for (int unit = first_unit; unit < total_units && ok; unit += unit_stride) {
@@ -550,16 +565,16 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
             }
           } else if (turn == me) {
             if (me == 0) { PLB_TRACE_STAMP(0, trace_slot); ++trace_slot; }
-            if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag)) {
+            if (!wait(empty_bar(stage), phase ^ 1u)) {
               atomicCAS(args.status, kStatusOk, kStatusProducerTimeout);
               ok = false;
               break;
             }
             if (me == 0) { PLB_TRACE_STAMP(0, trace_slot); ++trace_slot; }
             const uint32_t a_dst = smem_base + stage * stage_bytes;
-            if (leader) mbar_expect_tx(full_bar(stage), kPairFactor * uint32_t(args.stage_tx_bytes));
+            if (leader && on) mbar_expect_tx(full_bar(stage), kPairFactor * uint32_t(args.stage_tx_bytes));
             const uint32_t full = lead_bar(full_bar(stage));
-            issue_step(false, a_dst, full, group, r, s, kc, w_base, h_base, n0, n_col);
+            issue_step(on, false, a_dst, full, group, r, s, kc, w_base, h_base, n0, n_col);
             if (me == 0) { PLB_TRACE_STAMP(0, trace_slot); ++trace_slot; }
             stage += P;
             if (stage >= kStages) {
@@ -584,7 +599,7 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
         // (the producer whose turn it would be: its stage and phase are the next step's)
         if (!leader && ok && turn == me)
           for (int i = 0; i < kStages && ok; ++i) {
-            ok = mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag);
+            ok = wait(empty_bar(stage), phase ^ 1u);
             if (!ok) atomicCAS(args.status, kStatusOk, kStatusDrainTimeout);
             if (++stage == kStages) {
               stage = 0;
@@ -789,26 +804,28 @@ igemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ C
       // copies (a copy costs its issuing thread some hundred cycles, and the
       // first MMA waits for all of them), leaving the producers free to start
       // on the activations at once.
-      if (lane == 0 && first_unit < total_units) {
+      const uint32_t on = elect_one() ? 1u : 0u;
+      if ((kWalk || on) && first_unit < total_units) {
         for (int it = warp - 4; it < k_iters; it += 16) {
           int r, s, kc;
           step_coords(it, r, s, kc);
-          load_b(0u, 0u, f_group, r, s, kc, 0, true);
+          load_b(on, 0u, 0u, f_group, r, s, kc, 0, true);
         }
         wait_predecessor();
-        if (warp == 4 && leader)
+        if (warp == 4 && leader && on)
           mbar_expect_tx(resb_bar, kPairFactor * uint32_t(k_iters * args.b_box_bytes));
         const uint32_t resb_bar_lead = lead_bar(resb_bar);
         for (int it = warp - 4; it < k_iters; it += 16) {
           int r, s, kc;
           step_coords(it, r, s, kc);
-          load_b(resb_base + it * S::kBBytes, resb_bar_lead, f_group, r, s, kc, 0, false);
+          load_b(on, resb_base + it * S::kBBytes, resb_bar_lead, f_group, r, s, kc, 0, false);
         }
         if (warp == 4) PLB_TRACE_STAMP(2, 4012);
       }
       __syncwarp();
     } else {
-      if (lane == 0 && warp - 4 < max(first_loads, first_prefetches)) first_step(warp - 4, warp - 4 < first_loads);
+      const uint32_t on = elect_one() ? 1u : 0u;
+      if ((kWalk || on) && warp - 4 < max(first_loads, first_prefetches)) first_step(on, warp - 4, warp - 4 < first_loads);
       __syncwarp();
     }
     wait_predecessor();

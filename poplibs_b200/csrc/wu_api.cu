@@ -238,32 +238,36 @@ void planWu(const WuProblem &p, int sm_count, int force_split, unsigned plan_fla
       best = sbest;
     }
   }
-  // Both halves of the instruction's rows for up to 64 output channels: where a 16-pixel step
-  // lies in one row, and all tiles then take less.  A tile takes what its instructions do (one of
-  // n columns about 35 + 0.47 n cycles: measured 75, 95, 155 at 64, 128 and 256), or its way into
-  // and out of shared memory at 100 bytes a cycle (measured 91 to 110); and the tiles of a CTA
+  // Both halves of the instruction's rows for 64 output channels (fewer: the copies take longer
+  // than the instructions): where a 16-pixel step lies in one row, and all tiles then take less.  A tile takes what its instructions do (one of
+  // n columns about 35 + 0.47 n cycles: measured 75, 95, 155 at 64, 128 and 256), its way into
+  // and out of shared memory at 100 bytes a cycle (measured 91 to 110), or its copies by pixel (3.1
+  // cycles, 7.5 where its channels do not fill 128 bytes); and the tiles of a CTA
   // have to win the 2000 cycles that clearing the accumulators and the edge rows cost (3x3 float,
-  // 20 -> 36, 4 images of 33 x 29, four tiles a CTA: 12.6 us unpaired, 13.3 paired).
+  // 20 -> 36, 4 images of 33 x 29, four tiles a CTA: 12.6 us unpaired, 13.3 paired).  Boxes are eight pixels wide
+  // and more: of single columns of 16 images, 3x3, 4 groups of 16, 16 images of 107 x 107 took 44 us,
+  // unpaired 34.
   a->pair_rows = a->pair_shift = 0;
-  if (a->strip_mode && co <= 64) {
+  if (a->strip_mode && co == 64) {
     const int rows = (s.KH + 1) / 2, shift = rows * s.dilH;
-    auto cost = [&](int filter_rows, int fill) {
+    auto cost = [&](int filter_rows, int dy_rows, int x_rows) {
       const int each = a->ci_blk == 64 ? std::min(4, filter_rows) : 1, count = (filter_rows + each - 1) / each;
-      const double columns = filter_rows * a->ci_blk;
-      return std::max(4 * (35 * count + 0.47 * columns), (fill + 4 * (4096 * count + 32 * columns)) / 100);
+      const double columns = filter_rows * a->ci_blk, fill = (dy_rows + a->ci_blk64 * x_rows) * 128.0;
+      const double copies = dy_rows * 3.1 + a->ci_blk64 * x_rows * (ci % 64 ? 7.5 : 3.1);
+      return std::max({4 * (35 * count + 0.47 * columns), (fill + 4 * (4096 * count + 32 * columns)) / 100, copies});
     };
-    const double before = best * cost(s.KH, stage_bytes - kWuBlockBytes);
+    const double before = best * cost(s.KH, 64, a->strip_rows);
     const int columns = a->sgroups * a->ci_blocks * s.KW;
     const double splits = force_split > 0 ? force_split : std::max(1, (sm_count > 0 ? sm_count : 148) / columns);
-    double least = std::min(0.97 * before, before - 2000 * splits);
+    double least = std::min(0.94 * before, before - 2000 * splits);
     for (int h = 4; h >= 1; h >>= 1)
       for (int w = 64 / h; w >= 1; w >>= 1) {
         const int n = 64 / (w * h), dy_rows = w * n * (h + shift), strip_rows = w * n * (h + (rows - 1) * s.dilH);
         const int bytes = (dy_rows + a->ci_blk64 * strip_rows) * 128;
         if (h + shift > 256 || (w - 1) * s.strW + 1 > 256 || 3 * bytes > 200 * 1024) continue;
         const long tiles = long((s.OWc + w - 1) / w) * ((s.OHc + shift + h - 1) / h) * ((long(p.batch) + n - 1) / n);
-        if (tiles * cost(rows, bytes) >= least) continue;
-        least = tiles * cost(rows, bytes);
+        if (w < 8 || tiles * cost(rows, dy_rows, strip_rows) >= least) continue;
+        least = tiles * cost(rows, dy_rows, strip_rows);
         a->box_w = w;
         a->box_h = h;
         a->box_n = n;
@@ -293,8 +297,9 @@ void planWu(const WuProblem &p, int sm_count, int force_split, unsigned plan_fla
   a->ksplit = ksplit;
   if (plan) {
     plan->kernel = 1;
-    plan->tile_m = 128;
-    plan->tile_n = a->taps_per_group * a->ci_blk;
+    // (paired: 64 output channels' sums of all filter rows)
+    plan->tile_m = a->pair_rows ? 64 : 128;
+    plan->tile_n = (a->pair_rows ? s.KH : a->taps_per_group) * a->ci_blk;
     plan->tile_k_bytes = kWuPixelsPerStage * 2;
     plan->box_w = a->box_w;
     plan->box_h = a->box_h;

@@ -1,4 +1,4 @@
-"""Weight gradients of up to 64 output channels whose filter rows are shared out between the two
+"""Weight gradients of 64 output channels whose filter rows are shared out between the two
 halves of the tensor-core instruction's rows (poplibs_b200/csrc/wu_sm100.cuh), against the oracle.
 
 Small-integer data are exact in fp32 sums: bit for bit.
@@ -18,19 +18,19 @@ pytestmark = pytest.mark.gpu
 # below it, dilated rows, a horizontal stride, more than 64 input channels, and first layers
 LAYERS = {
     "3x3": (5, (34, 48), (3, 3), 64, 64, dict(padding=1)),
-    "3x3, 24 out": (2, (17, 64), (3, 3), 64, 24, dict(padding=1)),
+    "3x3, one image": (1, (49, 64), (3, 3), 64, 64, dict(padding=1)),
     "2 rows": (24, (12, 48), (2, 1), 64, 64, {}),
-    "4 rows": (2, (19, 35), (4, 3), 40, 8, dict(padding=1)),
+    "4 rows": (6, (19, 32), (4, 3), 64, 64, dict(padding=1)),
     "5x5": (8, (12, 48), (5, 5), 64, 64, dict(padding=2)),
-    "7 rows": (4, (24, 48), (7, 2), 64, 56, dict(padding=3)),
-    "8 rows": (2, (24, 16), (8, 1), 32, 32, dict(in_pad_lo=[3, 0], in_pad_hi=[4, 0])),
-    "many small images": (70, (14, 14), (3, 3), 64, 64, dict(padding=1)),
+    "7 rows": (4, (24, 48), (7, 2), 64, 64, dict(padding=3)),
+    "8 rows": (6, (24, 16), (8, 1), 64, 64, dict(in_pad_lo=[3, 0], in_pad_hi=[4, 0])),
+    "many small images": (101, (13, 8), (3, 3), 64, 64, dict(padding=1)),
     "dilated": (24, (17, 32), (3, 3), 64, 64, dict(k_dilation=[3, 2], padding=[3, 2])),
     "strided columns": (32, (13, 64), (3, 3), 64, 64, dict(stride=[1, 2], padding=1)),
     "128 in": (2, (24, 32), (3, 3), 128, 64, dict(padding=1)),
-    "160 in, 2 rows": (1, (24, 32), (2, 3), 160, 40, dict(padding=1)),
+    "160 in, 2 rows": (8, (24, 32), (2, 3), 160, 64, dict(padding=1)),
     "first, 7x7/2": (2, (64, 96), (7, 7), 3, 64, dict(stride=2, padding=3)),
-    "first, 3x3": (24, (30, 30), (3, 3), 3, 32, dict(padding=1)),
+    "first, 3x3": (8, (34, 64), (3, 3), 3, 64, dict(padding=1)),
     "no padding": (2, (33, 33), (3, 3), 64, 64, {}),
     "output truncated": (2, (32, 32), (3, 3), 64, 64, dict(padding=1, out_trunc_lo=[2, 0], out_trunc_hi=[1, 0])),
 }
@@ -50,9 +50,7 @@ def test_wu_pair_matches_oracle(gpu_ctx, name):
     dy = T.small_int_half(r, (n, co) + tuple(p.output_field()))
     want, _ = oracle.conv_wu(T.spec_from_params(p), x, dy)
     plan = capi.conv_wu_plan(p, capi.ConvOptions.make(split_k=1))
-    ci_blk = 64 if name.startswith("first") else min(256, (ci + 31) // 32 * 32)
-    kernel_h = 4 if name == "first, 7x7/2" else p.kernel[0]  # (rearranged)
-    assert plan.tile_n == (kernel_h + 1) // 2 * ci_blk and plan.halo_rows > 0
+    assert plan.tile_m == 64
     for split in (0, 1, 3):
         _, got = T.gpu_conv_wu(p, x, dy, opt=capi.ConvOptions.make(split_k=split))  # (1: paired, 0: if it pays)
         assert (got.astype(np.float64) == want.reshape(got.shape)).all(), split
@@ -67,7 +65,7 @@ def test_wu_pair_keeps_infinities_of_edge_rows_to_their_taps(gpu_ctx, pad, row, 
     height, width = oh + 2 * (1 - pad), ow + 2 * (1 - pad)
     p = capi.ConvParams.make(n, [height, width], [3, 3], ci, co, padding=pad)
     opt = capi.ConvOptions.make(split_k=2)
-    assert capi.conv_wu_plan(p, opt).tile_n == 128
+    assert capi.conv_wu_plan(p, opt).tile_m == 64
     r = T.rng(5)
     x = T.small_int_half(r, (n, ci, height, width))
     dy = T.small_int_half(r, (n, co, oh, ow), 1, 4)
