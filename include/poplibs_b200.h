@@ -540,7 +540,8 @@ typedef struct plb_plan {
                           lie and takes no workspace (kernel 3, and kernel 2 without the
                           rearranged input); the tiling and workspace here are then what the call
                           has under plan flags and constraints, or with a result that is not
-                          32-byte aligned (3-D, flipped and dilated inputs are rearranged first) */
+                          32-byte aligned (3-D, flipped and dilated inputs are rearranged first).
+                          A weight gradient's sums of shares of the pixels still take workspace */
   uint64_t flops;      /* 2 * MACs (padding excluded)                        */
   uint64_t bytes;      /* operands read once + output written once           */
   uint64_t workspace_bytes;

@@ -3,6 +3,7 @@
 #include <cmath>
 
 #include "patch.cuh"
+#include "rows.h"
 
 namespace plb {
 
@@ -183,6 +184,7 @@ bool patchable(const IgemmProblem *p, int n, int type) {
 bool patchSuits(int sm_count, const IgemmProblem *p, int n, int type, int contractions, int together, bool copied, bool packed,
                 bool slower_too) {
   if (!patchable(p, n, type)) return false;
+  if (n == 1 && rowsSuits(sm_count, *p, type)) return true;
   const double operand = (type == PLB_FLOAT ? 6.0 : type == PLB_QUARTER ? 1.0 : 2.0) * together * p->k_per_tap;
   const double columns = double(together) * p->n_total, wide = columns <= 64 ? 1 : columns <= 128 ? 1.6 : 2.6;
   const double tile_n = columns <= 64 ? 64 : columns <= 128 ? 128 : 256;
@@ -215,6 +217,7 @@ bool patchSuits(int sm_count, const IgemmProblem *p, int n, int type, int contra
 }
 
 int launchPatch(plb_context *ctx, const IgemmProblem *p, int n, int type, bool repair) {
+  if (n == 1 && rowsSuits(ctx->sm_count, *p, type)) return launchRows(ctx, *p);
   Tiling t;
   const bool act_vec = wholeLoads(*p, type);
   if (!tilingOf(ctx->sm_count, p, n, type, act_vec, &t)) return fail(PLB_ERR_UNSUPPORTED, "no tiling of the patch kernel");

@@ -1,0 +1,28 @@
+// Convolutions of narrow channel groups, a warp to a group (rows.cu), and their weight
+// gradients (rows_wu.cu).
+#pragma once
+
+#include "runtime.h"
+
+namespace plb {
+
+// Whether this problem (`type`: the operands' element type, all pointers the caller's) runs
+// on the kernel that walks the rows of a group with its weights in registers.
+bool rowsSuits(int sm_count, const IgemmProblem &p, int type);
+int launchRows(plb_context *ctx, const IgemmProblem &p);
+
+// Weight gradient of half channel groups, `chans` in and out each, of a kernel x kernel filter with
+// unit strides and dilations.
+struct RowsWuProblem {
+  const void *x, *dy;
+  int groups, chans, kernel, images;
+  int in_w, in_h;              // extent that is read, of rows and images of in_pitch_w, in_pitch_h pixels
+  int in_pitch_w, in_pitch_h;
+  int width, height;           // output pixels
+  int pad_w, pad_h;
+};
+// The shares of the pixels whose sums lie apart, [share][group][tap][out][in]; 0 where it does not suit.
+int rowsWuSplits(int sm_count, const RowsWuProblem &p);
+int launchRowsWu(plb_context *ctx, const RowsWuProblem &p, float *partial);
+
+}  // namespace plb

@@ -6,6 +6,7 @@
 #include <type_traits>
 
 #include "conv_geometry.h"
+#include "rows.h"
 #include "runtime.h"
 #include "small_channel.h"
 #include "wu_sm100.cuh"
@@ -77,6 +78,18 @@ struct WuProblem {
   const void *x = nullptr, *dy = nullptr;
   uint64_t x_chans = 0, dy_chans = 0, x_strides[3] = {}, dy_strides[3] = {};
 };
+
+// Narrow channel groups on the kernel that keeps a group's sums in a warp's registers: the shares of
+// the pixels whose sums it leaves apart, 0 where it does not apply.
+int rowsWuShares(int sm_count, const plb_conv_params &p, const WuShape &s, int force_split, unsigned plan_flags,
+                 const void *x, const void *dy, RowsWuProblem *q) {
+  if (p.input_type != PLB_HALF || force_split != 0 || plan_flags != 0 || p.in_chans_per_group != p.out_chans_per_group) return 0;
+  if (s.KH != s.KW || s.strH != 1 || s.strW != 1 || s.dilH != 1 || s.dilW != 1 || s.opH || s.opW || s.OHc != s.OH || s.OWc != s.OW) return 0;
+  const int c = int(p.in_chans_per_group);
+  *q = RowsWuProblem{static_cast<const uint8_t *>(x) + (size_t(s.tH) * s.W + s.tW) * p.groups * c * 2, dy, int(p.groups), c, s.KH,
+                     int(p.batch), s.We, s.He, s.W, s.H, s.OW, s.OH, s.padW, s.padH};
+  return rowsWuSplits(sm_count, *q);
+}
 
 // How the channels of a pixel lie in the operands the kernel reads, and how many
 // groups are contracted together (every sub'th group starts a super-group).
@@ -640,6 +653,11 @@ int plb_conv_wu_plan(const plb_conv_params *p_in, const plb_conv_options *opt, p
   if (!rearranged) w = generalProblem(*p, s, &x, &dy, &operands);
   planWu(w, 148, opt ? opt->split_k : 0, opt ? opt->plan_flags : 0, &a, plan);
   plan->workspace_bytes += rearranged ? rearrangedBytes(g2) : operands.bytes;
+  RowsWuProblem rows;
+  if (!rearranged && rowsWuShares(148, *p, s, opt ? opt->split_k : 0, opt ? unsigned(opt->plan_flags) : 0u, nullptr, nullptr, &rows)) {
+    plan->kernel = 3;
+    plan->in_place = 1;
+  }
   plan->flops = 2 * numberOfMacs(*p);
   const uint64_t es = dtypeBytes(p->input_type);
   plan->bytes = es * (uint64_t(p->batch) * s.H * s.W * p->groups * p->in_chans_per_group +
@@ -821,6 +839,22 @@ int plb_conv_wu(plb_context *ctx, const plb_conv_params *p, const plb_conv_optio
     const WuFold fold{uint32_t(s.KH), uint32_t(s.KW), uint32_t(co), uint32_t(ci), uint32_t(g2.s), uint32_t(g2.Cp),
                       uint32_t(g2.K2h), 0};
     return run(q, nullptr, &fold);
+  }
+  RowsWuProblem rows;
+  if (const int shares = rowsWuShares(ctx->sm_count, *p, s, force_split, plan_flags, d_acts, d_out_grads, &rows)) {
+    WuArgs a{};
+    a.sgroups = int(p->groups);
+    a.taps_h = s.KH;
+    a.taps_w = s.KW;
+    a.co_total = co;
+    a.ci_total = ci;
+    a.ksplit = shares;
+    void *ws = nullptr;
+    if (int rc = scratch(ctx, kSlotWuPartials, size_t(shares) * p->groups * w_elems * sizeof(float), &ws)) return rc;
+    a.partial = static_cast<float *>(ws);
+    if (int rc = launchRowsWu(ctx, rows, a.partial)) return rc;
+    ctx->launches++;
+    return launchWuReduce(ctx->stream, a, p->groups * w_elems, d_weight_grads, d_weight_grads_f32, nullptr);
   }
   const void *x = d_acts, *dy = d_out_grads;
   WuOperands operands;
