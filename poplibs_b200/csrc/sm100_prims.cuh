@@ -367,42 +367,37 @@ __device__ __forceinline__ void umma_ss(uint32_t tmem_d, uint64_t adesc, uint64_
 }
 
 // ---- programmatic dependent launch -------------------------------------------
-// The fp16 instruction where `on` holds, for a warp that issues together: with one thread in a
-// branch of its own, the compiler moves the operands to the uniform registers for each instruction.
-// kHint is for the A operand: consecutive instructions that read the same A tile (same
-// descriptor, same shape) can keep it in the tensor core's collector buffer instead of fetching
-// it from shared memory again: 1 = fill, 2 = use, 3 = last use, 0 = neither.
+// The fp16 instruction with a collector hint for the A operand: consecutive instructions that
+// read the same A tile (same descriptor, same shape) can keep it in the tensor core's collector
+// buffer instead of fetching it from shared memory again: 1 = fill, 2 = use, 3 = last use.
 template <int kHint>
-__device__ __forceinline__ void umma_ss_f16_if(uint32_t on, uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
-                                               uint32_t idesc, uint32_t accumulate) {
-#define PLB_UMMA_IF(collector)                                                                      \
+__device__ __forceinline__ void umma_ss_f16_collect_a(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
+                                                      uint32_t idesc, uint32_t accumulate) {
+#define PLB_UMMA_COLLECT(hint)                                                                      \
   asm volatile(                                                                                     \
       "{\n\t"                                                                                       \
-      ".reg .pred p, q;\n\t"                                                                        \
+      ".reg .pred p;\n\t"                                                                           \
       "setp.ne.b32 p, %4, 0;\n\t"                                                                   \
-      "setp.ne.b32 q, %5, 0;\n\t"                                                                   \
-      "@q tcgen05.mma.cta_group::1.kind::f16" collector " [%0], %1, %2, %3, p;\n\t"                 \
-      "}\n" ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(on) : "memory")
-  if constexpr (kHint == 0)
-    PLB_UMMA_IF("");
-  else if constexpr (kHint == 1)
-    PLB_UMMA_IF(".collector::a::fill");
+      "tcgen05.mma.cta_group::1.kind::f16.collector::a::" hint " [%0], %1, %2, %3, p;\n\t"          \
+      "}\n" ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory")
+  static_assert(kHint >= 1 && kHint <= 3, "collector hint");
+  if constexpr (kHint == 1)
+    PLB_UMMA_COLLECT("fill");
   else if constexpr (kHint == 2)
-    PLB_UMMA_IF(".collector::a::use");
+    PLB_UMMA_COLLECT("use");
   else
-    PLB_UMMA_IF(".collector::a::lastuse");
-#undef PLB_UMMA_IF
+    PLB_UMMA_COLLECT("lastuse");
+#undef PLB_UMMA_COLLECT
 }
-// The same on the accumulator lanes whose bits in `keep_lo` (lanes 0-63) and `keep_hi` are clear.
-__device__ __forceinline__ void umma_ss_f16_masked(uint32_t on, uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
+// The fp16 instruction on the accumulator lanes whose bits in `keep_lo` (lanes 0-63) and `keep_hi` are clear.
+__device__ __forceinline__ void umma_ss_f16_masked(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
                                                    uint32_t idesc, uint32_t keep_lo, uint32_t keep_hi) {
   asm volatile(
       "{\n\t"
-      ".reg .pred p, q;\n\t"
+      ".reg .pred p;\n\t"
       "setp.eq.b32 p, 0, 0;\n\t"
-      "setp.ne.b32 q, %6, 0;\n\t"
-      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%4, %4, %5, %5}, p;\n\t"
-      "}\n" ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(keep_lo), "r"(keep_hi), "r"(on) : "memory");
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%4, %4, %5, %5}, p;\n\t"
+      "}\n" ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(keep_lo), "r"(keep_hi) : "memory");
 }
 
 // A kernel launched with the programmatic-stream-serialization attribute may

@@ -16,10 +16,10 @@
 //
 // Roles: 7 warps load strips (two in flight), one thread issues the instructions, two groups
 // of 4 warps store alternate tiles.  Loads, results and operands share the SM's path to
-// shared memory and L1; a tile of 14 instructions (7x7) takes 1400 cycles of the 670 that the
+// shared memory and L1; a tile of 14 instructions (7x7) takes 1350 cycles of the 670 that the
 // instructions alone would, one of 6 (3x3) is bound by its results.  Measured against the rearranged
 // form: 3x3, 1 -> 96 on 147 images of 118 x 118 122 -> 96 us, 3x3/2, 4 -> 64 on 11 of 102 x 192 9.1 ->
-// 5.4, 7x7/2, 3 -> 64 on 256 of 224 x 224 162 -> 156 (medians of six).  (Whole lines of results, stored from 16
+// 5.4, 7x7/2, 3 -> 64 on 256 of 224 x 224 162 -> 147 (medians of six).  (Whole lines of results, stored from 16
 // x 256-bit reads of tensor memory, two issuers or four accumulators: no gain.)
 #include <algorithm>
 #include <atomic>
@@ -86,7 +86,8 @@ stemKernel(const __grid_constant__ StemArgs a) {
   __shared__ int abort_word;
   __shared__ __align__(16) float bias[256];
   const S2dShape &g = a.g;
-  const int tid = int(threadIdx.x), warp = tid >> 5, lane = tid & 31;
+  // (the warp is the same in all lanes, as the compiler sees it)
+  const int tid = int(threadIdx.x), warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   const uint32_t weights = smem_u32(stem_smem), strips = weights + a.weight_bytes;
   volatile int *abort_flag = &abort_word;
   auto stripFull = [&](int i) { return smem_u32(bars + i); };
@@ -128,7 +129,7 @@ stemKernel(const __grid_constant__ StemArgs a) {
   __syncthreads();
   tc_fence_after_sync();
   pdl_launch_dependents();  // (tensor memory is allocated: the next kernel cannot take it first)
-  const uint32_t tmem = *static_cast<volatile uint32_t *>(&tmem_slot);
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *static_cast<volatile uint32_t *>(&tmem_slot), 0);
   // strip u: image, first output row and column, and its tiles
   auto stripOf = [&](int u, int &n, int &oh0, int &ow0, int &rows, int &cols) {
     const int v = int(fast_div(uint32_t(u), a.fd_parts));
@@ -192,42 +193,45 @@ stemKernel(const __grid_constant__ StemArgs a) {
       mbar_arrive(stripFull(buf));
     }
   } else if (warp == kStemMmaWarp) {
-    // ---- instructions
-    if (elect_one()) {
-      int c = 0, k = 0;
-      for (int u = int(blockIdx.x); ok && u < a.units; u += int(gridDim.x), ++k) {
-        int n, oh0, ow0, rows, cols;
-        const int tiles = stripOf(u, n, oh0, ow0, rows, cols), buf = k & 1;
-        if (!mbar_wait(stripFull(buf), uint32_t(k >> 1 & 1), abort_flag)) {
+    // ---- instructions: all lanes walk, for each tile one issues, so that the operands come from
+    // uniform registers (with one thread in the whole role 200 sampled layers took 1.04 of their time,
+    // 7x7/2, 3 -> 64, 256 images of 224 x 224 153 us, now 147)
+    auto wait = [&](uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag)); };
+    const uint32_t b_step = uint32_t(a.co) * 2;
+    const uint64_t b_first = plainDesc(weights, uint32_t(a.co) * 16, 128);
+    const uint32_t down = uint32_t(a.pitch), plane1 = g.s == 2 ? a.plane_bytes >> 4 : down;
+    const uint32_t both = g.s == 2 ? down : 2 * down;
+    int c = 0, k = 0;
+    for (int u = int(blockIdx.x); ok && u < a.units; u += int(gridDim.x), ++k) {
+      int n, oh0, ow0, rows, cols;
+      const int tiles = stripOf(u, n, oh0, ow0, rows, cols), buf = k & 1;
+      if (!wait(stripFull(buf), uint32_t(k >> 1 & 1))) {
+        failed(kStatusMmaTimeout);
+        break;
+      }
+      tc_fence_after_sync();
+      const uint32_t strip = strips + uint32_t(buf) * a.strip_bytes;
+      for (int t = 0; t < tiles; ++t, ++c) {
+        const int acc = c & 1;
+        if (!wait(accFree(acc), uint32_t(c >> 1 & 1) ^ 1u)) {
           failed(kStatusMmaTimeout);
           break;
         }
         tc_fence_after_sync();
-        const uint32_t strip = strips + uint32_t(buf) * a.strip_bytes;
-        for (int t = 0; t < tiles; ++t, ++c) {
-          const int acc = c & 1;
-          if (!mbar_wait(accFree(acc), uint32_t(c >> 1 & 1) ^ 1u, abort_flag)) {
-            failed(kStatusMmaTimeout);
-            break;
-          }
-          tc_fence_after_sync();
-          uint64_t b = plainDesc(weights, uint32_t(a.co) * 16, 128);
-          const uint32_t d = tmem + uint32_t(acc * a.co_pad), b_step = uint32_t(a.co) * 2;
-          const uint64_t a0 = plainDesc(strip + uint32_t(t * 128) * 16, 16, 128);
+        const uint32_t d = tmem + uint32_t(acc * a.co_pad);
+        uint64_t b = b_first, ad = plainDesc(strip + uint32_t(t * 128) * 16, 16, 128);
+        if (elect_one()) {
           // (unrolled: a loop over single instructions paces them, 7x7 190 us)
-          auto filterRow = [&](uint64_t ad, bool first) {
-            umma_ss<false>(d, ad, b, a.idesc, first ? 0u : 1u);
+          auto filterRow = [&](uint64_t at, bool first) {
+            umma_ss<false>(d, at, b, a.idesc, first ? 0u : 1u);
             b += b_step;
 #pragma unroll 1
             for (int s = 2; s < a.taps; s += 2) {
-              ad += 2;
-              umma_ss<false>(d, ad, b, a.idesc, 1u);
+              at += 2;
+              umma_ss<false>(d, at, b, a.idesc, 1u);
               b += b_step;
             }
           };
-          const uint32_t down = uint32_t(a.pitch), plane1 = g.s == 2 ? a.plane_bytes >> 4 : down;
-          const uint32_t both = g.s == 2 ? down : 2 * down;
-          uint64_t ad = a0;
           if (a.taps == 4) {
             int r = 0;
             uint32_t acc_on = 0;
@@ -246,15 +250,18 @@ stemKernel(const __grid_constant__ StemArgs a) {
           }
           umma_commit(accFull(acc));
         }
-        if (ok) umma_commit(stripFree(buf));
+        __syncwarp();
       }
-      // the last commits arrive here: not before them may the block end, nor tensor memory go
-      // while instructions run (after a failure, too)
-      umma_commit(smem_u32(bars + 8));
-      if (!mbar_wait(smem_u32(bars + 8), 0, abort_flag)) failed(kStatusDrainTimeout);
-      for (int i = 0; ok && i < 2 && i < k; ++i)
-        if (!mbar_wait(stripFree((k - 1 - i) & 1), uint32_t((k - 1 - i) >> 1 & 1), abort_flag)) failed(kStatusDrainTimeout);
+      if (ok && elect_one()) umma_commit(stripFree(buf));
+      __syncwarp();
     }
+    // the last commits arrive here: not before them may the block end, nor tensor memory go
+    // while instructions run (after a failure, too)
+    if (elect_one()) umma_commit(smem_u32(bars + 8));
+    __syncwarp();
+    if (!wait(smem_u32(bars + 8), 0)) failed(kStatusDrainTimeout);
+    for (int i = 0; ok && i < 2 && i < k; ++i)
+      if (!wait(stripFree((k - 1 - i) & 1), uint32_t((k - 1 - i) >> 1 & 1))) failed(kStatusDrainTimeout);
     __syncwarp();
   } else {
     // ---- results
