@@ -529,6 +529,116 @@ chanFinishKernel(const float *__restrict__ partial_a, const float *__restrict__ 
   if (threadIdx.x == 0) finishChan<T>(fin, c, a, b);
 }
 
+// The same in one launch, where rows are whole vectors: the blocks of a cluster of up to eight have the
+// slabs, and the first reads the others' sums from their shared memory, in their order.  Bound by latency: the
+// launch, one or two batches of loads, the two meetings of the cluster.
+constexpr int kClusterThreads = 512, kClusterBlocks = 8;
+template <typename T, int kMode, int V>
+__global__ void __launch_bounds__(kClusterThreads, 1)
+chanClusterKernel(const T *__restrict__ x, const T *__restrict__ y, const T *__restrict__ centre, uint32_t rows,
+                  uint32_t chans, const ChanFinish fin) {
+  using Vec = ChanVec<T, V>;
+  using Raw = typename Vec::Raw;
+  constexpr bool kHasA = kMode != kSumCentredXX, kHasB = kMode != kSumX, kHasY = kMode == kSumXYAndY;
+  constexpr uint32_t kLanes = kColChans / V, kRowLanes = kClusterThreads / kLanes, kWarps = kClusterThreads / 32;
+  constexpr int kUnroll = kHasY ? 4 : 8;
+  __shared__ float red[2][kWarps][kColChans + 1];
+  __shared__ float sums[2][kColChans];
+  pdl_launch_dependents();
+  const uint32_t vx = threadIdx.x % kLanes, ry = threadIdx.x / kLanes, warp = threadIdx.x / 32;
+  const uint32_t c0 = blockIdx.x * kColChans + vx * V;
+  const bool mine = c0 < chans;
+  float a[V], b[V], m[V];
+#pragma unroll
+  for (int j = 0; j < V; ++j) a[j] = b[j] = m[j] = 0.f;
+  pdl_wait();  // inputs may come from the previous kernel in the stream
+  if (mine) {
+    if constexpr (kMode == kSumCentredXX)
+#pragma unroll
+      for (int j = 0; j < V; ++j) m[j] = toFloat(centre[c0 + j]);
+    const uint32_t step = gridDim.y * kRowLanes;
+    for (uint32_t r = blockIdx.y * kRowLanes + ry; r < rows; r += kUnroll * step) {
+      Raw rx[kUnroll];
+      [[maybe_unused]] Raw rv[kUnroll];
+#pragma unroll
+      for (int u = 0; u < kUnroll; ++u)
+        if (r + u * step < rows) {
+          rx[u] = *reinterpret_cast<const Raw *>(x + size_t(r + u * step) * chans + c0);
+          if constexpr (kHasY) rv[u] = *reinterpret_cast<const Raw *>(y + size_t(r + u * step) * chans + c0);
+        }
+#pragma unroll
+      for (int u = 0; u < kUnroll; ++u)
+        if (r + u * step < rows) {
+          float xv[V], yv[V];
+          Vec::unpack(rx[u], xv);
+          if constexpr (kHasY) Vec::unpack(rv[u], yv);
+#pragma unroll
+          for (int j = 0; j < V; ++j) addElement<T, kMode>(a[j], b[j], xv[j], kHasY ? yv[j] : 0.f, m[j]);
+        }
+    }
+  }
+  uint32_t first = 0, held = V;  // the columns of the vector this thread ends up with
+  bool writes = true;
+  foldWarp<V, kHasA, kHasB, 16>(a, b, kLanes, first, held, writes);
+  if (writes)
+#pragma unroll
+    for (int j = 0; j < V; ++j)
+      if (j < held) {
+        if constexpr (kHasA) red[0][warp][vx * V + first + j] = a[j];
+        if constexpr (kHasB) red[1][warp][vx * V + first + j] = b[j];
+      }
+  __syncthreads();
+  const uint32_t which = threadIdx.x / kColChans, col = threadIdx.x % kColChans, c = blockIdx.x * kColChans + col;
+  if (which < 2 && (which == 0 ? kHasA : kHasB)) {
+    float total = red[which][0][col];
+#pragma unroll
+    for (uint32_t k = 1; k < kWarps; ++k) total += red[which][k][col];
+    sums[which][col] = total;
+  }
+  if (gridDim.y > 1)
+    cluster_sync_all();
+  else
+    __syncthreads();
+  if (blockIdx.y == 0 && which == 0 && c < chans) {
+    float ta = 0.f, tb = 0.f;
+    for (uint32_t k = 0; k < gridDim.y; ++k) {
+      auto read = [&](const float *p) {
+        float v;
+        asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(map_to_cta(smem_u32(p), k)) : "memory");
+        return v;
+      };
+      if constexpr (kHasA) ta += read(&sums[0][col]);
+      if constexpr (kHasB) tb += read(&sums[1][col]);
+    }
+    finishChan<T>(fin, c, ta, tb);
+  }
+  if (gridDim.y > 1) cluster_sync_all();  // (no block leaves before its sums have been read)
+}
+template <typename T, int kMode, int V>
+int launchChanCluster(plb_context *ctx, uint64_t rows, uint32_t chans, const T *x, const T *y, const T *centre, const ChanFinish &fin) {
+  constexpr uint32_t kRowLanes = kClusterThreads / (kColChans / V);
+  // four rows a thread and more, as long as there are blocks for them
+  uint32_t blocks = 1;
+  while (blocks < kClusterBlocks && uint64_t(blocks) * kRowLanes * 4 < rows) blocks *= 2;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 1;
+  attr[0].val.clusterDim.y = blocks;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((chans + kColChans - 1) / kColChans, blocks);
+  cfg.blockDim = dim3(kClusterThreads);
+  cfg.stream = ctx->stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = (ctx->plan_flags & PLB_PLAN_NO_PDL) ? 1 : 2;
+  PLB_CUDA(cudaLaunchKernelEx(&cfg, chanClusterKernel<T, kMode, V>, x, y, centre, uint32_t(rows), chans, fin));
+  PLB_CUDA(cudaGetLastError());
+  ctx->launches++;
+  return PLB_OK;
+}
+
 template <typename T, int kMode>
 int launchChanColumns(plb_context *ctx, uint64_t rows, uint32_t chans, const T *x, const T *y, const T *centre,
                       const ChanFinish &fin) {
@@ -590,11 +700,17 @@ int chanSums(plb_context *ctx, const T *x, const T *y, const T *centre, uint64_t
   const uint64_t bytes = rows * chans * sizeof(T);
   const uint64_t most_slabs =
       std::max<uint64_t>({uint64_t(ctx->sm_count) / 4, uint64_t(ctx->sm_count) * 128 / std::max(chans, 1u), bytes / (256 * 1024)});
-  // Few rows: two short launches over narrow columns, where a block's wide row of sums
-  // would be most of the work and the last block's finish most of the time (324 x 253
-  // halves 7.8 -> 3.6 us, 1058 x 351 floats 7.7 -> 4.2, 8281 x 64 halves 5.7 -> 5.5; 16641
-  // x 64 5.7 against 6.9).  Rows that are no whole vectors have several times their
-  // width to finish and take them for longer (16641 x 255 halves 10.8 -> 7.5).
+  // Few rows: one launch of clusters over narrow columns (halves, with the two launches below before:
+  // 64 x 64 3.2 -> 2.2 us, 784 x 1024 5.3 -> 3.4, 4096 x 64 4.5 -> 3.4, 4096 x 256 7.0 -> 3.6, 8192 x 512 7.9 -> 4.6;
+  // floats alike).  Eight blocks have all the rows of a column: up to 64 columns slabs over the whole
+  // device are quicker from 8192 rows on (two sums 5.0 against 5.3), with up to 512, where those leave wide
+  // rows of sums, from 16384 (floats 10.0 against 11.1), above that from 6272 (floats 7.8 against 8.6).
+  if (vec && chans % kVec == 0 && rows <= (chans <= 64 ? 6144u : chans <= 512 ? 12544u : 4096u))
+    return launchChanCluster<T, kMode, kVec>(ctx, rows, chans, x, y, centre, fin);
+  // Rows that are no whole vectors, and those up to 8192: two short launches over narrow columns,
+  // where a block's wide row of sums would be most of the work and the last block's finish most of
+  // the time (324 x 253 halves 7.8 -> 3.6 us, 1058 x 351 floats 7.7 -> 4.2, 8281 x 64 halves 5.7 -> 5.5; 16641
+  // x 64 5.7 against 6.9; 16641 x 255 halves 10.8 -> 7.5).
   if (rows <= (vec && chans % kVec == 0 ? 8192u : 24576u) && bytes <= (uint64_t(16) << 20))
     return launchChanColumns<T, kMode>(ctx, rows, chans, x, y, centre, fin);
   if (!vec) return launchChanSums<T, kMode, 1, 512>(ctx, rows, chans, most_slabs, x, y, centre, fin);
