@@ -703,9 +703,10 @@ int chanSums(plb_context *ctx, const T *x, const T *y, const T *centre, uint64_t
   // Few rows: one launch of clusters over narrow columns (halves, with the two launches below before:
   // 64 x 64 3.2 -> 2.2 us, 784 x 1024 5.3 -> 3.4, 4096 x 64 4.5 -> 3.4, 4096 x 256 7.0 -> 3.6, 8192 x 512 7.9 -> 4.6;
   // floats alike).  Eight blocks have all the rows of a column: up to 64 columns slabs over the whole
-  // device are quicker from 8192 rows on (two sums 5.0 against 5.3), with up to 512, where those leave wide
-  // rows of sums, from 16384 (floats 10.0 against 11.1), above that from 6272 (floats 7.8 against 8.6).
-  if (vec && chans % kVec == 0 && rows <= (chans <= 64 ? 6144u : chans <= 512 ? 12544u : 4096u))
+  // device are quicker from 8192 rows on (two sums 5.0 against 5.3), up to 128 from 12544 (6.1 against 7.1), with
+  // up to 512, where those leave wide rows of sums, from 16384 (floats 10.0 against 11.1), above that from
+  // 6272 (floats 7.8 against 8.6).
+  if (vec && chans % kVec == 0 && rows <= (chans <= 64 ? 6144u : chans <= 128 ? 8192u : chans <= 512 ? 12544u : 4096u))
     return launchChanCluster<T, kMode, kVec>(ctx, rows, chans, x, y, centre, fin);
   // Rows that are no whole vectors, and those up to 8192: two short launches over narrow columns,
   // where a block's wide row of sums would be most of the work and the last block's finish most of

@@ -29,7 +29,7 @@ def test_sums(gpu_ctx, rows, chans, dtype):
     torch.cuda.synchronize()
     before = gpu_ctx.launch_count()
     gpu_ctx.conv_bias_update(plb, dx, rows, chans, capi.FLOAT, db, -0.5)
-    small = rows <= (6144 if chans <= 64 else 12544 if chans <= 512 else 4096) and chans % (8 if dtype == "half" else 4) == 0
+    small = rows <= (6144 if chans <= 64 else 8192 if chans <= 128 else 12544 if chans <= 512 else 4096) and chans % (8 if dtype == "half" else 4) == 0
     assert not small or gpu_ctx.launch_count() == before + 1
     gpu_ctx.norm_param_gradients(plb, dx, dy, rows, chans, 1.0, None, None, gamma, beta)
     gpu_ctx.norm_statistics(plb, dx, rows, chans, 1e-3, 1.0, mean, inv_std)
