@@ -17,7 +17,7 @@
 // about 30 MB on by the rate at which those blocks keep loads in flight (2.7 TB/s read and
 // written).  Shared memory's rows are whole eights of pixels, so that the swizzle of a lane's addresses
 // is the same in every row: with addresses formed per tap, a 16-pixel step took 160 instructions and
-// 32 groups of 8 on 32 images of 28 x 28 20.5 us, now 10.7 (17.8 in three launches on dense blocks).
+// 32 groups of 8 on 32 images of 28 x 28 20.5 us, now 10.0 (17.8 in three launches on dense blocks).
 #include <algorithm>
 #include <atomic>
 #include <cmath>
@@ -296,13 +296,15 @@ struct RowsTiling {
 
 int ceilDiv(long a, long b) { return int((a + b - 1) / b); }
 
-// The tile of the least estimated time: rounds of blocks, each its loads, its instructions
-// and its stores, shared by the blocks of an SM.
+// The tile of the least estimated time: rounds of blocks (those of the last begin as others end),
+// each its loads and stores, and the instructions of all the SM's warps or the latency of one
+// warp's walk.  Fitted to 1900 tiles of 110 layers, whose times it is 16 % off; the tile that it takes is 1.2 %
+// slower than a layer's best in the mean (with products alone for instructions, and whole rounds, 6 %).
 bool rowsTiling(int sms, const IgemmProblem &p, RowsTiling *best) {
   const int K = p.taps_w, c = p.k_per_tap;
   const long slabs = ceilDiv(long(p.groups) * c, 64);
-  // cycles of a 16-pixel step of a row: its instructions at the rate of the SM's four pipes
-  const double step = c == 8 ? K * (8.3 * (K / 2) + 4.2) : 2 * K * K * 8.3;
+  // cycles of a 16-pixel step of a row: its products at the rate of the SM's four pipes
+  const double products = c == 8 ? K * (8.3 * (K / 2) + 4.2) : 2 * K * K * 8.3;
   bool found = false;
   for (int steps = 1; steps <= 7; ++steps)
     for (int images = 1; images <= 2; ++images) {
@@ -319,13 +321,16 @@ bool rowsTiling(int sms, const IgemmProblem &p, RowsTiling *best) {
         if (t.smem > 110 * 1024) break;
         const int most = c == 8 || K == 5 ? 2 : 3, resident = std::max(1, std::min<int>(most, int(226 * 1024 / (t.smem + 1024))));
         t.blocks = slabs * ceilDiv(p.out_w, t.tile_w) * ceilDiv(p.out_h, rows) * ceilDiv(p.out_n, images);
-        const double rounds = std::ceil(double(t.blocks) / (sms * resident));
+        const double share = double(t.blocks) / (sms * resident), rounds = std::max(1.0, 0.425 * std::ceil(share) + 0.575 * share);
         const double here = std::min<double>(resident, std::ceil(double(t.blocks) / sms));
-        const double load = double(images) * (rows + K - 1) * (t.tile_w + K - 1) * kRowBytes / 30, store = double(rows) * t.tile_w * images * kRowBytes / 30;
-        const double walk = (rows + K - 1) * steps * step;
-        const double warps = 64 / c;
-        const double busy = std::max(walk * warps * here / 4, walk * 1.6 + (rows + K - 1) * 60.0);
-        t.us = float(2.3 + rounds * (1500 + here * (load + store) + busy) / 1900);
+        const double load = double(images) * (rows + K - 1) * (t.tile_w + K - 1) * kRowBytes;
+        const double store = double(images) * rows * std::min(t.tile_w, p.out_w) * kRowBytes;
+        // (an even number of steps of 3x3 filters is walked by twos)
+        const bool twos = steps % 2 == 0 && K == 3;
+        const double walked = (rows + K - 1.0) * steps;
+        const double all = walked * (0.747 * products + (twos ? 4.0 : 14.2)) * (64 / c) * here / 4;
+        const double one = walked * (1.34 * products + (twos ? 84 : 168));
+        t.us = float(1.49 + rounds * (1781 + here * (0.0413 * load + 0.0192 * store) + std::max(all, one)) / 1900);
         t.steps = steps;
         if (!found || t.us < best->us) *best = t;
         found = true;
@@ -337,7 +342,7 @@ bool rowsTiling(int sms, const IgemmProblem &p, RowsTiling *best) {
 }  // namespace
 
 // Of 300 sampled layers of 0.1 to 134 MB (2 to 32 groups, 3x3 and 5x5), those within the limits below
-// take 0.69 of their time on the other routes, nine passes of 600 more than 4 % longer, at most 10 %.
+// take 0.66 of their time on the other routes, a few passes of 600 more than 4 % longer, at most 10 %.
 // Beyond them the persistent blocks of the tensor-core route stream better (3x3, 8 groups of 16, 34 images of
 // 110 x 110, 105 MB, forward: 62 there, 81 here; 30.8 MB 26 and 28), 5x5 of 16 channels is bound by mma.sync
 // (10 MB: 21 and 25), and two groups of 8 leave six of a block's warps idle (12 MB: 27 and 34).
@@ -356,7 +361,7 @@ bool rowsSuits(int sm_count, const IgemmProblem &p, int type) {
   if (at % 16 != 0 || (reinterpret_cast<uintptr_t>(p.wgt) | p.wgt_strides[0] | p.wgt_strides[1]) % 4 != 0) return false;
   if (p.out_w > 1 << 20 || p.out_h > 1 << 20 || std::abs(p.pad_h) > 1 << 20 || std::abs(p.pad_w) > 1 << 20) return false;
   const double megabytes = 2e-6 * p.groups * c * p.out_w * p.out_h * p.out_n;
-  const double most = c == 16 ? (p.taps_w == 5 ? 5 : p.b_mn ? 60 : 28) : p.groups < 4 ? (p.taps_w == 5 ? 0.8 : 5) : p.taps_w == 5 || p.b_mn ? 1e9 : 100;
+  const double most = c == 16 ? (p.taps_w == 5 ? 5 : p.b_mn ? 60 : 28) : p.groups < 4 ? (p.taps_w == 5 ? 0.5 : 5) : p.taps_w == 5 || p.b_mn ? 1e9 : 100;
   RowsTiling t;
   return megabytes <= most && rowsTiling(sm_count, p, &t) && t.blocks <= 0x3fffffff;
 }
