@@ -529,6 +529,16 @@ chanFinishKernel(const float *__restrict__ partial_a, const float *__restrict__ 
   if (threadIdx.x == 0) finishChan<T>(fin, c, a, b);
 }
 
+// A power of two of values, neighbours first: the large sums are few.
+template <int N>
+__device__ __forceinline__ float pairwise(float (&v)[N]) {
+#pragma unroll
+  for (int d = 1; d < N; d *= 2)
+#pragma unroll
+    for (int k = 0; k + d < N; k += 2 * d) v[k] += v[k + d];
+  return v[0];
+}
+
 // The same in one launch, where rows are whole vectors: the blocks of a cluster of up to eight have the
 // slabs, and the first reads the others' sums from their shared memory, in their order.  Bound by latency: the
 // launch, one or two batches of loads, the two meetings of the cluster.
@@ -590,27 +600,28 @@ chanClusterKernel(const T *__restrict__ x, const T *__restrict__ y, const T *__r
   __syncthreads();
   const uint32_t which = threadIdx.x / kColChans, col = threadIdx.x % kColChans, c = blockIdx.x * kColChans + col;
   if (which < 2 && (which == 0 ? kHasA : kHasB)) {
-    float total = red[which][0][col];
+    float part[kWarps];
 #pragma unroll
-    for (uint32_t k = 1; k < kWarps; ++k) total += red[which][k][col];
-    sums[which][col] = total;
+    for (uint32_t k = 0; k < kWarps; ++k) part[k] = red[which][k][col];
+    sums[which][col] = pairwise(part);
   }
   if (gridDim.y > 1)
     cluster_sync_all();
   else
     __syncthreads();
   if (blockIdx.y == 0 && which == 0 && c < chans) {
-    float ta = 0.f, tb = 0.f;
-    for (uint32_t k = 0; k < gridDim.y; ++k) {
+    float ta[kClusterBlocks], tb[kClusterBlocks];
+#pragma unroll
+    for (uint32_t k = 0; k < kClusterBlocks; ++k) {
       auto read = [&](const float *p) {
         float v;
         asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(map_to_cta(smem_u32(p), k)) : "memory");
         return v;
       };
-      if constexpr (kHasA) ta += read(&sums[0][col]);
-      if constexpr (kHasB) tb += read(&sums[1][col]);
+      ta[k] = kHasA && k < gridDim.y ? read(&sums[0][col]) : 0.f;
+      tb[k] = kHasB && k < gridDim.y ? read(&sums[1][col]) : 0.f;
     }
-    finishChan<T>(fin, c, ta, tb);
+    finishChan<T>(fin, c, pairwise(ta), pairwise(tb));
   }
   if (gridDim.y > 1) cluster_sync_all();  // (no block leaves before its sums have been read)
 }
