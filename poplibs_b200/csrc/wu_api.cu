@@ -271,7 +271,10 @@ void planWu(const WuProblem &p, int sm_count, int force_split, unsigned plan_fla
     };
     const double before = best * cost(s.KH, 64, a->strip_rows);
     const int columns = a->sgroups * a->ci_blocks * s.KW;
-    const double splits = force_split > 0 ? force_split : std::max(1, (sm_count > 0 ? sm_count : 148) / columns);
+    // (a constraint to as many CTAs as there are tiles may be the saved plan of a call that had SMs for more:
+    // it is weighed as that call was, and leads to the same kernel)
+    const int room = std::max(1, (sm_count > 0 ? sm_count : 148) / columns);
+    const double splits = force_split <= 0 ? room : force_split < best ? force_split : std::max(force_split, room);
     double least = std::min(0.94 * before, before - 2000 * splits);
     for (int h = 4; h >= 1; h >>= 1)
       for (int w = 64 / h; w >= 1; w >>= 1) {

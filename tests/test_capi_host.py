@@ -249,6 +249,18 @@ def test_weight_update_plans_describe_what_runs():
     assert capi.conv_wu_plan(mk(4, [9, 9], [3, 3], 0, 64, padding=1)).tiles == 0
 
 
+@pytest.mark.parametrize("n,field,kernel,ci,co,groups", [
+    (39, [27, 7], [3, 1], 160, 64, 1), (30, [11, 7], [5, 2], 96, 60, 1), (7, [17, 37], [5, 1], 96, 64, 1),
+    (1, [29, 57], [7, 1], 8, 32, 2), (2, [25, 88], [7, 1], 16, 32, 2), (256, [56, 56], [3, 3], 64, 64, 1)])
+def test_saved_plans_of_weight_updates_reproduce_them(n, field, kernel, ci, co, groups):
+    """A plan's split and strips given as constraints lead to the same tiling, where the tiles are
+    fewer than the CTAs that there is room for, too."""
+    p = capi.ConvParams.make(n, field, kernel, ci, co, groups=groups, padding=[k // 2 for k in kernel])
+    free = capi.conv_wu_plan(p)
+    fixed = capi.conv_wu_plan(p, capi.ConvOptions.make(split_k=free.split_k, plan_flags=0 if free.halo_rows else capi.PLAN_NO_HALO))
+    assert bytes(free) == bytes(fixed)
+
+
 def test_plans_describe_the_operands_that_are_read():
     """Copies, pieces of floats and block-diagonal weights count as workspace; rows that are read
     where they lie are planned with their own pitch."""
