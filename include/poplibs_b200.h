@@ -522,7 +522,8 @@ PLB_API int plb_timer_stop(plb_context *ctx, float *milliseconds);
 /* ------------------------------------------------------------------------ */
 typedef struct plb_plan {
   int32_t kernel;      /* 0 = implicit GEMM (fwd/bwd/matmul), 1 = weight update, 2 = few input
-                          channels, 3 = a small product or layer (see in_place) */
+                          channels, 3 = a small product or layer (see in_place),
+                          or the weight update of narrow channel groups */
   int32_t tile_m;      /* output pixels (rows) per CTA tile                  */
   int32_t tile_n;      /* output channels (columns) per CTA tile             */
   int32_t tile_k_bytes;/* bytes of K per pipeline stage                      */
@@ -541,7 +542,8 @@ typedef struct plb_plan {
                           rearranged input); the tiling and workspace here are then what the call
                           has under plan flags and constraints, or with a result that is not
                           32-byte aligned (3-D, flipped and dilated inputs are rearranged first).
-                          A weight gradient's sums of shares of the pixels still take workspace */
+                          Weight updates are never in_place: their partial sums are workspace,
+                          with kernel 3 (narrow channel groups, split_k shares of the pixels), too */
   uint64_t flops;      /* 2 * MACs (padding excluded)                        */
   uint64_t bytes;      /* operands read once + output written once           */
   uint64_t workspace_bytes;

@@ -55,11 +55,12 @@ std::string cacheKey(const ConvParams &p, const poplar::OptionFlags &options, in
 std::string planConstraintsOf(const plb_plan &plan) {
   std::ostringstream os;
   const bool igemm = plan.kernel != 1;
+  // (a split or any of the knobs would send such a layer to another kernel)
+  const bool others = plan.in_place || plan.kernel == 3;
   os << "{\n"
      << "  \"0\": {\"partition\": {\"inChanSplit\": {\"serial\": 1, \"parallel\": "
-     << std::max(1, plan.in_place ? 1 : int(plan.split_k)) << "}}}";
-  // (any of these knobs would send such a layer to another kernel)
-  if (plan.in_place) {
+     << (others ? 1 : std::max(1, int(plan.split_k))) << "}}}";
+  if (others) {
     os << "\n}\n";
     return os.str();
   }

@@ -21,8 +21,18 @@ struct RowsWuProblem {
   int width, height;           // output pixels
   int pad_w, pad_h;
 };
-// The shares of the pixels whose sums lie apart, [share][group][tap][out][in]; 0 where it does not suit.
-int rowsWuSplits(int sm_count, const RowsWuProblem &p);
-int launchRowsWu(plb_context *ctx, const RowsWuProblem &p, float *partial);
+// Tiles of output pixels, and the shares of them whose sums lie apart, [share][group][tap][out][in].
+struct RowsWuTiling {
+  int tile_w, tile_h, tile_n, pitch;
+  size_t x_bytes, smem;
+  long tiles;
+  int splits;
+  float us;
+};
+// Whether it suits, and how.
+bool rowsWuSuits(int sm_count, const RowsWuProblem &p, RowsWuTiling *t);
+int launchRowsWu(plb_context *ctx, const RowsWuProblem &p, const RowsWuTiling &t, float *partial);
+// Blocks of a share, 64 channels each.
+inline int rowsWuSlabs(const RowsWuProblem &p) { return (p.groups * p.chans + 63) / 64; }
 
 }  // namespace plb

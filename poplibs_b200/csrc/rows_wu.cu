@@ -202,19 +202,11 @@ rowsWuKernel(const __grid_constant__ RowsWuArgs g) {
         }
 }
 
-struct RowsWuTiling {
-  int tile_w, tile_h, tile_n, pitch;
-  size_t x_bytes, smem;
-  long tiles;
-  int splits;
-  float us;
-};
-
 int ceilDiv(long a, long b) { return int((a + b - 1) / b); }
 
 bool rowsWuTiling(int sms, const RowsWuProblem &p, RowsWuTiling *best) {
   const int K = p.kernel, c = p.chans;
-  const long slabs = ceilDiv(long(p.groups) * c, 64);
+  const long slabs = rowsWuSlabs(p);
   // cycles of a 16-pixel step of a row
   const double step = (c == 8 ? K * (K / 2 + 1) : 2 * K * K) * 8.3;
   bool found = false;
@@ -254,23 +246,19 @@ bool rowsWuTiling(int sms, const RowsWuProblem &p, RowsWuTiling *best) {
 // Of 300 sampled layers (see rows.cu) 0.78 of the tensor-core route's time in all.  With 16 channels
 // the dense block wastes half as much, and rows that fill their sixteens of pixels badly, or large
 // layers, are quicker there (4 groups, 45 images of 20 x 20 10.6 us there, 13.4 here; 8 groups, 87 of 42 x 42 38.5 and 43).
-int rowsWuSplits(int sm_count, const RowsWuProblem &p) {
-  if ((p.chans != 8 && p.chans != 16) || p.groups < 2 || (p.kernel != 3 && !(p.kernel == 5 && p.chans == 8))) return 0;
-  if (p.width < 1 || p.height < 1 || p.images < 1) return 0;
-  if ((reinterpret_cast<uintptr_t>(p.x) | reinterpret_cast<uintptr_t>(p.dy)) % 16 != 0) return 0;
-  if (p.width > 1 << 20 || p.height > 1 << 20 || std::abs(p.pad_h) > 1 << 20 || std::abs(p.pad_w) > 1 << 20) return 0;
+bool rowsWuSuits(int sm_count, const RowsWuProblem &p, RowsWuTiling *t) {
+  if ((p.chans != 8 && p.chans != 16) || p.groups < 2 || (p.kernel != 3 && !(p.kernel == 5 && p.chans == 8))) return false;
+  if (p.width < 1 || p.height < 1 || p.images < 1) return false;
+  if ((reinterpret_cast<uintptr_t>(p.x) | reinterpret_cast<uintptr_t>(p.dy)) % 16 != 0) return false;
+  if (p.width > 1 << 20 || p.height > 1 << 20 || std::abs(p.pad_h) > 1 << 20 || std::abs(p.pad_w) > 1 << 20) return false;
   if (p.chans == 16) {
     const int stepped = p.width <= 8 ? 8 : (p.width + 15) / 16 * 16;
-    if (4 * p.width < 3 * stepped || 2e-6 * p.groups * 16 * p.width * p.height * p.images > 8) return 0;
+    if (4 * p.width < 3 * stepped || 2e-6 * p.groups * 16 * p.width * p.height * p.images > 8) return false;
   }
-  RowsWuTiling t;
-  if (!rowsWuTiling(sm_count, p, &t) || t.tiles > 0x3fffffff) return 0;
-  return t.splits;
+  return rowsWuTiling(sm_count, p, t) && t->tiles <= 0x3fffffff;
 }
 
-int launchRowsWu(plb_context *ctx, const RowsWuProblem &p, float *partial) {
-  RowsWuTiling t;
-  if (!rowsWuTiling(ctx->sm_count, p, &t)) return fail(PLB_ERR_UNSUPPORTED, "no tiling of the row kernel");
+int launchRowsWu(plb_context *ctx, const RowsWuProblem &p, const RowsWuTiling &t, float *partial) {
   RowsWuArgs g{};
   g.x = static_cast<const uint8_t *>(p.x);
   g.dy = static_cast<const uint8_t *>(p.dy);
@@ -295,7 +283,7 @@ int launchRowsWu(plb_context *ctx, const RowsWuProblem &p, float *partial) {
   g.tiles_w = ceilDiv(p.width, t.tile_w);
   g.tiles_h = ceilDiv(p.height, t.tile_h);
   g.tiles = int(t.tiles);
-  g.slabs = ceilDiv(g.chans, 64);
+  g.slabs = rowsWuSlabs(p);
   g.splits = t.splits;
   g.pitch = t.pitch;
   g.image_rows = t.tile_h + p.kernel - 1;

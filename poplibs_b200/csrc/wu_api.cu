@@ -79,16 +79,15 @@ struct WuProblem {
   uint64_t x_chans = 0, dy_chans = 0, x_strides[3] = {}, dy_strides[3] = {};
 };
 
-// Narrow channel groups on the kernel that keeps a group's sums in a warp's registers: the shares of
-// the pixels whose sums it leaves apart, 0 where it does not apply.
-int rowsWuShares(int sm_count, const plb_conv_params &p, const WuShape &s, int force_split, unsigned plan_flags,
-                 const void *x, const void *dy, RowsWuProblem *q) {
-  if (p.input_type != PLB_HALF || force_split != 0 || plan_flags != 0 || p.in_chans_per_group != p.out_chans_per_group) return 0;
-  if (s.KH != s.KW || s.strH != 1 || s.strW != 1 || s.dilH != 1 || s.dilW != 1 || s.opH || s.opW || s.OHc != s.OH || s.OWc != s.OW) return 0;
+// Whether narrow channel groups run on the kernel that keeps a group's sums in a warp's registers.
+bool narrowGroups(int sm_count, const plb_conv_params &p, const WuShape &s, int force_split, unsigned plan_flags,
+                  const void *x, const void *dy, RowsWuProblem *q, RowsWuTiling *t) {
+  if (p.input_type != PLB_HALF || force_split != 0 || plan_flags != 0 || p.in_chans_per_group != p.out_chans_per_group) return false;
+  if (s.KH != s.KW || s.strH != 1 || s.strW != 1 || s.dilH != 1 || s.dilW != 1 || s.opH || s.opW || s.OHc != s.OH || s.OWc != s.OW) return false;
   const int c = int(p.in_chans_per_group);
   *q = RowsWuProblem{static_cast<const uint8_t *>(x) + (size_t(s.tH) * s.W + s.tW) * p.groups * c * 2, dy, int(p.groups), c, s.KH,
                      int(p.batch), s.We, s.He, s.W, s.H, s.OW, s.OH, s.padW, s.padH};
-  return rowsWuSplits(sm_count, *q);
+  return rowsWuSuits(sm_count, *q, t);
 }
 
 // How the channels of a pixel lie in the operands the kernel reads, and how many
@@ -657,9 +656,24 @@ int plb_conv_wu_plan(const plb_conv_params *p_in, const plb_conv_options *opt, p
   planWu(w, 148, opt ? opt->split_k : 0, opt ? opt->plan_flags : 0, &a, plan);
   plan->workspace_bytes += rearranged ? rearrangedBytes(g2) : operands.bytes;
   RowsWuProblem rows;
-  if (!rearranged && rowsWuShares(148, *p, s, opt ? opt->split_k : 0, opt ? unsigned(opt->plan_flags) : 0u, nullptr, nullptr, &rows)) {
+  RowsWuTiling t;
+  if (!rearranged && narrowGroups(148, *p, s, opt ? opt->split_k : 0, opt ? unsigned(opt->plan_flags) : 0u, nullptr, nullptr, &rows, &t)) {
+    // 64 output channels a block, and with each those of its own group at every tap
+    *plan = plb_plan{};
     plan->kernel = 3;
-    plan->in_place = 1;
+    plan->tile_m = 64;
+    plan->tile_n = s.KH * s.KW * rows.chans;
+    plan->tile_k_bytes = t.tile_w * t.tile_h * t.tile_n * 2;
+    plan->box_w = t.tile_w;
+    plan->box_h = t.tile_h;
+    plan->box_n = t.tile_n;
+    plan->stages = 1;
+    plan->split_k = t.splits;
+    plan->tiles = rowsWuSlabs(rows);
+    plan->grid = plan->tiles * t.splits;
+    plan->b_mn_major = 1;
+    plan->halo_rows = s.KH - 1;
+    plan->workspace_bytes = size_t(t.splits) * p->groups * s.KH * s.KW * rows.chans * rows.chans * sizeof(float);
   }
   plan->flops = 2 * numberOfMacs(*p);
   const uint64_t es = dtypeBytes(p->input_type);
@@ -844,18 +858,19 @@ int plb_conv_wu(plb_context *ctx, const plb_conv_params *p, const plb_conv_optio
     return run(q, nullptr, &fold);
   }
   RowsWuProblem rows;
-  if (const int shares = rowsWuShares(ctx->sm_count, *p, s, force_split, plan_flags, d_acts, d_out_grads, &rows)) {
+  RowsWuTiling tiling;
+  if (narrowGroups(ctx->sm_count, *p, s, force_split, plan_flags, d_acts, d_out_grads, &rows, &tiling)) {
     WuArgs a{};
     a.sgroups = int(p->groups);
     a.taps_h = s.KH;
     a.taps_w = s.KW;
     a.co_total = co;
     a.ci_total = ci;
-    a.ksplit = shares;
+    a.ksplit = tiling.splits;
     void *ws = nullptr;
-    if (int rc = scratch(ctx, kSlotWuPartials, size_t(shares) * p->groups * w_elems * sizeof(float), &ws)) return rc;
+    if (int rc = scratch(ctx, kSlotWuPartials, size_t(tiling.splits) * p->groups * w_elems * sizeof(float), &ws)) return rc;
     a.partial = static_cast<float *>(ws);
-    if (int rc = launchRowsWu(ctx, rows, a.partial)) return rc;
+    if (int rc = launchRowsWu(ctx, rows, tiling, a.partial)) return rc;
     ctx->launches++;
     return launchWuReduce(ctx->stream, a, p->groups * w_elems, d_weight_grads, d_weight_grads_f32, nullptr);
   }

@@ -358,15 +358,19 @@ static void testGraphConstructionWithoutDevice() {
       const auto costs = internal::reportDetailedPlanEstimatedCosts(graph, q, {{"pass", "TRAINING_FWD"}});
       CHECK(costs.rearrangement.cycles == 0 && costs.total.memory == 0);
     }
-    std::ostringstream wu1, wu2;
-    reportWeightUpdatePlanInfo(wu1, graph, p, {{"planConstraintsOutputFilename", base}});
-    std::ifstream in(base + "_WU.json");
-    CHECK(bool(in));
-    std::stringstream text;
-    text << in.rdbuf();
-    reportWeightUpdatePlanInfo(wu2, graph, p, {{"planConstraints", text.str()}});
-    CHECK(wu1.str() == wu2.str());
-    std::remove((base + "_WU.json").c_str());
+    // (the second: narrow groups, whose partial sums take workspace)
+    for (const ConvParams &q : {p, ConvParams(HALF, HALF, 2, {9, 13}, {3, 3}, 8, 8, 16)}) {
+      std::ostringstream wu1, wu2;
+      reportWeightUpdatePlanInfo(wu1, graph, q, {{"planConstraintsOutputFilename", base}});
+      std::ifstream in(base + "_WU.json");
+      CHECK(bool(in));
+      std::stringstream text;
+      text << in.rdbuf();
+      reportWeightUpdatePlanInfo(wu2, graph, q, {{"planConstraints", text.str()}});
+      CHECK(wu1.str() == wu2.str());
+      CHECK(wu1.str().find("workspace bytes            0") == std::string::npos);
+      std::remove((base + "_WU.json").c_str());
+    }
   }
   // weights of a fully connected layer rearranged for its backward pass
   {

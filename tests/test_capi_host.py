@@ -261,6 +261,21 @@ def test_saved_plans_of_weight_updates_reproduce_them(n, field, kernel, ci, co, 
     assert bytes(free) == bytes(fixed)
 
 
+@pytest.mark.parametrize("groups,chans,n,field,k", [(2, 8, 256, [56, 56], 3), (32, 8, 32, [28, 28], 3), (8, 8, 64, [40, 40], 5), (4, 16, 4, [9, 8], 3)])
+def test_weight_update_plans_of_narrow_groups_describe_what_runs(groups, chans, n, field, k):
+    """The shares of the pixels, whose partial sums are workspace; not the tensor-core route's, which
+    constraints lead to."""
+    p = capi.ConvParams.make(n, field, [k, k], chans, chans, groups=groups, padding=k // 2)
+    plan = capi.conv_wu_plan(p)
+    assert (plan.kernel, plan.in_place, plan.halo_rows) == (3, 0, k - 1)
+    assert plan.workspace_bytes == plan.split_k * groups * k * k * chans * chans * 4
+    assert plan.tiles == (groups * chans + 63) // 64 and plan.grid == plan.tiles * plan.split_k
+    tiles = -(-field[1] // plan.box_w) * -(-field[0] // plan.box_h) * -(-n // plan.box_n)
+    assert 1 <= plan.split_k <= tiles and plan.grid <= 148 * 3
+    general = capi.conv_wu_plan(p, capi.ConvOptions.make(split_k=2))
+    assert (general.kernel, general.split_k) == (1, 2) and general.flops == plan.flops
+
+
 def test_plans_describe_the_operands_that_are_read():
     """Copies, pieces of floats and block-diagonal weights count as workspace; rows that are read
     where they lie are planned with their own pitch."""
