@@ -715,28 +715,29 @@ int convBwdStrided(plb_context *ctx, const plb_conv_params &p, const plb_conv_op
 // Whether a pass runs on the patch kernel (patch.cu), and its problem(s); `o` are the
 // caller's operands, `groups` those that the general route contracts together.
 bool fwdOnPatches(int sm_count, const plb_conv_params &p, const plb_conv_options *opt, int plan_flags, const ConvShape &s,
-                  const PassOperands &o, const float *bias, void *out, bool swapped, int groups, bool slower_too, IgemmProblem *r) {
+                  const PassOperands &o, const float *bias, void *out, bool swapped, int groups, bool slower_too, IgemmProblem *r,
+                  RowsTiling *rows) {
   if ((!pointwise(s) && (s.strH > 8 || s.strW > 8)) || s.KH <= 0 || s.KW <= 0) return false;
   *r = convFwdProblem(p, opt, s, o, bias, out, swapped);
   r->plan_flags |= plan_flags;
   const bool packed = p.groups == 1 && p.input_type != PLB_FLOAT && !swapped && !channelsFitTma(p, p.in_chans_per_group);
-  return patchSuits(sm_count, r, 1, p.input_type, 1, groups, operandsCopied(o, p.in_chans_per_group), packed, slower_too);
+  return patchSuits(sm_count, r, 1, p.input_type, 1, groups, operandsCopied(o, p.in_chans_per_group), packed, slower_too, rows);
 }
 // The one-launch routes of a forward pass, tried before the others: straight from the image
-// (`shape`), or on the patch kernel (`r`).  `slower_too`: where the others would be quicker, but
+// (`shape`), or on the patch kernel (`r`) or that for rows in its place (`rows`).  `slower_too`: where the others would be quicker, but
 // cannot have the scratch memory that they need.
 enum class FwdRoute { kOther, kStem, kPatch };
 FwdRoute fwdRoute(int sm_count, const plb_conv_params &p, const plb_conv_options *opt, int plan_flags, const ConvShape &s,
                   const PassOperands &o, const float *bias, void *out, bool swapped, int groups, bool slower_too, IgemmProblem *r,
-                  S2dShape *shape) {
+                  RowsTiling *rows, S2dShape *shape) {
   if (is16BitFloat(p.input_type) && p.groups == 1 && !channelsFitTma(p, p.in_chans_per_group) && !swapped &&
       stemLayer(sm_count, plan_flags, p, opt, out, slower_too, shape))
     return FwdRoute::kStem;
-  return fwdOnPatches(sm_count, p, opt, plan_flags, s, o, bias, out, swapped, groups, slower_too, r) ? FwdRoute::kPatch : FwdRoute::kOther;
+  return fwdOnPatches(sm_count, p, opt, plan_flags, s, o, bias, out, swapped, groups, slower_too, r, rows) ? FwdRoute::kPatch : FwdRoute::kOther;
 }
 // (the number of problems, 0 if it does not)
 int bwdOnPatches(int sm_count, const plb_conv_params &p, const plb_conv_options *opt, int plan_flags, const ConvShape &s,
-                 const PassOperands &o, void *dx, int groups, bool slower_too, IgemmProblem *r) {
+                 const PassOperands &o, void *dx, int groups, bool slower_too, IgemmProblem *r, RowsTiling *rows) {
   int n = 0, contractions = 0;
   if (s.strH == 1 && s.strW == 1) {
     r[n++] = convBwdProblem(p, opt, s, o, dx, false);
@@ -761,7 +762,7 @@ int bwdOnPatches(int sm_count, const plb_conv_params &p, const plb_conv_options 
   }
   if (n == 0) return 0;
   r[0].plan_flags |= plan_flags;
-  return patchSuits(sm_count, r, n, p.input_type, contractions, groups, operandsCopied(o, p.out_chans_per_group), false, slower_too) ? n : 0;
+  return patchSuits(sm_count, r, n, p.input_type, contractions, groups, operandsCopied(o, p.out_chans_per_group), false, slower_too, rows) ? n : 0;
 }
 
 // Narrow channel groups are contracted together (grouped.cu): `q` = the layer of
@@ -1094,10 +1095,11 @@ int plb_conv_plan(const plb_conv_params *p_in, const plb_conv_options *opt, int3
     const PassOperands o{p->input_type, nullptr, nullptr, bwd ? p->out_chans_per_group : p->in_chans_per_group,
                          bwd ? p->out_chans_per_group : p->in_chans_per_group, p->in_chans_per_group};
     S2dShape g;
+    RowsTiling rows;
     FwdRoute route = FwdRoute::kOther;
     if (!bwd)
-      route = fwdRoute(148, *p, opt, 0, s, o, nullptr, nullptr, false, int(together), false, r, &g);
-    else if (bwdOnPatches(148, *p, opt, 0, s, o, nullptr, int(together), false, r) > 0)
+      route = fwdRoute(148, *p, opt, 0, s, o, nullptr, nullptr, false, int(together), false, r, &rows, &g);
+    else if (bwdOnPatches(148, *p, opt, 0, s, o, nullptr, int(together), false, r, &rows) > 0)
       route = FwdRoute::kPatch;
     if (route == FwdRoute::kPatch) plan->kernel = 3;
     plan->in_place = route == FwdRoute::kOther ? 0 : 1;
@@ -1184,13 +1186,15 @@ int plb_convolution(plb_context *ctx, const plb_conv_params *p, const plb_conv_o
   // in one launch, without scratch, where that is quicker, or where scratch cannot be had
   auto inPlace = [&](bool slower_too, int *rc) {
     IgemmProblem r;
+    RowsTiling rows;
     S2dShape g;
     const int groups = groupsTogether(p->groups, p->in_chans_per_group, p->out_chans_per_group, p->input_type);
-    const FwdRoute route = fwdRoute(ctx->sm_count, *p, opt, ctx->plan_flags, s, separate, d_bias, d_out, swapped, groups, slower_too, &r, &g);
+    const FwdRoute route =
+        fwdRoute(ctx->sm_count, *p, opt, ctx->plan_flags, s, separate, d_bias, d_out, swapped, groups, slower_too, &r, &rows, &g);
     if (route == FwdRoute::kStem)
       *rc = launchStem(ctx, g, int(p->out_chans_per_group), p->input_type == PLB_BFLOAT16, d_in, d_weights, d_bias, d_out);
     else if (route == FwdRoute::kPatch)
-      *rc = launchPatch(ctx, &r, 1, p->input_type, groups > 1);
+      *rc = rows.blocks ? launchRows(ctx, r, rows) : launchPatch(ctx, &r, 1, p->input_type, groups > 1);
     return route != FwdRoute::kOther;
   };
   int done = PLB_OK;
@@ -1283,9 +1287,10 @@ int plb_conv_bwd(plb_context *ctx, const plb_conv_params *p, const plb_conv_opti
   // in one launch, without scratch, where that is quicker, or where scratch cannot be had
   auto inPlace = [&](bool slower_too, int *rc) {
     IgemmProblem r[kPatchMaxPhases];
+    RowsTiling rows;
     const int groups = groupsTogether(p->groups, p->in_chans_per_group, p->out_chans_per_group, p->input_type);
-    const int n = bwdOnPatches(ctx->sm_count, *p, opt, ctx->plan_flags, s, separate, d_in_grads, groups, slower_too, r);
-    if (n > 0) *rc = launchPatch(ctx, r, n, p->input_type, groups > 1);
+    const int n = bwdOnPatches(ctx->sm_count, *p, opt, ctx->plan_flags, s, separate, d_in_grads, groups, slower_too, r, &rows);
+    if (n > 0) *rc = rows.blocks ? launchRows(ctx, *r, rows) : launchPatch(ctx, r, n, p->input_type, groups > 1);
     return n > 0;
   };
   int done = PLB_OK;

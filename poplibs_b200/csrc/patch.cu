@@ -3,7 +3,6 @@
 #include <cmath>
 
 #include "patch.cuh"
-#include "rows.h"
 
 namespace plb {
 
@@ -182,9 +181,11 @@ bool patchable(const IgemmProblem *p, int n, int type) {
 // leave 26 of those, and give up 22 that gain (3x3, 2 groups of 32, 42 images of 13 x 13, where 294 blocks
 // wait for the same weights, 13.0 -> 7.5 us; 1x1, 2 groups of 32, 8 of 35 x 35 8.8 -> 5.6).
 bool patchSuits(int sm_count, const IgemmProblem *p, int n, int type, int contractions, int together, bool copied, bool packed,
-                bool slower_too) {
+                bool slower_too, RowsTiling *rows) {
+  rows->blocks = 0;
   if (!patchable(p, n, type)) return false;
-  if (n == 1 && rowsSuits(sm_count, *p, type)) return true;
+  if (n == 1 && rowsSuits(sm_count, *p, type, rows)) return true;
+  rows->blocks = 0;
   const double operand = (type == PLB_FLOAT ? 6.0 : type == PLB_QUARTER ? 1.0 : 2.0) * together * p->k_per_tap;
   const double columns = double(together) * p->n_total, wide = columns <= 64 ? 1 : columns <= 128 ? 1.6 : 2.6;
   const double tile_n = columns <= 64 ? 64 : columns <= 128 ? 128 : 256;
@@ -217,7 +218,6 @@ bool patchSuits(int sm_count, const IgemmProblem *p, int n, int type, int contra
 }
 
 int launchPatch(plb_context *ctx, const IgemmProblem *p, int n, int type, bool repair) {
-  if (n == 1 && rowsSuits(ctx->sm_count, *p, type)) return launchRows(ctx, *p);
   Tiling t;
   const bool act_vec = wholeLoads(*p, type);
   if (!tilingOf(ctx->sm_count, p, n, type, act_vec, &t)) return fail(PLB_ERR_UNSUPPORTED, "no tiling of the patch kernel");

@@ -287,52 +287,33 @@ rowsKernel(const __grid_constant__ RowsArgs g) {
     }
 }
 
-struct RowsTiling {
-  int tile_w, tile_h, tile_n, pitch, steps;
-  size_t smem;
-  long blocks;
-  float us;
-};
-
-int ceilDiv(long a, long b) { return int((a + b - 1) / b); }
-
 // The tile of the least estimated time: rounds of blocks (those of the last begin as others end),
 // each its loads and stores, and the instructions of all the SM's warps or the latency of one
 // warp's walk.  Fitted to 1900 tiles of 110 layers, whose times it is 16 % off; the tile that it takes is 1.2 %
 // slower than a layer's best in the mean (with products alone for instructions, and whole rounds, 6 %).
 bool rowsTiling(int sms, const IgemmProblem &p, RowsTiling *best) {
-  const int K = p.taps_w, c = p.k_per_tap;
-  const long slabs = ceilDiv(long(p.groups) * c, 64);
+  const int K = p.taps_w, c = p.k_per_tap, most = c == 8 || K == 5 ? 2 : 3;
+  const long slabs = upDiv(unsigned(p.groups * c), 64);
   // cycles of a 16-pixel step of a row: its products at the rate of the SM's four pipes
   const double products = c == 8 ? K * (8.3 * (K / 2) + 4.2) : 2 * K * K * 8.3;
   bool found = false;
-  for (int steps = 1; steps <= 7; ++steps)
-    for (int images = 1; images <= 2; ++images) {
-      if (images == 2 && (steps > 1 || p.out_w > 8)) continue;
-      RowsTiling t{};
-      t.tile_w = 16 * steps / images;
-      t.tile_n = images;
-      t.pitch = (t.tile_w + K - 1 + 7) / 8 * 8;
-      if (steps > 1 && t.tile_w - 16 >= p.out_w) break;
-      for (int rows = 1; rows <= p.out_h; ++rows) {
-        t.tile_h = ceilDiv(p.out_h, ceilDiv(p.out_h, rows));
-        if (t.tile_h != rows) continue;
-        t.smem = size_t(images) * (rows + K - 1) * t.pitch * kRowBytes;
-        if (t.smem > 110 * 1024) break;
-        const int most = c == 8 || K == 5 ? 2 : 3, resident = std::max(1, std::min<int>(most, int(226 * 1024 / (t.smem + 1024))));
-        t.blocks = slabs * ceilDiv(p.out_w, t.tile_w) * ceilDiv(p.out_h, rows) * ceilDiv(p.out_n, images);
-        const double share = double(t.blocks) / (sms * resident), rounds = std::max(1.0, 0.425 * std::ceil(share) + 0.575 * share);
-        const double here = std::min<double>(resident, std::ceil(double(t.blocks) / sms));
-        const double load = double(images) * (rows + K - 1) * (t.tile_w + K - 1) * kRowBytes;
-        const double store = double(images) * rows * std::min(t.tile_w, p.out_w) * kRowBytes;
-        // (an even number of steps of 3x3 filters is walked by twos)
-        const bool twos = steps % 2 == 0 && K == 3;
-        const double walked = (rows + K - 1.0) * steps;
-        const double all = walked * (0.747 * products + (twos ? 4.0 : 14.2)) * (64 / c) * here / 4;
-        const double one = walked * (1.34 * products + (twos ? 84 : 168));
-        t.us = float(1.49 + rounds * (1781 + here * (0.0413 * load + 0.0192 * store) + std::max(all, one)) / 1900);
-        t.steps = steps;
-        if (!found || t.us < best->us) *best = t;
+  for (int steps = 1; steps <= 7 && (steps == 1 || 16 * (steps - 1) < p.out_w); ++steps)
+    for (int images = 1; images <= (steps == 1 && p.out_w <= 8 ? 2 : 1); ++images) {
+      const int tile_w = 16 * steps / images, pitch = (tile_w + K - 1 + 7) / 8 * 8, row_bytes = images * pitch * kRowBytes;
+      const long columns = slabs * upDiv(p.out_w, tile_w) * upDiv(p.out_n, images);
+      // (an even number of steps of 3x3 filters is walked by twos)
+      const bool twos = steps % 2 == 0 && K == 3;
+      const double load = 0.0413 * images * (tile_w + K - 1) * kRowBytes, store = 0.0192 * images * std::min(tile_w, p.out_w) * kRowBytes;
+      const double all = steps * (0.747 * products + (twos ? 4.0 : 14.2)) * (64 / c) / 4, one = steps * (1.34 * products + (twos ? 84 : 168));
+      for (int rows = std::min(p.out_h, 110 * 1024 / row_bytes - (K - 1)); rows >= 1; --rows) {
+        const unsigned tiles = upDiv(p.out_h, rows);
+        rows = int(upDiv(p.out_h, tiles));  // (the fewest that make as many tiles)
+        const int smem = row_bytes * (rows + K - 1), resident = std::max(1, std::min(most, int(226u * 1024 / unsigned(smem + 1024))));
+        const long blocks = columns * tiles;
+        const double share = double(blocks) / (sms * resident), rounds = std::max(1.0, 0.425 * up(share) + 0.575 * share);
+        const double here = std::min(double(resident), up(double(blocks) / sms)), walked = rows + K - 1;
+        const float us = float(1.49 + rounds * (1781 + here * (load * walked + store * rows) + walked * std::max(all * here, one)) / 1900);
+        if (!found || us <= best->us) *best = RowsTiling{tile_w, rows, images, pitch, steps, size_t(smem), blocks, us};
         found = true;
       }
     }
@@ -346,7 +327,7 @@ bool rowsTiling(int sms, const IgemmProblem &p, RowsTiling *best) {
 // Beyond them the persistent blocks of the tensor-core route stream better (3x3, 8 groups of 16, 34 images of
 // 110 x 110, 105 MB, forward: 62 there, 81 here; 30.8 MB 26 and 28), 5x5 of 16 channels is bound by mma.sync
 // (10 MB: 21 and 25), and two groups of 8 leave six of a block's warps idle (12 MB: 27 and 34).
-bool rowsSuits(int sm_count, const IgemmProblem &p, int type) {
+bool rowsSuits(int sm_count, const IgemmProblem &p, int type, RowsTiling *t) {
   if (type != PLB_HALF || p.groups < 2 || p.out_f32 || p.beta != 0.f || p.addend || p.a_mn || p.plan_flags != 0 ||
       p.force_tile_n != 0 || p.force_split_k != 0)
     return false;
@@ -362,13 +343,10 @@ bool rowsSuits(int sm_count, const IgemmProblem &p, int type) {
   if (p.out_w > 1 << 20 || p.out_h > 1 << 20 || std::abs(p.pad_h) > 1 << 20 || std::abs(p.pad_w) > 1 << 20) return false;
   const double megabytes = 2e-6 * p.groups * c * p.out_w * p.out_h * p.out_n;
   const double most = c == 16 ? (p.taps_w == 5 ? 5 : p.b_mn ? 60 : 28) : p.groups < 4 ? (p.taps_w == 5 ? 0.5 : 5) : p.taps_w == 5 || p.b_mn ? 1e9 : 100;
-  RowsTiling t;
-  return megabytes <= most && rowsTiling(sm_count, p, &t) && t.blocks <= 0x3fffffff;
+  return megabytes <= most && rowsTiling(sm_count, p, t) && t->blocks <= 0x3fffffff;
 }
 
-int launchRows(plb_context *ctx, const IgemmProblem &p) {
-  RowsTiling t;
-  if (!rowsTiling(ctx->sm_count, p, &t)) return fail(PLB_ERR_UNSUPPORTED, "no tiling of the row kernel");
+int launchRows(plb_context *ctx, const IgemmProblem &p, const RowsTiling &t) {
   RowsArgs g{};
   g.act = static_cast<const uint8_t *>(p.act);
   g.wgt = static_cast<const uint8_t *>(p.wgt);
@@ -405,9 +383,9 @@ int launchRows(plb_context *ctx, const IgemmProblem &p) {
   g.image_rows = t.tile_h + p.taps_h - 1;
   g.second = uint32_t(t.tile_n > 1 ? g.image_rows * t.pitch : 8) * kRowBytes;
   g.first_rows = std::min(t.tile_h + p.taps_h - 1, std::max(p.taps_h, (t.tile_h / 2 + p.taps_h - 1) / p.taps_h * p.taps_h));
-  g.slabs = ceilDiv(g.chans, 64);
-  g.tiles_w = ceilDiv(p.out_w, t.tile_w);
-  g.tiles_h = ceilDiv(p.out_h, t.tile_h);
+  g.slabs = int(upDiv(g.chans, 64));
+  g.tiles_w = int(upDiv(p.out_w, t.tile_w));
+  g.tiles_h = int(upDiv(p.out_h, t.tile_h));
   g.fd_slabs = make_fastdiv(uint32_t(g.slabs));
   g.fd_tiles_w = make_fastdiv(uint32_t(g.tiles_w));
   g.fd_tiles_h = make_fastdiv(uint32_t(g.tiles_h));

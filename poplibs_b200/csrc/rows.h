@@ -6,10 +6,25 @@
 
 namespace plb {
 
+// For the searches of tilings, which every call makes: quotients of positive numbers below 2^31
+// rounded up, and the ceiling of one below 2^62 (std::ceil is a call).
+inline unsigned upDiv(unsigned a, unsigned b) { return (a + b - 1) / b; }
+inline double up(double v) {
+  const double whole = double((long long)v);
+  return whole < v ? whole + 1 : whole;
+}
+
+// Output pixels of a block, `steps` sixteens of them to a row of its images.
+struct RowsTiling {
+  int tile_w, tile_h, tile_n, pitch, steps;
+  size_t smem;
+  long blocks;
+  float us;
+};
 // Whether this problem (`type`: the operands' element type, all pointers the caller's) runs
-// on the kernel that walks the rows of a group with its weights in registers.
-bool rowsSuits(int sm_count, const IgemmProblem &p, int type);
-int launchRows(plb_context *ctx, const IgemmProblem &p);
+// on the kernel that walks the rows of a group with its weights in registers, and how.
+bool rowsSuits(int sm_count, const IgemmProblem &p, int type, RowsTiling *t);
+int launchRows(plb_context *ctx, const IgemmProblem &p, const RowsTiling &t);
 
 // Weight gradient of half channel groups, `chans` in and out each, of a kernel x kernel filter with
 // unit strides and dilations.

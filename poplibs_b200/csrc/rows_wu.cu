@@ -202,39 +202,31 @@ rowsWuKernel(const __grid_constant__ RowsWuArgs g) {
         }
 }
 
-int ceilDiv(long a, long b) { return int((a + b - 1) / b); }
-
 bool rowsWuTiling(int sms, const RowsWuProblem &p, RowsWuTiling *best) {
-  const int K = p.kernel, c = p.chans;
+  const int K = p.kernel, c = p.chans, most = c == 8 ? 2 : 3;
   const long slabs = rowsWuSlabs(p);
   // cycles of a 16-pixel step of a row
   const double step = (c == 8 ? K * (K / 2 + 1) : 2 * K * K) * 8.3;
+  const double sums = 1.0e-6 * p.groups * K * K * c * c * 4 / 2.5;
   bool found = false;
-  for (int steps = 1; steps <= 7; ++steps)
-    for (int images = 1; images <= 2; ++images) {
-      if (images == 2 && (steps > 1 || p.width > 8)) continue;
-      RowsWuTiling t{};
-      t.tile_w = 16 * steps / images;
-      t.tile_n = images;
-      t.pitch = (t.tile_w + K - 1 + 7) / 8 * 8;
-      if (steps > 1 && t.tile_w - 16 >= p.width) break;
-      for (int rows = 1; rows <= p.height; ++rows) {
-        t.tile_h = ceilDiv(p.height, ceilDiv(p.height, rows));
-        if (t.tile_h != rows) continue;
-        t.x_bytes = size_t(images) * (rows + K - 1) * t.pitch * kRowBytes;
-        t.smem = t.x_bytes + size_t(images) * rows * t.tile_w * kRowBytes;
-        if (t.smem > 110 * 1024) break;
-        const int most = c == 8 ? 2 : 3, resident = std::max(1, std::min<int>(most, int(226 * 1024 / (t.smem + 1024))));
-        t.tiles = long(ceilDiv(p.width, t.tile_w)) * ceilDiv(p.height, rows) * ceilDiv(p.images, images);
-        t.splits = int(std::max<long>(1, std::min<long>(t.tiles, sms * resident / slabs)));
-        const double rounds = ceilDiv(t.tiles, t.splits);
-        const double here = std::min<double>(resident, std::ceil(double(t.splits) * slabs / sms));
-        const double load = double(images) * ((rows + K - 1) * (t.tile_w + K - 1) + rows * t.tile_w) * kRowBytes / 30;
-        const double walk = (rows + K - 1) * steps * step;
+  for (int steps = 1; steps <= 7 && (steps == 1 || 16 * (steps - 1) < p.width); ++steps)
+    for (int images = 1; images <= (steps == 1 && p.width <= 8 ? 2 : 1); ++images) {
+      const int tile_w = 16 * steps / images, pitch = (tile_w + K - 1 + 7) / 8 * 8;
+      const int x_row = images * pitch * kRowBytes, dy_row = images * tile_w * kRowBytes;
+      const long columns = long(upDiv(p.width, tile_w)) * upDiv(p.images, images);
+      const double load = images * kRowBytes / 30.0;
+      for (int rows = std::min(p.height, (110 * 1024 - x_row * (K - 1)) / (x_row + dy_row)); rows >= 1; --rows) {
+        const unsigned parts = upDiv(p.height, rows);
+        rows = int(upDiv(p.height, parts));  // (the fewest that make as many tiles)
+        const int x_bytes = x_row * (rows + K - 1), smem = x_bytes + dy_row * rows;
+        const int resident = std::max(1, std::min(most, int(226u * 1024 / unsigned(smem + 1024))));
+        const long tiles = columns * parts, splits = std::max<long>(1, std::min<long>(tiles, sms * resident / slabs));
+        const double rounds = up(double(tiles) / double(splits)), here = std::min(double(resident), up(double(splits * slabs) / sms));
+        const double bytes = load * ((rows + K - 1) * (tile_w + K - 1) + rows * tile_w), walk = (rows + K - 1) * steps * step;
         const double busy = std::max(walk * (64 / c) * here / 4, walk * 1.6 + (rows + K - 1) * steps * 60.0);
-        t.us = float(2.3 + rounds * (1200 + here * load + busy) / 1900 + 2.5 +
-                     1.0e-6 * double(t.splits) * p.groups * K * K * c * c * 4 / 2.5);
-        if (!found || t.us < best->us) *best = t;
+        const float us = float(2.3 + rounds * (1200 + here * bytes + busy) / 1900 + 2.5 + double(splits) * sums);
+        if (!found || us <= best->us)
+          *best = RowsWuTiling{tile_w, rows, images, pitch, size_t(x_bytes), size_t(smem), tiles, int(splits), us};
         found = true;
       }
     }
@@ -280,8 +272,8 @@ int launchRowsWu(plb_context *ctx, const RowsWuProblem &p, const RowsWuTiling &t
   g.tile_w = t.tile_w;
   g.tile_h = t.tile_h;
   g.tile_n = t.tile_n;
-  g.tiles_w = ceilDiv(p.width, t.tile_w);
-  g.tiles_h = ceilDiv(p.height, t.tile_h);
+  g.tiles_w = int(upDiv(p.width, t.tile_w));
+  g.tiles_h = int(upDiv(p.height, t.tile_h));
   g.tiles = int(t.tiles);
   g.slabs = rowsWuSlabs(p);
   g.splits = t.splits;
