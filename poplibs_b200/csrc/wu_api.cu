@@ -312,7 +312,8 @@ void planWu(const WuProblem &p, int sm_count, int force_split, unsigned plan_fla
   a->ksplit = ksplit;
   if (plan) {
     plan->kernel = 1;
-    // (paired: 64 output channels' sums of all filter rows)
+    // (paired: a CTA's tile is 64 output channels' sums of all filter rows, in instructions of 128 rows and half
+    // the columns)
     plan->tile_m = a->pair_rows ? 64 : 128;
     plan->tile_n = (a->pair_rows ? s.KH : a->taps_per_group) * a->ci_blk;
     plan->tile_k_bytes = kWuPixelsPerStage * 2;
@@ -324,7 +325,7 @@ void planWu(const WuProblem &p, int sm_count, int force_split, unsigned plan_fla
     plan->tiles = units;
     plan->grid = units * ksplit;
     plan->b_mn_major = 1;
-    plan->halo_rows = a->pair_rows ? a->pair_shift : a->strip_mode ? halo : 0;
+    plan->halo_rows = a->pair_rows ? (a->pair_rows - 1) * s.dilH : a->strip_mode ? halo : 0;
     plan->workspace_bytes = size_t(ksplit) * p.sgroups * taps * co * ci * sizeof(float);
   }
 }

@@ -358,8 +358,8 @@ static void testGraphConstructionWithoutDevice() {
       const auto costs = internal::reportDetailedPlanEstimatedCosts(graph, q, {{"pass", "TRAINING_FWD"}});
       CHECK(costs.rearrangement.cycles == 0 && costs.total.memory == 0);
     }
-    // (the second: narrow groups, whose partial sums take workspace)
-    for (const ConvParams &q : {p, ConvParams(HALF, HALF, 2, {9, 13}, {3, 3}, 8, 8, 16)}) {
+    // (narrow groups, whose partial sums take workspace, and two filter rows in the halves of a tile)
+    for (const ConvParams &q : {p, ConvParams(HALF, HALF, 2, {9, 13}, {3, 3}, 8, 8, 16), ConvParams(HALF, HALF, 64, {64, 64}, {2, 1}, 64, 64, 1)}) {
       std::ostringstream wu1, wu2;
       reportWeightUpdatePlanInfo(wu1, graph, q, {{"planConstraintsOutputFilename", base}});
       std::ifstream in(base + "_WU.json");

@@ -251,14 +251,21 @@ def test_weight_update_plans_describe_what_runs():
 
 @pytest.mark.parametrize("n,field,kernel,ci,co,groups", [
     (39, [27, 7], [3, 1], 160, 64, 1), (30, [11, 7], [5, 2], 96, 60, 1), (7, [17, 37], [5, 1], 96, 64, 1),
-    (1, [29, 57], [7, 1], 8, 32, 2), (2, [25, 88], [7, 1], 16, 32, 2), (256, [56, 56], [3, 3], 64, 64, 1)])
+    (1, [29, 57], [7, 1], 8, 32, 2), (64, [64, 64], [2, 1], 64, 64, 1), (2, [25, 88], [7, 1], 16, 32, 2), (256, [56, 56], [3, 3], 64, 64, 1)])
 def test_saved_plans_of_weight_updates_reproduce_them(n, field, kernel, ci, co, groups):
     """A plan's split and strips given as constraints lead to the same tiling, where the tiles are
     fewer than the CTAs that there is room for, too."""
     p = capi.ConvParams.make(n, field, kernel, ci, co, groups=groups, padding=[k // 2 for k in kernel])
     free = capi.conv_wu_plan(p)
-    fixed = capi.conv_wu_plan(p, capi.ConvOptions.make(split_k=free.split_k, plan_flags=0 if free.halo_rows else capi.PLAN_NO_HALO))
+    fixed = capi.conv_wu_plan(p, capi.ConvOptions.make(split_k=free.split_k, plan_flags=0 if free.halo_rows or free.tile_m == 64 else capi.PLAN_NO_HALO))
     assert bytes(free) == bytes(fixed)
+
+
+@pytest.mark.parametrize("rows,dilation,halo", [(2, 1, 0), (3, 1, 1), (4, 2, 2), (7, 1, 3), (3, 3, 3)])
+def test_halved_weight_updates_say_how_many_more_rows_they_read(rows, dilation, halo):
+    """64 output channels' sums of all filter rows, from strips for one half of the filter rows."""
+    plan = capi.conv_wu_plan(capi.ConvParams.make(64, [64, 64], [rows, 1], 64, 64, k_dilation=[dilation, 1]))
+    assert (plan.tile_m, plan.tile_n, plan.halo_rows) == (64, rows * 64, halo)
 
 
 @pytest.mark.parametrize("groups,chans,n,field,k", [(2, 8, 256, [56, 56], 3), (32, 8, 32, [28, 28], 3), (8, 8, 64, [40, 40], 5), (4, 16, 4, [9, 8], 3)])
