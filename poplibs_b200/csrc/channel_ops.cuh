@@ -713,17 +713,24 @@ int chanSums(plb_context *ctx, const T *x, const T *y, const T *centre, uint64_t
       std::max<uint64_t>({uint64_t(ctx->sm_count) / 4, uint64_t(ctx->sm_count) * 128 / std::max(chans, 1u), bytes / (256 * 1024)});
   // Few rows: one launch of clusters over narrow columns (halves, with the two launches below before:
   // 64 x 64 3.2 -> 2.2 us, 784 x 1024 5.3 -> 3.4, 4096 x 64 4.5 -> 3.4, 4096 x 256 7.0 -> 3.6, 8192 x 512 7.9 -> 4.6;
-  // floats alike).  Eight blocks have all the rows of a column: up to 64 columns slabs over the whole
-  // device are quicker from 8192 rows on (two sums 5.0 against 5.3), up to 128 from 12544 (6.1 against 7.1), with
-  // up to 512, where those leave wide rows of sums, from 16384 (floats 10.0 against 11.1), above that from
-  // 6272 (floats 7.8 against 8.6).
-  if (vec && chans % kVec == 0 && rows <= (chans <= 64 ? 6144u : chans <= 128 ? 8192u : chans <= 512 ? 12544u : 4096u))
-    return launchChanCluster<T, kMode, kVec>(ctx, rows, chans, x, y, centre, fin);
-  // Rows that are no whole vectors, and those up to 8192: two short launches over narrow columns,
+  // floats alike).  Eight blocks have all the rows of 64 columns.  Up to 64 columns the other forms
+  // are quicker from 8192 rows on (two sums 5.0 against 5.3), up to 16 from 4096 (5000 x 8, two sums 3.6
+  // against 4.1), up to 128 from 12544 (6.1 against 7.1), up to 768, where slabs leave wide rows of sums
+  // (8192 x 768 halves 8.5 against 4.7), from 16384 (floats 10.0 against 11.1).  Wider
+  // rows have more clusters than the SMs hold at once, which is worth it where single blocks have
+  // a column (256 x 16384 halves 4.5, the two launches 8.2) or sums of moderate size come in few waves (1024 x 2048
+  // halves 3.4, 6.8; 4096 x 1024 6.2, slabs 7.8), not beyond (1024 x 16384 floats 45 against 19, 2048 x 4096
+  // halves 14.4 against 11.2, 4096 x 8192 28 against 22).
+  const bool whole = vec && chans % kVec == 0;
+  const bool clusters = chans <= 768 ? rows <= (chans <= 16 ? 4095u : chans <= 64 ? 6144u : chans <= 128 ? 8192u : 12544u)
+                                     : rows <= 4 * (kClusterThreads / (kColChans / kVec)) || bytes < (uint64_t(6) << 20) ||
+                                           (rows > 2560 && bytes <= (uint64_t(24) << 20));
+  if (whole && clusters) return launchChanCluster<T, kMode, kVec>(ctx, rows, chans, x, y, centre, fin);
+  // The others up to 8192, and more that are no whole vectors: two short launches over narrow columns,
   // where a block's wide row of sums would be most of the work and the last block's finish most of
   // the time (324 x 253 halves 7.8 -> 3.6 us, 1058 x 351 floats 7.7 -> 4.2, 8281 x 64 halves 5.7 -> 5.5; 16641
   // x 64 5.7 against 6.9; 16641 x 255 halves 10.8 -> 7.5).
-  if (rows <= (vec && chans % kVec == 0 ? 8192u : 24576u) && bytes <= (uint64_t(16) << 20))
+  if (rows <= (whole ? 8192u : 24576u) && bytes <= (uint64_t(16) << 20))
     return launchChanColumns<T, kMode>(ctx, rows, chans, x, y, centre, fin);
   if (!vec) return launchChanSums<T, kMode, 1, 512>(ctx, rows, chans, most_slabs, x, y, centre, fin);
   // Twice the warps keep the loads of a long slab going while a part of them adds (64
