@@ -9,9 +9,11 @@
 // shared memory: a row of activations, read once by ldmatrix for each horizontal tap (turned round:
 // the pixels are the reduction; two taps of 8 channels are the sixteen rows of an
 // instruction), is multiplied with the output gradients of all the rows that it meets, which are
-// kept in a ring of registers, one for each filter row.  Only products that exist are formed:
-// rows beyond the tile are skipped, pixels beyond the image are zero in both operands.  A second
-// kernel adds the shares in their order (wu_reduce4_kernel).
+// kept in a ring of registers, one for each filter row.  Rows beyond the tile are skipped, pixels
+// beyond the output are zero in both operands, so that an infinite activation meets no gradients that do not
+// exist.  Padding is multiplied as zeros: an infinite gradient makes NaNs of the sums of the taps that
+// reach padding from its pixel, as in the contraction (wu_sm100.cuh).  A second kernel adds the
+// shares in their order (wu_reduce4_kernel).
 //
 // Bound by latency and the loads' rate: two or three blocks share an SM, one multiplies while
 // another loads.  32 groups of 8 on 32 images of 28 x 28: 18.3 -> 14.7 us with the second kernel.
