@@ -77,3 +77,48 @@ def test_wu_pair_keeps_infinities_of_edge_rows_to_their_taps(gpu_ctx, pad, row, 
     for k in range(3):
         # tap k meets the input row where output row `row` + pad - k exists
         assert finite[:, 3, k].all() != (0 <= row + pad - k < oh), k
+
+
+# images, field, kernel, groups, channels of each in / out, type: the other operands that the planner
+# sends here: bfloat16, the pieces of floats, and groups contracted together to 64 output channels
+# (all of them, with channels left over, and some of several)
+FORMS = {
+    "bfloat16": (5, (34, 48), (3, 3), 1, 64, 64, "bfloat16"),
+    "bfloat16, 40 in, 7 rows": (3, (30, 32), (7, 3), 1, 40, 64, "bfloat16"),
+    "bfloat16, groups": (6, (24, 32), (5, 5), 4, 16, 16, "bfloat16"),
+    "float": (5, (34, 48), (3, 3), 1, 64, 64, "float32"),
+    "float, 5 rows": (4, (24, 48), (5, 5), 1, 64, 64, "float32"),
+    "float, groups": (3, (24, 32), (5, 5), 4, 16, 16, "float32"),
+    "4 groups of 16": (6, (24, 32), (5, 5), 4, 16, 16, "float16"),
+    "8 groups of 8": (6, (24, 32), (7, 7), 8, 8, 8, "float16"),
+    "3 groups of 20": (6, (24, 32), (5, 5), 3, 20, 20, "float16"),
+    "8 groups, 32 to 16": (6, (24, 32), (3, 3), 8, 32, 16, "float16"),
+    "10 groups, 32 to 16": (6, (24, 32), (3, 3), 10, 32, 16, "float16"),
+}
+
+
+@pytest.mark.parametrize("name", FORMS)
+def test_wu_pair_of_other_operands(gpu_ctx, name):
+    import torch
+    n, field, kernel, g, ci, co, dtype = FORMS[name]
+    plb = {"float16": capi.HALF, "bfloat16": capi.BFLOAT16, "float32": capi.FLOAT}[dtype]
+    pad = [k // 2 for k in kernel]
+    p = capi.ConvParams.make(n, list(field), list(kernel), ci, co, groups=g, input_type=plb,
+                             output_type=capi.FLOAT if plb == capi.FLOAT else capi.HALF, padding=pad)
+    torch.manual_seed(len(name))
+    # (floats of more bits than one piece has: the sums of their products are exact all the same)
+    most = 300 if plb == capi.FLOAT else 2
+    x = torch.randint(-most, most + 1, (n, *field, g * ci), device="cuda").to(getattr(torch, dtype))
+    dy = torch.randint(-2, 3, (n, *field, g * co), device="cuda").to(x.dtype)
+    dw = torch.full((g, *kernel, co, ci), 7.0, device="cuda")
+    nchw = lambda t: t.permute(0, 3, 1, 2).double()
+    want = torch.nn.grad.conv2d_weight(nchw(x), (g * co, ci, *kernel), nchw(dy), padding=pad, groups=g)
+    torch.cuda.synchronize()
+    for split in (1, 2):
+        opt = capi.ConvOptions.make(split_k=split)
+        assert capi.conv_wu_plan(p, opt).tile_m == 64
+        gpu_ctx.conv_wu(p, x, dy, None, dw, opt=opt)
+        gpu_ctx.synchronize()
+        assert torch.equal(dw.permute(0, 3, 4, 1, 2).reshape(want.shape).double(), want), split
+        dw.fill_(7.0)
+        torch.cuda.synchronize()
