@@ -173,8 +173,8 @@ bool patchable(const IgemmProblem *p, int n, int type) {
 // groups contracted together (`packed`: of all taps of a row together).  Of the 478 it takes
 // 127, which run in 0.59 of their time, two of them slower (by 6 and 11 %; 3x3, 2 groups of 8,
 // 3 images of 14 x 95 8.5 -> 4.4 us; 3x3/2, 32 groups of 8, 2 of 8 x 108, input gradient 20.6 ->
-// 9.3); 32 groups of 8 on 32 images of 28 x 28 stay (17.8 against 21.2), and so do ungrouped
-// layers that are one launch (56 x 56, 64 channels: 5.3 against 11.2).
+// 9.3); ungrouped layers that are one launch stay (56 x 56, 64 channels: 5.3 against 11.2).
+// Groups of 8 and 16 that the row kernel takes (rows.cu) are not estimated.
 // Unless the general route packs its operand rows, both times are estimated once more, fitted to
 // 4200 passes (median errors 7 and 8 %, a tenth of them 20 and 23 %): of 1800 that the first
 // estimates took, 103 were more than 8 % slower than on the general route, up to 1.7 times; the second

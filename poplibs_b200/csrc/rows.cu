@@ -17,7 +17,8 @@
 // about 30 MB on by the rate at which those blocks keep loads in flight (2.7 TB/s read and
 // written).  Shared memory's rows are whole eights of pixels, so that the swizzle of a lane's addresses
 // is the same in every row: with addresses formed per tap, a 16-pixel step took 160 instructions and
-// 32 groups of 8 on 32 images of 28 x 28 20.5 us, now 10.0 (17.8 in three launches on dense blocks).
+// 32 groups of 8 on 32 images of 28 x 28 20.5 us, now 10.0 (17.8 in three launches on dense blocks;
+// operands in L2, 11.5 us from memory).
 #include <algorithm>
 #include <atomic>
 #include <cmath>

@@ -16,7 +16,8 @@
 // shares in their order (wu_reduce4_kernel).
 //
 // Bound by latency and the loads' rate: two or three blocks share an SM, one multiplies while
-// another loads.  32 groups of 8 on 32 images of 28 x 28: 18.3 -> 14.7 us with the second kernel.
+// another loads.  32 groups of 8 on 32 images of 28 x 28: 18.3 -> 14.9 us with the second kernel (operands
+// in L2, 17.0 from memory).
 #include <algorithm>
 #include <atomic>
 #include <cmath>

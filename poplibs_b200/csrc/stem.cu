@@ -14,12 +14,12 @@
 // apart; a tile is 128 consecutive positions of the strip, the last T-1 of every row not
 // stored.
 //
-// Roles: 7 warps load strips (two in flight), one thread issues the instructions, two groups
+// Roles: 7 warps load strips (two in flight), one issues the instructions, two groups
 // of 4 warps store alternate tiles.  Loads, results and operands share the SM's path to
 // shared memory and L1; a tile of 14 instructions (7x7) takes 1350 cycles of the 670 that the
 // instructions alone would, one of 6 (3x3) is bound by its results.  Measured against the rearranged
 // form: 3x3, 1 -> 96 on 147 images of 118 x 118 122 -> 96 us, 3x3/2, 4 -> 64 on 11 of 102 x 192 9.1 ->
-// 5.4, 7x7/2, 3 -> 64 on 256 of 224 x 224 162 -> 147 (medians of six).  (Whole lines of results, stored from 16
+// 5.4, 7x7/2, 3 -> 64 on 256 of 224 x 224 162 -> 147 to 158 by the device's clock (medians of six).  (Whole lines of results, stored from 16
 // x 256-bit reads of tensor memory, two issuers or four accumulators: no gain.)
 #include <algorithm>
 #include <atomic>

@@ -251,14 +251,15 @@ void planWu(const WuProblem &p, int sm_count, int force_split, unsigned plan_fla
     }
   }
   // Both halves of the instruction's rows for 64 output channels (fewer: the copies take longer
-  // than the instructions): where a 16-pixel step lies in one row, and all tiles then take less.  A tile takes what its instructions do (one of
-  // n columns about 35 + 0.47 n cycles: measured 75, 95, 155 at 64, 128 and 256), its way into
-  // and out of shared memory at 100 bytes a cycle (measured 91 to 110), or its copies by pixel (3.1
-  // cycles, 7.5 where its channels do not fill 128 bytes); and the tiles of a CTA
-  // have to win the 2000 cycles that clearing the accumulators and the edge rows cost (3x3 float,
-  // 20 -> 36, 4 images of 33 x 29, four tiles a CTA: 12.6 us unpaired, 13.3 paired).  Boxes are eight pixels wide
-  // and more: of single columns of 16 images, 3x3, 4 groups of 16, 16 images of 107 x 107 took 44 us,
-  // unpaired 34.
+  // than the instructions): where a 16-pixel step lies in one row, and all tiles then take less.  A tile
+  // takes what its instructions do (one of n columns about 35 + 0.47 n cycles: measured 75, 95, 155 at 64,
+  // 128 and 256), its way into and out of shared memory at 100 bytes a cycle (measured 91 to 110), or
+  // its copies by pixel (3.1 cycles, 7.5 where its channels do not fill 128 bytes); and the tiles of a CTA
+  // have to win 2000 cycles for clearing the accumulators and the edge rows.  (That is on the safe side:
+  // it leaves 5x5, 64 channels, 2 images of 56 x 56 unpaired, 9.6 us, paired 8.7, and 3x3, 4 of 33 x 29, 7.4
+  // and 7.3; it was found with 40 output channels, 12.6 us unpaired and 13.3 paired, which are not paired
+  // now.)  Boxes are eight pixels wide and more: of single columns of 16 images, 3x3, 4 groups of 16, 16 images
+  // of 107 x 107 took 44 us, unpaired 34.
   a->pair_rows = a->pair_shift = 0;
   if (a->strip_mode && co == 64) {
     const int rows = (s.KH + 1) / 2, shift = rows * s.dilH;
