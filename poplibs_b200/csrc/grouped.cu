@@ -203,8 +203,8 @@ int repairNonFinite(plb_context *ctx, const IgemmProblem &p, int type, int in_di
   a.fmt_b = p.fmt_b;
   // Shared memory that is not used: its blocks start early and wait, and next to the contraction's CTAs, whose
   // registers leave room for one of them, and many to an SM they keep the next contraction's out
-  // (1x1, 16 groups of 4 -> 32, 53 images of 7 x 9 8.4 us without, 7.6 with 24 KB, 8.0 with 12; 320 passes of layers of
-  // narrow groups 0.985 of their time in all).
+  // (1x1, 16 groups of 4 -> 32, 53 images of 7 x 9 8.4 us without, 7.5 with; 322 passes of layers of narrow groups
+  // 0.985 of their time in all, 0.995 with 12 KB, 0.987 with 48).
   constexpr size_t kApart = 24 * 1024;
   return launchPdl(ctx, repairKernel, dim3(unsigned(ctx->sm_count)), dim3(128), kApart, a, (const int *)nonfiniteFlag(ctx));
 }

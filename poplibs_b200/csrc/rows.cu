@@ -324,7 +324,7 @@ bool rowsTiling(int sms, const IgemmProblem &p, RowsTiling *best) {
 }  // namespace
 
 // Of 300 sampled layers of 0.1 to 134 MB (2 to 32 groups, 3x3 and 5x5), those within the limits below
-// take 0.66 of their time on the other routes, a few passes of 600 more than 4 % longer, at most 10 %.
+// take 0.66 of their time on the other routes, a few passes of 600 more than 4 % longer, at most 13 %.
 // Beyond them the persistent blocks of the tensor-core route stream better (3x3, 8 groups of 16, 34 images of
 // 110 x 110, 105 MB, forward: 62 there, 81 here; 30.8 MB 26 and 28), 5x5 of 16 channels is bound by mma.sync
 // (10 MB: 21 and 25), and two groups of 8 leave six of a block's warps idle (12 MB: 27 and 34).

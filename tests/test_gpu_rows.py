@@ -13,8 +13,9 @@ from poplibs_b200 import capi
 pytestmark = pytest.mark.gpu
 
 # groups, channels, images, field, kernel, other parameters: rows of less than eight pixels (two images
-# side by side, an odd number of them), of parts, whole and several sixteens, tiles of part rows,
-# one row, more groups than a block takes and fewer, paddings on one side, flipped and truncated
+# side by side in the weight gradient), of parts, whole and several sixteens, one row, more groups than a
+# block takes and fewer, paddings on one side, flipped and truncated.  As small as this, all forward
+# passes and input gradients take tiles of sixteen columns; TILES and WU_TILES below have the others.
 LAYERS = {
     "two images a step": (8, 8, 5, (6, 7), 3, dict(padding=1)),
     "two images a step, 16": (4, 16, 4, (9, 8), 3, dict(padding=1)),
