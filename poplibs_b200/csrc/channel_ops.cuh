@@ -698,12 +698,11 @@ int launchChanSums(plb_context *ctx, uint64_t rows, uint32_t chans, uint64_t mos
                    ctx->d_ticket, fin);
 }
 
+// The forms that leave partial sums in scratch memory.  `vec`: in loads of 16 bytes.
 template <typename T, int kMode>
-int chanSums(plb_context *ctx, const T *x, const T *y, const T *centre, uint64_t rows, uint32_t chans,
-             const ChanFinish &fin) {
+int chanSumsScratch(plb_context *ctx, const T *x, const T *y, const T *centre, uint64_t rows, uint32_t chans, bool vec,
+                    const ChanFinish &fin) {
   constexpr int kVec = 16 / sizeof(T);
-  // (a super-row's columns are counted in 32 bits)
-  const bool vec = aligned16(x) && (y == nullptr || aligned16(y)) && uint64_t(chans) * kVec <= 0xffffffffull;
   // Slabs: one per SM, but each slab's row of sums is work for the last block.  Up
   // to 128 columns that is nothing; wider rows take fewer slabs, down to one per four
   // SMs, unless a slab has 256 KB to read and more (25088 x 256 halves: 9.4 us with 148
@@ -711,6 +710,28 @@ int chanSums(plb_context *ctx, const T *x, const T *y, const T *centre, uint64_t
   const uint64_t bytes = rows * chans * sizeof(T);
   const uint64_t most_slabs =
       std::max<uint64_t>({uint64_t(ctx->sm_count) / 4, uint64_t(ctx->sm_count) * 128 / std::max(chans, 1u), bytes / (256 * 1024)});
+  // The others up to 8192, and more that are no whole vectors: two short launches over narrow columns,
+  // where a block's wide row of sums would be most of the work and the last block's finish most of
+  // the time (324 x 253 halves 7.8 -> 3.6 us, 1058 x 351 floats 7.7 -> 4.2, 8281 x 64 halves 5.7 -> 5.5; 16641
+  // x 64 5.7 against 6.9; 16641 x 255 halves 10.8 -> 7.5).
+  if (rows <= (vec && chans % kVec == 0 ? 8192u : 24576u) && bytes <= (uint64_t(16) << 20))
+    return launchChanColumns<T, kMode>(ctx, rows, chans, x, y, centre, fin);
+  if (!vec) return launchChanSums<T, kMode, 1, 512>(ctx, rows, chans, most_slabs, x, y, centre, fin);
+  // Twice the warps keep the loads of a long slab going while a part of them adds (64
+  // images of 56x56, 256 channels, 103 MB: 20.4 us, with 512 threads 22.0); elsewhere they only
+  // add to what every warp executes once (32 images of 56x56, 64 channels: 7.1 us, 6.8).
+  if (bytes >= (uint64_t(64) << 20))
+    return launchChanSums<T, kMode, kVec, 1024>(ctx, rows, chans, most_slabs, x, y, centre, fin);
+  return launchChanSums<T, kMode, kVec, 512>(ctx, rows, chans, most_slabs, x, y, centre, fin);
+}
+
+template <typename T, int kMode>
+int chanSums(plb_context *ctx, const T *x, const T *y, const T *centre, uint64_t rows, uint32_t chans,
+             const ChanFinish &fin) {
+  constexpr int kVec = 16 / sizeof(T);
+  // (a super-row's columns are counted in 32 bits)
+  const bool vec = aligned16(x) && (y == nullptr || aligned16(y)) && uint64_t(chans) * kVec <= 0xffffffffull;
+  const uint64_t bytes = rows * chans * sizeof(T);
   // Few rows: one launch of clusters over narrow columns (halves, with the two launches below before:
   // 64 x 64 3.2 -> 2.2 us, 784 x 1024 5.3 -> 3.4, 4096 x 64 4.5 -> 3.4, 4096 x 256 7.0 -> 3.6, 8192 x 512 7.9 -> 4.6;
   // floats alike).  Eight blocks have all the rows of 64 columns.  Up to 64 columns the other forms
@@ -726,19 +747,11 @@ int chanSums(plb_context *ctx, const T *x, const T *y, const T *centre, uint64_t
                                      : rows <= 4 * (kClusterThreads / (kColChans / kVec)) || bytes < (uint64_t(6) << 20) ||
                                            (rows > 2560 && bytes <= (uint64_t(24) << 20));
   if (whole && clusters) return launchChanCluster<T, kMode, kVec>(ctx, rows, chans, x, y, centre, fin);
-  // The others up to 8192, and more that are no whole vectors: two short launches over narrow columns,
-  // where a block's wide row of sums would be most of the work and the last block's finish most of
-  // the time (324 x 253 halves 7.8 -> 3.6 us, 1058 x 351 floats 7.7 -> 4.2, 8281 x 64 halves 5.7 -> 5.5; 16641
-  // x 64 5.7 against 6.9; 16641 x 255 halves 10.8 -> 7.5).
-  if (rows <= (whole ? 8192u : 24576u) && bytes <= (uint64_t(16) << 20))
-    return launchChanColumns<T, kMode>(ctx, rows, chans, x, y, centre, fin);
-  if (!vec) return launchChanSums<T, kMode, 1, 512>(ctx, rows, chans, most_slabs, x, y, centre, fin);
-  // Twice the warps keep the loads of a long slab going while a part of them adds (64
-  // images of 56x56, 256 channels, 103 MB: 20.4 us, with 512 threads 22.0); elsewhere they only
-  // add to what every warp executes once (32 images of 56x56, 64 channels: 7.1 us, 6.8).
-  if (bytes >= (uint64_t(64) << 20))
-    return launchChanSums<T, kMode, kVec, 1024>(ctx, rows, chans, most_slabs, x, y, centre, fin);
-  return launchChanSums<T, kMode, kVec, 512>(ctx, rows, chans, most_slabs, x, y, centre, fin);
+  ctx->scratch_refused = false;
+  const int rc = chanSumsScratch<T, kMode>(ctx, x, y, centre, rows, chans, vec, fin);
+  // (in a stream capture scratch cannot grow: few rows do without it, however long that takes)
+  return rc != PLB_OK && ctx->scratch_refused && whole && rows <= 12544
+             ? launchChanCluster<T, kMode, kVec>(ctx, rows, chans, x, y, centre, fin) : rc;
 }
 
 // ---- maps ------------------------------------------------------------------------

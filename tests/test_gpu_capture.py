@@ -62,6 +62,17 @@ def test_ragged_float_product(gpu_ctx):
     assert (got == a.cpu().numpy().astype(np.float64) @ b.cpu().numpy().astype(np.float64)).all()
 
 
+@pytest.mark.parametrize("dtype,rows,chans", [("float", 1024, 4096), ("half", 2048, 8192), ("half", 5000, 8)])
+def test_channel_sums_of_few_rows(gpu_ctx, dtype, rows, chans):
+    """Sums that other forms make more quickly, with scratch."""
+    plb, np_type = (capi.HALF, np.float16) if dtype == "half" else (capi.FLOAT, np.float32)
+    x = ints(T.rng(3), (rows, chans), np_type)
+    beta, gamma = T.empty_dev((chans,), np.float32), T.empty_dev((chans,), np.float32)
+    got = captured(lambda ctx: ctx.norm_param_gradients(plb, x, x, rows, chans, 1.0, None, None, gamma, beta), beta)
+    want = x.cpu().numpy().astype(np.float64)
+    assert (got == want.sum(0)).all() and (gamma.cpu().numpy() == (want * want).sum(0)).all()
+
+
 def test_refused_calls_leave_the_capture(gpu_ctx):
     """A layer that needs copies of its operands, and a call that needs nothing in the same graph."""
     ragged = capi.ConvParams.make(4, [33, 29], [3, 3], 20, 36, padding=1)
